@@ -8,7 +8,7 @@ runtime's own choices.
 # ---- CTA shape: 8 compute warps + 1 producer warp that streams weights ahead of them + 1 finisher warp
 COMPUTE_WARPS = 8
 COMPUTE_THREADS = 32 * COMPUTE_WARPS
-NUM_THREADS = COMPUTE_THREADS + 96     # + producer warp + finisher warp + feeder warp
+NUM_THREADS = COMPUTE_THREADS + 128    # + producer warp + finisher warp + feeder warp + issuer warp
 
 # ---- weight-streaming GEMV path (linear with <= 8 activation rows)
 GEMV_MAX_ROWS = 8
@@ -26,8 +26,8 @@ INST_US, SM_GBPS = 2.0, 40.0    # split-K cost model: fixed us per instruction, 
 # 256-wide output tiles (one activation k-tile feeds two weight tiles) for ops with more than WIDE_MIN_ROWS rows:
 # us per 64-element k-tile of a 128 x 128 / 128 x 256 tile and us per epilogue, from the kernel's timeline (two issuing
 # threads; a 128 x 256 k-tile is one 32 KB weight slot and one N = 256 instruction per 16 K-elements)
-GEMM_BN_WIDE, WIDE_MIN_ROWS = 256, 128
-KTILE_US, KTILE_US_WIDE, EPILOGUE_US, EPILOGUE_US_WIDE = 0.27, 0.42, 3.5, 7.0
+GEMM_BM_WIDE, GEMM_BN_WIDE, WIDE_MIN_ROWS = 256, 256, 128
+KTILE_US, KTILE_US_WIDE, EPILOGUE_US, EPILOGUE_US_WIDE = 0.27, 0.66, 3.5, 3.0
 
 # ---- pointwise / norm / attention tiling
 EW_ROWS, EW_COLS = 32, 512

@@ -1,6 +1,6 @@
 // The persistent megakernel and its C ABI (include/megacute_b200.h).  sm_100a only.
 //
-// One launch executes a whole graph.  grid = number of SMs, one CTA per SM, 10 warps:
+// One launch executes a whole graph.  grid = number of SMs, one CTA per SM, 12 warps:
 //   warps 0-7  compute: fetch this CTA's next instruction (global indices c, c+grid, ...), wait
 //              for its dependency counters (acquire), run the op, publish its arrivals (release);
 //   warp 8     producer: walks the same instruction list ahead of the compute warps and streams
@@ -9,7 +9,9 @@
 //              weights depend on nothing in the launch, so HBM keeps streaming while the compute
 //              warps sit in a dependency hop;
 //   warp 9     finisher: adds the compute warps' partial tiles of a streaming linear, runs its
-//              epilogue and sends the instruction's arrivals.
+//              epilogue and sends the instruction's arrivals;
+//   warp 10    feeder: tiles and MMAs of the tcgen05 prefill attention, activation tiles of the 256 x 256 tile GEMM;
+//   warp 11    issuer: MMAs of the 256 x 256 tile GEMM.
 // This replaces the reference's JIT-traced kernel (megacute/kernel.py:251-571) and its per-op
 // role bodies (megacute/ops/*.py).
 #include <cuda.h>          // CUtensorMap and cuTensorMapEncodeTiled's signature (resolved at run time, libcuda is not linked)
@@ -57,10 +59,16 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         }
         c->w_slot = c->w_phase = 0;
         for (int s = 0; s < kTcWideSlots; ++s) {
-            mbar_init(&c->ww_full[s], 1);
+            mbar_init(&c->ww_full[s], 2);
             mbar_init(&c->ww_empty[s], 1);
         }
-        c->ww_slot = c->ww_phase = 0;
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&c->wacc_full[s], 1);
+            mbar_init(&c->wacc_empty[s], kComputeWarps / 2);
+        }
+        for (int s = 0; s < 4; ++s) mbar_init(&c->wide_told[s], 1);
+        mbar_init(&c->gemm_go, 1);
+        c->wide_uses = c->wide_done = 0;
         mbar_init(&c->attn_go, 1);
         mbar_init(&c->acc_full, kTcIssuers);
         for (int s = 0; s < kKvSlots; ++s) {
@@ -85,10 +93,13 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         // ---------------- finisher warp: epilogues of the streaming linear ----------------
         mk_gemv_finisher(p);
     } else if (warp == kFeederWarp) {
-        // ---------------- feeder warp: tiles and MMAs of the tcgen05 prefill attention ----------------
+        // ---------------- feeder warp: tiles and MMAs of the tcgen05 prefill attention, activation tiles of 256 x 256 tile GEMMs ----------------
         // (a warp of its own rather than a branch of the producer's loop: the call in that loop cost every decode step
         // 0.5 %, whether or not the graph had such an op; here a graph without one costs a walk over the instruction list)
-        mk_attention_feeder(p);
+        mk_feeder(p);
+    } else if (warp == kIssuerWarp) {
+        // ---------------- issuer warp: MMAs of 256 x 256 tile GEMMs ----------------
+        mk_wide_issuer(p);
     } else {
         // ---------------- compute warps ----------------
         // Instruction metadata runs one instruction ahead in shared memory (Meta): while instruction
@@ -148,7 +159,7 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                     break;
                 case MK_OP_GEMM: {
                     // (runs this instruction and the CTA's following ones for as long as they are the body's own: walk.cuh)
-                    const int last = (op->i[10] == 256 && op->ptr[11]) ? mk_run_gemm_wide(p, idx) : mk_run_gemm(p, idx);
+                    const int last = is_wide_gemm(op) ? mk_run_gemm_wide(p, idx) : mk_run_gemm(p, idx);
                     aborting = last < 0;
                     if (!aborting) {
                         slot += (last - idx) / (int)gridDim.x;
@@ -408,7 +419,7 @@ static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
                     break;
                 case MK_OP_GEMM:
                     if (d.i[4] <= 0) why = "tile GEMM: split count";
-                    else if (a0 < 0 || a0 * 128 >= d.i[0]) why = "tile GEMM: m tile outside M";
+                    else if (a0 < 0 || a0 * (long long)(d.i[10] == 256 ? 256 : 128) >= d.i[0]) why = "tile GEMM: m tile outside M";
                     else if (d.i[10] != 0 && d.i[10] != 128 && !(d.i[10] == 256 && d.i[1] % 256 == 0)) why = "tile GEMM: weight rows per tile";
                     else if (a1 < 0 || a1 * (long long)(d.i[10] == 256 ? 256 : 128) >= d.i[1]) why = "tile GEMM: n tile outside N";
                     else if (a2 < 0 || a2 >= d.i[4]) why = "tile GEMM: K split index";
@@ -631,7 +642,7 @@ int mk_program_set_ops(mk_program* p, const mk_op_desc* ops, int n_ops, void* st
         // mixing fp16 activations with bf16 weights raised an illegal-instruction fault): only the packed
         // copy can provide them.  Without one, the op runs the mma.sync body, which converts in registers.
         if (xh && (pack_off || (d.ptr[1] & 15) || d.ld[1] % 8 != 0)) continue;
-        if (!encode_tile_map(maps, d.ptr[0], d.i[0], d.i[2], d.ld[0], d.i[0] <= 64 ? 64 : 128, false, d.i[9] == mk::DT_F16)) continue;
+        if (!encode_tile_map(maps, d.ptr[0], d.i[0], d.i[2], d.ld[0], d.i[10] == 256 ? 256 : d.i[0] <= 64 ? 64 : 128, false, xh)) continue;
         // weights: the packed copy, made when a matrix (address, shape, pitch) is bound for the first
         // time and kept while it stays bound -- rebinding other operands (a new input tensor every
         // call) must not copy gigabytes of weights again; weights changed in place need

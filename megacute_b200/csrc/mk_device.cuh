@@ -14,10 +14,11 @@ namespace mk {
 // ---- CTA shape (mirrors megacute_b200/config.py) --------------------------------------------
 constexpr int kComputeWarps = 8;
 constexpr int kComputeThreads = kComputeWarps * 32;
-constexpr int kThreads = kComputeThreads + 96;           // + one producer warp + one finisher warp + one feeder warp
+constexpr int kThreads = kComputeThreads + 128;          // + one producer warp + one finisher warp + one feeder warp + one issuer warp
 constexpr int kProducerWarp = kComputeWarps;
 constexpr int kFinisherWarp = kComputeWarps + 1;
-constexpr int kFeederWarp = kComputeWarps + 2;           // tile requests and MMA issue of the tcgen05 prefill attention
+constexpr int kFeederWarp = kComputeWarps + 2;           // tile requests and MMA issue of the tcgen05 prefill attention; activation tiles of 256 x 256 tile GEMMs
+constexpr int kIssuerWarp = kComputeWarps + 3;           // MMA issue of 256 x 256 tile GEMMs
 
 // ---- shared memory map -----------------------------------------------------------------------
 constexpr int kGemvRows = 8;                              // weight rows per ring stage
@@ -72,13 +73,20 @@ __host__ __device__ inline void kv_split_range(int n, int S, int s, int& k_begin
     k_end = k_begin + per < n ? k_begin + per : n;
 }
 constexpr int kTcWSlots = 8;
-constexpr int kTcWideSlots = 4;                           // ... of a 128 x 256 tile: the same memory as pairs of slots (256 rows x 64 K-elements, 32 KB)
-constexpr int kTcIssuers = 2;                             // threads that issue tcgen05.mma, each into an accumulator of its own
+// 256 x 256 tiles (op_gemm_tc_wide.cuh): three stages of one weight slot (256 rows x 64 K-elements, 32 KB, in the ring's
+// memory) and one activation slot (the same, in the work area); the rest of the ring's memory holds the epilogue's
+// staging rows (4 KB per compute warp) and the tile's bias
+constexpr int kTcWideSlots = 3;
+constexpr int kTcWideBytes = 2 * kTcTileBytes;            // one slot
+constexpr int kTcWideStageOff = kTcWideSlots * kTcWideBytes;
+constexpr int kTcWideBiasOff = kTcWideStageOff + kComputeWarps * 4096;
+static_assert(kTcWideBiasOff + 256 * 2 <= kRingBytes && kTcXOff + kTcWideSlots * kTcWideBytes <= kWorkBytes, "256 x 256 tiles");
+constexpr int kTcIssuers = 2;                             // threads that issue tcgen05.mma of a 128 x 128 tile, each into an accumulator of its own
 // k-tiles alternate between the issuing threads, and a thread waits for a stage or slot by the parity of its barrier's
 // phase: that is only sound if the same thread consumed the stage's previous round (a thread waiting one round early
 // would find the parity of the round before that complete and read a tile still in flight -- with five activation
 // stages this happened, rarely, as a hang or a launch failure).  So every stage count is a multiple of the issuers.
-static_assert(kTcXStages % kTcIssuers == 0 && kTcXHalfStages % kTcIssuers == 0 && kTcWSlots % kTcIssuers == 0 && kTcWideSlots % kTcIssuers == 0, "stage counts vs issuing threads");
+static_assert(kTcXStages % kTcIssuers == 0 && kTcXHalfStages % kTcIssuers == 0 && kTcWSlots % kTcIssuers == 0, "stage counts vs issuing threads");
 __host__ __device__ constexpr int tc_wslot_off(int slot) { return slot * kTcTileBytes; }
 static_assert(kTcWSlots * kTcTileBytes <= kRingBytes, "weight slots");
 
@@ -97,6 +105,9 @@ struct Params {
     unsigned long long timeout_ns;
     int pf_stages;                // how many ring stages ahead of the ring the producer prefetches into L2
 };
+
+// a tile GEMM bound to the 256 x 256 tcgen05 body (op_gemm_tc_wide.cuh)
+__device__ __forceinline__ bool is_wide_gemm(const mk_op_desc* op) { return op->kind == MK_OP_GEMM && op->i[10] == 256 && op->ptr[11] != 0; }
 
 // Instruction metadata staged in shared memory one instruction ahead of its use.  Everything an
 // instruction needs before its first useful load (its words, its op descriptor, its wait and
@@ -127,8 +138,16 @@ struct Ctrl {                     // lives in the last kCtrlBytes of shared memo
     unsigned long long x_empty[2 * kTcXStages];  // ... the MMAs that read it have completed
     unsigned long long w_full[kTcWSlots];    // ... a weight k-tile has landed in its slot of the ring
     unsigned long long w_empty[kTcWSlots];   // ... the MMAs that read it have completed
-    unsigned long long ww_full[kTcWideSlots];    // ... the same for the 32 KB slots of 128 x 256 tiles (barriers and positions of their
-    unsigned long long ww_empty[kTcWideSlots];   //     own: the producer drains one kind before it fills the other)
+    unsigned long long ww_full[kTcWideSlots];    // 256 x 256 tiles: both operands' k-tiles of a stage have landed (armed once for each)
+    unsigned long long ww_empty[kTcWideSlots];   // ... the MMAs that read the stage have completed
+    unsigned long long wacc_full[2];             // ... every MMA into the accumulator of the tile's rows 0..127 / 128..255 has completed
+    unsigned long long wacc_empty[2];            // ... the four compute warps of those rows have read it
+    unsigned long long gemm_go;                  // ... the compute warps have turned to the first of a run of such instructions: the work
+                                                 //     area is theirs, tensor memory is allocated
+    unsigned long long wide_told[4];             // ... the feeder has written wide_info[]: what the issuing thread runs next
+    int4 wide_info[4];                           //     k-tiles (0: end of the list), accumulators, fp16 operands, sequence number
+    uint32_t wide_uses;                          // ... instructions executed (parity of wacc_full); written behind the barrier that ends one
+    uint32_t wide_done;                          // ... the same at the end of the latest run: the staging rows in the ring's memory are free
     unsigned long long acc_full;      // ... every MMA of the instruction has completed (one arrival per issuing thread)
     unsigned long long kv_full[kKvSlots];    // many-sequence decode attention: a K or V tile has landed in its slot
     unsigned long long kv_empty[kKvSlots];   // ... every compute warp has read it
@@ -143,7 +162,6 @@ struct Ctrl {                     // lives in the last kCtrlBytes of shared memo
     uint32_t x_par;                       // ... bit s: parity of the next completion of x_full[s] and of x_empty[s] (between
                                           //     instructions both have completed equally often); set at an instruction's end
     uint8_t w_slot, w_phase;              // ... the MMA thread's position in the weight slots
-    uint8_t ww_slot, ww_phase;            // ... and in the 32 KB slots
     uint32_t acc_uses;                // ... instructions that have used acc_full (its parity)
     int abort;                    // set once a wait of this CTA gave up or saw the global abort
     int flag;                     // scratch broadcast word (split-KV last arriver)
@@ -432,7 +450,7 @@ __device__ __forceinline__ void report(const Params& p, Ctrl* c, int code, int s
     }
 }
 
-enum { WHERE_RING_FULL = 1, WHERE_RING_EMPTY = 2, WHERE_DEP = 3, WHERE_DRAIN = 4, WHERE_COMBINE = 5, WHERE_CHECK_ARM = 6, WHERE_CHECK_RELEASE = 7 };
+enum { WHERE_RING_FULL = 1, WHERE_RING_EMPTY = 2, WHERE_DEP = 3, WHERE_DRAIN = 4, WHERE_COMBINE = 5, WHERE_CHECK_ARM = 6, WHERE_CHECK_RELEASE = 7, WHERE_STAGING = 8 };
 
 // `patience`: multiple of the time limit this wait allows.  A role that by design waits through everything the CTA does
 // before (the finisher warp, for the dependencies of a streaming linear far down the program) gives twice the limit, so
@@ -450,6 +468,24 @@ __device__ __forceinline__ bool wait_barrier(const Params& p, Ctrl* c, unsigned 
             if (t0 == 0) t0 = now;
             else if (now - t0 > p.timeout_ns * patience) {
                 report(p, c, MK_DEV_TIMEOUT_BARRIER, seq, where, (int)(bar - c->full), (int)parity, 0);
+                return false;
+            }
+        }
+    }
+}
+
+// the same for a shared-memory word that only grows
+__device__ __forceinline__ bool wait_word(const Params& p, Ctrl* c, const uint32_t* word, uint32_t want, int seq, int where) {
+    unsigned long long t0 = 0;
+    for (uint32_t it = 1;; ++it) {
+        if (*(const volatile uint32_t*)word >= want) return true;
+        if ((it & 1023u) == 0) {
+            if (*(volatile int*)&c->abort) return false;
+            if (ld_volatile(&p.status[MK_ST_CODE]) != 0) { c->abort = 1; return false; }
+            unsigned long long now = globaltimer();
+            if (t0 == 0) t0 = now;
+            else if (now - t0 > p.timeout_ns * 2) {
+                report(p, c, MK_DEV_TIMEOUT_BARRIER, seq, where, (int)*(const volatile uint32_t*)word, (int)want, 0);
                 return false;
             }
         }

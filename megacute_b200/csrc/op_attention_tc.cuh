@@ -34,7 +34,7 @@
 // 6 causal, 7 out dtype, 8 dtype of q, k, v; f 0 scale.  args: 0 b, 1 h, 2 query tile.
 #pragma once
 #include "mk_device.cuh"
-#include "op_gemm_tc.cuh"
+#include "tc.cuh"
 
 namespace mk {
 

@@ -27,54 +27,9 @@
 #include "mk_device.cuh"
 #include "mma.cuh"
 #include "op_gemv_common.cuh"
+#include "tc.cuh"
 
 namespace mk {
-
-// instruction descriptor, kind::f16: D = f32 (bits 4-5 = 1), A format (bits 7-9) and B format (bits 10-12):
-// 0 = fp16, 1 = bf16, both K-major, N = 128 (bits 17-22 = N / 8), M = 128 (bits 24-28 = M / 16).  Both
-// operands have one type: bf16, or -- when the activations are runtime-private ones kept in fp16, see
-// passes.promote_temps -- fp16, with the packed weight copy converted to fp16 by the host library.
-__device__ __forceinline__ uint32_t tc_idesc_n(bool fp16, uint32_t n) {
-    const uint32_t fmt = fp16 ? 0u : 1u;
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
-}
-__device__ __forceinline__ uint32_t tc_idesc(bool fp16) { return tc_idesc_n(fp16, 128); }
-
-// shared-memory matrix descriptor of a K-major tile with the 128-byte swizzle: start address,
-// leading byte offset 16 (unused by swizzled K-major layouts), 1024 bytes between 8-row groups,
-// descriptor version 1, layout type 2 (128-byte swizzle).  Advancing 16 K-elements inside the
-// swizzle atom adds 32 bytes to the start address.
-__device__ __forceinline__ uint64_t tc_smem_desc(uint32_t saddr) {
-    return (uint64_t)((saddr & 0x3ffffu) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-__device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// arrives on the mbarrier once every tcgen05.mma this thread has issued so far has completed
-__device__ __forceinline__ void tc_commit(unsigned long long* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-// 32 consecutive fp32 columns of this thread's lane (warp-wide, lanes 32 (warp & 3) .. +31)
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, float* v) {
-    uint32_t r[32];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, "
-        "%18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"          // in the same statement: no use of the registers can move above it
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
-          "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-          "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]),
-          "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
-#pragma unroll
-    for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]);
-}
 
 // the same columns of two accumulators, `second` columns apart, added (second == 0: one accumulator)
 __device__ __forceinline__ void tc_ld32_sum(uint32_t taddr, uint32_t second, float* v) {
@@ -90,20 +45,15 @@ __device__ __forceinline__ void tc_ld32_sum(uint32_t taddr, uint32_t second, flo
 // State the next tile GEMM instruction of this CTA starts from, written by one thread behind the barrier that
 // ends the epilogue: the accumulator barrier's use count, the parities of the activation stages (stage s was
 // used once more per full round through the stages, and once more if s < nk mod stages) and the position in
-// the weight slots (of the kind the instruction used).
+// the weight slots.
 __device__ __forceinline__ void tc_finish_state(Ctrl* c, uint32_t uses, uint32_t xpar0, uint32_t ws0, uint32_t wph0, int nk,
-                                                uint32_t xstages, bool wide) {
+                                                uint32_t xstages) {
     c->acc_uses = uses + 1;
     const uint32_t full = (uint32_t)nk / xstages, rem = (uint32_t)nk - full * xstages;
     c->x_par = xpar0 ^ ((full & 1u) ? (1u << xstages) - 1u : 0u) ^ ((1u << rem) - 1u);
     const uint32_t pos = ws0 + (uint32_t)nk;               // one weight slot per k-tile
-    if (wide) {
-        c->ww_slot = (uint8_t)(pos % kTcWideSlots);
-        c->ww_phase = (uint8_t)((wph0 ^ (pos / kTcWideSlots)) & 1u);
-    } else {
-        c->w_slot = (uint8_t)(pos % kTcWSlots);
-        c->w_phase = (uint8_t)((wph0 ^ (pos / kTcWSlots)) & 1u);
-    }
+    c->w_slot = (uint8_t)(pos % kTcWSlots);
+    c->w_phase = (uint8_t)((wph0 ^ (pos / kTcWSlots)) & 1u);
 }
 
 // Epilogue, second half.  The accumulator tile has been copied to shared memory (fp32, row pitch
@@ -392,7 +342,7 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
     }
     tc_fence_before();
     const bool aborting = compute_sync_or(!ok || *(volatile int*)&c->abort);
-    if (t == 0) tc_finish_state(c, uses, xpar0, ws0, wph0, nk, xstages, false);
+    if (t == 0) tc_finish_state(c, uses, xpar0, ws0, wph0, nk, xstages);
     if (aborting) return -1;
     return 0;
 }

@@ -1,162 +1,352 @@
-// MK_OP_GEMM on tcgen05 with 128 x 256 output tiles (descriptor i 10 = 256): the body of op_gemm_tc.cuh with two
-// accumulator halves of 128 columns in tensor memory.  One activation k-tile feeds two weight tiles, which halves
-// the activation bytes per flop: the main loop of a tile GEMM is bound by the operand bytes an SM draws from L2
-// (~64 GB/s measured: 0.5 us per 32 KB k-tile of a 128 x 128 tile, 0.75 us per 48 KB of a 128 x 256 one with
-// twice the flops).  The two weight tiles of a k-tile travel through the same single-tile ring slots, one after
-// the other (the producer warp knows the shape: op_gemv_common.cuh); the epilogue handles the halves in turn,
-// each exactly as the narrow tile's.  A body of its own (and a translation unit of its own, op_gemm_wide.cu)
-// rather than a parameter of the narrow one: sharing the code cost the narrow tile's main loop spilled registers.
+// MK_OP_GEMM on tcgen05 with 256 x 256 output tiles (descriptor i 10 = 256): linears with many activation rows.
+//
+// What bounds a tile GEMM whose operands live in L2 is the bytes an SM draws from there: measured on B200 (all 148 SMs,
+// stand-alone loop) a 128 x 256 tile takes 0.46 us per 64-element k-tile of 48 KB (104 GB/s per SM) where its MMAs take
+// 0.29; a 256 x 256 tile needs 64 KB for twice the flops and takes 0.82, 11 % less per flop, and a single thread that
+// issues four N = 256 instructions per commit keeps the tensor pipe full (2.15 PFLOP/s with the operands in place).  So
+// one instruction is a 256 x 256 tile: two 128 x 256 accumulators (rows 0..127 and 128..255: all 512 columns of tensor
+// memory), three stages of 64 KB, and four roles that run ahead of one another across instruction boundaries:
+//   weights      producer warp -> one 32 KB copy per k-tile (op_gemv_common.cuh), as early as a slot is free
+//   activations  feeder warp (wide_feed): waits for the instruction's dependencies itself, then one bulk tensor copy of
+//                256 rows x 64 columns per k-tile; rows beyond M are zero-filled
+//   MMA          issuer warp, one thread (wide_issuer): waits for a stage (armed once by each loader), 4 + 4 instructions, one commit.
+//                It is told what to run by the feeder through Ctrl::wide_info and never touches global memory.
+//   epilogue     the compute warps: warp w owns rows 32 (w & 3) .. +31 of accumulator w >> 2; it reads its 32 x 256 part, hands
+//                the accumulator back and writes the rows from registers while the next tile's main loop runs
+// The loads of the next tile therefore run through this one's epilogue, and its MMAs start as soon as the accumulators have
+// been read.  (With one role after the other per instruction, 128 x 256 tiles: prefill gate/up 20.5 us per 128 x 256 x 2048
+// block of which 13.8 were main loop; DiT gelu tiles 28 us of which 7.)
+// A run of such instructions on a CTA starts with the compute warps' arrival on gemm_go: the work area, where the
+// activation slots are, belongs to other bodies before it and after the run's last accumulator.
+// A body and a translation unit of its own (op_gemm_wide.cu): sharing code with the 128 x 128 body cost that one spilled registers.
 #pragma once
-#include "op_gemm_tc.cuh"
+#include "mk_device.cuh"
+#include "mma.cuh"
+#include "tc.cuh"
 
 namespace mk {
 
-__device__ __forceinline__ int op_gemm_tc_wide(const Params& p, Ctrl* c, uint8_t* ring, uint8_t* work, const mk_op_desc* op, int a0,
-                                          int a1, int a2, int seq) {
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int M = op->i[0], N = op->i[1], K = op->i[2], splits = op->i[4];
-    const int swi = op->i[8];
-    constexpr int halves = 2;                                             // 128-column accumulator halves of the output tile
-    const int m0 = a0 * 128, n0 = a1 * 128 * halves;
-    const int kc = K / splits, kbeg = a2 * kc, nk = kc / 64;
+// ---- feeder warp: activation tiles of one instruction (all lanes; lane 0 requests) ---------------------------------------
+// `first`: the instruction before it on this CTA is not of this kind -- wait for the compute warps to turn to it.
+struct WideFeed {
+    uint32_t slot = 0, phase = 0;        // position in the stages
+    uint32_t go = 0;                     // parity of gemm_go
+    uint32_t count = 0;                  // instructions fed
+};
+__device__ __forceinline__ bool wide_feed(const Params& p, Ctrl* c, uint8_t* work, const mk_op_desc* op, const Inst& in, bool first,
+                                          WideFeed& f) {
+    const int lane = threadIdx.x & 31;
+    const int M = op->i[0], kc = op->i[2] / op->i[4], kbeg = in.a2 * kc, nk = kc / 64, m0 = in.a0 * 256;
     const uint8_t* tmaps = reinterpret_cast<const uint8_t*>(op->ptr[11]);
-    uint8_t* xs = work + kTcXOff;
-    // activation stages: whole 128-row tiles, or twice as many 64-row half tiles
-    const int xbytes = M <= 64 ? kTcTileBytes / 2 : kTcTileBytes;
-    const uint32_t xstages = M <= 64 ? kTcXHalfStages : kTcXStages;
+    bool ok = true;
+    if (first) {
+        if (lane == 0) ok = wait_barrier(p, c, &c->gemm_go, f.go, in.seq, WHERE_DEP, 2);
+        f.go ^= 1u;
+        if (!__all_sync(0xffffffffu, ok)) return false;
+    }
+    for (int k = lane; k < in.nwait; k += 32) {
+        const int2 w = __ldg(p.waits + in.wait_off + k);
+        ok = wait_counter(p, c, w.x, w.y, in.seq) && ok;
+    }
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    if (lane == 0) {
+        // the work area was last written through the generic proxy, and so were the activations, by other SMs
+        asm volatile("fence.proxy.async;" ::: "memory");
+        unsigned long long keep;
+        asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(keep));
+        for (int kt = 0; kt < nk; ++kt) {
+            ok = wait_barrier(p, c, &c->ww_empty[f.slot], f.phase ^ 1u, in.seq, WHERE_RING_EMPTY, 2);
+            if (!ok) break;
+            if (kt == 0) {
+                // what the issuing thread needs to know.  Four entries: the stage just found free was filled three k-tiles ago, so the
+                // issuing thread is at most three instructions behind
+                const uint32_t e = f.count & 3u;
+                c->wide_info[e] = make_int4(nk, M - m0 > 128 ? 2 : 1, op->i[9] == DT_F16 ? 1 : 0, in.seq);
+                mbar_arrive(&c->wide_told[e]);
+            }
+            mbar_arrive_expect_tx(&c->ww_full[f.slot], (uint32_t)kTcWideBytes);
+            tma_load_2d(work + kTcXOff + f.slot * kTcWideBytes, tmaps, kbeg + kt * 64, m0, &c->ww_full[f.slot], keep);
+            if (++f.slot == kTcWideSlots) { f.slot = 0; f.phase ^= 1u; }
+        }
+    }
+    ++f.count;
+    return __all_sync(0xffffffffu, ok);
+}
+// end of the instruction list: the issuing thread leaves
+__device__ __forceinline__ void wide_feed_end(Ctrl* c, const WideFeed& f) {
+    if ((threadIdx.x & 31) == 0) {
+        const uint32_t e = f.count & 3u;
+        c->wide_info[e] = make_int4(0, 0, 0, 0);
+        mbar_arrive(&c->wide_told[e]);
+    }
+}
 
-    // Tensor memory is allocated by the CTA's first tile GEMM instruction and kept until the kernel
-    // ends (the kernel frees it on every path); the permit to allocate is never relinquished.
-    // (the test is on a word that only changes behind a barrier, so every thread takes the same branch -- not on the
-    // address itself, which the allocation writes while the other warps are still arriving at the test)
-    const uint32_t uses = *(volatile uint32_t*)&c->acc_uses;
-    if (*(volatile uint32_t*)&c->tmem_ready == 0) {            // (the attention op may have allocated it already)
-        if (warp == 0) {
-            __syncwarp();          // (.sync.aligned: the whole warp, converged)
+// ---- issuer warp, lane 0 -----------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void wide_issuer(const Params& p, Ctrl* c, uint8_t* ring, uint8_t* work) {
+    const uint64_t ad0 = tc_smem_desc(smem_u32(work + kTcXOff)), bd0 = tc_smem_desc(smem_u32(ring));
+    uint32_t s = 0, ph = 0;
+    for (uint32_t n = 0;; ++n) {
+        if (!wait_barrier(p, c, &c->wide_told[n & 3u], (n >> 2) & 1u, 0, WHERE_DEP, 4)) return;
+        const int4 info = c->wide_info[n & 3u];
+        const int nk = info.x;
+        if (nk <= 0) return;
+        const bool both = info.y == 2;                       // rows 128..255 of the tile exist
+        const uint32_t idesc = tc_idesc_n(info.z != 0, 256);
+        const uint32_t tmem = *(volatile uint32_t*)&c->tmem_base;
+        uint32_t acc = 0;
+        for (int kt = 0; kt < nk; ++kt) {
+            if (!wait_barrier(p, c, &c->ww_full[s], ph, info.w, WHERE_RING_FULL, 2)) return;
+            if (kt == 0 && !wait_barrier(p, c, &c->wacc_empty[0], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return;
+            tc_fence_after();
+            const uint64_t ad = ad0 + s * (kTcWideBytes >> 4), bd = bd0 + s * (kTcWideBytes >> 4);
+#pragma unroll
+            for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem, ad + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+            if (kt == nk - 1) tc_commit(&c->wacc_full[0]);
+            if (kt == 0) {
+                if (!wait_barrier(p, c, &c->wacc_empty[1], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return;
+                tc_fence_after();
+            }
+            if (both) {
+#pragma unroll
+                for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem + 256, ad + (kTcTileBytes >> 4) + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+            }
+            acc = 1;
+            if (!check_phase(p, c, &c->ww_empty[s], ph, info.w, WHERE_CHECK_RELEASE)) return;
+            tc_commit(&c->ww_empty[s]);
+            if (++s == kTcWideSlots) { s = 0; ph ^= 1u; }
+        }
+        tc_commit(&c->wacc_full[1]);
+        if (p.trace_cap > 0) c->t_phase[1] = (long long)globaltimer();
+    }
+}
+
+// ---- compute warps: epilogue ---------------------------------------------------------------------------------------------------
+// A warp's part of the tile: 32 rows (one per lane of tensor memory) x 256 columns.  Rows are turned into row-contiguous
+// global accesses through 4 KB of shared memory of the warp's own, 128 bytes per row, 16-byte chunks swizzled by the row.
+__device__ __forceinline__ uint4* wide_chunk(uint8_t* stg, int row, int ch) { return reinterpret_cast<uint4*>(stg + row * 128 + ((ch ^ (row & 7)) << 4)); }
+// What an epilogue function starts with.  The functions are called, not inlined (side by side they spill), and the wait is
+// behind their entry: the registers they save there are saved while the main loop runs.
+struct WideAcc {
+    unsigned long long* full;            // the accumulator is complete with this parity
+    unsigned long long* release;         // ... has been read
+    uint32_t parity, tacc;               // tensor-memory address of the warp's lanes
+    uint8_t* stg;                        // the warp's staging rows
+    const uint8_t* bias;                 // the tile's 256 bias values in shared memory, or null
+    int seq;
+};
+__device__ __forceinline__ bool wide_wait(const Params& p, Ctrl* c, const WideAcc& a) {
+    int ok = 1;
+    if ((threadIdx.x & 31) == 0) ok = wait_barrier(p, c, a.full, a.parity, a.seq, WHERE_COMBINE, 2) ? 1 : 0;
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    tc_fence_after();
+    phase_mark(p, c, 2);
+    __syncwarp();                        // (the tensor-memory loads are .sync.aligned: whole warp, converged)
+    return ok != 0;
+}
+__device__ __forceinline__ void wide_release(unsigned long long* bar) {
+    tc_fence_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+}
+__device__ __forceinline__ void wide_bias(const uint8_t* bias, int col, float* v) {          // 32 columns from shared memory (the same for all lanes)
+#pragma unroll
+    for (int j = 0; j < 32; j += 8) {
+        float b[8];
+        unpack8(*reinterpret_cast<const uint4*>(bias + (col + j) * 2), b);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[j + e] += b[e];
+    }
+}
+
+// 16-bit outputs, no residual, 64 output columns at a time: the last two such chunks stay packed in registers until the accumulator
+// has been handed back (all four do not fit the kernel's register cap).  ACT: 0 none, 1 gelu, 2 any (run time).
+template <bool F16, bool SWI, int ACT>
+static __device__ __noinline__ void wide_store16(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc a, int row0, int n0) {
+    constexpr int kChunks = SWI ? 2 : 4, kKept = 2;
+    const int lane = threadIdx.x & 31;
+    const int act = op->i[3];
+    const int rows = op->i[0] - row0;
+    const long long ldo = (long long)op->ld[2] * 2;
+    const int r = lane >> 3, cc = lane & 7;
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + (long long)(row0 + r) * ldo + (SWI ? n0 / 2 : n0) * 2 + cc * 16;
+    auto flush = [&](int ch, const uint32_t* q) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) *wide_chunk(a.stg, lane, j) = make_uint4(q[4 * j], q[4 * j + 1], q[4 * j + 2], q[4 * j + 3]);
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (j * 4 + r < rows) *reinterpret_cast<uint4*>(O + (long long)(j * 4) * ldo + ch * 128) = *wide_chunk(a.stg, j * 4 + r, cc);
+        __syncwarp();
+    };
+    if (!wide_wait(p, c, a)) return;
+    const uint32_t tacc = a.tacc;
+    uint32_t pk[kKept * 32];
+#pragma unroll
+    for (int ch = 0; ch < kChunks; ++ch) {
+        uint32_t q[32];
+#pragma unroll
+        for (int hf = 0; hf < 2; ++hf) {
+            float v[32];
+            if (SWI) {                                       // gate columns 128 ch + 32 hf .. +31, up columns 64 further
+                float u[32];
+                tc_ld32(tacc + ch * 128 + hf * 32, v);
+                tc_ld32(tacc + ch * 128 + 64 + hf * 32, u);
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = v[j] * sigmoidf_(v[j]) * u[j];
+            } else {
+                tc_ld32(tacc + ch * 64 + hf * 32, v);
+                if (a.bias) wide_bias(a.bias, ch * 64 + hf * 32, v);
+            }
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                float y0 = v[2 * j], y1 = v[2 * j + 1];
+                if (ACT == 1) { y0 = apply_act(ACT_GELU, y0); y1 = apply_act(ACT_GELU, y1); }
+                if (ACT == 2) { y0 = apply_act(act, y0); y1 = apply_act(act, y1); }
+                q[hf * 16 + j] = F16 ? pack2h(y0, y1) : pack2(y0, y1);
+            }
+        }
+        if (ch < kChunks - kKept) {
+            flush(ch, q);
+        } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j) pk[(ch - (kChunks - kKept)) * 32 + j] = q[j];
+        }
+    }
+    wide_release(a.release);
+#pragma unroll
+    for (int k = 0; k < kKept; ++k) flush(kChunks - kKept + k, pk + 32 * k);
+}
+
+// Everything else -- residual, fp32 output, split-K partial (reduce-add): 32 columns at a time through shared memory as fp32.
+// RK: 0 no residual, 1 16-bit, 2 fp32; the residual of the next 32 columns is requested before this one's are used.
+template <int RK>
+static __device__ __noinline__ void wide_store_any(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc a, int row0, int n0) {
+    const int lane = threadIdx.x & 31;
+    const int act = op->i[3], odt = op->i[5], rdt = op->i[7];
+    const bool accum = op->i[6] != 0, swi = op->i[8] != 0;
+    const int groups = swi ? 4 : 8;
+    const int rows = op->i[0] - row0;
+    const int r = lane >> 3, c4 = (lane & 7) * 4, osz = odt == DT_F32 ? 4 : 2;
+    const long long ldo = (long long)op->ld[2] * osz, ldr = (long long)op->ld[4] * (RK == 2 ? 4 : 2);
+    const int col0 = swi ? n0 / 2 : n0;
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + (long long)(row0 + r) * ldo + (col0 + c4) * osz;
+    const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]) + (long long)(row0 + r) * ldr + (col0 + c4) * (RK == 2 ? 4 : 2);
+    uint4 res[RK ? 8 : 1];
+    auto request = [&](int g) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            res[RK ? j : 0] = make_uint4(0u, 0u, 0u, 0u);
+            if (j * 4 + r < rows) {
+                const uint8_t* at = R + (long long)(j * 4) * ldr + g * 32 * (RK == 2 ? 4 : 2);
+                if (RK == 2) res[RK ? j : 0] = __ldcg(reinterpret_cast<const uint4*>(at));
+                else { const uint2 w = __ldcg(reinterpret_cast<const uint2*>(at)); res[RK ? j : 0].x = w.x; res[RK ? j : 0].y = w.y; }
+            }
+        }
+    };
+    if (RK) request(0);
+    if (!wide_wait(p, c, a)) return;
+    const uint32_t tacc = a.tacc;
+#pragma unroll 1
+    for (int g = 0; g < groups; ++g) {
+        float v[32];
+        if (swi) {
+            float u[32];
+            tc_ld32(tacc + (g >> 1) * 128 + (g & 1) * 32, v);
+            tc_ld32(tacc + (g >> 1) * 128 + 64 + (g & 1) * 32, u);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = v[j] * sigmoidf_(v[j]) * u[j];
+        } else {
+            tc_ld32(tacc + g * 32, v);
+            if (a.bias) wide_bias(a.bias, g * 32, v);
+            if (act != ACT_NONE) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = apply_act(act, v[j]);
+            }
+        }
+        if (g == groups - 1) wide_release(a.release);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(wide_chunk(a.stg, lane, j)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+        __syncwarp();
+        float4 o[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            o[j] = *reinterpret_cast<const float4*>(wide_chunk(a.stg, j * 4 + r, lane & 7));
+            if (RK == 1) {
+                float2 lo, hi;
+                if (rdt == DT_F16) { lo = unpack2h(res[RK ? j : 0].x); hi = unpack2h(res[RK ? j : 0].y); }
+                else { lo = make_float2(bf16_lo(res[RK ? j : 0].x), bf16_hi(res[RK ? j : 0].x)); hi = make_float2(bf16_lo(res[RK ? j : 0].y), bf16_hi(res[RK ? j : 0].y)); }
+                o[j].x += lo.x; o[j].y += lo.y; o[j].z += hi.x; o[j].w += hi.y;
+            } else if (RK == 2) {
+                o[j].x += __uint_as_float(res[RK ? j : 0].x); o[j].y += __uint_as_float(res[RK ? j : 0].y);
+                o[j].z += __uint_as_float(res[RK ? j : 0].z); o[j].w += __uint_as_float(res[RK ? j : 0].w);
+            }
+        }
+        if (RK && g + 1 < groups) request(g + 1);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            if (j * 4 + r >= rows) break;
+            uint8_t* at = O + (long long)(j * 4) * ldo + g * 32 * osz;
+            if (accum) {
+                if (odt == DT_F32) red_add_f32x4(reinterpret_cast<float*>(at), o[j].x, o[j].y, o[j].z, o[j].w);
+                else red_add_bf16x4(at, &o[j].x);
+            } else if (odt == DT_F32) *reinterpret_cast<float4*>(at) = o[j];
+            else *reinterpret_cast<uint2*>(at) = make_uint2(pack2t(odt, o[j].x, o[j].y), pack2t(odt, o[j].z, o[j].w));
+        }
+        __syncwarp();
+    }
+}
+
+template <bool F16>
+__device__ __forceinline__ void wide_store16_any(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
+    if (op->i[8]) wide_store16<F16, true, 0>(p, c, op, a, row0, n0);
+    else if (op->i[3] == ACT_NONE) wide_store16<F16, false, 0>(p, c, op, a, row0, n0);
+    else if (op->i[3] == ACT_GELU) wide_store16<F16, false, 1>(p, c, op, a, row0, n0);
+    else wide_store16<F16, false, 2>(p, c, op, a, row0, n0);
+}
+
+// Before the first instruction of a run: tensor memory (allocated by the CTA's first tcgen05 instruction and kept until the
+// kernel ends; the branch is taken on a word that only changes behind a barrier, see op_gemm_tc), then the go for the feeder.
+__device__ __forceinline__ void wide_begin_run(Ctrl* c) {
+    const int t = threadIdx.x;
+    if (*(volatile uint32_t*)&c->tmem_ready == 0) {
+        if (t < 32) {
+            __syncwarp();
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&c->tmem_base)), "r"(kTcCols)
                          : "memory");
         }
         tc_fence_before();
         compute_sync();
         tc_fence_after();
-        if (t == 0) c->tmem_ready = 1;                          // (read again only behind the barrier that ends this instruction)
+        if (t == 0) c->tmem_ready = 1;
     }
-    const uint32_t tmem = *(volatile uint32_t*)&c->tmem_base;
-    const uint32_t apar = uses & 1u;
+    if (t == 0) mbar_arrive(&c->gemm_go);
+}
 
-    phase_mark(p, c, 0);
-    const uint32_t xpar0 = c->x_par;
-    const uint32_t ws0 = c->ww_slot, wph0 = c->ww_phase;
-    if (warp == 2 && lane < 2) {
-        // ---- activation tiles: {64 K-elements, 128 rows} at (kbeg + 64 kt, m0) ---- (as in the narrow tile)
-        asm volatile("fence.proxy.async;" ::: "memory");
-        unsigned long long keep;
-        asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(keep));
-        // (two lanes, every other k-tile each: one lane's wait / expect / copy sequence takes as long as a k-tile's MMAs)
-        uint32_t s = lane, round = 1;
-        for (int kt = lane; kt < nk; kt += 2) {
-            if (!wait_barrier(p, c, &c->x_empty[s], ((xpar0 >> s) & 1u) ^ round, seq, WHERE_RING_EMPTY)) break;
-            if (!check_phase(p, c, &c->x_full[s], ((xpar0 >> s) & 1u) ^ round ^ 1u, seq, WHERE_CHECK_ARM)) break;
-            mbar_arrive_expect_tx(&c->x_full[s], (uint32_t)xbytes);
-            tma_load_2d(xs + s * xbytes, tmaps, kbeg + kt * 64, m0, &c->x_full[s], keep);
-            s += 2;
-            if (s >= xstages) { s -= xstages; round ^= 1u; }
-        }
-    } else if ((warp == 3 || warp == 1) && lane == 0) {
-        // ---- MMAs: accumulator[128 activation rows][256 weight rows] += x tile . w slot^T ----
-        // Two issuing threads as in the narrow tile, each with a 256-column accumulator (columns 256 i ..) and every
-        // other k-tile.  A k-tile is one activation stage and one 32 KB weight slot (the producer warp puts both weight
-        // tiles of the k-tile there, one barrier): one N = 256 instruction per 16 K-elements.
-        const uint32_t i = warp == 3 ? 0u : 1u;
-        const uint32_t idesc = tc_idesc_n(op->i[9] == DT_F16, 256);
-        const uint64_t ad0 = tc_smem_desc(smem_u32(xs)), bd0 = tc_smem_desc(smem_u32(ring));
-        const uint32_t xunits = (uint32_t)xbytes >> 4;
-        const uint32_t acc_at = tmem + 256 * i;
-        uint32_t acc = 0, s = i, round = 0;
-        uint32_t ws = ws0 + i, wph = wph0;
-        if (ws >= kTcWideSlots) { ws -= kTcWideSlots; wph ^= 1u; }
-        for (int kt = (int)i; kt < nk; kt += kTcIssuers) {
-            if (!wait_barrier(p, c, &c->ww_full[ws], wph, seq, WHERE_RING_FULL) ||
-                !wait_barrier(p, c, &c->x_full[s], ((xpar0 >> s) & 1u) ^ round, seq, WHERE_RING_FULL))
-                break;
-            tc_fence_after();
-            const uint64_t ad = ad0 + s * xunits, bd = bd0 + ws * (2 * kTcTileBytes >> 4);
-#pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16) {
-                tc_mma(acc_at, ad + 2 * k16, bd + 2 * k16, idesc, acc);
-                acc = 1;
-            }
-            if (!check_phase(p, c, &c->x_empty[s], ((xpar0 >> s) & 1u) ^ round, seq, WHERE_CHECK_RELEASE) ||
-                !check_phase(p, c, &c->ww_empty[ws], wph, seq, WHERE_CHECK_RELEASE))
-                break;
-            tc_commit(&c->x_empty[s]);
-            tc_commit(&c->ww_empty[ws]);
-            s += kTcIssuers;
-            if (s >= xstages) { s -= xstages; round ^= 1u; }
-            ws += kTcIssuers;
-            if (ws >= kTcWideSlots) { ws -= kTcWideSlots; wph ^= 1u; }
-        }
-        tc_commit(&c->acc_full);
-        if (p.trace_cap > 0 && i == 0) c->t_phase[1] = (long long)globaltimer();     // last MMA issued
-    }
-    __syncwarp();
-
-    // ---- epilogue: warp w owns lanes 32 (w & 3) .. +31 (activation rows) and column half w >> 2 ----
-    int ok = 1;
-    if (lane == 0) ok = wait_barrier(p, c, &c->acc_full, apar, seq, WHERE_COMBINE) ? 1 : 0;
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    tc_fence_after();
-    phase_mark(p, c, 2);                                                    // accumulator complete
-    __syncwarp();                                                           // (the tensor-memory loads below are .sync.aligned: whole warp, converged)
-    // Per 128-column accumulator half -- first: tensor memory -> shared memory.  Warp w reads lanes
-    // 32 (w & 3) .. +31 (activation rows) and column half w >> 2; the activation stages are free now
-    // (every MMA has completed).  Then row-contiguous global accesses from shared memory.
+// Epilogue of one instruction; all compute threads.  (A wait that gives up has raised Ctrl::abort; the barrier of publish()
+// makes that known to every thread.)
+__device__ __forceinline__ void op_gemm_tc_wide(const Params& p, Ctrl* c, uint8_t* ring, const mk_op_desc* op, int a0, int a1, int seq) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int qd = warp & 3, h = warp >> 2;
-    float* stage = reinterpret_cast<float*>(work + kTcXOff);
-    const int rows = min(128, M - m0);
-    const uint32_t two = nk > 1 ? 256u : 0u;                               // columns to the second issuing thread's accumulator, if it has a part
-#pragma unroll 1
-    for (int hf = 0; hf < halves; ++hf) {
-        const int nh = n0 + 128 * hf;                                        // first weight row of this half
-        if (hf) compute_sync();                                              // the previous half's rows have been read
-        if (ok && qd * 32 < rows) {
-            const uint32_t tl = tmem + ((uint32_t)(qd * 32) << 16) + 128 * hf;
-            float* srow = stage + (qd * 32 + lane) * kTcStagePitch;
-            float v[32];
-            if (swi) {
-                // gate columns 32 h .. +31 and the up columns 64 further of the same outputs
-                float u[32];
-                tc_ld32_sum(tl + h * 32, two, v);
-                tc_ld32_sum(tl + 64 + h * 32, two, u);
-#pragma unroll
-                for (int j = 0; j < 32; j += 4)
-                    *reinterpret_cast<float4*>(srow + h * 32 + j) =
-                        make_float4(v[j] * sigmoidf_(v[j]) * u[j], v[j + 1] * sigmoidf_(v[j + 1]) * u[j + 1],
-                                    v[j + 2] * sigmoidf_(v[j + 2]) * u[j + 2], v[j + 3] * sigmoidf_(v[j + 3]) * u[j + 3]);
-            } else {
-#pragma unroll 1
-                for (int ch = 0; ch < 2; ++ch) {
-                    const int tcol = h * 64 + ch * 32;
-                    if (nh + tcol >= N) break;
-                    tc_ld32_sum(tl + tcol, two, v);
-#pragma unroll
-                    for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(srow + tcol + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-                }
-            }
-        }
-        tc_fence_before();
+    const uint32_t par = *(volatile uint32_t*)&c->wide_uses & 1u;
+    const int n0 = a1 * 256, row0 = a0 * 256 + h * 128 + qd * 32;
+    phase_mark(p, c, 0);
+    const uint8_t* bias = nullptr;
+    if (op->ptr[3] && !op->i[6] && !op->i[8]) {                 // (behind the barrier that ended the previous instruction)
+        uint8_t* bs = ring + kTcWideBiasOff;
+        if (t < 32) reinterpret_cast<uint4*>(bs)[t] = __ldg(reinterpret_cast<const uint4*>(op->ptr[3] + (uint64_t)n0 * 2) + t);
         compute_sync();
-        if (ok) {
-            if (swi) tc_write_rows(op, stage, m0, rows, 64, nh / 2, N / 2);
-            else if (op->i[6]) tc_write_rows(op, stage, m0, rows, 128, nh, N);          // split-K partial: reduce-add
-            else tc_store_rows(op, stage, m0, rows, nh, N);
-        }
+        bias = bs;
     }
-    tc_fence_before();
-    const bool aborting = compute_sync_or(!ok || *(volatile int*)&c->abort);
-    if (t == 0) tc_finish_state(c, uses, xpar0, ws0, wph0, nk, xstages, true);
-    if (aborting) return -1;
-    return 0;
+    const WideAcc a{&c->wacc_full[h], &c->wacc_empty[h], par, *(volatile uint32_t*)&c->tmem_base + ((uint32_t)(qd * 32) << 16) + 256u * h,
+                    ring + kTcWideStageOff + warp * 4096, bias, seq};
+    const bool fast = !op->ptr[4] && !op->i[6];
+    if (row0 >= op->i[0]) {                                     // (rows beyond M)
+        if (wide_wait(p, c, a)) wide_release(a.release);
+    } else if (fast && op->i[5] == DT_F16) wide_store16_any<true>(p, c, op, a, row0, n0);
+    else if (fast && op->i[5] == DT_BF16) wide_store16_any<false>(p, c, op, a, row0, n0);
+    else if (op->i[6] || !op->ptr[4]) wide_store_any<0>(p, c, op, a, row0, n0);
+    else if (op->i[7] == DT_F32) wide_store_any<2>(p, c, op, a, row0, n0);
+    else wide_store_any<1>(p, c, op, a, row0, n0);
 }
 
 }  // namespace mk

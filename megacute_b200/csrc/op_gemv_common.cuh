@@ -196,7 +196,7 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
     uint32_t kvphase = 0, kvgo = 0;
     enum { MODE_STAGES = 0, MODE_WTILES = 1, MODE_KVTILES = 2, MODE_WWIDE = 3 };
     int wwslot = 0;
-    uint32_t wwphase = 0;
+    uint32_t wwphase = 0, wide_count = 0;            // (and instructions of that kind streamed)
     int mode = MODE_STAGES;
     // Wait until the compute side has released every slot of the kind used so far (slot s was last
     // filled in the current round if s < position, else in the previous one).
@@ -208,7 +208,9 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
                     ok = wait_barrier(p, c, &c->w_empty[s], (wphase ^ (s < wslot ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
             } else if (kind == MODE_WWIDE) {
                 for (int s = 0; s < kTcWideSlots && ok; ++s)
-                    ok = wait_barrier(p, c, &c->ww_empty[s], (wwphase ^ (s < wwslot ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
+                    ok = wait_barrier(p, c, &c->ww_empty[s], (wwphase ^ (s < wwslot ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY, 2) ? 1 : 0;
+                // ... and until the run's epilogues have read their staging rows behind the slots
+                if (ok) ok = wait_word(p, c, &c->wide_done, wide_count, rc.seq, WHERE_STAGING) ? 1 : 0;
             } else if (kind == MODE_KVTILES) {
                 for (int s = 0; s < kKvSlots && ok; ++s)
                     ok = wait_barrier(p, c, &c->kv_empty[s], (kvphase ^ (s < kvslot ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
@@ -265,44 +267,37 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
             continue;
         }
         if (rc.gemm && rc.wide == 2) {
-            // 128 x 256 tile GEMM: the two weight tiles of a k-tile (256 rows x 64 K-elements, adjacent in the packed
-            // array) fill one 32 KB slot and complete one barrier, so that the issuing thread pays one wait, four
-            // N = 256 MMAs and one commit per k-tile and operand (measured stand-alone with two issuing threads:
-            // 0.28 us per k-tile against 0.40 with a barrier pair per 16 KB tile).
+            // 256 x 256 tile GEMM: the two weight tiles of a k-tile (256 rows x 64 K-elements, adjacent in the packed
+            // array) fill one 32 KB slot; its barrier is armed a second time by the feeder warp, for the activations.
+            // One lane: a k-tile's MMAs take 0.58 us, the lane's wait / expect / copy sequence 0.2.
             if (!enter(MODE_WWIDE)) return;
             const int nkt = rc.nk >> 1;
-            // Two lanes, every other k-tile each.  Lanes run in lockstep, so a step waits for the slower lane's slot: with
-            // as many lanes as slots the four copies left in bursts, once the last slot of the previous burst had been
-            // consumed, and the consumer starved for a copy's latency per burst (0.57 us per k-tile; 0.48 before).
-            constexpr int kLanes = 2;
-            const unsigned long long wpol = rc.reread ? keep_policy : stream_policy;
-            bool mine = true;
-            if (lane < kLanes) {
+            int ok = 1;
+            if (lane == 0) {
+                const unsigned long long wpol = rc.reread ? keep_policy : stream_policy;
                 const uint8_t* src = rc.wpack ? rc.wpack + rc.wtile0 * (long long)kTcTileBytes : nullptr;
                 const long long kstep = (long long)rc.wstride * kTcTileBytes;
-                uint32_t sl = (uint32_t)wwslot + lane, ph = wwphase;
-                if (sl >= kTcWideSlots) { sl -= kTcWideSlots; ph ^= 1u; }
+                int sl = wwslot;
+                uint32_t ph = wwphase;
 #pragma unroll 1
-                for (int kt = lane; kt < nkt; kt += kLanes) {
-                    if (!wait_barrier(p, c, &c->ww_empty[sl], ph ^ 1u, rc.seq, WHERE_RING_EMPTY)) { mine = false; break; }
-                    if (!check_phase(p, c, &c->ww_full[sl], ph, rc.seq, WHERE_CHECK_ARM)) { mine = false; break; }
-                    uint8_t* dst = ring + sl * (2 * kTcTileBytes);
-                    mbar_arrive_expect_tx(&c->ww_full[sl], 2u * kTcTileBytes);
+                for (int kt = 0; kt < nkt; ++kt) {
+                    if (!wait_barrier(p, c, &c->ww_empty[sl], ph ^ 1u, rc.seq, WHERE_RING_EMPTY, 2)) { ok = 0; break; }
+                    uint8_t* dst = ring + sl * kTcWideBytes;
+                    mbar_arrive_expect_tx(&c->ww_full[sl], (uint32_t)kTcWideBytes);
                     if (src) {
-                        bulk_g2s_hint(dst, src + kt * kstep, 2u * kTcTileBytes, &c->ww_full[sl], wpol);
+                        bulk_g2s_hint(dst, src + kt * kstep, (uint32_t)kTcWideBytes, &c->ww_full[sl], wpol);
                     } else {
                         tma_load_2d(dst, rc.wmap, rc.kbeg + kt * 64, rc.n0, &c->ww_full[sl], wpol);
                         tma_load_2d(dst + kTcTileBytes, rc.wmap, rc.kbeg + kt * 64, rc.n0 + 128, &c->ww_full[sl], wpol);
                     }
-                    sl += kLanes;
-                    if (sl >= kTcWideSlots) { sl -= kTcWideSlots; ph ^= 1u; }
+                    if (++sl == kTcWideSlots) { sl = 0; ph ^= 1u; }
                 }
             }
-            const bool ok = __all_sync(0xffffffffu, mine);
             const uint32_t wpos = (uint32_t)wwslot + (uint32_t)nkt;
             wwslot = (int)(wpos % kTcWideSlots);
             wwphase ^= (wpos / kTcWideSlots) & 1u;
-            if (!ok) return;
+            ++wide_count;
+            if (!__shfl_sync(0xffffffffu, ok, 0)) return;
             rc.idx += gridDim.x;
             rc.seek(p);
             continue;
@@ -331,9 +326,8 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
                     uint8_t* dst = ring + tc_wslot_off(sl);
                     if (!check_phase(p, c, &c->w_full[sl], ph, rc.seq, WHERE_CHECK_ARM)) { mine = false; break; }
                     mbar_arrive_expect_tx(&c->w_full[sl], (uint32_t)kTcTileBytes);
-                    const int ktile = rc.wide == 2 ? kt >> 1 : kt, half = rc.wide == 2 ? kt & 1 : 0;
-                    if (src) bulk_g2s_hint(dst, src + ktile * kstep + half * kTcTileBytes, (uint32_t)kTcTileBytes, &c->w_full[sl], wpol);
-                    else tma_load_2d(dst, rc.wmap, rc.kbeg + ktile * 64, rc.n0 + half * 128, &c->w_full[sl], wpol);
+                    if (src) bulk_g2s_hint(dst, src + kt * kstep, (uint32_t)kTcTileBytes, &c->w_full[sl], wpol);
+                    else tma_load_2d(dst, rc.wmap, rc.kbeg + kt * 64, rc.n0, &c->w_full[sl], wpol);
                     sl += kLanes;
                     if (sl >= kTcWSlots) { sl -= kTcWSlots; ph ^= 1u; }
                 }

@@ -24,14 +24,17 @@ __device__ int mk_op_gemv_general(const Params& p, const mk_op_desc* op, int o0,
 // arrivals of each itself (begin_op says why).  Returns the index of the last instruction executed, -1 when the CTA is
 // aborting.  (The ring position is untouched: the weight tiles have slots of their own.)
 __device__ int mk_run_gemm(const Params& p, int idx);
-// (the same with 128 x 256 output tiles; only for ops the host library bound to the tcgen05 body)
+// (the same with 256 x 256 output tiles; only for ops the host library bound to the tcgen05 body)
 __device__ int mk_run_gemm_wide(const Params& p, int idx);
+// body of the issuer warp: the MMAs of every 256 x 256 tile, until the feeder warp says that the list has ended
+__device__ void mk_wide_issuer(const Params& p);
 __device__ void mk_op_attention(const mk_op_desc* op, int a0, int a1, int a2);
 // (the tcgen05 body, for ops the host library attached tensor maps to; returns -1 when aborting)
 __device__ int mk_op_attention_tc(const Params& p, const mk_op_desc* op, int a0, int a1, int a2, int seq);
 // body of the feeder warp: walks the CTA's instruction list and, for every prefill attention bound to the tcgen05 body,
-// requests its tiles and issues its MMAs (one thread); runs until the list ends or the CTA aborts
-__device__ void mk_attention_feeder(const Params& p);
+// requests its tiles and issues its MMAs (one thread), for every 256 x 256 tile GEMM requests its activation tiles; runs
+// until the list ends or the CTA aborts
+__device__ void mk_feeder(const Params& p);
 // (waits for its own dependencies and publishes its own arrivals; returns whether the CTA is aborting)
 __device__ bool mk_op_decode_attn(const Params& p, const mk_op_desc* op, int a0, int a1, int a2, int nwait, int wait_off,
                                   int seq, int narrive, int arrive_off);

@@ -18,11 +18,12 @@ namespace mk {
 
 // The kernel's loop has fetched instruction `idx` (its metadata is staged, the staging for the following ones is
 // under way) and chosen this body for it.  mine(op): does the body run this op too?  body(op, a0, a1, a2, seq) runs
-// one instruction between its dependency wait and its arrivals, < 0 when the CTA is aborting.
+// one instruction between its dependency wait and its arrivals, < 0 when the CTA is aborting.  after() runs behind the
+// arrivals, i.e. behind a barrier over the compute warps.
 // Returns the index of the last instruction executed, or -1 when aborting.  All compute threads call this together;
 // every decision in it is made on words that change only behind a barrier.
-template <class Mine, class Body>
-__device__ __forceinline__ int run_own_insts(const Params& p, Ctrl* c, int idx, Mine mine, Body body) {
+template <class Mine, class Body, class After>
+__device__ __forceinline__ int run_own_insts(const Params& p, Ctrl* c, int idx, Mine mine, Body body, After after) {
     Meta* mt = &c->meta;
     for (;;) {
         if (threadIdx.x == 0) c->run_idx = idx;                 // (read back behind the barrier of publish())
@@ -42,6 +43,7 @@ __device__ __forceinline__ int run_own_insts(const Params& p, Ctrl* c, int idx, 
             const int4 w2 = mt->inst[s3][2];
             if (publish(p, c, w2.z, w2.z <= kMetaArrives ? -1 - s2 : w2.w)) return -1;
         }
+        after();
         if (p.trace_cap > 0 && threadIdx.x == 0) {
             trace_rec_rt(p, 1, slot, seq, c->t_fetch, c->t_dep, (long long)globaltimer());
             trace_rec_rt(p, 2, slot, seq, c->t_phase[0], c->t_phase[1], c->t_phase[2]);

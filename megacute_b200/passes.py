@@ -392,9 +392,9 @@ def wide_tiles(g: Graph, sm_count: int) -> Graph:
             N = op.w.rows
             splits = op.splits if op.kind == "LinearSplit" else 1
             if N % C.GEMM_BN_WIDE == 0 and K % (64 * splits) == 0 and M > C.WIDE_MIN_ROWS and force != "0":
-                mt, kt = -(-M // C.GEMM_BM), K // 64 // splits
+                mt, mtw, kt = -(-M // C.GEMM_BM), -(-M // C.GEMM_BM_WIDE), K // 64 // splits
                 narrow = -(-(mt * (N // C.GEMM_BN) * splits) // sm_count) * (kt * C.KTILE_US + C.EPILOGUE_US)
-                wide = -(-(mt * (N // C.GEMM_BN_WIDE) * splits) // sm_count) * (kt * C.KTILE_US_WIDE + C.EPILOGUE_US_WIDE)
+                wide = -(-(mtw * (N // C.GEMM_BN_WIDE) * splits) // sm_count) * (kt * C.KTILE_US_WIDE + C.EPILOGUE_US_WIDE)
                 if wide < narrow or force == "1":
                     op = op.clone(bn=C.GEMM_BN_WIDE)
         ops.append(op)

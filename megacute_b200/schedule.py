@@ -108,6 +108,11 @@ def is_gemv(op: Op) -> bool:
     return op.kind == "Linear" and gemv_eligible(op.x.rows, op.x.cols)
 
 
+def gemm_rows(op: Op) -> int:
+    """Activation rows of a tile linear's output tile."""
+    return C.GEMM_BM_WIDE if op.bn == C.GEMM_BN_WIDE else C.GEMM_BM
+
+
 def tile_op(op: Op, sm_count: int) -> Tiled:
     k = op.kind
     if k == "Linear" and is_gemv(op):
@@ -128,14 +133,15 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
         out = op.out if k == "Linear" else op.ws
         M = out.rows
         swi = k == "Linear" and op.act == "swiglu"
-        BN = op.bn or C.GEMM_BN                       # weight rows per tile: 128, or 256 (passes.wide_tiles)
+        BN = op.bn or C.GEMM_BN                       # tile: 128 x 128, or 256 x 256 (passes.wide_tiles)
+        BM = gemm_rows(op)
         on = BN // 2 if swi else BN
-        m, nn = gemm_raster(_ceil(M, C.GEMM_BM), _ceil(out.cols, on))
+        m, nn = gemm_raster(_ceil(M, BM), _ceil(out.cols, on), 8 * C.GEMM_BM // BM)
         splits = op.splits if k == "LinearSplit" else 1
         kc = op.x.cols // splits
         m, nn, ks = np.repeat(m, splits), np.repeat(nn, splits), np.tile(np.arange(splits), len(m))
         n = len(m)
-        r0, r1 = m * C.GEMM_BM, (m + 1) * C.GEMM_BM
+        r0, r1 = m * BM, (m + 1) * BM
         acc = [_acc(op.x, READ, r0, r1, ks * kc, (ks + 1) * kc, n=n),
                _acc(op.w, READ, nn * BN, (nn + 1) * BN, ks * kc, (ks + 1) * kc, n=n),
                _acc(out, ACCUM if k == "LinearSplit" else WRITE, r0, r1, nn * on, (nn + 1) * on, n=n)]

@@ -30,7 +30,7 @@ import torch
 
 from . import config as C
 from .graph import Graph
-from .schedule import CONFLICTS, Schedule, finalize_rows, is_gemv, norm_rows, tile_op
+from .schedule import CONFLICTS, Schedule, finalize_rows, gemm_rows, is_gemv, norm_rows, tile_op
 
 
 class VerifyError(AssertionError):
@@ -125,7 +125,7 @@ def op_grid(op, sm_count: int):
         out = op.out if k == "Linear" else op.ws
         swi = k == "Linear" and op.act == "swiglu"
         bn = op.bn or C.GEMM_BN
-        return (_ceil(out.rows, C.GEMM_BM), _ceil(out.cols, bn // 2 if swi else bn),
+        return (_ceil(out.rows, gemm_rows(op)), _ceil(out.cols, bn // 2 if swi else bn),
                 op.splits if k == "LinearSplit" else 1)
     if k == "SplitFinalize":
         return (_ceil(op.out.rows, finalize_rows(*op.out.shape)), _ceil(op.out.cols, C.EW_COLS))
