@@ -23,11 +23,10 @@ GEMM_BM, GEMM_BN, GEMM_BK = 128, 128, 32
 MIN_SPLIT_KTILES = 8            # k-tiles (of GEMM_BK) per K split
 MAX_K_SPLITS = 8
 INST_US, SM_GBPS = 2.0, 40.0    # split-K cost model: fixed us per instruction, GB/s one SM draws from HBM
-# 256-wide output tiles (one activation k-tile feeds two weight tiles) for ops with more than WIDE_MIN_ROWS rows:
-# us per 64-element k-tile of a 128 x 128 / 128 x 256 tile and us per epilogue, from the kernel's timeline (two issuing
-# threads; a 128 x 256 k-tile is one 32 KB weight slot and one N = 256 instruction per 16 K-elements)
+# output tiles of a tile linear: 128 x 128, and for ops with more than WIDE_MIN_ROWS rows 256 x 128 and 256 x 256; cost
+# model (us, from the kernel's timeline with every SM streaming): per tile, per 64-element k-tile, once per op
 GEMM_BM_WIDE, GEMM_BN_WIDE, WIDE_MIN_ROWS = 256, 256, 128
-KTILE_US, KTILE_US_WIDE, EPILOGUE_US, EPILOGUE_US_WIDE = 0.27, 0.66, 3.5, 3.0
+GEMM_COST_US = {(128, 128): (4.0, 0.30, 0.0), (256, 128): (2.0, 0.50, 4.0), (256, 256): (3.0, 0.80, 5.0)}
 
 # ---- pointwise / norm / attention tiling
 EW_ROWS, EW_COLS = 32, 512

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         }
         mbar_init(&c->epi_done, 1);
         mbar_init(&c->deps_met, 1);
-        for (int s = 0; s < 2 * kTcXStages; ++s) {
+        for (int s = 0; s < kTcXHalfStages; ++s) {
             mbar_init(&c->x_full[s], 1);
             mbar_init(&c->x_empty[s], 1);
         }
@@ -58,9 +58,9 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
             mbar_init(&c->w_empty[s], 1);
         }
         c->w_slot = c->w_phase = 0;
-        for (int s = 0; s < kTcWideSlots; ++s) {
-            mbar_init(&c->ww_full[s], 2);
-            mbar_init(&c->ww_empty[s], 1);
+        for (int s = 0; s < 2 * kWideStages; ++s) {
+            mbar_init(&c->ww_full[0][0] + s, 2);
+            mbar_init(&c->ww_empty[0][0] + s, 1);
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&c->wacc_full[s], 1);
@@ -215,9 +215,9 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                 if (globaltimer() - t0 > 20000000ull) break;
             }
         }
-        for (int s = 0; s < kTcWideSlots; ++s) {
+        for (int s = 0; s < 2 * kWideStages; ++s) {
             unsigned long long t0 = globaltimer();
-            while (!(mbar_try_wait(&c->ww_full[s], 0) || mbar_try_wait(&c->ww_full[s], 1))) {
+            while (!(mbar_try_wait(&c->ww_full[0][0] + s, 0) || mbar_try_wait(&c->ww_full[0][0] + s, 1))) {
                 if (globaltimer() - t0 > 20000000ull) break;
             }
         }
@@ -386,6 +386,7 @@ static bool encode_tile_map(void* out, uint64_t base, long long rows, long long 
 // and every operand the epilogue touches with 16-byte vectors aligned for them.
 static bool tile_gemm_on_tcgen05(const mk_op_desc& d) {
     const int N = d.i[1], K = d.i[2], splits = d.i[4], odt = d.i[5], rdt = d.i[7], swi = d.i[8];
+    if (d.i[11] == 256 && N % 128) return false;              // (the 256-row tiles' epilogue has whole columns only)
     if (splits <= 0 || K % splits || (K / splits) % 64) return false;
     const int n_out = swi ? N / 2 : N;
     if (n_out % 8 || (swi && N % 128)) return false;
@@ -419,8 +420,8 @@ static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
                     break;
                 case MK_OP_GEMM:
                     if (d.i[4] <= 0) why = "tile GEMM: split count";
-                    else if (a0 < 0 || a0 * (long long)(d.i[10] == 256 ? 256 : 128) >= d.i[0]) why = "tile GEMM: m tile outside M";
-                    else if (d.i[10] != 0 && d.i[10] != 128 && !(d.i[10] == 256 && d.i[1] % 256 == 0)) why = "tile GEMM: weight rows per tile";
+                    else if (a0 < 0 || a0 * (long long)(d.i[11] == 256 ? 256 : 128) >= d.i[0]) why = "tile GEMM: m tile outside M";
+                    else if (d.i[10] != 0 && d.i[10] != 128 && !(d.i[10] == 256 && d.i[11] == 256 && d.i[1] % 256 == 0)) why = "tile GEMM: weight rows per tile";
                     else if (a1 < 0 || a1 * (long long)(d.i[10] == 256 ? 256 : 128) >= d.i[1]) why = "tile GEMM: n tile outside N";
                     else if (a2 < 0 || a2 >= d.i[4]) why = "tile GEMM: K split index";
                     break;
@@ -642,7 +643,7 @@ int mk_program_set_ops(mk_program* p, const mk_op_desc* ops, int n_ops, void* st
         // mixing fp16 activations with bf16 weights raised an illegal-instruction fault): only the packed
         // copy can provide them.  Without one, the op runs the mma.sync body, which converts in registers.
         if (xh && (pack_off || (d.ptr[1] & 15) || d.ld[1] % 8 != 0)) continue;
-        if (!encode_tile_map(maps, d.ptr[0], d.i[0], d.i[2], d.ld[0], d.i[10] == 256 ? 256 : d.i[0] <= 64 ? 64 : 128, false, xh)) continue;
+        if (!encode_tile_map(maps, d.ptr[0], d.i[0], d.i[2], d.ld[0], d.i[11] == 256 ? 256 : d.i[0] <= 64 ? 64 : 128, false, xh)) continue;
         // weights: the packed copy, made when a matrix (address, shape, pitch) is bound for the first
         // time and kept while it stays bound -- rebinding other operands (a new input tensor every
         // call) must not copy gigabytes of weights again; weights changed in place need

@@ -53,7 +53,7 @@ constexpr int kTcCols = 512;                              // tensor-memory colum
                                                           // or two S tiles and O (prefill attention)
 constexpr uint32_t kTcNoTmem = 0xffffffffu;               // Ctrl::tmem_base before the CTA's first allocation
 static_assert((kRingBytes + kTcXOff) % 1024 == 0 && kTcXOff + kTcXStages * kTcTileBytes <= kWorkBytes &&
-                  kTcXOff + (kTcXHalfStages + 1) * (kTcTileBytes / 2) <= kWorkBytes && kTcXHalfStages <= 2 * kTcXStages,
+                  kTcXOff + (kTcXHalfStages + 1) * (kTcTileBytes / 2) <= kWorkBytes && kTcXHalfStages >= kTcXStages,
               "activation tiles");
 // many-sequence decode attention (op_decode_bulk.cuh): the ring's memory as seven slots, each one tile of
 // 16 whole cache rows (at most 1 KB each) stored as four 4-row groups 32 bytes apart beyond their size.
@@ -73,14 +73,22 @@ __host__ __device__ inline void kv_split_range(int n, int S, int s, int& k_begin
     k_end = k_begin + per < n ? k_begin + per : n;
 }
 constexpr int kTcWSlots = 8;
-// 256 x 256 tiles (op_gemm_tc_wide.cuh): three stages of one weight slot (256 rows x 64 K-elements, 32 KB, in the ring's
-// memory) and one activation slot (the same, in the work area); the rest of the ring's memory holds the epilogue's
-// staging rows (4 KB per compute warp) and the tile's bias
-constexpr int kTcWideSlots = 3;
-constexpr int kTcWideBytes = 2 * kTcTileBytes;            // one slot
-constexpr int kTcWideStageOff = kTcWideSlots * kTcWideBytes;
-constexpr int kTcWideBiasOff = kTcWideStageOff + kComputeWarps * 4096;
-static_assert(kTcWideBiasOff + 256 * 2 <= kRingBytes && kTcXOff + kTcWideSlots * kTcWideBytes <= kWorkBytes, "256 x 256 tiles");
+// tiles of 256 rows (op_gemm_tc_wide.cuh), of two kinds: 256 columns (kind 0) with three stages of 32 KB of weights and 32 KB of
+// activations, 128 columns (kind 1) with four stages of 16 KB and 32 KB.  Weight slots are in the ring's memory, three
+// activation slots in the work area, the fourth behind the weight slots; the rest of the ring's memory holds the epilogue's
+// staging rows (4 KB per compute warp) and the tile's bias.
+constexpr int kWideStages = 4;                            // barriers per kind
+constexpr int kWideXBytes = 2 * kTcTileBytes;             // one activation slot
+constexpr int kWideStageOff = 3 * 2 * kTcTileBytes;
+constexpr int kWideBiasOff = kWideStageOff + kComputeWarps * 4096;
+__host__ __device__ constexpr int wide_stages(int kind) { return kind ? 4 : 3; }
+__host__ __device__ constexpr int wide_wbytes(int kind) { return kind ? kTcTileBytes : 2 * kTcTileBytes; }
+// byte offsets in the ring's memory and the work area behind it
+__host__ __device__ constexpr int wide_woff(int kind, int s) { return s * wide_wbytes(kind); }
+__host__ __device__ constexpr int wide_xoff(int s) { return s < 3 ? kRingBytes + kTcXOff + s * kWideXBytes : 4 * kTcTileBytes; }
+static_assert(kWideBiasOff + 256 * 2 <= kRingBytes && kTcXOff + 3 * kWideXBytes <= kWorkBytes && wide_xoff(3) + kWideXBytes <= kWideStageOff &&
+                  wide_woff(1, 3) + wide_wbytes(1) <= wide_xoff(3) && wide_woff(0, 2) + wide_wbytes(0) <= kWideStageOff,
+              "tiles of 256 rows");
 constexpr int kTcIssuers = 2;                             // threads that issue tcgen05.mma of a 128 x 128 tile, each into an accumulator of its own
 // k-tiles alternate between the issuing threads, and a thread waits for a stage or slot by the parity of its barrier's
 // phase: that is only sound if the same thread consumed the stage's previous round (a thread waiting one round early
@@ -106,8 +114,8 @@ struct Params {
     int pf_stages;                // how many ring stages ahead of the ring the producer prefetches into L2
 };
 
-// a tile GEMM bound to the 256 x 256 tcgen05 body (op_gemm_tc_wide.cuh)
-__device__ __forceinline__ bool is_wide_gemm(const mk_op_desc* op) { return op->kind == MK_OP_GEMM && op->i[10] == 256 && op->ptr[11] != 0; }
+// a tile GEMM bound to the tcgen05 body with 256-row tiles (op_gemm_tc_wide.cuh)
+__device__ __forceinline__ bool is_wide_gemm(const mk_op_desc* op) { return op->kind == MK_OP_GEMM && op->i[11] == 256 && op->ptr[11] != 0; }
 
 // Instruction metadata staged in shared memory one instruction ahead of its use.  Everything an
 // instruction needs before its first useful load (its words, its op descriptor, its wait and
@@ -134,18 +142,18 @@ struct Ctrl {                     // lives in the last kCtrlBytes of shared memo
     unsigned long long slot_free[4];  // ... the finisher warp has read them
     unsigned long long epi_done;      // ... the finisher has issued the instruction's last stores (its arrivals follow)
     unsigned long long deps_met;      // ... the compute warps have seen the instruction's dependencies met
-    unsigned long long x_full[2 * kTcXStages];   // tcgen05 tile GEMM: an activation k-tile has landed in the work area
-    unsigned long long x_empty[2 * kTcXStages];  // ... the MMAs that read it have completed
+    unsigned long long x_full[kTcXHalfStages];   // tcgen05 tile GEMM: an activation k-tile has landed in the work area
+    unsigned long long x_empty[kTcXHalfStages];  // ... the MMAs that read it have completed
     unsigned long long w_full[kTcWSlots];    // ... a weight k-tile has landed in its slot of the ring
     unsigned long long w_empty[kTcWSlots];   // ... the MMAs that read it have completed
-    unsigned long long ww_full[kTcWideSlots];    // 256 x 256 tiles: both operands' k-tiles of a stage have landed (armed once for each)
-    unsigned long long ww_empty[kTcWideSlots];   // ... the MMAs that read the stage have completed
+    unsigned long long ww_full[2][kWideStages];  // tiles of 256 rows, per kind: both operands' k-tiles of a stage have landed (armed once for each)
+    unsigned long long ww_empty[2][kWideStages]; // ... the MMAs that read the stage have completed
     unsigned long long wacc_full[2];             // ... every MMA into the accumulator of the tile's rows 0..127 / 128..255 has completed
     unsigned long long wacc_empty[2];            // ... the four compute warps of those rows have read it
     unsigned long long gemm_go;                  // ... the compute warps have turned to the first of a run of such instructions: the work
                                                  //     area is theirs, tensor memory is allocated
     unsigned long long wide_told[4];             // ... the feeder has written wide_info[]: what the issuing thread runs next
-    int4 wide_info[4];                           //     k-tiles (0: end of the list), accumulators, fp16 operands, sequence number
+    int4 wide_info[4];                           //     k-tiles (0: end of the list), accumulators | weight tiles << 4, fp16 operands, sequence number
     uint32_t wide_uses;                          // ... instructions executed (parity of wacc_full); written behind the barrier that ends one
     uint32_t wide_done;                          // ... the same at the end of the latest run: the staging rows in the ring's memory are free
     unsigned long long acc_full;      // ... every MMA of the instruction has completed (one arrival per issuing thread)

@@ -21,7 +21,7 @@ __device__ void mk_feeder(const Params& p) {
         if (opi < 0 || opi >= p.n_ops) return;
         const mk_op_desc* op = p.ops + opi;
         if (is_wide_gemm(op)) {
-            if (!wide_feed(p, m.ctrl, m.work, op, in, !in_run, wf)) return;
+            if (!wide_feed(p, m.ctrl, m.ring, op, in, !in_run, wf)) return;
             in_run = true;
             continue;
         }

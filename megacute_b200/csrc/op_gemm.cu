@@ -13,12 +13,12 @@ __device__ int mk_run_gemm(const Params& p, int idx) {
         [&](const mk_op_desc* op, int a0, int a1, int a2, int seq) -> int {
             // the host library attached tensor maps: tcgen05 body, weights through the producer's ring
             // (the weight tiles have slots and barriers of their own: the ring position is untouched)
-            // (256 x 256 tiles have a translation unit of their own, op_gemm_wide.cu: the kernel calls it directly)
+            // (tiles of 256 rows have a translation unit of their own, op_gemm_wide.cu: the kernel calls it directly)
             if (op->ptr[11]) return op_gemm_tc(p, m.ctrl, m.ring, m.work, op, a0, a1, a2, seq);
-            // (a 256 x 256 output tile, i 10, is four 128 x 128 ones for this body)
-            const int halves = op->i[10] == 256 ? 2 : 1;
-            for (int q = 0; q < halves * halves; ++q) {
-                const int mt = a0 * halves + q / halves, n = a1 * halves + q % halves;
+            // (an output tile of 256 rows, i 11, or columns, i 10, is two or four 128 x 128 ones for this body)
+            const int mh = op->i[11] == 256 ? 2 : 1, nh = op->i[10] == 256 ? 2 : 1;
+            for (int q = 0; q < mh * nh; ++q) {
+                const int mt = a0 * mh + q / nh, n = a1 * nh + q % nh;
                 if (mt * 128 >= op->i[0]) break;
                 // ops with at most 64 activation rows have a single m tile: hold 64 rows and stream deeper
                 if (op->i[0] <= 64) {

@@ -29,11 +29,12 @@ namespace mk {
 // ---- feeder warp: activation tiles of one instruction (all lanes; lane 0 requests) ---------------------------------------
 // `first`: the instruction before it on this CTA is not of this kind -- wait for the compute warps to turn to it.
 struct WideFeed {
-    uint32_t slot = 0, phase = 0;        // position in the stages
+    uint32_t slot[2] = {0, 0}, phase[2] = {0, 0};      // position in the stages of each kind
+    int kind = 0;                        // of the latest instruction
     uint32_t go = 0;                     // parity of gemm_go
     uint32_t count = 0;                  // instructions fed
 };
-__device__ __forceinline__ bool wide_feed(const Params& p, Ctrl* c, uint8_t* work, const mk_op_desc* op, const Inst& in, bool first,
+__device__ __forceinline__ bool wide_feed(const Params& p, Ctrl* c, uint8_t* ring, const mk_op_desc* op, const Inst& in, bool first,
                                           WideFeed& f) {
     const int lane = threadIdx.x & 31;
     const int M = op->i[0], kc = op->i[2] / op->i[4], kbeg = in.a2 * kc, nk = kc / 64, m0 = in.a0 * 256;
@@ -54,20 +55,30 @@ __device__ __forceinline__ bool wide_feed(const Params& p, Ctrl* c, uint8_t* wor
         asm volatile("fence.proxy.async;" ::: "memory");
         unsigned long long keep;
         asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(keep));
-        for (int kt = 0; kt < nk; ++kt) {
-            ok = wait_barrier(p, c, &c->ww_empty[f.slot], f.phase ^ 1u, in.seq, WHERE_RING_EMPTY, 2);
+        const int kind = op->i[10] == 256 ? 0 : 1;
+        if (!first && kind != f.kind) {      // another division of the same memory: once the MMAs have read everything
+            const int k = f.kind;
+            for (uint32_t s = 0; s < (uint32_t)wide_stages(k) && ok; ++s)
+                ok = wait_barrier(p, c, &c->ww_empty[k][s], (f.phase[k] ^ (s < f.slot[k] ? 1u : 0u)) ^ 1u, in.seq, WHERE_RING_EMPTY, 2);
+        }
+        f.kind = kind;
+        uint32_t slot = f.slot[kind], phase = f.phase[kind];
+        for (int kt = 0; kt < nk && ok; ++kt) {
+            ok = wait_barrier(p, c, &c->ww_empty[kind][slot], phase ^ 1u, in.seq, WHERE_RING_EMPTY, 2);
             if (!ok) break;
             if (kt == 0) {
-                // what the issuing thread needs to know.  Four entries: the stage just found free was filled three k-tiles ago, so the
-                // issuing thread is at most three instructions behind
+                // what the issuing thread needs to know.  Four entries: the stage just found free was filled three or four k-tiles ago,
+                // so the issuing thread is done with the instruction before the four latest
                 const uint32_t e = f.count & 3u;
-                c->wide_info[e] = make_int4(nk, M - m0 > 128 ? 2 : 1, op->i[9] == DT_F16 ? 1 : 0, in.seq);
+                c->wide_info[e] = make_int4(nk, (M - m0 > 128 ? 2 : 1) | (op->i[10] >> 7) << 4, op->i[9] == DT_F16 ? 1 : 0, in.seq);
                 mbar_arrive(&c->wide_told[e]);
             }
-            mbar_arrive_expect_tx(&c->ww_full[f.slot], (uint32_t)kTcWideBytes);
-            tma_load_2d(work + kTcXOff + f.slot * kTcWideBytes, tmaps, kbeg + kt * 64, m0, &c->ww_full[f.slot], keep);
-            if (++f.slot == kTcWideSlots) { f.slot = 0; f.phase ^= 1u; }
+            mbar_arrive_expect_tx(&c->ww_full[kind][slot], (uint32_t)kWideXBytes);
+            tma_load_2d(ring + wide_xoff((int)slot), tmaps, kbeg + kt * 64, m0, &c->ww_full[kind][slot], keep);
+            if (++slot == (uint32_t)wide_stages(kind)) { slot = 0; phase ^= 1u; }
         }
+        f.slot[kind] = slot;
+        f.phase[kind] = phase;
     }
     ++f.count;
     return __all_sync(0xffffffffu, ok);
@@ -82,23 +93,24 @@ __device__ __forceinline__ void wide_feed_end(Ctrl* c, const WideFeed& f) {
 }
 
 // ---- issuer warp, lane 0 -----------------------------------------------------------------------------------------------------
-__device__ __forceinline__ void wide_issuer(const Params& p, Ctrl* c, uint8_t* ring, uint8_t* work) {
-    const uint64_t ad0 = tc_smem_desc(smem_u32(work + kTcXOff)), bd0 = tc_smem_desc(smem_u32(ring));
-    uint32_t s = 0, ph = 0;
+__device__ __forceinline__ void wide_issuer(const Params& p, Ctrl* c, uint8_t* ring) {
+    const uint64_t d0 = tc_smem_desc(smem_u32(ring));
+    uint32_t slot[2] = {0, 0}, phase[2] = {0, 0};
     for (uint32_t n = 0;; ++n) {
         if (!wait_barrier(p, c, &c->wide_told[n & 3u], (n >> 2) & 1u, 0, WHERE_DEP, 4)) return;
         const int4 info = c->wide_info[n & 3u];
         const int nk = info.x;
         if (nk <= 0) return;
-        const bool both = info.y == 2;                       // rows 128..255 of the tile exist
-        const uint32_t idesc = tc_idesc_n(info.z != 0, 256);
+        const bool both = (info.y & 15) == 2;                // rows 128..255 of the tile exist
+        const uint32_t idesc = tc_idesc_n(info.z != 0, 128u * (uint32_t)(info.y >> 4));
         const uint32_t tmem = *(volatile uint32_t*)&c->tmem_base;
-        uint32_t acc = 0;
+        const int kind = (info.y >> 4) == 2 ? 0 : 1;
+        uint32_t acc = 0, s = slot[kind], ph = phase[kind];
         for (int kt = 0; kt < nk; ++kt) {
-            if (!wait_barrier(p, c, &c->ww_full[s], ph, info.w, WHERE_RING_FULL, 2)) return;
+            if (!wait_barrier(p, c, &c->ww_full[kind][s], ph, info.w, WHERE_RING_FULL, 2)) return;
             if (kt == 0 && !wait_barrier(p, c, &c->wacc_empty[0], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return;
             tc_fence_after();
-            const uint64_t ad = ad0 + s * (kTcWideBytes >> 4), bd = bd0 + s * (kTcWideBytes >> 4);
+            const uint64_t ad = d0 + (uint32_t)(wide_xoff((int)s) >> 4), bd = d0 + (uint32_t)(wide_woff(kind, (int)s) >> 4);
 #pragma unroll
             for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem, ad + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
             if (kt == nk - 1) tc_commit(&c->wacc_full[0]);
@@ -111,10 +123,12 @@ __device__ __forceinline__ void wide_issuer(const Params& p, Ctrl* c, uint8_t* r
                 for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem + 256, ad + (kTcTileBytes >> 4) + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
             }
             acc = 1;
-            if (!check_phase(p, c, &c->ww_empty[s], ph, info.w, WHERE_CHECK_RELEASE)) return;
-            tc_commit(&c->ww_empty[s]);
-            if (++s == kTcWideSlots) { s = 0; ph ^= 1u; }
+            if (!check_phase(p, c, &c->ww_empty[kind][s], ph, info.w, WHERE_CHECK_RELEASE)) return;
+            tc_commit(&c->ww_empty[kind][s]);
+            if (++s == (uint32_t)wide_stages(kind)) { s = 0; ph ^= 1u; }
         }
+        slot[kind] = s;
+        phase[kind] = ph;
         tc_commit(&c->wacc_full[1]);
         if (p.trace_cap > 0) c->t_phase[1] = (long long)globaltimer();
     }
@@ -124,8 +138,7 @@ __device__ __forceinline__ void wide_issuer(const Params& p, Ctrl* c, uint8_t* r
 // A warp's part of the tile: 32 rows (one per lane of tensor memory) x 256 columns.  Rows are turned into row-contiguous
 // global accesses through 4 KB of shared memory of the warp's own, 128 bytes per row, 16-byte chunks swizzled by the row.
 __device__ __forceinline__ uint4* wide_chunk(uint8_t* stg, int row, int ch) { return reinterpret_cast<uint4*>(stg + row * 128 + ((ch ^ (row & 7)) << 4)); }
-// What an epilogue function starts with.  The functions are called, not inlined (side by side they spill), and the wait is
-// behind their entry: the registers they save there are saved while the main loop runs.
+// What an epilogue works on.
 struct WideAcc {
     unsigned long long* full;            // the accumulator is complete with this parity
     unsigned long long* release;         // ... has been read
@@ -158,73 +171,65 @@ __device__ __forceinline__ void wide_bias(const uint8_t* bias, int col, float* v
     }
 }
 
-// 16-bit outputs, no residual, 64 output columns at a time: the last two such chunks stay packed in registers until the accumulator
-// has been handed back (all four do not fit the kernel's register cap).  ACT: 0 none, 1 gelu, 2 any (run time).
+// 16-bit outputs, no residual: 128 columns of the accumulator at a time; the last of them stay packed in registers until the
+// accumulator has been handed back.  ACT: 0 none, 1 gelu, 2 any (run time).
 template <bool F16, bool SWI, int ACT>
-static __device__ __noinline__ void wide_store16(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc a, int row0, int n0) {
-    constexpr int kChunks = SWI ? 2 : 4, kKept = 2;
+__device__ __forceinline__ void wide_store16(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
+    constexpr int kChunks = SWI ? 1 : 2;                     // of 64 output columns per 128 of the accumulator
     const int lane = threadIdx.x & 31;
-    const int act = op->i[3];
+    const int act = op->i[3], units = op->i[10] >> 7;
     const int rows = op->i[0] - row0;
     const long long ldo = (long long)op->ld[2] * 2;
     const int r = lane >> 3, cc = lane & 7;
     uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + (long long)(row0 + r) * ldo + (SWI ? n0 / 2 : n0) * 2 + cc * 16;
-    auto flush = [&](int ch, const uint32_t* q) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) *wide_chunk(a.stg, lane, j) = make_uint4(q[4 * j], q[4 * j + 1], q[4 * j + 2], q[4 * j + 3]);
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (j * 4 + r < rows) *reinterpret_cast<uint4*>(O + (long long)(j * 4) * ldo + ch * 128) = *wide_chunk(a.stg, j * 4 + r, cc);
-        __syncwarp();
-    };
     if (!wide_wait(p, c, a)) return;
-    const uint32_t tacc = a.tacc;
-    uint32_t pk[kKept * 32];
+#pragma unroll 1
+    for (int u = 0; u < units; ++u) {
+        uint32_t pk[kChunks * 32];
 #pragma unroll
-    for (int ch = 0; ch < kChunks; ++ch) {
-        uint32_t q[32];
-#pragma unroll
-        for (int hf = 0; hf < 2; ++hf) {
+        for (int hf = 0; hf < 2 * kChunks; ++hf) {
+            const uint32_t tacc = a.tacc + u * 128 + hf * 32;
             float v[32];
-            if (SWI) {                                       // gate columns 128 ch + 32 hf .. +31, up columns 64 further
-                float u[32];
-                tc_ld32(tacc + ch * 128 + hf * 32, v);
-                tc_ld32(tacc + ch * 128 + 64 + hf * 32, u);
+            tc_ld32(tacc, v);
+            if (SWI) {                                       // gate columns 32 hf .. +31, up columns 64 further
+                float g[32];
+                tc_ld32(tacc + 64, g);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = v[j] * sigmoidf_(v[j]) * u[j];
-            } else {
-                tc_ld32(tacc + ch * 64 + hf * 32, v);
-                if (a.bias) wide_bias(a.bias, ch * 64 + hf * 32, v);
+                for (int j = 0; j < 32; ++j) v[j] = v[j] * sigmoidf_(v[j]) * g[j];
+            } else if (a.bias) {
+                wide_bias(a.bias, u * 128 + hf * 32, v);
             }
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 float y0 = v[2 * j], y1 = v[2 * j + 1];
                 if (ACT == 1) { y0 = apply_act(ACT_GELU, y0); y1 = apply_act(ACT_GELU, y1); }
                 if (ACT == 2) { y0 = apply_act(act, y0); y1 = apply_act(act, y1); }
-                q[hf * 16 + j] = F16 ? pack2h(y0, y1) : pack2(y0, y1);
+                pk[hf * 16 + j] = F16 ? pack2h(y0, y1) : pack2(y0, y1);
             }
         }
-        if (ch < kChunks - kKept) {
-            flush(ch, q);
-        } else {
+        if (u == units - 1) wide_release(a.release);
 #pragma unroll
-            for (int j = 0; j < 32; ++j) pk[(ch - (kChunks - kKept)) * 32 + j] = q[j];
+        for (int ch = 0; ch < kChunks; ++ch) {
+            const uint32_t* q = pk + ch * 32;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) *wide_chunk(a.stg, lane, j) = make_uint4(q[4 * j], q[4 * j + 1], q[4 * j + 2], q[4 * j + 3]);
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                if (j * 4 + r < rows) *reinterpret_cast<uint4*>(O + (long long)(j * 4) * ldo + (u * kChunks + ch) * 128) = *wide_chunk(a.stg, j * 4 + r, cc);
+            __syncwarp();
         }
     }
-    wide_release(a.release);
-#pragma unroll
-    for (int k = 0; k < kKept; ++k) flush(kChunks - kKept + k, pk + 32 * k);
 }
 
 // Everything else -- residual, fp32 output, split-K partial (reduce-add): 32 columns at a time through shared memory as fp32.
 // RK: 0 no residual, 1 16-bit, 2 fp32; the residual of the next 32 columns is requested before this one's are used.
 template <int RK>
-static __device__ __noinline__ void wide_store_any(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc a, int row0, int n0) {
+__device__ __forceinline__ void wide_store_any(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
     const int lane = threadIdx.x & 31;
     const int act = op->i[3], odt = op->i[5], rdt = op->i[7];
     const bool accum = op->i[6] != 0, swi = op->i[8] != 0;
-    const int groups = swi ? 4 : 8;
+    const int groups = (op->i[10] >> 5) >> (swi ? 1 : 0);
     const int rows = op->i[0] - row0;
     const int r = lane >> 3, c4 = (lane & 7) * 4, osz = odt == DT_F32 ? 4 : 2;
     const long long ldo = (long long)op->ld[2] * osz, ldr = (long long)op->ld[4] * (RK == 2 ? 4 : 2);
@@ -296,12 +301,17 @@ static __device__ __noinline__ void wide_store_any(const Params& p, Ctrl* c, con
     }
 }
 
-template <bool F16>
-__device__ __forceinline__ void wide_store16_any(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
-    if (op->i[8]) wide_store16<F16, true, 0>(p, c, op, a, row0, n0);
-    else if (op->i[3] == ACT_NONE) wide_store16<F16, false, 0>(p, c, op, a, row0, n0);
-    else if (op->i[3] == ACT_GELU) wide_store16<F16, false, 1>(p, c, op, a, row0, n0);
-    else wide_store16<F16, false, 2>(p, c, op, a, row0, n0);
+// The epilogue of an op, chosen once per run of instructions: each has a function of its own around it (op_gemm_wide.cu) and so a
+// register allocation of its own -- called per instruction they pay ~60 saved and restored registers each time, inlined
+// side by side they spill, and with the shared memory taken every such access is an L2 round trip behind the operand stream.
+enum { WIDE_PLAIN = 0, WIDE_SWIGLU, WIDE_GELU, WIDE_ACT, WIDE_ANY0, WIDE_ANY1, WIDE_ANY2 };      // (+ 16: fp16 output, the first four)
+__device__ __forceinline__ int wide_variant(const mk_op_desc* op) {
+    const int odt = op->i[5];
+    if (op->i[6]) return WIDE_ANY0;
+    if (op->ptr[4]) return op->i[7] == DT_F32 ? WIDE_ANY2 : WIDE_ANY1;
+    if (odt == DT_F32) return WIDE_ANY0;
+    const int v = op->i[8] ? WIDE_SWIGLU : op->i[3] == ACT_NONE ? WIDE_PLAIN : op->i[3] == ACT_GELU ? WIDE_GELU : WIDE_ACT;
+    return v + (odt == DT_F16 ? 16 : 0);
 }
 
 // Before the first instruction of a run: tensor memory (allocated by the CTA's first tcgen05 instruction and kept until the
@@ -324,29 +334,33 @@ __device__ __forceinline__ void wide_begin_run(Ctrl* c) {
 
 // Epilogue of one instruction; all compute threads.  (A wait that gives up has raised Ctrl::abort; the barrier of publish()
 // makes that known to every thread.)
+template <int V>
 __device__ __forceinline__ void op_gemm_tc_wide(const Params& p, Ctrl* c, uint8_t* ring, const mk_op_desc* op, int a0, int a1, int seq) {
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const int t = threadIdx.x, warp = t >> 5;
     const int qd = warp & 3, h = warp >> 2;
     const uint32_t par = *(volatile uint32_t*)&c->wide_uses & 1u;
-    const int n0 = a1 * 256, row0 = a0 * 256 + h * 128 + qd * 32;
+    const int n0 = a1 * op->i[10], row0 = a0 * 256 + h * 128 + qd * 32;
     phase_mark(p, c, 0);
     const uint8_t* bias = nullptr;
     if (op->ptr[3] && !op->i[6] && !op->i[8]) {                 // (behind the barrier that ended the previous instruction)
-        uint8_t* bs = ring + kTcWideBiasOff;
-        if (t < 32) reinterpret_cast<uint4*>(bs)[t] = __ldg(reinterpret_cast<const uint4*>(op->ptr[3] + (uint64_t)n0 * 2) + t);
+        uint8_t* bs = ring + kWideBiasOff;
+        if (t < op->i[10] / 8) reinterpret_cast<uint4*>(bs)[t] = __ldg(reinterpret_cast<const uint4*>(op->ptr[3] + (uint64_t)n0 * 2) + t);
         compute_sync();
         bias = bs;
     }
     const WideAcc a{&c->wacc_full[h], &c->wacc_empty[h], par, *(volatile uint32_t*)&c->tmem_base + ((uint32_t)(qd * 32) << 16) + 256u * h,
-                    ring + kTcWideStageOff + warp * 4096, bias, seq};
-    const bool fast = !op->ptr[4] && !op->i[6];
+                    ring + kWideStageOff + warp * 4096, bias, seq};
     if (row0 >= op->i[0]) {                                     // (rows beyond M)
         if (wide_wait(p, c, a)) wide_release(a.release);
-    } else if (fast && op->i[5] == DT_F16) wide_store16_any<true>(p, c, op, a, row0, n0);
-    else if (fast && op->i[5] == DT_BF16) wide_store16_any<false>(p, c, op, a, row0, n0);
-    else if (op->i[6] || !op->ptr[4]) wide_store_any<0>(p, c, op, a, row0, n0);
-    else if (op->i[7] == DT_F32) wide_store_any<2>(p, c, op, a, row0, n0);
-    else wide_store_any<1>(p, c, op, a, row0, n0);
+        return;
+    }
+    constexpr bool f16 = (V & 16) != 0;
+    constexpr int kind = V & 15;
+    if constexpr (kind == WIDE_PLAIN) wide_store16<f16, false, 0>(p, c, op, a, row0, n0);
+    else if constexpr (kind == WIDE_SWIGLU) wide_store16<f16, true, 0>(p, c, op, a, row0, n0);
+    else if constexpr (kind == WIDE_GELU) wide_store16<f16, false, 1>(p, c, op, a, row0, n0);
+    else if constexpr (kind == WIDE_ACT) wide_store16<f16, false, 2>(p, c, op, a, row0, n0);
+    else wide_store_any<kind - WIDE_ANY0>(p, c, op, a, row0, n0);
 }
 
 }  // namespace mk

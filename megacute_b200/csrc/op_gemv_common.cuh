@@ -107,16 +107,15 @@ struct StageCursor {
                 continue;
             }
             if (op->kind == MK_OP_GEMM && op->ptr[11]) {
-                // a 256-wide output tile (i 10) takes two 128-row weight tiles per k-tile, one after the
-                // other through the same single-tile slots: `kt` counts weight tiles, `wide` of them per k-tile
+                // a 256-row output tile (i 11; slots of its own) takes one or two 128-row weight tiles (i 10) per k-tile
                 const int kc = op->i[2] / op->i[4];
-                wide = op->i[10] == 256 ? 2 : 1;
+                wide = is_wide_gemm(op) ? op->i[10] >> 7 : 0;
                 reread = op->i[0] > 256;      // (two row tiles run side by side and share the line in flight: measured, evict-first is then the faster)
-                gemm = true; kv = false; seq = in.seq; kt = 0; nk = kc / 64 * wide; kbeg = in.a2 * kc; n0 = in.a1 * 128 * wide;
+                gemm = true; kv = false; seq = in.seq; kt = 0; nk = kc / 64; kbeg = in.a2 * kc; n0 = in.a1 * 128 * max(wide, 1);
                 wmap = reinterpret_cast<const uint8_t*>(op->ptr[11]) + 128;
                 wpack = reinterpret_cast<const uint8_t*>(op->ptr[10]);
                 wstride = (op->i[1] + 127) / 128;
-                wtile0 = (long long)(kbeg / 64) * wstride + in.a1 * wide;
+                wtile0 = (long long)(kbeg / 64) * wstride + in.a1 * max(wide, 1);
                 if (nk > 0) return;
                 continue;
             }
@@ -194,23 +193,24 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
     uint32_t wphase = 0;
     int kvslot = 0;
     uint32_t kvphase = 0, kvgo = 0;
-    enum { MODE_STAGES = 0, MODE_WTILES = 1, MODE_KVTILES = 2, MODE_WWIDE = 3 };
-    int wwslot = 0;
-    uint32_t wwphase = 0, wide_count = 0;            // (and instructions of that kind streamed)
+    enum { MODE_STAGES = 0, MODE_WTILES = 1, MODE_KVTILES = 2, MODE_WWIDE = 3 };     // (MODE_WWIDE + kind: 256-row tiles)
+    int wwslot[2] = {0, 0};
+    uint32_t wwphase[2] = {0, 0}, wide_count = 0;    // (and instructions of those kinds streamed)
     int mode = MODE_STAGES;
     // Wait until the compute side has released every slot of the kind used so far (slot s was last
     // filled in the current round if s < position, else in the previous one).
-    auto drain = [&](int kind) -> bool {
+    auto drain = [&](int kind, int next) -> bool {
         int ok = 1;
         if (lane == 0) {
             if (kind == MODE_WTILES) {
                 for (int s = 0; s < kTcWSlots && ok; ++s)
                     ok = wait_barrier(p, c, &c->w_empty[s], (wphase ^ (s < wslot ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
-            } else if (kind == MODE_WWIDE) {
-                for (int s = 0; s < kTcWideSlots && ok; ++s)
-                    ok = wait_barrier(p, c, &c->ww_empty[s], (wwphase ^ (s < wwslot ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY, 2) ? 1 : 0;
+            } else if (kind >= MODE_WWIDE) {
+                const int k = kind - MODE_WWIDE;
+                for (int s = 0; s < wide_stages(k) && ok; ++s)
+                    ok = wait_barrier(p, c, &c->ww_empty[k][s], (wwphase[k] ^ (s < wwslot[k] ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY, 2) ? 1 : 0;
                 // ... and until the run's epilogues have read their staging rows behind the slots
-                if (ok) ok = wait_word(p, c, &c->wide_done, wide_count, rc.seq, WHERE_STAGING) ? 1 : 0;
+                if (ok && next < MODE_WWIDE) ok = wait_word(p, c, &c->wide_done, wide_count, rc.seq, WHERE_STAGING) ? 1 : 0;
             } else if (kind == MODE_KVTILES) {
                 for (int s = 0; s < kKvSlots && ok; ++s)
                     ok = wait_barrier(p, c, &c->kv_empty[s], (kvphase ^ (s < kvslot ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
@@ -223,7 +223,7 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
     };
     auto enter = [&](int kind) -> bool {              // make the ring's memory serve `kind`
         if (mode == kind) return true;
-        if (!drain(mode)) return false;
+        if (!drain(mode, kind)) return false;
         mode = kind;
         return true;
     };
@@ -266,36 +266,40 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
             rc.seek(p);
             continue;
         }
-        if (rc.gemm && rc.wide == 2) {
-            // 256 x 256 tile GEMM: the two weight tiles of a k-tile (256 rows x 64 K-elements, adjacent in the packed
-            // array) fill one 32 KB slot; its barrier is armed a second time by the feeder warp, for the activations.
+        if (rc.gemm && rc.wide) {
+            // tile GEMM with 256 activation rows: the one or two weight tiles of a k-tile (128 rows x 64 K-elements each, adjacent
+            // in the packed array) fill one slot of its kind; its barrier is armed a second time by the feeder warp, for the activations.
             // One lane: a k-tile's MMAs take 0.58 us, the lane's wait / expect / copy sequence 0.2.
-            if (!enter(MODE_WWIDE)) return;
-            const int nkt = rc.nk >> 1;
+            const int kind = rc.wide == 2 ? 0 : 1, stages = wide_stages(kind);
+            if (!enter(MODE_WWIDE + kind)) return;
+            const int nkt = rc.nk;
+            const uint32_t wbytes = (uint32_t)wide_wbytes(kind);
+            unsigned long long* full = c->ww_full[kind];
+            unsigned long long* empty = c->ww_empty[kind];
             int ok = 1;
             if (lane == 0) {
                 const unsigned long long wpol = rc.reread ? keep_policy : stream_policy;
                 const uint8_t* src = rc.wpack ? rc.wpack + rc.wtile0 * (long long)kTcTileBytes : nullptr;
                 const long long kstep = (long long)rc.wstride * kTcTileBytes;
-                int sl = wwslot;
-                uint32_t ph = wwphase;
+                int sl = wwslot[kind];
+                uint32_t ph = wwphase[kind];
 #pragma unroll 1
                 for (int kt = 0; kt < nkt; ++kt) {
-                    if (!wait_barrier(p, c, &c->ww_empty[sl], ph ^ 1u, rc.seq, WHERE_RING_EMPTY, 2)) { ok = 0; break; }
-                    uint8_t* dst = ring + sl * kTcWideBytes;
-                    mbar_arrive_expect_tx(&c->ww_full[sl], (uint32_t)kTcWideBytes);
+                    if (!wait_barrier(p, c, empty + sl, ph ^ 1u, rc.seq, WHERE_RING_EMPTY, 2)) { ok = 0; break; }
+                    uint8_t* dst = ring + wide_woff(kind, sl);
+                    mbar_arrive_expect_tx(full + sl, wbytes);
                     if (src) {
-                        bulk_g2s_hint(dst, src + kt * kstep, (uint32_t)kTcWideBytes, &c->ww_full[sl], wpol);
+                        bulk_g2s_hint(dst, src + kt * kstep, wbytes, full + sl, wpol);
                     } else {
-                        tma_load_2d(dst, rc.wmap, rc.kbeg + kt * 64, rc.n0, &c->ww_full[sl], wpol);
-                        tma_load_2d(dst + kTcTileBytes, rc.wmap, rc.kbeg + kt * 64, rc.n0 + 128, &c->ww_full[sl], wpol);
+                        tma_load_2d(dst, rc.wmap, rc.kbeg + kt * 64, rc.n0, full + sl, wpol);
+                        if (rc.wide == 2) tma_load_2d(dst + kTcTileBytes, rc.wmap, rc.kbeg + kt * 64, rc.n0 + 128, full + sl, wpol);
                     }
-                    if (++sl == kTcWideSlots) { sl = 0; ph ^= 1u; }
+                    if (++sl == stages) { sl = 0; ph ^= 1u; }
                 }
             }
-            const uint32_t wpos = (uint32_t)wwslot + (uint32_t)nkt;
-            wwslot = (int)(wpos % kTcWideSlots);
-            wwphase ^= (wpos / kTcWideSlots) & 1u;
+            const uint32_t wpos = (uint32_t)wwslot[kind] + (uint32_t)nkt;
+            wwslot[kind] = (int)(wpos % stages);
+            wwphase[kind] ^= (wpos / stages) & 1u;
             ++wide_count;
             if (!__shfl_sync(0xffffffffu, ok, 0)) return;
             rc.idx += gridDim.x;

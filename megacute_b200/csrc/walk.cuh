@@ -16,6 +16,26 @@
 
 namespace mk {
 
+// Behind the barrier that ends instruction `idx`: is the CTA's next one (its metadata has been staged during this one) of the kind
+// mine() says?
+template <class Mine>
+__device__ __forceinline__ bool next_is(const Params& p, Ctrl* c, int idx, Mine mine) {
+    const int next = idx + (int)gridDim.x;
+    if (next >= p.n_insts) return false;
+    const int slot = (next - (int)blockIdx.x) / (int)gridDim.x;
+    const int opi = c->meta.inst[slot % 3][0].x - 1;
+    return opi >= 0 && opi < p.n_ops && mine(&c->meta.desc[slot & 1]);
+}
+// What the kernel's loop does when it fetches instruction `idx`: stage the metadata of the two behind it.
+__device__ __forceinline__ void stage_following(const Params& p, Ctrl* c, int idx) {
+    if ((threadIdx.x >> 5) != 1) return;
+    Meta* mt = &c->meta;
+    const int lane = threadIdx.x & 31, slot = (idx - (int)blockIdx.x) / (int)gridDim.x;
+    stage_row(p, mt, idx + 2 * (int)gridDim.x, (slot + 2) % 3, lane);
+    if (idx + (int)gridDim.x < p.n_insts) stage_op(p, mt, (slot + 1) % 3, (slot & 1) ^ 1, lane);
+    cp_async_commit();
+}
+
 // The kernel's loop has fetched instruction `idx` (its metadata is staged, the staging for the following ones is
 // under way) and chosen this body for it.  mine(op): does the body run this op too?  body(op, a0, a1, a2, seq) runs
 // one instruction between its dependency wait and its arrivals, < 0 when the CTA is aborting.  after() runs behind the
@@ -48,18 +68,9 @@ __device__ __forceinline__ int run_own_insts(const Params& p, Ctrl* c, int idx, 
             trace_rec_rt(p, 1, slot, seq, c->t_fetch, c->t_dep, (long long)globaltimer());
             trace_rec_rt(p, 2, slot, seq, c->t_phase[0], c->t_phase[1], c->t_phase[2]);
         }
-        // the CTA's next instruction: staged during this one, visible behind the barrier of publish()
-        const int next = idx + (int)gridDim.x;
-        if (next >= p.n_insts) break;
-        const int opi = mt->inst[(slot + 1) % 3][0].x - 1;
-        if (opi < 0 || opi >= p.n_ops || !mine(&mt->desc[s2 ^ 1])) break;
-        idx = next;
-        if ((threadIdx.x >> 5) == 1) {           // what the kernel's loop does when it fetches an instruction
-            const int lane = threadIdx.x & 31;
-            stage_row(p, mt, idx + 2 * (int)gridDim.x, (slot + 3) % 3, lane);
-            if (idx + (int)gridDim.x < p.n_insts) stage_op(p, mt, (slot + 2) % 3, s2, lane);
-            cp_async_commit();
-        }
+        if (!next_is(p, c, idx, mine)) break;
+        idx += (int)gridDim.x;
+        stage_following(p, c, idx);
     }
     return idx;
 }

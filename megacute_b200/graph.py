@@ -108,8 +108,8 @@ class View:
 # An operand listed in both columns is updated in place by the op.  Optional operands may be
 # None.  The semantic definition of each kind is in the builder method's docstring below.
 OP_TABLE = {
-    "Linear":          (("x", "w", "bias", "residual", "norm_w"), ("out",), ("act", "rms_eps", "bn")),
-    "LinearSplit":     (("x", "w", "norm_w"), ("ws",), ("splits", "rms_eps", "bn")),
+    "Linear":          (("x", "w", "bias", "residual", "norm_w"), ("out",), ("act", "rms_eps", "bm", "bn")),
+    "LinearSplit":     (("x", "w", "norm_w"), ("ws",), ("splits", "rms_eps", "bm", "bn")),
     "SplitFinalize":   (("ws", "bias", "residual"), ("out", "ws"), ("act",)),
     "Unary":           (("x",), ("out",), ("fn",)),
     "Binary":          (("a", "b", "gate"), ("out",), ("fn", "b_group", "gate_group")),

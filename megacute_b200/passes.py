@@ -378,11 +378,11 @@ def fuse_finalize_attention(g: Graph) -> Graph:
 
 
 def wide_tiles(g: Graph, sm_count: int) -> Graph:
-    """Tile linears with many rows get 128 x 256 output tiles when that is modelled faster: the main
-    loop of a tile GEMM is bound by the operand bytes an SM draws from L2, and a 256-wide tile reuses
-    each activation k-tile for two weight tiles (48 KB instead of 64 KB per 128 x 256 x 64 block).
-    rounds x (k-tiles x time per k-tile + epilogue), rounds = instructions per SM.
-    MEGACUTE_B200_WIDE_TILES=0 / 1 forces the choice where the shape allows it."""
+    """Tile linears with more than WIDE_MIN_ROWS rows get tiles of 256 rows -- 256 x 256 or 256 x 128, the form whose
+    epilogue runs beside the next tile's main loop and whose operands cost fewer bytes per flop
+    (csrc/op_gemm_tc_wide.cuh) -- where that is modelled faster than 128 x 128 tiles:
+    rounds x (k-tiles x time per k-tile + time per tile) + time per op, rounds = instructions per SM.
+    MEGACUTE_B200_WIDE_TILES=0 / 1 forces 128 x 128 / 256 x 256 where the shape allows it."""
     force = os.environ.get("MEGACUTE_B200_WIDE_TILES")
     out = g.derive()
     ops = []
@@ -391,12 +391,20 @@ def wide_tiles(g: Graph, sm_count: int) -> Graph:
             M, K = op.x.shape
             N = op.w.rows
             splits = op.splits if op.kind == "LinearSplit" else 1
-            if N % C.GEMM_BN_WIDE == 0 and K % (64 * splits) == 0 and M > C.WIDE_MIN_ROWS and force != "0":
-                mt, mtw, kt = -(-M // C.GEMM_BM), -(-M // C.GEMM_BM_WIDE), K // 64 // splits
-                narrow = -(-(mt * (N // C.GEMM_BN) * splits) // sm_count) * (kt * C.KTILE_US + C.EPILOGUE_US)
-                wide = -(-(mtw * (N // C.GEMM_BN_WIDE) * splits) // sm_count) * (kt * C.KTILE_US_WIDE + C.EPILOGUE_US_WIDE)
-                if wide < narrow or force == "1":
-                    op = op.clone(bn=C.GEMM_BN_WIDE)
+            kt = K // 64 // splits
+
+            def cost(bm, bn):
+                tile, k, once = C.GEMM_COST_US[bm, bn]
+                return -(-(-(-M // bm) * (N // bn) * splits) // sm_count) * (kt * k + tile) + once
+
+            shapes = [(bm, bn) for bm, bn in C.GEMM_COST_US if bm == C.GEMM_BM or (N % bn == 0 and K % (64 * splits) == 0 and M > C.WIDE_MIN_ROWS)]
+            best = min(shapes, key=lambda s: cost(*s))
+            if force == "0":
+                best = (C.GEMM_BM, C.GEMM_BN)
+            elif force == "1" and (C.GEMM_BM_WIDE, C.GEMM_BN_WIDE) in shapes:
+                best = (C.GEMM_BM_WIDE, C.GEMM_BN_WIDE)
+            if best != (C.GEMM_BM, C.GEMM_BN):
+                op = op.clone(bm=best[0], bn=best[1])
         ops.append(op)
     out.ops = ops
     return out

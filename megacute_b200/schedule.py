@@ -110,7 +110,7 @@ def is_gemv(op: Op) -> bool:
 
 def gemm_rows(op: Op) -> int:
     """Activation rows of a tile linear's output tile."""
-    return C.GEMM_BM_WIDE if op.bn == C.GEMM_BN_WIDE else C.GEMM_BM
+    return op.bm or C.GEMM_BM
 
 
 def tile_op(op: Op, sm_count: int) -> Tiled:
@@ -133,7 +133,7 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
         out = op.out if k == "Linear" else op.ws
         M = out.rows
         swi = k == "Linear" and op.act == "swiglu"
-        BN = op.bn or C.GEMM_BN                       # tile: 128 x 128, or 256 x 256 (passes.wide_tiles)
+        BN = op.bn or C.GEMM_BN                       # tile: 128 x 128, 256 x 128 or 256 x 256 (passes.wide_tiles)
         BM = gemm_rows(op)
         on = BN // 2 if swi else BN
         m, nn = gemm_raster(_ceil(M, BM), _ceil(out.cols, on), 8 * C.GEMM_BM // BM)
