@@ -92,12 +92,24 @@ __device__ __forceinline__ void wide_feed_end(Ctrl* c, const WideFeed& f) {
     }
 }
 
-// ---- issuer warp, lane 0 -----------------------------------------------------------------------------------------------------
+// ---- issuer warp -------------------------------------------------------------------------------------------------------------
+// The whole warp walks the loop and one elected lane issues: under a branch that only one lane takes, the compiler builds each
+// instruction's operands in ordinary registers and moves them over one by one, and an N = 128 instruction (64 cycles of the tensor
+// pipe) then takes 100 cycles to issue instead of 85 (measured stand-alone; N = 256, 128 cycles, is not affected).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{ .reg .pred q; elect.sync _|q, 0xffffffff; selp.u32 %0, 1, 0, q; }" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ bool issuer_wait(const Params& p, Ctrl* c, unsigned long long* bar, uint32_t parity, int seq, int where, unsigned patience) {
+    const bool ok = wait_barrier(p, c, bar, parity, seq, where, patience);
+    return __all_sync(0xffffffffu, ok) != 0;
+}
 __device__ __forceinline__ void wide_issuer(const Params& p, Ctrl* c, uint8_t* ring) {
     const uint64_t d0 = tc_smem_desc(smem_u32(ring));
     uint32_t slot[2] = {0, 0}, phase[2] = {0, 0};
     for (uint32_t n = 0;; ++n) {
-        if (!wait_barrier(p, c, &c->wide_told[n & 3u], (n >> 2) & 1u, 0, WHERE_DEP, 4)) return;
+        if (!issuer_wait(p, c, &c->wide_told[n & 3u], (n >> 2) & 1u, 0, WHERE_DEP, 4)) return;
         const int4 info = c->wide_info[n & 3u];
         const int nk = info.x;
         if (nk <= 0) return;
@@ -107,30 +119,60 @@ __device__ __forceinline__ void wide_issuer(const Params& p, Ctrl* c, uint8_t* r
         const int kind = (info.y >> 4) == 2 ? 0 : 1;
         uint32_t acc = 0, s = slot[kind], ph = phase[kind];
         for (int kt = 0; kt < nk; ++kt) {
-            if (!wait_barrier(p, c, &c->ww_full[kind][s], ph, info.w, WHERE_RING_FULL, 2)) return;
-            if (kt == 0 && !wait_barrier(p, c, &c->wacc_empty[0], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return;
+            if (!issuer_wait(p, c, &c->ww_full[kind][s], ph, info.w, WHERE_RING_FULL, 2)) return;
+            if (kt == 0) {
+                if (!issuer_wait(p, c, &c->wacc_empty[0], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return;
+                // (the two halves of a 256-column tile are issued one after the other: the first may start before the second's
+                // accumulator has been read)
+                if (kind && !issuer_wait(p, c, &c->wacc_empty[1], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return;
+            }
             tc_fence_after();
             const uint64_t ad = d0 + (uint32_t)(wide_xoff((int)s) >> 4), bd = d0 + (uint32_t)(wide_woff(kind, (int)s) >> 4);
+            if (kind) {
+                // N = 128: an instruction into the accumulator the previous one wrote starts late, so the two accumulators take turns
+                if (elect_one()) {
+                    if (both) {
 #pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem, ad + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
-            if (kt == nk - 1) tc_commit(&c->wacc_full[0]);
-            if (kt == 0) {
-                if (!wait_barrier(p, c, &c->wacc_empty[1], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return;
-                tc_fence_after();
-            }
-            if (both) {
+                        for (int k16 = 0; k16 < 4; ++k16) {
+                            tc_mma(tmem, ad + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+                            tc_mma(tmem + 256, ad + (kTcTileBytes >> 4) + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+                        }
+                    } else {
 #pragma unroll
-                for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem + 256, ad + (kTcTileBytes >> 4) + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+                        for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem, ad + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+                    }
+                    if (kt == nk - 1) tc_commit(&c->wacc_full[0]);
+                    tc_commit(&c->ww_empty[kind][s]);
+                }
+            } else {
+                if (elect_one()) {
+#pragma unroll
+                    for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem, ad + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+                    if (kt == nk - 1) tc_commit(&c->wacc_full[0]);
+                }
+                if (kt == 0) {
+                    if (!issuer_wait(p, c, &c->wacc_empty[1], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return;
+                    tc_fence_after();
+                }
+                if (elect_one()) {
+                    if (both) {
+#pragma unroll
+                        for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem + 256, ad + (kTcTileBytes >> 4) + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+                    }
+                    tc_commit(&c->ww_empty[kind][s]);
+                }
             }
+            __syncwarp();
             acc = 1;
-            if (!check_phase(p, c, &c->ww_empty[kind][s], ph, info.w, WHERE_CHECK_RELEASE)) return;
-            tc_commit(&c->ww_empty[kind][s]);
             if (++s == (uint32_t)wide_stages(kind)) { s = 0; ph ^= 1u; }
         }
         slot[kind] = s;
         phase[kind] = ph;
-        tc_commit(&c->wacc_full[1]);
-        if (p.trace_cap > 0) c->t_phase[1] = (long long)globaltimer();
+        if (elect_one()) {
+            tc_commit(&c->wacc_full[1]);
+            if (p.trace_cap > 0) c->t_phase[1] = (long long)globaltimer();
+        }
+        __syncwarp();
     }
 }
 

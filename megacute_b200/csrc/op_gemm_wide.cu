@@ -54,7 +54,6 @@ __device__ int mk_run_gemm_wide(const Params& p, int idx) {
 
 __device__ void mk_wide_issuer(const Params& p) {
     const SmemMap m = smem_map();
-    if ((threadIdx.x & 31) == 0) wide_issuer(p, m.ctrl, m.ring);
-    __syncwarp();
+    wide_issuer(p, m.ctrl, m.ring);
 }
 }  // namespace mk
