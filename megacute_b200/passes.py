@@ -227,6 +227,27 @@ def choose_k_splits(M: int, N: int, K: int, sm_count: int) -> int:
     return best
 
 
+def plan_tiles(M: int, N: int, K: int, sm_count: int, max_splits: int, finalize: bool) -> tuple:
+    """(K splits, tile rows, tile columns) of a tile linear with more than WIDE_MIN_ROWS rows: the plan with the lowest
+    modelled time  rounds x (k-tiles x time per k-tile + time per tile) + time per op [+ reduce-adds, and the
+    SplitFinalize behind them], rounds = instructions per SM, with constants from the kernel's timeline
+    (config.GEMM_COST_US).  Tiles of 256 rows -- 256 x 256 or 256 x 128 -- are the form whose epilogue runs beside the next
+    tile's main loop and whose operands cost fewer bytes per flop (csrc/op_gemm_tc_wide.cuh)."""
+    best, best_cost = (1, C.GEMM_BM, C.GEMM_BN), float("inf")
+    for (bm, bn), (tile, k, once) in C.GEMM_COST_US.items():
+        if bm != C.GEMM_BM and N % bn:
+            continue
+        for s in range(1, max_splits + 1):
+            whole = K % (64 * s) == 0
+            if (s > 1 and (K % (C.GEMM_BK * s) or K // C.GEMM_BK // s < C.MIN_SPLIT_KTILES)) or (bm != C.GEMM_BM and not whole):
+                continue
+            rounds = -(-(-(-M // bm) * -(-N // bn) * s) // sm_count)
+            cost = rounds * (K / 64 / s * k + tile) + once + (M * N * s * 4 / (C.REDUCE_GBPS * 1e3) + (C.FINALIZE_US if finalize else 0.0) if s > 1 else 0.0)
+            if cost < best_cost - 1e-9:
+                best, best_cost = (s, bm, bn), cost
+    return best
+
+
 def split_k(g: Graph, sm_count: int) -> Graph:
     out = g.derive()
     alias: dict[int, View] = {}      # id of a dropped output buffer -> residual view that now holds it
@@ -236,13 +257,16 @@ def split_k(g: Graph, sm_count: int) -> Graph:
         op = op0.clone(**{k: _retarget(v, alias) for k, v in op0.view_fields()}) if alias else op0
         if op.kind == "Linear" and op.act != "swiglu" and not gemv_eligible(op.x.rows, op.x.cols):
             M, K = op.x.shape
-            s = choose_k_splits(M, op.w.rows, K, sm_count)
+            r = op.residual
+            whole = op.out.rect == (0, op.out.buf.rows, 0, op.out.buf.cols)
+            inplace = (r is not None and op.bias is None and op.act is None and op.norm_w is None
+                       and r.buf.kind == "temp" and op.out.buf.kind == "temp" and whole
+                       and not _reads_buffer(src[i + 1:], r.buf))
+            if M > C.WIDE_MIN_ROWS:
+                s = plan_tiles(M, op.w.rows, K, sm_count, C.MAX_K_SPLITS, not inplace)[0]
+            else:
+                s = choose_k_splits(M, op.w.rows, K, sm_count)
             if s > 1:
-                r = op.residual
-                whole = op.out.rect == (0, op.out.buf.rows, 0, op.out.buf.cols)
-                inplace = (r is not None and op.bias is None and op.act is None and op.norm_w is None
-                           and r.buf.kind == "temp" and op.out.buf.kind == "temp" and whole
-                           and not _reads_buffer(src[i + 1:], r.buf))
                 if inplace:
                     alias[op.out.buf.id] = r
                     new = Op("LinearSplit", x=op.x, w=op.w, ws=r, splits=s)
@@ -317,6 +341,9 @@ def promote_temps(g: Graph) -> Graph:
     for op in g.ops:
         for name, v in op.view_fields():
             users.setdefault(v.buf.id, []).append((op, name))
+    # the residual stream that K splits reduce-add into, however large: added in bf16, eight partial sums per layer are rounded to
+    # eight bits one by one (measured: 4 layers of the 1B shape over 600 tokens, logits 1.5e-2 rel-L2 apart from one run to the next)
+    accumulated = {op.ws.buf.id for op in g.ops if op.kind == "LinearSplit"}
     swap: dict[int, Buffer] = {}
     for b in g.buffers:
         if b.kind != "temp" or b.dtype != torch.bfloat16 or b.id not in users:
@@ -324,7 +351,7 @@ def promote_temps(g: Graph) -> Graph:
         if any(v.buf is b for v in g.outputs):
             continue
         for dt in (torch.float32, torch.float16):
-            if dt == torch.float32 and b.rows * b.cols * 4 > F32_TEMP_BYTES:
+            if dt == torch.float32 and b.rows * b.cols * 4 > F32_TEMP_BYTES and b.id not in accumulated:
                 continue
             if all(_accepts(op, name, dt) for op, name in users[b.id]):
                 swap[b.id] = Buffer(b.name, b.rows, b.cols, dt, "temp")
@@ -378,10 +405,7 @@ def fuse_finalize_attention(g: Graph) -> Graph:
 
 
 def wide_tiles(g: Graph, sm_count: int) -> Graph:
-    """Tile linears with more than WIDE_MIN_ROWS rows get tiles of 256 rows -- 256 x 256 or 256 x 128, the form whose
-    epilogue runs beside the next tile's main loop and whose operands cost fewer bytes per flop
-    (csrc/op_gemm_tc_wide.cuh) -- where that is modelled faster than 128 x 128 tiles:
-    rounds x (k-tiles x time per k-tile + time per tile) + time per op, rounds = instructions per SM.
+    """Output tile of every tile linear with more than WIDE_MIN_ROWS rows (plan_tiles, with the K splits split_k chose).
     MEGACUTE_B200_WIDE_TILES=0 / 1 forces 128 x 128 / 256 x 256 where the shape allows it."""
     force = os.environ.get("MEGACUTE_B200_WIDE_TILES")
     out = g.derive()
@@ -391,20 +415,13 @@ def wide_tiles(g: Graph, sm_count: int) -> Graph:
             M, K = op.x.shape
             N = op.w.rows
             splits = op.splits if op.kind == "LinearSplit" else 1
-            kt = K // 64 // splits
-
-            def cost(bm, bn):
-                tile, k, once = C.GEMM_COST_US[bm, bn]
-                return -(-(-(-M // bm) * (N // bn) * splits) // sm_count) * (kt * k + tile) + once
-
-            shapes = [(bm, bn) for bm, bn in C.GEMM_COST_US if bm == C.GEMM_BM or (N % bn == 0 and K % (64 * splits) == 0 and M > C.WIDE_MIN_ROWS)]
-            best = min(shapes, key=lambda s: cost(*s))
-            if force == "0":
-                best = (C.GEMM_BM, C.GEMM_BN)
-            elif force == "1" and (C.GEMM_BM_WIDE, C.GEMM_BN_WIDE) in shapes:
-                best = (C.GEMM_BM_WIDE, C.GEMM_BN_WIDE)
-            if best != (C.GEMM_BM, C.GEMM_BN):
-                op = op.clone(bm=best[0], bn=best[1])
+            if M > C.WIDE_MIN_ROWS and K % (64 * splits) == 0 and force != "0":
+                # (a split op is planned as `splits` independent products over K / splits)
+                _, bm, bn = plan_tiles(M, N, K // splits, max(1, sm_count // splits), 1, False)
+                if force == "1" and N % C.GEMM_BN_WIDE == 0:
+                    bm, bn = C.GEMM_BM_WIDE, C.GEMM_BN_WIDE
+                if bm != C.GEMM_BM:
+                    op = op.clone(bm=bm, bn=bn)
         ops.append(op)
     out.ops = ops
     return out
