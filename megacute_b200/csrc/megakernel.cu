@@ -144,7 +144,8 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
             // around the bodies whose entry is cheap
                         const int ppos = pos.stage | ((int)pos.phase << 8);
             int npos = ppos;
-            bool known = true, aborting = false, traced = false;
+            bool known = true, aborting = false;
+            int run_last = idx - 1;                 // (a body that keeps the walk: the index of the last instruction it ran, or -1 when aborting)
             switch (op->kind) {
                 case MK_OP_GEMV:
                     if (op->flags & GEMV_F_UNITS) {
@@ -157,17 +158,11 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                         aborting = publish(p, c, in.narrive, arrive_off);
                     }
                     break;
-                case MK_OP_GEMM: {
+                case MK_OP_GEMM:
                     // (runs this instruction and the CTA's following ones for as long as they are the body's own: walk.cuh)
-                    const int last = is_wide_gemm(op) ? mk_run_gemm_wide(p, idx) : mk_run_gemm(p, idx);
-                    aborting = last < 0;
-                    if (!aborting) {
-                        slot += (last - idx) / (int)gridDim.x;
-                        idx = last;
-                    }
-                    traced = true;
+                    run_last = is_wide_gemm(op) ? mk_run_gemm_wide(p, idx) : mk_run_gemm(p, idx);
                     break;
-                }
+                case MK_OP_ELTWISE: run_last = mk_run_eltwise(p, op, idx); break;
                 case MK_OP_ATTENTION:
                     if (wait_deps(p, c, in.nwait, wait_off, in.seq)) { aborting = true; break; }
                     if (TRACE && threadIdx.x == 0) c->t_dep = (long long)globaltimer();
@@ -178,6 +173,9 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                 case MK_OP_DECODE_ATTN:
                     aborting = mk_op_decode_attn(p, op, in.a0, in.a1, in.a2, in.nwait, wait_off, in.seq, in.narrive, arrive_off);
                     break;
+                case MK_OP_NORM:
+                    if (op->i[3] > 1) { run_last = mk_run_norm(p, op, idx); break; }
+                    [[fallthrough]];
                 default:
                     if (wait_deps(p, c, in.nwait, wait_off, in.seq)) { aborting = true; break; }
                     if (TRACE && threadIdx.x == 0) c->t_dep = (long long)globaltimer();
@@ -185,10 +183,18 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                     aborting = publish(p, c, in.narrive, arrive_off);
                     break;
             }
+            const bool ran = run_last != idx - 1;
+            if (ran) {
+                aborting = run_last < 0;
+                if (!aborting) {
+                    slot += (run_last - idx) / (int)gridDim.x;
+                    idx = run_last;
+                }
+            }
             if (!known && threadIdx.x == 0) report(p, c, MK_DEV_BAD_INST, in.seq, 1, op->kind, idx, 0);
             pos.stage = npos & 0xff;
             pos.phase = (uint32_t)(npos >> 8);
-            if (TRACE && threadIdx.x == 0 && !traced) {
+            if (TRACE && threadIdx.x == 0 && !ran) {
                 const bool marks = op->kind == MK_OP_GEMV || op->kind == MK_OP_DECODE_ATTN || op->kind == MK_OP_GEMM || op->kind == MK_OP_ATTENTION;
                 trace_rec<TRACE>(p, 1, slot, in.seq, t0, c->t_dep, c->t_pub ? c->t_pub : (long long)globaltimer());
                 if (marks) trace_rec<TRACE>(p, 2, slot, in.seq, c->t_phase[0], c->t_phase[1], c->t_phase[2]);
@@ -429,7 +435,7 @@ static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
                     if (d.i[5] <= 0 || a0 < 0 || a0 >= ceil_div(d.i[0], d.i[5]) || a1 < 0 || a1 * 512 >= d.i[1]) why = "finalize: tile outside the output";
                     break;
                 case MK_OP_ELTWISE:
-                    if (a0 < 0 || a0 * 32 >= d.i[0] || a1 < 0 || a1 * 512 >= d.i[1]) why = "pointwise: tile outside the output";
+                    if (d.i[10] <= 0 || a0 < 0 || a0 * d.i[10] >= d.i[0] || a1 < 0 || a1 * 512 >= d.i[1]) why = "pointwise: tile outside the output";
                     break;
                 case MK_OP_NORM:
                     if (d.i[3] <= 0 || a0 < 0 || a0 * d.i[3] >= d.i[0]) why = "norm: row group outside the rows";

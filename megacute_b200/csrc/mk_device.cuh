@@ -414,6 +414,18 @@ __device__ __forceinline__ void unpack8_raw(const Raw8& r, int dtype, float* f) 
         f[4] = __uint_as_float(r.hi.x); f[5] = __uint_as_float(r.hi.y); f[6] = __uint_as_float(r.hi.z); f[7] = __uint_as_float(r.hi.w);
     }
 }
+// a raw vector of 8 elements: 16 bytes when the element type is known to be 16-bit, else room for fp32
+template <bool SIXTEEN> struct Raw8x;
+template <> struct Raw8x<true> {
+    uint4 v;
+    __device__ __forceinline__ void load(const void* base, long long elem, int) { v = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + elem)); }
+    __device__ __forceinline__ void unpack(int dtype, float* f) const { Raw8 r; r.lo = v; r.hi = v; unpack8_raw(r, dtype == DT_F16 ? DT_F16 : DT_BF16, f); }
+};
+template <> struct Raw8x<false> {
+    Raw8 v;
+    __device__ __forceinline__ void load(const void* base, long long elem, int dtype) { v = load8_raw(base, elem, dtype); }
+    __device__ __forceinline__ void unpack(int dtype, float* f) const { unpack8_raw(v, dtype, f); }
+};
 __device__ __forceinline__ void store8(void* base, long long elem, int dtype, const float* f) {
     if (dtype == DT_BF16) {
         *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(base) + elem) = pack8(f);

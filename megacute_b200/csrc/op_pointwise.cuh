@@ -7,18 +7,6 @@
 namespace mk {
 
 constexpr int kEwRows = 32, kEwCols = 512;                 // config.py EW_ROWS / EW_COLS
-enum { EW_UNARY = 0, EW_BINARY, EW_SWIGLU, EW_MODULATE, EW_ROPE, EW_GATED };
-enum { BIN_ADD = 0, BIN_SUB, BIN_MUL, BIN_MAX, BIN_MIN };
-
-__device__ __forceinline__ float apply_bin(int fn, float a, float b) {
-    switch (fn) {
-        case BIN_ADD: return a + b;
-        case BIN_SUB: return a - b;
-        case BIN_MUL: return a * b;
-        case BIN_MAX: return fmaxf(a, b);
-        default: return fminf(a, b);
-    }
-}
 
 // MK_OP_FINALIZE: out = act(ws + bias) + residual; ws = 0.
 // ptr 0 ws (fp32), 1 out, 2 bias, 3 residual; i 0 R, 1 C, 2 act, 3 out dtype, 4 residual dtype,
@@ -53,259 +41,6 @@ static __device__ __noinline__ void op_finalize(const mk_op_desc* op, int a0, in
     }
 }
 
-// a raw vector of 8 elements: 16 bytes when the element type is known to be 16-bit, else room for fp32
-template <bool SIXTEEN> struct Raw8x;
-template <> struct Raw8x<true> {
-    uint4 v;
-    __device__ __forceinline__ void load(const void* base, long long elem, int) { v = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + elem)); }
-    __device__ __forceinline__ void unpack(int dtype, float* f) const { Raw8 r; r.lo = v; r.hi = v; unpack8_raw(r, dtype == DT_F16 ? DT_F16 : DT_BF16, f); }
-};
-template <> struct Raw8x<false> {
-    Raw8 v;
-    __device__ __forceinline__ void load(const void* base, long long elem, int dtype) { v = load8_raw(base, elem, dtype); }
-    __device__ __forceinline__ void unpack(int dtype, float* f) const { unpack8_raw(v, dtype, f); }
-};
-
-// Binary / modulate tile whose rows all read ONE row of the second (and third) operand -- a per-image gate, scale or
-// shift over that image's tokens: the thread keeps its 8 columns of them and streams a, eight rows in flight when a is 16-bit.
-template <int MODE>
-static __device__ __noinline__ void eltwise_tile_one_group(const mk_op_desc* op, int r0, int col, int rows, int rowp, int rpp) {
-    const int fn = op->i[3], group = op->i[4];
-    const int adt = op->i[6], bdt = op->i[7], cdt = op->i[8], odt = op->i[9];
-    const void* A = reinterpret_cast<const void*>(op->ptr[0]);
-    void* O = reinterpret_cast<void*>(op->ptr[3]);
-    const long long grow = r0 / group;
-    float b[8], cc[8];
-    load8(reinterpret_cast<const void*>(op->ptr[1]), grow * op->ld[1] + col, bdt, b);
-    if (MODE == EW_MODULATE) {
-        load8(reinterpret_cast<const void*>(op->ptr[2]), grow * op->ld[2] + col, cdt, cc);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) b[e] += 1.0f;
-    }
-    auto body = [&](auto tag) {
-        constexpr bool S16 = decltype(tag)::value;
-        constexpr int UN = S16 ? 8 : 4;
-        for (int rr = rowp; rr < rows; rr += UN * rpp) {
-            Raw8x<S16> ra[UN];
-#pragma unroll
-            for (int u = 0; u < UN; ++u)
-                if (rr + u * rpp < rows) ra[u].load(A, (long long)(r0 + rr + u * rpp) * op->ld[0] + col, adt);
-#pragma unroll
-            for (int u = 0; u < UN; ++u) {
-                if (rr + u * rpp >= rows) continue;
-                float a[8];
-                ra[u].unpack(adt, a);
-                if (MODE == EW_MODULATE) {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) a[e] = fmaf(a[e], b[e], cc[e]);
-                } else if (fn == BIN_MUL) {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) a[e] *= b[e];
-                } else if (fn == BIN_ADD) {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) a[e] += b[e];
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) a[e] = apply_bin(fn, a[e], b[e]);
-                }
-                store8(O, (long long)(r0 + rr + u * rpp) * op->ld[3] + col, odt, a);
-            }
-        }
-    };
-    if (adt != DT_F32) body(std::true_type{});
-    else body(std::false_type{});
-}
-
-// One tile of a pointwise op other than rope.  A pointwise instruction is a few thousand elements; with the mode, the
-// function and the tile geometry as run-time switches and divisions inside the vector loop it was instruction-bound
-// (8.7 us for a 32 x 512 modulate tile: ~300 instructions per 8-element vector at a fraction of an instruction per
-// cycle; more loads in flight changed nothing).  Here the mode is a template parameter, the function is switched once
-// per vector, a thread keeps its columns and walks rows (no division in the loop), and two rows are in flight.
-template <int MODE, bool SIXTEEN>
-static __device__ __noinline__ void eltwise_tile(const mk_op_desc* op, int r0, int c0, int rows, int cols) {
-    const int fn = op->i[3], group = op->i[4];
-    const int adt = op->i[6], bdt = op->i[7], cdt = op->i[8], odt = op->i[9];
-    const void* A = reinterpret_cast<const void*>(op->ptr[0]);
-    const void* B = reinterpret_cast<const void*>(op->ptr[1]);
-    const void* Cp = reinterpret_cast<const void*>(op->ptr[2]);
-    void* O = reinterpret_cast<void*>(op->ptr[3]);
-    constexpr bool HASB = MODE != EW_UNARY, HASC = MODE == EW_MODULATE, GROUPED = MODE == EW_BINARY || MODE == EW_MODULATE;
-    const int vpr = cols >> 3;                                   // vectors per row: at most 64
-    // threads cover whole rows side by side: thread -> (row of the pass, vector of the row)
-    const int tpr = vpr <= 1 ? 1 : vpr <= 2 ? 2 : vpr <= 4 ? 4 : vpr <= 8 ? 8 : vpr <= 16 ? 16 : vpr <= 32 ? 32 : 64;   // threads per row
-    const int rpp = kComputeThreads / tpr;                       // rows per pass
-    const int vec = threadIdx.x & (tpr - 1), rowp = threadIdx.x / tpr;
-    if (vec >= vpr) return;
-    const int col = c0 + vec * 8;
-    if (GROUPED && (r0 / group) == ((r0 + rows - 1) / group)) {
-        // every row of the tile reads the same row of b (and c): a thread's column of them is loaded once, and only a streams
-        eltwise_tile_one_group<MODE>(op, r0, col, rows, rowp, rpp);
-        return;
-    }
-    // rows in flight per thread: with 16-bit operands a vector is four registers and a thread's whole share of the tile
-    // (eight rows) fits; otherwise two (more spill, and a spill is an L2 round trip like the loads it was to hide)
-    constexpr int UN = SIXTEEN ? (HASC ? 2 : HASB ? 4 : 8) : 2;
-    for (int rr = rowp; rr < rows; rr += UN * rpp) {
-        Raw8x<SIXTEEN> ra[UN], rb[HASB ? UN : 1], rc[HASC ? UN : 1];
-#pragma unroll
-        for (int u = 0; u < UN; ++u) {
-            const int r = r0 + rr + u * rpp;
-            if (rr + u * rpp >= rows) continue;
-            ra[u].load(A, (long long)r * op->ld[0] + col, adt);
-            const long long rb_row = GROUPED ? r / group : r;
-            if (HASB) rb[u].load(B, rb_row * op->ld[1] + col, bdt);
-            if (HASC) rc[u].load(Cp, rb_row * op->ld[2] + col, cdt);
-        }
-#pragma unroll
-        for (int u = 0; u < UN; ++u) {
-            const int r = r0 + rr + u * rpp;
-            if (rr + u * rpp >= rows) continue;
-            float a[8], b[8], cc[8];
-            ra[u].unpack(adt, a);
-            if (HASB) rb[u].unpack(bdt, b);
-            if (MODE == EW_UNARY) {
-                switch (fn) {
-                    case ACT_NONE: break;
-                    case ACT_SILU:
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) a[e] = a[e] * sigmoidf_(a[e]);
-                        break;
-                    default:
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) a[e] = apply_act(fn, a[e]);
-                }
-            } else if (MODE == EW_BINARY) {
-                switch (fn) {
-                    case BIN_ADD:
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) a[e] += b[e];
-                        break;
-                    case BIN_MUL:
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) a[e] *= b[e];
-                        break;
-                    default:
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) a[e] = apply_bin(fn, a[e], b[e]);
-                }
-            } else if (MODE == EW_SWIGLU) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) a[e] = apply_act(fn, a[e]) * b[e];
-            } else {  // EW_MODULATE: x * (1 + scale[g]) + shift[g]
-                rc[u].unpack(cdt, cc);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) a[e] = fmaf(a[e], 1.0f + b[e], cc[e]);
-            }
-            store8(O, (long long)r * op->ld[3] + col, odt, a);
-        }
-    }
-}
-
-// EW_GATED: out = fn(a, b * c[r / group]) -- a gated residual, x + y * gate[image] (passes.fuse_pointwise).  a and b
-// stream (two rows in flight), the gate row of a tile is loaded once when the tile lies in one group.
-static __device__ __noinline__ void eltwise_tile_gated(const mk_op_desc* op, int r0, int c0, int rows, int cols) {
-    const int fn = op->i[3], group = op->i[4];
-    const int adt = op->i[6], bdt = op->i[7], cdt = op->i[8], odt = op->i[9];
-    const void* A = reinterpret_cast<const void*>(op->ptr[0]);
-    const void* B = reinterpret_cast<const void*>(op->ptr[1]);
-    const void* G = reinterpret_cast<const void*>(op->ptr[2]);
-    void* O = reinterpret_cast<void*>(op->ptr[3]);
-    const int vpr = cols >> 3;
-    const int tpr = vpr <= 1 ? 1 : vpr <= 2 ? 2 : vpr <= 4 ? 4 : vpr <= 8 ? 8 : vpr <= 16 ? 16 : vpr <= 32 ? 32 : 64;
-    const int rpp = kComputeThreads / tpr;
-    const int vec = threadIdx.x & (tpr - 1), rowp = threadIdx.x / tpr;
-    if (vec >= vpr) return;
-    const int col = c0 + vec * 8;
-    const bool one = (r0 / group) == ((r0 + rows - 1) / group);
-    float gt[8];
-    if (one) load8(G, (long long)(r0 / group) * op->ld[2] + col, cdt, gt);
-    constexpr int UN = 2;
-    for (int rr = rowp; rr < rows; rr += UN * rpp) {
-        Raw8 ra[UN], rb[UN];
-#pragma unroll
-        for (int u = 0; u < UN; ++u) {
-            const int r = r0 + rr + u * rpp;
-            if (rr + u * rpp >= rows) continue;
-            ra[u] = load8_raw(A, (long long)r * op->ld[0] + col, adt);
-            rb[u] = load8_raw(B, (long long)r * op->ld[1] + col, bdt);
-        }
-#pragma unroll
-        for (int u = 0; u < UN; ++u) {
-            const int r = r0 + rr + u * rpp;
-            if (rr + u * rpp >= rows) continue;
-            float a[8], b[8];
-            unpack8_raw(ra[u], adt, a);
-            unpack8_raw(rb[u], bdt, b);
-            if (!one) load8(G, (long long)(r / group) * op->ld[2] + col, cdt, gt);
-            if (fn == BIN_ADD) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) a[e] = fmaf(b[e], gt[e], a[e]);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) a[e] = apply_bin(fn, a[e], b[e] * gt[e]);
-            }
-            store8(O, (long long)r * op->ld[3] + col, odt, a);
-        }
-    }
-}
-
-// MK_OP_ELTWISE.  ptr 0 a (x / gate), 1 b (b / up / scale / cos), 2 c (shift / sin), 3 out
-// i 0 R, 1 C, 2 mode, 3 fn (activation or binary code), 4 group (rows of a per row of b; rope: seq),
-//   5 head_dim (rope), 6..9 dtypes of a, b, c, out (DT_*).  args: 0 row tile, 1 col tile.
-static __device__ __noinline__ void op_eltwise(const mk_op_desc* op, int a0, int a1) {
-    const int R = op->i[0], Cc = op->i[1], mode = op->i[2], fn = op->i[3], group = op->i[4];
-    const int adt = op->i[6], bdt = op->i[7], cdt = op->i[8], odt = op->i[9];
-    const int r0 = a0 * kEwRows, c0 = a1 * kEwCols;
-    const int rows = min(kEwRows, R - r0), cols = min(kEwCols, Cc - c0);
-    const void* A = reinterpret_cast<const void*>(op->ptr[0]);
-    const void* B = reinterpret_cast<const void*>(op->ptr[1]);
-    const void* Cp = reinterpret_cast<const void*>(op->ptr[2]);
-    void* O = reinterpret_cast<void*>(op->ptr[3]);
-    if (mode == EW_ROPE) {
-        const int D = op->i[5], half = D >> 1, hv = half >> 3;        // vectors per half head
-        const int heads = cols / D;
-        const int units = rows * heads * hv;
-        for (int u = threadIdx.x; u < units; u += kComputeThreads) {
-            const int r = r0 + u / (heads * hv);
-            const int rem = u % (heads * hv);
-            const int col = c0 + (rem / hv) * D + (rem % hv) * 8;
-            const int tok = r % group, dc = (rem % hv) * 8;
-            float x1[8], x2[8], c1[8], c2[8], s1[8], s2[8], o1[8], o2[8];
-            load8(A, (long long)r * op->ld[0] + col, adt, x1);
-            load8(A, (long long)r * op->ld[0] + col + half, adt, x2);
-            load8(B, (long long)tok * op->ld[1] + dc, bdt, c1);
-            load8(B, (long long)tok * op->ld[1] + dc + half, bdt, c2);
-            load8(Cp, (long long)tok * op->ld[2] + dc, cdt, s1);
-            load8(Cp, (long long)tok * op->ld[2] + dc + half, cdt, s2);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                o1[e] = x1[e] * c1[e] - x2[e] * s1[e];
-                o2[e] = x2[e] * c2[e] + x1[e] * s2[e];
-            }
-            store8(O, (long long)r * op->ld[3] + col, odt, o1);
-            store8(O, (long long)r * op->ld[3] + col + half, odt, o2);
-        }
-        return;
-    }
-    if (mode == EW_GATED) { eltwise_tile_gated(op, r0, c0, rows, cols); return; }
-    const bool all16 = adt != DT_F32 && (mode == EW_UNARY || bdt != DT_F32) && (mode != EW_MODULATE || cdt != DT_F32);
-    if (all16) {
-        switch (mode) {
-            case EW_UNARY: eltwise_tile<EW_UNARY, true>(op, r0, c0, rows, cols); break;
-            case EW_BINARY: eltwise_tile<EW_BINARY, true>(op, r0, c0, rows, cols); break;
-            case EW_SWIGLU: eltwise_tile<EW_SWIGLU, true>(op, r0, c0, rows, cols); break;
-            default: eltwise_tile<EW_MODULATE, true>(op, r0, c0, rows, cols); break;
-        }
-        return;
-    }
-    switch (mode) {
-        case EW_UNARY: eltwise_tile<EW_UNARY, false>(op, r0, c0, rows, cols); break;
-        case EW_BINARY: eltwise_tile<EW_BINARY, false>(op, r0, c0, rows, cols); break;
-        case EW_SWIGLU: eltwise_tile<EW_SWIGLU, false>(op, r0, c0, rows, cols); break;
-        default: eltwise_tile<EW_MODULATE, false>(op, r0, c0, rows, cols); break;
-    }
-}
-
 // (Each instance is a function of its own: inlined into one body, the longer variants' registers and spills fell on
 // the one-vector-per-thread case too, which is the norm of every decode step.)
 // A row (or a lane's share of it) of at most NPER vectors per thread stays in registers between the two passes: every
@@ -313,7 +48,7 @@ static __device__ __noinline__ void op_eltwise(const mk_op_desc* op, int a0, int
 // the vectors of a 2048-column row cost eight L2 round trips in each pass: 11 us per 8-row instruction.)
 template <int NPER, bool MOD, bool X16 = false>
 static __device__ __noinline__ void norm_kept(const mk_op_desc* op, int r, int first, int step, int nvec, bool live, uint8_t* work) {
-    const int Cc = op->i[1], rms = op->i[2], rpi = op->i[3], xdt = op->i[4], odt = op->i[5];
+    const int Cc = op->i[1], rms = op->i[2], xdt = op->i[4], odt = op->i[5];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const void* X = reinterpret_cast<const void*>(op->ptr[0]);
     void* O = reinterpret_cast<void*>(op->ptr[1]);
@@ -359,14 +94,12 @@ static __device__ __noinline__ void norm_kept(const mk_op_desc* op, int r, int f
     }
     s = warp_sum(s);
     ss = warp_sum(ss);
-    if (rpi == 1) {
-        float* sh = reinterpret_cast<float*>(work);
-        if (lane == 0) { sh[warp * 2] = s; sh[warp * 2 + 1] = ss; }
-        compute_sync();
-        s = 0.f; ss = 0.f;
+    float* sh = reinterpret_cast<float*>(work);
+    if (lane == 0) { sh[warp * 2] = s; sh[warp * 2 + 1] = ss; }
+    compute_sync();
+    s = 0.f; ss = 0.f;
 #pragma unroll
-        for (int w8 = 0; w8 < kComputeWarps; ++w8) { s += sh[w8 * 2]; ss += sh[w8 * 2 + 1]; }
-    }
+    for (int w8 = 0; w8 < kComputeWarps; ++w8) { s += sh[w8 * 2]; ss += sh[w8 * 2 + 1]; }
     if (!live) return;
     const float mean = rms ? 0.f : s / (float)Cc;
     const float var = ss / (float)Cc - mean * mean;
@@ -404,13 +137,13 @@ static __device__ __noinline__ void norm_kept(const mk_op_desc* op, int r, int f
     }
 }
 
-// MK_OP_NORM.  ptr 0 x, 1 out, 2 weight, 3 bias, 4 scale, 5 shift (adaLN modulation of the normalised row fused in:
-// out = norm(x) * (1 + scale[r / group]) + shift[r / group]; or null); i 0 R, 1 C, 2 rms, 3 rows per instruction (8: one
-// row per warp, 1: one row over the whole CTA), 4 x dtype, 5 out dtype, 6 group, 7 scale dtype, 8 shift dtype; f 0 eps.
+// MK_OP_NORM with one row per instruction, spread over the whole CTA (i 3 = 1: ops of few rows; more rows per instruction:
+// op_stream.cuh).  ptr 0 x, 1 out, 2 weight, 3 bias, 4 scale, 5 shift (adaLN modulation of the normalised row fused in:
+// out = norm(x) * (1 + scale[r / group]) + shift[r / group]; or null); i 0 R, 1 C, 2 rms, 3 rows per instruction, 4 x dtype, 5 out dtype, 6 group, 7 scale dtype, 8 shift dtype; f 0 eps.
 // args: 0 row tile.
 // var = E[x^2] - mean^2 in fp32 (as the reference's norm kernel, megacute/ops/norm.py:94-114).
 static __device__ __noinline__ void op_norm(const mk_op_desc* op, int a0, uint8_t* work) {
-    const int R = op->i[0], Cc = op->i[1], rms = op->i[2], rpi = op->i[3], xdt = op->i[4], odt = op->i[5];
+    const int R = op->i[0], Cc = op->i[1], rms = op->i[2], xdt = op->i[4], odt = op->i[5];
     const float eps = op->f[0];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const void* X = reinterpret_cast<const void*>(op->ptr[0]);
@@ -418,9 +151,7 @@ static __device__ __noinline__ void op_norm(const mk_op_desc* op, int a0, uint8_
     const void* W = reinterpret_cast<const void*>(op->ptr[2]);
     const void* Bv = reinterpret_cast<const void*>(op->ptr[3]);
     const int nvec = Cc >> 3;
-    int r, first, step;
-    if (rpi == 1) { r = a0; first = threadIdx.x; step = kComputeThreads; }
-    else { r = a0 * kComputeWarps + warp; first = lane; step = 32; }
+    const int r = a0, first = threadIdx.x, step = kComputeThreads;
     const bool live = r < R;
     const int nper = (nvec + step - 1) / step;          // vectors per thread
     if (op->ptr[4] && nper <= 4) { norm_kept<4, true>(op, r, first, step, nvec, live, work); return; }
@@ -438,14 +169,12 @@ static __device__ __noinline__ void op_norm(const mk_op_desc* op, int a0, uint8_
         }
         s = warp_sum(s);
         ss = warp_sum(ss);
-        if (rpi == 1) {
-            float* sh = reinterpret_cast<float*>(work);
-            if (lane == 0) { sh[warp * 2] = s; sh[warp * 2 + 1] = ss; }
-            compute_sync();
-            s = 0.f; ss = 0.f;
+        float* sh = reinterpret_cast<float*>(work);
+        if (lane == 0) { sh[warp * 2] = s; sh[warp * 2 + 1] = ss; }
+        compute_sync();
+        s = 0.f; ss = 0.f;
 #pragma unroll
-            for (int w8 = 0; w8 < kComputeWarps; ++w8) { s += sh[w8 * 2]; ss += sh[w8 * 2 + 1]; }
-        }
+        for (int w8 = 0; w8 < kComputeWarps; ++w8) { s += sh[w8 * 2]; ss += sh[w8 * 2 + 1]; }
         if (!live || first >= nvec) return;
         const float mean = rms ? 0.f : s / (float)Cc;
         const float rstd = rsqrt_approx(ss / (float)Cc - mean * mean + eps);
@@ -481,14 +210,12 @@ static __device__ __noinline__ void op_norm(const mk_op_desc* op, int a0, uint8_
         }
     s = warp_sum(s);
     ss = warp_sum(ss);
-    if (rpi == 1) {
-        float* sh = reinterpret_cast<float*>(work);
-        if (lane == 0) { sh[warp * 2] = s; sh[warp * 2 + 1] = ss; }
-        compute_sync();
-        s = 0.f; ss = 0.f;
+    float* sh = reinterpret_cast<float*>(work);
+    if (lane == 0) { sh[warp * 2] = s; sh[warp * 2 + 1] = ss; }
+    compute_sync();
+    s = 0.f; ss = 0.f;
 #pragma unroll
-        for (int w8 = 0; w8 < kComputeWarps; ++w8) { s += sh[w8 * 2]; ss += sh[w8 * 2 + 1]; }
-    }
+    for (int w8 = 0; w8 < kComputeWarps; ++w8) { s += sh[w8 * 2]; ss += sh[w8 * 2 + 1]; }
     if (!live) return;
     const float mean = rms ? 0.f : s / (float)Cc;
     const float var = ss / (float)Cc - mean * mean;

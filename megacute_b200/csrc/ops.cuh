@@ -41,7 +41,10 @@ __device__ bool mk_op_decode_attn(const Params& p, const mk_op_desc* op, int a0,
 // (many-sequence form: all kv heads of a sequence per instruction, whole cache rows through bulk copies)
 __device__ bool mk_op_decode_bulk(const Params& p, const mk_op_desc* op, int b, int s, int nwait, int wait_off, int seq,
                                   int narrive, int arrive_off);
-// finalize / eltwise / norm / rope_append / increment / gather / argmax; returns false for an unknown kind
+// pointwise tiles and norms with several rows per instruction (op_stream.cuh): like mk_run_gemm, for runs of their own kind
+__device__ int mk_run_eltwise(const Params& p, const mk_op_desc* op, int idx);
+__device__ int mk_run_norm(const Params& p, const mk_op_desc* op, int idx);
+// finalize / norm of one row / rope_append / increment / gather / argmax; returns false for an unknown kind
 __device__ bool mk_op_pointwise(const mk_op_desc* op, int a0, int a1);
 
 struct SmemMap {

@@ -14,7 +14,7 @@ view's first element.  Field meaning per kind (the kernel side repeats it next t
                accumulate, residual dtype, swiglu, x dtype (bf16 or fp16), weight rows per tile (128 / 256), activation rows per tile (128 / 256)  (ptr 10, 11: set by the C
                library when it binds the op to its tcgen05 body: packed weight tiles, tensor maps)
   FINALIZE     ptr ws, out, bias, residual; i R, C, act, out dtype, residual dtype, rows per instruction
-  ELTWISE      ptr a, b, c, out; i R, C, mode, fn, group, head_dim, dtypes of a, b, c, out
+  ELTWISE      ptr a, b, c, out; i R, C, mode, fn, group, head_dim, dtypes of a, b, c, out, rows per instruction
                (mode EW_GATED: out = fn(a, b * c[r // group]), a gated residual)
   NORM         ptr x, out, weight, bias, scale, shift (adaLN modulation fused in, or none); i R, C, rms, rows per
                instruction, x dtype, out dtype, rows per scale / shift row, their dtypes; f eps
@@ -37,7 +37,7 @@ import torch
 
 from . import config as C
 from .graph import DTYPE_CODE, ELEM_BYTES, Op, View
-from .schedule import argmax_chunk_cols, finalize_rows, gemm_rows, is_gemv, norm_rows
+from .schedule import argmax_chunk_cols, ew_rows, finalize_rows, gemm_rows, is_gemv, norm_rows
 
 BF16 = torch.bfloat16
 F16 = torch.float16
@@ -131,7 +131,7 @@ def fill(d, op: Op, addr) -> None:
             ptrs, ints = [op.x, op.scale, op.shift, op.out], [R, Cc, C.EW_MODULATE, 0, op.group, 0]
         else:
             ptrs, ints = [op.x, op.cos, op.sin, op.out], [R, Cc, C.EW_ROPE, 0, op.seq, op.head_dim]
-        ints += [dt(v) for v in ptrs]
+        ints += [dt(v) for v in ptrs] + [ew_rows(R, Cc)]
     elif k == "Norm":
         d.kind = C.OP_NORM
         ptrs = [op.x, op.out, op.weight, op.bias, op.scale, op.shift]

@@ -155,6 +155,8 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
         TR, TC = C.EW_ROWS, C.EW_COLS
         if k == "SplitFinalize":
             TR = finalize_rows(R, Cc)
+        else:
+            TR = ew_rows(R, Cc)
         if k == "Rope":
             assert TC % op.head_dim == 0, "rope: head_dim must divide the pointwise tile width"
         rt, ct = np.divmod(np.arange(_ceil(R, TR) * _ceil(Cc, TC)), _ceil(Cc, TC))
@@ -284,9 +286,20 @@ def finalize_rows(rows: int, cols: int) -> int:
 
 
 def norm_rows(rows: int) -> int:
-    """Rows per norm instruction: one per compute warp, or a single row spread over the whole CTA
-    when the op has few rows (decode)."""
-    return 1 if rows <= C.WIDE_NORM_ROWS else C.NORM_ROWS
+    """Rows per norm instruction: a single row spread over the whole CTA when the op has few rows (decode),
+    else a multiple of the compute warps that gives each SM about one instruction."""
+    if rows <= C.WIDE_NORM_ROWS:
+        return 1
+    return C.NORM_ROWS * max(1, min(C.NORM_MAX_ROWS // C.NORM_ROWS, _ceil(_ceil(rows, C.NORM_ROWS), C.STREAM_INSTS)))
+
+
+def ew_rows(rows: int, cols: int) -> int:
+    """Rows per pointwise instruction: the smallest power of two that leaves the op about one instruction
+    per SM, within EW_MIN_ROWS .. EW_MAX_ROWS."""
+    tr, ct = C.EW_MIN_ROWS, _ceil(cols, C.EW_COLS)
+    while tr < C.EW_MAX_ROWS and _ceil(rows, tr) * ct > C.STREAM_INSTS:
+        tr *= 2
+    return tr
 
 
 # --------------------------------------------------------------------------------------------

@@ -30,7 +30,7 @@ import torch
 
 from . import config as C
 from .graph import Graph
-from .schedule import CONFLICTS, Schedule, finalize_rows, gemm_rows, is_gemv, norm_rows, tile_op
+from .schedule import CONFLICTS, Schedule, ew_rows, finalize_rows, gemm_rows, is_gemv, norm_rows, tile_op
 
 
 class VerifyError(AssertionError):
@@ -130,7 +130,7 @@ def op_grid(op, sm_count: int):
     if k == "SplitFinalize":
         return (_ceil(op.out.rows, finalize_rows(*op.out.shape)), _ceil(op.out.cols, C.EW_COLS))
     if k in ("Unary", "Binary", "SwiGLU", "Modulate", "Rope"):
-        return (_ceil(op.out.rows, C.EW_ROWS), _ceil(op.out.cols, C.EW_COLS))
+        return (_ceil(op.out.rows, ew_rows(*op.out.shape)), _ceil(op.out.cols, C.EW_COLS))
     if k == "Norm":
         return (_ceil(op.x.rows, norm_rows(op.x.rows)),)
     if k == "Attention":
