@@ -400,6 +400,7 @@ static bool tile_gemm_on_tcgen05(const mk_op_desc& d) {
     if (!vec_ok(d.ptr[2], d.ld[2], odt)) return false;
     if (d.ptr[3] && (d.ptr[3] & 15)) return false;
     if (d.ptr[4] && !vec_ok(d.ptr[4], d.ld[4], rdt)) return false;
+    if (d.ptr[5] && (!vec_ok(d.ptr[5], d.ld[5], d.i[13]) || d.i[11] != 256 || d.i[12] <= 0)) return false;
     return true;
 }
 
@@ -430,6 +431,7 @@ static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
                     else if (d.i[10] != 0 && d.i[10] != 128 && !(d.i[10] == 256 && d.i[11] == 256 && d.i[1] % 256 == 0)) why = "tile GEMM: weight rows per tile";
                     else if (a1 < 0 || a1 * (long long)(d.i[10] == 256 ? 256 : 128) >= d.i[1]) why = "tile GEMM: n tile outside N";
                     else if (a2 < 0 || a2 >= d.i[4]) why = "tile GEMM: K split index";
+                    else if (d.ptr[5] && d.i[12] <= 0) why = "tile GEMM: rows per gate row";
                     break;
                 case MK_OP_FINALIZE:
                     if (d.i[5] <= 0 || a0 < 0 || a0 >= ceil_div(d.i[0], d.i[5]) || a1 < 0 || a1 * 512 >= d.i[1]) why = "finalize: tile outside the output";

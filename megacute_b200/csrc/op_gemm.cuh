@@ -11,11 +11,11 @@
 // by streaming the weights), 64 rows per tile (warp tile 32 x 32): no MMAs on padding rows and more
 // weight bytes in flight.
 //
-// ptr 0 x, 1 w, 2 out (or ws), 3 bias, 4 residual
+// ptr 0 x, 1 w, 2 out (or ws), 3 bias, 4 residual, 5 gate (out = residual + act(.) * gate[r / i12], 256-row tiles only; or null)
 // i 0 M, 1 N (weight rows), 2 K, 3 act, 4 splits, 5 out dtype, 6 accumulate, 7 residual dtype,
 //   8 swiglu (weight tile = 64 gate rows then 64 up rows; the tile writes 64 output columns),
 //   9 x dtype (DT_BF16 or DT_F16), 10 weight rows per output tile (128, or 256: the n tile argument then
-//   names a pair of 128-row tiles)
+//   names a pair of 128-row tiles), 11 activation rows per output tile (128 or 256), 12 rows per gate row, 13 gate dtype
 // args: 0 m tile, 1 n tile, 2 k split
 #pragma once
 #include "mk_device.cuh"
@@ -145,6 +145,12 @@ static __device__ __noinline__ void op_gemm(const mk_op_desc* op, int a0, int a1
                     }
                     v0 = apply_act(act, v0);
                     v1 = apply_act(act, v1);
+                    if (op->ptr[5]) {                          // gated residual: gate row r / i12
+                        const void* G = reinterpret_cast<const void*>(op->ptr[5]);
+                        const long long eg = (long long)(r / op->i[12]) * op->ld[5] + col;
+                        v0 *= load1(G, eg, op->i[13]);
+                        v1 *= load1(G, eg + 1, op->i[13]);
+                    }
                     if (op->ptr[4]) {
                         const void* R = reinterpret_cast<const void*>(op->ptr[4]);
                         v0 += load1(R, (long long)r * op->ld[4] + col, rdt);

@@ -213,131 +213,183 @@ __device__ __forceinline__ void wide_bias(const uint8_t* bias, int col, float* v
     }
 }
 
-// 16-bit outputs, no residual: 128 columns of the accumulator at a time; the last of them stay packed in registers until the
-// accumulator has been handed back.  ACT: 0 none, 1 gelu, 2 any (run time).
+// an activation chosen at run time on 32 values: the switch outside the loop
+__device__ __forceinline__ void act_all(int act, float* v) {
+    if (act == ACT_RELU) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = fmaxf(v[j], 0.0f);
+    } else if (act == ACT_SILU) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) v[j] = v[j] * sigmoidf_(v[j]);
+    } else {
+#pragma unroll 1
+        for (int j = 0; j < 32; j += 8) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = apply_act(act, v[e]);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {                     // (rotate: register indices stay constant)
+                const float t = v[e];
+                v[e] = v[8 + e]; v[8 + e] = v[16 + e]; v[16 + e] = v[24 + e]; v[24 + e] = t;
+            }
+        }
+    }
+}
+
+// 16-bit outputs, no residual: 32 output columns at a time into the staging rows, 64 at a time from there.  A loop, not 256 columns
+// of straight-line code that keeps them packed in registers to hand the accumulator back early: fetching that code took longer
+// than executing this (gelu tile: 13 us from the accumulator to the arrival, 4.4 of them instruction issue).
+// ACT: 0 none, 1 gelu, 2 any (run time).
 template <bool F16, bool SWI, int ACT>
 __device__ __forceinline__ void wide_store16(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
-    constexpr int kChunks = SWI ? 1 : 2;                     // of 64 output columns per 128 of the accumulator
     const int lane = threadIdx.x & 31;
-    const int act = op->i[3], units = op->i[10] >> 7;
+    const int act = op->i[3], groups = (op->i[10] >> 5) >> (SWI ? 1 : 0);
     const int rows = op->i[0] - row0;
     const long long ldo = (long long)op->ld[2] * 2;
     const int r = lane >> 3, cc = lane & 7;
     uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + (long long)(row0 + r) * ldo + (SWI ? n0 / 2 : n0) * 2 + cc * 16;
     if (!wide_wait(p, c, a)) return;
 #pragma unroll 1
-    for (int u = 0; u < units; ++u) {
-        uint32_t pk[kChunks * 32];
-#pragma unroll
-        for (int hf = 0; hf < 2 * kChunks; ++hf) {
-            const uint32_t tacc = a.tacc + u * 128 + hf * 32;
-            float v[32];
+    for (int g = 0; g < groups; ++g) {
+        float v[32];
+        if (SWI) {                                           // gate columns 128 (g / 2) + 32 (g % 2) .. +31, up columns 64 further
+            float u[32];
+            const uint32_t tacc = a.tacc + (g >> 1) * 128 + (g & 1) * 32;
             tc_ld32(tacc, v);
-            if (SWI) {                                       // gate columns 32 hf .. +31, up columns 64 further
-                float g[32];
-                tc_ld32(tacc + 64, g);
+            tc_ld32(tacc + 64, u);
+            if (g == groups - 1) wide_release(a.release);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = v[j] * sigmoidf_(v[j]) * g[j];
-            } else if (a.bias) {
-                wide_bias(a.bias, u * 128 + hf * 32, v);
+            for (int j = 0; j < 32; ++j) v[j] = v[j] * sigmoidf_(v[j]) * u[j];
+        } else {
+            tc_ld32(a.tacc + g * 32, v);
+            if (g == groups - 1) wide_release(a.release);
+            if (a.bias) wide_bias(a.bias, g * 32, v);
+            if (ACT == 1) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j) v[j] = apply_act(ACT_GELU, v[j]);
             }
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                float y0 = v[2 * j], y1 = v[2 * j + 1];
-                if (ACT == 1) { y0 = apply_act(ACT_GELU, y0); y1 = apply_act(ACT_GELU, y1); }
-                if (ACT == 2) { y0 = apply_act(act, y0); y1 = apply_act(act, y1); }
-                pk[hf * 16 + j] = F16 ? pack2h(y0, y1) : pack2(y0, y1);
-            }
+            if (ACT == 2) act_all(act, v);
         }
-        if (u == units - 1) wide_release(a.release);
 #pragma unroll
-        for (int ch = 0; ch < kChunks; ++ch) {
-            const uint32_t* q = pk + ch * 32;
-#pragma unroll
-            for (int j = 0; j < 8; ++j) *wide_chunk(a.stg, lane, j) = make_uint4(q[4 * j], q[4 * j + 1], q[4 * j + 2], q[4 * j + 3]);
-            __syncwarp();
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-                if (j * 4 + r < rows) *reinterpret_cast<uint4*>(O + (long long)(j * 4) * ldo + (u * kChunks + ch) * 128) = *wide_chunk(a.stg, j * 4 + r, cc);
-            __syncwarp();
+        for (int j = 0; j < 4; ++j) {
+            const float* f = v + 8 * j;
+            *wide_chunk(a.stg, lane, (g & 1) * 4 + j) =
+                F16 ? make_uint4(pack2h(f[0], f[1]), pack2h(f[2], f[3]), pack2h(f[4], f[5]), pack2h(f[6], f[7])) : pack8(f);
         }
+        if (!(g & 1)) continue;
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+            if (j * 4 + r < rows) *reinterpret_cast<uint4*>(O + (long long)(j * 4) * ldo + (g >> 1) * 128) = *wide_chunk(a.stg, j * 4 + r, cc);
+        __syncwarp();
     }
 }
 
 // Everything else -- residual, fp32 output, split-K partial (reduce-add): 32 columns at a time through shared memory as fp32.
-// RK: 0 no residual, 1 16-bit, 2 fp32; the residual of the next 32 columns is requested before this one's are used.
-template <int RK>
+// RK: 0 no residual, 1 16-bit, 2 fp32.  Residual (and gate) are requested DEPTH such steps ahead, the first ones while the main
+// loop still runs: a step takes 0.4 us, an L2 round trip beside the operand stream 1.5 (one step ahead: 20 us per tile).
+// The queue moves through registers one step per iteration, which costs less than unrolled code.
+// GATE: the result is multiplied by a gate row per i 12 rows (an adaLN-Zero block's gated residual) before the residual is added.
+__device__ __forceinline__ void wide_quad(int dtype, const uint4& w, float* f) {              // four values, raw bits of `dtype`
+    if (dtype == DT_F32) {
+        f[0] = __uint_as_float(w.x); f[1] = __uint_as_float(w.y); f[2] = __uint_as_float(w.z); f[3] = __uint_as_float(w.w);
+    } else if (dtype == DT_F16) {
+        const float2 lo = unpack2h(w.x), hi = unpack2h(w.y);
+        f[0] = lo.x; f[1] = lo.y; f[2] = hi.x; f[3] = hi.y;
+    } else {
+        f[0] = bf16_lo(w.x); f[1] = bf16_hi(w.x); f[2] = bf16_lo(w.y); f[3] = bf16_hi(w.y);
+    }
+}
+__device__ __forceinline__ uint4 wide_quad_load(int dtype, const uint8_t* base, long long elem) {
+    if (dtype == DT_F32) return __ldcg(reinterpret_cast<const uint4*>(base + elem * 4));
+    const uint2 w = __ldcg(reinterpret_cast<const uint2*>(base + elem * 2));
+    return make_uint4(w.x, w.y, 0u, 0u);
+}
+template <int RK, bool GATE>
 __device__ __forceinline__ void wide_store_any(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
+    constexpr int kDepth = RK == 0 ? 1 : RK == 1 ? 4 : 2;
     const int lane = threadIdx.x & 31;
     const int act = op->i[3], odt = op->i[5], rdt = op->i[7];
     const bool accum = op->i[6] != 0, swi = op->i[8] != 0;
     const int groups = (op->i[10] >> 5) >> (swi ? 1 : 0);
-    const int rows = op->i[0] - row0;
+    const int rows = min(32, op->i[0] - row0);
     const int r = lane >> 3, c4 = (lane & 7) * 4, osz = odt == DT_F32 ? 4 : 2;
-    const long long ldo = (long long)op->ld[2] * osz, ldr = (long long)op->ld[4] * (RK == 2 ? 4 : 2);
-    const int col0 = swi ? n0 / 2 : n0;
-    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + (long long)(row0 + r) * ldo + (col0 + c4) * osz;
-    const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]) + (long long)(row0 + r) * ldr + (col0 + c4) * (RK == 2 ? 4 : 2);
-    uint4 res[RK ? 8 : 1];
-    auto request = [&](int g) {
+    const long long ldo = (long long)op->ld[2] * osz, ldr = op->ld[4];
+    const int col0 = (swi ? n0 / 2 : n0) + c4;
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + (long long)(row0 + r) * ldo + col0 * osz;
+    const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]);
+    const uint8_t* G = reinterpret_cast<const uint8_t*>(op->ptr[5]);
+    // (16-bit residuals: two registers per row; rows beyond the tensor read its last row)
+    uint4 q32[RK == 2 ? kDepth : 1][RK == 2 ? 8 : 1], qg[GATE ? kDepth : 1];
+    uint2 q16[RK == 1 ? kDepth : 1][RK == 1 ? 8 : 1];
+    const int group = GATE ? op->i[12] : 1, gdt = op->i[13];
+    const bool one = GATE && row0 / group == (row0 + rows - 1) / group;                // the warp's rows share a gate row
+    auto request = [&](int d, int g) {
+        g = min(g, groups - 1);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            res[RK ? j : 0] = make_uint4(0u, 0u, 0u, 0u);
-            if (j * 4 + r < rows) {
-                const uint8_t* at = R + (long long)(j * 4) * ldr + g * 32 * (RK == 2 ? 4 : 2);
-                if (RK == 2) res[RK ? j : 0] = __ldcg(reinterpret_cast<const uint4*>(at));
-                else { const uint2 w = __ldcg(reinterpret_cast<const uint2*>(at)); res[RK ? j : 0].x = w.x; res[RK ? j : 0].y = w.y; }
-            }
+            const long long e = (long long)(row0 + min(j * 4 + r, rows - 1)) * ldr + col0 + g * 32;
+            if (RK == 1) q16[RK == 1 ? d : 0][RK == 1 ? j : 0] = __ldcg(reinterpret_cast<const uint2*>(R + e * 2));
+            if (RK == 2) q32[RK == 2 ? d : 0][RK == 2 ? j : 0] = __ldcg(reinterpret_cast<const uint4*>(R + e * 4));
         }
+        if (GATE && one) qg[GATE ? d : 0] = wide_quad_load(gdt, G, (long long)(row0 / group) * op->ld[5] + col0 + g * 32);
     };
-    if (RK) request(0);
+    if (RK) {
+#pragma unroll
+        for (int d = 0; d < kDepth; ++d) request(d, d);
+    }
     if (!wide_wait(p, c, a)) return;
-    const uint32_t tacc = a.tacc;
 #pragma unroll 1
     for (int g = 0; g < groups; ++g) {
         float v[32];
         if (swi) {
             float u[32];
-            tc_ld32(tacc + (g >> 1) * 128 + (g & 1) * 32, v);
-            tc_ld32(tacc + (g >> 1) * 128 + 64 + (g & 1) * 32, u);
+            tc_ld32(a.tacc + (g >> 1) * 128 + (g & 1) * 32, v);
+            tc_ld32(a.tacc + (g >> 1) * 128 + 64 + (g & 1) * 32, u);
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = v[j] * sigmoidf_(v[j]) * u[j];
         } else {
-            tc_ld32(tacc + g * 32, v);
+            tc_ld32(a.tacc + g * 32, v);
             if (a.bias) wide_bias(a.bias, g * 32, v);
-            if (act != ACT_NONE) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = apply_act(act, v[j]);
-            }
+            if (act != ACT_NONE) act_all(act, v);
         }
         if (g == groups - 1) wide_release(a.release);
 #pragma unroll
         for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(wide_chunk(a.stg, lane, j)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         __syncwarp();
-        float4 o[8];
+        float gt[4] = {1.f, 1.f, 1.f, 1.f};
+        if (GATE && one) wide_quad(gdt, qg[0], gt);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-            o[j] = *reinterpret_cast<const float4*>(wide_chunk(a.stg, j * 4 + r, lane & 7));
-            if (RK == 1) {
-                float2 lo, hi;
-                if (rdt == DT_F16) { lo = unpack2h(res[RK ? j : 0].x); hi = unpack2h(res[RK ? j : 0].y); }
-                else { lo = make_float2(bf16_lo(res[RK ? j : 0].x), bf16_hi(res[RK ? j : 0].x)); hi = make_float2(bf16_lo(res[RK ? j : 0].y), bf16_hi(res[RK ? j : 0].y)); }
-                o[j].x += lo.x; o[j].y += lo.y; o[j].z += hi.x; o[j].w += hi.y;
-            } else if (RK == 2) {
-                o[j].x += __uint_as_float(res[RK ? j : 0].x); o[j].y += __uint_as_float(res[RK ? j : 0].y);
-                o[j].z += __uint_as_float(res[RK ? j : 0].z); o[j].w += __uint_as_float(res[RK ? j : 0].w);
+            float4 o = *reinterpret_cast<const float4*>(wide_chunk(a.stg, j * 4 + r, lane & 7));
+            if (GATE) {
+                if (!one) wide_quad(gdt, wide_quad_load(gdt, G, (long long)((row0 + min(j * 4 + r, rows - 1)) / group) * op->ld[5] + col0 + g * 32), gt);
+                o.x *= gt[0]; o.y *= gt[1]; o.z *= gt[2]; o.w *= gt[3];
             }
-        }
-        if (RK && g + 1 < groups) request(g + 1);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            if (j * 4 + r >= rows) break;
+            if (RK) {
+                float f[4];
+                if (RK == 1) wide_quad(rdt, make_uint4(q16[0][RK == 1 ? j : 0].x, q16[0][RK == 1 ? j : 0].y, 0u, 0u), f);
+                else wide_quad(DT_F32, q32[0][RK == 2 ? j : 0], f);
+                o.x += f[0]; o.y += f[1]; o.z += f[2]; o.w += f[3];
+            }
+            if (j * 4 + r >= rows) continue;
             uint8_t* at = O + (long long)(j * 4) * ldo + g * 32 * osz;
             if (accum) {
-                if (odt == DT_F32) red_add_f32x4(reinterpret_cast<float*>(at), o[j].x, o[j].y, o[j].z, o[j].w);
-                else red_add_bf16x4(at, &o[j].x);
-            } else if (odt == DT_F32) *reinterpret_cast<float4*>(at) = o[j];
-            else *reinterpret_cast<uint2*>(at) = make_uint2(pack2t(odt, o[j].x, o[j].y), pack2t(odt, o[j].z, o[j].w));
+                if (odt == DT_F32) red_add_f32x4(reinterpret_cast<float*>(at), o.x, o.y, o.z, o.w);
+                else red_add_bf16x4(at, &o.x);
+            } else if (odt == DT_F32) *reinterpret_cast<float4*>(at) = o;
+            else *reinterpret_cast<uint2*>(at) = make_uint2(pack2t(odt, o.x, o.y), pack2t(odt, o.z, o.w));
+        }
+        if (RK) {
+#pragma unroll
+            for (int d = 0; d + 1 < kDepth; ++d) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (RK == 1) q16[RK == 1 ? d : 0][RK == 1 ? j : 0] = q16[RK == 1 ? d + 1 : 0][RK == 1 ? j : 0];
+                    if (RK == 2) q32[RK == 2 ? d : 0][RK == 2 ? j : 0] = q32[RK == 2 ? d + 1 : 0][RK == 2 ? j : 0];
+                }
+                if (GATE) qg[GATE ? d : 0] = qg[GATE ? d + 1 : 0];
+            }
+            request(kDepth - 1, g + kDepth);
         }
         __syncwarp();
     }
@@ -346,10 +398,11 @@ __device__ __forceinline__ void wide_store_any(const Params& p, Ctrl* c, const m
 // The epilogue of an op, chosen once per run of instructions: each has a function of its own around it (op_gemm_wide.cu) and so a
 // register allocation of its own -- called per instruction they pay ~60 saved and restored registers each time, inlined
 // side by side they spill, and with the shared memory taken every such access is an L2 round trip behind the operand stream.
-enum { WIDE_PLAIN = 0, WIDE_SWIGLU, WIDE_GELU, WIDE_ACT, WIDE_ANY0, WIDE_ANY1, WIDE_ANY2 };      // (+ 16: fp16 output, the first four)
+enum { WIDE_PLAIN = 0, WIDE_SWIGLU, WIDE_GELU, WIDE_ACT, WIDE_ANY0, WIDE_ANY1, WIDE_ANY2, WIDE_GATE1, WIDE_GATE2 };      // (+ 16: fp16 output, the first four)
 __device__ __forceinline__ int wide_variant(const mk_op_desc* op) {
     const int odt = op->i[5];
     if (op->i[6]) return WIDE_ANY0;
+    if (op->ptr[5]) return op->i[7] == DT_F32 ? WIDE_GATE2 : WIDE_GATE1;
     if (op->ptr[4]) return op->i[7] == DT_F32 ? WIDE_ANY2 : WIDE_ANY1;
     if (odt == DT_F32) return WIDE_ANY0;
     const int v = op->i[8] ? WIDE_SWIGLU : op->i[3] == ACT_NONE ? WIDE_PLAIN : op->i[3] == ACT_GELU ? WIDE_GELU : WIDE_ACT;
@@ -402,7 +455,8 @@ __device__ __forceinline__ void op_gemm_tc_wide(const Params& p, Ctrl* c, uint8_
     else if constexpr (kind == WIDE_SWIGLU) wide_store16<f16, true, 0>(p, c, op, a, row0, n0);
     else if constexpr (kind == WIDE_GELU) wide_store16<f16, false, 1>(p, c, op, a, row0, n0);
     else if constexpr (kind == WIDE_ACT) wide_store16<f16, false, 2>(p, c, op, a, row0, n0);
-    else wide_store_any<kind - WIDE_ANY0>(p, c, op, a, row0, n0);
+    else if constexpr (kind >= WIDE_GATE1) wide_store_any<kind - WIDE_GATE1 + 1, true>(p, c, op, a, row0, n0);
+    else wide_store_any<kind - WIDE_ANY0, false>(p, c, op, a, row0, n0);
 }
 
 }  // namespace mk

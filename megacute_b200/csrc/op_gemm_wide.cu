@@ -38,6 +38,8 @@ __device__ int mk_run_gemm_wide(const Params& p, int idx) {
             case WIDE_ACT + 16: last = wide_run<WIDE_ACT + 16>(p, idx); break;
             case WIDE_ANY1: last = wide_run<WIDE_ANY1>(p, idx); break;
             case WIDE_ANY2: last = wide_run<WIDE_ANY2>(p, idx); break;
+            case WIDE_GATE1: last = wide_run<WIDE_GATE1>(p, idx); break;
+            case WIDE_GATE2: last = wide_run<WIDE_GATE2>(p, idx); break;
             default: last = wide_run<WIDE_ANY0>(p, idx); break;
         }
         if (last < 0) return -1;

@@ -108,7 +108,7 @@ class View:
 # An operand listed in both columns is updated in place by the op.  Optional operands may be
 # None.  The semantic definition of each kind is in the builder method's docstring below.
 OP_TABLE = {
-    "Linear":          (("x", "w", "bias", "residual", "norm_w"), ("out",), ("act", "rms_eps", "bm", "bn")),
+    "Linear":          (("x", "w", "bias", "residual", "norm_w", "gate"), ("out",), ("act", "rms_eps", "bm", "bn", "gate_group")),
     "LinearSplit":     (("x", "w", "norm_w"), ("ws",), ("splits", "rms_eps", "bm", "bn")),
     "SplitFinalize":   (("ws", "bias", "residual"), ("out", "ws"), ("act",)),
     "Unary":           (("x",), ("out",), ("fn",)),
@@ -206,6 +206,8 @@ def _chk_linear(o):
         assert o.residual.shape == (M, N)
     if o.norm_w is not None:
         assert o.norm_w.shape == (1, K) and o.rms_eps is not None
+    if o.gate is not None:          # set by passes.fuse_gated_linear only: out = residual + act(x @ w.T + bias) * gate[r // gate_group]
+        assert o.residual is not None and o.act != "swiglu" and o.gate.shape == (M // o.gate_group, N)
 
 
 def _chk_linear_split(o):

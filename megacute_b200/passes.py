@@ -293,7 +293,7 @@ def _accepts(op: Op, field: str, dtype) -> bool:
         streaming = gemv_eligible(op.x.rows, op.x.cols)
         if field == "x":                                # the tensor core takes 16-bit operands; the streaming linear converts
             return streaming or not f32
-        return field in ("out", "residual")
+        return field in ("out", "residual", "gate")
     if k == "LinearSplit":
         return (field == "ws" and f32) or (field == "x" and not f32)
     if k == "SplitFinalize":
@@ -481,8 +481,30 @@ def fuse_pointwise(g: Graph) -> Graph:
     return out
 
 
+def fuse_gated_linear(g: Graph) -> Graph:
+    """A tile linear with 256-row tiles followed by a gated residual (``x + y * gate[g]``, made by fuse_pointwise) does the
+    gating in its epilogue: a pass over three activation-sized tensors and a dependency hop less, and the product is not
+    rounded in between.  (Few-row linears keep the op: their epilogues have no room for a third operand's latency.)
+    MEGACUTE_B200_NO_POINTWISE_FUSION=1 keeps the ops apart."""
+    if os.environ.get("MEGACUTE_B200_NO_POINTWISE_FUSION") == "1":
+        return g
+    out = g.derive()
+    ops: list[Op] = []
+    for i, op in enumerate(g.ops):
+        prev = ops[-1] if ops else None
+        if (op.kind == "Binary" and op.gate is not None and op.fn == "add" and prev is not None and prev.kind == "Linear"
+                and prev.bm == C.GEMM_BM_WIDE and prev.act != "swiglu" and prev.residual is None and prev.gate is None
+                and op.b.same(prev.out) and prev.out.buf.kind == "temp" and not _reads_buffer(g.ops[i + 1:], prev.out.buf, g.outputs)
+                and all(v.buf is not prev.x.buf for v in op.writes)):
+            ops[-1] = prev.clone(out=op.out, residual=op.a, gate=op.gate, gate_group=op.gate_group)
+            continue
+        ops.append(op)
+    out.ops = ops
+    return out
+
+
 def run_all(g: Graph, sm_count: int) -> Graph:
     """The pass pipeline of ``compile`` (reference order: runtime.py:235, plus wide_tiles, split_argmax,
-    fuse_pointwise, promote_temps and fuse_finalize_attention)."""
+    fuse_pointwise, fuse_gated_linear, promote_temps and fuse_finalize_attention)."""
     g = split_argmax(split_kv(fuse_rope_attention(wide_tiles(split_k(fold_norms(g), sm_count), sm_count)), sm_count), sm_count)
-    return fuse_finalize_attention(promote_temps(fuse_pointwise(g)))
+    return fuse_finalize_attention(promote_temps(fuse_gated_linear(fuse_pointwise(g))))

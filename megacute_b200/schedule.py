@@ -148,6 +148,9 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
         if k == "Linear":
             acc += [_acc(op.bias, READ, 0, 1, nn * on, (nn + 1) * on, n=n),
                     _acc(op.residual, READ, r0, r1, nn * on, (nn + 1) * on, n=n)]
+            if op.gate is not None:
+                gg = op.gate_group
+                acc.append(_acc(op.gate, READ, r0 // gg, -(-np.minimum(r1, M) // gg), nn * on, (nn + 1) * on, n=n, covers=False))
             assert op.norm_w is None and op.rms_eps is None, "norm folding is only done on the streaming path"
         return Tiled(_args(n, m, nn, ks), [a for a in acc if a is not None])
     if k in ("SplitFinalize", "Unary", "Binary", "SwiGLU", "Modulate", "Rope"):

@@ -58,6 +58,8 @@ def operand_windows(op) -> dict:
         win = {"x": (M, K), "w": (w_rows, K), ("out" if k == "Linear" else "ws"): (M, n_out)}
         if k == "Linear":
             win.update(bias=(1, n_out), residual=(M, n_out), norm_w=(1, K))
+            if op.gate is not None:
+                win["gate"] = (_ceil(M, op.gate_group), n_out)
         return win
     if k == "SplitFinalize":
         R, Cc = op.out.shape
