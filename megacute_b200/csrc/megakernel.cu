@@ -160,9 +160,9 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                     break;
                 case MK_OP_GEMM:
                     // (runs this instruction and the CTA's following ones for as long as they are the body's own: walk.cuh)
-                    run_last = is_wide_gemm(op) ? mk_run_gemm_wide(p, idx) : mk_run_gemm(p, idx);
+                    run_last = is_wide_gemm(op) ? mk_run_gemm_wide(p, idx, slot) : mk_run_gemm(p, idx, slot);
                     break;
-                case MK_OP_ELTWISE: run_last = mk_run_eltwise(p, op, idx); break;
+                case MK_OP_ELTWISE: run_last = mk_run_eltwise(p, op, idx, slot); break;
                 case MK_OP_ATTENTION:
                     if (wait_deps(p, c, in.nwait, wait_off, in.seq)) { aborting = true; break; }
                     if (TRACE && threadIdx.x == 0) c->t_dep = (long long)globaltimer();
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                     aborting = mk_op_decode_attn(p, op, in.a0, in.a1, in.a2, in.nwait, wait_off, in.seq, in.narrive, arrive_off);
                     break;
                 case MK_OP_NORM:
-                    if (op->i[3] > 1) { run_last = mk_run_norm(p, op, idx); break; }
+                    if (op->i[3] > 1) { run_last = mk_run_norm(p, op, idx, slot); break; }
                     [[fallthrough]];
                 default:
                     if (wait_deps(p, c, in.nwait, wait_off, in.seq)) { aborting = true; break; }
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
             if (ran) {
                 aborting = run_last < 0;
                 if (!aborting) {
-                    slot += (run_last - idx) / (int)gridDim.x;
+                    slot += (run_last - idx) / (int)gridDim.x;       // (not Ctrl::run_slot: thread 0 may be in the next run already)
                     idx = run_last;
                 }
             }

@@ -121,7 +121,7 @@ __device__ __forceinline__ bool is_wide_gemm(const mk_op_desc* op) { return op->
 // instruction needs before its first useful load (its words, its op descriptor, its wait and
 // arrival lists) would otherwise be a chain of dependent global loads, each a round trip to L2 or
 // DRAM on the critical path between two dependent instructions.
-constexpr int kMetaWaits = 16;    // longer lists are read from global memory
+constexpr int kMetaWaits = 12;    // longer lists are read from global memory
 constexpr int kMetaArrives = 8;
 struct Meta {
     mk_op_desc desc[2];           // current / next instruction's op
@@ -175,7 +175,7 @@ struct Ctrl {                     // lives in the last kCtrlBytes of shared memo
     int flag;                     // scratch broadcast word (split-KV last arriver)
     long long t_dep;              // tracing: when the dependencies of the current instruction were met
     long long t_fetch;            // tracing: when a body that keeps the walk (walk.cuh) turned to the current instruction
-    int run_idx;                  // index of the instruction such a body is executing
+    int run_idx, run_slot;        // index of the instruction such a body is executing, and its number in the CTA's list
     long long t_pub;              // tracing: when its arrivals were published (0: the op left no mark)
     long long t_phase[3];         // tracing: op-internal phase marks (role 2 records)
 };
@@ -475,9 +475,11 @@ enum { WHERE_RING_FULL = 1, WHERE_RING_EMPTY = 2, WHERE_DEP = 3, WHERE_DRAIN = 4
 // `patience`: multiple of the time limit this wait allows.  A role that by design waits through everything the CTA does
 // before (the finisher warp, for the dependencies of a streaming linear far down the program) gives twice the limit, so
 // that when something earlier is stuck, the wait that is stuck reports first.
-__device__ __forceinline__ bool wait_barrier(const Params& p, Ctrl* c, unsigned long long* bar, uint32_t parity,
-                                             int seq, int where, unsigned patience = 1) {
-    if (mbar_test_wait(bar, parity)) return true;
+// The spinning part is a function of its own, not inlined: the bodies run cold, so what a wait costs when it does not have to
+// wait is the code that has to be fetched around it (with the loop and its error report inlined at every wait, the kernel's
+// own function was 122 KB).
+static __device__ __noinline__ bool wait_barrier_spin(const Params& p, Ctrl* c, unsigned long long* bar, uint32_t parity,
+                                                      int seq, int where, unsigned patience) {
     unsigned long long t0 = 0;
     for (uint32_t it = 1;; ++it) {
         if (mbar_try_wait(bar, parity)) return true;
@@ -492,6 +494,11 @@ __device__ __forceinline__ bool wait_barrier(const Params& p, Ctrl* c, unsigned 
             }
         }
     }
+}
+__device__ __forceinline__ bool wait_barrier(const Params& p, Ctrl* c, unsigned long long* bar, uint32_t parity,
+                                             int seq, int where, unsigned patience = 1) {
+    if (mbar_test_wait(bar, parity)) return true;
+    return wait_barrier_spin(p, c, bar, parity, seq, where, patience);
 }
 
 // the same for a shared-memory word that only grows
@@ -527,9 +534,8 @@ __device__ __forceinline__ bool check_phase(const Params& p, Ctrl* c, unsigned l
     return true;
 }
 
-__device__ __forceinline__ bool wait_counter(const Params& p, Ctrl* c, int counter, int target, int seq) {
+static __device__ __noinline__ bool wait_counter_spin(const Params& p, Ctrl* c, int counter, int want, int seq) {
     const int* addr = p.counters + counter;
-    const int want = target * p.epoch;
     unsigned long long t0 = 0;
     for (uint32_t it = 1;; ++it) {
         int v = ld_acquire(addr);
@@ -545,6 +551,11 @@ __device__ __forceinline__ bool wait_counter(const Params& p, Ctrl* c, int count
             }
         }
     }
+}
+__device__ __forceinline__ bool wait_counter(const Params& p, Ctrl* c, int counter, int target, int seq) {
+    const int want = target * p.epoch;
+    if (ld_acquire(p.counters + counter) >= want) return true;
+    return wait_counter_spin(p, c, counter, want, seq);
 }
 
 // One decoded instruction, held in registers (never address-taken, so it is never demoted to
@@ -585,6 +596,7 @@ __device__ __forceinline__ bool compute_sync_or(int pred) {
 // the CTA is aborting.  wait_off < 0 names the staged list Meta::waits[-1 - wait_off].
 __device__ __forceinline__ bool wait_deps(const Params& p, Ctrl* c, int nwait, int wait_off, int seq) {
     const int2* tab = wait_off < 0 ? c->meta.waits[-1 - wait_off] : p.waits + wait_off;
+#pragma unroll 1
     for (int k = threadIdx.x; k < nwait; k += kComputeThreads) {
         const int2 w = tab[k];
         wait_counter(p, c, w.x, w.y, seq);
@@ -606,6 +618,7 @@ __device__ __forceinline__ bool publish(const Params& p, Ctrl* c, int narrive, i
     // red.release.gpu, whose release is cumulative over them: no per-thread gpu-scope fence needed.
     if (compute_sync_or(*(volatile int*)&c->abort)) return true;
     if (first >= 0) red_release_add(p.counters + first, 1);
+#pragma unroll 1
     for (int k = threadIdx.x + kComputeThreads; k < narrive; k += kComputeThreads) red_release_add(p.counters + tab[k], 1);
     // The arriving lanes rejoin their warp here: a tail "if (lane arrives) red; return" may be compiled as an early return
     // of the other lanes, and the .sync.aligned instructions of the next op body (tcgen05.alloc / ld, mma.sync) want the

@@ -5,10 +5,10 @@
 #include "walk.cuh"
 
 namespace mk {
-__device__ int mk_run_gemm(const Params& p, int idx) {
+__device__ int mk_run_gemm(const Params& p, int idx, int slot) {
     const SmemMap m = smem_map();
     return run_own_insts(
-        p, m.ctrl, idx,
+        p, m.ctrl, idx, slot,
         [](const mk_op_desc* op) { return op->kind == MK_OP_GEMM && !is_wide_gemm(op); },
         [&](const mk_op_desc* op, int a0, int a1, int a2, int seq) -> int {
             // the host library attached tensor maps: tcgen05 body, weights through the producer's ring

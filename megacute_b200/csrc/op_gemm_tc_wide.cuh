@@ -284,59 +284,110 @@ __device__ __forceinline__ void wide_store16(const Params& p, Ctrl* c, const mk_
     }
 }
 
-// Everything else -- residual, fp32 output, split-K partial (reduce-add): 32 columns at a time through shared memory as fp32.
-// RK: 0 no residual, 1 16-bit, 2 fp32.  Residual (and gate) are requested DEPTH such steps ahead, the first ones while the main
-// loop still runs: a step takes 0.4 us, an L2 round trip beside the operand stream 1.5 (one step ahead: 20 us per tile).
-// The queue moves through registers one step per iteration, which costs less than unrolled code.
-// GATE: the result is multiplied by a gate row per i 12 rows (an adaLN-Zero block's gated residual) before the residual is added.
-__device__ __forceinline__ void wide_quad(int dtype, const uint4& w, float* f) {              // four values, raw bits of `dtype`
-    if (dtype == DT_F32) {
-        f[0] = __uint_as_float(w.x); f[1] = __uint_as_float(w.y); f[2] = __uint_as_float(w.z); f[3] = __uint_as_float(w.w);
-    } else if (dtype == DT_F16) {
-        const float2 lo = unpack2h(w.x), hi = unpack2h(w.y);
-        f[0] = lo.x; f[1] = lo.y; f[2] = hi.x; f[3] = hi.y;
-    } else {
-        f[0] = bf16_lo(w.x); f[1] = bf16_hi(w.x); f[2] = bf16_lo(w.y); f[3] = bf16_hi(w.y);
+// four values of a type known at compile time, as raw bits
+template <int DT> struct Quad {
+    uint2 v;
+    __device__ __forceinline__ void load(const uint8_t* base, long long elem) { v = __ldcg(reinterpret_cast<const uint2*>(base + elem * 2)); }
+    __device__ __forceinline__ float4 get() const {
+        if (DT == DT_F16) {
+            const float2 lo = unpack2h(v.x), hi = unpack2h(v.y);
+            return make_float4(lo.x, lo.y, hi.x, hi.y);
+        }
+        return make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
+    }
+};
+template <> struct Quad<DT_F32> {
+    float4 v;
+    __device__ __forceinline__ void load(const uint8_t* base, long long elem) { v = __ldcg(reinterpret_cast<const float4*>(base + elem * 4)); }
+    __device__ __forceinline__ float4 get() const { return v; }
+};
+template <int DT>
+__device__ __forceinline__ void put4(uint8_t* at, const float4& o) {
+    if (DT == DT_F32) *reinterpret_cast<float4*>(at) = o;
+    else if (DT == DT_F16) *reinterpret_cast<uint2*>(at) = make_uint2(pack2h(o.x, o.y), pack2h(o.z, o.w));
+    else *reinterpret_cast<uint2*>(at) = make_uint2(pack2(o.x, o.y), pack2(o.z, o.w));
+}
+__device__ __forceinline__ float4 load4_any(const uint8_t* base, long long elem, int dtype) {
+    if (dtype == DT_F32) { Quad<DT_F32> q; q.load(base, elem); return q.get(); }
+    if (dtype == DT_F16) { Quad<DT_F16> q; q.load(base, elem); return q.get(); }
+    Quad<DT_BF16> q; q.load(base, elem); return q.get();
+}
+
+// With a residual (out = acc + bias [times a gate row per i 12 rows: an adaLN-Zero block's gated residual] + residual): 32 columns at
+// a time through shared memory as fp32, so that a warp's accesses cover whole 64- or 128-byte row pieces.  kDepth such steps
+// of the residual are requested ahead, the first while the main loop still runs, each into registers of its own: a step
+// takes 0.4 us, an L2 round trip beside the operand stream 2 us (one step ahead, or several in a queue that moves through
+// registers -- a move waits for its load -- 2.1 - 2.6 us per step).
+template <int RDT, int ODT, bool GATE>
+__device__ __forceinline__ void wide_store_res(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
+    constexpr int kDepth = RDT == DT_F32 ? 2 : 4;
+    const int lane = threadIdx.x & 31;
+    const int groups = op->i[10] >> 5;
+    const int rows = min(32, op->i[0] - row0);
+    const int r = lane >> 3, c4 = (lane & 7) * 4;
+    constexpr int osz = ODT == DT_F32 ? 4 : 2, rsz = RDT == DT_F32 ? 4 : 2;
+    int ldo = op->ld[2] * osz, ldr = op->ld[4] * rsz;          // bytes between rows (32 of them stay within 2^31)
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + (long long)(row0 + r) * ldo + (n0 + c4) * osz;
+    const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]) + (long long)row0 * ldr + (n0 + c4) * rsz;
+    const int gdt = op->i[13];
+    const uint8_t* G = GATE ? reinterpret_cast<const uint8_t*>(op->ptr[5]) + ((long long)(row0 / op->i[12]) * op->ld[5] + n0 + c4) * 2 : nullptr;
+    Quad<RDT> q[kDepth][8];
+    Quad<DT_BF16> gate[GATE ? kDepth : 1];
+    auto request = [&](int d, int g) {                       // (rows beyond the tensor read its last row, steps beyond the tile its last step)
+        g = min(g, groups - 1);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) q[d][j].load(R + min(j * 4 + r, rows - 1) * ldr, g * 32);
+        if (GATE) gate[GATE ? d : 0].load(G, g * 32);
+    };
+#pragma unroll
+    for (int d = 0; d < kDepth; ++d) request(d, d);
+    if (!wide_wait(p, c, a)) return;
+#pragma unroll 1
+    for (int g0 = 0; g0 < groups; g0 += kDepth) {            // (128 or 256 columns: 4 or 8 steps)
+#pragma unroll
+        for (int d = 0; d < kDepth; ++d) {
+            const int g = g0 + d;
+            // (the row offsets are computed where they are used: kept for the whole loop they spill)
+            asm volatile("" : "+r"(ldo), "+r"(ldr));
+            float v[32];
+            tc_ld32(a.tacc + g * 32, v);
+            if (g == groups - 1) wide_release(a.release);
+            if (a.bias) wide_bias(a.bias, g * 32, v);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(wide_chunk(a.stg, lane, j)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+            __syncwarp();
+            float4 gt = make_float4(1.f, 1.f, 1.f, 1.f);
+            if (GATE) {
+                if (gdt == DT_F16) { Quad<DT_F16> h; h.v = gate[GATE ? d : 0].v; gt = h.get(); }
+                else gt = gate[GATE ? d : 0].get();
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                float4 o = *reinterpret_cast<const float4*>(wide_chunk(a.stg, j * 4 + r, lane & 7));
+                const float4 f = q[d][j].get();
+                if (GATE) o = make_float4(fmaf(o.x, gt.x, f.x), fmaf(o.y, gt.y, f.y), fmaf(o.z, gt.z, f.z), fmaf(o.w, gt.w, f.w));
+                else o = make_float4(o.x + f.x, o.y + f.y, o.z + f.z, o.w + f.w);
+                if (j * 4 + r < rows) put4<ODT>(O + j * 4 * ldo + g * 32 * osz, o);
+            }
+            request(d, g + kDepth);
+            __syncwarp();
+        }
     }
 }
-__device__ __forceinline__ uint4 wide_quad_load(int dtype, const uint8_t* base, long long elem) {
-    if (dtype == DT_F32) return __ldcg(reinterpret_cast<const uint4*>(base + elem * 4));
-    const uint2 w = __ldcg(reinterpret_cast<const uint2*>(base + elem * 2));
-    return make_uint4(w.x, w.y, 0u, 0u);
-}
-template <int RK, bool GATE>
+
+// Everything else -- fp32 output, split-K partial (reduce-add), an activation in front of a residual: the same without requests ahead.
 __device__ __forceinline__ void wide_store_any(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
-    constexpr int kDepth = RK == 0 ? 1 : RK == 1 ? 4 : 2;
     const int lane = threadIdx.x & 31;
     const int act = op->i[3], odt = op->i[5], rdt = op->i[7];
     const bool accum = op->i[6] != 0, swi = op->i[8] != 0;
     const int groups = (op->i[10] >> 5) >> (swi ? 1 : 0);
     const int rows = min(32, op->i[0] - row0);
     const int r = lane >> 3, c4 = (lane & 7) * 4, osz = odt == DT_F32 ? 4 : 2;
-    const long long ldo = (long long)op->ld[2] * osz, ldr = op->ld[4];
+    const long long ldo = (long long)op->ld[2] * osz;
     const int col0 = (swi ? n0 / 2 : n0) + c4;
     uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + (long long)(row0 + r) * ldo + col0 * osz;
-    const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]);
-    const uint8_t* G = reinterpret_cast<const uint8_t*>(op->ptr[5]);
-    // (16-bit residuals: two registers per row; rows beyond the tensor read its last row)
-    uint4 q32[RK == 2 ? kDepth : 1][RK == 2 ? 8 : 1], qg[GATE ? kDepth : 1];
-    uint2 q16[RK == 1 ? kDepth : 1][RK == 1 ? 8 : 1];
-    const int group = GATE ? op->i[12] : 1, gdt = op->i[13];
-    const bool one = GATE && row0 / group == (row0 + rows - 1) / group;                // the warp's rows share a gate row
-    auto request = [&](int d, int g) {
-        g = min(g, groups - 1);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const long long e = (long long)(row0 + min(j * 4 + r, rows - 1)) * ldr + col0 + g * 32;
-            if (RK == 1) q16[RK == 1 ? d : 0][RK == 1 ? j : 0] = __ldcg(reinterpret_cast<const uint2*>(R + e * 2));
-            if (RK == 2) q32[RK == 2 ? d : 0][RK == 2 ? j : 0] = __ldcg(reinterpret_cast<const uint4*>(R + e * 4));
-        }
-        if (GATE && one) qg[GATE ? d : 0] = wide_quad_load(gdt, G, (long long)(row0 / group) * op->ld[5] + col0 + g * 32);
-    };
-    if (RK) {
-#pragma unroll
-        for (int d = 0; d < kDepth; ++d) request(d, d);
-    }
+    const uint8_t* R = accum ? nullptr : reinterpret_cast<const uint8_t*>(op->ptr[4]);
+    const uint8_t* G = accum ? nullptr : reinterpret_cast<const uint8_t*>(op->ptr[5]);
     if (!wide_wait(p, c, a)) return;
 #pragma unroll 1
     for (int g = 0; g < groups; ++g) {
@@ -356,40 +407,25 @@ __device__ __forceinline__ void wide_store_any(const Params& p, Ctrl* c, const m
 #pragma unroll
         for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(wide_chunk(a.stg, lane, j)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         __syncwarp();
-        float gt[4] = {1.f, 1.f, 1.f, 1.f};
-        if (GATE && one) wide_quad(gdt, qg[0], gt);
-#pragma unroll
+#pragma unroll 1
         for (int j = 0; j < 8; ++j) {
+            if (j * 4 + r >= rows) break;
             float4 o = *reinterpret_cast<const float4*>(wide_chunk(a.stg, j * 4 + r, lane & 7));
-            if (GATE) {
-                if (!one) wide_quad(gdt, wide_quad_load(gdt, G, (long long)((row0 + min(j * 4 + r, rows - 1)) / group) * op->ld[5] + col0 + g * 32), gt);
-                o.x *= gt[0]; o.y *= gt[1]; o.z *= gt[2]; o.w *= gt[3];
+            if (G) {
+                const float4 f = load4_any(G, (long long)((row0 + j * 4 + r) / op->i[12]) * op->ld[5] + col0 + g * 32, op->i[13]);
+                o.x *= f.x; o.y *= f.y; o.z *= f.z; o.w *= f.w;
             }
-            if (RK) {
-                float f[4];
-                if (RK == 1) wide_quad(rdt, make_uint4(q16[0][RK == 1 ? j : 0].x, q16[0][RK == 1 ? j : 0].y, 0u, 0u), f);
-                else wide_quad(DT_F32, q32[0][RK == 2 ? j : 0], f);
-                o.x += f[0]; o.y += f[1]; o.z += f[2]; o.w += f[3];
+            if (R) {
+                const float4 f = load4_any(R, (long long)(row0 + j * 4 + r) * op->ld[4] + col0 + g * 32, rdt);
+                o.x += f.x; o.y += f.y; o.z += f.z; o.w += f.w;
             }
-            if (j * 4 + r >= rows) continue;
             uint8_t* at = O + (long long)(j * 4) * ldo + g * 32 * osz;
             if (accum) {
                 if (odt == DT_F32) red_add_f32x4(reinterpret_cast<float*>(at), o.x, o.y, o.z, o.w);
                 else red_add_bf16x4(at, &o.x);
-            } else if (odt == DT_F32) *reinterpret_cast<float4*>(at) = o;
-            else *reinterpret_cast<uint2*>(at) = make_uint2(pack2t(odt, o.x, o.y), pack2t(odt, o.z, o.w));
-        }
-        if (RK) {
-#pragma unroll
-            for (int d = 0; d + 1 < kDepth; ++d) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    if (RK == 1) q16[RK == 1 ? d : 0][RK == 1 ? j : 0] = q16[RK == 1 ? d + 1 : 0][RK == 1 ? j : 0];
-                    if (RK == 2) q32[RK == 2 ? d : 0][RK == 2 ? j : 0] = q32[RK == 2 ? d + 1 : 0][RK == 2 ? j : 0];
-                }
-                if (GATE) qg[GATE ? d : 0] = qg[GATE ? d + 1 : 0];
-            }
-            request(kDepth - 1, g + kDepth);
+            } else if (odt == DT_F32) put4<DT_F32>(at, o);
+            else if (odt == DT_F16) put4<DT_F16>(at, o);
+            else put4<DT_BF16>(at, o);
         }
         __syncwarp();
     }
@@ -398,13 +434,14 @@ __device__ __forceinline__ void wide_store_any(const Params& p, Ctrl* c, const m
 // The epilogue of an op, chosen once per run of instructions: each has a function of its own around it (op_gemm_wide.cu) and so a
 // register allocation of its own -- called per instruction they pay ~60 saved and restored registers each time, inlined
 // side by side they spill, and with the shared memory taken every such access is an L2 round trip behind the operand stream.
-enum { WIDE_PLAIN = 0, WIDE_SWIGLU, WIDE_GELU, WIDE_ACT, WIDE_ANY0, WIDE_ANY1, WIDE_ANY2, WIDE_GATE1, WIDE_GATE2 };      // (+ 16: fp16 output, the first four)
+// WIDE_PLAIN .. WIDE_ACT: + 16 for fp16 output.  WIDE_RES: + residual dtype | output dtype << 2 | gate << 4.
+enum { WIDE_PLAIN = 0, WIDE_SWIGLU, WIDE_GELU, WIDE_ACT, WIDE_ANY, WIDE_RES = 32 };
 __device__ __forceinline__ int wide_variant(const mk_op_desc* op) {
     const int odt = op->i[5];
-    if (op->i[6]) return WIDE_ANY0;
-    if (op->ptr[5]) return op->i[7] == DT_F32 ? WIDE_GATE2 : WIDE_GATE1;
-    if (op->ptr[4]) return op->i[7] == DT_F32 ? WIDE_ANY2 : WIDE_ANY1;
-    if (odt == DT_F32) return WIDE_ANY0;
+    if (op->i[6]) return WIDE_ANY;
+    const bool gate32 = !op->ptr[5] || (op->i[12] % 32 == 0 && op->i[13] != DT_F32);         // a warp's 32 rows share a 16-bit gate row
+    if (op->ptr[4]) return op->i[3] == ACT_NONE && !op->i[8] && gate32 ? WIDE_RES + (op->i[7] | odt << 2 | (op->ptr[5] ? 16 : 0)) : WIDE_ANY;
+    if (odt == DT_F32) return WIDE_ANY;
     const int v = op->i[8] ? WIDE_SWIGLU : op->i[3] == ACT_NONE ? WIDE_PLAIN : op->i[3] == ACT_GELU ? WIDE_GELU : WIDE_ACT;
     return v + (odt == DT_F16 ? 16 : 0);
 }
@@ -449,14 +486,17 @@ __device__ __forceinline__ void op_gemm_tc_wide(const Params& p, Ctrl* c, uint8_
         if (wide_wait(p, c, a)) wide_release(a.release);
         return;
     }
-    constexpr bool f16 = (V & 16) != 0;
-    constexpr int kind = V & 15;
-    if constexpr (kind == WIDE_PLAIN) wide_store16<f16, false, 0>(p, c, op, a, row0, n0);
-    else if constexpr (kind == WIDE_SWIGLU) wide_store16<f16, true, 0>(p, c, op, a, row0, n0);
-    else if constexpr (kind == WIDE_GELU) wide_store16<f16, false, 1>(p, c, op, a, row0, n0);
-    else if constexpr (kind == WIDE_ACT) wide_store16<f16, false, 2>(p, c, op, a, row0, n0);
-    else if constexpr (kind >= WIDE_GATE1) wide_store_any<kind - WIDE_GATE1 + 1, true>(p, c, op, a, row0, n0);
-    else wide_store_any<kind - WIDE_ANY0, false>(p, c, op, a, row0, n0);
+    if constexpr (V >= WIDE_RES) {
+        wide_store_res<V & 3, (V >> 2) & 3, (V & 16) != 0>(p, c, op, a, row0, n0);
+    } else {
+        constexpr bool f16 = (V & 16) != 0;
+        constexpr int kind = V & 15;
+        if constexpr (kind == WIDE_PLAIN) wide_store16<f16, false, 0>(p, c, op, a, row0, n0);
+        else if constexpr (kind == WIDE_SWIGLU) wide_store16<f16, true, 0>(p, c, op, a, row0, n0);
+        else if constexpr (kind == WIDE_GELU) wide_store16<f16, false, 1>(p, c, op, a, row0, n0);
+        else if constexpr (kind == WIDE_ACT) wide_store16<f16, false, 2>(p, c, op, a, row0, n0);
+        else wide_store_any(p, c, op, a, row0, n0);
+    }
 }
 
 }  // namespace mk

@@ -9,10 +9,10 @@
 namespace mk {
 
 template <int V>
-static __device__ __noinline__ int wide_run(const Params& p, int idx) {
+static __device__ __noinline__ int wide_run(const Params& p, int idx, int slot) {
     const SmemMap m = smem_map();
     return run_own_insts(
-        p, m.ctrl, idx, [](const mk_op_desc* op) { return is_wide_gemm(op) && wide_variant(op) == V; },
+        p, m.ctrl, idx, slot, [](const mk_op_desc* op) { return is_wide_gemm(op) && wide_variant(op) == V; },
         [&](const mk_op_desc* op, int a0, int a1, int, int seq) -> int {
             op_gemm_tc_wide<V>(p, m.ctrl, m.ring, op, a0, a1, seq);
             return 0;
@@ -20,37 +20,33 @@ static __device__ __noinline__ int wide_run(const Params& p, int idx) {
         [&] { if (threadIdx.x == 0) m.ctrl->wide_uses += 1; });
 }
 
-__device__ int mk_run_gemm_wide(const Params& p, int idx) {
+__device__ int mk_run_gemm_wide(const Params& p, int idx, int slot) {
     const SmemMap m = smem_map();
     const Meta* mt = &m.ctrl->meta;
     wide_begin_run(m.ctrl);
     for (;;) {
-        const int slot = (idx - (int)blockIdx.x) / (int)gridDim.x;
         int last;
         switch (wide_variant(&mt->desc[slot & 1])) {
-            case WIDE_PLAIN: last = wide_run<WIDE_PLAIN>(p, idx); break;
-            case WIDE_SWIGLU: last = wide_run<WIDE_SWIGLU>(p, idx); break;
-            case WIDE_GELU: last = wide_run<WIDE_GELU>(p, idx); break;
-            case WIDE_ACT: last = wide_run<WIDE_ACT>(p, idx); break;
-            case WIDE_PLAIN + 16: last = wide_run<WIDE_PLAIN + 16>(p, idx); break;
-            case WIDE_SWIGLU + 16: last = wide_run<WIDE_SWIGLU + 16>(p, idx); break;
-            case WIDE_GELU + 16: last = wide_run<WIDE_GELU + 16>(p, idx); break;
-            case WIDE_ACT + 16: last = wide_run<WIDE_ACT + 16>(p, idx); break;
-            case WIDE_ANY1: last = wide_run<WIDE_ANY1>(p, idx); break;
-            case WIDE_ANY2: last = wide_run<WIDE_ANY2>(p, idx); break;
-            case WIDE_GATE1: last = wide_run<WIDE_GATE1>(p, idx); break;
-            case WIDE_GATE2: last = wide_run<WIDE_GATE2>(p, idx); break;
-            default: last = wide_run<WIDE_ANY0>(p, idx); break;
+#define MK_W(V) case (V): last = wide_run<(V)>(p, idx, slot); break
+            MK_W(WIDE_PLAIN); MK_W(WIDE_SWIGLU); MK_W(WIDE_GELU); MK_W(WIDE_ACT);
+            MK_W(WIDE_PLAIN + 16); MK_W(WIDE_SWIGLU + 16); MK_W(WIDE_GELU + 16); MK_W(WIDE_ACT + 16);
+#define MK_WR(R) MK_W(WIDE_RES + (R)); MK_W(WIDE_RES + ((R) | DT_F32 << 2)); MK_W(WIDE_RES + ((R) | DT_F16 << 2)); \
+                 MK_W(WIDE_RES + ((R) | 16)); MK_W(WIDE_RES + ((R) | DT_F32 << 2 | 16)); MK_W(WIDE_RES + ((R) | DT_F16 << 2 | 16))
+            MK_WR(DT_BF16); MK_WR(DT_F32); MK_WR(DT_F16);
+#undef MK_WR
+#undef MK_W
+            default: last = wide_run<WIDE_ANY>(p, idx, slot); break;
         }
         if (last < 0) return -1;
-        const int next = last + (int)gridDim.x;
-        if (!next_is(p, m.ctrl, last, [](const mk_op_desc* op) { return is_wide_gemm(op); })) {
+        slot += (last - idx) / (int)gridDim.x;                  // (the last instruction's; not Ctrl::run_slot: thread 0 may be in the next run already)
+        if (!next_is(p, m.ctrl, last, slot, [](const mk_op_desc* op) { return is_wide_gemm(op); })) {
             // (behind the last instruction's barrier: nobody reads the staging rows any more)
             if (threadIdx.x == 0) *(volatile uint32_t*)&m.ctrl->wide_done = m.ctrl->wide_uses;
             return last;
         }
-        idx = next;
-        stage_following(p, m.ctrl, idx);
+        idx = last + (int)gridDim.x;
+        ++slot;
+        stage_following(p, m.ctrl, idx, slot);
     }
 }
 

@@ -19,13 +19,13 @@ __device__ int mk_op_gemv_units(const Params& p, const mk_op_desc* op, int o0, i
 // body of the finisher warp (op_gemv_mma.cuh): runs until the CTA's instruction list ends
 __device__ void mk_gemv_finisher(const Params& p);
 __device__ int mk_op_gemv_general(const Params& p, const mk_op_desc* op, int o0, int o1, int seq, int packed_pos);
-// Tile GEMM.  The kernel's loop has fetched instruction `idx` and chosen this body; the body runs it and every
+// Tile GEMM.  The kernel's loop has fetched instruction `idx`, the CTA's `slot`-th, and chosen this body; the body runs it and every
 // following instruction of the CTA that is its own (walk.cuh), waiting for the dependencies and publishing the
 // arrivals of each itself (begin_op says why).  Returns the index of the last instruction executed, -1 when the CTA is
 // aborting.  (The ring position is untouched: the weight tiles have slots of their own.)
-__device__ int mk_run_gemm(const Params& p, int idx);
+__device__ int mk_run_gemm(const Params& p, int idx, int slot);
 // (the same with 256 x 256 output tiles; only for ops the host library bound to the tcgen05 body)
-__device__ int mk_run_gemm_wide(const Params& p, int idx);
+__device__ int mk_run_gemm_wide(const Params& p, int idx, int slot);
 // body of the issuer warp: the MMAs of every 256 x 256 tile, until the feeder warp says that the list has ended
 __device__ void mk_wide_issuer(const Params& p);
 __device__ void mk_op_attention(const mk_op_desc* op, int a0, int a1, int a2);
@@ -42,8 +42,8 @@ __device__ bool mk_op_decode_attn(const Params& p, const mk_op_desc* op, int a0,
 __device__ bool mk_op_decode_bulk(const Params& p, const mk_op_desc* op, int b, int s, int nwait, int wait_off, int seq,
                                   int narrive, int arrive_off);
 // pointwise tiles and norms with several rows per instruction (op_stream.cuh): like mk_run_gemm, for runs of their own kind
-__device__ int mk_run_eltwise(const Params& p, const mk_op_desc* op, int idx);
-__device__ int mk_run_norm(const Params& p, const mk_op_desc* op, int idx);
+__device__ int mk_run_eltwise(const Params& p, const mk_op_desc* op, int idx, int slot);
+__device__ int mk_run_norm(const Params& p, const mk_op_desc* op, int idx, int slot);
 // finalize / norm of one row / rope_append / increment / gather / argmax; returns false for an unknown kind
 __device__ bool mk_op_pointwise(const mk_op_desc* op, int a0, int a1);
 
