@@ -14,6 +14,7 @@
 //   warp 11    issuer: MMAs of the 256 x 256 tile GEMM.
 // This replaces the reference's JIT-traced kernel (megacute/kernel.py:251-571) and its per-op
 // role bodies (megacute/ops/*.py).
+#define MK_INLINE_WAITS 1
 #include <cuda.h>          // CUtensorMap and cuTensorMapEncodeTiled's signature (resolved at run time, libcuda is not linked)
 
 #include <cstdio>

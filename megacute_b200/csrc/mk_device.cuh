@@ -475,10 +475,15 @@ enum { WHERE_RING_FULL = 1, WHERE_RING_EMPTY = 2, WHERE_DEP = 3, WHERE_DRAIN = 4
 // `patience`: multiple of the time limit this wait allows.  A role that by design waits through everything the CTA does
 // before (the finisher warp, for the dependencies of a streaming linear far down the program) gives twice the limit, so
 // that when something earlier is stuck, the wait that is stuck reports first.
-// The spinning part is a function of its own, not inlined: the bodies run cold, so what a wait costs when it does not have to
-// wait is the code that has to be fetched around it (with the loop and its error report inlined at every wait, the kernel's
-// own function was 122 KB).
-static __device__ __noinline__ bool wait_barrier_spin(const Params& p, Ctrl* c, unsigned long long* bar, uint32_t parity,
+// The spinning part is a function of its own in the bodies of tile ops: those run cold, so what a wait costs when it does not have
+// to wait is the code that has to be fetched around it.  The streaming bodies of a decode step inline it (MK_INLINE_WAITS, set
+// by their translation units): there every wait does wait, and the call costs more than the code (batch-1 step 877 -> 912 us).
+#ifdef MK_INLINE_WAITS
+#define MK_SPIN __device__ __forceinline__
+#else
+#define MK_SPIN static __device__ __noinline__
+#endif
+MK_SPIN bool wait_barrier_spin(const Params& p, Ctrl* c, unsigned long long* bar, uint32_t parity,
                                                       int seq, int where, unsigned patience) {
     unsigned long long t0 = 0;
     for (uint32_t it = 1;; ++it) {
@@ -534,7 +539,7 @@ __device__ __forceinline__ bool check_phase(const Params& p, Ctrl* c, unsigned l
     return true;
 }
 
-static __device__ __noinline__ bool wait_counter_spin(const Params& p, Ctrl* c, int counter, int want, int seq) {
+MK_SPIN bool wait_counter_spin(const Params& p, Ctrl* c, int counter, int want, int seq) {
     const int* addr = p.counters + counter;
     unsigned long long t0 = 0;
     for (uint32_t it = 1;; ++it) {

@@ -1,4 +1,5 @@
 // Translation unit of MK_OP_DECODE_ATTN.
+#define MK_INLINE_WAITS 1
 #include "op_decode.cuh"
 #include "ops.cuh"
 

@@ -1,5 +1,6 @@
 // Translation unit of the many-sequence form of MK_OP_DECODE_ATTN (compute-warp side; the copies are
 // issued by the producer warp, op_gemv_common.cuh).
+#define MK_INLINE_WAITS 1
 #include "op_decode_bulk.cuh"
 #include "ops.cuh"
 

@@ -1,4 +1,5 @@
 // Translation unit of the tensor-core streaming path of MK_OP_GEMV.
+#define MK_INLINE_WAITS 1
 #include "op_gemv_mma.cuh"
 #include "ops.cuh"
 

@@ -1,4 +1,5 @@
 // Translation unit of the general (2..8 row, or odd K) path of MK_OP_GEMV.
+#define MK_INLINE_WAITS 1
 #include "op_gemv.cuh"
 #include "ops.cuh"
 
