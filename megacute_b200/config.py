@@ -39,7 +39,7 @@ NORM_ROWS, NORM_MAX_ROWS = COMPUTE_WARPS, 64
 EW_MIN_ROWS, EW_MAX_ROWS, STREAM_INSTS = 4, 128, 148
 WIDE_NORM_ROWS = 256
 ROPE_APPEND_ROWS = COMPUTE_WARPS
-ATTN_BQ, ATTN_BK = 128, 64
+ATTN_BQ, ATTN_BK = 256, 64          # queries per prefill attention instruction (two tiles of 128), keys per tile of the mma.sync body
 DECODE_KEYS_PER_TILE = 64
 MIN_SPLIT_KEYS = 64
 MAX_KV_SPLITS = 32

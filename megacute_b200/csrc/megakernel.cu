@@ -71,6 +71,18 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         mbar_init(&c->gemm_go, 1);
         c->wide_uses = c->wide_done = 0;
         mbar_init(&c->attn_go, 1);
+        mbar_init(&c->ring_granted, 1);
+        mbar_init(&c->ring_returned, 1);
+        mbar_init(&c->attn.q_full, 1);
+        mbar_init(&c->attn.q_free, 1);
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&c->attn.k_full[s], 1); mbar_init(&c->attn.k_empty[s], 2);
+            mbar_init(&c->attn.v_full[s], 1); mbar_init(&c->attn.v_empty[s], 2);
+            mbar_init(&c->attn.s_full[s], 1); mbar_init(&c->attn.p_full[s], kComputeWarps / 2);
+            mbar_init(&c->attn.pv_done[s], 1); mbar_init(&c->attn.o_free[s], kComputeWarps / 2);
+            c->at_blocks[0][s] = 0;
+        }
+        c->at_turn = 0;
         mbar_init(&c->acc_full, kTcIssuers);
         for (int s = 0; s < kKvSlots; ++s) {
             mbar_init(&c->kv_full[s], 1);
@@ -94,13 +106,13 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         // ---------------- finisher warp: epilogues of the streaming linear ----------------
         mk_gemv_finisher(p);
     } else if (warp == kFeederWarp) {
-        // ---------------- feeder warp: tiles and MMAs of the tcgen05 prefill attention, activation tiles of 256 x 256 tile GEMMs ----------------
+        // ---------------- feeder warp: tiles of the tcgen05 prefill attention, activation tiles of tile GEMMs with 256-row tiles ----------------
         // (a warp of its own rather than a branch of the producer's loop: the call in that loop cost every decode step
         // 0.5 %, whether or not the graph had such an op; here a graph without one costs a walk over the instruction list)
         mk_feeder(p);
     } else if (warp == kIssuerWarp) {
-        // ---------------- issuer warp: MMAs of 256 x 256 tile GEMMs ----------------
-        mk_wide_issuer(p);
+        // ---------------- issuer warp: MMAs of tile GEMMs with 256-row tiles and of the tcgen05 prefill attention ----------------
+        mk_issuer(p);
     } else {
         // ---------------- compute warps ----------------
         // Instruction metadata runs one instruction ahead in shared memory (Meta): while instruction
@@ -165,11 +177,12 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                     break;
                 case MK_OP_ELTWISE: run_last = mk_run_eltwise(p, op, idx, slot); break;
                 case MK_OP_ATTENTION:
+                    if (op->ptr[11]) { run_last = mk_run_attention(p, op, idx, slot); break; }
                     if (wait_deps(p, c, in.nwait, wait_off, in.seq)) { aborting = true; break; }
                     if (TRACE && threadIdx.x == 0) c->t_dep = (long long)globaltimer();
-                    if (op->ptr[11]) aborting = mk_op_attention_tc(p, op, in.a0, in.a1, in.a2, in.seq) < 0;
-                    else mk_op_attention(op, in.a0, in.a1, in.a2);
-                    aborting = publish(p, c, in.narrive, arrive_off) || aborting;
+                    // (256 queries: two tiles of this body)
+                    for (int q = 2 * in.a2; q < 2 * in.a2 + 2 && q * 128 < op->i[1]; ++q) mk_op_attention(op, in.a0, in.a1, q);
+                    aborting = publish(p, c, in.narrive, arrive_off);
                     break;
                 case MK_OP_DECODE_ATTN:
                     aborting = mk_op_decode_attn(p, op, in.a0, in.a1, in.a2, in.nwait, wait_off, in.seq, in.narrive, arrive_off);
@@ -225,6 +238,13 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         for (int s = 0; s < 2 * kWideStages; ++s) {
             unsigned long long t0 = globaltimer();
             while (!(mbar_try_wait(&c->ww_full[0][0] + s, 0) || mbar_try_wait(&c->ww_full[0][0] + s, 1))) {
+                if (globaltimer() - t0 > 20000000ull) break;
+            }
+        }
+        for (int s = 0; s < 5; ++s) {                              // tiles of the tcgen05 attention
+            unsigned long long* bar = s == 0 ? &c->attn.q_full : s < 3 ? &c->attn.k_full[s - 1] : &c->attn.v_full[s - 3];
+            unsigned long long t0 = globaltimer();
+            while (!(mbar_try_wait(bar, 0) || mbar_try_wait(bar, 1))) {
                 if (globaltimer() - t0 > 20000000ull) break;
             }
         }
@@ -444,7 +464,7 @@ static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
                     if (d.i[3] <= 0 || a0 < 0 || a0 * d.i[3] >= d.i[0]) why = "norm: row group outside the rows";
                     break;
                 case MK_OP_ATTENTION:
-                    if (a0 < 0 || a0 >= d.i[0] || a1 < 0 || a1 >= d.i[3] || a2 < 0 || a2 * 128 >= d.i[1]) why = "attention: (batch, head, query tile)";
+                    if (a0 < 0 || a0 >= d.i[0] || a1 < 0 || a1 >= d.i[3] || a2 < 0 || a2 * 256 >= d.i[1]) why = "attention: (batch, head, query tile)";
                     break;
                 case MK_OP_ROPE_APPEND:
                     if (a0 < 0 || a0 * 8 >= d.i[0]) why = "rope_append: row group outside the batch";
@@ -621,20 +641,18 @@ int mk_program_set_ops(mk_program* p, const mk_op_desc* ops, int n_ops, void* st
     for (int k = 0; k < n_ops; ++k) {
         mk_op_desc& d = h_ops[k];
         if (d.kind == MK_OP_ATTENTION) {
-            // head_dim 64: tensor maps over q, k, v select the tcgen05 body (op_attention_tc.cuh)
+            // tensor maps over q, k, v select the tcgen05 body (op_attention_tc.cuh)
             d.ptr[11] = 0;
             uint8_t* maps = h_tmaps + (size_t)k * kMapBytes;
-            const long long B = d.i[0], Sq = d.i[1], Sk = d.i[2], H = d.i[3], KVH = d.i[4];
-            // On unless MEGACUTE_B200_ATTN_TCGEN05=0: measured on 4 x 4096 causal tokens (32 heads, 8 kv heads, 16 layers)
-            // the tcgen05 body (softmax on all eight compute warps, tiles and MMAs fed by the producer warp) takes
-            // 14.5 ms of attention against the mma.sync body's 31 ms.
+            const long long B = d.i[0], Sq = d.i[1], Sk = d.i[2], H = d.i[3], KVH = d.i[4], D = d.i[5];
+            // On unless MEGACUTE_B200_ATTN_TCGEN05=0.
             const char* attn_tc = getenv("MEGACUTE_B200_ATTN_TCGEN05");
             if (attn_tc && attn_tc[0] == '0') continue;
-            if (tc_off || d.i[5] != 64 || (d.ptr[3] & 15) || d.ld[3] % 8) continue;
+            if (tc_off || (D != 64 && D != 128) || (d.ptr[3] & 15) || d.ld[3] % 8) continue;
             const bool h16 = d.i[8] == mk::DT_F16;
-            if (encode_tile_map(maps, d.ptr[0], B * Sq, H * 64, d.ld[0], 128, false, h16) &&
-                encode_tile_map(maps + 128, d.ptr[1], B * Sk, KVH * 64, d.ld[1], 128, false, h16) &&
-                encode_tile_map(maps + 256, d.ptr[2], B * Sk, KVH * 64, d.ld[2], 128, false, h16)) {
+            if (encode_tile_map(maps, d.ptr[0], B * Sq, H * D, d.ld[0], 128, false, h16) &&
+                encode_tile_map(maps + 128, d.ptr[1], B * Sk, KVH * D, d.ld[1], 128, false, h16) &&
+                encode_tile_map(maps + 256, d.ptr[2], B * Sk, KVH * D, d.ld[2], 128, false, h16)) {
                 d.ptr[11] = reinterpret_cast<uint64_t>(p->d_tmaps + (size_t)k * kMapBytes);
                 any_map = true;
                 ++n_attn;

@@ -117,6 +117,9 @@ struct Params {
 // a tile GEMM bound to the tcgen05 body with 256-row tiles (op_gemm_tc_wide.cuh)
 __device__ __forceinline__ bool is_wide_gemm(const mk_op_desc* op) { return op->kind == MK_OP_GEMM && op->i[11] == 256 && op->ptr[11] != 0; }
 
+// a prefill attention bound to the tcgen05 body (op_attention_tc.cuh)
+__device__ __forceinline__ bool is_attention_tc(const mk_op_desc* op) { return op->kind == MK_OP_ATTENTION && op->ptr[11] != 0; }
+
 // Instruction metadata staged in shared memory one instruction ahead of its use.  Everything an
 // instruction needs before its first useful load (its words, its op descriptor, its wait and
 // arrival lists) would otherwise be a chain of dependent global loads, each a round trip to L2 or
@@ -130,8 +133,10 @@ struct Meta {
     int arrives[2][kMetaArrives];
 };
 
-struct AttnBars {                 // tcgen05 prefill attention (op_attention_tc.cuh): re-initialised by every instruction
-    unsigned long long q_full, k_full[2], k_empty[2], v_full, v_empty, s_full[2], s_empty[2], p_full, pv_done;
+struct AttnBars {                 // tcgen05 prefill attention (op_attention_tc.cuh)
+    unsigned long long q_full, q_free;               // the two Q tiles have landed / every product that reads them has completed
+    unsigned long long k_full[2], k_empty[2], v_full[2], v_empty[2];      // ... the K, V stages (released once per Q tile)
+    unsigned long long s_full[2], p_full[2], pv_done[2], o_free[2];       // per Q tile: scores there; read, and P written; P V done; O read
 };
 
 struct Ctrl {                     // lives in the last kCtrlBytes of shared memory
@@ -162,8 +167,9 @@ struct Ctrl {                     // lives in the last kCtrlBytes of shared memo
     unsigned long long kv_go;                // ... (unfused form) the instruction's dependencies are met: the row appended in this launch may be read
     uint32_t kv_cons;                        // ... the compute warps' position in the slots (slot | phase << 8)
     AttnBars attn;
-    unsigned long long attn_go;              // tcgen05 prefill attention: the compute warps are at the instruction (dependencies met,
-                                             // barriers initialised); the feeding thread of the producer warp may start
+    unsigned long long attn_go;              // tcgen05 prefill attention: the compute warps have turned to the first of a run
+    unsigned long long ring_granted, ring_returned;      // ... head_dim 128: the run may use the ring's memory / is done with it
+    uint32_t at_blocks[2][2], at_turn;       // ... blocks of each Q tile so far, written for the next instruction during this one; whose turn
     uint32_t tmem_base;               // ... tensor-memory address of the accumulator (written by tcgen05.alloc)
     uint32_t tmem_ready;              // ... 1 once it is allocated; written behind the barrier that follows the allocation, so all
                                       //     threads of an instruction read the same value (tmem_base changes while they arrive)

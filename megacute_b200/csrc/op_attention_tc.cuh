@@ -1,61 +1,57 @@
-// MK_OP_ATTENTION on the 5th-generation tensor cores (tcgen05 + tensor memory), head_dim 64.
-// One instruction = (batch b, head h, 128-query tile), as the mma.sync body (op_attention.cuh); the host
-// library selects this body by attaching three tensor maps (q, k, v: {columns, rows} bf16, boxes of 64
-// columns x 128 rows, 128-byte swizzle, zero fill) through ptr 11.
+// MK_OP_ATTENTION on the 5th-generation tensor cores (tcgen05 + tensor memory), head_dim 64 or 128.
+// One instruction = (batch b, head h, 256 queries): two tiles of 128 queries that share every K and V tile.  The host
+// library selects this body by attaching three tensor maps (q, k, v: {columns, rows}, boxes of 64 columns x 128 rows,
+// 128-byte swizzle, zero fill) through ptr 11.
 //
-//   S = Q K_j^T      tcgen05.mma 128 x 128 x 16 (x 4 for head_dim 64): Q and the 128-key tile K_j are K-major
-//                    operands in shared memory; S lives in tensor memory, columns 0..127, fp32
-//   softmax          all eight compute warps, two threads per query row: a tensor-memory lane is a query row and a
-//                    warp reaches the 32 lanes of its quarter (warp & 3), so warps w and w + 4 share 32 rows and take
-//                    64 of the block's 128 score columns each (read from tensor memory once for the maximum and once
-//                    for the exponentials, 32 at a time: 64 held at once spill under the kernel's register cap).  The two threads of a row agree on the maximum
-//                    through shared memory (bf16 values: any common reference near the maximum will do, see the
-//                    lazy rescale) and add their partial row sums at the end.  Log2 domain, scale * log2(e) folded
-//                    into the subtraction; P rounded to the operand type and written to shared memory as the
-//                    K-major A operand of the second product (a thread's 64 keys are one 128-byte row of one tile).
-//                    The running maximum is only raised when it grows by more than 2^8 (the reference's lazy
-//                    rescale, megacute/ops/attention.py:37,252-262): then the row's sum and its O row in tensor
-//                    memory are scaled down.  (One thread per row, four warps: one warp per scheduler, issue-active
-//                    18 %, 8.8 us per 128-key block against 0.4 us of MMA; the mma.sync body took 4.3 us.)
-//   O += P V_j       tcgen05.mma 128 x 64 x 16 (x 8 for 128 keys): V_j as loaded ([key][64 dims], dims
-//                    contiguous) is the MN-major B operand; O lives in tensor memory, columns 256..319
-//   out = O / l      read back with tcgen05.ld, half a row per thread; a fully masked row yields 0
+//   S = Q_t K_j^T    tcgen05.mma 128 x 128 x 16: Q tile and 128-key tile as K-major operands in shared memory; S in tensor memory
+//   softmax          compute warps 4 t .. 4 t + 3, one thread per query row of tile t (a tensor-memory lane): the row's 128 scores are
+//                    read twice, 32 at a time, for the maximum and for the exponentials, so nothing is exchanged between
+//                    threads.  Log2 domain, scale * log2(e) folded into the subtraction.  The running maximum is only raised
+//                    when it grows by more than 2^8 (the reference's lazy rescale, megacute/ops/attention.py:37,252-262): then
+//                    the row's sum and its O row in tensor memory are scaled down.
+//   O += P V_j       P, rounded to the operand type, goes back to tensor memory as the A operand; V_j as loaded ([key][64 dims])
+//                    is the MN-major B operand; O in tensor memory
+//   out = O / l      read back, a row per thread; a fully masked row yields 0
+// While one tile's scores are multiplied the other tile's are exponentiated: 128 x 128 exponentials take the SM's special
+// function units 1024 cycles, the products of a block 600 to 1100.  (One tile per instruction, two threads per row that agreed
+// on the maximum through shared memory, P through shared memory: 3800 cycles per block.)
 //
-// Tile requests and MMA issue are ONE thread of the feeder warp (mk_attention_feeder walks the CTA's instruction list
-// for these ops): it polls the barriers without blocking (mbarrier.test_wait costs ~1 ns) and does
-// whatever is possible next -- K_j into two buffers, V_j into one, each refilled as soon as the product that read
-// it has completed; S of block j + 1 (two S tiles in tensor memory) ahead of P V of block j, so the tensor core works
-// on the next scores while the softmax of this block runs.  The compute warps tell it through `attn_go` that the
-// instruction's dependencies are met and its barriers initialised (nothing of the previous instruction is pending:
-// every copy was waited for and the last commit of an instruction arrives behind all earlier ones).  Every wait is
-// bounded.  head_dim 128 and operands the tensor maps cannot describe run the mma.sync body.
+// Three roles run ahead of one another across the instructions of a run, as in the tile GEMM (op_gemm_tc_wide.cuh):
+//   feeder warp      waits for the instruction's dependencies itself, requests Q, then K and V through two stages each
+//   issuer warp      the products of both tiles, whatever is possible next; told by the feeder through Ctrl::wide_info
+//   compute warps    softmax and output
+// Barriers are initialised once per launch; every role counts.  Tensor memory (columns): S at 0 and 128; head_dim 64: O at 256 and
+// 320, P at 384 and 448; head_dim 128: O at 256 and 384, P over S (the next scores of a tile then wait for its P V).
+// Shared memory: head_dim 64: two Q tiles, two K and two V stages in the work area; head_dim 128: Q in the work area, K and V in the
+// ring's memory, which the producer warp grants for a run (Ctrl::ring_granted / ring_returned).
+// Every wait is bounded.  Operands the tensor maps cannot describe run the mma.sync body.
 //
 // ptr 0 q, 1 k, 2 v, 3 out, 11 tensor maps; i 0 batch, 1 seq_q, 2 seq_k, 3 heads, 4 kv_heads, 5 head_dim,
-// 6 causal, 7 out dtype, 8 dtype of q, k, v; f 0 scale.  args: 0 b, 1 h, 2 query tile.
+// 6 causal, 7 out dtype, 8 dtype of q, k, v; f 0 scale.  args: 0 b, 1 h, 2 query tile pair.
 #pragma once
 #include "mk_device.cuh"
 #include "tc.cuh"
 
 namespace mk {
 
-constexpr int kAtQOff = kTcXOff;                              // shared-memory map of the work area (1024-byte aligned tiles)
-constexpr int kAtKOff = kAtQOff + kTcTileBytes;               // two K buffers
-constexpr int kAtVOff = kAtKOff + 2 * kTcTileBytes;
-constexpr int kAtPOff = kAtVOff + kTcTileBytes;               // P: two 128 x 64 K-major tiles (keys 0..63, 64..127)
-static_assert(kAtPOff + 2 * kTcTileBytes <= kWorkBytes, "attention tiles exceed the work area");
-constexpr uint32_t kAtSCol = 0, kAtOCol = 256;                // tensor-memory columns: S buffers at 0 and 128, O at 256
-static_assert(kAtOCol + 64 <= kTcCols, "attention accumulators exceed the tensor memory held");
 constexpr float kAtRescale = 8.0f;                            // raise the running maximum only past 2^8
+// byte offsets from the ring's start
+template <int D> struct AtMap {
+    static constexpr int kTile = 128 * D * 2;                 // one tile of Q, K or V: D / 64 sub-tiles of 128 x 64
+    static constexpr int kQ = kRingBytes + kTcXOff;
+    static constexpr int kK = D == 64 ? kQ + 2 * kTile : 0;
+    static constexpr int kV = kK + 2 * kTile;
+    static constexpr uint32_t kS = 0, kO = 256, kP = D == 64 ? 384 : 0;                     // tensor-memory columns of tile 0 ...
+    static constexpr uint32_t kOStep = D, kPStep = D == 64 ? 64 : 128;                      // ... and to tile 1 (S: 128)
+};
+static_assert(AtMap<64>::kV + 2 * AtMap<64>::kTile <= kRingBytes + kWorkBytes, "attention tiles, head_dim 64");
+static_assert(AtMap<128>::kV + 2 * AtMap<128>::kTile <= kRingBytes && AtMap<128>::kQ + 2 * AtMap<128>::kTile <= kRingBytes + kWorkBytes, "attention tiles, head_dim 128");
 
-// instruction descriptors, kind::f16, fp32 accumulator, M = 128; operand format bits 7-9 / 10-12: 1 = bf16, 0 = fp16
-// (q, k, v -- and with them P -- are bf16, or fp16 when they are runtime-private activations)
-__device__ __forceinline__ uint32_t at_idesc_s(bool f16) {      // N = 128, A and B K-major
-    const uint32_t f = f16 ? 0u : 1u;
-    return (1u << 4) | (f << 7) | (f << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
-}
-__device__ __forceinline__ uint32_t at_idesc_o(bool f16) {      // N = 64, B MN-major
-    const uint32_t f = f16 ? 0u : 1u;
-    return (1u << 4) | (f << 7) | (f << 10) | (1u << 16) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
+__device__ __forceinline__ int at_blocks(const mk_op_desc* op, int qi, int t) {        // 128-key blocks of tile t (0: no such queries)
+    const int q0 = qi * 256 + t * 128;
+    if (q0 >= op->i[1]) return 0;
+    const int kend = op->i[6] ? min(op->i[2], q0 + 128) : op->i[2];
+    return (kend + 127) / 128;
 }
 
 // 2-D tiled bulk tensor copy global -> shared without a cache hint
@@ -81,278 +77,343 @@ __device__ __forceinline__ void tc_st32(uint32_t taddr, const float* v) {
         "r"(__float_as_uint(v[28])), "r"(__float_as_uint(v[29])), "r"(__float_as_uint(v[30])), "r"(__float_as_uint(v[31]))
         : "memory");
 }
-__device__ __forceinline__ void tc_mma_i(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// 16 words of this thread's lane (32 values of a 16-bit operand), not waited for
+__device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t* w) {
     asm volatile(
-        "{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]), "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]), "r"(w[8]), "r"(w[9]), "r"(w[10]),
+        "r"(w[11]), "r"(w[12]), "r"(w[13]), "r"(w[14]), "r"(w[15])
+        : "memory");
+}
+__device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// D = A B (+ D) with A in tensor memory
+__device__ __forceinline__ void tc_mma_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{ .reg .pred p; setp.ne.b32 p, %4, 0; tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p; }" ::"r"(tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
 
-// barrier of the two warps (w, w + 4) that share the query rows of tensor-memory quarter q
-__device__ __forceinline__ void at_pair_sync(int q) { asm volatile("bar.sync %0, 64;" ::"r"(2 + q) : "memory"); }
-
-// Tile requests and MMA issue of one instruction: one thread of the feeder warp.  Returns false when aborting.
-__device__ __forceinline__ bool attention_tc_feed(const Params& p, Ctrl* c, uint8_t* work, const mk_op_desc* op, int b, int h, int qi,
-                                                  int seq, uint32_t go_parity) {
-    constexpr int D = 64;
-    const int Sq = op->i[1], Sk = op->i[2], H = op->i[3], KVH = op->i[4];
-    const bool causal = op->i[6] != 0, f16 = op->i[8] == DT_F16;
-    const int hk = h / (H / KVH);
-    const int q0 = qi * 128;
-    const int kend = causal ? min(Sk, q0 + 128) : Sk;
-    const int nb = (kend + 127) / 128;
+// ---- feeder warp ---------------------------------------------------------------------------------------------------------------
+struct AtFeed {
+    uint32_t go = 0, granted = 0;        // parities of attn_go, ring_granted
+    uint32_t insts = 0, tiles = 0;       // instructions and K (V) tiles requested
+};
+// All lanes; lane 0 requests.  `first`: the CTA's previous instruction is not an attention of the same head_dim.  `told`: entry of
+// Ctrl::wide_info to use (shared with the tile GEMM).
+template <int D>
+__device__ __forceinline__ bool at_feed(const Params& p, Ctrl* c, uint8_t* ring, const mk_op_desc* op, const Inst& in, bool first, AtFeed& f,
+                                        uint32_t told) {
+    using M = AtMap<D>;
+    const int lane = threadIdx.x & 31;
+    const int Sq = op->i[1], Sk = op->i[2], hk = in.a1 / (op->i[3] / op->i[4]);
+    const int nb0 = at_blocks(op, in.a2, 0), nb1 = at_blocks(op, in.a2, 1), nb = max(nb0, nb1);
     const uint8_t* tmaps = reinterpret_cast<const uint8_t*>(op->ptr[11]);
     AttnBars* a = &c->attn;
-    // the compute warps have met the dependencies, initialised the barriers and (first time) allocated tensor memory;
-    // they may be busy with earlier instructions for a long time: twice the time limit, so that a stuck wait there reports first
-    if (!wait_barrier(p, c, &c->attn_go, go_parity, seq, WHERE_DEP, 2)) return false;
-    tc_fence_after();
+    bool ok = true;
+    if (first) {
+        // the compute warps may be busy with earlier instructions for a long time: twice the time limit, so that a stuck wait there reports first
+        if (lane == 0) ok = wait_barrier(p, c, &c->attn_go, f.go, in.seq, WHERE_DEP, 2);
+        f.go ^= 1u;
+        if (D == 128) {
+            if (lane == 0 && ok) ok = wait_barrier(p, c, &c->ring_granted, f.granted, in.seq, WHERE_RING_EMPTY, 2);
+            f.granted ^= 1u;
+        }
+        if (!__all_sync(0xffffffffu, ok)) return false;
+    }
+    for (int k = lane; k < in.nwait; k += 32) {
+        const int2 w = __ldg(p.waits + in.wait_off + k);
+        ok = wait_counter(p, c, w.x, w.y, in.seq) && ok;
+    }
+    if (!__all_sync(0xffffffffu, ok)) return false;
+    if (lane == 0) {
+        // the tiles' memory was last written through the generic proxy, and so were q, k and v, by other SMs
+        asm volatile("fence.proxy.async;" ::: "memory");
+        ok = wait_barrier(p, c, &a->q_free, (f.insts & 1u) ^ 1u, in.seq, WHERE_RING_EMPTY, 2);
+        if (ok) {
+            const int qtiles = in.a2 * 256 + 128 < Sq ? 2 : 1, qrow = in.a0 * Sq + in.a2 * 256;
+            mbar_arrive_expect_tx(&a->q_full, (uint32_t)(qtiles * M::kTile));
+            for (int t = 0; t < qtiles; ++t)
+                for (int s = 0; s < D / 64; ++s)
+                    tma_load_2d_plain(ring + M::kQ + t * M::kTile + s * kTcTileBytes, tmaps, in.a1 * D + s * 64, qrow + t * 128, &a->q_full);
+            c->wide_info[told & 3u] = make_int4(-(nb0 | nb1 << 15), D, op->i[8] == DT_F16 ? 1 : 0, in.seq);
+            mbar_arrive(&c->wide_told[told & 3u]);
+        }
+        const int krow = in.a0 * Sk;
+        for (int j = 0; j < nb && ok; ++j) {
+            const uint32_t n = f.tiles + (uint32_t)j, u = n & 1u, ph = (n >> 1) & 1u;
+            ok = wait_barrier(p, c, &a->k_empty[u], ph ^ 1u, in.seq, WHERE_RING_EMPTY, 2);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&a->k_full[u], (uint32_t)M::kTile);
+            for (int s = 0; s < D / 64; ++s)
+                tma_load_2d_plain(ring + M::kK + u * M::kTile + s * kTcTileBytes, tmaps + 128, hk * D + s * 64, krow + j * 128, &a->k_full[u]);
+            ok = wait_barrier(p, c, &a->v_empty[u], ph ^ 1u, in.seq, WHERE_RING_EMPTY, 2);
+            if (!ok) break;
+            mbar_arrive_expect_tx(&a->v_full[u], (uint32_t)M::kTile);
+            for (int s = 0; s < D / 64; ++s)
+                tma_load_2d_plain(ring + M::kV + u * M::kTile + s * kTcTileBytes, tmaps + 256, hk * D + s * 64, krow + j * 128, &a->v_full[u]);
+        }
+    }
+    ++f.insts;
+    f.tiles += (uint32_t)nb;
+    return __all_sync(0xffffffffu, ok) != 0;
+}
+
+// ---- issuer warp ---------------------------------------------------------------------------------------------------------------
+struct AtIssue {
+    uint32_t insts = 0, tiles = 0;       // instructions, K / V tiles
+    uint32_t blocks[2] = {0, 0};         // blocks of each tile (parities of s_full, p_full, pv_done)
+    uint32_t outs[2] = {0, 0};           // instructions that had the tile (parity of o_free)
+};
+// Every lane asks the barriers (their answers can differ while one completes: the vote makes the warp take one path).
+__device__ __forceinline__ bool at_ready(unsigned long long* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)) != 0; }
+// The whole warp polls, one elected lane issues.  Returns false when aborting.
+template <int D>
+__device__ __forceinline__ bool at_issue(const Params& p, Ctrl* c, uint8_t* ring, const int4& info, AtIssue& f) {
+    using M = AtMap<D>;
+    AttnBars* a = &c->attn;
+    const int nbt[2] = {(-info.x) & 0x7fff, (-info.x) >> 15};
+    const int nb = max(nbt[0], nbt[1]);
     const uint32_t tmem = *(volatile uint32_t*)&c->tmem_base;
-    uint8_t* qs = work + kAtQOff;
-    uint8_t* ks = work + kAtKOff;
-    uint8_t* vs = work + kAtVOff;
-    uint8_t* ps = work + kAtPOff;
-    // earlier instructions wrote the work area through the generic proxy
-    asm volatile("fence.proxy.async;" ::: "memory");
-    const int qrow = b * Sq + q0, krow = b * Sk;
-    mbar_arrive_expect_tx(&a->q_full, (uint32_t)kTcTileBytes);
-    tma_load_2d_plain(qs, tmaps, h * D, qrow, &a->q_full);
-    const uint64_t qd = tc_smem_desc(smem_u32(qs));
-    const uint64_t vd = tc_smem_desc(smem_u32(vs));       // V as MN-major operand: 8-key groups 1024 bytes apart; 16 keys further = 2048 bytes
-    const uint64_t pd0 = tc_smem_desc(smem_u32(ps)), pd1 = tc_smem_desc(smem_u32(ps + kTcTileBytes));
-    const uint32_t idesc_s = at_idesc_s(f16), idesc_o = at_idesc_o(f16);
-    // Block j uses K and S buffer j & 1, for the (j >> 1)-th time: a "full" barrier of a buffer completes with parity
-    // (j >> 1) & 1; before the buffer is used again its "empty" barrier must have completed with the parity of the previous use.
-    int kl = 0, vl = 0, si = 0, pi = 0;                   // K tiles requested, V tiles requested, S products issued, P V products issued
-    bool q_ready = false;
+    const uint32_t fmt = info.z ? 0u : 1u;                    // operand format: 0 fp16, 1 bf16
+    // fp32 accumulator, M = 128; S: N = 128, both operands K-major; O: N = D, B MN-major
+    const uint32_t base = (1u << 4) | (fmt << 7) | (fmt << 10) | ((128u >> 4) << 24);
+    const uint32_t idesc_s = base | ((128u >> 3) << 17), idesc_o = base | (1u << 16) | (((uint32_t)D >> 3) << 17);
+    const uint64_t d0 = tc_smem_desc(smem_u32(ring));
+    // MN-major: 8-key groups 1024 bytes apart (the descriptor's stride), 64-column sub-tiles 16 KB apart (its leading offset)
+    const uint64_t v0 = D == 64 ? d0 : d0 - (1ull << 16) + ((uint64_t)(kTcTileBytes >> 4) << 16);
+    int si[2] = {0, 0}, pf[2] = {0, 0}, pi[2] = {0, 0};       // S issued, softmax blocks handed over, P V issued
+    bool q_ready = false, q_done = false;
     uint32_t idle = 0;
     unsigned long long t0 = 0;
-    while (pi < nb) {
+    while (pi[0] < nbt[0] || pi[1] < nbt[1]) {
         bool progress = false;
-        if (kl < nb && (kl < 2 || mbar_test_wait(&a->k_empty[kl & 1], (uint32_t)((kl - 2) >> 1) & 1u))) {
-            const int u = kl & 1;
-            mbar_arrive_expect_tx(&a->k_full[u], (uint32_t)kTcTileBytes);
-            tma_load_2d_plain(ks + u * kTcTileBytes, tmaps + 128, hk * D, krow + kl * 128, &a->k_full[u]);
-            ++kl;
-            progress = true;
-        }
-        if (vl < nb && (vl == 0 || mbar_test_wait(&a->v_empty, (uint32_t)(vl - 1) & 1u))) {
-            mbar_arrive_expect_tx(&a->v_full, (uint32_t)kTcTileBytes);
-            tma_load_2d_plain(vs, tmaps + 256, hk * D, krow + vl * 128, &a->v_full);
-            ++vl;
-            progress = true;
-        }
-        if (!q_ready) q_ready = mbar_test_wait(&a->q_full, 0u);
-        // S of block si (at most one block ahead of the P V products), into tensor-memory buffer si & 1
-        if (q_ready && si < nb && si <= pi + 1 && si < kl && mbar_test_wait(&a->k_full[si & 1], (uint32_t)(si >> 1) & 1u) &&
-            (si < 2 || mbar_test_wait(&a->s_empty[si & 1], (uint32_t)((si - 2) >> 1) & 1u))) {
-            const int u = si & 1;
-            tc_fence_after();
-            const uint64_t kd = tc_smem_desc(smem_u32(ks + u * kTcTileBytes));
+        if (!q_ready) q_ready = at_ready(&a->q_full, f.insts & 1u);
 #pragma unroll
-            for (int k16 = 0; k16 < D / 16; ++k16) tc_mma_i(tmem + kAtSCol + 128 * u, qd + 2 * k16, kd + 2 * k16, idesc_s, k16 ? 1u : 0u);
-            tc_commit(&a->k_empty[u]);
-            tc_commit(&a->s_full[u]);
-            ++si;
-            progress = true;
-        }
-        if (pi < si && pi < vl && mbar_test_wait(&a->p_full, (uint32_t)pi & 1u) && mbar_test_wait(&a->v_full, (uint32_t)pi & 1u)) {
-            tc_fence_after();
+        for (int t = 0; t < 2; ++t) {
+            // S of the tile's next block: K there, and the scores of the block before read (head_dim 128: and multiplied, P lies over them)
+            if (q_ready && si[t] < nbt[t] && si[t] <= pf[t]) {
+                const uint32_t n = f.tiles + (uint32_t)si[t], u = n & 1u;
+                bool go = at_ready(&a->k_full[u], (n >> 1) & 1u);
+                if (D == 128 && f.blocks[t] + (uint32_t)si[t] > 0)
+                    go = go && pi[t] == si[t] && at_ready(&a->pv_done[t], (f.blocks[t] + (uint32_t)si[t] - 1u) & 1u);
+                if (go) {
+                    tc_fence_after();
+                    const uint64_t qd = d0 + (uint32_t)((M::kQ + t * M::kTile) >> 4), kd = d0 + ((uint32_t)M::kK >> 4) + u * (uint32_t)(M::kTile >> 4);
+                    const bool alone = si[t] >= nbt[t ^ 1];                // the other tile does not read this K tile
+                    if (elect_one()) {
 #pragma unroll
-            for (int k16 = 0; k16 < 8; ++k16) {
-                const uint64_t pd = (k16 < 4 ? pd0 : pd1) + 2 * (k16 & 3);       // 16 keys further inside a 64-key tile: 32 bytes
-                tc_mma_i(tmem + kAtOCol, pd, vd + 128 * k16, idesc_o, (pi > 0 || k16 > 0) ? 1u : 0u);   // 16 keys of V: 2048 bytes
+                        for (int k16 = 0; k16 < D / 16; ++k16) {
+                            const uint32_t off = (k16 & 3) * 2 + (k16 >> 2) * (kTcTileBytes >> 4);
+                            tc_mma(tmem + M::kS + 128 * t, qd + off, kd + off, idesc_s, k16 ? 1u : 0u);
+                        }
+                        tc_commit(&a->s_full[t]);
+                        tc_commit(&a->k_empty[u]);
+                        if (alone) tc_commit(&a->k_empty[u]);
+                    }
+                    __syncwarp();
+                    ++si[t];
+                    progress = true;
+                }
             }
-            tc_commit(&a->v_empty);
-            tc_commit(&a->pv_done);
-            ++pi;
-            progress = true;
+            if (pf[t] < si[t] && at_ready(&a->p_full[t], (f.blocks[t] + (uint32_t)pf[t]) & 1u)) { ++pf[t]; progress = true; }
+            if (pi[t] < pf[t]) {
+                const uint32_t n = f.tiles + (uint32_t)pi[t], u = n & 1u;
+                // (the first P V overwrites O: the compute warps must have read the previous instruction's)
+                bool go = at_ready(&a->v_full[u], (n >> 1) & 1u);
+                if (pi[t] == 0 && f.outs[t] > 0) go = go && at_ready(&a->o_free[t], (f.outs[t] - 1u) & 1u);
+                if (go) {
+                    tc_fence_after();
+                    const uint64_t vd = v0 + ((uint32_t)M::kV >> 4) + u * (uint32_t)(M::kTile >> 4);
+                    const bool alone = pi[t] >= nbt[t ^ 1];
+                    const uint32_t acc = pi[t] > 0 ? 1u : 0u;
+                    if (elect_one()) {
+#pragma unroll
+                        for (int k16 = 0; k16 < 8; ++k16)                  // 16 keys: 8 columns of P, 2048 bytes of V
+                            tc_mma_ta(tmem + M::kO + M::kOStep * t, tmem + M::kP + M::kPStep * t + 8 * k16, vd + 128 * k16, idesc_o, acc | (k16 ? 1u : 0u));
+                        tc_commit(&a->pv_done[t]);
+                        tc_commit(&a->v_empty[u]);
+                        if (alone) tc_commit(&a->v_empty[u]);
+                    }
+                    __syncwarp();
+                    ++pi[t];
+                    progress = true;
+                }
+            }
+        }
+        if (!q_done && si[0] == nbt[0] && si[1] == nbt[1]) {               // every product that reads Q has been issued
+            if (elect_one()) tc_commit(&a->q_free);
+            __syncwarp();
+            q_done = true;
         }
         if (progress) { idle = 0; t0 = 0; continue; }
-        if ((++idle & 1023u) == 0) {                       // nothing to do: the time limit of every other wait applies
-            if (*(volatile int*)&c->abort) return false;
-            if (ld_volatile(&p.status[MK_ST_CODE]) != 0) { c->abort = 1; return false; }
+        if ((++idle & 1023u) == 0) {                                       // nothing to do: the time limit of every other wait applies (twice: role)
+            bool stop = *(volatile int*)&c->abort != 0;
+            if (!stop && ld_volatile(&p.status[MK_ST_CODE]) != 0) { c->abort = 1; stop = true; }
             const unsigned long long now = globaltimer();
             if (t0 == 0) t0 = now;
-            else if (now - t0 > p.timeout_ns) {
-                report(p, c, MK_DEV_TIMEOUT_BARRIER, seq, WHERE_RING_FULL, (int)(&a->p_full - c->full), pi, si);
-                return false;
+            else if (!stop && now - t0 > 2 * p.timeout_ns) {
+                report(p, c, MK_DEV_TIMEOUT_BARRIER, info.w, WHERE_RING_FULL, (int)(&a->p_full[0] - c->full), pi[0], si[0]);
+                stop = true;
             }
+            if (__any_sync(0xffffffffu, stop)) return false;
         }
+    }
+    ++f.insts;
+    f.tiles += (uint32_t)nb;
+    for (int t = 0; t < 2; ++t) {
+        f.blocks[t] += (uint32_t)nbt[t];
+        f.outs[t] += nbt[t] > 0 ? 1u : 0u;
     }
     return true;
 }
 
-// All compute threads call this (the instruction's dependencies are met).  Returns 0, or -1 when aborting.
-__device__ __forceinline__ int op_attention_tc(const Params& p, Ctrl* c, uint8_t* work, const mk_op_desc* op, int b, int h, int qi,
-                                               int seq) {
-    constexpr int D = 64;
-    constexpr float NEG_INF = -__builtin_huge_valf();
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int Sq = op->i[1], Sk = op->i[2], odt = op->i[7];
-    const bool causal = op->i[6] != 0, f16 = op->i[8] == DT_F16;
-    const int q0 = qi * 128;
-    const int kend = causal ? min(Sk, q0 + 128) : Sk;
-    const int nb = (kend + 127) / 128;                                   // 128-key blocks
-    AttnBars* a = &c->attn;
-
-    // ---- tensor memory (shared with the tile GEMM; allocated once per launch) and this instruction's barriers ----
-    const bool first_use = *(volatile uint32_t*)&c->tmem_ready == 0;     // (written behind the barrier below: the same for every thread)
-    if (first_use) {
-        if (warp == 0) {
-            __syncwarp();          // (.sync.aligned: the whole warp, converged)
+// ---- compute warps -------------------------------------------------------------------------------------------------------------
+__device__ __forceinline__ void at_begin_run(Ctrl* c) {
+    const int t = threadIdx.x;
+    if (*(volatile uint32_t*)&c->tmem_ready == 0) {                       // (a word that only changes behind a barrier: see op_gemm_tc)
+        if (t < 32) {
+            __syncwarp();
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&c->tmem_base)), "r"(kTcCols)
                          : "memory");
         }
         tc_fence_before();
+        compute_sync();
+        tc_fence_after();
+        if (t == 0) c->tmem_ready = 1;
     }
-    if (t == 0) {
-        mbar_init(&a->q_full, 1);
-        for (int u = 0; u < 2; ++u) {
-            mbar_init(&a->k_full[u], 1); mbar_init(&a->k_empty[u], 1);
-            mbar_init(&a->s_full[u], 1); mbar_init(&a->s_empty[u], kComputeWarps);
-        }
-        mbar_init(&a->v_full, 1); mbar_init(&a->v_empty, 1);
-        mbar_init(&a->p_full, kComputeWarps); mbar_init(&a->pv_done, 1);
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    compute_sync();
-    tc_fence_after();
-    if (t == 0 && first_use) c->tmem_ready = 1;
-    if (t == 0) mbar_arrive(&c->attn_go);                               // the feeding thread (feeder warp) may start
-    const uint32_t tmem = *(volatile uint32_t*)&c->tmem_base;
-    uint8_t* ps = work + kAtPOff;
-    __nv_bfloat16* xb = reinterpret_cast<__nv_bfloat16*>(work);          // 512 bytes in front of the tiles: 2 x 128 row maxima (bf16),
-    float* xf = reinterpret_cast<float*>(work);                          // at the end 128 partial row sums
-    int ok = 1;
+    if (t == 0) mbar_arrive(&c->attn_go);
+}
 
-    // ---- softmax, rescale, read-back: thread = (query row r, column half) ----
-    const int qd = warp & 3, half = warp >> 2;
-    const int r = qd * 32 + lane;
-    const int qrow = q0 + r;                                             // position in the sequence
-    const uint32_t tl = tmem + ((uint32_t)(qd * 32) << 16);
+// Softmax and output of one instruction.  (A wait that gives up has raised Ctrl::abort; the barrier of publish() makes that known
+// to every thread.)
+template <int D>
+__device__ __forceinline__ void op_attention_tc(const Params& p, Ctrl* c, const mk_op_desc* op, int b, int h, int qi, int seq) {
+    using M = AtMap<D>;
+    constexpr float NEG_INF = -__builtin_huge_valf();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = warp >> 2, qd = warp & 3;
+    const int Sq = op->i[1], Sk = op->i[2], odt = op->i[7];
+    const bool causal = op->i[6] != 0, f16 = op->i[8] == DT_F16;
+    const int q0 = qi * 256 + t * 128, qrow = q0 + qd * 32 + lane;         // position in the sequence
+    const int kend = causal ? min(Sk, q0 + 128) : Sk;
+    const int nb = at_blocks(op, qi, t);
+    AttnBars* a = &c->attn;
+    const uint32_t turn = *(volatile uint32_t*)&c->at_turn & 1u;
+    const uint32_t base = c->at_blocks[turn][t];                           // blocks of this tile so far
+    if ((threadIdx.x & 127) == 0) c->at_blocks[turn ^ 1u][t] = base + (uint32_t)nb;
+    phase_mark(p, c, 0);
+    if (nb == 0) return;
+    const uint32_t tl = *(volatile uint32_t*)&c->tmem_base + ((uint32_t)(qd * 32) << 16);
+    const uint32_t scol = tl + M::kS + 128 * t, pcol = tl + M::kP + M::kPStep * t, ocol = tl + M::kO + M::kOStep * t;
     const float sl2 = op->f[0] * kLog2e;
     float m_used = NEG_INF, l = 0.f;
-    uint8_t* prow = ps + half * kTcTileBytes + r * 128;                  // this thread's 64 keys: row r of P tile `half`
+    bool ok = true;
+#pragma unroll 1
     for (int j = 0; j < nb; ++j) {
-        const int u = j & 1;
-        ok = wait_barrier(p, c, &a->s_full[u], (uint32_t)(j >> 1) & 1u, seq, WHERE_COMBINE) && ok;
+        ok = wait_barrier(p, c, &a->s_full[t], (base + (uint32_t)j) & 1u, seq, WHERE_COMBINE, 2) && ok;
+        __syncwarp();
         tc_fence_after();
-        if (p.trace_cap > 0 && t == 0 && j == 0) c->t_phase[0] = (long long)globaltimer();      // first scores ready
-        // Two passes over the thread's 64 scores, 32 at a time (held all at once they do not fit the kernel's
-        // 168-register cap beside the exponentials: 80 registers spilled).  Tensor memory is read twice instead.
-        const uint32_t scol = tl + kAtSCol + 128 * u + half * 64;
-        const int key0 = j * 128 + half * 64;
-        const bool edge = key0 + 64 > kend || (causal && key0 + 64 > q0);      // a block with masked keys: those count as -inf
+        const int key0 = j * 128;
+        const bool edge = key0 + 128 > kend || (causal && key0 + 128 > q0);    // a block with masked keys: those count as -inf
+        const int last = causal ? min(kend - 1, qrow) : kend - 1;              // last key of this row
         float m4[4] = {NEG_INF, NEG_INF, NEG_INF, NEG_INF};
 #pragma unroll 1
-        for (int ch = 0; ch < 2; ++ch) {
+        for (int ch = 0; ch < 4; ++ch) {
             float s[32];
             tc_ld32(scol + ch * 32, s);
             if (edge) {
+                const int n = last - (key0 + ch * 32);                         // this row's last live score of the chunk
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                    const int key = key0 + ch * 32 + e;
-                    if (key >= kend || (causal && key > qrow)) s[e] = NEG_INF;
-                }
+                for (int e = 0; e < 32; ++e) s[e] = e <= n ? s[e] : NEG_INF;
             }
 #pragma unroll
             for (int e = 0; e < 32; e += 4) {
                 m4[0] = fmaxf(m4[0], s[e]); m4[1] = fmaxf(m4[1], s[e + 1]); m4[2] = fmaxf(m4[2], s[e + 2]); m4[3] = fmaxf(m4[3], s[e + 3]);
             }
         }
-        // the row's maximum over both halves, as a value both threads of the row compute alike
-        const __nv_bfloat16 mine = __float2bfloat16_rn(fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * sl2);
-        xb[half * 128 + r] = mine;
-        at_pair_sync(qd);
-        const float mx = fmaxf(__bfloat162float(mine), __bfloat162float(xb[(half ^ 1) * 128 + r]));
-        at_pair_sync(qd);                                                // (the slot is written again in the next block)
+        const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * sl2;
         // lazy rescale: keep the old maximum unless the new one is more than 2^8 above it
         float factor = 1.f;
         if (mx > m_used + kAtRescale || (m_used == NEG_INF && mx != NEG_INF)) {
             factor = m_used == NEG_INF ? 0.f : ex2(m_used - mx);
             m_used = mx;
         }
-        // the P buffer and (for a rescale) O are free once the previous block's P V has completed
-        if (j > 0) ok = wait_barrier(p, c, &a->pv_done, (uint32_t)(j - 1) & 1u, seq, WHERE_COMBINE) && ok;
+        // P's place and (for a rescale) O are free once the previous block's P V has completed
+        if (j > 0) ok = wait_barrier(p, c, &a->pv_done[t], (base + (uint32_t)j - 1u) & 1u, seq, WHERE_COMBINE, 2) && ok;
+        __syncwarp();
         tc_fence_after();
-        if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {           // (both warps of a row see the same factors)
+        if (j > 0 && __any_sync(0xffffffffu, factor != 1.f)) {
             l *= factor;
-            float o[32];
-            tc_ld32(tl + kAtOCol + half * 32, o);
+#pragma unroll 1
+            for (int ch = 0; ch < D / 32; ++ch) {
+                float o[32];
+                tc_ld32(ocol + ch * 32, o);
 #pragma unroll
-            for (int e = 0; e < 32; ++e) o[e] *= factor;
-            tc_st32(tl + kAtOCol + half * 32, o);
+                for (int e = 0; e < 32; ++e) o[e] *= factor;
+                tc_st32(ocol + ch * 32, o);
+            }
         }
-        // P = 2^(s * scale - m), rounded to the operand type, into the swizzled K-major tile; partial row sums
-        const float mm = m_used == NEG_INF ? 0.f : m_used;               // (a row without a live key so far: every s is -inf)
+        // P = 2^(s * scale - m), rounded to the operand type; row sum
+        const float mm = m_used == NEG_INF ? 0.f : m_used;                     // (a row without a live key so far: every s is -inf)
         float l4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
-        for (int ch = 0; ch < 2; ++ch) {
+        for (int ch = 0; ch < 4; ++ch) {
             float s[32];
             tc_ld32(scol + ch * 32, s);
             if (edge) {
+                const int n = last - (key0 + ch * 32);
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                    const int key = key0 + ch * 32 + e;
-                    if (key >= kend || (causal && key > qrow)) s[e] = NEG_INF;           // 2^-inf = 0
-                }
+                for (int e = 0; e < 32; ++e) s[e] = e <= n ? s[e] : NEG_INF;   // 2^-inf = 0
             }
+            uint32_t w[16];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {                                // 8 keys = one 16-byte chunk
-                float pe[8];
-#pragma unroll
-                for (int e = 0; e < 8; ++e) {
-                    pe[e] = ex2(fmaf(s[q * 8 + e], sl2, -mm));
-                    l4[e & 3] += pe[e];
-                }
-                uint4 w;
-                if (f16) w = make_uint4(pack2h(pe[0], pe[1]), pack2h(pe[2], pe[3]), pack2h(pe[4], pe[5]), pack2h(pe[6], pe[7]));
-                else w = make_uint4(pack2(pe[0], pe[1]), pack2(pe[2], pe[3]), pack2(pe[4], pe[5]), pack2(pe[6], pe[7]));
-                *reinterpret_cast<uint4*>(prow + (((ch * 4 + q) ^ (r & 7)) << 4)) = w;
+            for (int e = 0; e < 32; e += 2) {
+                const float p0 = ex2(fmaf(s[e], sl2, -mm)), p1 = ex2(fmaf(s[e + 1], sl2, -mm));
+                l4[(e >> 1) & 1] += p0;
+                l4[2 + ((e >> 1) & 1)] += p1;
+                s[e] = p0; s[e + 1] = p1;
             }
+            if (f16) {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) w[e] = pack2h(s[2 * e], s[2 * e + 1]);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 16; ++e) w[e] = pack2(s[2 * e], s[2 * e + 1]);
+            }
+            tc_st16(pcol + ch * 16, w);                                        // (head_dim 128: over scores already read)
         }
         l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
-        // S has been read (the next block's S may overwrite it); P is in shared memory for the tensor core
+        tc_wait_st();
         tc_fence_before();
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncwarp();
-        if (lane == 0) {
-            mbar_arrive(&a->s_empty[u]);
-            mbar_arrive(&a->p_full);
-        }
+        if (lane == 0) mbar_arrive(&a->p_full[t]);                             // S read, P written
     }
-    if (p.trace_cap > 0 && t == 0) c->t_phase[1] = (long long)globaltimer();                        // last P handed over
+    phase_mark(p, c, 1);                                                       // last P handed over
     // ---- out = O / l ----
-    if (nb > 0) ok = wait_barrier(p, c, &a->pv_done, (uint32_t)(nb - 1) & 1u, seq, WHERE_COMBINE) && ok;
+    ok = wait_barrier(p, c, &a->pv_done[t], (base + (uint32_t)nb - 1u) & 1u, seq, WHERE_COMBINE, 2) && ok;
+    __syncwarp();
     tc_fence_after();
-    if (half == 1) xf[r] = l;
-    at_pair_sync(qd);
-    if (half == 0) { l += xf[r]; xf[r] = l; }
-    at_pair_sync(qd);
-    if (half == 1) l = xf[r];
     const float inv = l == 0.f ? 0.f : rcp(l);
-    {
-        uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[3]) + (((long long)b * Sq + qrow) * op->ld[3] + h * D + half * 32) * 2;
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[3]) + (((long long)b * Sq + qrow) * op->ld[3] + h * D) * 2;
+#pragma unroll 1
+    for (int ch = 0; ch < D / 32; ++ch) {
         float o[32];
-        if (nb > 0) {
-            tc_ld32(tl + kAtOCol + half * 32, o);
-        } else {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) o[e] = 0.f;
+        tc_ld32(ocol + ch * 32, o);
+        if (ch == D / 32 - 1) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&a->o_free[t]);
         }
         if (ok && qrow < Sq) {
 #pragma unroll
             for (int e = 0; e < 32; e += 8)
-                *reinterpret_cast<uint4*>(O + e * 2) =
+                *reinterpret_cast<uint4*>(O + (ch * 32 + e) * 2) =
                     make_uint4(pack2t(odt, o[e] * inv, o[e + 1] * inv), pack2t(odt, o[e + 2] * inv, o[e + 3] * inv),
                                pack2t(odt, o[e + 4] * inv, o[e + 5] * inv), pack2t(odt, o[e + 6] * inv, o[e + 7] * inv));
         }
+        __syncwarp();
     }
-    tc_fence_before();
-    const bool aborting = compute_sync_or(!ok || *(volatile int*)&c->abort);
-    phase_mark(p, c, 2);                                                                               // output written
-    return aborting ? -1 : 0;
+    phase_mark(p, c, 2);                                                       // output written
 }
 
 }  // namespace mk

@@ -9,7 +9,7 @@
 //   weights      producer warp -> one 32 KB copy per k-tile (op_gemv_common.cuh), as early as a slot is free
 //   activations  feeder warp (wide_feed): waits for the instruction's dependencies itself, then one bulk tensor copy of
 //                256 rows x 64 columns per k-tile; rows beyond M are zero-filled
-//   MMA          issuer warp, one thread (wide_issuer): waits for a stage (armed once by each loader), 4 + 4 instructions, one commit.
+//   MMA          issuer warp, one thread (wide_issue): waits for a stage (armed once by each loader), 4 + 4 instructions, one commit.
 //                It is told what to run by the feeder through Ctrl::wide_info and never touches global memory.
 //   epilogue     the compute warps: warp w owns rows 32 (w & 3) .. +31 of accumulator w >> 2; it reads its 32 x 256 part, hands
 //                the accumulator back and writes the rows from registers while the next tile's main loop runs
@@ -96,84 +96,81 @@ __device__ __forceinline__ void wide_feed_end(Ctrl* c, const WideFeed& f) {
 // The whole warp walks the loop and one elected lane issues: under a branch that only one lane takes, the compiler builds each
 // instruction's operands in ordinary registers and moves them over one by one, and an N = 128 instruction (64 cycles of the tensor
 // pipe) then takes 100 cycles to issue instead of 85 (measured stand-alone; N = 256, 128 cycles, is not affected).
-__device__ __forceinline__ bool elect_one() {
-    uint32_t p;
-    asm volatile("{ .reg .pred q; elect.sync _|q, 0xffffffff; selp.u32 %0, 1, 0, q; }" : "=r"(p));
-    return p != 0;
-}
 __device__ __forceinline__ bool issuer_wait(const Params& p, Ctrl* c, unsigned long long* bar, uint32_t parity, int seq, int where, unsigned patience) {
     const bool ok = wait_barrier(p, c, bar, parity, seq, where, patience);
     return __all_sync(0xffffffffu, ok) != 0;
 }
-__device__ __forceinline__ void wide_issuer(const Params& p, Ctrl* c, uint8_t* ring) {
+struct WideIssue {
+    uint32_t slot[2] = {0, 0}, phase[2] = {0, 0};      // position in the stages of each kind
+    uint32_t count = 0;                                 // instructions
+};
+// The MMAs of one instruction.  Returns false when aborting.
+__device__ __forceinline__ bool wide_issue(const Params& p, Ctrl* c, uint8_t* ring, const int4& info, WideIssue& f) {
     const uint64_t d0 = tc_smem_desc(smem_u32(ring));
-    uint32_t slot[2] = {0, 0}, phase[2] = {0, 0};
-    for (uint32_t n = 0;; ++n) {
-        if (!issuer_wait(p, c, &c->wide_told[n & 3u], (n >> 2) & 1u, 0, WHERE_DEP, 4)) return;
-        const int4 info = c->wide_info[n & 3u];
-        const int nk = info.x;
-        if (nk <= 0) return;
-        const bool both = (info.y & 15) == 2;                // rows 128..255 of the tile exist
-        const uint32_t idesc = tc_idesc_n(info.z != 0, 128u * (uint32_t)(info.y >> 4));
-        const uint32_t tmem = *(volatile uint32_t*)&c->tmem_base;
-        const int kind = (info.y >> 4) == 2 ? 0 : 1;
-        uint32_t acc = 0, s = slot[kind], ph = phase[kind];
-        for (int kt = 0; kt < nk; ++kt) {
-            if (!issuer_wait(p, c, &c->ww_full[kind][s], ph, info.w, WHERE_RING_FULL, 2)) return;
-            if (kt == 0) {
-                if (!issuer_wait(p, c, &c->wacc_empty[0], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return;
-                // (the two halves of a 256-column tile are issued one after the other: the first may start before the second's
-                // accumulator has been read)
-                if (kind && !issuer_wait(p, c, &c->wacc_empty[1], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return;
-            }
-            tc_fence_after();
-            const uint64_t ad = d0 + (uint32_t)(wide_xoff((int)s) >> 4), bd = d0 + (uint32_t)(wide_woff(kind, (int)s) >> 4);
-            if (kind) {
-                // N = 128: an instruction into the accumulator the previous one wrote starts late, so the two accumulators take turns
-                if (elect_one()) {
-                    if (both) {
+    const int nk = info.x;
+    const uint32_t n = f.count;
+    const bool both = (info.y & 15) == 2;                // rows 128..255 of the tile exist
+    const uint32_t idesc = tc_idesc_n(info.z != 0, 128u * (uint32_t)(info.y >> 4));
+    const uint32_t tmem = *(volatile uint32_t*)&c->tmem_base;
+    const int kind = (info.y >> 4) == 2 ? 0 : 1;
+    uint32_t acc = 0, s = f.slot[kind], ph = f.phase[kind];
+    for (int kt = 0; kt < nk; ++kt) {
+        if (!issuer_wait(p, c, &c->ww_full[kind][s], ph, info.w, WHERE_RING_FULL, 2)) return false;
+        if (kt == 0) {
+            if (!issuer_wait(p, c, &c->wacc_empty[0], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return false;
+            // (the two halves of a 256-column tile are issued one after the other: the first may start before the second's
+            // accumulator has been read)
+            if (kind && !issuer_wait(p, c, &c->wacc_empty[1], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return false;
+        }
+        tc_fence_after();
+        const uint64_t ad = d0 + (uint32_t)(wide_xoff((int)s) >> 4), bd = d0 + (uint32_t)(wide_woff(kind, (int)s) >> 4);
+        if (kind) {
+            // N = 128: an instruction into the accumulator the previous one wrote starts late, so the two accumulators take turns
+            if (elect_one()) {
+                if (both) {
 #pragma unroll
-                        for (int k16 = 0; k16 < 4; ++k16) {
-                            tc_mma(tmem, ad + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
-                            tc_mma(tmem + 256, ad + (kTcTileBytes >> 4) + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
-                        }
-                    } else {
-#pragma unroll
-                        for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem, ad + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+                    for (int k16 = 0; k16 < 4; ++k16) {
+                        tc_mma(tmem, ad + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+                        tc_mma(tmem + 256, ad + (kTcTileBytes >> 4) + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
                     }
-                    if (kt == nk - 1) tc_commit(&c->wacc_full[0]);
-                    tc_commit(&c->ww_empty[kind][s]);
-                }
-            } else {
-                if (elect_one()) {
+                } else {
 #pragma unroll
                     for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem, ad + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
-                    if (kt == nk - 1) tc_commit(&c->wacc_full[0]);
                 }
-                if (kt == 0) {
-                    if (!issuer_wait(p, c, &c->wacc_empty[1], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return;
-                    tc_fence_after();
-                }
-                if (elect_one()) {
-                    if (both) {
-#pragma unroll
-                        for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem + 256, ad + (kTcTileBytes >> 4) + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
-                    }
-                    tc_commit(&c->ww_empty[kind][s]);
-                }
+                if (kt == nk - 1) tc_commit(&c->wacc_full[0]);
+                tc_commit(&c->ww_empty[kind][s]);
             }
-            __syncwarp();
-            acc = 1;
-            if (++s == (uint32_t)wide_stages(kind)) { s = 0; ph ^= 1u; }
-        }
-        slot[kind] = s;
-        phase[kind] = ph;
-        if (elect_one()) {
-            tc_commit(&c->wacc_full[1]);
-            if (p.trace_cap > 0) c->t_phase[1] = (long long)globaltimer();
+        } else {
+            if (elect_one()) {
+#pragma unroll
+                for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem, ad + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+                if (kt == nk - 1) tc_commit(&c->wacc_full[0]);
+            }
+            if (kt == 0) {
+                if (!issuer_wait(p, c, &c->wacc_empty[1], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return false;
+                tc_fence_after();
+            }
+            if (elect_one()) {
+                if (both) {
+#pragma unroll
+                    for (int k16 = 0; k16 < 4; ++k16) tc_mma(tmem + 256, ad + (kTcTileBytes >> 4) + 2 * k16, bd + 2 * k16, idesc, acc | (k16 ? 1u : 0u));
+                }
+                tc_commit(&c->ww_empty[kind][s]);
+            }
         }
         __syncwarp();
+        acc = 1;
+        if (++s == (uint32_t)wide_stages(kind)) { s = 0; ph ^= 1u; }
     }
+    f.slot[kind] = s;
+    f.phase[kind] = ph;
+    if (elect_one()) {
+        tc_commit(&c->wacc_full[1]);
+        if (p.trace_cap > 0) c->t_phase[1] = (long long)globaltimer();
+    }
+    __syncwarp();
+    ++f.count;
+    return true;
 }
 
 // ---- compute warps: epilogue ---------------------------------------------------------------------------------------------------

@@ -50,8 +50,4 @@ __device__ int mk_run_gemm_wide(const Params& p, int idx, int slot) {
     }
 }
 
-__device__ void mk_wide_issuer(const Params& p) {
-    const SmemMap m = smem_map();
-    wide_issuer(p, m.ctrl, m.ring);
-}
 }  // namespace mk

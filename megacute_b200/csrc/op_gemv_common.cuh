@@ -65,6 +65,7 @@ struct StageCursor {
     // tile GEMM on the tcgen05 path (op_gemm_tc.cuh): the weight k-tiles [kt, nk) of the instruction
     // are still to be copied, through the tensor map `wmap`, from coordinates (kbeg + 64 kt, n0)
     bool gemm;
+    bool attn;                   // tcgen05 attention of head_dim 128: its K and V tiles use the ring's memory
     int kt, nk, kbeg, n0, wide;
     bool reread;                 // the weight tiles are read again and again, by the instructions of many row tiles (more than two)
     const void* wmap;
@@ -95,7 +96,7 @@ struct StageCursor {
                 const int posv = reinterpret_cast<const volatile int*>(op->ptr[3])[(long long)in.a0 * op->i[12]];
                 int k_begin, k_end;
                 kv_split_range(fused ? posv : posv + 1, S, in.a2, k_begin, k_end);
-                gemm = false; kv = true; seq = in.seq;
+                gemm = false; kv = true; attn = false; seq = in.seq;
                 kv_t = 0; kv_nt = (k_end - k_begin + kKvTileRows - 1) / kKvTileRows; kv_which = 0;
                 kv_rb = KVH * 64 * 2;
                 kv_gated = !fused;
@@ -106,6 +107,8 @@ struct StageCursor {
                 if (kv_nt > 0 || kv_gated) return;     // (a gated instruction without tiles still consumes its kv_go)
                 continue;
             }
+            attn = is_attention_tc(op) && op->i[5] == 128;
+            if (attn) { gemm = false; kv = false; seq = in.seq; return; }
             if (op->kind == MK_OP_GEMM && op->ptr[11]) {
                 // a 256-row output tile (i 11; slots of its own) takes one or two 128-row weight tiles (i 10) per k-tile
                 const int kc = op->i[2] / op->i[4];
@@ -140,7 +143,7 @@ struct StageCursor {
     }
     __device__ __forceinline__ bool valid(const Params& p) const { return idx < p.n_insts; }
     __device__ __forceinline__ void advance(const Params& p) {
-        if (gemm || kv) {                             // (the L2 prefetch cursor: whole instruction at once)
+        if (gemm || kv || attn) {                     // (the L2 prefetch cursor: whole instruction at once)
             idx += gridDim.x;
             seek(p);
             return;
@@ -155,7 +158,7 @@ struct StageCursor {
     __device__ __forceinline__ void piece(int lane, const __nv_bfloat16*& src, int& bytes, int& dst_off) const {
         const bool swi = flags & GEMV_F_SWIGLU;
         src = w; bytes = 0; dst_off = 0;
-        if (gemm || kv) return;
+        if (gemm || kv || attn) return;
         if (flags & GEMV_F_UNITS) {
             const int r = lane & 15;
             const int o = o0 + (swi ? g >> 1 : g) * 16 + r;
@@ -193,7 +196,8 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
     uint32_t wphase = 0;
     int kvslot = 0;
     uint32_t kvphase = 0, kvgo = 0;
-    enum { MODE_STAGES = 0, MODE_WTILES = 1, MODE_KVTILES = 2, MODE_WWIDE = 3 };     // (MODE_WWIDE + kind: 256-row tiles)
+    enum { MODE_STAGES = 0, MODE_WTILES = 1, MODE_KVTILES = 2, MODE_ATTN = 3, MODE_WWIDE = 4 };     // (MODE_WWIDE + kind: 256-row tiles)
+    uint32_t returned = 0;                           // parity of ring_returned
     int wwslot[2] = {0, 0};
     uint32_t wwphase[2] = {0, 0}, wide_count = 0;    // (and instructions of those kinds streamed)
     int mode = MODE_STAGES;
@@ -201,7 +205,7 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
     // filled in the current round if s < position, else in the previous one).
     auto drain = [&](int kind, int next) -> bool {
         int ok = 1;
-        if (lane == 0) {
+        if (lane == 0 && kind != MODE_ATTN) {         // (an attention run returns the memory itself)
             if (kind == MODE_WTILES) {
                 for (int s = 0; s < kTcWSlots && ok; ++s)
                     ok = wait_barrier(p, c, &c->w_empty[s], (wphase ^ (s < wslot ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
@@ -228,6 +232,23 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
         return true;
     };
     while (rc.valid(p)) {
+        if (rc.attn) {
+            // a run of tcgen05 attentions of head_dim 128: the ring's memory is theirs until the compute warps are through
+            if (!enter(MODE_ATTN)) return;
+            int ok = 1;
+            if (lane == 0) {
+                mbar_arrive(&c->ring_granted);
+                ok = wait_barrier(p, c, &c->ring_returned, returned, rc.seq, WHERE_RING_EMPTY, 4) ? 1 : 0;
+            }
+            if (!__shfl_sync(0xffffffffu, ok, 0)) return;
+            returned ^= 1u;
+            for (rc.idx += gridDim.x; rc.idx < p.n_insts; rc.idx += gridDim.x) {       // past the run
+                const int opi = __ldg(p.insts + (long long)rc.idx * 4).x - 1;
+                if (opi < 0 || opi >= p.n_ops || !(is_attention_tc(p.ops + opi) && p.ops[opi].i[5] == 128)) break;
+            }
+            rc.seek(p);
+            continue;
+        }
         if (rc.kv) {
             // decode attention, many-sequence form: one tile of 16 whole cache rows per slot, as four
             // copies of four rows issued by four lanes at once; K and V tiles alternate.  The whole

@@ -26,14 +26,13 @@ __device__ int mk_op_gemv_general(const Params& p, const mk_op_desc* op, int o0,
 __device__ int mk_run_gemm(const Params& p, int idx, int slot);
 // (the same with 256 x 256 output tiles; only for ops the host library bound to the tcgen05 body)
 __device__ int mk_run_gemm_wide(const Params& p, int idx, int slot);
-// body of the issuer warp: the MMAs of every 256 x 256 tile, until the feeder warp says that the list has ended
-__device__ void mk_wide_issuer(const Params& p);
+// body of the issuer warp: the MMAs of every tile GEMM with 256-row tiles and of every tcgen05 attention, until the feeder warp says that the list has ended
+__device__ void mk_issuer(const Params& p);
 __device__ void mk_op_attention(const mk_op_desc* op, int a0, int a1, int a2);
-// (the tcgen05 body, for ops the host library attached tensor maps to; returns -1 when aborting)
-__device__ int mk_op_attention_tc(const Params& p, const mk_op_desc* op, int a0, int a1, int a2, int seq);
-// body of the feeder warp: walks the CTA's instruction list and, for every prefill attention bound to the tcgen05 body,
-// requests its tiles and issues its MMAs (one thread), for every 256 x 256 tile GEMM requests its activation tiles; runs
-// until the list ends or the CTA aborts
+// (the tcgen05 body, for ops the host library attached tensor maps to: like mk_run_gemm, for runs of one head_dim)
+__device__ int mk_run_attention(const Params& p, const mk_op_desc* op, int idx, int slot);
+// body of the feeder warp: walks the CTA's instruction list and requests the tiles of every prefill attention bound to the
+// tcgen05 body and the activation tiles of every tile GEMM with 256-row tiles; runs until the list ends or the CTA aborts
 __device__ void mk_feeder(const Params& p);
 // (waits for its own dependencies and publishes its own arrivals; returns whether the CTA is aborting)
 __device__ bool mk_op_decode_attn(const Params& p, const mk_op_desc* op, int a0, int a1, int a2, int nwait, int wait_off,
