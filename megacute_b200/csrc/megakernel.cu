@@ -78,10 +78,11 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         for (int s = 0; s < 2; ++s) {
             mbar_init(&c->attn.k_full[s], 1); mbar_init(&c->attn.k_empty[s], 2);
             mbar_init(&c->attn.v_full[s], 1); mbar_init(&c->attn.v_empty[s], 2);
-            mbar_init(&c->attn.s_full[s], 1); mbar_init(&c->attn.p_full[s], kComputeWarps / 2);
+            mbar_init(&c->attn.p_full[s], kComputeWarps / 2);
             mbar_init(&c->attn.pv_done[s], 1); mbar_init(&c->attn.o_free[s], kComputeWarps / 2);
             c->at_blocks[0][s] = 0;
         }
+        for (int s = 0; s < 3; ++s) mbar_init(&c->attn.s_full[s], 1);
         c->at_turn = 0;
         mbar_init(&c->acc_full, kTcIssuers);
         for (int s = 0; s < kKvSlots; ++s) {

@@ -136,7 +136,8 @@ struct Meta {
 struct AttnBars {                 // tcgen05 prefill attention (op_attention_tc.cuh)
     unsigned long long q_full, q_free;               // the two Q tiles have landed / every product that reads them has completed
     unsigned long long k_full[2], k_empty[2], v_full[2], v_empty[2];      // ... the K, V stages (released once per Q tile)
-    unsigned long long s_full[2], p_full[2], pv_done[2], o_free[2];       // per Q tile: scores there; read, and P written; P V done; O read
+    unsigned long long s_full[3];                                         // scores there, by the block's number
+    unsigned long long p_full[2], pv_done[2], o_free[2];                  // per Q tile: scores read, and P written; P V done; O read
 };
 
 struct Ctrl {                     // lives in the last kCtrlBytes of shared memory
@@ -169,13 +170,14 @@ struct Ctrl {                     // lives in the last kCtrlBytes of shared memo
     AttnBars attn;
     unsigned long long attn_go;              // tcgen05 prefill attention: the compute warps have turned to the first of a run
     unsigned long long ring_granted, ring_returned;      // ... head_dim 128: the run may use the ring's memory / is done with it
-    uint32_t at_blocks[2][2], at_turn;       // ... blocks of each Q tile so far, written for the next instruction during this one; whose turn
+    uint32_t at_blocks[2][2];                // ... blocks of each Q tile so far, written for the next instruction during this one
     uint32_t tmem_base;               // ... tensor-memory address of the accumulator (written by tcgen05.alloc)
-    uint32_t tmem_ready;              // ... 1 once it is allocated; written behind the barrier that follows the allocation, so all
-                                      //     threads of an instruction read the same value (tmem_base changes while they arrive)
     uint32_t x_par;                       // ... bit s: parity of the next completion of x_full[s] and of x_empty[s] (between
                                           //     instructions both have completed equally often); set at an instruction's end
     uint8_t w_slot, w_phase;              // ... the MMA thread's position in the weight slots
+    uint8_t at_turn;                      // tcgen05 prefill attention: which at_blocks is current (bit 0)
+    uint8_t tmem_ready;               // 1 once tensor memory is allocated; written behind the barrier that follows the allocation, so
+                                      //     all threads of an instruction read the same value (tmem_base changes while they arrive)
     uint32_t acc_uses;                // ... instructions that have used acc_full (its parity)
     int abort;                    // set once a wait of this CTA gave up or saw the global abort
     int flag;                     // scratch broadcast word (split-KV last arriver)

@@ -1,6 +1,6 @@
 // Translation unit of MK_OP_ATTENTION on tcgen05 (tensor maps attached by the host library), and of the feeder and issuer warps.
-#include "op_attention_tc.cuh"
 #include "op_gemm_tc_wide.cuh"
+#include "op_attention_tc.cuh"
 #include "ops.cuh"
 #include "walk.cuh"
 

@@ -41,8 +41,8 @@ template <int D> struct AtMap {
     static constexpr int kQ = kRingBytes + kTcXOff;
     static constexpr int kK = D == 64 ? kQ + 2 * kTile : 0;
     static constexpr int kV = kK + 2 * kTile;
-    static constexpr uint32_t kS = 0, kO = 256, kP = D == 64 ? 384 : 0;                     // tensor-memory columns of tile 0 ...
-    static constexpr uint32_t kOStep = D, kPStep = D == 64 ? 64 : 128;                      // ... and to tile 1 (S: 128)
+    static constexpr uint32_t kScores = D == 64 ? 3 : 2;      // tensor-memory buffers of scores, 128 columns each from column 0
+    static constexpr uint32_t kO = kScores * 128;             // ... then O of tile 0 and of tile 1
 };
 static_assert(AtMap<64>::kV + 2 * AtMap<64>::kTile <= kRingBytes + kWorkBytes, "attention tiles, head_dim 64");
 static_assert(AtMap<128>::kV + 2 * AtMap<128>::kTile <= kRingBytes && AtMap<128>::kQ + 2 * AtMap<128>::kTile <= kRingBytes + kWorkBytes, "attention tiles, head_dim 128");
@@ -93,6 +93,34 @@ __device__ __forceinline__ void tc_mma_ta(uint32_t tmem_d, uint32_t tmem_a, uint
         "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+
+// two fp32 operations in one instruction
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{ .reg .b64 x, y, z, w; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; mov.b64 z, {%6, %7}; fma.rn.f32x2 w, x, y, z; mov.b64 {%0, %1}, w; }"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{ .reg .b64 x, y, w; mov.b64 x, {%2, %3}; mov.b64 y, {%4, %5}; add.rn.f32x2 w, x, y; mov.b64 {%0, %1}, w; }"
+        : "=f"(d.x), "=f"(d.y)
+        : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ uint32_t pack2h_fast(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
+}
+
+// The blocks of an instruction in the order in which the issuer takes them: the tiles in turns, then what one of them has more.
+__device__ __forceinline__ int at_order(int t, int j, int both) { return j < both ? 2 * j + t : both + j; }
 
 // ---- feeder warp ---------------------------------------------------------------------------------------------------------------
 struct AtFeed {
@@ -162,19 +190,19 @@ __device__ __forceinline__ bool at_feed(const Params& p, Ctrl* c, uint8_t* ring,
 // ---- issuer warp ---------------------------------------------------------------------------------------------------------------
 struct AtIssue {
     uint32_t insts = 0, tiles = 0;       // instructions, K / V tiles
-    uint32_t blocks[2] = {0, 0};         // blocks of each tile (parities of s_full, p_full, pv_done)
+    uint32_t blocks[2] = {0, 0};         // blocks of each tile (parities of p_full, pv_done; together: place of the next scores)
     uint32_t outs[2] = {0, 0};           // instructions that had the tile (parity of o_free)
 };
-// Every lane asks the barriers (their answers can differ while one completes: the vote makes the warp take one path).
+// Every lane asks the barrier (the answers can differ while a phase completes: the vote makes the warp take one path).
 __device__ __forceinline__ bool at_ready(unsigned long long* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_test_wait(bar, parity)) != 0; }
-// The whole warp polls, one elected lane issues.  Returns false when aborting.
+// The whole warp waits, one elected lane issues.  Returns false when aborting.
 template <int D>
 __device__ __forceinline__ bool at_issue(const Params& p, Ctrl* c, uint8_t* ring, const int4& info, AtIssue& f) {
     using M = AtMap<D>;
     AttnBars* a = &c->attn;
     const int nbt[2] = {(-info.x) & 0x7fff, (-info.x) >> 15};
-    const int nb = max(nbt[0], nbt[1]);
-    const uint32_t tmem = *(volatile uint32_t*)&c->tmem_base;
+    const int both = min(nbt[0], nbt[1]), total = nbt[0] + nbt[1], tail = nbt[1] > nbt[0] ? 1 : 0;
+    const uint32_t tmem = *(volatile uint32_t*)&c->tmem_base, first = f.blocks[0] + f.blocks[1];
     const uint32_t fmt = info.z ? 0u : 1u;                    // operand format: 0 fp16, 1 bf16
     // fp32 accumulator, M = 128; S: N = 128, both operands K-major; O: N = D, B MN-major
     const uint32_t base = (1u << 4) | (fmt << 7) | (fmt << 10) | ((128u >> 4) << 24);
@@ -182,85 +210,62 @@ __device__ __forceinline__ bool at_issue(const Params& p, Ctrl* c, uint8_t* ring
     const uint64_t d0 = tc_smem_desc(smem_u32(ring));
     // MN-major: 8-key groups 1024 bytes apart (the descriptor's stride), 64-column sub-tiles 16 KB apart (its leading offset)
     const uint64_t v0 = D == 64 ? d0 : d0 - (1ull << 16) + ((uint64_t)(kTcTileBytes >> 4) << 16);
-    int si[2] = {0, 0}, pf[2] = {0, 0}, pi[2] = {0, 0};       // S issued, softmax blocks handed over, P V issued
-    bool q_ready = false, q_done = false;
-    uint32_t idle = 0;
-    unsigned long long t0 = 0;
-    while (pi[0] < nbt[0] || pi[1] < nbt[1]) {
-        bool progress = false;
-        if (!q_ready) q_ready = at_ready(&a->q_full, f.insts & 1u);
+    auto await = [&](unsigned long long* bar, uint32_t parity) {
+        for (int i = 0; i < 64; ++i)                          // (a few microseconds of asking: try_wait answers later)
+            if (at_ready(bar, parity)) return true;
+        return issuer_wait(p, c, bar, parity, info.w, WHERE_RING_FULL, 2);
+    };
+    auto tile_of = [&](int n) { return n < 2 * both ? n & 1 : tail; };
+    auto block_of = [&](int n) { return n < 2 * both ? n >> 1 : n - both; };
+    // scores of the n-th block into their buffer: the block that had it before has been multiplied (its P V is ahead in the pipe)
+    auto scores = [&](int n) {
+        const int t = tile_of(n), j = block_of(n);
+        const uint32_t k = f.tiles + (uint32_t)j, u = k & 1u, seq = first + (uint32_t)n, buf = seq % M::kScores;
+        if (!await(&a->k_full[u], (k >> 1) & 1u)) return false;
+        tc_fence_after();
+        const uint64_t qd = d0 + (uint32_t)((M::kQ + t * M::kTile) >> 4), kd = d0 + ((uint32_t)M::kK >> 4) + u * (uint32_t)(M::kTile >> 4);
+        const bool alone = j >= both;                         // the other tile does not read this K tile
+        if (elect_one()) {
 #pragma unroll
-        for (int t = 0; t < 2; ++t) {
-            // S of the tile's next block: K there, and the scores of the block before read (head_dim 128: and multiplied, P lies over them)
-            if (q_ready && si[t] < nbt[t] && si[t] <= pf[t]) {
-                const uint32_t n = f.tiles + (uint32_t)si[t], u = n & 1u;
-                bool go = at_ready(&a->k_full[u], (n >> 1) & 1u);
-                if (D == 128 && f.blocks[t] + (uint32_t)si[t] > 0)
-                    go = go && pi[t] == si[t] && at_ready(&a->pv_done[t], (f.blocks[t] + (uint32_t)si[t] - 1u) & 1u);
-                if (go) {
-                    tc_fence_after();
-                    const uint64_t qd = d0 + (uint32_t)((M::kQ + t * M::kTile) >> 4), kd = d0 + ((uint32_t)M::kK >> 4) + u * (uint32_t)(M::kTile >> 4);
-                    const bool alone = si[t] >= nbt[t ^ 1];                // the other tile does not read this K tile
-                    if (elect_one()) {
+            for (int k16 = 0; k16 < D / 16; ++k16) {
+                const uint32_t off = (k16 & 3) * 2 + (k16 >> 2) * (kTcTileBytes >> 4);
+                tc_mma(tmem + 128 * buf, qd + off, kd + off, idesc_s, k16 ? 1u : 0u);
+            }
+            tc_commit(&a->s_full[seq % 3u]);
+            tc_commit(&a->k_empty[u]);
+            if (alone) tc_commit(&a->k_empty[u]);
+            if (n == total - 1) tc_commit(&a->q_free);        // every product that reads Q has been issued
+        }
+        __syncwarp();
+        return true;
+    };
+    if (!await(&a->q_full, f.insts & 1u)) return false;
+    for (int n = 0; n < (int)M::kScores && n < total; ++n)
+        if (!scores(n)) return false;
+    for (int n = 0; n < total; ++n) {
+        const int t = tile_of(n), j = block_of(n);
+        const uint32_t k = f.tiles + (uint32_t)j, u = k & 1u, buf = (first + (uint32_t)n) % M::kScores;
+        if (!await(&a->p_full[t], (f.blocks[t] + (uint32_t)j) & 1u)) return false;
+        if (!await(&a->v_full[u], (k >> 1) & 1u)) return false;
+        // (the first P V overwrites O: the compute warps must have read the previous instruction's)
+        if (j == 0 && f.outs[t] > 0 && !await(&a->o_free[t], (f.outs[t] - 1u) & 1u)) return false;
+        tc_fence_after();
+        const uint64_t vd = v0 + ((uint32_t)M::kV >> 4) + u * (uint32_t)(M::kTile >> 4);
+        const bool alone = j >= both;
+        const uint32_t acc = j > 0 ? 1u : 0u;
+        if (elect_one()) {
 #pragma unroll
-                        for (int k16 = 0; k16 < D / 16; ++k16) {
-                            const uint32_t off = (k16 & 3) * 2 + (k16 >> 2) * (kTcTileBytes >> 4);
-                            tc_mma(tmem + M::kS + 128 * t, qd + off, kd + off, idesc_s, k16 ? 1u : 0u);
-                        }
-                        tc_commit(&a->s_full[t]);
-                        tc_commit(&a->k_empty[u]);
-                        if (alone) tc_commit(&a->k_empty[u]);
-                    }
-                    __syncwarp();
-                    ++si[t];
-                    progress = true;
-                }
-            }
-            if (pf[t] < si[t] && at_ready(&a->p_full[t], (f.blocks[t] + (uint32_t)pf[t]) & 1u)) { ++pf[t]; progress = true; }
-            if (pi[t] < pf[t]) {
-                const uint32_t n = f.tiles + (uint32_t)pi[t], u = n & 1u;
-                // (the first P V overwrites O: the compute warps must have read the previous instruction's)
-                bool go = at_ready(&a->v_full[u], (n >> 1) & 1u);
-                if (pi[t] == 0 && f.outs[t] > 0) go = go && at_ready(&a->o_free[t], (f.outs[t] - 1u) & 1u);
-                if (go) {
-                    tc_fence_after();
-                    const uint64_t vd = v0 + ((uint32_t)M::kV >> 4) + u * (uint32_t)(M::kTile >> 4);
-                    const bool alone = pi[t] >= nbt[t ^ 1];
-                    const uint32_t acc = pi[t] > 0 ? 1u : 0u;
-                    if (elect_one()) {
-#pragma unroll
-                        for (int k16 = 0; k16 < 8; ++k16)                  // 16 keys: 8 columns of P, 2048 bytes of V
-                            tc_mma_ta(tmem + M::kO + M::kOStep * t, tmem + M::kP + M::kPStep * t + 8 * k16, vd + 128 * k16, idesc_o, acc | (k16 ? 1u : 0u));
-                        tc_commit(&a->pv_done[t]);
-                        tc_commit(&a->v_empty[u]);
-                        if (alone) tc_commit(&a->v_empty[u]);
-                    }
-                    __syncwarp();
-                    ++pi[t];
-                    progress = true;
-                }
-            }
+            for (int k16 = 0; k16 < 8; ++k16)                  // 16 keys: 8 columns of P, 2048 bytes of V
+                tc_mma_ta(tmem + M::kO + D * t, tmem + 128 * buf + 8 * k16, vd + 128 * k16, idesc_o, acc | (k16 ? 1u : 0u));
+            tc_commit(&a->pv_done[t]);
+            tc_commit(&a->v_empty[u]);
+            if (alone) tc_commit(&a->v_empty[u]);
         }
-        if (!q_done && si[0] == nbt[0] && si[1] == nbt[1]) {               // every product that reads Q has been issued
-            if (elect_one()) tc_commit(&a->q_free);
-            __syncwarp();
-            q_done = true;
-        }
-        if (progress) { idle = 0; t0 = 0; continue; }
-        if ((++idle & 1023u) == 0) {                                       // nothing to do: the time limit of every other wait applies (twice: role)
-            bool stop = *(volatile int*)&c->abort != 0;
-            if (!stop && ld_volatile(&p.status[MK_ST_CODE]) != 0) { c->abort = 1; stop = true; }
-            const unsigned long long now = globaltimer();
-            if (t0 == 0) t0 = now;
-            else if (!stop && now - t0 > 2 * p.timeout_ns) {
-                report(p, c, MK_DEV_TIMEOUT_BARRIER, info.w, WHERE_RING_FULL, (int)(&a->p_full[0] - c->full), pi[0], si[0]);
-                stop = true;
-            }
-            if (__any_sync(0xffffffffu, stop)) return false;
-        }
+        __syncwarp();
+        if (n + (int)M::kScores < total && !scores(n + (int)M::kScores)) return false;
     }
     ++f.insts;
-    f.tiles += (uint32_t)nb;
+    f.tiles += (uint32_t)max(nbt[0], nbt[1]);
     for (int t = 0; t < 2; ++t) {
         f.blocks[t] += (uint32_t)nbt[t];
         f.outs[t] += nbt[t] > 0 ? 1u : 0u;
@@ -271,7 +276,7 @@ __device__ __forceinline__ bool at_issue(const Params& p, Ctrl* c, uint8_t* ring
 // ---- compute warps -------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void at_begin_run(Ctrl* c) {
     const int t = threadIdx.x;
-    if (*(volatile uint32_t*)&c->tmem_ready == 0) {                       // (a word that only changes behind a barrier: see op_gemm_tc)
+    if (*(volatile uint8_t*)&c->tmem_ready == 0) {                       // (a word that only changes behind a barrier: see op_gemm_tc)
         if (t < 32) {
             __syncwarp();
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&c->tmem_base)), "r"(kTcCols)
@@ -298,19 +303,22 @@ __device__ __forceinline__ void op_attention_tc(const Params& p, Ctrl* c, const 
     const int kend = causal ? min(Sk, q0 + 128) : Sk;
     const int nb = at_blocks(op, qi, t);
     AttnBars* a = &c->attn;
-    const uint32_t turn = *(volatile uint32_t*)&c->at_turn & 1u;
-    const uint32_t base = c->at_blocks[turn][t];                           // blocks of this tile so far
+    const uint32_t turn = (uint32_t)*(volatile uint8_t*)&c->at_turn & 1u;
+    const uint32_t base = c->at_blocks[turn][t], seq0 = base + c->at_blocks[turn][t ^ 1];      // blocks of this tile, of both so far
+    const int both = min(nb, at_blocks(op, qi, t ^ 1));
     if ((threadIdx.x & 127) == 0) c->at_blocks[turn ^ 1u][t] = base + (uint32_t)nb;
     phase_mark(p, c, 0);
     if (nb == 0) return;
     const uint32_t tl = *(volatile uint32_t*)&c->tmem_base + ((uint32_t)(qd * 32) << 16);
-    const uint32_t scol = tl + M::kS + 128 * t, pcol = tl + M::kP + M::kPStep * t, ocol = tl + M::kO + M::kOStep * t;
+    const uint32_t ocol = tl + M::kO + D * t;
     const float sl2 = op->f[0] * kLog2e;
     float m_used = NEG_INF, l = 0.f;
     bool ok = true;
 #pragma unroll 1
     for (int j = 0; j < nb; ++j) {
-        ok = wait_barrier(p, c, &a->s_full[t], (base + (uint32_t)j) & 1u, seq, WHERE_COMBINE, 2) && ok;
+        const uint32_t n = seq0 + (uint32_t)at_order(t, j, both);
+        const uint32_t scol = tl + 128 * (n % M::kScores);                     // the scores, and P over those already read
+        ok = wait_barrier(p, c, &a->s_full[n % 3u], (n / 3u) & 1u, seq, WHERE_COMBINE, 2) && ok;
         __syncwarp();
         tc_fence_after();
         const int key0 = j * 128;
@@ -327,8 +335,9 @@ __device__ __forceinline__ void op_attention_tc(const Params& p, Ctrl* c, const 
                 for (int e = 0; e < 32; ++e) s[e] = e <= n ? s[e] : NEG_INF;
             }
 #pragma unroll
-            for (int e = 0; e < 32; e += 4) {
-                m4[0] = fmaxf(m4[0], s[e]); m4[1] = fmaxf(m4[1], s[e + 1]); m4[2] = fmaxf(m4[2], s[e + 2]); m4[3] = fmaxf(m4[3], s[e + 3]);
+            for (int e = 0; e < 32; e += 8) {
+                m4[0] = max3(m4[0], s[e], s[e + 1]); m4[1] = max3(m4[1], s[e + 2], s[e + 3]);
+                m4[2] = max3(m4[2], s[e + 4], s[e + 5]); m4[3] = max3(m4[3], s[e + 6], s[e + 7]);
             }
         }
         const float mx = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * sl2;
@@ -338,7 +347,7 @@ __device__ __forceinline__ void op_attention_tc(const Params& p, Ctrl* c, const 
             factor = m_used == NEG_INF ? 0.f : ex2(m_used - mx);
             m_used = mx;
         }
-        // P's place and (for a rescale) O are free once the previous block's P V has completed
+        // (for a rescale) O is complete once the previous block's P V is
         if (j > 0) ok = wait_barrier(p, c, &a->pv_done[t], (base + (uint32_t)j - 1u) & 1u, seq, WHERE_COMBINE, 2) && ok;
         __syncwarp();
         tc_fence_after();
@@ -355,7 +364,8 @@ __device__ __forceinline__ void op_attention_tc(const Params& p, Ctrl* c, const 
         }
         // P = 2^(s * scale - m), rounded to the operand type; row sum
         const float mm = m_used == NEG_INF ? 0.f : m_used;                     // (a row without a live key so far: every s is -inf)
-        float l4[4] = {0.f, 0.f, 0.f, 0.f};
+        const float2 scale2 = make_float2(sl2, sl2), off2 = make_float2(-mm, -mm);
+        float2 l4[4] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
 #pragma unroll 1
         for (int ch = 0; ch < 4; ++ch) {
             float s[32];
@@ -368,21 +378,21 @@ __device__ __forceinline__ void op_attention_tc(const Params& p, Ctrl* c, const 
             uint32_t w[16];
 #pragma unroll
             for (int e = 0; e < 32; e += 2) {
-                const float p0 = ex2(fmaf(s[e], sl2, -mm)), p1 = ex2(fmaf(s[e + 1], sl2, -mm));
-                l4[(e >> 1) & 1] += p0;
-                l4[2 + ((e >> 1) & 1)] += p1;
-                s[e] = p0; s[e + 1] = p1;
+                const float2 y = fma2(make_float2(s[e], s[e + 1]), scale2, off2);
+                const float2 q = make_float2(ex2(y.x), ex2(y.y));
+                l4[(e >> 1) & 3] = add2(l4[(e >> 1) & 3], q);
+                s[e] = q.x; s[e + 1] = q.y;
             }
-            if (f16) {
+            if (f16) {                                                         // (at most 2^8: nothing to saturate)
 #pragma unroll
-                for (int e = 0; e < 16; ++e) w[e] = pack2h(s[2 * e], s[2 * e + 1]);
+                for (int e = 0; e < 16; ++e) w[e] = pack2h_fast(s[2 * e], s[2 * e + 1]);
             } else {
 #pragma unroll
                 for (int e = 0; e < 16; ++e) w[e] = pack2(s[2 * e], s[2 * e + 1]);
             }
-            tc_st16(pcol + ch * 16, w);                                        // (head_dim 128: over scores already read)
+            tc_st16(scol + ch * 16, w);
         }
-        l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+        l += ((l4[0].x + l4[0].y) + (l4[1].x + l4[1].y)) + ((l4[2].x + l4[2].y) + (l4[3].x + l4[3].y));
         tc_wait_st();
         tc_fence_before();
         __syncwarp();

@@ -213,7 +213,7 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
     // (the test is on a word that only changes behind a barrier, so every thread takes the same branch -- not on the
     // address itself, which the allocation writes while the other warps are still arriving at the test)
     const uint32_t uses = *(volatile uint32_t*)&c->acc_uses;
-    if (*(volatile uint32_t*)&c->tmem_ready == 0) {            // (the attention op may have allocated it already)
+    if (*(volatile uint8_t*)&c->tmem_ready == 0) {            // (the attention op may have allocated it already)
         if (warp == 0) {
             __syncwarp();          // (.sync.aligned: the whole warp, converged)
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&c->tmem_base)), "r"(kTcCols)

@@ -447,7 +447,7 @@ __device__ __forceinline__ int wide_variant(const mk_op_desc* op) {
 // kernel ends; the branch is taken on a word that only changes behind a barrier, see op_gemm_tc), then the go for the feeder.
 __device__ __forceinline__ void wide_begin_run(Ctrl* c) {
     const int t = threadIdx.x;
-    if (*(volatile uint32_t*)&c->tmem_ready == 0) {
+    if (*(volatile uint8_t*)&c->tmem_ready == 0) {
         if (t < 32) {
             __syncwarp();
             asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&c->tmem_base)), "r"(kTcCols)
