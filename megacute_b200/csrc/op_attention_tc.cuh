@@ -9,19 +9,24 @@
 //                    threads.  Log2 domain, scale * log2(e) folded into the subtraction.  The running maximum is only raised
 //                    when it grows by more than 2^8 (the reference's lazy rescale, megacute/ops/attention.py:37,252-262): then
 //                    the row's sum and its O row in tensor memory are scaled down.
-//   O += P V_j       P, rounded to the operand type, goes back to tensor memory as the A operand; V_j as loaded ([key][64 dims])
+//   O += P V_j       P, rounded to the operand type, goes back to tensor memory, over the scores, as the A operand; V_j as loaded ([key][64 dims])
 //                    is the MN-major B operand; O in tensor memory
 //   out = O / l      read back, a row per thread; a fully masked row yields 0
-// While one tile's scores are multiplied the other tile's are exponentiated: 128 x 128 exponentials take the SM's special
-// function units 1024 cycles, the products of a block 600 to 1100.  (One tile per instruction, two threads per row that agreed
-// on the maximum through shared memory, P through shared memory: 3800 cycles per block.)
+// Bound by the special function units: the exponentials of a block of both tiles take 2048 cycles, its products 1024 (head_dim 64)
+// or 2048 (128).  What keeps the distance is latency between the roles, so the scores of a block are multiplied ahead: the blocks
+// of both tiles are numbered in one sequence, and the scores of block n + 3 (head_dim 128: n + 2) are issued right behind
+// block n's P V, into the same tensor-memory buffer, where P lies over the scores.  Products execute in the order of issue, so
+// nothing has to be waited for in between, and the tiles fall out of step by themselves: one exponentiates while the other waits.
+// Per block of both tiles, 4 x 4096 causal, 32 heads: one buffer a tile, scores requested after P V 5900 cycles; scores first,
+// fp32 operations in pairs 4400; three buffers 3600.  (Taken back, each slower: the tiles made to exponentiate in turns with a
+// barrier; two 32-column loads in flight.)
 //
 // Three roles run ahead of one another across the instructions of a run, as in the tile GEMM (op_gemm_tc_wide.cuh):
 //   feeder warp      waits for the instruction's dependencies itself, requests Q, then K and V through two stages each
-//   issuer warp      the products of both tiles, whatever is possible next; told by the feeder through Ctrl::wide_info
+//   issuer warp      the products of both tiles in one fixed order; told by the feeder through Ctrl::wide_info
 //   compute warps    softmax and output
-// Barriers are initialised once per launch; every role counts.  Tensor memory (columns): S at 0 and 128; head_dim 64: O at 256 and
-// 320, P at 384 and 448; head_dim 128: O at 256 and 384, P over S (the next scores of a tile then wait for its P V).
+// Barriers are initialised once per launch; every role counts.  Tensor memory (columns): three (two) buffers of scores from 0, O of
+// both tiles behind them.
 // Shared memory: head_dim 64: two Q tiles, two K and two V stages in the work area; head_dim 128: Q in the work area, K and V in the
 // ring's memory, which the producer warp grants for a run (Ctrl::ring_granted / ring_returned).
 // Every wait is bounded.  Operands the tensor maps cannot describe run the mma.sync body.
@@ -114,6 +119,7 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
     asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
     return d;
 }
+// two fp16 from fp32 of at most 2^8: nothing to saturate
 __device__ __forceinline__ uint32_t pack2h_fast(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
@@ -383,7 +389,7 @@ __device__ __forceinline__ void op_attention_tc(const Params& p, Ctrl* c, const 
                 l4[(e >> 1) & 3] = add2(l4[(e >> 1) & 3], q);
                 s[e] = q.x; s[e + 1] = q.y;
             }
-            if (f16) {                                                         // (at most 2^8: nothing to saturate)
+            if (f16) {
 #pragma unroll
                 for (int e = 0; e < 16; ++e) w[e] = pack2h_fast(s[2 * e], s[2 * e + 1]);
             } else {
