@@ -174,8 +174,8 @@ __device__ __forceinline__ bool wide_issue(const Params& p, Ctrl* c, uint8_t* ri
 }
 
 // ---- compute warps: epilogue ---------------------------------------------------------------------------------------------------
-// A warp's part of the tile: 32 rows (one per lane of tensor memory) x 256 columns.  Rows are turned into row-contiguous
-// global accesses through 4 KB of shared memory of the warp's own, 128 bytes per row, 16-byte chunks swizzled by the row.
+// A warp's part of the tile: 32 rows (one per lane of tensor memory) x 256 columns, and 4 KB of shared memory of its own: a gate row,
+// or (wide_store_any) rows of 128 bytes, 16-byte chunks swizzled by the row.
 __device__ __forceinline__ uint4* wide_chunk(uint8_t* stg, int row, int ch) { return reinterpret_cast<uint4*>(stg + row * 128 + ((ch ^ (row & 7)) << 4)); }
 // What an epilogue works on.
 struct WideAcc {
@@ -232,18 +232,62 @@ __device__ __forceinline__ void act_all(int act, float* v) {
     }
 }
 
-// 16-bit outputs, no residual: 32 output columns at a time into the staging rows, 64 at a time from there.  A loop, not 256 columns
-// of straight-line code that keeps them packed in registers to hand the accumulator back early: fetching that code took longer
-// than executing this (gelu tile: 13 us from the accumulator to the arrival, 4.4 of them instruction issue).
-// ACT: 0 none, 1 gelu, 2 any (run time).
+// A thread writes (and, with a residual, reads) whole 32-byte pieces of its own row: whole sectors, as good as 128 bytes of four
+// rows at a time, without the detour through shared memory that the operands of the next tile are streaming through (64
+// bytes a cycle in, 96 out to the tensor core).  DiT, 32 images: 8.95 -> 8.82 ms together with the prefetch of the residual; what is
+// left (4.6 us for 256 x 256 16-bit outputs, 11 with a residual) is the memory system taking the bursts of all SMs at once.
+// `whole`: the rows start on 32-byte boundaries; else two 16-byte accesses.
+__device__ __forceinline__ void st32B(uint8_t* at, const uint32_t* w, bool whole) {
+    if (whole)
+        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(at), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+                     "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
+                     : "memory");
+    else {
+        reinterpret_cast<uint4*>(at)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        reinterpret_cast<uint4*>(at)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+}
+__device__ __forceinline__ void ld32B(const uint8_t* at, uint32_t* w, bool whole) {
+    if (whole)
+        asm volatile("ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                     : "l"(at)
+                     : "memory");
+    else {
+        const uint4 a = __ldcg(reinterpret_cast<const uint4*>(at)), b = __ldcg(reinterpret_cast<const uint4*>(at) + 1);
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    }
+}
+// 32 columns of a row, converted
+template <int DT>
+__device__ __forceinline__ void put32(uint8_t* at, const float* v, bool whole) {
+    uint32_t w[8];
+    if (DT == DT_F32) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(v[8 * k + e]);
+            st32B(at + 32 * k, w, whole);
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) w[e] = DT == DT_F16 ? pack2h(v[16 * k + 2 * e], v[16 * k + 2 * e + 1]) : pack2(v[16 * k + 2 * e], v[16 * k + 2 * e + 1]);
+            st32B(at + 32 * k, w, whole);
+        }
+    }
+}
+
+// 16-bit outputs, no residual, 32 output columns at a time.  A loop, not 256 columns of straight-line code: fetching that code took
+// longer than executing this.  ACT: 0 none, 1 gelu, 2 any (run time).
 template <bool F16, bool SWI, int ACT>
 __device__ __forceinline__ void wide_store16(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
     const int lane = threadIdx.x & 31;
     const int act = op->i[3], groups = (op->i[10] >> 5) >> (SWI ? 1 : 0);
-    const int rows = op->i[0] - row0;
-    const long long ldo = (long long)op->ld[2] * 2;
-    const int r = lane >> 3, cc = lane & 7;
-    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + (long long)(row0 + r) * ldo + (SWI ? n0 / 2 : n0) * 2 + cc * 16;
+    const bool live = row0 + lane < op->i[0];
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + ((long long)(row0 + lane) * op->ld[2] + (SWI ? n0 / 2 : n0)) * 2;
+    const bool whole = ((op->ptr[2] | (uint64_t)op->ld[2] * 2) & 31) == 0;
     if (!wide_wait(p, c, a)) return;
 #pragma unroll 1
     for (int g = 0; g < groups; ++g) {
@@ -266,38 +310,11 @@ __device__ __forceinline__ void wide_store16(const Params& p, Ctrl* c, const mk_
             }
             if (ACT == 2) act_all(act, v);
         }
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float* f = v + 8 * j;
-            *wide_chunk(a.stg, lane, (g & 1) * 4 + j) =
-                F16 ? make_uint4(pack2h(f[0], f[1]), pack2h(f[2], f[3]), pack2h(f[4], f[5]), pack2h(f[6], f[7])) : pack8(f);
-        }
-        if (!(g & 1)) continue;
-        __syncwarp();
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
-            if (j * 4 + r < rows) *reinterpret_cast<uint4*>(O + (long long)(j * 4) * ldo + (g >> 1) * 128) = *wide_chunk(a.stg, j * 4 + r, cc);
+        if (live) put32<F16 ? DT_F16 : DT_BF16>(O + g * 64, v, whole);
         __syncwarp();
     }
 }
 
-// four values of a type known at compile time, as raw bits
-template <int DT> struct Quad {
-    uint2 v;
-    __device__ __forceinline__ void load(const uint8_t* base, long long elem) { v = __ldcg(reinterpret_cast<const uint2*>(base + elem * 2)); }
-    __device__ __forceinline__ float4 get() const {
-        if (DT == DT_F16) {
-            const float2 lo = unpack2h(v.x), hi = unpack2h(v.y);
-            return make_float4(lo.x, lo.y, hi.x, hi.y);
-        }
-        return make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
-    }
-};
-template <> struct Quad<DT_F32> {
-    float4 v;
-    __device__ __forceinline__ void load(const uint8_t* base, long long elem) { v = __ldcg(reinterpret_cast<const float4*>(base + elem * 4)); }
-    __device__ __forceinline__ float4 get() const { return v; }
-};
 template <int DT>
 __device__ __forceinline__ void put4(uint8_t* at, const float4& o) {
     if (DT == DT_F32) *reinterpret_cast<float4*>(at) = o;
@@ -305,67 +322,75 @@ __device__ __forceinline__ void put4(uint8_t* at, const float4& o) {
     else *reinterpret_cast<uint2*>(at) = make_uint2(pack2(o.x, o.y), pack2(o.z, o.w));
 }
 __device__ __forceinline__ float4 load4_any(const uint8_t* base, long long elem, int dtype) {
-    if (dtype == DT_F32) { Quad<DT_F32> q; q.load(base, elem); return q.get(); }
-    if (dtype == DT_F16) { Quad<DT_F16> q; q.load(base, elem); return q.get(); }
-    Quad<DT_BF16> q; q.load(base, elem); return q.get();
+    if (dtype == DT_F32) return __ldcg(reinterpret_cast<const float4*>(base + elem * 4));
+    const uint2 v = __ldcg(reinterpret_cast<const uint2*>(base + elem * 2));
+    if (dtype == DT_F16) {
+        const float2 lo = unpack2h(v.x), hi = unpack2h(v.y);
+        return make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+    return make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
 }
 
-// With a residual (out = acc + bias [times a gate row per i 12 rows: an adaLN-Zero block's gated residual] + residual): 32 columns at
-// a time through shared memory as fp32, so that a warp's accesses cover whole 64- or 128-byte row pieces.  kDepth such steps
-// of the residual are requested ahead, the first while the main loop still runs, each into registers of its own: a step
-// takes 0.4 us, an L2 round trip beside the operand stream 2 us (one step ahead, or several in a queue that moves through
-// registers -- a move waits for its load -- 2.1 - 2.6 us per step).
+// With a residual (out = acc + bias [times a gate row per i 12 rows: an adaLN-Zero block's gated residual] + residual): kDepth steps of 32
+// columns of the residual are requested ahead, the first while the main loop still runs, each into registers of its own (an L2
+// round trip beside the operand stream takes 2 us).
 template <int RDT, int ODT, bool GATE>
 __device__ __forceinline__ void wide_store_res(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
-    constexpr int kDepth = RDT == DT_F32 ? 2 : 4;
+    constexpr int kDepth = RDT == DT_F32 ? 2 : 4, kWords = RDT == DT_F32 ? 32 : 16;
+    constexpr int osz = ODT == DT_F32 ? 4 : 2, rsz = RDT == DT_F32 ? 4 : 2;
     const int lane = threadIdx.x & 31;
     const int groups = op->i[10] >> 5;
-    const int rows = min(32, op->i[0] - row0);
-    const int r = lane >> 3, c4 = (lane & 7) * 4;
-    constexpr int osz = ODT == DT_F32 ? 4 : 2, rsz = RDT == DT_F32 ? 4 : 2;
-    int ldo = op->ld[2] * osz, ldr = op->ld[4] * rsz;          // bytes between rows (32 of them stay within 2^31)
-    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + (long long)(row0 + r) * ldo + (n0 + c4) * osz;
-    const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]) + (long long)row0 * ldr + (n0 + c4) * rsz;
-    const int gdt = op->i[13];
-    const uint8_t* G = GATE ? reinterpret_cast<const uint8_t*>(op->ptr[5]) + ((long long)(row0 / op->i[12]) * op->ld[5] + n0 + c4) * 2 : nullptr;
-    Quad<RDT> q[kDepth][8];
-    Quad<DT_BF16> gate[GATE ? kDepth : 1];
-    auto request = [&](int d, int g) {                       // (rows beyond the tensor read its last row, steps beyond the tile its last step)
+    const bool live = row0 + lane < op->i[0];
+    const int row = live ? row0 + lane : op->i[0] - 1;       // (rows beyond the tensor read its last row)
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + ((long long)row * op->ld[2] + n0) * osz;
+    const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]) + ((long long)row * op->ld[4] + n0) * rsz;
+    const bool owhole = ((op->ptr[2] | (uint64_t)op->ld[2] * osz) & 31) == 0, rwhole = ((op->ptr[4] | (uint64_t)op->ld[4] * rsz) & 31) == 0;
+    const bool g16 = GATE && op->i[13] == DT_F16;
+    uint32_t q[kDepth][kWords];
+    auto request = [&](int d, int g) {                       // (steps beyond the tile read its last step)
         g = min(g, groups - 1);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) q[d][j].load(R + min(j * 4 + r, rows - 1) * ldr, g * 32);
-        if (GATE) gate[GATE ? d : 0].load(G, g * 32);
+        for (int k = 0; k < kWords / 8; ++k) ld32B(R + g * 32 * rsz + 32 * k, q[d] + 8 * k, rwhole);
     };
 #pragma unroll
     for (int d = 0; d < kDepth; ++d) request(d, d);
+    // the rest of the row comes into L2 while the main loop runs (HBM has little to do then, and much during the epilogues)
+    for (int b = kDepth * 32 * rsz; b < groups * 32 * rsz; b += 128) asm volatile("prefetch.global.L2 [%0];" ::"l"(R + b) : "memory");
+    if (GATE) {                                              // the gate row of the warp's rows: 256 columns in its staging rows
+        const uint8_t* G = reinterpret_cast<const uint8_t*>(op->ptr[5]) + ((long long)(row0 / op->i[12]) * op->ld[5] + n0) * 2;
+        if (lane < groups * 4) reinterpret_cast<uint4*>(a.stg)[lane] = __ldcg(reinterpret_cast<const uint4*>(G) + lane);
+        __syncwarp();
+    }
     if (!wide_wait(p, c, a)) return;
 #pragma unroll 1
     for (int g0 = 0; g0 < groups; g0 += kDepth) {            // (128 or 256 columns: 4 or 8 steps)
 #pragma unroll
         for (int d = 0; d < kDepth; ++d) {
             const int g = g0 + d;
-            // (the row offsets are computed where they are used: kept for the whole loop they spill)
-            asm volatile("" : "+r"(ldo), "+r"(ldr));
             float v[32];
             tc_ld32(a.tacc + g * 32, v);
             if (g == groups - 1) wide_release(a.release);
             if (a.bias) wide_bias(a.bias, g * 32, v);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(wide_chunk(a.stg, lane, j)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-            __syncwarp();
-            float4 gt = make_float4(1.f, 1.f, 1.f, 1.f);
-            if (GATE) {
-                if (gdt == DT_F16) { Quad<DT_F16> h; h.v = gate[GATE ? d : 0].v; gt = h.get(); }
-                else gt = gate[GATE ? d : 0].get();
-            }
+            for (int j = 0; j < 32; j += 8) {
+                float gt[8], f[8];
+                if (GATE) {
+                    const uint4 w = *reinterpret_cast<const uint4*>(a.stg + (g * 32 + j) * 2);
+                    if (g16) {
+                        const float2 x = unpack2h(w.x), y = unpack2h(w.y), z = unpack2h(w.z), u = unpack2h(w.w);
+                        gt[0] = x.x; gt[1] = x.y; gt[2] = y.x; gt[3] = y.y; gt[4] = z.x; gt[5] = z.y; gt[6] = u.x; gt[7] = u.y;
+                    } else unpack8(w, gt);
+                }
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float4 o = *reinterpret_cast<const float4*>(wide_chunk(a.stg, j * 4 + r, lane & 7));
-                const float4 f = q[d][j].get();
-                if (GATE) o = make_float4(fmaf(o.x, gt.x, f.x), fmaf(o.y, gt.y, f.y), fmaf(o.z, gt.z, f.z), fmaf(o.w, gt.w, f.w));
-                else o = make_float4(o.x + f.x, o.y + f.y, o.z + f.z, o.w + f.w);
-                if (j * 4 + r < rows) put4<ODT>(O + j * 4 * ldo + g * 32 * osz, o);
+                for (int e = 0; e < 8; e += 2) {
+                    if (RDT == DT_F32) { f[e] = __uint_as_float(q[d][(j + e) % kWords]); f[e + 1] = __uint_as_float(q[d][(j + e + 1) % kWords]); }
+                    else if (RDT == DT_F16) { const float2 x = unpack2h(q[d][(j + e) / 2]); f[e] = x.x; f[e + 1] = x.y; }
+                    else { f[e] = bf16_lo(q[d][(j + e) / 2]); f[e + 1] = bf16_hi(q[d][(j + e) / 2]); }
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[j + e] = GATE ? fmaf(v[j + e], gt[e], f[e]) : v[j + e] + f[e];
             }
+            if (live) put32<ODT>(O + g * 32 * osz, v, owhole);
             request(d, g + kDepth);
             __syncwarp();
         }
