@@ -16,6 +16,8 @@
 //   8 swiglu (weight tile = 64 gate rows then 64 up rows; the tile writes 64 output columns),
 //   9 x dtype (DT_BF16 or DT_F16), 10 weight rows per output tile (128, or 256: the n tile argument then
 //   names a pair of 128-row tiles), 11 activation rows per output tile (128 or 256), 12 rows per gate row, 13 gate dtype
+// Rotated heads (ptr 6 cos, 7 sin, or null): the first i 14 output columns are heads of i 15 (64 or 128) columns; row r is rotated
+// (rotate-half) by row r mod i 16 of the tables, of dtype i 17.  No bias, activation or residual beside it.
 // args: 0 m tile, 1 n tile, 2 k split
 #pragma once
 #include "mk_device.cuh"
@@ -170,6 +172,20 @@ static __device__ __noinline__ void op_gemm(const mk_op_desc* op, int a0, int a1
         }
     }
     compute_sync();          // the tile buffers are free for the next instruction
+    if (op->ptr[6]) {        // rotated heads: in place, from the tile as written (behind the barrier)
+        const int D = op->i[15], half = D >> 1, tdt = op->i[17];
+        const void* C = reinterpret_cast<const void*>(op->ptr[6]);
+        const void* S = reinterpret_cast<const void*>(op->ptr[7]);
+#pragma unroll 1
+        for (int u = t; u < BM * (kGemmBN / 2); u += kComputeThreads) {
+            const int r = m0 + u / (kGemmBN / 2), q = u % (kGemmBN / 2), d = q % half, col = n0 + q / half * D + d;
+            if (r >= M || col >= op->i[14]) continue;
+            const long long e = (long long)r * ldo + col, ec = (long long)(r % op->i[16]) * op->ld[6] + d, es = (long long)(r % op->i[16]) * op->ld[7] + d;
+            const float x1 = load1(O, e, odt), x2 = load1(O, e + half, odt);
+            store1(O, e, odt, x1 * load1(C, ec, tdt) - x2 * load1(S, es, tdt));
+            store1(O, e + half, odt, x2 * load1(C, ec + half, tdt) + x1 * load1(S, es + half, tdt));
+        }
+    }
 }
 
 }  // namespace mk

@@ -175,6 +175,49 @@ static __device__ __noinline__ void tc_store_rows_t(const mk_op_desc* op, const 
         else *reinterpret_cast<uint2*>(O + row * ldo * 2) = make_uint2(pack2(f[0], f[1]), pack2(f[2], f[3]));
     }
 }
+// Rotated heads (descriptor: op_gemm.cuh): the other half of a head is in the staging rows too.  All table rows of a warp are
+// requested before the first is used.
+template <int ODT>
+static __device__ __noinline__ void tc_store_rows_rope(const mk_op_desc* op, const float* stage, int m0, int rows, int col0, int n_out) {
+    constexpr int kRows = 128 / kComputeWarps;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int c4 = lane * 4, col = col0 + c4;
+    if (col >= n_out) return;
+    const int D = op->i[15], half = D >> 1, seq = op->i[16], d = c4 & (D - 1);
+    const bool rot = col < op->i[14], low = d < half, t16 = op->i[17] == DT_F16;
+    const int other = low ? c4 + half : c4 - half;
+    const long long ldo = op->ld[2];
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + ((long long)m0 * ldo + col) * 2;
+    uint2 cs[kRows], sn[kRows];
+    if (rot) {
+        int tok = (m0 + warp) % seq;
+#pragma unroll
+        for (int j = 0; j < kRows; ++j) {
+            if (warp + j * kComputeWarps < rows) {
+                cs[j] = __ldcg(reinterpret_cast<const uint2*>(op->ptr[6] + ((long long)tok * op->ld[6] + d) * 2));
+                sn[j] = __ldcg(reinterpret_cast<const uint2*>(op->ptr[7] + ((long long)tok * op->ld[7] + d) * 2));
+            }
+            tok += kComputeWarps;
+            while (tok >= seq) tok -= seq;
+        }
+    }
+    auto get = [&](uint32_t w) { return t16 ? unpack2h(w) : make_float2(bf16_lo(w), bf16_hi(w)); };
+    const float sign = low ? -1.f : 1.f;
+#pragma unroll
+    for (int j = 0; j < kRows; ++j) {
+        const int row = warp + j * kComputeWarps;
+        if (row >= rows) break;
+        float4 f = *reinterpret_cast<const float4*>(stage + row * kTcStagePitch + c4);
+        if (rot) {
+            const float4 g = *reinterpret_cast<const float4*>(stage + row * kTcStagePitch + other);
+            const float2 c01 = get(cs[j].x), c23 = get(cs[j].y), s01 = get(sn[j].x), s23 = get(sn[j].y);
+            f = make_float4(f.x * c01.x + g.x * (sign * s01.x), f.y * c01.y + g.y * (sign * s01.y), f.z * c23.x + g.z * (sign * s23.x),
+                            f.w * c23.y + g.w * (sign * s23.y));
+        }
+        *reinterpret_cast<uint2*>(O + row * ldo * 2) =
+            ODT == DT_F16 ? make_uint2(pack2h(f.x, f.y), pack2h(f.z, f.w)) : make_uint2(pack2(f.x, f.y), pack2(f.z, f.w));
+    }
+}
 template <int ODT>
 __device__ __forceinline__ void tc_store_rows_o(const mk_op_desc* op, const float* stage, int m0, int rows, int col0, int n_out) {
     const int rk = !op->ptr[4] ? 0 : op->i[7] == DT_F32 ? 2 : 1;
@@ -338,6 +381,10 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
     if (ok) {
         if (swi) tc_write_rows(op, stage, m0, rows, 64, a1 * 64, N / 2);
         else if (op->i[6]) tc_write_rows(op, stage, m0, rows, 128, n0, N);              // split-K partial: reduce-add
+        else if (op->ptr[6]) {
+            if (op->i[5] == DT_F16) tc_store_rows_rope<DT_F16>(op, stage, m0, rows, n0, N);
+            else tc_store_rows_rope<DT_BF16>(op, stage, m0, rows, n0, N);
+        }
         else tc_store_rows(op, stage, m0, rows, n0, N);
     }
     tc_fence_before();

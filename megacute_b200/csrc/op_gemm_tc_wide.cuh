@@ -258,11 +258,18 @@ __device__ __forceinline__ void ld32B(const uint8_t* at, uint32_t* w, bool whole
         w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
     }
 }
-// 32 columns of a row, converted
+// 16 columns of a row as 16-bit, 32 columns of a row
+template <int DT>
+__device__ __forceinline__ void put16(uint8_t* at, const float* v, bool whole) {
+    uint32_t w[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) w[e] = DT == DT_F16 ? pack2h(v[2 * e], v[2 * e + 1]) : pack2(v[2 * e], v[2 * e + 1]);
+    st32B(at, w, whole);
+}
 template <int DT>
 __device__ __forceinline__ void put32(uint8_t* at, const float* v, bool whole) {
-    uint32_t w[8];
     if (DT == DT_F32) {
+        uint32_t w[8];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
 #pragma unroll
@@ -270,12 +277,8 @@ __device__ __forceinline__ void put32(uint8_t* at, const float* v, bool whole) {
             st32B(at + 32 * k, w, whole);
         }
     } else {
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-#pragma unroll
-            for (int e = 0; e < 8; ++e) w[e] = DT == DT_F16 ? pack2h(v[16 * k + 2 * e], v[16 * k + 2 * e + 1]) : pack2(v[16 * k + 2 * e], v[16 * k + 2 * e + 1]);
-            st32B(at + 32 * k, w, whole);
-        }
+        put16<DT>(at, v, whole);
+        put16<DT>(at + 32, v + 16, whole);
     }
 }
 
@@ -397,6 +400,84 @@ __device__ __forceinline__ void wide_store_res(const Params& p, Ctrl* c, const m
     }
 }
 
+// 16 columns of this thread's lane, twice
+__device__ __forceinline__ void tc_ld16x2(uint32_t ta, uint32_t tb, float* a, float* b) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]), "=f"(a[7]), "=f"(a[8]), "=f"(a[9]),
+          "=f"(a[10]), "=f"(a[11]), "=f"(a[12]), "=f"(a[13]), "=f"(a[14]), "=f"(a[15]), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(b[3]),
+          "=f"(b[4]), "=f"(b[5]), "=f"(b[6]), "=f"(b[7]), "=f"(b[8]), "=f"(b[9]), "=f"(b[10]), "=f"(b[11]), "=f"(b[12]), "=f"(b[13]),
+          "=f"(b[14]), "=f"(b[15])
+        : "r"(ta), "r"(tb)
+        : "memory");
+}
+// 16-bit outputs whose first i 14 columns are heads (i 15 = 64 or 128 columns each) to be rotated: row r by row r mod i 16 of the 16-bit
+// cos and sin tables (ptr 6, 7).  16 columns of both halves of a head at a time, for all heads of the tile, so that a thread
+// reads its table row once per tile (64 KB beside 128 KB of output; once per head it would be 256).  The first such piece of
+// the tables is requested into registers while the main loop runs, the one after the current into the thread's 128 bytes of the
+// warp's staging rows (a second set of registers spills).
+template <bool F16, bool T16>
+__device__ __forceinline__ void wide_store_rope(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
+    constexpr int ODT = F16 ? DT_F16 : DT_BF16;
+    const int lane = threadIdx.x & 31;
+    const int cols = op->i[10], D = op->i[15], half = D >> 1, rot = op->i[14] - n0;
+    const bool live = row0 + lane < op->i[0];
+    const int row = live ? row0 + lane : op->i[0] - 1, tok = row % op->i[16];
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + ((long long)row * op->ld[2] + n0) * 2;
+    const uint8_t* C = reinterpret_cast<const uint8_t*>(op->ptr[6]) + (long long)tok * op->ld[6] * 2;
+    const uint8_t* S = reinterpret_cast<const uint8_t*>(op->ptr[7]) + (long long)tok * op->ld[7] * 2;
+    const bool whole = ((op->ptr[2] | (uint64_t)op->ld[2] * 2) & 31) == 0;
+    uint4 q[8];                                              // cos of both halves, sin of both halves
+    auto from = [&](int k, int d) { return (k < 4 ? C : S) + (d + (k & 2 ? half : 0)) * 2 + (k & 1) * 16; };
+    auto next = [&](int d) {
+        if (d < half && rot > 0)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) cp_async16(wide_chunk(a.stg, lane, k), from(k, d), true);
+        cp_async_commit();
+    };
+    auto get = [&](uint32_t w) { return T16 ? unpack2h(w) : make_float2(bf16_lo(w), bf16_hi(w)); };
+    if (rot > 0)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) q[k] = __ldcg(reinterpret_cast<const uint4*>(from(k, 0)));
+    next(16);
+    if (!wide_wait(p, c, a)) return;
+#pragma unroll 1
+    for (int d = 0;;) {
+#pragma unroll 1
+        for (int h = 0; h < cols; h += D) {
+            float x1[16], x2[16];
+            __syncwarp();
+            tc_ld16x2(a.tacc + h + d, a.tacc + h + half + d, x1, x2);
+            if (d + 16 == half && h + D == cols) wide_release(a.release);
+            if (h < rot) {
+#pragma unroll
+                for (int e = 0; e < 16; e += 2) {
+                    const uint32_t* t = reinterpret_cast<const uint32_t*>(q);
+                    const float2 c1 = get(t[e / 2]), c2 = get(t[8 + e / 2]), s1 = get(t[16 + e / 2]), s2 = get(t[24 + e / 2]);
+                    const float u0 = x1[e], v0 = x2[e], u1 = x1[e + 1], v1 = x2[e + 1];
+                    x1[e] = u0 * c1.x - v0 * s1.x;
+                    x2[e] = v0 * c2.x + u0 * s2.x;
+                    x1[e + 1] = u1 * c1.y - v1 * s1.y;
+                    x2[e + 1] = v1 * c2.y + u1 * s2.y;
+                }
+            }
+            if (live) {
+                put16<ODT>(O + (h + d) * 2, x1, whole);
+                put16<ODT>(O + (h + half + d) * 2, x2, whole);
+            }
+        }
+        d += 16;
+        if (d >= half) break;
+        asm volatile("cp.async.wait_all;" ::: "memory");     // (the thread's own copies)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) q[k] = *wide_chunk(a.stg, lane, k);
+        next(d + 16);
+    }
+    __syncwarp();
+}
+
 // Everything else -- fp32 output, split-K partial (reduce-add), an activation in front of a residual: the same without requests ahead.
 __device__ __forceinline__ void wide_store_any(const Params& p, Ctrl* c, const mk_op_desc* op, const WideAcc& a, int row0, int n0) {
     const int lane = threadIdx.x & 31;
@@ -456,14 +537,15 @@ __device__ __forceinline__ void wide_store_any(const Params& p, Ctrl* c, const m
 // The epilogue of an op, chosen once per run of instructions: each has a function of its own around it (op_gemm_wide.cu) and so a
 // register allocation of its own -- called per instruction they pay ~60 saved and restored registers each time, inlined
 // side by side they spill, and with the shared memory taken every such access is an L2 round trip behind the operand stream.
-// WIDE_PLAIN .. WIDE_ACT: + 16 for fp16 output.  WIDE_RES: + residual dtype | output dtype << 2 | gate << 4.
-enum { WIDE_PLAIN = 0, WIDE_SWIGLU, WIDE_GELU, WIDE_ACT, WIDE_ANY, WIDE_RES = 32 };
+// WIDE_PLAIN .. WIDE_ROPE_T16 (fp16 tables): + 16 for fp16 output.  WIDE_RES: + residual dtype | output dtype << 2 | gate << 4.
+enum { WIDE_PLAIN = 0, WIDE_SWIGLU, WIDE_GELU, WIDE_ACT, WIDE_ANY, WIDE_ROPE, WIDE_ROPE_T16, WIDE_RES = 32 };
 __device__ __forceinline__ int wide_variant(const mk_op_desc* op) {
     const int odt = op->i[5];
     if (op->i[6]) return WIDE_ANY;
     const bool gate32 = !op->ptr[5] || (op->i[12] % 32 == 0 && op->i[13] != DT_F32);         // a warp's 32 rows share a 16-bit gate row
     if (op->ptr[4]) return op->i[3] == ACT_NONE && !op->i[8] && gate32 ? WIDE_RES + (op->i[7] | odt << 2 | (op->ptr[5] ? 16 : 0)) : WIDE_ANY;
     if (odt == DT_F32) return WIDE_ANY;
+    if (op->ptr[6]) return (op->i[17] == DT_F16 ? WIDE_ROPE_T16 : WIDE_ROPE) + (odt == DT_F16 ? 16 : 0);
     const int v = op->i[8] ? WIDE_SWIGLU : op->i[3] == ACT_NONE ? WIDE_PLAIN : op->i[3] == ACT_GELU ? WIDE_GELU : WIDE_ACT;
     return v + (odt == DT_F16 ? 16 : 0);
 }
@@ -516,6 +598,7 @@ __device__ __forceinline__ void op_gemm_tc_wide(const Params& p, Ctrl* c, uint8_
         if constexpr (kind == WIDE_PLAIN) wide_store16<f16, false, 0>(p, c, op, a, row0, n0);
         else if constexpr (kind == WIDE_SWIGLU) wide_store16<f16, true, 0>(p, c, op, a, row0, n0);
         else if constexpr (kind == WIDE_GELU) wide_store16<f16, false, 1>(p, c, op, a, row0, n0);
+        else if constexpr (kind == WIDE_ROPE || kind == WIDE_ROPE_T16) wide_store_rope<f16, kind == WIDE_ROPE_T16>(p, c, op, a, row0, n0);
         else if constexpr (kind == WIDE_ACT) wide_store16<f16, false, 2>(p, c, op, a, row0, n0);
         else wide_store_any(p, c, op, a, row0, n0);
     }

@@ -29,6 +29,7 @@ __device__ int mk_run_gemm_wide(const Params& p, int idx, int slot) {
         switch (wide_variant(&mt->desc[slot & 1])) {
 #define MK_W(V) case (V): last = wide_run<(V)>(p, idx, slot); break
             MK_W(WIDE_PLAIN); MK_W(WIDE_SWIGLU); MK_W(WIDE_GELU); MK_W(WIDE_ACT);
+            MK_W(WIDE_ROPE); MK_W(WIDE_ROPE + 16); MK_W(WIDE_ROPE_T16); MK_W(WIDE_ROPE_T16 + 16);
             MK_W(WIDE_PLAIN + 16); MK_W(WIDE_SWIGLU + 16); MK_W(WIDE_GELU + 16); MK_W(WIDE_ACT + 16);
 #define MK_WR(R) MK_W(WIDE_RES + (R)); MK_W(WIDE_RES + ((R) | DT_F32 << 2)); MK_W(WIDE_RES + ((R) | DT_F16 << 2)); \
                  MK_W(WIDE_RES + ((R) | 16)); MK_W(WIDE_RES + ((R) | DT_F32 << 2 | 16)); MK_W(WIDE_RES + ((R) | DT_F16 << 2 | 16))

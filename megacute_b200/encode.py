@@ -110,11 +110,14 @@ def fill(d, op: Op, addr) -> None:
         split = k == "LinearSplit"
         out = op.ws if split else op.out
         gate = None if split else op.gate
-        ptrs = [op.x, op.w, out, None if split else op.bias, None if split else op.residual, gate]
+        rope = None if split else op.cos
+        ptrs = [op.x, op.w, out, None if split else op.bias, None if split else op.residual, gate, rope, op.sin if rope is not None else None]
         act = None if split else op.act
         ints = [op.x.rows, op.w.rows, op.x.cols, C.ACT_CODE[act], op.splits if split else 1, dt(out), int(split),
                 0 if split else dt(op.residual), int(act == "swiglu"), dt(op.x), int(op.bn or C.GEMM_BN), gemm_rows(op),
                 int(op.gate_group) if gate is not None else 1, dt(gate)]
+        if rope is not None:
+            ints += [op.rope_cols, op.head_dim, op.seq, dt(rope)]
     elif k == "SplitFinalize":
         d.kind = C.OP_FINALIZE
         ptrs = [op.ws, op.out, op.bias, op.residual]

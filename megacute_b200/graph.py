@@ -108,7 +108,8 @@ class View:
 # An operand listed in both columns is updated in place by the op.  Optional operands may be
 # None.  The semantic definition of each kind is in the builder method's docstring below.
 OP_TABLE = {
-    "Linear":          (("x", "w", "bias", "residual", "norm_w", "gate"), ("out",), ("act", "rms_eps", "bm", "bn", "gate_group")),
+    "Linear":          (("x", "w", "bias", "residual", "norm_w", "gate", "cos", "sin"), ("out",),
+                        ("act", "rms_eps", "bm", "bn", "gate_group", "rope_cols", "head_dim", "seq")),
     "LinearSplit":     (("x", "w", "norm_w"), ("ws",), ("splits", "rms_eps", "bm", "bn")),
     "SplitFinalize":   (("ws", "bias", "residual"), ("out", "ws"), ("act",)),
     "Unary":           (("x",), ("out",), ("fn",)),

@@ -503,8 +503,58 @@ def fuse_gated_linear(g: Graph) -> Graph:
     return out
 
 
+def fuse_rope_linear(g: Graph) -> Graph:
+    """A tile linear whose leading output columns are read only by Ropes whose results go to prefill attention rotates them in
+    its epilogue: the heads lie whole in a tile and the fp32 accumulators are at hand, so two passes over q and k, their
+    dependency hop and a rounding go.  q and k stay where they are, side by side with v.  (With head_dim 64 or 128, 16-bit tables and
+    nothing else between product and rotation: what the epilogues know.)  MEGACUTE_B200_NO_POINTWISE_FUSION=1 keeps the ops apart."""
+    if os.environ.get("MEGACUTE_B200_NO_POINTWISE_FUSION") == "1":
+        return g
+    out = g.derive()
+    ops = list(g.ops)
+    alias: dict[int, View] = {}
+    fused: dict[int, Op] = {}
+    for i, lin in enumerate(ops):
+        if (lin.kind != "Linear" or gemv_eligible(lin.x.rows, lin.x.cols) or lin.act is not None or lin.bias is not None
+                or lin.residual is not None or lin.gate is not None or lin.rms_eps is not None):
+            continue
+        buf = lin.out.buf
+        if buf.kind != "temp" or lin.out.rect != (0, buf.rows, 0, buf.cols) or any(v.buf is buf for v in g.outputs):
+            continue
+        ropes = [k for k in range(i + 1, len(ops)) if ops[k].kind == "Rope" and ops[k].x.buf is buf]
+        if not ropes:
+            continue
+        first, col = ops[ropes[0]], 0
+        ok = first.head_dim in (64, 128) and first.cos.buf.dtype != torch.float32
+        for k in sorted(ropes, key=lambda k: ops[k].x.col0):
+            r = ops[k]
+            ok = (ok and r.x.rect == (0, buf.rows, col, col + r.x.cols) and r.x.cols == r.heads * r.head_dim
+                  and r.cos.same(first.cos) and r.sin.same(first.sin) and (r.seq, r.head_dim) == (first.seq, first.head_dim)
+                  and r.cos.buf.dtype == r.sin.buf.dtype and r.out.buf.kind == "temp" and r.out.buf is not buf
+                  and r.out.rect == (0, r.out.buf.rows, 0, r.out.buf.cols) and not any(v.buf is r.out.buf for v in g.outputs)
+                  and all(o.kind == "Attention" for o in ops if any(v.buf is r.out.buf for v in o.reads))
+                  and sum(any(v.buf is r.out.buf for v in o.writes) for o in ops) == 1)
+            col += r.x.cols
+        # nothing else touches the columns that are now rotated in place
+        for k, o in enumerate(ops):
+            if k != i and k not in ropes:
+                ok = ok and not any(v.buf is buf for v in o.writes) and not any(v.buf is buf and v.col0 < col for v in o.reads)
+        if not ok:
+            continue
+        fused[i] = lin.clone(cos=first.cos, sin=first.sin, rope_cols=col, head_dim=first.head_dim, seq=first.seq)
+        for k in ropes:
+            alias[ops[k].out.buf.id] = ops[k].x
+            fused[k] = None
+    out.ops = []
+    for i, op in enumerate(ops):
+        op = fused.get(i, op)
+        if op is not None:
+            out.ops.append(op.clone(**{k: _retarget(v, alias) for k, v in op.view_fields()}) if alias else op)
+    return out
+
+
 def run_all(g: Graph, sm_count: int) -> Graph:
     """The pass pipeline of ``compile`` (reference order: runtime.py:235, plus wide_tiles, split_argmax,
-    fuse_pointwise, fuse_gated_linear, promote_temps and fuse_finalize_attention)."""
+    fuse_pointwise, fuse_gated_linear, fuse_rope_linear, promote_temps and fuse_finalize_attention)."""
     g = split_argmax(split_kv(fuse_rope_attention(wide_tiles(split_k(fold_norms(g), sm_count), sm_count)), sm_count), sm_count)
-    return fuse_finalize_attention(promote_temps(fuse_gated_linear(fuse_pointwise(g))))
+    return fuse_finalize_attention(promote_temps(fuse_rope_linear(fuse_gated_linear(fuse_pointwise(g)))))

@@ -151,6 +151,7 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
             if op.gate is not None:
                 gg = op.gate_group
                 acc.append(_acc(op.gate, READ, r0 // gg, -(-np.minimum(r1, M) // gg), nn * on, (nn + 1) * on, n=n, covers=False))
+            acc += [_acc(op.cos, READ, n=n), _acc(op.sin, READ, n=n)]
             assert op.norm_w is None and op.rms_eps is None, "norm folding is only done on the streaming path"
         return Tiled(_args(n, m, nn, ks), [a for a in acc if a is not None])
     if k in ("SplitFinalize", "Unary", "Binary", "SwiGLU", "Modulate", "Rope"):

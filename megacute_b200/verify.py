@@ -60,6 +60,8 @@ def operand_windows(op) -> dict:
             win.update(bias=(1, n_out), residual=(M, n_out), norm_w=(1, K))
             if op.gate is not None:
                 win["gate"] = (_ceil(M, op.gate_group), n_out)
+            if op.cos is not None:
+                win.update(cos=(min(op.seq, M), op.head_dim), sin=(min(op.seq, M), op.head_dim))
         return win
     if k == "SplitFinalize":
         R, Cc = op.out.shape

@@ -162,6 +162,10 @@ class Evaluator:
                 y = y * self.rd(o.gate).repeat_interleave(o.gate_group, 0)
             if o.residual is not None:
                 y = y + self.rd(o.residual)
+            if getattr(o, "cos", None) is not None:     # (this repository's fused form: the first rope_cols columns rotated)
+                p = torch.arange(y.shape[0], device=self.dev) % o.seq
+                n = o.rope_cols
+                y = torch.cat([rotate_half(y[:, :n], self.rd(o.cos)[p], self.rd(o.sin)[p], o.head_dim), y[:, n:]], 1)
         self.wr(o.out, y)
 
     def op_LinearSplit(self, o):
