@@ -415,7 +415,7 @@ static bool encode_tile_map(void* out, uint64_t base, long long rows, long long 
 static bool tile_gemm_on_tcgen05(const mk_op_desc& d) {
     const int N = d.i[1], K = d.i[2], splits = d.i[4], odt = d.i[5], rdt = d.i[7], swi = d.i[8];
     if (d.i[11] == 256 && N % 128) return false;              // (the 256-row tiles' epilogue has whole columns only)
-    if (splits <= 0 || K % splits || (K / splits) % 64) return false;
+    if (splits <= 0 || K % 64 || d.i[18] % 64) return false;
     const int n_out = swi ? N / 2 : N;
     if (n_out % 8 || (swi && N % 128)) return false;
     auto vec_ok = [](uint64_t ptr, int ld, int dt) { return !(ptr & 15) && ld % (dt == 1 ? 4 : 8) == 0; };
@@ -449,11 +449,15 @@ static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
                     if (!(0 <= a0 && a0 < a1 && a1 <= d.i[1])) why = "streaming linear: output range outside [0, N)";
                     break;
                 case MK_OP_GEMM:
-                    if (d.i[4] <= 0) why = "tile GEMM: split count";
+                    if (d.i[4] <= 0 || d.i[18] <= 0 || d.i[19] < 0 || d.i[19] >= d.i[4] ||
+                        (long long)d.i[18] * d.i[4] + (long long)d.i[19] * (d.i[2] & 63 ? 32 : 64) != d.i[2])
+                        why = "tile GEMM: split count";
                     else if (a0 < 0 || a0 * (long long)(d.i[11] == 256 ? 256 : 128) >= d.i[0]) why = "tile GEMM: m tile outside M";
                     else if (d.i[10] != 0 && d.i[10] != 128 && !(d.i[10] == 256 && d.i[11] == 256 && d.i[1] % 256 == 0)) why = "tile GEMM: weight rows per tile";
                     else if (a1 < 0 || a1 * (long long)(d.i[10] == 256 ? 256 : 128) >= d.i[1]) why = "tile GEMM: n tile outside N";
                     else if (a2 < 0 || a2 >= d.i[4]) why = "tile GEMM: K split index";
+                    else if (d.ptr[6] && ((d.i[15] != 64 && d.i[15] != 128) || d.i[16] <= 0 || d.i[14] % d.i[15] || d.i[14] > d.i[1]))
+                        why = "tile GEMM: rotated heads";
                     else if (d.ptr[5] && d.i[12] <= 0) why = "tile GEMM: rows per gate row";
                     break;
                 case MK_OP_FINALIZE:

@@ -117,6 +117,14 @@ struct Params {
 // a tile GEMM bound to the tcgen05 body with 256-row tiles (op_gemm_tc_wide.cuh)
 __device__ __forceinline__ bool is_wide_gemm(const mk_op_desc* op) { return op->kind == MK_OP_GEMM && op->i[11] == 256 && op->ptr[11] != 0; }
 
+// K range of a tile GEMM's K split `s`: i 18 columns, the first i 19 splits a k-tile (64; K not a multiple of 64: 32) more, so that any
+// number of splits may be chosen.  The host has divided: the producer warp meets this on the way to its next weight tile.
+__device__ __forceinline__ void gemm_k_range(const mk_op_desc* op, int s, int& kbeg, int& kc) {
+    const int unit = op->i[2] & 63 ? 32 : 64, base = op->i[18], more = op->i[19];
+    kbeg = s * base + min(s, more) * unit;
+    kc = base + (s < more ? unit : 0);
+}
+
 // a prefill attention bound to the tcgen05 body (op_attention_tc.cuh)
 __device__ __forceinline__ bool is_attention_tc(const mk_op_desc* op) { return op->kind == MK_OP_ATTENTION && op->ptr[11] != 0; }
 

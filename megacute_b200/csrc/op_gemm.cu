@@ -22,7 +22,7 @@ __device__ int mk_run_gemm(const Params& p, int idx, int slot) {
                 if (mt * 128 >= op->i[0]) break;
                 // ops with at most 64 activation rows have a single m tile: hold 64 rows and stream deeper
                 if (op->i[0] <= 64) {
-                    if ((op->i[2] / op->i[4]) % 64 == 0) op_gemm<64, 64, 3>(op, mt, n, a2, m.work);
+                    if (op->i[2] % 64 == 0) op_gemm<64, 64, 3>(op, mt, n, a2, m.work);
                     else op_gemm<64, 32, 6>(op, mt, n, a2, m.work);
                 } else {
                     op_gemm<128, 32, 4>(op, mt, n, a2, m.work);

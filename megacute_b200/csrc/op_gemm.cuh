@@ -12,10 +12,11 @@
 // weight bytes in flight.
 //
 // ptr 0 x, 1 w, 2 out (or ws), 3 bias, 4 residual, 5 gate (out = residual + act(.) * gate[r / i12], 256-row tiles only; or null)
-// i 0 M, 1 N (weight rows), 2 K, 3 act, 4 splits, 5 out dtype, 6 accumulate, 7 residual dtype,
+// i 0 M, 1 N (weight rows), 2 K, 3 act, 4 K splits, 5 out dtype, 6 accumulate, 7 residual dtype,
 //   8 swiglu (weight tile = 64 gate rows then 64 up rows; the tile writes 64 output columns),
 //   9 x dtype (DT_BF16 or DT_F16), 10 weight rows per output tile (128, or 256: the n tile argument then
 //   names a pair of 128-row tiles), 11 activation rows per output tile (128 or 256), 12 rows per gate row, 13 gate dtype
+// K split s takes i 18 columns, the first i 19 splits one k-tile more (gemm_k_range).
 // Rotated heads (ptr 6 cos, 7 sin, or null): the first i 14 output columns are heads of i 15 (64 or 128) columns; row r is rotated
 // (rotate-half) by row r mod i 16 of the tables, of dtype i 17.  No bias, activation or residual beside it.
 // args: 0 m tile, 1 n tile, 2 k split
@@ -35,13 +36,15 @@ static __device__ __noinline__ void op_gemm(const mk_op_desc* op, int a0, int a1
     constexpr int MI = BM / 32;
     constexpr int kATileBytes = BM * kGemmRowBytes, kBTileBytes = kGemmBN * kGemmRowBytes;
     static_assert(kGemmStages * (kATileBytes + kBTileBytes) <= kWorkBytes, "GEMM stages exceed the work area");
-    const int M = op->i[0], N = op->i[1], K = op->i[2], act = op->i[3], splits = op->i[4];
+    const int M = op->i[0], N = op->i[1], act = op->i[3];
     const int odt = op->i[5], accum = op->i[6], rdt = op->i[7], swi = op->i[8];
     const bool xh = op->i[9] == DT_F16;
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int wm = warp >> 2, wn = warp & 3;
     const int m0 = a0 * kGemmBM, n0 = a1 * kGemmBN;
-    const int kc = K / splits, kbeg = a2 * kc, nk = kc / kGemmBK;
+    int kbeg, kc;
+    gemm_k_range(op, a2, kbeg, kc);
+    const int nk = kc / kGemmBK;
     const __nv_bfloat16* X = reinterpret_cast<const __nv_bfloat16*>(op->ptr[0]);
     const __nv_bfloat16* Wt = reinterpret_cast<const __nv_bfloat16*>(op->ptr[1]);
     const long long ldx = op->ld[0], ldw = op->ld[1];

@@ -241,10 +241,12 @@ __device__ __forceinline__ void tc_store_rows(const mk_op_desc* op, const float*
 __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* ring, uint8_t* work, const mk_op_desc* op, int a0,
                                           int a1, int a2, int seq) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const int M = op->i[0], N = op->i[1], K = op->i[2], splits = op->i[4];
+    const int M = op->i[0], N = op->i[1];
     const int swi = op->i[8];
     const int m0 = a0 * 128, n0 = a1 * 128;
-    const int kc = K / splits, kbeg = a2 * kc, nk = kc / 64;
+    int kbeg, kc;
+    gemm_k_range(op, a2, kbeg, kc);
+    const int nk = kc / 64;
     const uint8_t* tmaps = reinterpret_cast<const uint8_t*>(op->ptr[11]);
     uint8_t* xs = work + kTcXOff;
     // activation stages: whole 128-row tiles, or twice as many 64-row half tiles

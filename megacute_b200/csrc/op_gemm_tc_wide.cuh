@@ -37,7 +37,9 @@ struct WideFeed {
 __device__ __forceinline__ bool wide_feed(const Params& p, Ctrl* c, uint8_t* ring, const mk_op_desc* op, const Inst& in, bool first,
                                           WideFeed& f) {
     const int lane = threadIdx.x & 31;
-    const int M = op->i[0], kc = op->i[2] / op->i[4], kbeg = in.a2 * kc, nk = kc / 64, m0 = in.a0 * 256;
+    int kbeg, kc;
+    gemm_k_range(op, in.a2, kbeg, kc);
+    const int M = op->i[0], nk = kc / 64, m0 = in.a0 * 256;
     const uint8_t* tmaps = reinterpret_cast<const uint8_t*>(op->ptr[11]);
     bool ok = true;
     if (first) {

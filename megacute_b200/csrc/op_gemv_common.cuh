@@ -111,10 +111,11 @@ struct StageCursor {
             if (attn) { gemm = false; kv = false; seq = in.seq; return; }
             if (op->kind == MK_OP_GEMM && op->ptr[11]) {
                 // a 256-row output tile (i 11; slots of its own) takes one or two 128-row weight tiles (i 10) per k-tile
-                const int kc = op->i[2] / op->i[4];
+                int kc;
+                gemm_k_range(op, in.a2, kbeg, kc);
                 wide = is_wide_gemm(op) ? op->i[10] >> 7 : 0;
                 reread = op->i[0] > 256;      // (two row tiles run side by side and share the line in flight: measured, evict-first is then the faster)
-                gemm = true; kv = false; seq = in.seq; kt = 0; nk = kc / 64; kbeg = in.a2 * kc; n0 = in.a1 * 128 * max(wide, 1);
+                gemm = true; kv = false; seq = in.seq; kt = 0; nk = kc / 64; n0 = in.a1 * 128 * max(wide, 1);
                 wmap = reinterpret_cast<const uint8_t*>(op->ptr[11]) + 128;
                 wpack = reinterpret_cast<const uint8_t*>(op->ptr[10]);
                 wstride = (op->i[1] + 127) / 128;

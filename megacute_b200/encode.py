@@ -38,7 +38,7 @@ import torch
 
 from . import config as C
 from .graph import DTYPE_CODE, ELEM_BYTES, Op, View
-from .schedule import argmax_chunk_cols, ew_rows, finalize_rows, gemm_rows, is_gemv, norm_rows
+from .schedule import argmax_chunk_cols, ew_rows, finalize_rows, gemm_k_split, gemm_rows, is_gemv, norm_rows
 
 BF16 = torch.bfloat16
 F16 = torch.float16
@@ -116,8 +116,8 @@ def fill(d, op: Op, addr) -> None:
         ints = [op.x.rows, op.w.rows, op.x.cols, C.ACT_CODE[act], op.splits if split else 1, dt(out), int(split),
                 0 if split else dt(op.residual), int(act == "swiglu"), dt(op.x), int(op.bn or C.GEMM_BN), gemm_rows(op),
                 int(op.gate_group) if gate is not None else 1, dt(gate)]
-        if rope is not None:
-            ints += [op.rope_cols, op.head_dim, op.seq, dt(rope)]
+        ints += [op.rope_cols, op.head_dim, op.seq, dt(rope)] if rope is not None else [0, 0, 1, 0]
+        ints += gemm_k_split(op.x.cols, op.splits if split else 1)[:2]
     elif k == "SplitFinalize":
         d.kind = C.OP_FINALIZE
         ptrs = [op.ws, op.out, op.bias, op.residual]

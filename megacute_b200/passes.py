@@ -207,7 +207,9 @@ def _retarget(v, alias):
 
 def choose_k_splits(M: int, N: int, K: int, sm_count: int) -> int:
     """Split count for a tile GEMM.  Cost of a plan = waves x (fixed cost per instruction + operand
-    bytes of one instruction at one SM's share of HBM bandwidth)."""
+    bytes of one instruction at one SM's share of HBM bandwidth).  Even splits only: six or nine of uneven length, which fill
+    144 of 148 SMs where four or eight fill 96 or 128, cost in reduce-adds what they save in streaming (batch-64 decode 0.2 %
+    slower)."""
     bm, bn, bk = C.GEMM_BM, C.GEMM_BN, C.GEMM_BK
     mt, nt, kt = -(-M // bm), -(-N // bn), K // bk
     rows = min(M, bm)
@@ -238,11 +240,10 @@ def plan_tiles(M: int, N: int, K: int, sm_count: int, max_splits: int, finalize:
         if bm != C.GEMM_BM and N % bn:
             continue
         for s in range(1, max_splits + 1):
-            whole = K % (64 * s) == 0
-            if (s > 1 and (K % (C.GEMM_BK * s) or K // C.GEMM_BK // s < C.MIN_SPLIT_KTILES)) or (bm != C.GEMM_BM and not whole):
+            if (s > 1 and K // s < C.MIN_SPLIT_KTILES * C.GEMM_BK) or (bm != C.GEMM_BM and K % 64):
                 continue
             rounds = -(-(-(-M // bm) * -(-N // bn) * s) // sm_count)
-            cost = rounds * (K / 64 / s * k + tile) + once + (M * N * s * 4 / (C.REDUCE_GBPS * 1e3) + (C.FINALIZE_US if finalize else 0.0) if s > 1 else 0.0)
+            cost = rounds * (-(-(K / 64) // s) * k + tile) + once + (M * N * s * 4 / (C.REDUCE_GBPS * 1e3) + (C.FINALIZE_US if finalize else 0.0) if s > 1 else 0.0)
             if cost < best_cost - 1e-9:
                 best, best_cost = (s, bm, bn), cost
     return best
@@ -415,9 +416,9 @@ def wide_tiles(g: Graph, sm_count: int) -> Graph:
             M, K = op.x.shape
             N = op.w.rows
             splits = op.splits if op.kind == "LinearSplit" else 1
-            if M > C.WIDE_MIN_ROWS and K % (64 * splits) == 0 and force != "0":
+            if M > C.WIDE_MIN_ROWS and K % 64 == 0 and force != "0":
                 # (a split op is planned as `splits` independent products over K / splits)
-                _, bm, bn = plan_tiles(M, N, K // splits, max(1, sm_count // splits), 1, False)
+                _, bm, bn = plan_tiles(M, N, -(-K // 64 // splits) * 64, max(1, sm_count // splits), 1, False)
                 if force == "1" and N % C.GEMM_BN_WIDE == 0:
                     bm, bn = C.GEMM_BM_WIDE, C.GEMM_BN_WIDE
                 if bm != C.GEMM_BM:

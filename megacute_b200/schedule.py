@@ -113,6 +113,15 @@ def gemm_rows(op: Op) -> int:
     return op.bm or C.GEMM_BM
 
 
+def gemm_k_split(K: int, splits: int) -> tuple:
+    """(columns of a K split, number of leading splits that take one k-tile more, columns of a k-tile): whole k-tiles, as even
+    as they go."""
+    unit = 64 if K % 64 == 0 else C.GEMM_BK
+    per, more = divmod(K // unit, splits)
+    assert per > 0, f"linear K={K} has fewer k-tiles than its {splits} splits"
+    return per * unit, more, unit
+
+
 def tile_op(op: Op, sm_count: int) -> Tiled:
     k = op.kind
     if k == "Linear" and is_gemv(op):
@@ -138,12 +147,13 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
         on = BN // 2 if swi else BN
         m, nn = gemm_raster(_ceil(M, BM), _ceil(out.cols, on), 8 * C.GEMM_BM // BM)
         splits = op.splits if k == "LinearSplit" else 1
-        kc = op.x.cols // splits
+        kc, more, ku = gemm_k_split(op.x.cols, splits)
         m, nn, ks = np.repeat(m, splits), np.repeat(nn, splits), np.tile(np.arange(splits), len(m))
         n = len(m)
         r0, r1 = m * BM, (m + 1) * BM
-        acc = [_acc(op.x, READ, r0, r1, ks * kc, (ks + 1) * kc, n=n),
-               _acc(op.w, READ, nn * BN, (nn + 1) * BN, ks * kc, (ks + 1) * kc, n=n),
+        k0, k1 = ks * kc + np.minimum(ks, more) * ku, (ks + 1) * kc + np.minimum(ks + 1, more) * ku
+        acc = [_acc(op.x, READ, r0, r1, k0, k1, n=n),
+               _acc(op.w, READ, nn * BN, (nn + 1) * BN, k0, k1, n=n),
                _acc(out, ACCUM if k == "LinearSplit" else WRITE, r0, r1, nn * on, (nn + 1) * on, n=n)]
         if k == "Linear":
             acc += [_acc(op.bias, READ, 0, 1, nn * on, (nn + 1) * on, n=n),
