@@ -205,11 +205,12 @@ def _retarget(v, alias):
     return View(r.buf, r.row0 + v.row0, r.col0 + v.col0, v.rows, v.cols)
 
 
-def choose_k_splits(M: int, N: int, K: int, sm_count: int) -> int:
+def choose_k_splits(M: int, N: int, K: int, sm_count: int, finalize: bool) -> int:
     """Split count for a tile GEMM.  Cost of a plan = waves x (fixed cost per instruction + operand
     bytes of one instruction at one SM's share of HBM bandwidth).  Even splits only: six or nine of uneven length, which fill
     144 of 148 SMs where four or eight fill 96 or 128, cost in reduce-adds what they save in streaming (batch-64 decode 0.2 %
-    slower)."""
+    slower).  A SplitFinalize behind the op is a dependency hop of its own (adaLN modulations of 32 images, K = 1024: two splits
+    and it 14 us, one instruction per tile 10)."""
     bm, bn, bk = C.GEMM_BM, C.GEMM_BN, C.GEMM_BK
     mt, nt, kt = -(-M // bm), -(-N // bn), K // bk
     rows = min(M, bm)
@@ -223,7 +224,7 @@ def choose_k_splits(M: int, N: int, K: int, sm_count: int) -> int:
     for s in range(2, C.MAX_K_SPLITS + 1):
         if kt % s or kt // s < C.MIN_SPLIT_KTILES:
             continue
-        c = cost(mt * nt * s, K // s)
+        c = cost(mt * nt * s, K // s) + (C.FINALIZE_US if finalize else 0.0)
         if c < best_cost:
             best, best_cost = s, c
     return best
@@ -266,7 +267,9 @@ def split_k(g: Graph, sm_count: int) -> Graph:
             if M > C.WIDE_MIN_ROWS:
                 s = plan_tiles(M, op.w.rows, K, sm_count, C.MAX_K_SPLITS, not inplace)[0]
             else:
-                s = choose_k_splits(M, op.w.rows, K, sm_count)
+                # (the fused decode attention reads the sums itself: fuse_finalize_attention)
+                hop = not inplace and not any(o.kind in ("RopeAppend", "DecodeAttention") and any(v.buf is op.out.buf for v in o.reads) for o in src[i + 1:])
+                s = choose_k_splits(M, op.w.rows, K, sm_count, hop)
             if s > 1:
                 if inplace:
                     alias[op.out.buf.id] = r
