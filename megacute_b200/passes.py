@@ -557,8 +557,35 @@ def fuse_rope_linear(g: Graph) -> Graph:
     return out
 
 
+HOIST_MIN_OPS = 4
+
+
+def hoist_linears(g: Graph) -> Graph:
+    """A linear whose operands are ready HOIST_MIN_OPS or more ops before its place moves up behind the last op it depends on.
+    An SM runs its instructions in order: the adaLN modulation of a DiT block, which only needs the conditioning vector, cost every
+    block its 10 us among ops that wait for one another (its weights cold, half the SMs without a tile); one behind the
+    other, the modulations of all blocks stream at the rate of HBM."""
+    out = g.derive()
+    ops: list[Op] = []
+    for op in g.ops:
+        j = len(ops)
+        if op.kind in ("Linear", "LinearSplit", "SplitFinalize"):
+            reads, writes = {v.buf.id for v in op.reads}, {v.buf.id for v in op.writes}
+            while j > 0:
+                o = ops[j - 1]
+                w = {v.buf.id for v in o.writes}
+                if w & (reads | writes) or writes & {v.buf.id for v in o.reads}:
+                    break
+                j -= 1
+            if len(ops) - j < HOIST_MIN_OPS:
+                j = len(ops)
+        ops.insert(j, op)
+    out.ops = ops
+    return out
+
+
 def run_all(g: Graph, sm_count: int) -> Graph:
     """The pass pipeline of ``compile`` (reference order: runtime.py:235, plus wide_tiles, split_argmax,
-    fuse_pointwise, fuse_gated_linear, fuse_rope_linear, promote_temps and fuse_finalize_attention)."""
+    fuse_pointwise, fuse_gated_linear, fuse_rope_linear, promote_temps, fuse_finalize_attention and hoist_linears)."""
     g = split_argmax(split_kv(fuse_rope_attention(wide_tiles(split_k(fold_norms(g), sm_count), sm_count)), sm_count), sm_count)
-    return fuse_finalize_attention(promote_temps(fuse_rope_linear(fuse_gated_linear(fuse_pointwise(g)))))
+    return hoist_linears(fuse_finalize_attention(promote_temps(fuse_rope_linear(fuse_gated_linear(fuse_pointwise(g))))))
