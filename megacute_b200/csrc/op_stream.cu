@@ -1,7 +1,7 @@
 // Translation unit of the ops that stream activations: pointwise tiles and norms of many rows.  Every variant is a function of its
 // own around the walk, with the registers it needs: inlined side by side they spill 2 KB per thread.
-#include "op_stream.cuh"
 #include "ops.cuh"
+#include "op_stream.cuh"
 #include "walk.cuh"
 
 namespace mk {
@@ -46,6 +46,7 @@ __device__ int mk_run_norm(const Params& p, const mk_op_desc* op, int idx, int s
 #define MK_N(V) case (V): return norm_run<(V)>(p, idx, slot)
 #define MK_NT(V) MK_N((V) | DT_BF16); MK_N((V) | DT_F16); MK_N((V) | DT_F32); MK_N((V) | 4 | DT_BF16); MK_N((V) | 4 | DT_F16); MK_N((V) | 4 | DT_F32)
         MK_NT(0); MK_NT(16); MK_NT(32); MK_NT(8); MK_NT(8 | 16);
+        MK_NT(NORM_DEEP); MK_NT(NORM_DEEP | 16); MK_NT(NORM_DEEP | 32); MK_NT(NORM_DEEP | 8); MK_NT(NORM_DEEP | 8 | 16);
 #undef MK_NT
 #undef MK_N
         default: return norm_run<NORM_ANY>(p, idx, slot);

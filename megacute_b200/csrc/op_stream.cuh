@@ -8,6 +8,7 @@
 #pragma once
 #include <type_traits>
 #include "mk_device.cuh"
+#include "ops.cuh"
 
 namespace mk {
 
@@ -214,6 +215,7 @@ __device__ __forceinline__ void eltwise_tile_gated(const mk_op_desc* op, int r0,
 template <int DT> struct Vec8 {
     uint4 v;
     __device__ __forceinline__ void load(const void* base, long long elem) { v = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(base) + elem)); }
+    __device__ __forceinline__ void raw(const uint4& w, const uint4&) { v = w; }
     __device__ __forceinline__ void get(float* f) const {
         if (DT == DT_F16) {
             const float2 a = unpack2h(v.x), b = unpack2h(v.y), c = unpack2h(v.z), d = unpack2h(v.w);
@@ -228,6 +230,10 @@ template <> struct Vec8<DT_F32> {
     __device__ __forceinline__ void load(const void* base, long long elem) {
         const float4* p = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(base) + elem);
         a = __ldcg(p); b = __ldcg(p + 1);
+    }
+    __device__ __forceinline__ void raw(const uint4& p, const uint4& q) {
+        a = make_float4(__uint_as_float(p.x), __uint_as_float(p.y), __uint_as_float(p.z), __uint_as_float(p.w));
+        b = make_float4(__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w));
     }
     __device__ __forceinline__ void get(float* f) const { f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w; }
 };
@@ -306,12 +312,18 @@ __device__ __forceinline__ void op_eltwise(const mk_op_desc* op, int a0, int a1)
 }
 
 // ---- norms ---------------------------------------------------------------------------------------------------------------------
-// MK_OP_NORM with i 3 >= 8 rows per instruction (descriptor: op_pointwise.cuh): rows r0 + warp, + 8, ..., a row per warp, the
-// next one requested before this one is used.  Gain and, when the instruction's rows lie in one group, scale and shift are
-// requested once and stay in registers.  NPER: 8-element vectors of a row per lane.  HW: gain.  MOD: scale and shift.
-template <int NPER, int XDT, int ODT, bool HW, bool MOD>
+// MK_OP_NORM with i 3 >= 8 rows per instruction (descriptor: op_pointwise.cuh): rows r0 + warp, + 8, ..., a row per warp.  Bound by
+// memory latency: an SM gets what it has requested per round trip (2 us with all SMs streaming), so each warp keeps 12 KB of
+// rows on their way through the work area (DEEP; 64 rows of 2048 fp16: 26.8 -> 14.4 us).  A lane reads back what it
+// copied itself.  With one or two rows per warp there is nothing to run ahead of: the next row in registers (8 rows 5.1 us, 6.0
+// through the work area).  Gain, and scale and shift of the current
+// group of rows, stay in registers.  NPER: 8-element vectors of a row per lane.  HW: gain.  MOD: scale and shift.
+constexpr int kNormAhead = 12288;                          // bytes of rows a warp has requested
+template <int NPER, int XDT, int ODT, bool HW, bool MOD, bool DEEP>
 __device__ __forceinline__ void norm_stream(const mk_op_desc* op, int r0, int rows) {
-    constexpr bool kAhead = XDT != DT_F32 || NPER <= 4;               // (two fp32 rows of 2048 do not fit)
+    constexpr bool kAhead = !DEEP && (XDT != DT_F32 || NPER <= 4);    // (two fp32 rows of 2048 do not fit)
+    constexpr int kPlanes = XDT == DT_F32 ? 2 : 1, kRow = NPER * kPlanes * 512, kDepth = kNormAhead / kRow;     // 16 bytes of a vector per plane
+    static_assert(kDepth >= 1 && kTcXOff + kComputeWarps * kNormAhead <= kWorkBytes, "norm rows exceed the work area");
     const int Cc = op->i[1], rms = op->i[2], group = max(1, op->i[6]);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = Cc >> 3;
     const void* X = reinterpret_cast<const void*>(op->ptr[0]);
@@ -322,9 +334,22 @@ __device__ __forceinline__ void norm_stream(const mk_op_desc* op, int r0, int ro
     float sc[MOD ? NPER * 8 : 1], sh[MOD ? NPER * 8 : 1];
     // (columns beyond the row are clamped to its last vector and left out of the sums and stores)
     auto column = [&](int u) { return (long long)min(lane + u * 32, nvec - 1) * 8; };
+    uint8_t* buf = smem_map().work + kTcXOff + warp * kNormAhead + lane * 16;
+    Vec8<XDT> x[NPER], nx[kAhead ? NPER : 1];
     auto fetch = [&](int rr, Vec8<XDT>* x) {
 #pragma unroll
         for (int u = 0; u < NPER; ++u) x[u].load(X, (r0 + rr) * ldx + column(u));
+    };
+    auto request = [&](int rr, int slot) {
+        if (rr < rows) {
+#pragma unroll
+            for (int u = 0; u < NPER; ++u)
+#pragma unroll
+                for (int k = 0; k < kPlanes; ++k)
+                    cp_async16(buf + slot * kRow + (u * kPlanes + k) * 512,
+                               reinterpret_cast<const uint8_t*>(X) + ((r0 + rr) * ldx + column(u)) * (kPlanes * 2) + k * 16, true);
+        }
+        cp_async_commit();
     };
     auto modulation = [&](long long g) {
 #pragma unroll
@@ -334,24 +359,38 @@ __device__ __forceinline__ void norm_stream(const mk_op_desc* op, int r0, int ro
         }
     };
     if (warp >= rows) return;
-    Vec8<XDT> x[NPER], nx[kAhead ? NPER : 1];
-    if (kAhead) fetch(warp, nx);
-    const bool one = MOD && r0 / group == (r0 + rows - 1) / group;
+    if (DEEP) {
+#pragma unroll
+        for (int d = 0; d < kDepth; ++d) request(warp + d * kComputeWarps, d);
+    } else if (kAhead) {
+        fetch(warp, nx);
+    }
+    int grp = (r0 + warp) / group;
     if (HW) {
 #pragma unroll
         for (int u = 0; u < NPER; ++u) gw[HW ? u : 0].load(reinterpret_cast<const void*>(op->ptr[2]), column(u));
     }
-    if (MOD && one) modulation(r0 / group);
+    if (MOD) modulation(grp);
+    int slot = 0;
 #pragma unroll 1
     for (int rr = warp; rr < rows; rr += kComputeWarps) {
-        if (kAhead) {
+        if (DEEP) {
+            cp_async_wait<kDepth - 1>();
+#pragma unroll
+            for (int u = 0; u < NPER; ++u) {
+                const uint4* at = reinterpret_cast<const uint4*>(buf + slot * kRow + u * kPlanes * 512);
+                x[u].raw(at[0], at[kPlanes == 2 ? 32 : 0]);
+            }
+            request(rr + kDepth * kComputeWarps, slot);
+            if (++slot == kDepth) slot = 0;
+        } else if (kAhead) {
 #pragma unroll
             for (int u = 0; u < NPER; ++u) x[u] = nx[kAhead ? u : 0];
             fetch(min(rr + kComputeWarps, rows - 1), nx);
         } else {
             fetch(rr, x);
         }
-        if (MOD && !one) modulation((r0 + rr) / group);
+        if (MOD && (r0 + rr) / group != grp) { grp = (r0 + rr) / group; modulation(grp); }
         float s = 0.f, ss = 0.f;
 #pragma unroll
         for (int u = 0; u < NPER; ++u) {
@@ -447,19 +486,20 @@ __device__ __forceinline__ void norm_two_pass(const mk_op_desc* op, int r0, int 
     }
 }
 
-// Variant of a norm: x dtype (bits 0-1), fp16 output (bit 2), vectors per lane (bit 3: 8, else 4), gain (bit 4), modulation (bit 5)
-constexpr int NORM_ANY = 64;
+// Variant of a norm: x dtype (bits 0-1), fp16 output (bit 2), vectors per lane (bit 3: 8, else 4), gain (bit 4), modulation (bit 5),
+// three or more rows per warp (bit 6)
+constexpr int NORM_DEEP = 64, NORM_ANY = 128;
 __device__ __forceinline__ int norm_variant(const mk_op_desc* op) {
     const int nper = ((op->i[1] >> 3) + 31) / 32;
     const bool w = op->ptr[2] != 0, mod = op->ptr[4] != 0;
     if (op->ptr[3] || (w && mod) || op->i[5] == DT_F32 || nper > (mod ? 4 : 8)) return NORM_ANY;
-    return op->i[4] | (op->i[5] == DT_F16 ? 4 : 0) | (nper > 4 ? 8 : 0) | (w ? 16 : 0) | (mod ? 32 : 0);
+    return (op->i[3] > 2 * kComputeWarps ? NORM_DEEP : 0) | op->i[4] | (op->i[5] == DT_F16 ? 4 : 0) | (nper > 4 ? 8 : 0) | (w ? 16 : 0) | (mod ? 32 : 0);
 }
 template <int V>
 __device__ __forceinline__ void op_norm_rows(const mk_op_desc* op, int a0) {
     const int r0 = a0 * op->i[3], rows = min(op->i[3], op->i[0] - r0);
     if constexpr (V == NORM_ANY) norm_two_pass(op, r0, rows);
-    else norm_stream<(V & 8) ? 8 : 4, V & 3, (V & 4) ? DT_F16 : DT_BF16, (V & 16) != 0, (V & 32) != 0>(op, r0, rows);
+    else norm_stream<(V & 8) ? 8 : 4, V & 3, (V & 4) ? DT_F16 : DT_BF16, (V & 16) != 0, (V & 32) != 0, (V & NORM_DEEP) != 0>(op, r0, rows);
 }
 
 }  // namespace mk
