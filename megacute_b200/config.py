@@ -26,7 +26,7 @@ INST_US, SM_GBPS = 2.0, 40.0    # split-K cost model: fixed us per instruction, 
 # output tiles of a tile linear: 128 x 128, and for ops with more than WIDE_MIN_ROWS rows 256 x 128 and 256 x 256; cost
 # model (us, from the kernel's timeline with every SM streaming): per tile, per 64-element k-tile, once per op
 GEMM_BM_WIDE, GEMM_BN_WIDE, WIDE_MIN_ROWS = 256, 256, 128
-GEMM_COST_US = {(128, 128): (4.0, 0.28, 0.0), (256, 128): (2.5, 0.45, 4.0), (256, 256): (3.0, 0.72, 5.0)}
+GEMM_COST_US = {(128, 128): (6.0, 0.28, 0.0), (256, 128): (2.5, 0.45, 4.0), (256, 256): (2.0, 0.70, 4.0)}
 REDUCE_GBPS, FINALIZE_US = 2000.0, 8.0       # a K-split op: bytes of its fp32 reduce-adds; the SplitFinalize hop behind it
 
 # ---- pointwise / norm / attention tiling
