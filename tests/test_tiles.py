@@ -1,0 +1,143 @@
+"""Edges of the tile shapes: 256-row GEMM tiles and their epilogues, uneven K splits, rotated heads in a linear's
+epilogue, the two-tile prefill attention, norms of many rows per instruction -- against the fp32 oracle."""
+import pytest
+import torch
+
+import megacute_b200 as mc
+from megacute_b200 import passes
+from megacute_b200 import workloads as W
+from oracle.graph_oracle import rel_l2
+from tests.helpers import TOL
+from tests.test_gpu_ops import rnd, run_both
+
+F32, BF = torch.float32, torch.bfloat16
+# one rounding of an fp32 value to bf16: at most 2^-9 of it, so at most 2^-9 in rel-L2; 5 % for fp32 sums of K <= 2048
+# products (K 2^-24) and the approximate exponentials of the activations (2^-20)
+ONE_ROUNDING = 1.05 * 2.0 ** -9
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,plan,kw", [
+    (129, 256, 64, (1, 256, 256), {}),                                          # one k-tile, one row in the lower half
+    (256, 128, 192, (1, 256, 128), {"bias": True}),
+    (257, 384, 256, (1, 256, 128), {"res": BF}),                                # a second row tile of one row
+    (300, 512, 2048, (1, 256, 256), {"act": "gelu_tanh", "bias": True}),
+    (300, 256, 320, (1, 256, 128), {"act": "relu"}),
+    (400, 512, 128, (1, 256, 256), {"act": "swiglu"}),
+    (385, 256, 448, (1, 256, 256), {"res": F32}),
+    (513, 256, 64, (1, 256, 256), {"res": BF, "act": "silu"}),                  # (activation in front of a residual)
+    (320, 512, 256, (1, 256, 256), {"gate": 64}),                               # gated residual, 64 rows per gate row
+    (320, 128, 256, (1, 256, 128), {"gate": 40}),                               # (a warp's rows span two gate rows)
+    (600, 256, 320, (3, 256, 128), {"bias": True}),                             # 5 k-tiles in 3 splits
+    (200, 256, 448, (4, 128, 128), {"act": "relu"}),                            # 7 in 4, 128 x 128 tiles
+    (150, 136, 96, (1, 128, 128), {}),                                          # K of whole 32s: the mma.sync body
+])
+def test_tile_epilogues(cuda, monkeypatch, M, N, K, plan, kw):
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: plan if a[4] > 1 else (1, *plan[1:]))
+    g = mc.Graph()
+    n_out = N // 2 if kw.get("act") == "swiglu" else N
+    x, w = g.input("x", (M, K)), g.param("w", (N, K))
+    t = {"x": rnd((M, K), 1.0, 1), "w": rnd((N, K), K ** -0.5, 2)}
+    bias = res = None
+    if kw.get("bias"):
+        bias, t["b"] = g.param("b", (1, n_out)), rnd((1, n_out), 0.5, 3)
+    if kw.get("res"):
+        res, t["r"] = g.input("r", (M, n_out), kw["res"]), rnd((M, n_out), 1.0, 4).to(kw["res"])
+    y = g.linear(x, w, bias=bias, act=kw.get("act"), residual=res)
+    if kw.get("gate"):
+        r, gate = g.input("r", (M, N)), g.input("gate", (M // kw["gate"], N))
+        t["r"], t["gate"] = rnd((M, N), 1.0, 4), rnd((M // kw["gate"], N), 1.0, 5)
+        y = g.add(r, g.binary(y, gate, "mul", b_group=kw["gate"]))
+    g.output(y)
+    outs, ref, _, _, prog = run_both(g, t, cuda, steps=2)                       # twice: split-K workspaces are zeroed again
+    for a, b in zip(outs, ref):
+        assert rel_l2(a, b) < ONE_ROUNDING
+    if plan[0] == 1:
+        lin = [o for o in prog.g.ops if o.kind == "Linear"][0]
+        assert (lin.bm or 128, lin.bn or 128) == plan[1:] and prog.tcgen05_ops == (1 if K % 64 == 0 else 0)
+        assert (lin.gate is not None) == bool(kw.get("gate"))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("tcgen05", [True, False])
+@pytest.mark.parametrize("B,S,D,tile", [(1, 150, 64, (128, 128)), (3, 50, 128, (128, 128)), (2, 129, 64, (256, 256)), (1, 257, 128, (256, 128)),
+                                        (1, 300, 128, (256, 256))])
+def test_rotated_heads(cuda, monkeypatch, B, S, D, tile, tcgen05):
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, *tile))
+    if not tcgen05:
+        monkeypatch.setenv("MEGACUTE_B200_NO_TCGEN05", "1")
+    H, KVH, K = 2, 1, 192
+    g = mc.Graph()
+    x, w = g.input("x", (B * S, K)), g.param("w", ((H + 2 * KVH) * D, K))
+    cos, sin = g.input("cos", (S, D)), g.input("sin", (S, D))
+    qkv = g.linear(x, w)
+    q = g.rope(qkv.cols_slice(0, H * D), cos, sin, heads=H, head_dim=D, seq=S)
+    k = g.rope(qkv.cols_slice(H * D, KVH * D), cos, sin, heads=KVH, head_dim=D, seq=S)
+    g.output(g.attention(q, k, qkv.cols_slice((H + KVH) * D, KVH * D), batch=B, heads=H, kv_heads=KVH, head_dim=D, causal=True))
+    cs, sn = W.rope_tables(S, D)
+    t = {"x": rnd((B * S, K), 1.0, 1), "w": rnd(((H + 2 * KVH) * D, K), 0.1, 2), "cos": cs, "sin": sn}
+    outs, ref, _, _, prog = run_both(g, t, cuda)
+    assert not any(o.kind == "Rope" for o in prog.g.ops)
+    assert rel_l2(outs[0], ref[0]) < TOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,Sq,Sk,H,KVH,D,causal", [
+    (1, 1, 1, 1, 1, 64, False), (2, 128, 128, 2, 1, 64, True), (1, 129, 129, 3, 1, 64, True), (1, 255, 640, 2, 2, 64, False),
+    (3, 257, 257, 2, 1, 64, True), (1, 385, 385, 4, 2, 64, True), (1, 700, 65, 2, 1, 64, False),
+    (1, 64, 300, 1, 1, 128, False), (2, 130, 130, 2, 1, 128, True), (1, 520, 520, 3, 1, 128, True), (1, 256, 1000, 2, 2, 128, False),
+])
+def test_prefill_attention_tiles(cuda, B, Sq, Sk, H, KVH, D, causal):
+    """Odd numbers of query tiles and key blocks, one tile only, masked and ragged last blocks.  Two layers of the op: the CTA's
+    buffers do not start at their first phase."""
+    g = mc.Graph()
+    q, k, v = g.input("q", (B * Sq, H * D)), g.input("k", (B * Sk, KVH * D)), g.input("v", (B * Sk, KVH * D))
+    a = g.attention(q, k, v, batch=B, heads=H, kv_heads=KVH, head_dim=D, causal=causal)
+    b = g.attention(a, k, v, batch=B, heads=H, kv_heads=KVH, head_dim=D, causal=causal)
+    g.output(a, b)
+    t = {"q": rnd((B * Sq, H * D), 2.0, 1), "k": rnd((B * Sk, KVH * D), 2.0, 2), "v": rnd((B * Sk, KVH * D), 1.0, 3)}
+    outs, ref, *_ = run_both(g, t, cuda, steps=2)
+    for x, y in zip(outs, ref):
+        assert rel_l2(x, y) < TOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols,dtype,rms,group", [
+    (257, 2048, BF, True, 0), (1190, 1024, BF, True, 0), (2390, 1000, BF, False, 0), (3001, 2048, F32, True, 0), (2400, 1024, BF, False, 40),
+    (9600, 256, BF, True, 0), (2500, 8, F32, True, 0),
+])
+def test_norm_many_rows(cuda, rows, cols, dtype, rms, group):
+    """8, 16, 24 and 64 rows per instruction, a last instruction with fewer, modulation rows that change inside one."""
+    g = mc.Graph()
+    x = g.input("x", (rows, cols), dtype)
+    t = {"x": rnd((rows, cols), 2.0, 1, 0.3).to(dtype)}
+    y = g.rms_norm(x, g.param("w", (1, cols))) if rms else g.layer_norm(x)
+    if rms:
+        t["w"] = rnd((1, cols), 0.1, 2, 1.0)
+    if group:
+        n = rows // group
+        y = g.modulate(y, g.input("sc", (n, cols)), g.input("sh", (n, cols)), group=group)
+        t["sc"], t["sh"] = rnd((n, cols), 0.3, 3), rnd((n, cols), 0.3, 4)
+    g.output(y)
+    outs, ref, *_ = run_both(g, t, cuda)
+    assert rel_l2(outs[0], ref[0]) < ONE_ROUNDING
+
+
+def test_hoisted_linears_keep_their_order():
+    """A linear moves behind the op it depends on and in front of unrelated ones only; what reads or overwrites its operands stays put."""
+    g = mc.Graph()
+    c, w = g.input("c", (32, 64)), g.param("w", (64, 64))
+    s = g.unary(c, "silu")
+    x = g.input("x", (32, 64))
+    for _ in range(6):
+        x = g.add(x, g.unary(x, "relu"))
+    late = g.linear(s, w)
+    near = g.linear(x, w)
+    g.output(g.add(g.add(x, late), near))
+    ops = passes.hoist_linears(g).ops
+    assert [o.kind for o in ops[:2]] == ["Unary", "Linear"] and ops[1].x.same(s)
+    seen = {b.id for b in g.inputs + g.params}
+    for o in ops:
+        assert all(v.buf.id in seen for v in o.reads)
+        seen |= {v.buf.id for v in o.writes}
+    assert len(ops) == len(g.ops) and ops[-3].x.same(x)
