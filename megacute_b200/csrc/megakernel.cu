@@ -10,8 +10,8 @@
 //              warps sit in a dependency hop;
 //   warp 9     finisher: adds the compute warps' partial tiles of a streaming linear, runs its
 //              epilogue and sends the instruction's arrivals;
-//   warp 10    feeder: tiles and MMAs of the tcgen05 prefill attention, activation tiles of the 256 x 256 tile GEMM;
-//   warp 11    issuer: MMAs of the 256 x 256 tile GEMM.
+//   warp 10    feeder: Q, K and V tiles of the tcgen05 prefill attention, activation tiles of the 256-row tile GEMM;
+//   warp 11    issuer: MMAs of both.
 // This replaces the reference's JIT-traced kernel (megacute/kernel.py:251-571) and its per-op
 // role bodies (megacute/ops/*.py).
 #define MK_INLINE_WAITS 1

@@ -17,8 +17,8 @@ constexpr int kComputeThreads = kComputeWarps * 32;
 constexpr int kThreads = kComputeThreads + 128;          // + one producer warp + one finisher warp + one feeder warp + one issuer warp
 constexpr int kProducerWarp = kComputeWarps;
 constexpr int kFinisherWarp = kComputeWarps + 1;
-constexpr int kFeederWarp = kComputeWarps + 2;           // tile requests and MMA issue of the tcgen05 prefill attention; activation tiles of 256 x 256 tile GEMMs
-constexpr int kIssuerWarp = kComputeWarps + 3;           // MMA issue of 256 x 256 tile GEMMs
+constexpr int kFeederWarp = kComputeWarps + 2;           // tile requests of the tcgen05 prefill attention; activation tiles of 256-row tile GEMMs
+constexpr int kIssuerWarp = kComputeWarps + 3;           // MMA issue of both
 
 // ---- shared memory map -----------------------------------------------------------------------
 constexpr int kGemvRows = 8;                              // weight rows per ring stage
@@ -49,8 +49,8 @@ constexpr int kTcXStages = 6;                             // activation stages o
 constexpr int kTcXHalfStages = 10;                        // ... or of 64 rows (ops with at most 64): the MMA still reads 128 rows from a
                                                           // stage's start, so half a tile of the work area must follow the last one
 constexpr int kTcXOff = 512;                              // first 1024-aligned byte of the work area
-constexpr int kTcCols = 512;                              // tensor-memory columns held by the CTA: a 128 x 256 accumulator (tile GEMM),
-                                                          // or two S tiles and O (prefill attention)
+constexpr int kTcCols = 512;                              // tensor-memory columns held by the CTA: all of them (two 128 x 256 accumulators of
+                                                          // the tile GEMM, scores and O of the prefill attention)
 constexpr uint32_t kTcNoTmem = 0xffffffffu;               // Ctrl::tmem_base before the CTA's first allocation
 static_assert((kRingBytes + kTcXOff) % 1024 == 0 && kTcXOff + kTcXStages * kTcTileBytes <= kWorkBytes &&
                   kTcXOff + (kTcXHalfStages + 1) * (kTcTileBytes / 2) <= kWorkBytes && kTcXHalfStages >= kTcXStages,

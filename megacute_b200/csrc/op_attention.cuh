@@ -1,13 +1,13 @@
-// MK_OP_ATTENTION: prefill flash attention, one instruction = (batch b, head h, 128-query tile).
+// MK_OP_ATTENTION, mma.sync body: prefill flash attention, one instruction = (batch b, head h, 256 queries, as two tiles of 128).
 //   out = softmax(q k^T * scale [+ causal mask]) v,   GQA: query head h reads kv head h / (H / KVH)
 // 8 warps x 16 query rows.  K and V stream through a 2-stage cp.async pipeline of 64-key tiles;
 // S = Q K^T and O += P V are warp-level mma.sync m16n8k16 bf16 -> fp32 with the online softmax
 // kept in registers in the log2 domain; P is rounded to bf16 before P V (as the reference's
-// kernel does, megacute/ops/attention.py:293).  A fully masked row yields 0.  This is the
-// portable first implementation; the tcgen05 / TMEM version is the planned replacement.
+// kernel does, megacute/ops/attention.py:293).  A fully masked row yields 0.  Runs what the tcgen05
+// body (op_attention_tc.cuh) does not take: other head_dims, operands its tensor maps cannot describe.
 //
 // ptr 0 q, 1 k, 2 v, 3 out; i 0 batch, 1 seq_q, 2 seq_k, 3 heads, 4 kv_heads, 5 head_dim,
-// 6 causal, 7 out dtype (DT_BF16 or DT_F16), 8 dtype of q, k and v (DT_BF16 or DT_F16); f 0 scale.  args: 0 b, 1 h, 2 query tile.
+// 6 causal, 7 out dtype (DT_BF16 or DT_F16), 8 dtype of q, k and v (DT_BF16 or DT_F16); f 0 scale.  args: 0 b, 1 h, 2 query tile pair.
 #pragma once
 #include "mk_device.cuh"
 #include "mma.cuh"

@@ -1,4 +1,4 @@
-// MK_OP_GEMM on tcgen05 with 256 x 256 output tiles (descriptor i 10 = 256): linears with many activation rows.
+// MK_OP_GEMM on tcgen05 with output tiles of 256 rows (descriptor i 11 = 256) and 256 or 128 columns (i 10): linears with many rows.
 //
 // What bounds a tile GEMM whose operands live in L2 is the bytes an SM draws from there: measured on B200 (all 148 SMs,
 // stand-alone loop) a 128 x 256 tile takes 0.46 us per 64-element k-tile of 48 KB (104 GB/s per SM) where its MMAs take
@@ -13,6 +13,10 @@
 //                It is told what to run by the feeder through Ctrl::wide_info and never touches global memory.
 //   epilogue     the compute warps: warp w owns rows 32 (w & 3) .. +31 of accumulator w >> 2; it reads its 32 x 256 part, hands
 //                the accumulator back and writes the rows from registers while the next tile's main loop runs
+// Tiles of 256 x 128 (kind 1; kind 0: 256 x 256) have four stages of 48 KB and half the accumulator columns.  They cost 0.45 us per
+// k-tile where half a 256 x 256 tile costs 0.36 -- 128-column instructions read as many operand bytes for half the flops, and
+// shared memory (128 bytes a cycle for the tensor core's reads and the copies' writes together) is what both are bound by --
+// and are chosen where they fill the SMs better (passes.plan_tiles).
 // The loads of the next tile therefore run through this one's epilogue, and its MMAs start as soon as the accumulators have
 // been read.  (With one role after the other per instruction, 128 x 256 tiles: prefill gate/up 20.5 us per 128 x 256 x 2048
 // block of which 13.8 were main loop; DiT gelu tiles 28 us of which 7.)

@@ -1,4 +1,4 @@
-// Translation unit of MK_OP_GEMM with 256 x 256 output tiles on the tcgen05 body (descriptor i 10 = 256 and tensor
+// Translation unit of MK_OP_GEMM with output tiles of 256 rows on the tcgen05 body (descriptor i 11 = 256 and tensor
 // maps attached).  Separate from op_gemm.cu so that each tile shape gets its own register allocation: inlined side
 // by side, the wider tile's extra live state spilled registers of the narrow tile's main loop (spills are L2 round
 // trips here: batch-64 decode 7 % slower, the MLP block 14 %).

@@ -24,7 +24,7 @@ __device__ int mk_op_gemv_general(const Params& p, const mk_op_desc* op, int o0,
 // arrivals of each itself (begin_op says why).  Returns the index of the last instruction executed, -1 when the CTA is
 // aborting.  (The ring position is untouched: the weight tiles have slots of their own.)
 __device__ int mk_run_gemm(const Params& p, int idx, int slot);
-// (the same with 256 x 256 output tiles; only for ops the host library bound to the tcgen05 body)
+// (the same with output tiles of 256 rows; only for ops the host library bound to the tcgen05 body)
 __device__ int mk_run_gemm_wide(const Params& p, int idx, int slot);
 // body of the issuer warp: the MMAs of every tile GEMM with 256-row tiles and of every tcgen05 attention, until the feeder warp says that the list has ended
 __device__ void mk_issuer(const Params& p);

@@ -10,10 +10,11 @@ view's first element.  Field meaning per kind (the kernel side repeats it next t
 
   GEMV         ptr x, w, out, bias, residual, norm gain; i M, N_out, K, act, x dtype, out dtype,
                residual dtype; f eps; flags 1 = swiglu, 2 = rms-normalise x, 4 = tensor-core streaming path
-  GEMM         ptr x, w, out, bias, residual, gate; i M, N (weight rows), K, act, splits, out dtype,
-               accumulate, residual dtype, swiglu, x dtype (bf16 or fp16), weight rows per tile (128 / 256), activation rows per tile (128 / 256), rows per
-               gate row, gate dtype  (ptr 10, 11: set by the C
-               library when it binds the op to its tcgen05 body: packed weight tiles, tensor maps)
+  GEMM         ptr x, w, out, bias, residual, gate, cos, sin; i M, N (weight rows), K, act, splits, out dtype,
+               accumulate, residual dtype, swiglu, x dtype (bf16 or fp16), weight rows per tile (128 / 256),
+               activation rows per tile (128 / 256), rows per gate row, gate dtype, rotated columns, head_dim, seq,
+               table dtype, K columns per split, splits with a k-tile more  (ptr 10, 11: set by the C library when
+               it binds the op to its tcgen05 body: packed weight tiles, tensor maps)
   FINALIZE     ptr ws, out, bias, residual; i R, C, act, out dtype, residual dtype, rows per instruction
   ELTWISE      ptr a, b, c, out; i R, C, mode, fn, group, head_dim, dtypes of a, b, c, out, rows per instruction
                (mode EW_GATED: out = fn(a, b * c[r // group]), a gated residual)
