@@ -30,6 +30,7 @@ ONE_ROUNDING = 1.05 * 2.0 ** -9
     (320, 128, 256, (1, 256, 128), {"gate": 40}),                               # (a warp's rows span two gate rows)
     (600, 256, 320, (3, 256, 128), {"bias": True}),                             # 5 k-tiles in 3 splits
     (200, 256, 448, (4, 128, 128), {"act": "relu"}),                            # 7 in 4, 128 x 128 tiles
+    (135, 264, 448, (3, 128, 128), {"bias": True, "res": F32}),                 # (ragged in both directions, finished with a residual)
     (150, 136, 96, (1, 128, 128), {}),                                          # K of whole 32s: the mma.sync body
 ])
 def test_tile_epilogues(cuda, monkeypatch, M, N, K, plan, kw):
