@@ -199,7 +199,7 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
         return Tiled(_args(n, rt, ct), [a for a in acc if a is not None])
     if k == "Norm":
         R = op.x.rows
-        rows = norm_rows(R)
+        rows = norm_rows(R, op.scale is not None)
         rt = np.arange(_ceil(R, rows))
         n = len(rt)
         acc = [_acc(op.x, READ, rt * rows, (rt + 1) * rows, n=n), _acc(op.weight, READ, n=n), _acc(op.bias, READ, n=n),
@@ -299,12 +299,17 @@ def finalize_rows(rows: int, cols: int) -> int:
     return tr
 
 
-def norm_rows(rows: int) -> int:
+def norm_rows(rows: int, modulated: bool = False) -> int:
     """Rows per norm instruction: a single row spread over the whole CTA when the op has few rows (decode),
-    else a multiple of the compute warps that gives each SM about one instruction."""
+    else a multiple of the compute warps that gives each SM about one instruction.  Modulated rows (a DiT block's): 16, 32 or 64, so
+    that an instruction waits for one 256-row tile of the linear before it and its rows share a scale and shift row
+    (56 -> 64 rows at 32 images, 24 -> 32 at 12: 0.4 and 1.6 % of the step)."""
     if rows <= C.WIDE_NORM_ROWS:
         return 1
-    return C.NORM_ROWS * max(1, min(C.NORM_MAX_ROWS // C.NORM_ROWS, _ceil(_ceil(rows, C.NORM_ROWS), C.STREAM_INSTS)))
+    per = max(1, min(C.NORM_MAX_ROWS // C.NORM_ROWS, _ceil(_ceil(rows, C.NORM_ROWS), C.STREAM_INSTS)))
+    if modulated and per > 2:
+        per = 4 if per <= 4 else 8
+    return C.NORM_ROWS * per
 
 
 def ew_rows(rows: int, cols: int) -> int:
