@@ -15,6 +15,9 @@ runtime's kernel:
   split_kv             decode attention instructions are multiplied along the key axis so that every
                        SM streams keys; the last split of a (sequence, kv head) pair to finish
                        combines the partials inside the op.
+  fuse_gated_linear, fuse_rope_linear   gated residuals and the rotation of q and k into the epilogue of the
+                       tile linear before them.
+  hoist_linears        linears whose operands are ready long before their place move up.
 """
 
 from __future__ import annotations
