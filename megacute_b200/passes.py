@@ -502,6 +502,8 @@ def fuse_gated_linear(g: Graph) -> Graph:
         if (op.kind == "Binary" and op.gate is not None and op.fn == "add" and prev is not None and prev.kind == "Linear"
                 and prev.bm == C.GEMM_BM_WIDE and prev.act != "swiglu" and prev.residual is None and prev.gate is None
                 and op.b.same(prev.out) and prev.out.buf.kind == "temp" and not _reads_buffer(g.ops[i + 1:], prev.out.buf, g.outputs)
+                # (the product is not stored any more: neither the residual nor the gate may be it)
+                and op.a.buf is not prev.out.buf and op.gate.buf is not prev.out.buf
                 and all(v.buf is not prev.x.buf for v in op.writes)):
             ops[-1] = prev.clone(out=op.out, residual=op.a, gate=op.gate, gate_group=op.gate_group)
             continue

@@ -1,0 +1,44 @@
+"""What the graph rewrites must refuse: graphs that look like the fused pattern and are not.  The rewritten graph has to
+evaluate to what the graph says, in the oracle, which runs ops one after the other and rejects a read of a tensor that nothing wrote."""
+import pytest
+import torch
+
+import megacute_b200 as mc
+from megacute_b200 import passes
+from oracle.graph_oracle import evaluate, rel_l2
+
+BF = torch.bfloat16
+SMS = 148
+
+
+def rnd(shape, std=1.0, seed=0):
+    return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * std).to(BF)
+
+
+def check_rewritten(g, tensors, tol=1e-5):
+    """run_all(g) agrees with g (fp32 on both sides: sums in another order at most).  Returns its op kinds."""
+    want, _ = evaluate(g, tensors)
+    out = passes.run_all(g, SMS)
+    got, _ = evaluate(out, tensors)
+    for a, b in zip(got, want):
+        assert rel_l2(a, b) < tol
+    return [o.kind for o in out.ops]
+
+
+@pytest.mark.parametrize("form", ["residual first", "gated first", "gate is the product"])
+def test_gated_residual_of_the_product_itself(monkeypatch, form):
+    """y + y * gate with y = linear(x): the linear of 256-row tiles still has to write y."""
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 256))
+    g = mc.Graph()
+    x, w = g.input("x", (384, 64)), g.param("w", (256, 64))
+    y = g.linear(x, w)
+    t = {"x": rnd((384, 64)), "w": rnd((256, 64), 0.1, 1)}
+    if form == "gate is the product":
+        r = g.input("r", (384, 256))
+        t["r"] = rnd((384, 256), 1.0, 2)
+        g.output(g.add(r, g.binary(y, y.rows_slice(0, 192), "mul", b_group=2)))
+    else:
+        z = g.binary(y, g.input("gate", (6, 256)), "mul", b_group=64)
+        t["gate"] = rnd((6, 256), 1.0, 2)
+        g.output(g.add(y, z) if form == "residual first" else g.add(z, y))
+    assert check_rewritten(g, t) == ["Linear", "Binary"]
