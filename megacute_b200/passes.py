@@ -544,10 +544,12 @@ def fuse_rope_linear(g: Graph) -> Graph:
                   and all(o.kind == "Attention" for o in ops if any(v.buf is r.out.buf for v in o.reads))
                   and sum(any(v.buf is r.out.buf for v in o.writes) for o in ops) == 1)
             col += r.x.cols
-        # nothing else touches the columns that are now rotated in place
+        # nothing else touches the columns that are now rotated in place, and the tables are what they are when the linear runs
         for k, o in enumerate(ops):
             if k != i and k not in ropes:
                 ok = ok and not any(v.buf is buf for v in o.writes) and not any(v.buf is buf and v.col0 < col for v in o.reads)
+            if i < k < ropes[-1]:
+                ok = ok and not any(v.buf is t.buf for v in o.writes for t in (first.cos, first.sin))
         if not ok:
             continue
         fused[i] = lin.clone(cos=first.cos, sin=first.sin, rope_cols=col, head_dim=first.head_dim, seq=first.seq)

@@ -42,3 +42,28 @@ def test_gated_residual_of_the_product_itself(monkeypatch, form):
         t["gate"] = rnd((6, 256), 1.0, 2)
         g.output(g.add(y, z) if form == "residual first" else g.add(z, y))
     assert check_rewritten(g, t) == ["Linear", "Binary"]
+
+
+def rotated(g, S, H=2, KVH=1, D=64, tables=lambda c, s: (c, s), qkv_dtype=None):
+    """x -> q, k, v of one prompt -> rotated q and k -> attention.  `tables`: ops between the linear and the rotation."""
+    x, w = g.input("x", (S, 64)), g.param("w", ((H + 2 * KVH) * D, 64))
+    c, s = g.input("cos", (S, D)), g.input("sin", (S, D))
+    qkv = g.linear(x, w, out=g.temp((S, w.rows), dtype=qkv_dtype))
+    c, s = tables(c, s)
+    q = g.rope(qkv.cols_slice(0, H * D), c, s, heads=H, head_dim=D, seq=S)
+    k = g.rope(qkv.cols_slice(H * D, KVH * D), c, s, heads=KVH, head_dim=D, seq=S)
+    v = qkv.cols_slice((H + KVH) * D, KVH * D)
+    if qkv_dtype:
+        v = g.unary(v, "identity")
+    g.output(g.attention(q, k, v, batch=1, heads=H, kv_heads=KVH, head_dim=D, causal=True))
+    return {"x": rnd((S, 64)), "w": rnd((w.rows, 64), 0.1, 1), "cos": rnd((S, D), 1.0, 2), "sin": rnd((S, D), 1.0, 3)}
+
+
+def test_rotation_stays_behind_the_op_that_makes_its_tables():
+    g = mc.Graph()
+    t = rotated(g, 80)
+    assert check_rewritten(g, t) == ["Linear", "Attention"]
+    for which in (0, 1):
+        g = mc.Graph()
+        t = rotated(g, 80, tables=lambda c, s: (g.unary(c, "neg"), s) if which == 0 else (c, g.unary(s, "neg")))
+        assert check_rewritten(g, t) == ["Linear", "Unary", "Rope", "Rope", "Attention"]
