@@ -541,6 +541,7 @@ def fuse_rope_linear(g: Graph) -> Graph:
                   and r.cos.same(first.cos) and r.sin.same(first.sin) and (r.seq, r.head_dim) == (first.seq, first.head_dim)
                   and r.cos.buf.dtype == r.sin.buf.dtype and r.out.buf.kind == "temp" and r.out.buf is not buf
                   and r.out.rect == (0, r.out.buf.rows, 0, r.out.buf.cols) and not any(v.buf is r.out.buf for v in g.outputs)
+                  and r.out.buf.dtype == buf.dtype       # (attention reads the linear's buffer in its place: fp32 it does not take)
                   and all(o.kind == "Attention" for o in ops if any(v.buf is r.out.buf for v in o.reads))
                   and sum(any(v.buf is r.out.buf for v in o.writes) for o in ops) == 1)
             col += r.x.cols

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import megacute_b200 as mc
-from megacute_b200 import passes
+from megacute_b200 import encode, passes
 from oracle.graph_oracle import evaluate, rel_l2
 
 BF = torch.bfloat16
@@ -67,3 +67,12 @@ def test_rotation_stays_behind_the_op_that_makes_its_tables():
         g = mc.Graph()
         t = rotated(g, 80, tables=lambda c, s: (g.unary(c, "neg"), s) if which == 0 else (c, g.unary(s, "neg")))
         assert check_rewritten(g, t) == ["Linear", "Unary", "Rope", "Rope", "Attention"]
+
+
+def test_rotation_of_an_fp32_product_keeps_its_op():
+    """q and k computed in fp32 and rotated into 16 bits: attention cannot read the fp32 buffer."""
+    g = mc.Graph()
+    t = rotated(g, 80, qkv_dtype=torch.float32)
+    assert "Rope" in check_rewritten(g, t)
+    for op in passes.run_all(g, SMS).ops:
+        encode.validate(op)
