@@ -266,6 +266,7 @@ def split_k(g: Graph, sm_count: int) -> Graph:
             whole = op.out.rect == (0, op.out.buf.rows, 0, op.out.buf.cols)
             inplace = (r is not None and op.bias is None and op.act is None and op.norm_w is None
                        and r.buf.kind == "temp" and op.out.buf.kind == "temp" and whole
+                       and all(v.buf is not r.buf for v in (op.x, op.w))       # (other instructions still read those)
                        and not _reads_buffer(src[i + 1:], r.buf))
             if M > C.WIDE_MIN_ROWS:
                 s = plan_tiles(M, op.w.rows, K, sm_count, C.MAX_K_SPLITS, not inplace)[0]

@@ -76,3 +76,13 @@ def test_rotation_of_an_fp32_product_keeps_its_op():
     assert "Rope" in check_rewritten(g, t)
     for op in passes.run_all(g, SMS).ops:
         encode.validate(op)
+
+
+@pytest.mark.parametrize("rows", [16, 64, 300])
+def test_k_splits_do_not_add_into_their_own_input(rows):
+    """h + linear(h): the splits of one tile must not be added into rows of h that another tile still reads."""
+    g = mc.Graph()
+    h = g.unary(g.input("x", (rows, 2048)), "relu")
+    g.output(g.unary(g.linear(h, g.param("w", (2048, 2048)), residual=h), "identity"))
+    split = [o for o in passes.run_all(g, SMS).ops if o.kind == "LinearSplit"]
+    assert (split or rows > 128) and all(o.ws.buf is not v.buf for o in split for v in o.reads)
