@@ -267,7 +267,9 @@ def split_k(g: Graph, sm_count: int) -> Graph:
             inplace = (r is not None and op.bias is None and op.act is None and op.norm_w is None
                        and r.buf.kind == "temp" and op.out.buf.kind == "temp" and whole
                        and all(v.buf is not r.buf for v in (op.x, op.w))       # (other instructions still read those)
-                       and not _reads_buffer(src[i + 1:], r.buf))
+                       # nobody needs the residual as it was, under its own name or under that of an output added into it before,
+                       # and nobody puts anything else there
+                       and not any(_retarget(v, alias).buf is r.buf for o in src[i + 1:] for v in o.reads + o.writes))
             if M > C.WIDE_MIN_ROWS:
                 s = plan_tiles(M, op.w.rows, K, sm_count, C.MAX_K_SPLITS, not inplace)[0]
             else:

@@ -86,3 +86,20 @@ def test_k_splits_do_not_add_into_their_own_input(rows):
     g.output(g.unary(g.linear(h, g.param("w", (2048, 2048)), residual=h), "identity"))
     split = [o for o in passes.run_all(g, SMS).ops if o.kind == "LinearSplit"]
     assert (split or rows > 128) and all(o.ws.buf is not v.buf for o in split for v in o.reads)
+
+
+@pytest.mark.parametrize("form", ["read again", "overwritten"])
+def test_k_splits_are_not_added_into_a_residual_that_lives_on(form):
+    """Two linears add to the residual stream one after the other; the value in between is read (or the first one's memory is used
+    for something else) afterwards."""
+    g = mc.Graph()
+    x, w, w2 = g.input("x", (16, 2048)), g.param("w", (2048, 2048)), g.param("w2", (2048, 2048))
+    r = g.unary(x, "relu")
+    y1 = g.linear(x, w, residual=r)
+    if form == "read again":
+        g.output(g.add(y1, g.linear(x, w2, residual=y1)))
+    else:
+        g.unary(x, "silu", out=r)
+        g.output(g.unary(y1, "identity"))
+    kinds = check_rewritten(g, {"x": rnd((16, 2048)), "w": rnd((2048, 2048), 0.02, 1), "w2": rnd((2048, 2048), 0.02, 2)})
+    assert "SplitFinalize" in kinds
