@@ -474,13 +474,13 @@ def fuse_pointwise(g: Graph) -> Graph:
         prev = ops[-1] if ops else None
         private = lambda v: v.buf.kind == "temp" and not _reads_buffer(g.ops[i + 1:], v.buf, g.outputs)
         if (op.kind == "Modulate" and prev is not None and prev.kind == "Norm" and prev.scale is None
-                and op.x.same(prev.out) and private(prev.out)):
+                and op.x.same(prev.out) and private(prev.out) and all(v.buf is not prev.out.buf for v in (op.scale, op.shift))):
             ops[-1] = prev.clone(out=op.out, scale=op.scale, shift=op.shift, group=op.group)
             continue
         if (op.kind == "Binary" and op.fn == "add" and op.b_group == 1 and op.gate is None and prev is not None
                 and prev.kind == "Binary" and prev.fn == "mul" and prev.gate is None and prev.b_group > 1):
             for mine, other in ((op.b, op.a), (op.a, op.b)):
-                if mine.same(prev.out) and private(prev.out) and other.shape == op.out.shape:
+                if mine.same(prev.out) and private(prev.out) and other.shape == op.out.shape and other.buf is not prev.out.buf:
                     ops[-1] = op.clone(a=other, b=prev.a, gate=prev.b, gate_group=prev.b_group)
                     break
             else:

@@ -103,3 +103,15 @@ def test_k_splits_are_not_added_into_a_residual_that_lives_on(form):
         g.output(g.unary(y1, "identity"))
     kinds = check_rewritten(g, {"x": rnd((16, 2048)), "w": rnd((2048, 2048), 0.02, 1), "w2": rnd((2048, 2048), 0.02, 2)})
     assert "SplitFinalize" in kinds
+
+
+def test_pointwise_pairs_whose_middle_is_read_twice():
+    """z + z with z = y * gate, and a norm modulated by itself: the op in the middle has to run."""
+    g = mc.Graph()
+    z = g.mul(g.input("a", (64, 64)), g.input("b", (4, 64)))
+    g.output(g.add(z, z))
+    assert check_rewritten(g, {"a": rnd((64, 64)), "b": rnd((4, 64), 1.0, 1)}) == ["Binary", "Binary"]
+    g = mc.Graph()
+    n, s = g.rms_norm(g.input("a", (64, 64))), g.input("s", (64, 64))
+    g.output(g.modulate(g.modulate(n, n, s, group=1), s, s, group=1))
+    assert check_rewritten(g, {"a": rnd((64, 64)), "s": rnd((64, 64), 1.0, 1)}) == ["Norm", "Modulate", "Modulate"]
