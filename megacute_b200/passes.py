@@ -34,6 +34,13 @@ def _reads_buffer(ops, buf, outputs=()) -> bool:
     return any(v.buf is buf for op in ops for v in op.reads) or any(v.buf is buf for v in outputs)
 
 
+def _overwrites(op, views, in_place=None) -> bool:
+    """Does op write a buffer that one of `views` -- operands an op fused with it would read in all its instructions -- lies in?
+    `in_place`: one more operand, that the fused op reads and writes element by element or row by row: it may be what op writes."""
+    clash = lambda w, v: v is not None and w.buf is v.buf
+    return any(clash(w, v) for w in op.writes for v in views) or any(clash(w, in_place) and not w.same(in_place) for w in op.writes)
+
+
 def gemv_eligible(M: int, K: int) -> bool:
     """Does a linear with M activation rows of length K run on the weight-streaming GEMV path?
     The whole activation is kept in shared memory as fp32."""
@@ -55,10 +62,9 @@ def fold_norms(g: Graph) -> Graph:
             u = ops[j]
             ok = ok and u.kind == "Linear" and op.out.same(u.x) and u.rms_eps is None
             ok = ok and all(v is None or v.buf is not op.out.buf for v in (u.residual, u.bias))
-        # the raw input must not be rewritten between the norm and its last user
+        # the raw input must not be rewritten between the norm and its last user, nor by that (its instructions read whole rows)
         if ok:
-            between = ops[i + 1:users[-1]]
-            ok = not any(w.buf is op.x.buf for o in between for w in o.writes)
+            ok = not any(_overwrites(o, (op.x, op.weight)) for o in ops[i + 1:users[-1] + 1])
         if not ok:
             continue
         for j in users:
@@ -75,7 +81,7 @@ def fuse_rope_attention(g: Graph) -> Graph:
         prev = ops[-1] if ops else None
         if (op.kind == "DecodeAttention" and op.k_new is None and prev is not None and prev.kind == "RopeAppend"
                 and op.q.same(prev.q_out) and op.k_cache.same(prev.k_cache) and op.v_cache.same(prev.v_cache)
-                and op.pos.same(prev.pos) and prev.q_out.buf.kind == "temp"
+                and op.pos.same(prev.pos) and prev.q_out.buf.kind == "temp" and not _overwrites(op, prev.reads)
                 and not _reads_buffer(g.ops[i + 1:], prev.q_out.buf, g.outputs)):
             H, KVH, D = prev.heads, prev.kv_heads, prev.head_dim
             qkv = prev.qkv
@@ -474,11 +480,13 @@ def fuse_pointwise(g: Graph) -> Graph:
         prev = ops[-1] if ops else None
         private = lambda v: v.buf.kind == "temp" and not _reads_buffer(g.ops[i + 1:], v.buf, g.outputs)
         if (op.kind == "Modulate" and prev is not None and prev.kind == "Norm" and prev.scale is None
-                and op.x.same(prev.out) and private(prev.out) and all(v.buf is not prev.out.buf for v in (op.scale, op.shift))):
+                and op.x.same(prev.out) and private(prev.out) and all(v.buf is not prev.out.buf for v in (op.scale, op.shift))
+                and not _overwrites(op, (prev.weight, prev.bias), in_place=prev.x)):
             ops[-1] = prev.clone(out=op.out, scale=op.scale, shift=op.shift, group=op.group)
             continue
         if (op.kind == "Binary" and op.fn == "add" and op.b_group == 1 and op.gate is None and prev is not None
-                and prev.kind == "Binary" and prev.fn == "mul" and prev.gate is None and prev.b_group > 1):
+                and prev.kind == "Binary" and prev.fn == "mul" and prev.gate is None and prev.b_group > 1
+                and not _overwrites(op, (prev.b,), in_place=prev.a)):
             for mine, other in ((op.b, op.a), (op.a, op.b)):
                 if mine.same(prev.out) and private(prev.out) and other.shape == op.out.shape and other.buf is not prev.out.buf:
                     ops[-1] = op.clone(a=other, b=prev.a, gate=prev.b, gate_group=prev.b_group)
@@ -507,7 +515,7 @@ def fuse_gated_linear(g: Graph) -> Graph:
                 and op.b.same(prev.out) and prev.out.buf.kind == "temp" and not _reads_buffer(g.ops[i + 1:], prev.out.buf, g.outputs)
                 # (the product is not stored any more: neither the residual nor the gate may be it)
                 and op.a.buf is not prev.out.buf and op.gate.buf is not prev.out.buf
-                and all(v.buf is not prev.x.buf for v in op.writes)):
+                and not _overwrites(op, prev.reads)):
             ops[-1] = prev.clone(out=op.out, residual=op.a, gate=op.gate, gate_group=op.gate_group)
             continue
         ops.append(op)

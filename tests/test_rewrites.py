@@ -115,3 +115,49 @@ def test_pointwise_pairs_whose_middle_is_read_twice():
     n, s = g.rms_norm(g.input("a", (64, 64))), g.input("s", (64, 64))
     g.output(g.modulate(g.modulate(n, n, s, group=1), s, s, group=1))
     assert check_rewritten(g, {"a": rnd((64, 64)), "s": rnd((64, 64), 1.0, 1)}) == ["Norm", "Modulate", "Modulate"]
+
+
+def test_fused_ops_do_not_overwrite_what_they_read():
+    """Graphs that put the second op's result where the first one's operands are.  Op by op they are right; in one op an instruction
+    would write what another still reads."""
+    def kinds(build):
+        g = mc.Graph()
+        build(g)
+        return [o.kind for o in passes.run_all(g, SMS).ops]
+
+    def norm_linear_in_place(g):                    # x = x + linear(rms_norm(x))
+        x = g.state("x", (2, 256))
+        g.linear(g.rms_norm(x), g.param("w", (256, 256)), residual=x, out=x)
+
+    def modulate_shifted(g):                        # the rows one further
+        x, s = g.state("x", (65, 64)), g.input("s", (1, 64))
+        g.modulate(g.rms_norm(x.rows_slice(0, 64)), s, s, group=64, out=x.rows_slice(1, 64))
+
+    def modulate_in_place(g):
+        x, s = g.state("x", (64, 64)), g.input("s", (1, 64))
+        g.modulate(g.rms_norm(x), s, s, group=64, out=x)
+
+    def gated_over_its_gate(g):
+        x = g.state("x", (64, 64))
+        g.add(g.input("r", (64, 64)), g.binary(g.input("y", (64, 64)), x.rows_slice(0, 4), "mul", b_group=16), out=x)
+
+    def attention_over_qkv(g):
+        qkv, pos = g.state("qkv", (1, 256)), g.state("pos", (1, 1), torch.int32)
+        c, s, k, v = g.input("c", (128, 64)), g.input("s", (128, 64)), g.state("k", (128, 64)), g.state("v", (128, 64))
+        q = g.rope_append(qkv, c, s, pos, k, v, heads=2, kv_heads=1, head_dim=64, max_seq=128)
+        g.decode_attention(q, k, v, pos, heads=2, kv_heads=1, head_dim=64, max_seq=128, out=qkv.cols_slice(64, 128))
+
+    assert kinds(norm_linear_in_place) == ["Norm", "Linear"]
+    assert kinds(modulate_shifted) == ["Norm", "Modulate"] and kinds(modulate_in_place) == ["Norm"]
+    assert kinds(gated_over_its_gate) == ["Binary", "Binary"]
+    assert kinds(attention_over_qkv) == ["RopeAppend", "DecodeAttention"]
+
+
+def test_gated_residual_over_the_weights(monkeypatch):
+    """The linear's other row tiles still read what the gated residual is put over."""
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 256))
+    g = mc.Graph()
+    w = g.state("w", (512, 256))
+    y = g.linear(g.input("x", (512, 256)), w.rows_slice(0, 256))
+    g.add(g.input("r", (512, 256)), g.binary(y, g.input("gate", (8, 256)), "mul", b_group=64), out=w)
+    assert [o.kind for o in passes.run_all(g, SMS).ops] == ["Linear", "Binary"]
