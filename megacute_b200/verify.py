@@ -11,6 +11,7 @@ them.  Both are properties of the tables, so both are decided here, on the host,
     here per op kind from the descriptor's integers -- must lie inside the view the descriptor was
     encoded from, row pitch included; and every instruction's arguments must lie inside the op's
     tiling.  (The C library repeats the argument check at bind time for callers of the C ABI.)
+    And no op may read, or add into, a temp that no earlier op wrote (a rewrite that dropped the op that made it).
 
 ``check_hazards(sched, g)``
     Happens-before closure over the encoded wait / arrival tables.  Instruction j happens before i
@@ -19,6 +20,8 @@ them.  Both are properties of the tables, so both are decided here, on the host,
     all of them), transitively.  Every pair of instructions of different ops whose accesses
     conflict (read/write, write/write, accumulate/read-or-write on intersecting rectangles of one
     buffer) must be so ordered, earlier program position first.  Exact: no sampling of executions.
+    The instructions of one op run in no order at all: one of them may not write what another reads (ops whose
+    instructions coordinate among themselves -- decode attention, argmax -- excepted).
 
 ``Program(..., debug=True)`` and ``MEGACUTE_B200_VERIFY=1`` run both at compile time.
 """
@@ -30,7 +33,7 @@ import torch
 
 from . import config as C
 from .graph import Graph
-from .schedule import CONFLICTS, Schedule, ew_rows, finalize_rows, gemm_rows, is_gemv, norm_rows, tile_op
+from .schedule import CONFLICTS, Schedule, _overlap, _rect_hits, ew_rows, finalize_rows, gemm_rows, is_gemv, norm_rows, tile_op
 
 
 class VerifyError(AssertionError):
@@ -155,7 +158,13 @@ def op_grid(op, sm_count: int):
 def check_tables(g: Graph, sched: Schedule, tensors: dict | None = None) -> None:
     """Operand windows inside their views, views inside their buffers (and, with ``tensors`` -- buffer id
     -> bound tensor -- inside the bound storage), instruction arguments inside the op's tiling."""
+    written: dict[int, list] = {}                 # temp -> rectangles written so far
     for kk, op in enumerate(g.ops):
+        for v in op.reads + (op.writes if op.accumulate else []):
+            if v.buf.kind == "temp" and not any(_rect_hits(v.rect, r) for r in written.get(v.buf.id, ())):
+                raise VerifyError(f"op {kk} {op.kind}: reads temp {v}, which no earlier op writes")
+        for v in op.writes:
+            written.setdefault(v.buf.id, []).append(v.rect)
         win = operand_windows(op)
         for name, v in op.view_fields():
             if name not in win:
@@ -249,6 +258,13 @@ def check_hazards(s: Schedule, g: Graph) -> int:
             kb, ab = accs[x]
             for y in range(x):
                 ka, aa = accs[y]
+                if ka == kb and aa.kind != ab.kind and g.ops[ka].kind not in ("DecodeAttention", "Argmax") and _rect_hits(aa.rect, ab.rect):
+                    o = _overlap(ab.boxes, aa.boxes)
+                    np.fill_diagonal(o, False)
+                    if o.any():
+                        i, j = (int(n[0]) + s.node_ranges[ka][0] for n in np.nonzero(o))
+                        raise VerifyError(f"op {ka} {g.ops[ka].kind}: instructions {i} ({ab.kind}) and {j} ({aa.kind}) touch intersecting "
+                                          f"rectangles of buffer '{aa.buf.name}' with nothing between them")
                 if ka == kb or aa.kind not in CONFLICTS[ab.kind]:
                     continue
                 ra, rb = aa.rect, ab.rect

@@ -5,6 +5,8 @@ import torch
 
 import megacute_b200 as mc
 from megacute_b200 import encode, passes
+from megacute_b200.schedule import schedule
+from megacute_b200.verify import VerifyError, check_hazards, check_tables
 from oracle.graph_oracle import evaluate, rel_l2
 
 BF = torch.bfloat16
@@ -161,3 +163,35 @@ def test_gated_residual_over_the_weights(monkeypatch):
     y = g.linear(g.input("x", (512, 256)), w.rows_slice(0, 256))
     g.add(g.input("r", (512, 256)), g.binary(y, g.input("gate", (8, 256)), "mul", b_group=64), out=w)
     assert [o.kind for o in passes.run_all(g, SMS).ops] == ["Linear", "Binary"]
+
+
+def test_verifier_rejects_reads_of_temps_nothing_wrote():
+    g = mc.Graph()
+    y = g.unary(g.input("x", (64, 64)), "relu")
+    g.output(g.add(y, y))
+    check_tables(g, schedule(g, SMS))
+    bad = g.derive()
+    bad.ops = bad.ops[1:]
+    with pytest.raises(VerifyError, match="no earlier op writes"):
+        check_tables(bad, schedule(bad, SMS))
+    # a K split added into a residual that was never made
+    g = mc.Graph()
+    r = g.unary(g.input("x", (16, 2048)), "relu")
+    g.output(g.unary(g.linear(g.input("h", (16, 2048)), g.param("w", (2048, 2048)), residual=r), "identity"))
+    out = passes.run_all(g, SMS)
+    assert "SplitFinalize" not in [o.kind for o in out.ops]
+    check_tables(out, schedule(out, SMS))
+    out.ops = [o for o in out.ops if o.kind != "Unary" or o.x.buf.kind == "temp"]
+    with pytest.raises(VerifyError, match="no earlier op writes"):
+        check_tables(out, schedule(out, SMS))
+
+
+def test_verifier_rejects_an_op_that_overwrites_its_own_operand():
+    """Instructions of one op run side by side: element by element in place is right, a linear over its own input is not."""
+    g = mc.Graph()
+    x = g.state("x", (300, 256))
+    g.unary(x, "relu", out=x)
+    check_hazards(schedule(g, SMS), g)
+    g.linear(x, g.param("w", (256, 256)), out=x)
+    with pytest.raises(VerifyError, match="with nothing between them"):
+        check_hazards(schedule(g, SMS), g)
