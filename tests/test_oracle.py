@@ -54,7 +54,7 @@ def test_builders_match_reference_graphs():
             assert x == y, (name, x, y)
 
 
-@pytest.mark.skipif(not REF.exists(), reason="reference tree not mounted")
+@pytest.mark.skipif(not (REF / "megacute").exists(), reason="reference tree not mounted")
 def test_reference_builder_files_run_unchanged():
     """examples/llama/model.py and examples/dit/model.py do `from megacute import Graph`: with this
     package registered under that name they build the same graphs as the fixtures."""
@@ -213,7 +213,7 @@ def test_oracle_agrees_with_reference_rewritten_graphs(name):
         assert "splits" in want["flags"]
 
 
-@pytest.mark.skipif(not REF.exists(), reason="reference tree not mounted")
+@pytest.mark.skipif(not (REF / "megacute").exists(), reason="reference tree not mounted")
 def test_reference_passes_live():
     """With the reference checkout at hand: rewrite a reference-built graph with its own passes now and
     evaluate both forms (the fixture above is this, frozen)."""
