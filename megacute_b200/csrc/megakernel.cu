@@ -655,6 +655,8 @@ int mk_program_set_ops(mk_program* p, const mk_op_desc* ops, int n_ops, void* st
             const char* attn_tc = getenv("MEGACUTE_B200_ATTN_TCGEN05");
             if (attn_tc && attn_tc[0] == '0') continue;
             if (tc_off || (D != 64 && D != 128) || (d.ptr[3] & 15) || d.ld[3] % 8) continue;
+            // (that body takes a row's maximum before it scales, and counts masked scores as -inf: the scale has to be positive)
+            if (!(d.f[0] > 0.f)) continue;
             const bool h16 = d.i[8] == mk::DT_F16;
             if (encode_tile_map(maps, d.ptr[0], B * Sq, H * D, d.ld[0], 128, false, h16) &&
                 encode_tile_map(maps + 128, d.ptr[1], B * Sk, KVH * D, d.ld[1], 128, false, h16) &&

@@ -103,6 +103,20 @@ def test_prefill_attention_tiles(cuda, B, Sq, Sk, H, KVH, D, causal):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("scale", [-0.3, 0.0])
+@pytest.mark.parametrize("D", [64, 128])
+def test_prefill_attention_scale_not_positive(cuda, D, scale):
+    """A negative scale turns the order of the scores around; zero gives every unmasked key the same weight."""
+    S, H = 200, 2
+    g = mc.Graph()
+    q, k, v = (g.unary(g.input(n, (S, H * D)), "identity") for n in "qkv")       # (private tensors: fp16)
+    g.output(g.attention(q, k, v, batch=1, heads=H, head_dim=D, causal=True, scale=scale))
+    t = {n: rnd((S, H * D), 1.0, i) for i, n in enumerate("qkv")}
+    outs, ref, _, _, prog = run_both(g, t, cuda, steps=2)
+    assert rel_l2(outs[0], ref[0]) < TOL and prog.tcgen05_attention_ops == 0
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("rows,cols,dtype,rms,group", [
     (257, 2048, BF, True, 0), (1190, 1024, BF, True, 0), (2390, 1000, BF, False, 0), (3001, 2048, F32, True, 0), (2400, 1024, BF, False, 40),
     (9600, 256, BF, True, 0), (2500, 8, F32, True, 0),
