@@ -33,7 +33,8 @@ constexpr int kSegElems = 2048;
 constexpr int kSegStride = kSegElems * 2 + 16;            // bytes between row segments of a stage
 constexpr int kStageBytes = 16 * kSegStride;              // 65 792 B
 constexpr int kStages = 2;
-constexpr int kRingBytes = kStages * kStageBytes;         // 128.5 KB, written only by bulk copies
+constexpr int kRingBytes = kStages * kStageBytes;         // 128.5 KB, written by bulk copies (and, behind the slots of 256-row tiles, by those
+                                                          // tiles' epilogues: the producer fences before other copies go there)
 constexpr int kWorkBytes = 96 * 1024 + 512;               // scratch of the instruction being executed (with the 512 bytes in front of
                                                           // its first 1024-byte boundary: six whole 16 KB operand tiles)
 constexpr int kXbufBytes = 64 * 1024;                     // GEMV: fp32 activation rows (front of work)
@@ -522,11 +523,14 @@ __device__ __forceinline__ bool wait_barrier(const Params& p, Ctrl* c, unsigned 
     return wait_barrier_spin(p, c, bar, parity, seq, where, patience);
 }
 
-// the same for a shared-memory word that only grows
+// the same for a shared-memory word that only grows, written behind a __threadfence_block()
 __device__ __forceinline__ bool wait_word(const Params& p, Ctrl* c, const uint32_t* word, uint32_t want, int seq, int where) {
     unsigned long long t0 = 0;
     for (uint32_t it = 1;; ++it) {
-        if (*(const volatile uint32_t*)word >= want) return true;
+        if (*(const volatile uint32_t*)word >= want) {
+            __threadfence_block();
+            return true;
+        }
         if ((it & 1023u) == 0) {
             if (*(volatile int*)&c->abort) return false;
             if (ld_volatile(&p.status[MK_ST_CODE]) != 0) { c->abort = 1; return false; }

@@ -42,7 +42,10 @@ __device__ int mk_run_gemm_wide(const Params& p, int idx, int slot) {
         slot += (last - idx) / (int)gridDim.x;                  // (the last instruction's; not Ctrl::run_slot: thread 0 may be in the next run already)
         if (!next_is(p, m.ctrl, last, slot, [](const mk_op_desc* op) { return is_wide_gemm(op); })) {
             // (behind the last instruction's barrier: nobody reads the staging rows any more)
-            if (threadIdx.x == 0) *(volatile uint32_t*)&m.ctrl->wide_done = m.ctrl->wide_uses;
+            if (threadIdx.x == 0) {
+                __threadfence_block();
+                *(volatile uint32_t*)&m.ctrl->wide_done = m.ctrl->wide_uses;
+            }
             return last;
         }
         idx = last + (int)gridDim.x;

@@ -224,7 +224,14 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
                     ok = wait_barrier(p, c, &c->empty[s], (pos.phase ^ (s < pos.stage ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
             }
         }
-        return __shfl_sync(0xffffffffu, ok, 0) != 0;
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        if (kind >= MODE_WWIDE && next < MODE_WWIDE) {
+            // those rows (and the bias) were written with plain stores and cp.async, by the compute warps; bulk copies are next,
+            // from any lane: each orders its own behind what lane 0 has seen
+            __syncwarp();
+            asm volatile("fence.proxy.async;" ::: "memory");
+        }
+        return ok != 0;
     };
     auto enter = [&](int kind) -> bool {              // make the ring's memory serve `kind`
         if (mode == kind) return true;

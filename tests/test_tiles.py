@@ -6,7 +6,7 @@ import torch
 import megacute_b200 as mc
 from megacute_b200 import passes
 from megacute_b200 import workloads as W
-from oracle.graph_oracle import rel_l2
+from oracle.graph_oracle import evaluate, rel_l2
 from tests.helpers import TOL
 from tests.test_gpu_ops import rnd, run_both
 
@@ -156,3 +156,40 @@ def test_hoisted_linears_keep_their_order():
         assert all(v.buf.id in seen for v in o.reads)
         seen |= {v.buf.id for v in o.writes}
     assert len(ops) == len(g.ops) and ops[-3].x.same(x)
+
+
+@pytest.mark.gpu
+def test_ring_changes_hands_behind_256_row_tiles(cuda, monkeypatch):
+    """The epilogues of 256-row tiles leave a bias row, gate rows or staged rows in the ring's memory; 128-row tiles and streaming
+    linears that depend on nothing follow at once, with copies into the same bytes.  Every SM has each of them, three times over."""
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 128))
+    monkeypatch.setattr(passes, "hoist_linears", lambda g: g)                   # (keeps the order below)
+    M, N, K, Ns = 2048, 2432, 64, 148 * 128
+    g = mc.Graph()
+    x, xs, x1 = g.input("x", (M, K)), g.input("xs", (100, K)), g.input("x1", (1, K))
+    t = {"x": rnd((M, K), 1.0, 1), "xs": rnd((100, K), 1.0, 2), "x1": rnd((1, K), 1.0, 3)}
+
+    def p(name, rows, cols, std):
+        t[name] = rnd((rows, cols), std, len(t))
+        return g.param(name, (rows, cols))
+
+    for i in range(3):
+        a = g.linear(x, p(f"wa{i}", N, K, 0.1), bias=p(f"ba{i}", 1, N, 1.0), act="relu")
+        s = g.linear(xs, p(f"ws{i}", Ns, K, 0.1))
+        r = g.temp((M, N))
+        g.unary(a, "identity", out=r)
+        b = g.add(r, g.binary(g.linear(x, p(f"wb{i}", N, K, 0.1)), p(f"gb{i}", M // 64, N, 1.0), "mul", b_group=64))
+        v = g.linear(x1, p(f"wv{i}", Ns, K, 0.1))
+        c = g.linear(x, p(f"wc{i}", N, K, 0.1), act="relu", residual=a)
+        s2 = g.linear(xs, p(f"wt{i}", Ns, K, 0.1))
+        g.output(a, s, b, v, c, s2)
+    prog = mc.compile(g)
+    dev = {k: w.to(cuda) for k, w in t.items()}
+    ref, _ = evaluate(g, dev, cuda)
+    for _ in range(10):
+        for o, want in zip(prog(**dev), ref):
+            # every output row on its own: a damaged tile does not hide in the whole tensor
+            err = (o.float() - want).norm(dim=1) / want.norm(dim=1)
+            assert float(err.max()) < TOL
+    prog.check()
+    assert sum(o.kind == "Linear" and o.bm == 256 for o in prog.g.ops) == 9
