@@ -558,6 +558,14 @@ __device__ __forceinline__ bool check_phase(const Params& p, Ctrl* c, unsigned l
 #endif
     return true;
 }
+// ... by a whole warp, which goes one way
+__device__ __forceinline__ bool check_phase_warp(const Params& p, Ctrl* c, unsigned long long* bar, uint32_t parity, int seq, int where) {
+#ifdef MK_CHECK
+    return __all_sync(0xffffffffu, check_phase(p, c, bar, parity, seq, where)) != 0;
+#else
+    return true;
+#endif
+}
 
 MK_SPIN bool wait_counter_spin(const Params& p, Ctrl* c, int counter, int want, int seq) {
     const int* addr = p.counters + counter;

@@ -163,7 +163,8 @@ __device__ __forceinline__ bool at_feed(const Params& p, Ctrl* c, uint8_t* ring,
     if (lane == 0) {
         // the tiles' memory was last written through the generic proxy, and so were q, k and v, by other SMs
         asm volatile("fence.proxy.async;" ::: "memory");
-        ok = wait_barrier(p, c, &a->q_free, (f.insts & 1u) ^ 1u, in.seq, WHERE_RING_EMPTY, 2);
+        ok = wait_barrier(p, c, &a->q_free, (f.insts & 1u) ^ 1u, in.seq, WHERE_RING_EMPTY, 2) &&
+             check_phase(p, c, &a->q_full, f.insts & 1u, in.seq, WHERE_CHECK_ARM);
         if (ok) {
             const int qtiles = in.a2 * 256 + 128 < Sq ? 2 : 1, qrow = in.a0 * Sq + in.a2 * 256;
             mbar_arrive_expect_tx(&a->q_full, (uint32_t)(qtiles * M::kTile));
@@ -176,12 +177,12 @@ __device__ __forceinline__ bool at_feed(const Params& p, Ctrl* c, uint8_t* ring,
         const int krow = in.a0 * Sk;
         for (int j = 0; j < nb && ok; ++j) {
             const uint32_t n = f.tiles + (uint32_t)j, u = n & 1u, ph = (n >> 1) & 1u;
-            ok = wait_barrier(p, c, &a->k_empty[u], ph ^ 1u, in.seq, WHERE_RING_EMPTY, 2);
+            ok = wait_barrier(p, c, &a->k_empty[u], ph ^ 1u, in.seq, WHERE_RING_EMPTY, 2) && check_phase(p, c, &a->k_full[u], ph, in.seq, WHERE_CHECK_ARM);
             if (!ok) break;
             mbar_arrive_expect_tx(&a->k_full[u], (uint32_t)M::kTile);
             for (int s = 0; s < D / 64; ++s)
                 tma_load_2d_plain(ring + M::kK + u * M::kTile + s * kTcTileBytes, tmaps + 128, hk * D + s * 64, krow + j * 128, &a->k_full[u]);
-            ok = wait_barrier(p, c, &a->v_empty[u], ph ^ 1u, in.seq, WHERE_RING_EMPTY, 2);
+            ok = wait_barrier(p, c, &a->v_empty[u], ph ^ 1u, in.seq, WHERE_RING_EMPTY, 2) && check_phase(p, c, &a->v_full[u], ph, in.seq, WHERE_CHECK_ARM);
             if (!ok) break;
             mbar_arrive_expect_tx(&a->v_full[u], (uint32_t)M::kTile);
             for (int s = 0; s < D / 64; ++s)
@@ -221,6 +222,7 @@ __device__ __forceinline__ bool at_issue(const Params& p, Ctrl* c, uint8_t* ring
             if (at_ready(bar, parity)) return true;
         return issuer_wait(p, c, bar, parity, info.w, WHERE_RING_FULL, 2);
     };
+    auto released = [&](unsigned long long* bar, uint32_t parity) { return check_phase_warp(p, c, bar, parity, info.w, WHERE_CHECK_RELEASE); };
     auto tile_of = [&](int n) { return n < 2 * both ? n & 1 : tail; };
     auto block_of = [&](int n) { return n < 2 * both ? n >> 1 : n - both; };
     // scores of the n-th block into their buffer: the block that had it before has been multiplied (its P V is ahead in the pipe)
@@ -228,6 +230,8 @@ __device__ __forceinline__ bool at_issue(const Params& p, Ctrl* c, uint8_t* ring
         const int t = tile_of(n), j = block_of(n);
         const uint32_t k = f.tiles + (uint32_t)j, u = k & 1u, seq = first + (uint32_t)n, buf = seq % M::kScores;
         if (!await(&a->k_full[u], (k >> 1) & 1u)) return false;
+        if (!(released(&a->s_full[seq % 3u], (seq / 3u) & 1u) && released(&a->k_empty[u], (k >> 1) & 1u))) return false;
+        if (n == total - 1 && !released(&a->q_free, f.insts & 1u)) return false;
         tc_fence_after();
         const uint64_t qd = d0 + (uint32_t)((M::kQ + t * M::kTile) >> 4), kd = d0 + ((uint32_t)M::kK >> 4) + u * (uint32_t)(M::kTile >> 4);
         const bool alone = j >= both;                         // the other tile does not read this K tile
@@ -255,6 +259,7 @@ __device__ __forceinline__ bool at_issue(const Params& p, Ctrl* c, uint8_t* ring
         if (!await(&a->v_full[u], (k >> 1) & 1u)) return false;
         // (the first P V overwrites O: the compute warps must have read the previous instruction's)
         if (j == 0 && f.outs[t] > 0 && !await(&a->o_free[t], (f.outs[t] - 1u) & 1u)) return false;
+        if (!(released(&a->pv_done[t], (f.blocks[t] + (uint32_t)j) & 1u) && released(&a->v_empty[u], (k >> 1) & 1u))) return false;
         tc_fence_after();
         const uint64_t vd = v0 + ((uint32_t)M::kV >> 4) + u * (uint32_t)(M::kTile >> 4);
         const bool alone = j >= both;
@@ -402,7 +407,7 @@ __device__ __forceinline__ void op_attention_tc(const Params& p, Ctrl* c, const 
         tc_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&a->p_full[t]);                             // S read, P written
+        if (lane == 0 && check_phase(p, c, &a->p_full[t], (base + (uint32_t)j) & 1u, seq, WHERE_CHECK_RELEASE)) mbar_arrive(&a->p_full[t]);      // S read, P written
     }
     phase_mark(p, c, 1);                                                       // last P handed over
     // ---- out = O / l ----

@@ -79,6 +79,8 @@ __device__ __forceinline__ bool wide_feed(const Params& p, Ctrl* c, uint8_t* rin
                 c->wide_info[e] = make_int4(nk, (M - m0 > 128 ? 2 : 1) | (op->i[10] >> 7) << 4, op->i[9] == DT_F16 ? 1 : 0, in.seq);
                 mbar_arrive(&c->wide_told[e]);
             }
+            ok = check_phase(p, c, &c->ww_full[kind][slot], phase, in.seq, WHERE_CHECK_ARM);
+            if (!ok) break;
             mbar_arrive_expect_tx(&c->ww_full[kind][slot], (uint32_t)kWideXBytes);
             tma_load_2d(ring + wide_xoff((int)slot), tmaps, kbeg + kt * 64, m0, &c->ww_full[kind][slot], keep);
             if (++slot == (uint32_t)wide_stages(kind)) { slot = 0; phase ^= 1u; }
@@ -128,6 +130,10 @@ __device__ __forceinline__ bool wide_issue(const Params& p, Ctrl* c, uint8_t* ri
             // accumulator has been read)
             if (kind && !issuer_wait(p, c, &c->wacc_empty[1], (n & 1u) ^ 1u, info.w, WHERE_COMBINE, 2)) return false;
         }
+        if (!check_phase_warp(p, c, &c->ww_empty[kind][s], ph, info.w, WHERE_CHECK_RELEASE)) return false;
+        if (kt == nk - 1 && !(check_phase_warp(p, c, &c->wacc_full[0], n & 1u, info.w, WHERE_CHECK_RELEASE) &&
+                              check_phase_warp(p, c, &c->wacc_full[1], n & 1u, info.w, WHERE_CHECK_RELEASE)))
+            return false;
         tc_fence_after();
         const uint64_t ad = d0 + (uint32_t)(wide_xoff((int)s) >> 4), bd = d0 + (uint32_t)(wide_woff(kind, (int)s) >> 4);
         if (kind) {
@@ -201,10 +207,10 @@ __device__ __forceinline__ bool wide_wait(const Params& p, Ctrl* c, const WideAc
     __syncwarp();                        // (the tensor-memory loads are .sync.aligned: whole warp, converged)
     return ok != 0;
 }
-__device__ __forceinline__ void wide_release(unsigned long long* bar) {
+__device__ __forceinline__ void wide_release(const Params& p, Ctrl* c, const WideAcc& a) {
     tc_fence_before();
     __syncwarp();
-    if ((threadIdx.x & 31) == 0) mbar_arrive(bar);
+    if ((threadIdx.x & 31) == 0 && check_phase(p, c, a.release, a.parity, a.seq, WHERE_CHECK_RELEASE)) mbar_arrive(a.release);
 }
 __device__ __forceinline__ void wide_bias(const uint8_t* bias, int col, float* v) {          // 32 columns from shared memory (the same for all lanes)
 #pragma unroll
@@ -306,12 +312,12 @@ __device__ __forceinline__ void wide_store16(const Params& p, Ctrl* c, const mk_
             const uint32_t tacc = a.tacc + (g >> 1) * 128 + (g & 1) * 32;
             tc_ld32(tacc, v);
             tc_ld32(tacc + 64, u);
-            if (g == groups - 1) wide_release(a.release);
+            if (g == groups - 1) wide_release(p, c, a);
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = v[j] * sigmoidf_(v[j]) * u[j];
         } else {
             tc_ld32(a.tacc + g * 32, v);
-            if (g == groups - 1) wide_release(a.release);
+            if (g == groups - 1) wide_release(p, c, a);
             if (a.bias) wide_bias(a.bias, g * 32, v);
             if (ACT == 1) {
 #pragma unroll
@@ -378,7 +384,7 @@ __device__ __forceinline__ void wide_store_res(const Params& p, Ctrl* c, const m
             const int g = g0 + d;
             float v[32];
             tc_ld32(a.tacc + g * 32, v);
-            if (g == groups - 1) wide_release(a.release);
+            if (g == groups - 1) wide_release(p, c, a);
             if (a.bias) wide_bias(a.bias, g * 32, v);
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
@@ -456,7 +462,7 @@ __device__ __forceinline__ void wide_store_rope(const Params& p, Ctrl* c, const 
             float x1[16], x2[16];
             __syncwarp();
             tc_ld16x2(a.tacc + h + d, a.tacc + h + half + d, x1, x2);
-            if (d + 16 == half && h + D == cols) wide_release(a.release);
+            if (d + 16 == half && h + D == cols) wide_release(p, c, a);
             if (h < rot) {
 #pragma unroll
                 for (int e = 0; e < 16; e += 2) {
@@ -512,7 +518,7 @@ __device__ __forceinline__ void wide_store_any(const Params& p, Ctrl* c, const m
             if (a.bias) wide_bias(a.bias, g * 32, v);
             if (act != ACT_NONE) act_all(act, v);
         }
-        if (g == groups - 1) wide_release(a.release);
+        if (g == groups - 1) wide_release(p, c, a);
 #pragma unroll
         for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(wide_chunk(a.stg, lane, j)) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
         __syncwarp();
@@ -593,7 +599,7 @@ __device__ __forceinline__ void op_gemm_tc_wide(const Params& p, Ctrl* c, uint8_
     const WideAcc a{&c->wacc_full[h], &c->wacc_empty[h], par, *(volatile uint32_t*)&c->tmem_base + ((uint32_t)(qd * 32) << 16) + 256u * h,
                     ring + kWideStageOff + warp * 4096, bias, seq};
     if (row0 >= op->i[0]) {                                     // (rows beyond M)
-        if (wide_wait(p, c, a)) wide_release(a.release);
+        if (wide_wait(p, c, a)) wide_release(p, c, a);
         return;
     }
     if constexpr (V >= WIDE_RES) {

@@ -282,6 +282,7 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
                     int ok = 1;
                     if (lane == 0) {
                         ok = wait_barrier(p, c, &c->kv_empty[kvslot], kvphase ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
+                        if (ok && !check_phase(p, c, &c->kv_full[kvslot], kvphase, rc.seq, WHERE_CHECK_ARM)) ok = 0;
                         if (ok) mbar_arrive_expect_tx(&c->kv_full[kvslot], tile_bytes);
                     }
                     if (!__shfl_sync(0xffffffffu, ok, 0)) return;      // (also: the expected bytes are registered before any copy is issued)
@@ -316,6 +317,7 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
                 for (int kt = 0; kt < nkt; ++kt) {
                     if (!wait_barrier(p, c, empty + sl, ph ^ 1u, rc.seq, WHERE_RING_EMPTY, 2)) { ok = 0; break; }
                     uint8_t* dst = ring + wide_woff(kind, sl);
+                    if (!check_phase(p, c, full + sl, ph, rc.seq, WHERE_CHECK_ARM)) { ok = 0; break; }
                     mbar_arrive_expect_tx(full + sl, wbytes);
                     if (src) {
                         bulk_g2s_hint(dst, src + kt * kstep, wbytes, full + sl, wpol);
@@ -397,6 +399,7 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
         const __nv_bfloat16* src; int bytes, off;
         rc.piece(lane, src, bytes, off);
         const int total = __reduce_add_sync(0xffffffffu, bytes);
+        if (!check_phase_warp(p, c, &c->full[pos.stage], pos.phase, rc.seq, WHERE_CHECK_ARM)) return;
         if (lane == 0) mbar_arrive_expect_tx(&c->full[pos.stage], (uint32_t)total);
         __syncwarp();
         if (bytes) bulk_g2s_hint(ring + pos.stage * kStageBytes + off, src, (uint32_t)bytes, &c->full[pos.stage], stream_policy);
