@@ -159,7 +159,8 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                         const int ppos = pos.stage | ((int)pos.phase << 8);
             int npos = ppos;
             bool known = true, aborting = false;
-            int run_last = idx - 1;                 // (a body that keeps the walk: the index of the last instruction it ran, or -1 when aborting)
+            constexpr int kNotRun = -2;
+            int run_last = kNotRun;                 // (a body that keeps the walk: the index of the last instruction it ran, or -1 when aborting)
             switch (op->kind) {
                 case MK_OP_GEMV:
                     if (op->flags & GEMV_F_UNITS) {
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                     aborting = publish(p, c, in.narrive, arrive_off);
                     break;
             }
-            const bool ran = run_last != idx - 1;
+            const bool ran = run_last != kNotRun;
             if (ran) {
                 aborting = run_last < 0;
                 if (!aborting) {

@@ -278,6 +278,47 @@ def test_timeout_is_reported_not_hung(cuda):
     assert torch.equal(again, good)
 
 
+@pytest.mark.parametrize("first", ["norm", "pointwise", "128-row tile", "256-row tile", "attention"])
+def test_timeout_of_the_first_instruction(cuda, monkeypatch, first):
+    """The very first instruction of the program waits for a counter that is never reached: CTA 0 leaves, although its body would
+    have gone on with the CTA's next instructions, and the program works once the wait is put right."""
+    from megacute_b200 import _lib, passes
+    from megacute_b200.runtime import Program
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 128) if first == "256-row tile" else (1, 128, 128))
+    M, N = 4096, 1024
+    g = mc.Graph()
+    x = g.input("x", (M, N))
+    t = {"x": rnd((M, N), 1.0, 1)}
+    if first == "norm":
+        y = g.rms_norm(x)
+    elif first == "pointwise":
+        y = g.unary(x, "silu")
+    elif first == "attention":
+        y = g.attention(x, x, x, batch=8, heads=16, head_dim=64, causal=True)
+    else:
+        t["w"] = rnd((N, N), 0.03, 2)
+        y = g.linear(x, g.param("w", (N, N)))
+    g.output(g.unary(y, "neg"))
+    prog = Program(g)
+    s = prog.sched
+    s.wait_ptr = s.wait_ptr.copy()
+    s.wait_ptr[1:] += 1
+    s.wait_cnt, s.wait_tgt = np.concatenate([[0], s.wait_cnt]), np.concatenate([[1000], s.wait_tgt])
+    prog.compile()
+    prog.set_timeout(0.05)
+    dev = {k: v.to(cuda) for k, v in t.items()}
+    prog(**dev)
+    with pytest.raises(_lib.MegakernelTimeout):
+        prog.check()
+    _lib.check(_lib.load().mk_program_poke_wait(prog._handle, 0, 0, 0))
+    prog.reset()
+    prog.set_timeout(2.0)
+    out = prog(**dev)
+    prog.check()
+    ref, _ = evaluate(g, t)
+    assert rel_l2(out.float().cpu(), ref[0]) < TOL
+
+
 def test_timeline(cuda):
     g, params, st, ids = small_decode(B=1, n=2)
     prog = mc.compile(g, trace=True)
