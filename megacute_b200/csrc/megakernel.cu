@@ -436,6 +436,7 @@ static bool tile_gemm_on_tcgen05(const mk_op_desc& d) {
 static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
     const int W = MK_INST_WORDS;
     auto ceil_div = [](long long a, long long b) { return (a + b - 1) / b; };
+    auto is_float = [](int dt) { return dt == mk::DT_BF16 || dt == mk::DT_F32 || dt == mk::DT_F16; };
     for (int k = 0; k < p->n_insts; ++k) {
         const int32_t* w = p->h_insts.data() + (size_t)k * W;
         const int opi = w[0] - 1;
@@ -466,9 +467,12 @@ static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
                     break;
                 case MK_OP_ELTWISE:
                     if (d.i[10] <= 0 || a0 < 0 || a0 * d.i[10] >= d.i[0] || a1 < 0 || a1 * 512 >= d.i[1]) why = "pointwise: tile outside the output";
+                    else if (d.i[2] < 0 || d.i[2] > 5 || !is_float(d.i[6]) || !is_float(d.i[7]) || !is_float(d.i[8]) || !is_float(d.i[9])) why = "pointwise: mode or dtype";
+                    else if (d.i[4] <= 0 || (d.i[2] == 4 && (d.i[5] <= 0 || d.i[5] % 16 || 512 % d.i[5]))) why = "pointwise: rows per group or head_dim";
                     break;
                 case MK_OP_NORM:
                     if (d.i[3] <= 0 || a0 < 0 || a0 * d.i[3] >= d.i[0]) why = "norm: row group outside the rows";
+                    else if (!is_float(d.i[4]) || !is_float(d.i[5]) || !is_float(d.i[7]) || !is_float(d.i[8])) why = "norm: dtype";
                     break;
                 case MK_OP_ATTENTION:
                     if (a0 < 0 || a0 >= d.i[0] || a1 < 0 || a1 >= d.i[3] || a2 < 0 || a2 * 256 >= d.i[1]) why = "attention: (batch, head, query tile)";

@@ -38,7 +38,9 @@ __device__ int mk_run_eltwise(const Params& p, const mk_op_desc* op, int idx, in
         MK_ROPE(DT_F32, DT_BF16); MK_ROPE(DT_F32, DT_F16); MK_ROPE(DT_F32, DT_F32);
 #undef MK_ROPE
 #undef MK_EW
-        default: return -1;
+        default:                                             // (no such variant: the mode or a dtype is not one)
+            if (threadIdx.x == 0) report(p, smem_map().ctrl, MK_DEV_BAD_INST, smem_map().ctrl->meta.inst[slot % 3][3].x, 2, op->i[2], idx, 0);
+            return -1;
     }
 }
 __device__ int mk_run_norm(const Params& p, const mk_op_desc* op, int idx, int slot) {

@@ -147,3 +147,32 @@ def test_grid_larger_than_the_device_is_an_argument_error(cuda):
     rc = lib.mk_launch_noalloc(cuda.index or 0, dummy.data_ptr(), 1, None, 0, None, 0, dummy.data_ptr(), 1, 1,
                                caps.sm_count + 1, None, None)
     assert rc == -2
+
+
+def test_unknown_pointwise_mode_is_reported(cuda):
+    """A descriptor with a mode that does not exist: refused when it is bound, reported by the kernel where nothing is bound."""
+    g = mc.Graph()
+    g.output(g.unary(g.unary(g.input("x", (2048, 1024)), "relu"), "neg"))
+    x = torch.ones(2048, 1024, dtype=BF, device=cuda)
+    prog = mc.compile(g)
+    want = prog(x=x).clone()
+    prog.check()
+    lib = _lib.load()
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    bad = (_lib.OpDesc * len(prog.g.ops))()
+    for field, value in ((2, 9), (6, 3), (9, 7), (4, 0)):
+        ctypes.memmove(bad, prog._desc, ctypes.sizeof(bad))
+        bad[0].i[field] = value
+        rc = lib.mk_program_set_ops(prog._handle, ctypes.addressof(bad), len(prog.g.ops), stream)
+        assert rc == -2 and b"pointwise" in lib.mk_last_cuda_error()
+    assert torch.equal(prog(x=x), want)
+    prog.check()
+    ctypes.memmove(bad, prog._desc, ctypes.sizeof(bad))
+    bad[0].i[2] = 9
+    insts, waits, arrives = (a.to(cuda) for a in prog._tables)
+    desc = torch.frombuffer(bytearray(bytes(bad)), dtype=torch.uint8).to(cuda)
+    status = (ctypes.c_int32 * _lib.ST_WORDS)()
+    s = prog.sched
+    rc = lib.mk_launch_noalloc(cuda.index or 0, insts.data_ptr(), s.n, waits.data_ptr(), len(s.wait_cnt), arrives.data_ptr(), len(s.arr_cnt),
+                               desc.data_ptr(), len(prog.g.ops), s.num_counters, prog.sm_count, stream, status)
+    assert rc == -4 and status[0] == 3                 # MK_E_DEVICE, MK_DEV_BAD_INST
