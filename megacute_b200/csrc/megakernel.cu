@@ -454,8 +454,11 @@ static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
                     if (d.i[4] <= 0 || d.i[18] <= 0 || d.i[19] < 0 || d.i[19] >= d.i[4] ||
                         (long long)d.i[18] * d.i[4] + (long long)d.i[19] * (d.i[2] & 63 ? 32 : 64) != d.i[2])
                         why = "tile GEMM: split count";
+                    else if (d.i[11] != 0 && d.i[11] != 128 && d.i[11] != 256) why = "tile GEMM: activation rows per tile";
+                    // (128, or 0 for it; beside 256 activation rows 128 or 256, in so many words: every role of that body reads it)
+                    else if (d.i[11] == 256 ? !(d.i[10] == 128 || (d.i[10] == 256 && d.i[1] % 256 == 0)) : (d.i[10] != 0 && d.i[10] != 128))
+                        why = "tile GEMM: weight rows per tile";
                     else if (a0 < 0 || a0 * (long long)(d.i[11] == 256 ? 256 : 128) >= d.i[0]) why = "tile GEMM: m tile outside M";
-                    else if (d.i[10] != 0 && d.i[10] != 128 && !(d.i[10] == 256 && d.i[11] == 256 && d.i[1] % 256 == 0)) why = "tile GEMM: weight rows per tile";
                     else if (a1 < 0 || a1 * (long long)(d.i[10] == 256 ? 256 : 128) >= d.i[1]) why = "tile GEMM: n tile outside N";
                     else if (a2 < 0 || a2 >= d.i[4]) why = "tile GEMM: K split index";
                     else if (d.ptr[6] && ((d.i[15] != 64 && d.i[15] != 128) || d.i[16] <= 0 || d.i[14] % d.i[15] || d.i[14] > d.i[1]))

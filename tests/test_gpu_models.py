@@ -391,6 +391,12 @@ def test_bind_checks_instruction_arguments(cuda):
     bad[k].i[0] = 100                                    # M = 100: the instruction of m tile 1 now starts past the rows
     rc = lib.mk_program_set_ops(prog._handle, ctypes.addressof(bad), len(prog.g.ops), stream)
     assert rc == -2 and b"m tile" in lib.mk_last_cuda_error()
+    # 256 activation rows per tile want the weight rows in so many words, 128 or 256; other heights there are none
+    for rows, cols in ((256, 0), (256, 64), (64, 128), (512, 128), (128, 256)):
+        ctypes.memmove(bad, prog._desc, ctypes.sizeof(bad))
+        bad[k].i[10], bad[k].i[11] = cols, rows
+        rc = lib.mk_program_set_ops(prog._handle, ctypes.addressof(bad), len(prog.g.ops), stream)
+        assert rc == -2 and b"rows per tile" in lib.mk_last_cuda_error()
     again = prog(**dev)                                  # the refused table changed nothing
     prog.check()
     assert torch.equal(again, good)
