@@ -95,14 +95,16 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         c->tmem_base = kTcNoTmem;
         c->tmem_ready = 0;
         c->abort = 0;
+        c->x_left[0] = c->x_left[1] = 0xff;
         c->flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
 
+    uint32_t left = 0;               // producer and feeder: copies in flight when they left their loop
     if (warp == kProducerWarp) {
         // ---------------- producer warp ----------------
-        producer_loop<TRACE>(p, c, ring);
+        left = producer_loop<TRACE>(p, c, ring);
     } else if (warp == kFinisherWarp) {
         // ---------------- finisher warp: epilogues of the streaming linear ----------------
         mk_gemv_finisher(p);
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         // ---------------- feeder warp: tiles of the tcgen05 prefill attention, activation tiles of tile GEMMs with 256-row tiles ----------------
         // (a warp of its own rather than a branch of the producer's loop: the call in that loop cost every decode step
         // 0.5 %, whether or not the graph had such an op; here a graph without one costs a walk over the instruction list)
-        mk_feeder(p);
+        left = mk_feeder(p);
     } else if (warp == kIssuerWarp) {
         // ---------------- issuer warp: MMAs of tile GEMMs with 256-row tiles and of the tcgen05 prefill attention ----------------
         mk_issuer(p);
@@ -220,44 +222,16 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         asm volatile("cp.async.wait_all;" ::: "memory");      // staged metadata of instructions that never ran
     }
     __syncthreads();
-    // Abort path only: bulk copies may still be landing in the ring.  Wait (bounded) for the
-    // latest fill of every stage before the CTA gives its shared memory back.
-    if (c->abort && threadIdx.x == kProducerWarp * 32) {
-        for (int s = 0; s < kStages; ++s) {
-            unsigned long long t0 = globaltimer();
-            // a stage whose fill was issued has a pending phase; both parities are polled because
-            // the role that knew the parity has already left its loop
-            while (!(mbar_try_wait(&c->full[s], 0) || mbar_try_wait(&c->full[s], 1))) {
-                if (globaltimer() - t0 > 20000000ull) break;      // 20 ms
-            }
+    // Abort path only: bulk copies may still be landing in shared memory, and products reading it.  The roles that requested copies
+    // wait (bounded) for theirs; a pause then covers what cannot be waited for (a copy takes a few microseconds).
+    if (c->abort && (threadIdx.x & 31) == 0) {
+        if (warp == kFeederWarp) mk_feeder_landed(left);
+        if (warp == kProducerWarp) {
+            wait_landed(c->full + (left >> 16), (left >> 12) & 15, left);
+            mk_gemm_landed();
+            const unsigned long long t0 = globaltimer();
+            while (globaltimer() - t0 < 200000ull) {}
         }
-        for (int s = 0; s < kTcWSlots; ++s) {
-            unsigned long long t0 = globaltimer();
-            while (!(mbar_try_wait(&c->w_full[s], 0) || mbar_try_wait(&c->w_full[s], 1))) {
-                if (globaltimer() - t0 > 20000000ull) break;
-            }
-        }
-        for (int s = 0; s < 2 * kWideStages; ++s) {
-            unsigned long long t0 = globaltimer();
-            while (!(mbar_try_wait(&c->ww_full[0][0] + s, 0) || mbar_try_wait(&c->ww_full[0][0] + s, 1))) {
-                if (globaltimer() - t0 > 20000000ull) break;
-            }
-        }
-        for (int s = 0; s < 5; ++s) {                              // tiles of the tcgen05 attention
-            unsigned long long* bar = s == 0 ? &c->attn.q_full : s < 3 ? &c->attn.k_full[s - 1] : &c->attn.v_full[s - 3];
-            unsigned long long t0 = globaltimer();
-            while (!(mbar_try_wait(bar, 0) || mbar_try_wait(bar, 1))) {
-                if (globaltimer() - t0 > 20000000ull) break;
-            }
-        }
-        for (int s = 0; s < kKvSlots; ++s) {                       // KV tiles of the many-sequence decode attention
-            unsigned long long t0 = globaltimer();
-            while (!(mbar_try_wait(&c->kv_full[s], 0) || mbar_try_wait(&c->kv_full[s], 1))) {
-                if (globaltimer() - t0 > 20000000ull) break;
-            }
-        }
-        unsigned long long t0 = globaltimer();
-        while (globaltimer() - t0 < 200000ull) {}                  // let in-flight copies retire
     }
     __syncthreads();
     // tensor memory of the tile GEMM (allocated by the CTA's first such instruction) goes back here

@@ -181,8 +181,10 @@ struct Ctrl {                     // lives in the last kCtrlBytes of shared memo
     unsigned long long ring_granted, ring_returned;      // ... head_dim 128: the run may use the ring's memory / is done with it
     uint32_t at_blocks[2][2];                // ... blocks of each Q tile so far, written for the next instruction during this one
     uint32_t tmem_base;               // ... tensor-memory address of the accumulator (written by tcgen05.alloc)
-    uint32_t x_par;                       // ... bit s: parity of the next completion of x_full[s] and of x_empty[s] (between
+    uint16_t x_par;                       // ... bit s: parity of the next completion of x_full[s] and of x_empty[s] (between
                                           //     instructions both have completed equally often); set at an instruction's end
+    uint8_t x_left[2];                    // ... during one, by the lane that arms every other stage, once it has: next stage | round << 4 |
+                                          //     ten stages << 5; read on the abort path only.  0xff between instructions
     uint8_t w_slot, w_phase;              // ... the MMA thread's position in the weight slots
     uint8_t at_turn;                      // tcgen05 prefill attention: which at_blocks is current (bit 0)
     uint8_t tmem_ready;               // 1 once tensor memory is allocated; written behind the barrier that follows the allocation, so
@@ -541,6 +543,26 @@ __device__ __forceinline__ bool wait_word(const Params& p, Ctrl* c, const uint32
                 return false;
             }
         }
+    }
+}
+
+// Bulk copies that a role may have left in flight, returned when it leaves its loop and used on the abort path only: first barrier
+// (counted from Ctrl::full[0]) << 16 | number << 12 | bit s: the parity of the phase that barrier s was last armed for (never armed: 1,
+// which counts as complete).
+// Those parities, of `n` barriers armed one after the other; the next is `slot`, in the round of parity `phase`:
+__device__ __forceinline__ uint32_t armed_parities(int n, int slot, uint32_t phase) {
+    return ((phase ? 0u : ~0u) ^ ((1u << slot) - 1u)) & ((1u << n) - 1u);
+}
+__device__ __forceinline__ uint32_t copies_left(Ctrl* c, const unsigned long long* first, int n, uint32_t parities) {
+    return (uint32_t)(first - c->full) << 16 | (uint32_t)n << 12 | parities;
+}
+// Abort path: wait until the latest copy armed on each of `n` barriers has landed.  (A stage of the 256-row tiles that only one of
+// its two loaders has armed never completes: the limit, far beyond any copy's time, ends that wait.)
+static __device__ __noinline__ void wait_landed(unsigned long long* first, int n, uint32_t parities) {
+    for (int s = 0; s < n; ++s) {
+        const unsigned long long t0 = globaltimer();
+        while (!mbar_try_wait(first + s, (parities >> s) & 1u))
+            if (globaltimer() - t0 > 2000000ull) break;       // 2 ms
     }
 }
 

@@ -25,32 +25,36 @@ __device__ int mk_run_attention(const Params& p, const mk_op_desc* op, int idx, 
     return op->i[5] == 64 ? attention_run<64>(p, idx, slot) : attention_run<128>(p, idx, slot);
 }
 
-__device__ void mk_feeder(const Params& p) {
+__device__ uint32_t mk_feeder(const Params& p) {
     const SmemMap m = smem_map();
     WideFeed wf;
     AtFeed af;
     int run = 0;                                              // what the CTA's previous instruction was: 1 a 256-row tile, head_dim of an attention, 0 neither
     // the whole warp walks the list (and leaves together: the kernel ends with CTA-wide barriers)
-    for (int idx = blockIdx.x; idx < p.n_insts; idx += gridDim.x) {
+    int idx = blockIdx.x;
+    for (; idx < p.n_insts; idx += gridDim.x) {
         const Inst in = fetch_inst(p, idx);
         const int opi = in.opi - 1;
-        if (opi < 0 || opi >= p.n_ops) return;
+        if (opi < 0 || opi >= p.n_ops) break;
         const mk_op_desc* op = p.ops + opi;
         if (is_wide_gemm(op)) {
-            if (!wide_feed(p, m.ctrl, m.ring, op, in, run != 1, wf)) return;
+            if (!wide_feed(p, m.ctrl, m.ring, op, in, run != 1, wf)) break;
             run = 1;
         } else if (is_attention_tc(op)) {
             const int D = op->i[5];
             const bool ok = D == 64 ? at_feed<64>(p, m.ctrl, m.ring, op, in, run != D, af, wf.count) : at_feed<128>(p, m.ctrl, m.ring, op, in, run != D, af, wf.count);
             ++wf.count;
-            if (!ok) return;
+            if (!ok) break;
             run = D;
         } else {
             run = 0;
         }
     }
-    wide_feed_end(m.ctrl, wf);
+    if (idx >= p.n_insts) wide_feed_end(m.ctrl, wf);          // (else the CTA is aborting, and so is the issuer)
+    return at_feed_left(af);
 }
+
+__device__ void mk_feeder_landed(uint32_t left) { at_wait_landed(&smem_map().ctrl->attn, left); }
 
 // The issuer warp runs what the feeder tells it, in order.
 __device__ void mk_issuer(const Params& p) {

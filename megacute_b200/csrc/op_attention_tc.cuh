@@ -132,7 +132,18 @@ __device__ __forceinline__ int at_order(int t, int j, int both) { return j < bot
 struct AtFeed {
     uint32_t go = 0, granted = 0;        // parities of attn_go, ring_granted
     uint32_t insts = 0, tiles = 0;       // instructions and K (V) tiles requested
+    uint32_t q = 0, k = 0, v = 0;        // (lane 0) phases armed
 };
+// Lane 0: parities of the phases last armed, as in armed_parities: q, k (2 bits), v (2 bits).
+__device__ __forceinline__ uint32_t at_feed_left(const AtFeed& f) {
+    return ((f.q & 1u) ^ 1u) | armed_parities(2, f.k & 1u, (f.k >> 1) & 1u) << 1 | armed_parities(2, f.v & 1u, (f.v >> 1) & 1u) << 3;
+}
+// Abort path: tiles requested and not yet landed
+__device__ __forceinline__ void at_wait_landed(AttnBars* a, uint32_t left) {
+    wait_landed(&a->q_full, 1, left);
+    wait_landed(a->k_full, 2, left >> 1);
+    wait_landed(a->v_full, 2, left >> 3);
+}
 // All lanes; lane 0 requests.  `first`: the CTA's previous instruction is not an attention of the same head_dim.  `told`: entry of
 // Ctrl::wide_info to use (shared with the tile GEMM).
 template <int D>
@@ -168,6 +179,7 @@ __device__ __forceinline__ bool at_feed(const Params& p, Ctrl* c, uint8_t* ring,
         if (ok) {
             const int qtiles = in.a2 * 256 + 128 < Sq ? 2 : 1, qrow = in.a0 * Sq + in.a2 * 256;
             mbar_arrive_expect_tx(&a->q_full, (uint32_t)(qtiles * M::kTile));
+            ++f.q;
             for (int t = 0; t < qtiles; ++t)
                 for (int s = 0; s < D / 64; ++s)
                     tma_load_2d_plain(ring + M::kQ + t * M::kTile + s * kTcTileBytes, tmaps, in.a1 * D + s * 64, qrow + t * 128, &a->q_full);
@@ -180,11 +192,13 @@ __device__ __forceinline__ bool at_feed(const Params& p, Ctrl* c, uint8_t* ring,
             ok = wait_barrier(p, c, &a->k_empty[u], ph ^ 1u, in.seq, WHERE_RING_EMPTY, 2) && check_phase(p, c, &a->k_full[u], ph, in.seq, WHERE_CHECK_ARM);
             if (!ok) break;
             mbar_arrive_expect_tx(&a->k_full[u], (uint32_t)M::kTile);
+            ++f.k;
             for (int s = 0; s < D / 64; ++s)
                 tma_load_2d_plain(ring + M::kK + u * M::kTile + s * kTcTileBytes, tmaps + 128, hk * D + s * 64, krow + j * 128, &a->k_full[u]);
             ok = wait_barrier(p, c, &a->v_empty[u], ph ^ 1u, in.seq, WHERE_RING_EMPTY, 2) && check_phase(p, c, &a->v_full[u], ph, in.seq, WHERE_CHECK_ARM);
             if (!ok) break;
             mbar_arrive_expect_tx(&a->v_full[u], (uint32_t)M::kTile);
+            ++f.v;
             for (int s = 0; s < D / 64; ++s)
                 tma_load_2d_plain(ring + M::kV + u * M::kTile + s * kTcTileBytes, tmaps + 256, hk * D + s * 64, krow + j * 128, &a->v_full[u]);
         }

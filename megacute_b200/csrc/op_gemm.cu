@@ -32,4 +32,5 @@ __device__ int mk_run_gemm(const Params& p, int idx, int slot) {
         },
         [] {});
 }
+__device__ void mk_gemm_landed() { wait_x_landed(smem_map().ctrl); }
 }  // namespace mk

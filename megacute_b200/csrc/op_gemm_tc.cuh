@@ -50,7 +50,8 @@ __device__ __forceinline__ void tc_finish_state(Ctrl* c, uint32_t uses, uint32_t
                                                 uint32_t xstages) {
     c->acc_uses = uses + 1;
     const uint32_t full = (uint32_t)nk / xstages, rem = (uint32_t)nk - full * xstages;
-    c->x_par = xpar0 ^ ((full & 1u) ? (1u << xstages) - 1u : 0u) ^ ((1u << rem) - 1u);
+    c->x_par = (uint16_t)(xpar0 ^ ((full & 1u) ? (1u << xstages) - 1u : 0u) ^ ((1u << rem) - 1u));
+    c->x_left[0] = c->x_left[1] = 0xff;
     const uint32_t pos = ws0 + (uint32_t)nk;               // one weight slot per k-tile
     c->w_slot = (uint8_t)(pos % kTcWSlots);
     c->w_phase = (uint8_t)((wph0 ^ (pos / kTcWSlots)) & 1u);
@@ -236,6 +237,17 @@ __device__ __forceinline__ void tc_store_rows(const mk_op_desc* op, const float*
     else tc_store_rows_o<DT_BF16>(op, stage, m0, rows, col0, n_out);
 }
 
+// Abort path: the activation tiles of an instruction that did not end have landed.  Stage s of lane s mod 2 was armed in this round if it
+// lies in front of the lane's next one, else in the round before (the one before the instruction: complete).
+static __device__ __noinline__ void wait_x_landed(Ctrl* c) {
+    for (int lane = 0; lane < 2; ++lane) {
+        const int left = c->x_left[lane], next = left & 15, stages = left & 32 ? kTcXHalfStages : kTcXStages;
+        if (left == 0xff) continue;
+        for (int s = lane; s < stages; s += 2)
+            wait_landed(&c->x_full[s], 1, (((uint32_t)c->x_par >> s) ^ ((uint32_t)left >> 4) ^ (s < next ? 1u : 0u)) & 1u);
+    }
+}
+
 // All compute threads call this after the instruction's dependencies are met.  Returns 0, or -1
 // when the CTA is aborting.
 __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* ring, uint8_t* work, const mk_op_desc* op, int a0,
@@ -296,6 +308,7 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
             s += 2;
             if (s >= xstages) { s -= xstages; round ^= 1u; }
         }
+        c->x_left[lane] = (uint8_t)(s | round << 4 | (xstages == kTcXHalfStages ? 32u : 0u));
     } else if ((warp == 3 || warp == 1) && lane == 0) {
         // ---- MMAs: accumulator[128 activation rows][128 weight rows] += x tile . w tile^T ----
         // Two issuing threads, each with an accumulator of its own (columns 128 i ..): this one takes the
@@ -391,8 +404,8 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
     }
     tc_fence_before();
     const bool aborting = compute_sync_or(!ok || *(volatile int*)&c->abort);
+    if (aborting) return -1;                                            // (x_par and x_left stay: wait_x_landed)
     if (t == 0) tc_finish_state(c, uses, xpar0, ws0, wph0, nk, xstages);
-    if (aborting) return -1;
     return 0;
 }
 

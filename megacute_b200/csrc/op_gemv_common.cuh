@@ -175,9 +175,21 @@ struct StageCursor {
     }
 };
 
+// What the ring's memory serves.
+enum { MODE_STAGES = 0, MODE_WTILES = 1, MODE_KVTILES = 2, MODE_ATTN = 3, MODE_WWIDE = 4 };     // (MODE_WWIDE + kind: 256-row tiles)
+
+// Copies in flight when the producer leaves its loop in a mode, with its next slot (out of line: once per launch).
+static __device__ __noinline__ uint32_t producer_left(Ctrl* c, int mode, int slot, uint32_t phase) {
+    if (mode == MODE_ATTN) return 0;
+    const int n = mode == MODE_STAGES ? kStages : mode == MODE_WTILES ? kTcWSlots : mode == MODE_KVTILES ? kKvSlots : wide_stages(mode - MODE_WWIDE);
+    const unsigned long long* first = mode == MODE_STAGES ? c->full : mode == MODE_WTILES ? c->w_full : mode == MODE_KVTILES ? c->kv_full : c->ww_full[mode - MODE_WWIDE];
+    return copies_left(c, first, n, armed_parities(n, slot, phase));
+}
+
 // Producer warp main loop.  TRACE: role-0 records (seq, first stage issued, -, last stage issued).
+// Returns the copies left in flight, should the CTA be aborting (lane 0's value: see copies_left).
 template <bool TRACE>
-__device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t* ring) {
+__device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint8_t* ring) {
     const int lane = threadIdx.x & 31;
     RingPos pos;
     StageCursor rc, pc;
@@ -197,7 +209,6 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
     uint32_t wphase = 0;
     int kvslot = 0;
     uint32_t kvphase = 0, kvgo = 0;
-    enum { MODE_STAGES = 0, MODE_WTILES = 1, MODE_KVTILES = 2, MODE_ATTN = 3, MODE_WWIDE = 4 };     // (MODE_WWIDE + kind: 256-row tiles)
     uint32_t returned = 0;                           // parity of ring_returned
     int wwslot[2] = {0, 0};
     uint32_t wwphase[2] = {0, 0}, wide_count = 0;    // (and instructions of those kinds streamed)
@@ -242,13 +253,13 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
     while (rc.valid(p)) {
         if (rc.attn) {
             // a run of tcgen05 attentions of head_dim 128: the ring's memory is theirs until the compute warps are through
-            if (!enter(MODE_ATTN)) return;
+            if (!enter(MODE_ATTN)) goto left;
             int ok = 1;
             if (lane == 0) {
                 mbar_arrive(&c->ring_granted);
                 ok = wait_barrier(p, c, &c->ring_returned, returned, rc.seq, WHERE_RING_EMPTY, 4) ? 1 : 0;
             }
-            if (!__shfl_sync(0xffffffffu, ok, 0)) return;
+            if (!__shfl_sync(0xffffffffu, ok, 0)) goto left;
             returned ^= 1u;
             for (rc.idx += gridDim.x; rc.idx < p.n_insts; rc.idx += gridDim.x) {       // past the run
                 const int opi = __ldg(p.insts + (long long)rc.idx * 4).x - 1;
@@ -262,11 +273,11 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
             // copies of four rows issued by four lanes at once; K and V tiles alternate.  The whole
             // instruction is streamed from this tight loop: measured, a single lane that issued every
             // copy and walked the outer loop per slot spent ~950 cycles per 16 KB slot (32 GB/s).
-            if (!enter(MODE_KVTILES)) return;
+            if (!enter(MODE_KVTILES)) goto left;
             if (rc.kv_gated) {                        // unfused form: the appended row is readable once the dependencies are met
                 int go = 1;
                 if (lane == 0) go = wait_barrier(p, c, &c->kv_go, kvgo, rc.seq, WHERE_DEP) ? 1 : 0;
-                if (!__shfl_sync(0xffffffffu, go, 0)) return;
+                if (!__shfl_sync(0xffffffffu, go, 0)) goto left;
                 kvgo ^= 1u;
             }
             const int g = lane & 3;
@@ -285,7 +296,7 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
                         if (ok && !check_phase(p, c, &c->kv_full[kvslot], kvphase, rc.seq, WHERE_CHECK_ARM)) ok = 0;
                         if (ok) mbar_arrive_expect_tx(&c->kv_full[kvslot], tile_bytes);
                     }
-                    if (!__shfl_sync(0xffffffffu, ok, 0)) return;      // (also: the expected bytes are registered before any copy is issued)
+                    if (!__shfl_sync(0xffffffffu, ok, 0)) goto left;   // (also: the expected bytes are registered before any copy is issued)
                     if (lane < kKvTileRows / kKvGroupRows)
                         bulk_g2s_hint(dst + kvslot * kKvSlotBytes, src[w], group_bytes, &c->kv_full[kvslot], stream_policy);
                     src[w] += step[w];
@@ -301,7 +312,7 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
             // in the packed array) fill one slot of its kind; its barrier is armed a second time by the feeder warp, for the activations.
             // One lane: a k-tile's MMAs take 0.58 us, the lane's wait / expect / copy sequence 0.2.
             const int kind = rc.wide == 2 ? 0 : 1, stages = wide_stages(kind);
-            if (!enter(MODE_WWIDE + kind)) return;
+            if (!enter(MODE_WWIDE + kind)) goto left;
             const int nkt = rc.nk;
             const uint32_t wbytes = (uint32_t)wide_wbytes(kind);
             unsigned long long* full = c->ww_full[kind];
@@ -327,12 +338,13 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
                     }
                     if (++sl == stages) { sl = 0; ph ^= 1u; }
                 }
+                if (!ok) { wwslot[kind] = sl; wwphase[kind] = ph; }
             }
+            if (!__shfl_sync(0xffffffffu, ok, 0)) goto left;
             const uint32_t wpos = (uint32_t)wwslot[kind] + (uint32_t)nkt;
             wwslot[kind] = (int)(wpos % stages);
             wwphase[kind] ^= (wpos / stages) & 1u;
             ++wide_count;
-            if (!__shfl_sync(0xffffffffu, ok, 0)) return;
             rc.idx += gridDim.x;
             rc.seek(p);
             continue;
@@ -346,14 +358,14 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
             // copy sequence takes ~0.2 us (measured: 16 KB copies from one thread top out at 68 GB/s
             // however many are in flight), more than the MMAs of a tile; walking the outer loop (cursor,
             // warp votes) once per tile cost ~950 cycles.
-            if (!enter(MODE_WTILES)) return;
+            if (!enter(MODE_WTILES)) goto left;
             constexpr int kLanes = 4;
             const unsigned long long wpol = rc.reread ? keep_policy : stream_policy;
             bool mine = true;
+            uint32_t sl = (uint32_t)wslot + lane, ph = wphase;
             if (lane < kLanes) {
                 const uint8_t* src = rc.wpack ? rc.wpack + rc.wtile0 * (long long)kTcTileBytes : nullptr;
                 const long long kstep = (long long)rc.wstride * kTcTileBytes;
-                uint32_t sl = (uint32_t)wslot + lane, ph = wphase;
                 if (sl >= kTcWSlots) { sl -= kTcWSlots; ph ^= 1u; }
 #pragma unroll 1
                 for (int kt = lane; kt < rc.nk; kt += kLanes) {
@@ -368,15 +380,18 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
                 }
             }
             const bool ok = __all_sync(0xffffffffu, mine);
+            if (!ok) {                                       // (each lane knows the slots that it fills)
+                const uint32_t armed = __reduce_or_sync(0xffffffffu, lane < kLanes ? armed_parities(kTcWSlots, (int)sl, ph) & (0x11u << (sl % kLanes)) : 0u);
+                return copies_left(c, c->w_full, kTcWSlots, armed);
+            }
             const uint32_t wpos = (uint32_t)wslot + (uint32_t)rc.nk;
             wslot = (int)(wpos % kTcWSlots);
             wphase ^= (wpos / kTcWSlots) & 1u;
-            if (!ok) return;
             rc.idx += gridDim.x;
             rc.seek(p);
             continue;
         }
-        if (!enter(MODE_STAGES)) return;
+        if (!enter(MODE_STAGES)) goto left;
         // one lane looks whether the ring has a free stage (non-blocking)
         int free_now = 0;
         if (lane == 0) free_now = mbar_try_wait(&c->empty[pos.stage], pos.phase ^ 1u) ? 1 : 0;
@@ -394,12 +409,12 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
         if (!free_now) {
             int ok = 1;
             if (lane == 0) ok = wait_barrier(p, c, &c->empty[pos.stage], pos.phase ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
-            if (!__shfl_sync(0xffffffffu, ok, 0)) return;
+            if (!__shfl_sync(0xffffffffu, ok, 0)) goto left;
         }
         const __nv_bfloat16* src; int bytes, off;
         rc.piece(lane, src, bytes, off);
         const int total = __reduce_add_sync(0xffffffffu, bytes);
-        if (!check_phase_warp(p, c, &c->full[pos.stage], pos.phase, rc.seq, WHERE_CHECK_ARM)) return;
+        if (!check_phase_warp(p, c, &c->full[pos.stage], pos.phase, rc.seq, WHERE_CHECK_ARM)) goto left;
         if (lane == 0) mbar_arrive_expect_tx(&c->full[pos.stage], (uint32_t)total);
         __syncwarp();
         if (bytes) bulk_g2s_hint(ring + pos.stage * kStageBytes + off, src, (uint32_t)bytes, &c->full[pos.stage], stream_policy);
@@ -410,6 +425,15 @@ __device__ __forceinline__ void producer_loop(const Params& p, Ctrl* c, uint8_t*
         rc.advance(p);
         if (ahead > 0) --ahead;
     }
+left:
+    // (the kinds before the current one have been drained; lane 0 is the one that counts what a failing 256-row tile had requested)
+    int slot = pos.stage;
+    uint32_t phase = pos.phase;
+    if (mode == MODE_WTILES) { slot = wslot; phase = wphase; }
+    else if (mode == MODE_KVTILES) { slot = kvslot; phase = kvphase; }
+    else if (mode == MODE_WWIDE) { slot = wwslot[0]; phase = wwphase[0]; }
+    else if (mode == MODE_WWIDE + 1) { slot = wwslot[1]; phase = wwphase[1]; }
+    return producer_left(c, mode, slot, phase);
 }
 
 }  // namespace mk

@@ -24,6 +24,8 @@ __device__ int mk_op_gemv_general(const Params& p, const mk_op_desc* op, int o0,
 // arrivals of each itself (begin_op says why).  Returns the index of the last instruction executed, -1 when the CTA is
 // aborting.  (The ring position is untouched: the weight tiles have slots of their own.)
 __device__ int mk_run_gemm(const Params& p, int idx, int slot);
+// (abort path: its activation tiles still in flight have landed)
+__device__ void mk_gemm_landed();
 // (the same with output tiles of 256 rows; only for ops the host library bound to the tcgen05 body)
 __device__ int mk_run_gemm_wide(const Params& p, int idx, int slot);
 // body of the issuer warp: the MMAs of every tile GEMM with 256-row tiles and of every tcgen05 attention, until the feeder warp says that the list has ended
@@ -32,8 +34,11 @@ __device__ void mk_op_attention(const mk_op_desc* op, int a0, int a1, int a2);
 // (the tcgen05 body, for ops the host library attached tensor maps to: like mk_run_gemm, for runs of one head_dim)
 __device__ int mk_run_attention(const Params& p, const mk_op_desc* op, int idx, int slot);
 // body of the feeder warp: walks the CTA's instruction list and requests the tiles of every prefill attention bound to the
-// tcgen05 body and the activation tiles of every tile GEMM with 256-row tiles; runs until the list ends or the CTA aborts
-__device__ void mk_feeder(const Params& p);
+// tcgen05 body and the activation tiles of every tile GEMM with 256-row tiles; runs until the list ends or the CTA aborts.
+// Returns what mk_feeder_landed, on the abort path, waits for: the attention's tiles still in flight.  (Half a stage of a 256-row tile,
+// requested without the weights' half, cannot be waited for: the pause behind it covers that.)
+__device__ uint32_t mk_feeder(const Params& p);
+__device__ void mk_feeder_landed(uint32_t left);
 // (waits for its own dependencies and publishes its own arrivals; returns whether the CTA is aborting)
 __device__ bool mk_op_decode_attn(const Params& p, const mk_op_desc* op, int a0, int a1, int a2, int nwait, int wait_off,
                                   int seq, int narrive, int arrive_off);

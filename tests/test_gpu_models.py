@@ -125,6 +125,50 @@ def test_tile_linear_timeout_is_reported_not_hung(cuda):
     assert rel_l2(again, good) < 1e-3
 
 
+def test_timeout_anywhere_in_a_program_ends_the_launch(cuda, monkeypatch):
+    """A wait that cannot end, at the first waiting instruction of every op in turn: 128- and 256-row tiles, prefill attention of both
+    head sizes, norms, pointwise ops, a streaming linear.  Whatever the loading roles have requested by then, the launch ends, and the
+    program gives the same result once the wait is put right."""
+    from megacute_b200 import _lib, passes
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 256) if a[1] % 512 == 0 else (1, 128, 128))
+    monkeypatch.setattr(passes, "hoist_linears", lambda g: g)
+    S, E = 1024, 512
+    g = mc.Graph()
+    x, t = g.input("x", (S, E)), {"x": rnd((S, E), 1.0, 1)}
+
+    def w(rows, cols):
+        name = f"w{len(t)}"
+        t[name] = rnd((rows, cols), cols ** -0.5, len(t))
+        return g.param(name, (rows, cols))
+
+    for D in (64, 128):
+        qkv = g.linear(g.rms_norm(x), w(3 * E, E))
+        a = g.attention(*(qkv.cols_slice(i * E, E) for i in range(3)), batch=1, heads=E // D, head_dim=D, causal=True)
+        x = g.add(g.linear(g.unary(g.linear(a, w(E + 128, E)), "silu"), w(E, E + 128)), x)
+    g.output(x, g.linear(x.rows_slice(S - 1, 1), w(2048, E)))
+    prog = mc.compile(g)
+    dev = {k: v.to(cuda) for k, v in t.items()}
+    want = [o.clone() for o in prog(**dev)]
+    prog.check()
+    assert prog.tcgen05_attention_ops == 2 and {o.bm or 128 for o in prog.g.ops if o.kind == "Linear" and o.x.rows > 8} == {128, 256}
+    s, lib = prog.sched, _lib.load()
+    prog.set_timeout(0.02)
+    for k, (i0, i1) in enumerate(s.node_ranges):
+        i = next((i for i in range(i0, i1) if s.wait_ptr[i + 1] > s.wait_ptr[i]), None)
+        if i is None:
+            continue
+        at = int(s.wait_ptr[i])
+        _lib.check(lib.mk_program_poke_wait(prog._handle, at, int(s.wait_cnt[at]), 1000))
+        prog(**dev)
+        with pytest.raises(_lib.MegakernelTimeout):
+            prog.check()
+        _lib.check(lib.mk_program_poke_wait(prog._handle, at, int(s.wait_cnt[at]), int(s.wait_tgt[at])))
+        prog.reset()
+        outs = prog(**dev)
+        prog.check()
+        assert all(torch.equal(o, r) for o, r in zip(outs, want)), prog.g.ops[k].kind
+
+
 def test_streaming_and_tile_linears_alternate(cuda):
     """Streaming linears (<= 8 rows: two-stage weight ring) and tcgen05 tile linears (eight single-tile
     weight slots in the same shared memory) alternate in one launch, several instructions of each
