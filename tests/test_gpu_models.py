@@ -225,8 +225,6 @@ def test_mlp_block_config(cuda):
 ])
 @pytest.mark.parametrize("body", ["mma.sync", "tcgen05"])
 def test_prefill_attention(cuda, monkeypatch, B, Sq, Sk, H, KVH, D, causal, body):
-    if body == "tcgen05" and D != 64:
-        pytest.skip("the tcgen05 body takes head_dim 64")
     monkeypatch.setenv("MEGACUTE_B200_ATTN_TCGEN05", "1" if body == "tcgen05" else "0")     # (the default is the tcgen05 body)
     g = mc.Graph()
     q = g.input("q", (B * Sq, H * D))
@@ -510,8 +508,8 @@ def test_fused_step_feeds_itself(cuda, B, vocab):
     (1100, 512, 1280, None, False, False),
 ])
 def test_tile_linear_wide_tiles(cuda, monkeypatch, M, K, N, act, bias, res):
-    """128 x 256 output tiles (one activation k-tile feeds two weight tiles, two accumulator halves in tensor
-    memory): plain, swiglu and split-K epilogues, ragged last row tile, several tiles per CTA."""
+    """256 x 256 output tiles (two accumulators that fill tensor memory): plain, swiglu and split-K epilogues, ragged last
+    row tile.  (Several such tiles on a CTA: test_tiles.py::test_tile_kinds_follow_one_another_on_a_cta.)"""
     monkeypatch.setenv("MEGACUTE_B200_WIDE_TILES", "1")
     g = mc.Graph()
     x = g.input("x", (M, K))

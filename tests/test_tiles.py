@@ -89,17 +89,92 @@ def test_rotated_heads(cuda, monkeypatch, B, S, D, tile, tcgen05):
     (1, 64, 300, 1, 1, 128, False), (2, 130, 130, 2, 1, 128, True), (1, 520, 520, 3, 1, 128, True), (1, 256, 1000, 2, 2, 128, False),
 ])
 def test_prefill_attention_tiles(cuda, B, Sq, Sk, H, KVH, D, causal):
-    """Odd numbers of query tiles and key blocks, one tile only, masked and ragged last blocks.  Two layers of the op: the CTA's
-    buffers do not start at their first phase."""
+    """Odd numbers of query tiles and key blocks, one tile only, masked and ragged last blocks.  (A CTA has one instruction at most
+    here; several of them: test_attention_instructions_follow_one_another_on_a_cta.)"""
     g = mc.Graph()
     q, k, v = g.input("q", (B * Sq, H * D)), g.input("k", (B * Sk, KVH * D)), g.input("v", (B * Sk, KVH * D))
     a = g.attention(q, k, v, batch=B, heads=H, kv_heads=KVH, head_dim=D, causal=causal)
     b = g.attention(a, k, v, batch=B, heads=H, kv_heads=KVH, head_dim=D, causal=causal)
     g.output(a, b)
     t = {"q": rnd((B * Sq, H * D), 2.0, 1), "k": rnd((B * Sk, KVH * D), 2.0, 2), "v": rnd((B * Sk, KVH * D), 1.0, 3)}
-    outs, ref, *_ = run_both(g, t, cuda, steps=2)
+    outs, ref, _, _, prog = run_both(g, t, cuda, steps=2)
+    assert prog.tcgen05_attention_ops == 2
     for x, y in zip(outs, ref):
         assert rel_l2(x, y) < TOL
+
+
+def rows_close(outs, ref):
+    """Every row on its own: a damaged tile or head does not hide in the norm of the whole tensor."""
+    for o, want in zip(outs, ref):
+        err = (o.float() - want).norm(dim=1) / want.norm(dim=1)
+        assert torch.isfinite(err).all() and float(err.max()) < TOL
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("first,second", [(64, 64), (128, 128), (64, 128), (128, 64)])
+def test_attention_instructions_follow_one_another_on_a_cta(cuda, monkeypatch, first, second):
+    """Two to four attention instructions per SM and op, so that barriers, K and V stages, score buffers and O change hands between
+    instructions, from one head size to the other, and with what else uses the ring and the work area: 256-row tiles, streaming
+    linears, 128-row tiles, norms of several rows per warp."""
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 256) if a[1] % 256 == 0 else (1, 128, 128))
+    monkeypatch.setattr(passes, "hoist_linears", lambda g: g)
+    B, S = 16, 350                                            # two instructions per (sequence, head), the second with 94 queries
+    g = mc.Graph()
+    x, x1 = g.input("x", (B * S, 256)), g.input("x1", (1, 256))
+    t = {"x": rnd((B * S, 256), 1.0, 1), "x1": rnd((1, 256), 1.0, 2)}
+
+    def w(rows, cols):
+        name = f"w{len(t)}"
+        # (q, k and v of standard deviation 1/2, scores of 1/4 and at most about 2: the roundings of q and k, 2^-9 each, move a softmax
+        # weight by less than 2^-7.  So no row collects more than a few 16-bit roundings per block, 3e-3 to 5e-3 over the three)
+        t[name] = rnd((rows, cols), 0.5 * cols ** -0.5, len(t))
+        return g.param(name, (rows, cols))
+
+    y = x
+    for n, D in enumerate((first, second, first)):
+        H, KVH = 1024 // D, 512 // D
+        qkv = g.linear(y, w(2048, 256))
+        q, k, v = qkv.cols_slice(0, 1024), qkv.cols_slice(1024, 512), qkv.cols_slice(1536, 512)
+        a = g.attention(q, k, v, batch=B, heads=H, kv_heads=KVH, head_dim=D, causal=n != 1)
+        b = g.attention(a, k, v, batch=B, heads=H, kv_heads=KVH, head_dim=D, causal=n == 1)
+        g.output(a, b, g.linear(x1, w(148 * 16, 256)))
+        y = g.rms_norm(g.linear(g.linear(b, w(1024 + 128, 1024)), w(256, 1024 + 128)))
+    g.output(y)
+    prog = mc.compile(g)
+    att = [e - s for o, (s, e) in zip(prog.g.ops, prog.sched.node_ranges) if o.kind == "Attention"]
+    assert len(att) == 6 and min(att) > 1.7 * prog.sm_count             # (head_dim 128: 256 instructions, 64: 512)
+    dev = {n: u.to(cuda) for n, u in t.items()}
+    ref, _ = evaluate(g, dev, cuda)
+    for _ in range(3):
+        rows_close(prog(**dev), ref)
+    prog.check()
+    assert prog.tcgen05_attention_ops == 6
+
+
+@pytest.mark.gpu
+def test_tile_kinds_follow_one_another_on_a_cta(cuda, monkeypatch):
+    """256 x 256, 256 x 128 and 128 x 128 tiles in turns, two and more of each per SM, with one k-tile and with more k-tiles than there
+    are stages: each kind divides the same memory in its own way, and loads and MMAs of the next tile run ahead."""
+    plans = {2560: (1, 256, 256), 2432: (1, 256, 128), 1280: (1, 128, 128)}
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: plans[a[1]])
+    monkeypatch.setattr(passes, "hoist_linears", lambda g: g)
+    M = 4001                                                  # (the last row tile: 161 rows)
+    g = mc.Graph()
+    x, t = g.input("x", (M, 576)), {"x": rnd((M, 576), 1.0, 1)}
+    xs = {64: x.cols_slice(0, 64), 576: x}
+    order = [(2560, 64), (2432, 64), (2560, 576), (2432, 576), (1280, 576), (2432, 64), (2432, 576), (1280, 64), (2560, 576), (2560, 64)]
+    for i, (N, K) in enumerate(order):
+        t[f"w{i}"], t[f"b{i}"] = rnd((N, K), K ** -0.5, 10 + i), rnd((1, N), 0.5, 30 + i)
+        g.output(g.linear(xs[K], g.param(f"w{i}", (N, K)), bias=g.param(f"b{i}", (1, N)), act="relu" if i % 3 else None))
+    prog = mc.compile(g)
+    assert all((o.bm or 128, o.bn or 128) == plans[N][1:] for o, (N, _) in zip(prog.g.ops, order))
+    assert [e - s for s, e in prog.sched.node_ranges][:2] == [160, 304]
+    dev = {n: u.to(cuda) for n, u in t.items()}
+    ref, _ = evaluate(g, dev, cuda)
+    for _ in range(5):
+        rows_close(prog(**dev), ref)
+    prog.check()
+    assert prog.tcgen05_ops == len(order)
 
 
 @pytest.mark.gpu
@@ -187,9 +262,6 @@ def test_ring_changes_hands_behind_256_row_tiles(cuda, monkeypatch):
     dev = {k: w.to(cuda) for k, w in t.items()}
     ref, _ = evaluate(g, dev, cuda)
     for _ in range(10):
-        for o, want in zip(prog(**dev), ref):
-            # every output row on its own: a damaged tile does not hide in the whole tensor
-            err = (o.float() - want).norm(dim=1) / want.norm(dim=1)
-            assert float(err.max()) < TOL
+        rows_close(prog(**dev), ref)
     prog.check()
     assert sum(o.kind == "Linear" and o.bm == 256 for o in prog.g.ops) == 9
