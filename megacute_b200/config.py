@@ -33,10 +33,10 @@ REDUCE_GBPS, FINALIZE_US = 2000.0, 8.0       # a K-split op: bytes of its fp32 r
 EW_ROWS, EW_COLS = 32, 512
 FINALIZE_MIN_ROWS, FINALIZE_MIN_INSTS = 4, 96     # SplitFinalize: shorter tiles until the op has this many instructions
 # rows per norm instruction: a multiple of NORM_ROWS (a row per warp) up to NORM_MAX_ROWS; 1 when the op has few rows.
-# Both kinds of streaming op aim at STREAM_INSTS instructions, one per SM: what an instruction costs whatever its size
+# Both kinds of streaming op aim at one instruction per SM: what an instruction costs whatever its size
 # (dependency wait, arrival, first L2 round trip, ~3 us) is as long as streaming 100 KB
 NORM_ROWS, NORM_MAX_ROWS = COMPUTE_WARPS, 64
-EW_MIN_ROWS, EW_MAX_ROWS, STREAM_INSTS = 4, 128, 148
+EW_MIN_ROWS, EW_MAX_ROWS = 4, 128
 WIDE_NORM_ROWS = 256
 ROPE_APPEND_ROWS = COMPUTE_WARPS
 ATTN_BQ, ATTN_BK = 256, 64          # queries per prefill attention instruction (two tiles of 128), keys per tile of the mma.sync body

@@ -5,7 +5,7 @@ parameters are Python constants traced into the JIT kernel by the node classes
 (``megacute/ops/*.py`` ``__init__`` / ``host``).  Here the kernel is compiled once, ahead of time,
 and reads shapes, strides, flags and operand addresses from this table at run time.
 
-``fill(desc, op, addr)`` writes the fields; ``addr(view)`` returns the device byte address of the
+``fill(desc, op, addr, sm_count)`` writes the fields; ``addr(view)`` returns the device byte address of the
 view's first element.  Field meaning per kind (the kernel side repeats it next to the reader):
 
   GEMV         ptr x, w, out, bias, residual, norm gain; i M, N_out, K, act, x dtype, out dtype,
@@ -93,8 +93,8 @@ def gemv_units(op: Op) -> bool:
     return op.x.cols % 16 == 0
 
 
-def fill(d, op: Op, addr) -> None:
-    """Write op's descriptor into ``d`` (an ``_lib.OpDesc``)."""
+def fill(d, op: Op, addr, sm_count: int) -> None:
+    """Write op's descriptor, as scheduled for ``sm_count`` SMs, into ``d`` (an ``_lib.OpDesc``)."""
     ptrs: list = []
     ints: list = []
     d.flags = 0
@@ -138,11 +138,11 @@ def fill(d, op: Op, addr) -> None:
             ptrs, ints = [op.x, op.scale, op.shift, op.out], [R, Cc, C.EW_MODULATE, 0, op.group, 0]
         else:
             ptrs, ints = [op.x, op.cos, op.sin, op.out], [R, Cc, C.EW_ROPE, 0, op.seq, op.head_dim]
-        ints += [dt(v) for v in ptrs] + [ew_rows(R, Cc)]
+        ints += [dt(v) for v in ptrs] + [ew_rows(R, Cc, sm_count)]
     elif k == "Norm":
         d.kind = C.OP_NORM
         ptrs = [op.x, op.out, op.weight, op.bias, op.scale, op.shift]
-        ints = [op.x.rows, op.x.cols, int(bool(op.rms)), norm_rows(op.x.rows, op.scale is not None), dt(op.x), dt(op.out),
+        ints = [op.x.rows, op.x.cols, int(bool(op.rms)), norm_rows(op.x.rows, op.scale is not None, sm_count), dt(op.x), dt(op.out),
                 int(op.group or 1), dt(op.scale), dt(op.shift)]
         d.f[0] = float(op.eps)
     elif k == "Attention":

@@ -169,7 +169,7 @@ class Program:
             moved = {i for i, a in ptrs.items() if old[0].get(i) != a}
             todo = sorted({k for i in moved for k in self._ops_of_buf.get(i, ())})
         for k in todo:
-            encode.fill(self._desc[k], self.g.ops[k], self._addr)
+            encode.fill(self._desc[k], self.g.ops[k], self._addr, self.sm_count)
         _lib.check(_lib.load().mk_program_set_ops(self._handle, ctypes.addressof(self._desc), len(self.g.ops), stream),
                    "mk_program_set_ops")
         self._desc_key = (ptrs, vers)
@@ -201,7 +201,8 @@ class Program:
 
     @property
     def tcgen05_attention_ops(self) -> int:
-        """Prefill attention ops bound to the tcgen05 body at the last launch (head_dim 64)."""
+        """Prefill attention ops bound to the tcgen05 body at the last launch (head_dim 64 or 128, operands
+        that tensor maps can describe, a positive scale; the rest run the mma.sync body)."""
         return int(_lib.load().mk_program_tcgen05_attention_ops(self._handle)) if self._handle is not None else 0
 
     @property

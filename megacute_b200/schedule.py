@@ -170,7 +170,7 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
         if k == "SplitFinalize":
             TR = finalize_rows(R, Cc)
         else:
-            TR = ew_rows(R, Cc)
+            TR = ew_rows(R, Cc, sm_count)
         if k == "Rope":
             assert TC % op.head_dim == 0, "rope: head_dim must divide the pointwise tile width"
         rt, ct = np.divmod(np.arange(_ceil(R, TR) * _ceil(Cc, TC)), _ceil(Cc, TC))
@@ -199,7 +199,7 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
         return Tiled(_args(n, rt, ct), [a for a in acc if a is not None])
     if k == "Norm":
         R = op.x.rows
-        rows = norm_rows(R, op.scale is not None)
+        rows = norm_rows(R, op.scale is not None, sm_count)
         rt = np.arange(_ceil(R, rows))
         n = len(rt)
         acc = [_acc(op.x, READ, rt * rows, (rt + 1) * rows, n=n), _acc(op.weight, READ, n=n), _acc(op.bias, READ, n=n),
@@ -299,24 +299,24 @@ def finalize_rows(rows: int, cols: int) -> int:
     return tr
 
 
-def norm_rows(rows: int, modulated: bool = False) -> int:
+def norm_rows(rows: int, modulated: bool, sm_count: int) -> int:
     """Rows per norm instruction: a single row spread over the whole CTA when the op has few rows (decode),
     else a multiple of the compute warps that gives each SM about one instruction.  Modulated rows (a DiT block's): 16, 32 or 64, so
     that an instruction waits for one 256-row tile of the linear before it and its rows share a scale and shift row
     (56 -> 64 rows at 32 images, 24 -> 32 at 12: 0.4 and 1.6 % of the step)."""
     if rows <= C.WIDE_NORM_ROWS:
         return 1
-    per = max(1, min(C.NORM_MAX_ROWS // C.NORM_ROWS, _ceil(_ceil(rows, C.NORM_ROWS), C.STREAM_INSTS)))
+    per = max(1, min(C.NORM_MAX_ROWS // C.NORM_ROWS, _ceil(_ceil(rows, C.NORM_ROWS), sm_count)))
     if modulated and per > 2:
         per = 4 if per <= 4 else 8
     return C.NORM_ROWS * per
 
 
-def ew_rows(rows: int, cols: int) -> int:
+def ew_rows(rows: int, cols: int, sm_count: int) -> int:
     """Rows per pointwise instruction: the smallest power of two that leaves the op about one instruction
     per SM, within EW_MIN_ROWS .. EW_MAX_ROWS."""
     tr, ct = C.EW_MIN_ROWS, _ceil(cols, C.EW_COLS)
-    while tr < C.EW_MAX_ROWS and _ceil(rows, tr) * ct > C.STREAM_INSTS:
+    while tr < C.EW_MAX_ROWS and _ceil(rows, tr) * ct > sm_count:
         tr *= 2
     return tr
 

@@ -404,3 +404,19 @@ def test_ragged_positions_and_window_semantics():
         sc = torch.einsum("kgd,skd->kgs", qq, k) * D ** -0.5
         want = torch.einsum("kgs,skd->kgd", torch.softmax(sc, -1), v).reshape(1, H * D)
         assert rel_l2(got[0][b:b + 1], want) < 1e-5
+
+
+@pytest.mark.parametrize("sms", [148, 64])
+def test_rows_per_streaming_instruction_follow_the_sm_count(sms):
+    """Norms and pointwise ops of many rows: about one instruction per SM that the program is compiled for, the same number of rows in
+    the schedule and in the descriptor."""
+    from megacute_b200 import _lib, encode
+    g = mc.Graph()
+    x = g.input("x", (2048, 512))
+    g.output(g.unary(g.rms_norm(x), "relu"))
+    s = schedule(g, sms)
+    check_tables(g, s)
+    for op, (a, b), field in zip(g.ops, s.node_ranges, (3, 10)):
+        d = _lib.OpDesc()
+        encode.fill(d, op, lambda v: 0, sms)
+        assert sms // 2 < b - a <= sms and -(-2048 // d.i[field]) == b - a
