@@ -136,10 +136,11 @@ int mk_program_reset(mk_program* p, void* stream);
 /* Debug / test access to runtime-owned tables (synchronise the stream first). */
 int mk_program_epoch(mk_program* p);
 /* How many tile-GEMM ops of the last mk_program_set_ops() run on the tcgen05 tensor cores with
- * bulk-tensor-copied operands (the others, if any, run the mma.sync body: K range per instruction
- * not a multiple of 64, unaligned operands, or MEGACUTE_B200_NO_TCGEN05 set). */
+ * bulk-tensor-copied operands (the others, if any, run the mma.sync body: K not a multiple
+ * of 64, unaligned operands, or MEGACUTE_B200_NO_TCGEN05 set). */
 int mk_program_tcgen05_ops(mk_program* p);
-/* ... and how many prefill attention ops (head_dim 64; the others run the mma.sync body). */
+/* ... and how many prefill attention ops (head_dim 64 or 128, operands that tensor maps can describe, a positive
+ * scale; the others run the mma.sync body). */
 int mk_program_tcgen05_attention_ops(mk_program* p);
 /* Device memory the program holds for tile-image copies of the weights of those ops (made by
  * mk_program_set_ops unless MEGACUTE_B200_NO_WEIGHT_PACK is set, when a weight matrix is bound

@@ -24,7 +24,8 @@ MIN_SPLIT_KTILES = 8            # k-tiles (of GEMM_BK) per K split
 MAX_K_SPLITS = 8
 INST_US, SM_GBPS = 2.0, 40.0    # split-K cost model: fixed us per instruction, GB/s one SM draws from HBM
 # output tiles of a tile linear: 128 x 128, and for ops with more than WIDE_MIN_ROWS rows 256 x 128 and 256 x 256; cost
-# model (us, from the kernel's timeline with every SM streaming): per tile, per 64-element k-tile, once per op
+# model (us, fitted to the times of measured plans): per tile, per 64-element k-tile, once per op.  (In a long run at the power
+# cap a k-tile takes 0.26 - 0.30, 0.50 - 0.56 and 0.76 - 0.84: the same ratios)
 GEMM_BM_WIDE, GEMM_BN_WIDE, WIDE_MIN_ROWS = 256, 256, 128
 GEMM_COST_US = {(128, 128): (6.0, 0.28, 0.0), (256, 128): (2.5, 0.45, 4.0), (256, 256): (2.0, 0.70, 4.0)}
 REDUCE_GBPS, FINALIZE_US = 2000.0, 8.0       # a K-split op: bytes of its fp32 reduce-adds; the SplitFinalize hop behind it

@@ -4,7 +4,8 @@
 // S = Q K^T and O += P V are warp-level mma.sync m16n8k16 bf16 -> fp32 with the online softmax
 // kept in registers in the log2 domain; P is rounded to bf16 before P V (as the reference's
 // kernel does, megacute/ops/attention.py:293).  A fully masked row yields 0.  Runs what the tcgen05
-// body (op_attention_tc.cuh) does not take: other head_dims, operands its tensor maps cannot describe.
+// body (op_attention_tc.cuh) does not take: operands its tensor maps cannot describe, a scale that is not positive, launches without
+// tensor maps (mk_launch_noalloc).
 //
 // ptr 0 q, 1 k, 2 v, 3 out; i 0 batch, 1 seq_q, 2 seq_k, 3 heads, 4 kv_heads, 5 head_dim,
 // 6 causal, 7 out dtype (DT_BF16 or DT_F16), 8 dtype of q, k and v (DT_BF16 or DT_F16); f 0 scale.  args: 0 b, 1 h, 2 query tile pair.

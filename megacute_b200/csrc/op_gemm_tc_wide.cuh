@@ -2,7 +2,7 @@
 //
 // What bounds a tile GEMM whose operands live in L2 is the bytes an SM draws from there: measured on B200 (all 148 SMs,
 // stand-alone loop) a 128 x 256 tile takes 0.46 us per 64-element k-tile of 48 KB (104 GB/s per SM) where its MMAs take
-// 0.29; a 256 x 256 tile needs 64 KB for twice the flops and takes 0.82, 11 % less per flop, and a single thread that
+// 0.29; a 256 x 256 tile needs 64 KB for twice the flops, and a single thread that
 // issues four N = 256 instructions per commit keeps the tensor pipe full (2.15 PFLOP/s with the operands in place).  So
 // one instruction is a 256 x 256 tile: two 128 x 256 accumulators (rows 0..127 and 128..255: all 512 columns of tensor
 // memory), three stages of 64 KB, and four roles that run ahead of one another across instruction boundaries:
@@ -11,14 +11,17 @@
 //                256 rows x 64 columns per k-tile; rows beyond M are zero-filled
 //   MMA          issuer warp, one thread (wide_issue): waits for a stage (armed once by each loader), 4 + 4 instructions, one commit.
 //                It is told what to run by the feeder through Ctrl::wide_info and never touches global memory.
-//   epilogue     the compute warps: warp w owns rows 32 (w & 3) .. +31 of accumulator w >> 2; it reads its 32 x 256 part, hands
-//                the accumulator back and writes the rows from registers while the next tile's main loop runs
-// Tiles of 256 x 128 (kind 1; kind 0: 256 x 256) have four stages of 48 KB and half the accumulator columns.  They cost 0.45 us per
-// k-tile where half a 256 x 256 tile costs 0.36 -- 128-column instructions read as many operand bytes for half the flops, and
-// shared memory (128 bytes a cycle for the tensor core's reads and the copies' writes together) is what both are bound by --
-// and are chosen where they fill the SMs better (passes.plan_tiles).
-// The loads of the next tile therefore run through this one's epilogue, and its MMAs start as soon as the accumulators have
-// been read.  (With one role after the other per instruction, 128 x 256 tiles: prefill gate/up 20.5 us per 128 x 256 x 2048
+//   epilogue     the compute warps: warp w owns rows 32 (w & 3) .. +31 of accumulator w >> 2; it reads its 32 x 256 part in steps of
+//                32 columns, each written before the next is read, and hands the accumulator back with the last one
+// Tiles of 256 x 128 (kind 1; kind 0: 256 x 256) have four stages of 48 KB and half the accumulator columns.  Per k-tile, all SMs
+// streaming, four tiles per SM, K from 1024 to 8192: 256 x 256 0.76 - 0.84 us, 256 x 128 0.50 - 0.56 (half a 256 x 256 tile: 0.38 -
+// 0.42), 128 x 128 0.26 - 0.30 -- 128-column instructions read as many operand bytes for half the flops, and
+// shared memory (128 bytes a cycle for the tensor core's reads and the copies' writes together) is what both are bound by.
+// 256 x 128 is chosen where it fills the SMs better (passes.plan_tiles; its constants are fitted to measured plans, at the clocks
+// of a short launch).
+// The loads of the next tile therefore run through this one's epilogue, but only as far as there are stages: its MMAs wait for the
+// accumulators, and those are free after seven eighths (256 x 128: three quarters) of the epilogue's arithmetic and stores.
+// (With one role after the other per instruction, 128 x 256 tiles: prefill gate/up 20.5 us per 128 x 256 x 2048
 // block of which 13.8 were main loop; DiT gelu tiles 28 us of which 7.)
 // A run of such instructions on a CTA starts with the compute warps' arrival on gemm_go: the work area, where the
 // activation slots are, belongs to other bodies before it and after the run's last accumulator.

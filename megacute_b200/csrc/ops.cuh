@@ -3,7 +3,8 @@
 // unit with the kernel, ptxas' whole-program register allocation spills the inner loop of the
 // streaming linear to local memory (with 227 KB of the SM given to shared memory almost no L1 is
 // left, so each spill is an L2 round trip: 6x slower), however the calls are arranged.  Compiled
-// separately, each body gets its own allocation under the 168-register cap of a 9-warp CTA.
+// separately, each body gets its own allocation under a cap of 168 registers (12 warps of
+// 168 fill the SM's register file).
 //
 // All take the op descriptor and the instruction's arguments by value and find the CTA's shared
 // memory through the kernel's dynamic shared-memory window.

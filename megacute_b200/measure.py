@@ -14,7 +14,8 @@ driver, ``bench.py``):
   evenly over 256 .. 4096 tokens (a ragged batch: not possible in the reference)
 
 Synthetic bf16 inputs and weights of those shapes; each configuration is compiled once, warmed up
-twice, then timed over a few launches with CUDA events on the launching stream.  Prints one line
+twice, then timed over a few launches (20, 3 and 2 of the first three) with CUDA events on the launching stream: the clocks of a
+short region (a DiT launch takes 7.6 ms there and 8.4 at the power cap, after some hundred).  Prints one line
 per configuration: time per launch and TFLOP/s against the configuration's algorithmic flops.
 """
 
