@@ -309,7 +309,6 @@ struct mk_program {
     unsigned long long timeout_ns = 2000000000ull;
     int tcgen05_ops = 0;             // tile GEMMs bound to the tcgen05 body by the last set_ops
     int tcgen05_attn_ops = 0;        // ... prefill attention ops
-    int pf_stages = 0;               // L2 prefetch distance of the producer warp, in ring stages (0 = off)
 };
 
 static const size_t kMapBytes = 512;       // tensor-map space per op
@@ -599,7 +598,6 @@ int mk_program_create(int device, const int32_t* insts, int n_insts, const int32
     MK_TRY(cudaFuncSetAttribute(mk::megakernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mk::kSmemBytes));
     MK_TRY(cudaFuncSetAttribute(mk::megakernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mk::kSmemBytes));
 #undef MK_TRY
-    if (const char* e = getenv("MEGACUTE_B200_PF_STAGES")) p->pf_stages = atoi(e);
     *out = p;
     return MK_OK;
 }
@@ -765,7 +763,6 @@ int mk_launch(mk_program* p, void* stream) {
     prm.status = p->d_status;
     prm.epoch = p->epoch;
     prm.timeout_ns = p->timeout_ns;
-    prm.pf_stages = p->pf_stages;
     if (p->trace_cap > 0) mk::megakernel<true><<<p->grid, mk::kThreads, mk::kSmemBytes, st>>>(prm);
     else mk::megakernel<false><<<p->grid, mk::kThreads, mk::kSmemBytes, st>>>(prm);
     MK_CUDA(cudaGetLastError());
@@ -929,7 +926,6 @@ extern "C" int mk_launch_noalloc(int device, const int32_t* d_insts, int n_insts
     prm.status = d_status;
     prm.epoch = 1;
     prm.timeout_ns = 2000000000ull;
-    prm.pf_stages = 0;
     mk::megakernel<false><<<grid, mk::kThreads, mk::kSmemBytes, st>>>(prm);
     MK_CUDA(cudaGetLastError());
     if (status) {

@@ -112,7 +112,6 @@ struct Params {
     int* status;                  // MK_ST_WORDS words; word 0 != 0 aborts every waiter
     int epoch;
     unsigned long long timeout_ns;
-    int pf_stages;                // how many ring stages ahead of the ring the producer prefetches into L2
 };
 
 // a tile GEMM bound to the tcgen05 body with 256-row tiles (op_gemm_tc_wide.cuh)
@@ -277,9 +276,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const void* tmap, int x, 
             smem_u32(dst)),
         "l"(tmap), "r"(x), "r"(y), "r"(smem_u32(bar)), "l"(policy)
         : "memory");
-}
-__device__ __forceinline__ void bulk_prefetch_l2(const void* src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void cp_async16(void* dst, const void* src, bool valid) {
     int sz = valid ? 16 : 0;      // src-size 0: the 16 bytes are zero-filled

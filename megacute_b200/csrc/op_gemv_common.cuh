@@ -51,10 +51,7 @@ __device__ __forceinline__ int gemv_weight_row(bool swi, int o0, int group, int 
 // ---- producer side -------------------------------------------------------------------------------
 // The producer warp sees this CTA's streaming linears as one long sequence of ring stages.  A
 // StageCursor names one stage of that sequence (instruction, row group, K segment) and yields,
-// per lane, the weight-row segment that lane copies.  Two cursors walk the sequence: one feeds the
-// shared-memory ring with bulk copies, the other runs up to Params::pf_stages stages further
-// ahead and only asks L2 to fetch the same bytes (cp.async.bulk.prefetch.L2), so HBM keeps
-// streaming while the ring is full and the compute warps sit in a dependency hop.
+// per lane, the weight-row segment that lane copies.
 struct StageCursor {
     int idx;                 // global instruction index (this CTA's: idx = cta + k * grid); >= n_insts: end
     int seq, g, seg;         // instruction sequence number, row group and K segment inside it
@@ -143,23 +140,16 @@ struct StageCursor {
         }
     }
     __device__ __forceinline__ bool valid(const Params& p) const { return idx < p.n_insts; }
-    __device__ __forceinline__ void advance(const Params& p) {
-        if (gemm || kv || attn) {                     // (the L2 prefetch cursor: whole instruction at once)
-            idx += gridDim.x;
-            seek(p);
-            return;
-        }
-        if (++seg < nseg) return;
+    // the next stage of a streaming linear: false behind its last one
+    __device__ __forceinline__ bool advance() {
+        if (++seg < nseg) return true;
         seg = 0;
-        if (++g < ngroups) return;
-        idx += gridDim.x;
-        seek(p);
+        return ++g < ngroups;
     }
     // this lane's piece of the stage: source, bytes (0 = none) and offset inside the ring stage
     __device__ __forceinline__ void piece(int lane, const __nv_bfloat16*& src, int& bytes, int& dst_off) const {
         const bool swi = flags & GEMV_F_SWIGLU;
         src = w; bytes = 0; dst_off = 0;
-        if (gemm || kv || attn) return;
         if (flags & GEMV_F_UNITS) {
             const int r = lane & 15;
             const int o = o0 + (swi ? g >> 1 : g) * 16 + r;
@@ -192,11 +182,8 @@ template <bool TRACE>
 __device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint8_t* ring) {
     const int lane = threadIdx.x & 31;
     RingPos pos;
-    StageCursor rc, pc;
+    StageCursor rc;
     rc.idx = blockIdx.x;
-    rc.seek(p);
-    pc = rc;
-    int ahead = 0;                                   // stages the prefetch cursor is ahead of the ring cursor
     long long t_first = 0;
     int slot_first = 0;
     const unsigned long long stream_policy = l2_policy_evict_first();
@@ -213,47 +200,47 @@ __device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint
     int wwslot[2] = {0, 0};
     uint32_t wwphase[2] = {0, 0}, wide_count = 0;    // (and instructions of those kinds streamed)
     int mode = MODE_STAGES;
-    // Wait until the compute side has released every slot of the kind used so far (slot s was last
-    // filled in the current round if s < position, else in the previous one).
-    auto drain = [&](int kind, int next) -> bool {
+    // Make the ring's memory serve `next`: wait until the compute side has released every slot of the kind used so far (slot s was
+    // last filled in the current round if s < position, else in the previous one; an attention run returns the memory itself).
+    auto enter = [&](int next) -> bool {
         int ok = 1;
-        if (lane == 0 && kind != MODE_ATTN) {         // (an attention run returns the memory itself)
-            if (kind == MODE_WTILES) {
-                for (int s = 0; s < kTcWSlots && ok; ++s)
-                    ok = wait_barrier(p, c, &c->w_empty[s], (wphase ^ (s < wslot ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
-            } else if (kind >= MODE_WWIDE) {
-                const int k = kind - MODE_WWIDE;
-                for (int s = 0; s < wide_stages(k) && ok; ++s)
-                    ok = wait_barrier(p, c, &c->ww_empty[k][s], (wwphase[k] ^ (s < wwslot[k] ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY, 2) ? 1 : 0;
-                // ... and until the run's epilogues have read their staging rows behind the slots
-                if (ok && next < MODE_WWIDE) ok = wait_word(p, c, &c->wide_done, wide_count, rc.seq, WHERE_STAGING) ? 1 : 0;
-            } else if (kind == MODE_KVTILES) {
-                for (int s = 0; s < kKvSlots && ok; ++s)
-                    ok = wait_barrier(p, c, &c->kv_empty[s], (kvphase ^ (s < kvslot ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
-            } else {
-                for (int s = 0; s < kStages && ok; ++s)
-                    ok = wait_barrier(p, c, &c->empty[s], (pos.phase ^ (s < pos.stage ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
-            }
+        if (lane == 0 && mode != MODE_ATTN) {
+            const bool wide = mode >= MODE_WWIDE;
+            const int k = wide ? mode - MODE_WWIDE : 0;
+            unsigned long long* empty = mode == MODE_STAGES ? c->empty : mode == MODE_WTILES ? c->w_empty : mode == MODE_KVTILES ? c->kv_empty : c->ww_empty[k];
+            const int n = mode == MODE_STAGES ? kStages : mode == MODE_WTILES ? kTcWSlots : mode == MODE_KVTILES ? kKvSlots : wide_stages(k);
+            const int at = mode == MODE_STAGES ? pos.stage : mode == MODE_WTILES ? wslot : mode == MODE_KVTILES ? kvslot : wwslot[k];
+            const uint32_t ph = mode == MODE_STAGES ? pos.phase : mode == MODE_WTILES ? wphase : mode == MODE_KVTILES ? kvphase : wwphase[k];
+#pragma unroll 1
+            for (int s = 0; s < n && ok; ++s)
+                ok = wait_barrier(p, c, empty + s, (ph ^ (s < at ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY, wide ? 2 : 1) ? 1 : 0;
+            // ... and until a run of 256-row tiles' epilogues have read their staging rows behind the slots
+            if (ok && wide && next < MODE_WWIDE) ok = wait_word(p, c, &c->wide_done, wide_count, rc.seq, WHERE_STAGING) ? 1 : 0;
         }
         ok = __shfl_sync(0xffffffffu, ok, 0);
-        if (kind >= MODE_WWIDE && next < MODE_WWIDE) {
+        if (mode >= MODE_WWIDE && next < MODE_WWIDE) {
             // those rows (and the bias) were written with plain stores and cp.async, by the compute warps; bulk copies are next,
             // from any lane: each orders its own behind what lane 0 has seen
             __syncwarp();
             asm volatile("fence.proxy.async;" ::: "memory");
         }
+        if (ok) mode = next;
         return ok != 0;
     };
-    auto enter = [&](int kind) -> bool {              // make the ring's memory serve `kind`
-        if (mode == kind) return true;
-        if (!drain(mode, kind)) return false;
-        mode = kind;
-        return true;
-    };
-    while (rc.valid(p)) {
+    // One place that looks for the next instruction, and one that changes what the ring's memory serves: inlined wherever the loop
+    // needed them (and with a second cursor that asked L2 for stages further ahead, which made every step slower: batch 1 860 ->
+    // 890 us with one stage, 1030 with 16) they made the kernel 126 KB of code instead of 56, fetched cold by each launch: MLP block of
+    // one row 29.2 -> 28.1 us, batch-64 step 1570 -> 1563.
+    for (bool inside = false;;) {
+        if (!inside) {
+            rc.seek(p);
+            if (!rc.valid(p)) break;
+        }
+        inside = false;
+        const int kind = rc.attn ? MODE_ATTN : rc.kv ? MODE_KVTILES : !rc.gemm ? MODE_STAGES : rc.wide ? MODE_WWIDE + (rc.wide == 2 ? 0 : 1) : MODE_WTILES;
+        if (mode != kind && !enter(kind)) goto left;
         if (rc.attn) {
             // a run of tcgen05 attentions of head_dim 128: the ring's memory is theirs until the compute warps are through
-            if (!enter(MODE_ATTN)) goto left;
             int ok = 1;
             if (lane == 0) {
                 mbar_arrive(&c->ring_granted);
@@ -265,7 +252,6 @@ __device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint
                 const int opi = __ldg(p.insts + (long long)rc.idx * 4).x - 1;
                 if (opi < 0 || opi >= p.n_ops || !(is_attention_tc(p.ops + opi) && p.ops[opi].i[5] == 128)) break;
             }
-            rc.seek(p);
             continue;
         }
         if (rc.kv) {
@@ -273,7 +259,6 @@ __device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint
             // copies of four rows issued by four lanes at once; K and V tiles alternate.  The whole
             // instruction is streamed from this tight loop: measured, a single lane that issued every
             // copy and walked the outer loop per slot spent ~950 cycles per 16 KB slot (32 GB/s).
-            if (!enter(MODE_KVTILES)) goto left;
             if (rc.kv_gated) {                        // unfused form: the appended row is readable once the dependencies are met
                 int go = 1;
                 if (lane == 0) go = wait_barrier(p, c, &c->kv_go, kvgo, rc.seq, WHERE_DEP) ? 1 : 0;
@@ -304,30 +289,28 @@ __device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint
                 }
             }
             rc.idx += gridDim.x;
-            rc.seek(p);
             continue;
         }
         if (rc.gemm && rc.wide) {
             // tile GEMM with 256 activation rows: the one or two weight tiles of a k-tile (128 rows x 64 K-elements each, adjacent
             // in the packed array) fill one slot of its kind; its barrier is armed a second time by the feeder warp, for the activations.
             // One lane: a k-tile's MMAs take 0.58 us, the lane's wait / expect / copy sequence 0.2.
-            const int kind = rc.wide == 2 ? 0 : 1, stages = wide_stages(kind);
-            if (!enter(MODE_WWIDE + kind)) goto left;
+            const int wk = rc.wide == 2 ? 0 : 1, stages = wide_stages(wk);
             const int nkt = rc.nk;
-            const uint32_t wbytes = (uint32_t)wide_wbytes(kind);
-            unsigned long long* full = c->ww_full[kind];
-            unsigned long long* empty = c->ww_empty[kind];
+            const uint32_t wbytes = (uint32_t)wide_wbytes(wk);
+            unsigned long long* full = c->ww_full[wk];
+            unsigned long long* empty = c->ww_empty[wk];
             int ok = 1;
             if (lane == 0) {
                 const unsigned long long wpol = rc.reread ? keep_policy : stream_policy;
                 const uint8_t* src = rc.wpack ? rc.wpack + rc.wtile0 * (long long)kTcTileBytes : nullptr;
                 const long long kstep = (long long)rc.wstride * kTcTileBytes;
-                int sl = wwslot[kind];
-                uint32_t ph = wwphase[kind];
+                int sl = wwslot[wk];
+                uint32_t ph = wwphase[wk];
 #pragma unroll 1
                 for (int kt = 0; kt < nkt; ++kt) {
                     if (!wait_barrier(p, c, empty + sl, ph ^ 1u, rc.seq, WHERE_RING_EMPTY, 2)) { ok = 0; break; }
-                    uint8_t* dst = ring + wide_woff(kind, sl);
+                    uint8_t* dst = ring + wide_woff(wk, sl);
                     if (!check_phase(p, c, full + sl, ph, rc.seq, WHERE_CHECK_ARM)) { ok = 0; break; }
                     mbar_arrive_expect_tx(full + sl, wbytes);
                     if (src) {
@@ -338,15 +321,14 @@ __device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint
                     }
                     if (++sl == stages) { sl = 0; ph ^= 1u; }
                 }
-                if (!ok) { wwslot[kind] = sl; wwphase[kind] = ph; }
+                if (!ok) { wwslot[wk] = sl; wwphase[wk] = ph; }
             }
             if (!__shfl_sync(0xffffffffu, ok, 0)) goto left;
-            const uint32_t wpos = (uint32_t)wwslot[kind] + (uint32_t)nkt;
-            wwslot[kind] = (int)(wpos % stages);
-            wwphase[kind] ^= (wpos / stages) & 1u;
+            const uint32_t wpos = (uint32_t)wwslot[wk] + (uint32_t)nkt;
+            wwslot[wk] = (int)(wpos % stages);
+            wwphase[wk] ^= (wpos / stages) & 1u;
             ++wide_count;
             rc.idx += gridDim.x;
-            rc.seek(p);
             continue;
         }
         if (rc.gemm) {
@@ -358,7 +340,6 @@ __device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint
             // copy sequence takes ~0.2 us (measured: 16 KB copies from one thread top out at 68 GB/s
             // however many are in flight), more than the MMAs of a tile; walking the outer loop (cursor,
             // warp votes) once per tile cost ~950 cycles.
-            if (!enter(MODE_WTILES)) goto left;
             constexpr int kLanes = 4;
             const unsigned long long wpol = rc.reread ? keep_policy : stream_policy;
             bool mine = true;
@@ -388,29 +369,11 @@ __device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint
             wslot = (int)(wpos % kTcWSlots);
             wphase ^= (wpos / kTcWSlots) & 1u;
             rc.idx += gridDim.x;
-            rc.seek(p);
             continue;
         }
-        if (!enter(MODE_STAGES)) goto left;
-        // one lane looks whether the ring has a free stage (non-blocking)
-        int free_now = 0;
-        if (lane == 0) free_now = mbar_try_wait(&c->empty[pos.stage], pos.phase ^ 1u) ? 1 : 0;
-        free_now = __shfl_sync(0xffffffffu, free_now, 0);
-        if (!free_now && ahead < p.pf_stages && pc.valid(p)) {
-            // ring full: let L2 fetch a stage further down the stream
-            if (ahead == 0) { pc = rc; }
-            const __nv_bfloat16* src; int bytes, off;
-            pc.piece(lane, src, bytes, off);
-            if (bytes) bulk_prefetch_l2(src, (uint32_t)bytes);
-            pc.advance(p);
-            ++ahead;
-            continue;
-        }
-        if (!free_now) {
-            int ok = 1;
-            if (lane == 0) ok = wait_barrier(p, c, &c->empty[pos.stage], pos.phase ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
-            if (!__shfl_sync(0xffffffffu, ok, 0)) goto left;
-        }
+        int ok = 1;
+        if (lane == 0) ok = wait_barrier(p, c, &c->empty[pos.stage], pos.phase ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
+        if (!__shfl_sync(0xffffffffu, ok, 0)) goto left;
         const __nv_bfloat16* src; int bytes, off;
         rc.piece(lane, src, bytes, off);
         const int total = __reduce_add_sync(0xffffffffu, bytes);
@@ -422,8 +385,8 @@ __device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint
         const bool last = rc.g == rc.ngroups - 1 && rc.seg == rc.nseg - 1;
         if (TRACE && last && lane == 0) trace_rec<TRACE>(p, 0, slot_first, rc.seq, t_first, t_first, (long long)globaltimer());
         pos.advance();
-        rc.advance(p);
-        if (ahead > 0) --ahead;
+        inside = rc.advance();
+        if (!inside) rc.idx += gridDim.x;
     }
 left:
     // (the kinds before the current one have been drained; lane 0 is the one that counts what a failing 256-row tile had requested)
