@@ -332,19 +332,17 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
             if (idx % D == 0) { mine[GD + idx / D] = mx; mine[GD + G + idx / D] = l; }
         }
     }
-    __threadfence();
     compute_sync();
     phase_mark(p, c, 1);
     int* count = reinterpret_cast<int*>(op->ptr[10]) + (long long)pair * op->ld[10];
     if (t == 0) {
-        const int old = atomicAdd(count, 1);
+        const int old = arrive_acq_rel(count);
         c->flag = (old == S - 1);
         if (old == S - 1) *count = 0;          // back to zero for the next launch
     }
     compute_sync();
     phase_mark(p, c, 2);
     if (!c->flag) return;
-    __threadfence();
     // ---- last split to arrive: merge the S partials.  The S partial rows are copied into shared
     // memory with one wave of cp.async (one L2 round trip), then every thread merges one output. ----
     const float* base = part + (long long)pair * S * ldp;

@@ -330,19 +330,17 @@ __device__ __forceinline__ void decode_bulk_body(const Params& p, Ctrl* c, const
             *reinterpret_cast<float4*>(mine + g * D + q4 * 16 + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);
         if (q4 == 0) { mine[GD + g] = mrow; mine[GD + G + g] = lrow; }
     }
-    __threadfence();
     compute_sync();
     phase_mark(p, c, 1);
     int* count = reinterpret_cast<int*>(op->ptr[10]) + (long long)(b * KVH) * op->ld[10];
     if (t == 0) {
-        const int old = atomicAdd(count, 1);
+        const int old = arrive_acq_rel(count);
         c->flag = (old == S - 1);
         if (old == S - 1) *count = 0;          // back to zero for the next launch
     }
     compute_sync();
     phase_mark(p, c, 2);
     if (!c->flag) return;
-    __threadfence();
     // ---- last split to arrive: merge the S partials of every head (warp w: head w), straight from L2.
     // The loads of different splits are independent of each other: the loops are unrolled and free of
     // branches so that many are in flight at once (one split per L2 round trip costs ~1 us each). ----
