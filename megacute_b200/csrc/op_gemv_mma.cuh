@@ -64,16 +64,11 @@ __device__ __forceinline__ void gemv_mma(const Params& p, Ctrl* c, uint8_t* ring
     float4* red = reinterpret_cast<float4*>(work + kMmaRedOff);
     float* rowstat = reinterpret_cast<float*>(work + kMmaStatOff);
 
-    // ---- before the dependency wait: the norm gain of this thread's first vectors ----
+    // ---- before the dependency wait: the norm gain of this thread's first vector ----
     const int nv = K >> 3;
     const uint4* gain = (rms && op->ptr[5]) ? reinterpret_cast<const uint4*>(op->ptr[5]) : nullptr;
     const uint4 ones = make_uint4(0x3f803f80u, 0x3f803f80u, 0x3f803f80u, 0x3f803f80u);
-    uint4 g0[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int v = t + i * kComputeThreads;
-        g0[i] = (gain && v < nv) ? __ldg(gain + v) : ones;
-    }
+    const uint4 g0 = gain && t < nv ? __ldg(gain + t) : ones;
     // everything below that does not depend on the activations is also set up before the wait:
     // the op runs once per instruction, cold, and this code would otherwise sit between the
     // arrival of x and the first MMA
@@ -100,38 +95,31 @@ __device__ __forceinline__ void gemv_mma(const Params& p, Ctrl* c, uint8_t* ring
     }
 
     // ---- stage x * gain (high + low bf16 parts, fragment order); accumulate sum(x^2) per row ----
+    // (one vector of a row at a time here, four k-steps at a time below: what counts is that the body has few registers.  With four
+    // vectors and eight k-steps it saved and restored 43 callee-saved registers per call, 44 KB of local memory each way through a
+    // path of 32 bytes a cycle: batch 1 at context 1024 852 -> 831 us, at 16384 985 -> 970, five sequences 1172 -> 1137, an MLP block of
+    // one row 28.1 -> 27.0.  With two k-steps batch 1 is back at 844.)
     {
 #pragma unroll 1
         for (int m = 0; m < M; ++m) {
             float ss = 0.f;
 #pragma unroll 1
-            for (int vb = 0; vb < nv; vb += 4 * kComputeThreads) {            // batches of 4 vectors per thread
-                float f[4][8];
+            for (int v = t; v < nv; v += kComputeThreads) {
+                float f[8], gq[8];
+                load8(x, m * ldx + v * 8, xdt, f);
+                unpack8(v == t ? g0 : (gain ? __ldg(gain + v) : ones), gq);
+                uint32_t hi[4], lo[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {                                 // all loads of the batch first
-                    const int v = vb + t + i * kComputeThreads;
-                    if (v < nv) load8(x, m * ldx + v * 8, xdt, f[i]);
+                for (int j = 0; j < 4; ++j) {
+                    const float y0 = f[2 * j] * gq[2 * j], y1 = f[2 * j + 1] * gq[2 * j + 1];
+                    ss += f[2 * j] * f[2 * j] + f[2 * j + 1] * f[2 * j + 1];
+                    const float h0 = round_bf16(y0), h1 = round_bf16(y1);
+                    hi[j] = pack2(h0, h1);
+                    lo[j] = pack2(y0 - h0, y1 - h1);
                 }
+                uint32_t* d = reinterpret_cast<uint32_t*>(xf + m * xrow + (v >> 1) * 64 + (v & 1) * 4);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const int v = vb + t + i * kComputeThreads;
-                    if (v < nv) {
-                        float gq[8];
-                        unpack8(vb == 0 ? g0[i] : (gain ? __ldg(gain + v) : ones), gq);
-                        uint32_t hi[4], lo[4];
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float y0 = f[i][2 * j] * gq[2 * j], y1 = f[i][2 * j + 1] * gq[2 * j + 1];
-                            ss += f[i][2 * j] * f[i][2 * j] + f[i][2 * j + 1] * f[i][2 * j + 1];
-                            const float h0 = round_bf16(y0), h1 = round_bf16(y1);
-                            hi[j] = pack2(h0, h1);
-                            lo[j] = pack2(y0 - h0, y1 - h1);
-                        }
-                        uint32_t* d = reinterpret_cast<uint32_t*>(xf + m * xrow + (v >> 1) * 64 + (v & 1) * 4);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) { d[j * 4] = hi[j]; d[j * 4 + 2] = lo[j]; }
-                    }
-                }
+                for (int j = 0; j < 4; ++j) { d[j * 4] = hi[j]; d[j * 4 + 2] = lo[j]; }
             }
             if (rms) {
                 ss = warp_sum(ss);
@@ -160,42 +148,42 @@ __device__ __forceinline__ void gemv_mma(const Params& p, Ctrl* c, uint8_t* ring
                 uint32_t a_base = smem_u32(ring + pos.stage * kStageBytes) + a_lane;
                 uint32_t b_base = b_lane + seg * (kSegElems / 16) * 64;
 #pragma unroll 1
-                for (int half = 0; half < kSlice / 128 && left > 0; ++half) {     // batches of 8 k-steps
-                    uint32_t a[8][4];
+                for (int batch = 0; batch < kSlice / 64 && left > 0; ++batch) {     // batches of 4 k-steps
+                    uint32_t a[4][4];
                     // lanes of absent activation rows feed zeros and stay out of the load: with one
                     // row only a quarter of the warp touches shared memory
                     if (packed) {
-                        uint2 b[8];
+                        uint2 b[4];
 #pragma unroll
-                        for (int ks = 0; ks < 8; ++ks) {
+                        for (int ks = 0; ks < 4; ++ks) {
                             if (ks * 16 < left) {
                                 ldmatrix_x4(a_base + ks * 32, a[ks][0], a[ks][1], a[ks][2], a[ks][3]);
                                 b[ks] = bm < M ? lds64(b_base + ks * 64) : make_uint2(0u, 0u);
                             }
                         }
 #pragma unroll
-                        for (int ks = 0; ks < 8; ++ks)
+                        for (int ks = 0; ks < 4; ++ks)
                             if (ks * 16 < left) mma_bf16(accs[ks & 3], a[ks], b[ks].x, b[ks].y);
                     } else {
-                        uint4 b[8];
+                        uint4 b[4];
 #pragma unroll
-                        for (int ks = 0; ks < 8; ++ks) {
+                        for (int ks = 0; ks < 4; ++ks) {
                             if (ks * 16 < left) {
                                 ldmatrix_x4(a_base + ks * 32, a[ks][0], a[ks][1], a[ks][2], a[ks][3]);
                                 b[ks] = bm < M ? lds128(b_base + ks * 64) : make_uint4(0u, 0u, 0u, 0u);
                             }
                         }
 #pragma unroll
-                        for (int ks = 0; ks < 8; ++ks) {
+                        for (int ks = 0; ks < 4; ++ks) {
                             if (ks * 16 < left) {
                                 mma_bf16(accs[(ks & 1) * 2], a[ks], b[ks].x, b[ks].y);
                                 mma_bf16(accs[(ks & 1) * 2 + 1], a[ks], b[ks].z, b[ks].w);
                             }
                         }
                     }
-                    a_base += 8 * 32;
-                    b_base += 8 * 64;
-                    left -= 128;
+                    a_base += 4 * 32;
+                    b_base += 4 * 64;
+                    left -= 64;
                 }
             }
             // the stage goes back to the producer as soon as this warp has read its slice
