@@ -32,13 +32,13 @@
 namespace mk {
 
 // the same columns of two accumulators, `second` columns apart, added (second == 0: one accumulator)
-__device__ __forceinline__ void tc_ld32_sum(uint32_t taddr, uint32_t second, float* v) {
-    tc_ld32(taddr, v);
+__device__ __forceinline__ void tc_ld16_sum(uint32_t taddr, uint32_t second, float* v) {
+    tc_ld16(taddr, v);
     if (second) {
-        float w[32];
-        tc_ld32(taddr + second, w);
+        float w[16];
+        tc_ld16(taddr + second, w);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] += w[j];
+        for (int j = 0; j < 16; ++j) v[j] += w[j];
     }
 }
 
@@ -360,7 +360,9 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
     tc_fence_after();
     phase_mark(p, c, 2);                                                    // accumulator complete
     __syncwarp();                                                           // (the tensor-memory loads below are .sync.aligned: whole warp, converged)
-    // first half: tensor memory -> shared memory.  Warp w reads lanes 32 (w & 3) .. +31 (activation
+    // first half: tensor memory -> shared memory, 16 columns at a time (32 at a time needed so many registers that each call saved 320 bytes
+    // per thread instead of 204, with almost no L1 to take them: 64 sequences at context 1024 1544 -> 1526 us, prompt of 333 tokens
+    // 1865 -> 1845, MLP block of 256 rows 57.9 -> 56.6).  Warp w reads lanes 32 (w & 3) .. +31 (activation
     // rows) and column half w >> 2; the activation stages are free now (every MMA has completed).
     const int qd = warp & 3, h = warp >> 2;
     float* stage = reinterpret_cast<float*>(work + kTcXOff);
@@ -369,25 +371,29 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
     if (ok && qd * 32 < rows) {
         const uint32_t tl = tmem + ((uint32_t)(qd * 32) << 16);
         float* srow = stage + (qd * 32 + lane) * kTcStagePitch;
-        float v[32];
+        float v[16];
         if (swi) {
             // gate columns 32 h .. +31 and the up columns 64 further of the same outputs
-            float u[32];
-            tc_ld32_sum(tl + h * 32, two, v);
-            tc_ld32_sum(tl + 64 + h * 32, two, u);
-#pragma unroll
-            for (int j = 0; j < 32; j += 4)
-                *reinterpret_cast<float4*>(srow + h * 32 + j) =
-                    make_float4(v[j] * sigmoidf_(v[j]) * u[j], v[j + 1] * sigmoidf_(v[j + 1]) * u[j + 1],
-                                v[j + 2] * sigmoidf_(v[j + 2]) * u[j + 2], v[j + 3] * sigmoidf_(v[j + 3]) * u[j + 3]);
-        } else {
 #pragma unroll 1
             for (int ch = 0; ch < 2; ++ch) {
-                const int tcol = h * 64 + ch * 32;
-                if (n0 + tcol >= N) break;
-                tc_ld32_sum(tl + tcol, two, v);
+                const int tcol = h * 32 + ch * 16;
+                float u[16];
+                tc_ld16_sum(tl + tcol, two, v);
+                tc_ld16_sum(tl + 64 + tcol, two, u);
 #pragma unroll
-                for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(srow + tcol + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                for (int j = 0; j < 16; j += 4)
+                    *reinterpret_cast<float4*>(srow + tcol + j) =
+                        make_float4(v[j] * sigmoidf_(v[j]) * u[j], v[j + 1] * sigmoidf_(v[j + 1]) * u[j + 1],
+                                    v[j + 2] * sigmoidf_(v[j + 2]) * u[j + 2], v[j + 3] * sigmoidf_(v[j + 3]) * u[j + 3]);
+            }
+        } else {
+#pragma unroll 1
+            for (int ch = 0; ch < 4; ++ch) {
+                const int tcol = h * 64 + ch * 16;
+                if (n0 + tcol >= N) break;
+                tc_ld16_sum(tl + tcol, two, v);
+#pragma unroll
+                for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(srow + tcol + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             }
         }
     }

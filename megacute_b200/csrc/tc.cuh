@@ -38,6 +38,16 @@ __device__ __forceinline__ bool elect_one() {
     asm volatile("{ .reg .pred q; elect.sync _|q, 0xffffffff; selp.u32 %0, 1, 0, q; }" : "=r"(p));
     return p != 0;
 }
+// 16 consecutive fp32 columns of this thread's lane (warp-wide)
+__device__ __forceinline__ void tc_ld16(uint32_t taddr, float* v) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]), "=f"(v[8]), "=f"(v[9]),
+          "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15])
+        : "r"(taddr)
+        : "memory");
+}
 // 32 consecutive fp32 columns of this thread's lane (warp-wide, lanes 32 (warp & 3) .. +31)
 __device__ __forceinline__ void tc_ld32(uint32_t taddr, float* v) {
     uint32_t r[32];
