@@ -37,6 +37,10 @@ enum {
     MK_OP_ARGMAX = 11      /* ids[r] = argmax(x[r]): greedy sampling, column chunks merged in-op    */
 };
 
+/* mk_op_desc.flags: direct operands (mk_program_set_direct).  MK_OP_GEMV on the tensor-core path: x, output, residual;
+ * MK_OP_DECODE_ATTN, not its many-sequence form: q, k_new and v_new, output; MK_OP_GATHER: output.  fp32. */
+enum { MK_F_DIRECT_IN = 8, MK_F_DIRECT_OUT = 16, MK_F_DIRECT_RES = 32 };
+
 #define MK_MAX_PTRS 12
 #define MK_INST_WORDS 16
 
@@ -116,6 +120,14 @@ int mk_program_create(int device, const int32_t* insts, int n_insts, const int32
  * Every function of a program makes the program's device current for the duration of the call and
  * puts the caller's current device back before it returns. */
 int mk_program_set_ops(mk_program* p, const mk_op_desc* ops, int n_ops, void* stream);
+
+/* Memory of the direct operands: two copies of `bytes` bytes (a multiple of 16, 16-byte aligned), one behind the other, that
+ * launches use in turn; a descriptor's address of a direct operand is the one in the first copy.  Their readers wait for the
+ * values themselves -- every element holds the bits 0xffffffff until its writer of the launch has stored it -- so such
+ * buffers need no arrivals and waits in the tables, have exactly one writing op, which writes every element that is read, and only
+ * the readers named above.  Fills both copies on `stream`; mk_program_reset fills them again.  Call before the
+ * mk_program_set_ops that uses them. */
+int mk_program_set_direct(mk_program* p, void* memory, size_t bytes, void* stream);
 
 /* One launch of the persistent kernel on `stream` (asynchronous).  Replaces
  * self._compiled(views, insts, waits, arrives, counters, trace, epoch) (runtime.py:383-384);

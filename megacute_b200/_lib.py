@@ -53,6 +53,7 @@ SYMBOLS = {
     "mk_program_create": (ctypes.c_int, [ctypes.c_int, _P, ctypes.c_int, _P, ctypes.c_int, _P, ctypes.c_int,
                                          ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.c_int, ctypes.POINTER(_P)]),
     "mk_program_set_ops": (ctypes.c_int, [_P, _P, ctypes.c_int, _P]),
+    "mk_program_set_direct": (ctypes.c_int, [_P, _P, ctypes.c_size_t, _P]),
     "mk_launch": (ctypes.c_int, [_P, _P]),
     "mk_program_set_timeout": (ctypes.c_int, [_P, ctypes.c_uint64]),
     "mk_program_status": (ctypes.c_int, [_P, _P, _I32P]),

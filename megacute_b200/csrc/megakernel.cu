@@ -115,6 +115,9 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         left = mk_feeder(p);
     } else if (warp == kIssuerWarp) {
         // ---------------- issuer warp: MMAs of tile GEMMs with 256-row tiles and of the tcgen05 prefill attention ----------------
+        // (first of all the next launch's copies of the direct operands: this warp has nothing to do yet)
+        for (int i = blockIdx.x * 32 + (threadIdx.x & 31); i < p.direct_pieces; i += gridDim.x * 32)
+            p.direct_next[i] = make_uint4(kUnwritten, kUnwritten, kUnwritten, kUnwritten);
         mk_issuer(p);
     } else {
         // ---------------- compute warps ----------------
@@ -166,7 +169,9 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
             switch (op->kind) {
                 case MK_OP_GEMV:
                     if (op->flags & GEMV_F_UNITS) {
-                        npos = mk_op_gemv_units(p, op, in.a0, in.a1, in.seq, ppos, in.nwait, wait_off, in.narrive, arrive_off);
+                        npos = op->flags & GEMV_F_DIRECT_X
+                                   ? mk_op_gemv_direct(p, op, in.a0, in.a1, in.seq, ppos, in.nwait, wait_off, in.narrive, arrive_off)
+                                   : mk_op_gemv_units(p, op, in.a0, in.a1, in.seq, ppos, in.nwait, wait_off, in.narrive, arrive_off);
                         aborting = npos < 0;
                     } else {
                         if (wait_deps(p, c, in.nwait, wait_off, in.seq)) { aborting = true; break; }
@@ -197,7 +202,7 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                 default:
                     if (wait_deps(p, c, in.nwait, wait_off, in.seq)) { aborting = true; break; }
                     if (TRACE && threadIdx.x == 0) c->t_dep = (long long)globaltimer();
-                    known = mk_op_pointwise(op, in.a0, in.a1);
+                    known = mk_op_pointwise(op, in.a0, in.a1, p.direct_off);
                     aborting = publish(p, c, in.narrive, arrive_off);
                     break;
             }
@@ -309,6 +314,9 @@ struct mk_program {
     unsigned long long timeout_ns = 2000000000ull;
     int tcgen05_ops = 0;             // tile GEMMs bound to the tcgen05 body by the last set_ops
     int tcgen05_attn_ops = 0;        // ... prefill attention ops
+    uint8_t* direct = nullptr;       // direct operands (mk_program_set_direct): two copies of direct_bytes
+    size_t direct_bytes = 0;
+    int direct_turn = 0;             // ... the copy that the next launch uses
 };
 
 static const size_t kMapBytes = 512;       // tensor-map space per op
@@ -406,6 +414,25 @@ static bool tile_gemm_on_tcgen05(const mk_op_desc& d) {
 // the extents the descriptor states.  The kernel trusts its tables; this is where a table built for
 // another graph, or a descriptor with a shrunken extent, is caught -- as an error code here instead of
 // an out-of-bounds access on the device.  On failure the message names the instruction.
+static const char* direct_operands(const mk_program* p, const mk_op_desc& d) {
+    const int f = d.flags & (MK_F_DIRECT_IN | MK_F_DIRECT_OUT | MK_F_DIRECT_RES);
+    if (!f || (d.kind != MK_OP_GEMV && d.kind != MK_OP_DECODE_ATTN && d.kind != MK_OP_GATHER)) return nullptr;
+    auto inside = [&](int ptr, int dtype) {
+        return dtype == mk::DT_F32 && p->direct && d.ptr[ptr] >= (uint64_t)p->direct && d.ptr[ptr] < (uint64_t)p->direct + p->direct_bytes;
+    };
+    bool ok = true;
+    if (d.kind == MK_OP_GEMV) {
+        ok = (d.flags & mk::GEMV_F_UNITS) && (!(f & MK_F_DIRECT_IN) || inside(0, d.i[4])) && (!(f & MK_F_DIRECT_OUT) || inside(2, d.i[5])) &&
+             (!(f & MK_F_DIRECT_RES) || inside(4, d.i[6]));
+    } else if (d.kind == MK_OP_DECODE_ATTN) {
+        ok = !d.i[11] && !d.i[9] && (!(f & MK_F_DIRECT_IN) || (d.i[6] && inside(0, d.i[7]) && inside(5, d.i[7]) && inside(6, d.i[7]))) &&
+             (!(f & MK_F_DIRECT_OUT) || inside(4, d.i[8]));
+    } else {
+        ok = f == MK_F_DIRECT_OUT && inside(2, d.i[3]);
+    }
+    return ok ? nullptr : "direct operands: path, type or memory";
+}
+
 static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
     const int W = MK_INST_WORDS;
     auto ceil_div = [](long long a, long long b) { return (a + b - 1) / b; };
@@ -419,7 +446,8 @@ static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
         } else {
             const mk_op_desc& d = ops[opi];
             const long long a0 = w[1], a1 = w[2], a2 = w[3];
-            switch (d.kind) {
+            if (const char* bad = direct_operands(p, d)) why = bad;
+            else switch (d.kind) {
                 case MK_OP_GEMV:
                     if (!(0 <= a0 && a0 < a1 && a1 <= d.i[1])) why = "streaming linear: output range outside [0, N)";
                     break;
@@ -763,9 +791,13 @@ int mk_launch(mk_program* p, void* stream) {
     prm.status = p->d_status;
     prm.epoch = p->epoch;
     prm.timeout_ns = p->timeout_ns;
+    prm.direct_off = p->direct_turn ? (long long)p->direct_bytes : 0;
+    prm.direct_next = reinterpret_cast<uint4*>(p->direct + (p->direct_turn ? 0 : p->direct_bytes));
+    prm.direct_pieces = (int)(p->direct_bytes / 16);
     if (p->trace_cap > 0) mk::megakernel<true><<<p->grid, mk::kThreads, mk::kSmemBytes, st>>>(prm);
     else mk::megakernel<false><<<p->grid, mk::kThreads, mk::kSmemBytes, st>>>(prm);
     MK_CUDA(cudaGetLastError());
+    p->direct_turn ^= 1;
     return MK_OK;
 }
 
@@ -789,7 +821,19 @@ int mk_program_reset(mk_program* p, void* stream) {
     cudaStream_t st = (cudaStream_t)stream;
     MK_CUDA(cudaMemsetAsync(p->d_counters, 0, (size_t)p->n_counters * 4, st));
     MK_CUDA(cudaMemsetAsync(p->d_status, 0, MK_ST_WORDS * 4, st));
+    if (p->direct) MK_CUDA(cudaMemsetAsync(p->direct, 0xff, 2 * p->direct_bytes, st));
+    p->direct_turn = 0;
     p->epoch = 0;
+    return MK_OK;
+}
+
+int mk_program_set_direct(mk_program* p, void* memory, size_t bytes, void* stream) {
+    if (!p || !memory || bytes == 0 || bytes % 16 || bytes / 16 > 0x7fffffff || ((uintptr_t)memory & 15)) return MK_E_ARG;
+    MK_ON_DEVICE(p->device);
+    MK_CUDA(cudaMemsetAsync(memory, 0xff, 2 * bytes, (cudaStream_t)stream));
+    p->direct = reinterpret_cast<uint8_t*>(memory);
+    p->direct_bytes = bytes;
+    p->direct_turn = 0;
     return MK_OK;
 }
 
@@ -926,6 +970,9 @@ extern "C" int mk_launch_noalloc(int device, const int32_t* d_insts, int n_insts
     prm.status = d_status;
     prm.epoch = 1;
     prm.timeout_ns = 2000000000ull;
+    prm.direct_off = 0;
+    prm.direct_next = nullptr;
+    prm.direct_pieces = 0;
     mk::megakernel<false><<<grid, mk::kThreads, mk::kSmemBytes, st>>>(prm);
     MK_CUDA(cudaGetLastError());
     if (status) {

@@ -112,7 +112,23 @@ struct Params {
     int* status;                  // MK_ST_WORDS words; word 0 != 0 aborts every waiter
     int epoch;
     unsigned long long timeout_ns;
+    long long direct_off;         // direct operands (below): byte offset from a descriptor's address to this launch's copy
+    uint4* direct_next;           // ... the next launch's copies, to be filled with kUnwritten, and their 16-byte pieces
+    int direct_pieces;
 };
+
+// Direct operands: activations whose reader looks at the values themselves instead of a dependency counter.  A step of few rows is a
+// chain of ops that each need all of the one before.  Through a counter such a hop is the writer's release (a fence that waits for
+// everything the SM has in flight, the next weights among it: 0.4 - 1.3 us), the arrival, the reader's poll, a round trip to L2
+// that 148 SMs make side by side (0.7 - 1.6 us), and only then the load of the values, another one.  Instead every fp32 element of
+// such a buffer holds kUnwritten until its one writer of the launch stores it (relaxed, gpu scope), and the reader loads the values
+// until none is kUnwritten (relaxed, gpu scope; a 4-byte access is atomic, and no other access is ordered by it, so no fence is
+// needed).  A buffer has two copies that launches use in turn; during a launch the other copy, whose readers ended with the
+// launch before, is filled with kUnwritten again.  kUnwritten is a NaN that arithmetic does not make (its NaN is 0x7fffffff); a
+// value that happens to be it is stored as that one.
+// Which buffers: passes.direct_buffers.  A step of the 1B shape, batch 1, at context 1024 836 -> 760 us, at 16384 976 -> 898; two
+// ragged sequences 967 -> 903; eight, whose down projections are K splits and keep their counters, 1332 -> 1324.
+constexpr uint32_t kUnwritten = 0xffffffffu;
 
 // a tile GEMM bound to the tcgen05 body with 256-row tiles (op_gemm_tc_wide.cuh)
 __device__ __forceinline__ bool is_wide_gemm(const mk_op_desc* op) { return op->kind == MK_OP_GEMM && op->i[11] == 256 && op->ptr[11] != 0; }
@@ -395,6 +411,23 @@ __device__ __forceinline__ float2 unpack2h(uint32_t w) {
 }
 // two consecutive values in the 16-bit type `dtype` (DT_BF16 or DT_F16)
 __device__ __forceinline__ uint32_t pack2t(int dtype, float a, float b) { return dtype == DT_F16 ? pack2h(a, b) : pack2(a, b); }
+// direct operands: 8 elements (16-byte aligned) and one; the largest of the loaded words is kUnwritten if any is
+__device__ __forceinline__ uint32_t load8_direct(const float* at, float* f) {
+    uint32_t* w = reinterpret_cast<uint32_t*>(f);
+    asm volatile("ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]) : "l"(at) : "memory");
+    asm volatile("ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(at + 4) : "memory");
+    return max(max(max(w[0], w[1]), max(w[2], w[3])), max(max(w[4], w[5]), max(w[6], w[7])));
+}
+__device__ __forceinline__ float load1_direct(const float* at) {
+    uint32_t w;
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(w) : "l"(at) : "memory");
+    return __uint_as_float(w);
+}
+__device__ __forceinline__ void store1_direct(float* at, float v) {
+    uint32_t w = __float_as_uint(v);
+    if (w == kUnwritten) w = 0x7fffffffu;
+    asm volatile("st.relaxed.gpu.global.b32 [%0], %1;" ::"l"(at), "r"(w) : "memory");
+}
 // load 8 consecutive elements as fp32 from a bf16, fp32 or fp16 row; 16-byte aligned.
 // Loads go to L2 (ld.global.cg): activations are rewritten by other SMs inside one launch and L1
 // is not coherent, so a line cached by an earlier instruction of this SM could be stale.
@@ -617,6 +650,33 @@ __device__ __forceinline__ bool wait_counter(const Params& p, Ctrl* c, int count
     const int want = target * p.epoch;
     if (ld_acquire(p.counters + counter) >= want) return true;
     return wait_counter_spin(p, c, counter, want, seq);
+}
+
+// One more look at a direct operand that was not there yet: false when the wait has to end (time limit or abort).
+struct DirectWait {
+    uint32_t it = 0;
+    unsigned long long t0 = 0;
+    __device__ __forceinline__ bool again(const Params& p, Ctrl* c, int seq) {
+        if ((++it & 63u) != 0) return true;
+        if (*(volatile int*)&c->abort) return false;
+        if (ld_volatile(&p.status[MK_ST_CODE]) != 0) { c->abort = 1; return false; }
+        const unsigned long long now = globaltimer();
+        if (t0 == 0) t0 = now;
+        else if (now - t0 > p.timeout_ns) {
+            report(p, c, MK_DEV_TIMEOUT_COUNTER, seq, WHERE_DEP, -1, 0, 0);
+            return false;
+        }
+        return true;
+    }
+};
+
+// ... until it is there, for a value that has been written long before in all but the first hops of a program
+static __device__ __noinline__ float wait1_direct(const Params& p, Ctrl* c, const float* at, int seq) {
+    DirectWait w;
+    float v;
+    do v = load1_direct(at);
+    while (__float_as_uint(v) == kUnwritten && w.again(p, c, seq));
+    return v;
 }
 
 // One decoded instruction, held in registers (never address-taken, so it is never demoted to

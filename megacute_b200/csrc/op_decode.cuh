@@ -129,9 +129,19 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
             const long long e0 = which < 0 ? (long long)b * op->ld[0] + (kvh * G + chunk) * D
                                            : (long long)b * op->ld[5 + which] + kvh * D;
             float a[8], o[8];
-            load8(src, e0 + dp * 8, qdt, a);
             const bool rot = fused && which != 1;                         // v is not rotated
-            if (rot) load8(src, e0 + pd, qdt, o);
+            if (op->flags & MK_F_DIRECT_IN) {
+                const float* at = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(src) + p.direct_off) + e0;
+                DirectWait w;
+                uint32_t top;
+                do {
+                    top = load8_direct(at + dp * 8, a);
+                    if (rot) top = max(top, load8_direct(at + pd, o));
+                } while (top == kUnwritten && w.again(p, c, seq));
+            } else {
+                load8(src, e0 + dp * 8, qdt, a);
+                if (rot) load8(src, e0 + pd, qdt, o);
+            }
             float y[8];
 #pragma unroll
             for (int e = 0; e < 8; ++e) y[e] = rot ? a[e] * cs[e] + sign * o[e] * sn[e] : a[e];
@@ -311,13 +321,19 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
             reinterpret_cast<float*>(op->ptr[5 + which])[(long long)b * op->ld[5 + which] + kvh * D + t % D] = 0.f;
         }
     };
-    void* outp = reinterpret_cast<void*>(op->ptr[4]);
     const int odt = op->i[8];
+    const bool direct_out = op->flags & MK_F_DIRECT_OUT;
+    void* outp = reinterpret_cast<void*>(op->ptr[4] + (direct_out ? p.direct_off : 0));
+    auto put = [&](int idx, float v) {
+        const long long e = (long long)b * op->ld[4] + kvh * GD + idx;
+        if (direct_out) store1_direct(reinterpret_cast<float*>(outp) + e, v);
+        else store1(outp, e, odt, v);
+    };
     if (S == 1) {
         for (int idx = t; idx < GD; idx += kComputeThreads) {
             float mx, l;
             const float a = merged(idx, mx, l);
-            store1(outp, (long long)b * op->ld[4] + kvh * GD + idx, odt, l == 0.f ? 0.f : a * rcp(l));
+            put(idx, l == 0.f ? 0.f : a * rcp(l));
         }
         zero_inputs();
         return;
@@ -367,7 +383,7 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
             a = fmaf(w, sp[k * row_f + idx], a);
             l = fmaf(w, sp[k * row_f + GD + G + g], l);
         }
-        store1(outp, (long long)b * op->ld[4] + kvh * GD + idx, odt, l == 0.f ? 0.f : a * rcp(l));
+        put(idx, l == 0.f ? 0.f : a * rcp(l));
     }
     zero_inputs();
 }

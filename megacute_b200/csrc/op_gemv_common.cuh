@@ -11,7 +11,8 @@
 // descriptor: ptr 0 x, 1 w, 2 out, 3 bias, 4 residual, 5 norm gain
 //             i 0 M, 1 N_out, 2 K, 3 act, 4 x dtype, 5 out dtype, 6 residual dtype
 //             f 0 rms eps; flags bit0 swiglu (w rows interleaved in 64-row gate/up blocks,
-//             slots 0-3 = gate rows and 4-7 = up rows of 4 outputs), bit1 rms-normalise x first
+//             slots 0-3 = gate rows and 4-7 = up rows of 4 outputs), bit1 rms-normalise x first, bit2 units,
+//             bits 3, 4, 5 direct x, output, residual
 // instruction args: 0 o0, 1 o1 -- the output columns [o0, o1) this instruction produces.
 #pragma once
 #include "mk_device.cuh"
@@ -19,6 +20,9 @@
 namespace mk {
 
 constexpr int GEMV_F_SWIGLU = 1, GEMV_F_RMS = 2;
+// direct operands (mk_device.cuh; with GEMV_F_UNITS only): x, output, residual.  The wait list of an instruction with a direct x
+// is about the residual and the output: the finisher warp waits for it.
+constexpr int GEMV_F_DIRECT_X = MK_F_DIRECT_IN, GEMV_F_DIRECT_OUT = MK_F_DIRECT_OUT, GEMV_F_DIRECT_RES = MK_F_DIRECT_RES;
 // GEMV_F_UNITS (set by the host when K is a multiple of 16): the tensor-core streaming path.
 // A stage is 16 weight rows x one 2048-element K segment.  Each compute warp multiplies a 256-wide
 // K slice of the 16 rows with warp-level MMAs (weights are the A operand straight from the stage via

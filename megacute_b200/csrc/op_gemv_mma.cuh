@@ -53,6 +53,8 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
 
 // The op waits for its own dependencies so that loads which depend on nothing in the launch (the
 // norm gain) are already in flight when the wait ends.
+// DIRECT: x is a direct operand (mk_device.cuh).  A function of its own, so that neither form runs the other's code.
+template <bool DIRECT>
 __device__ __forceinline__ void gemv_mma(const Params& p, Ctrl* c, uint8_t* ring, uint8_t* work, const mk_op_desc* op,
                                          int o0, int o1, int seq, RingPos& pos, int nwait, int wait_off) {
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
@@ -86,9 +88,9 @@ __device__ __forceinline__ void gemv_mma(const Params& p, Ctrl* c, uint8_t* ring
     const uint32_t b_lane = smem_u32(xf) + (bm < M ? bm : 0) * xrow + (kw >> 4) * 64 + (lane & 3) * 16 +
                             (packed ? (bn >> 2) * 8 : 0);
     const int xdt = op->i[4];
-    const void* x = reinterpret_cast<const void*>(op->ptr[0]);
+    const void* x = reinterpret_cast<const void*>(op->ptr[0] + (DIRECT ? p.direct_off : 0));
     const long long ldx = op->ld[0];
-    if (wait_deps(p, c, nwait, wait_off, seq)) return;
+    if (wait_deps(p, c, DIRECT ? 0 : nwait, wait_off, seq)) return;
     if (t == 0) {
         mbar_arrive(&c->deps_met);          // the finisher may now read the residual of the first row group
         if (p.trace_cap > 0) c->t_dep = (long long)globaltimer();
@@ -106,7 +108,12 @@ __device__ __forceinline__ void gemv_mma(const Params& p, Ctrl* c, uint8_t* ring
 #pragma unroll 1
             for (int v = t; v < nv; v += kComputeThreads) {
                 float f[8], gq[8];
-                load8(x, m * ldx + v * 8, xdt, f);
+                if (DIRECT) {
+                    DirectWait w;
+                    while (load8_direct(reinterpret_cast<const float*>(x) + m * ldx + v * 8, f) == kUnwritten && w.again(p, c, seq)) {}
+                } else {
+                    load8(x, m * ldx + v * 8, xdt, f);
+                }
                 unpack8(v == t ? g0 : (gain ? __ldg(gain + v) : ones), gq);
                 uint32_t hi[4], lo[4];
 #pragma unroll
@@ -208,6 +215,16 @@ __device__ __forceinline__ void gemv_mma(const Params& p, Ctrl* c, uint8_t* ring
     phase_mark(p, c, 2);
 }
 
+// an instruction's whole wait list, by the calling warp
+static __device__ __noinline__ bool wait_list(const Params& p, Ctrl* c, int nwait, int wait_off, int seq) {
+    bool ok = true;
+    for (int k = threadIdx.x & 31; k < nwait; k += 32) {
+        const int2 w = __ldg(p.waits + wait_off + k);
+        ok = wait_counter(p, c, w.x, w.y, seq) && ok;
+    }
+    return __all_sync(0xffffffffu, ok) != 0;
+}
+
 // The finisher warp: walks the CTA's instructions like the producer does and, for every streaming
 // linear of the tensor-core path, turns the deposited partial tiles into outputs.
 // Lane l holds rows ob = o0 + 16 * group + (l >> 2) and ob + 8, activation rows m0 = 2 * (l & 3), m0 + 1
@@ -228,8 +245,9 @@ __device__ __forceinline__ void gemv_finisher(const Params& p, Ctrl* c, uint8_t*
         const int o0 = in.a0, o1 = in.a1, seq = in.seq;
         const int ngroups = (swi ? 2 : 1) * ((o1 - o0 + 15) / 16);
         const void* biasp = reinterpret_cast<const void*>(op->ptr[3]);
-        const void* resp = reinterpret_cast<const void*>(op->ptr[4]);
-        void* outp = reinterpret_cast<void*>(op->ptr[2]);
+        const bool direct_out = op->flags & GEMV_F_DIRECT_OUT, direct_res = op->flags & GEMV_F_DIRECT_RES;
+        const void* resp = reinterpret_cast<const void*>(op->ptr[4] + (direct_res ? p.direct_off : 0));
+        void* outp = reinterpret_cast<void*>(op->ptr[2] + (direct_out ? p.direct_off : 0));
         const long long ldo = op->ld[2], ldr = op->ld[4];
         const float eps = op->f[0];
         const bool packed = M <= 4;
@@ -244,6 +262,14 @@ __device__ __forceinline__ void gemv_finisher(const Params& p, Ctrl* c, uint8_t*
         bool ok = wait_barrier(p, c, &c->deps_met, (fullpar >> 4) & 1u, seq, WHERE_COMBINE, 2);
         fullpar ^= 16u;
         if (!ok) return;
+        // (the compute warps look at a direct x alone)
+        if ((op->flags & GEMV_F_DIRECT_X) && in.nwait > 0 && !wait_list(p, c, in.nwait, in.wait_off, seq)) return;
+        // (a direct residual was written hops ago: not there only when a program's first ops are late)
+        auto residual = [&](long long e) {
+            if (!direct_res) return load1(resp, e, rdt);
+            const float v = load1_direct(reinterpret_cast<const float*>(resp) + e);
+            return __float_as_uint(v) == kUnwritten ? wait1_direct(p, c, reinterpret_cast<const float*>(resp) + e, seq) : v;
+        };
 #pragma unroll 1
         for (int g = 0; g < ngroups; ++g) {
             const int sl = g & 3;
@@ -258,8 +284,8 @@ __device__ __forceinline__ void gemv_finisher(const Params& p, Ctrl* c, uint8_t*
                     if (o < o1) {
                         if (biasp) bias_v[h] = load1(biasp, o, 0);
                         if (resp) {
-                            if (m0 < M) res_v[h * 2] = load1(resp, (long long)m0 * ldr + o, rdt);
-                            if (m0 + 1 < M) res_v[h * 2 + 1] = load1(resp, (long long)(m0 + 1) * ldr + o, rdt);
+                            if (m0 < M) res_v[h * 2] = residual((long long)m0 * ldr + o);
+                            if (m0 + 1 < M) res_v[h * 2 + 1] = residual((long long)(m0 + 1) * ldr + o);
                         }
                     }
                 }
@@ -304,8 +330,9 @@ __device__ __forceinline__ void gemv_finisher(const Params& p, Ctrl* c, uint8_t*
                     if (swi && !(g & 1)) {
                         gate[e] = y;
                     } else if (o < o1 && m < M) {
-                        store1(outp, (long long)m * ldo + o, odt,
-                               swi ? gate[e] * sigmoidf_(gate[e]) * y : apply_act(act, y + bias_v[e >> 1]) + res_v[e]);
+                        const float r = swi ? gate[e] * sigmoidf_(gate[e]) * y : apply_act(act, y + bias_v[e >> 1]) + res_v[e];
+                        if (direct_out) store1_direct(reinterpret_cast<float*>(outp) + (long long)m * ldo + o, r);
+                        else store1(outp, (long long)m * ldo + o, odt, r);
                     }
                 }
             }

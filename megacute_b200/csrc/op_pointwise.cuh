@@ -319,7 +319,7 @@ static __device__ __noinline__ void op_rope_append(const mk_op_desc* op, int a0)
 // examples/llama/llama1b.py:103-104).  An index outside the table reads row 0.
 // ptr 0 table (bf16), 1 ids (int32 column), 2 out; i 0 rows, 1 cols, 2 table rows, 3 out dtype
 // args: 0 row tile (8 rows, one per warp), 1 col tile (kEwCols)
-static __device__ __noinline__ void op_gather(const mk_op_desc* op, int a0, int a1) {
+static __device__ __noinline__ void op_gather(const mk_op_desc* op, int a0, int a1, long long direct_off) {
     const int R = op->i[0], Cc = op->i[1], T = op->i[2], odt = op->i[3];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int r = a0 * kComputeWarps + warp;
@@ -331,7 +331,13 @@ static __device__ __noinline__ void op_gather(const mk_op_desc* op, int a0, int 
     for (int v = lane; v < (cols >> 3); v += 32) {
         float f[8];
         load8(row, c0 + v * 8, DT_BF16, f);
-        store8(reinterpret_cast<void*>(op->ptr[2]), (long long)r * op->ld[2] + c0 + v * 8, odt, f);
+        const long long e = (long long)r * op->ld[2] + c0 + v * 8;
+        if (op->flags & MK_F_DIRECT_OUT) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) store1_direct(reinterpret_cast<float*>(op->ptr[2] + direct_off) + e + j, f[j]);
+        } else {
+            store8(reinterpret_cast<void*>(op->ptr[2]), e, odt, f);
+        }
     }
 }
 

@@ -17,6 +17,9 @@ namespace mk {
 // (this op waits for its own dependencies and publishes its own arrivals; returns -1 when aborting)
 __device__ int mk_op_gemv_units(const Params& p, const mk_op_desc* op, int o0, int o1, int seq, int packed_pos, int nwait,
                                 int wait_off, int narrive, int arrive_off);
+// (the same when x is a direct operand)
+__device__ int mk_op_gemv_direct(const Params& p, const mk_op_desc* op, int o0, int o1, int seq, int packed_pos, int nwait,
+                                 int wait_off, int narrive, int arrive_off);
 // body of the finisher warp (op_gemv_mma.cuh): runs until the CTA's instruction list ends
 __device__ void mk_gemv_finisher(const Params& p);
 __device__ int mk_op_gemv_general(const Params& p, const mk_op_desc* op, int o0, int o1, int seq, int packed_pos);
@@ -50,7 +53,7 @@ __device__ bool mk_op_decode_bulk(const Params& p, const mk_op_desc* op, int b, 
 __device__ int mk_run_eltwise(const Params& p, const mk_op_desc* op, int idx, int slot);
 __device__ int mk_run_norm(const Params& p, const mk_op_desc* op, int idx, int slot);
 // finalize / norm of one row / rope_append / increment / gather / argmax; returns false for an unknown kind
-__device__ bool mk_op_pointwise(const mk_op_desc* op, int a0, int a1);
+__device__ bool mk_op_pointwise(const mk_op_desc* op, int a0, int a1, long long direct_off);
 
 struct SmemMap {
     uint8_t* ring;

@@ -8,6 +8,7 @@ and reads shapes, strides, flags and operand addresses from this table at run ti
 ``fill(desc, op, addr, sm_count)`` writes the fields; ``addr(view)`` returns the device byte address of the
 view's first element.  Field meaning per kind (the kernel side repeats it next to the reader):
 
+  (flags 8, 16, 32 of GEMV, DECODE_ATTN and GATHER: direct input, output, residual -- include/megacute_b200.h)
   GEMV         ptr x, w, out, bias, residual, norm gain; i M, N_out, K, act, x dtype, out dtype,
                residual dtype; f eps; flags 1 = swiglu, 2 = rms-normalise x, 4 = tensor-core streaming path
   GEMM         ptr x, w, out, bias, residual, gate, cos, sin; i M, N (weight rows), K, act, splits, out dtype,
@@ -93,8 +94,9 @@ def gemv_units(op: Op) -> bool:
     return op.x.cols % 16 == 0
 
 
-def fill(d, op: Op, addr, sm_count: int) -> None:
-    """Write op's descriptor, as scheduled for ``sm_count`` SMs, into ``d`` (an ``_lib.OpDesc``)."""
+def fill(d, op: Op, addr, sm_count: int, direct=frozenset()) -> None:
+    """Write op's descriptor, as scheduled for ``sm_count`` SMs, into ``d`` (an ``_lib.OpDesc``).  ``direct``: ids of the
+    direct buffers (passes.direct_buffers)."""
     ptrs: list = []
     ints: list = []
     d.flags = 0
@@ -181,6 +183,14 @@ def fill(d, op: Op, addr, sm_count: int) -> None:
         ints = [op.x.rows, op.x.cols, op.chunks, argmax_chunk_cols(op.x.cols, op.chunks), dt(op.x)]
     else:
         raise NotImplementedError(k)
+    if direct:
+        flag = lambda v, bit: bit if v is not None and v.buf.id in direct else 0
+        if k == "Linear" and is_gemv(op):
+            d.flags |= flag(op.x, C.F_DIRECT_IN) | flag(op.out, C.F_DIRECT_OUT) | flag(op.residual, C.F_DIRECT_RES)
+        elif k == "DecodeAttention":
+            d.flags |= flag(op.q, C.F_DIRECT_IN) | flag(op.out, C.F_DIRECT_OUT)
+        elif k == "Gather":
+            d.flags |= flag(op.out, C.F_DIRECT_OUT)
     for n, v in enumerate(ints):
         d.i[n] = int(v)
     for n, v in enumerate(ptrs):

@@ -576,6 +576,43 @@ def fuse_rope_linear(g: Graph) -> Graph:
     return out
 
 
+def direct_buffers(g: Graph) -> frozenset:
+    """Ids of the runtime-private fp32 buffers that need no dependency counters because their readers look at the values
+    themselves (csrc/mk_device.cuh: direct operands): written whole by one op that can mark its stores -- a streaming linear, the
+    per-head decode attention, an embedding gather -- and read only by ops that can wait for values: streaming linears (x,
+    residual) and the per-head decode attention (q, k_new, v_new).  In a step of few rows that is every hop but those through
+    a K-split linear."""
+    from .encode import gemv_units
+    streaming = lambda op: op.kind == "Linear" and gemv_eligible(op.x.rows, op.x.cols) and gemv_units(op)
+    per_head = lambda op: op.kind == "DecodeAttention" and not op.bulk and not op.zero_inputs
+    users: dict[int, list] = {}
+    for k, op in enumerate(g.ops):
+        for name, v in op.view_fields():
+            users.setdefault(v.buf.id, []).append((k, op, name, v))
+    outs = {v.buf.id for v in g.outputs}
+    direct = set()
+    for b in g.buffers:
+        if b.kind != "temp" or b.dtype != torch.float32 or b.id in outs or b.id not in users:
+            continue
+        writers = [u for u in users[b.id] if any(v.buf is b for v in u[1].writes) and u[2] in ("out", "ws")]
+        readers = [u for u in users[b.id] if u not in writers]
+        if len(writers) != 1 or not readers or any(v.buf is b for v in writers[0][1].reads):
+            continue
+        k, op, name, v = writers[0]
+        ok = name == "out" and v.rect == (0, b.rows, 0, b.cols) and (streaming(op) or per_head(op) or op.kind == "Gather")
+        for j, r, field, _ in readers:
+            ok = ok and j > k and not any(w.buf is b for w in r.writes) and (
+                (streaming(r) and field in ("x", "residual"))
+                or (per_head(r) and r.k_new is not None and field in ("q", "k_new", "v_new") and r.q.buf is r.k_new.buf is r.v_new.buf))
+        if ok:
+            direct.add(b)
+    # (one narrow hop alone gains nothing -- two linears of 256 to 1024 take 14.7 us either way, of 2048 16.4 and 16.3, of 4096 24.9 and
+    # 23.1 -- and keeps its counters; a model of 256 columns and eight layers 225 and 210)
+    if len(direct) == 1 and all(b.cols < C.DIRECT_MIN_COLS for b in direct):
+        return frozenset()
+    return frozenset(b.id for b in direct)
+
+
 HOIST_MIN_OPS = 4
 
 

@@ -24,7 +24,7 @@ import torch
 from . import _lib, config as C, encode
 from .graph import ELEM_BYTES, Graph
 from .layers import merge_layers
-from .passes import run_all
+from .passes import direct_buffers, run_all
 from .schedule import schedule
 
 
@@ -55,7 +55,8 @@ class Program:
         self.g = run_all(g, self.sm_count)
         for op in self.g.ops:
             encode.validate(op)
-        self.sched = schedule(self.g, self.sm_count)
+        self.direct = direct_buffers(self.g)
+        self.sched = schedule(self.g, self.sm_count, self.direct)
         if self.debug or os.environ.get("MEGACUTE_B200_VERIFY") == "1":
             # exact host checks of the tables (see verify.py); the happens-before closure keeps
             # n^2 / 8 bytes, so very long instruction streams (full prefill) get the table check only
@@ -73,6 +74,8 @@ class Program:
         self.epoch = 0
         self._handle = None
         self._bufs: dict[int, torch.Tensor] = {}
+        self._direct_mem = None                            # two copies of the direct buffers, which launches use in turn
+        self._direct_turn = 0                              # ... the one the next launch uses
         self._desc = (_lib.OpDesc * max(1, len(self.g.ops)))()
         self._desc_key = None
         self._ops_of_buf: dict[int, list[int]] = {}        # buffer id -> ops with an operand in it
@@ -117,7 +120,10 @@ class Program:
 
     # ---- buffers
     def buffer(self, buf) -> torch.Tensor:
-        return self._bufs[buf.id]
+        t = self._bufs[buf.id]
+        if buf.id in self.direct and self._direct_turn == 0:         # (the latest launch used the second copy, or there was none)
+            t = self._direct_mem.view(-1)[self._direct_mem.shape[1] + t.storage_offset():][:t.numel()].view(t.shape)
+        return t
 
     def _bind(self, bindings: dict):
         dev = torch.device("cuda", self.device)
@@ -130,6 +136,14 @@ class Program:
                 raise ValueError(f"'{b.name}': expected contiguous {dev} {b.dtype} {(b.rows, b.cols)}, "
                                  f"got {t.device} {t.dtype} {tuple(t.shape)}")
             self._bufs[b.id] = t
+        if self.direct and self._direct_mem is None:
+            size = lambda b: -(-b.rows * b.cols // 64) * 64
+            mine = [b for b in self.g.buffers if b.id in self.direct]
+            self._direct_mem = torch.empty(2, sum(size(b) for b in mine), dtype=torch.float32, device=dev)
+            at = 0
+            for b in mine:
+                self._bufs[b.id] = self._direct_mem[0, at:at + b.rows * b.cols].view(b.rows, b.cols)
+                at += size(b)
         for b in self.g.buffers:
             if b.id in self._bufs:
                 continue
@@ -168,8 +182,12 @@ class Program:
         else:
             moved = {i for i, a in ptrs.items() if old[0].get(i) != a}
             todo = sorted({k for i in moved for k in self._ops_of_buf.get(i, ())})
+        if old is None and self._direct_mem is not None:
+            _lib.check(_lib.load().mk_program_set_direct(self._handle, self._direct_mem.data_ptr(), self._direct_mem.shape[1] * 4, stream),
+                       "mk_program_set_direct")
+            self._direct_turn = 0
         for k in todo:
-            encode.fill(self._desc[k], self.g.ops[k], self._addr, self.sm_count)
+            encode.fill(self._desc[k], self.g.ops[k], self._addr, self.sm_count, self.direct)
         _lib.check(_lib.load().mk_program_set_ops(self._handle, ctypes.addressof(self._desc), len(self.g.ops), stream),
                    "mk_program_set_ops")
         self._desc_key = (ptrs, vers)
@@ -186,6 +204,7 @@ class Program:
             _lib.check(lib.mk_program_clear_trace(self._handle, stream))
         _lib.check(lib.mk_launch(self._handle, stream), "mk_launch")
         self.epoch = lib.mk_program_epoch(self._handle)
+        self._direct_turn ^= 1
         if self.debug:
             self.check()
         outs = [self._bufs[v.buf.id].as_strided(v.shape, (v.buf.cols, 1), v.row0 * v.buf.cols + v.col0)
@@ -242,6 +261,7 @@ class Program:
             if b.kind == "workspace" and b.id in self._bufs:
                 self._bufs[b.id].zero_()
         self.epoch = 0
+        self._direct_turn = 0
 
     def set_timeout(self, seconds: float):
         _lib.check(_lib.load().mk_program_set_timeout(self._handle, int(seconds * 1e9)))

@@ -19,6 +19,8 @@ Schedule.encode :249-271) with a different construction:
 4. All consumers that need the same set of producer instructions share one counter: the members
    arrive on it (release add), the consumers wait until it reaches ``len(members) * epoch``
    (acquire load).  Counters are never reset between launches.
+5. Direct buffers (``passes.direct_buffers``) have one writer per launch and readers that look at the values: they get
+   neither counters nor waits; which instructions a reader waits for in that way is kept for the host checks.
 """
 
 from __future__ import annotations
@@ -392,6 +394,7 @@ class Schedule:
     arr_cnt: np.ndarray
     num_counters: int
     counter_target: np.ndarray          # [num_counters] arrivals per launch
+    value_deps: dict                    # instruction -> arrays of the instructions whose results it waits for by value (direct buffers)
 
     @property
     def insts(self):
@@ -418,7 +421,7 @@ class Schedule:
         return "\n".join(lines)
 
 
-def schedule(g: Graph, sm_count: int = 148) -> Schedule:
+def schedule(g: Graph, sm_count: int = 148, direct=frozenset()) -> Schedule:
     tiled = [tile_op(op, sm_count) for op in g.ops]
     starts = np.concatenate([[0], np.cumsum([len(t.args) for t in tiled])]).astype(np.int64)
     n = int(starts[-1])
@@ -430,12 +433,25 @@ def schedule(g: Graph, sm_count: int = 148) -> Schedule:
     counter_key: dict[tuple, int] = {}
     counter_members: list[np.ndarray] = []        # global instruction ids
     waits_of = [[] for _ in range(n)]             # per instruction: [(counter, target)]
+    value_deps: dict[int, list] = {}
 
     for kb, tb in enumerate(tiled):
         nb = len(tb.args)
         dep: dict[int, np.ndarray] = {}           # producer op -> [nb, na] bool
         for acc in tb.accesses:
             if acc.buf.kind in ("input", "param"):
+                continue
+            if acc.buf.id in direct:                  # (one writer, before its readers: passes.direct_buffers)
+                if acc.kind == READ:
+                    (ka, ra), = records[acc.buf.id]
+                    o = _overlap(acc.boxes, ra.boxes)
+                    if (o == o[0]).all():
+                        members = np.nonzero(o[0])[0] + node_ranges[ka][0]
+                        per_inst = [members] * nb
+                    else:
+                        per_inst = [np.nonzero(row)[0] + node_ranges[ka][0] for row in o]
+                    for i, members in enumerate(per_inst):
+                        value_deps.setdefault(node_ranges[kb][0] + i, []).append(members)
                 continue
             ordered: set = set()
             need = CONFLICTS[acc.kind]
@@ -474,7 +490,7 @@ def schedule(g: Graph, sm_count: int = 148) -> Schedule:
                 for r in rows:
                     waits_of[b0 + r].append((c, len(members)))
         for acc in tb.accesses:
-            if acc.buf.kind not in ("input", "param"):
+            if acc.buf.kind not in ("input", "param") and not (acc.buf.id in direct and acc.kind == READ):
                 records.setdefault(acc.buf.id, []).append((kb, acc))
 
     wait_ptr = np.zeros(n + 1, np.int64)
@@ -491,4 +507,4 @@ def schedule(g: Graph, sm_count: int = 148) -> Schedule:
     arr_cnt = np.array([c for a in arr_lists for c in a], np.int64)
     target = np.array([len(m) for m in counter_members], np.int64)
     return Schedule(g, sm_count, n, op_of, args, node_ranges, wait_ptr, wait_cnt, wait_tgt, arr_ptr, arr_cnt,
-                    len(counter_members), target)
+                    len(counter_members), target, value_deps)

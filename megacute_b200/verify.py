@@ -17,7 +17,7 @@ them.  Both are properties of the tables, so both are decided here, on the host,
     Happens-before closure over the encoded wait / arrival tables.  Instruction j happens before i
     when the same CTA runs j earlier (CTA c runs c, c + grid, ... in order), or i waits on a counter
     that j arrives on (a wait's target is the number of arrivals on that counter, so it waits for
-    all of them), transitively.  Every pair of instructions of different ops whose accesses
+    all of them), or i looks at values of a direct buffer until j has written them, transitively.  Every pair of instructions of different ops whose accesses
     conflict (read/write, write/write, accumulate/read-or-write on intersecting rectangles of one
     buffer) must be so ordered, earlier program position first.  Exact: no sampling of executions.
     The instructions of one op run in no order at all: one of them may not write what another reads (ops whose
@@ -213,6 +213,7 @@ def happens_before(s: Schedule) -> np.ndarray:
     for i in range(n):
         for c in s.arr_cnt[s.arr_ptr[i]:s.arr_ptr[i + 1]]:
             members[int(c)].append(i)
+    behind_values: dict[int, np.ndarray] = {}                    # the same per array of value_deps (shared by an op's instructions)
     behind_counter: dict[int, np.ndarray] = {}                   # counter -> everything that happens before its last arrival
     for i in range(n):
         row = reach[i]
@@ -236,6 +237,18 @@ def happens_before(s: Schedule) -> np.ndarray:
                     byte, m = bit(j)
                     acc[byte] |= m
                 behind_counter[c] = acc
+            row |= acc
+        for mem in s.value_deps.get(i, ()):
+            if len(mem) and int(mem[-1]) >= i:
+                raise VerifyError(f"instruction {i}: looks at values that instruction {int(mem[-1])} writes, which is not earlier in program order")
+            acc = behind_values.get(id(mem))
+            if acc is None:
+                acc = np.zeros(nb, np.uint8)
+                for j in mem:
+                    acc |= reach[int(j)]
+                    byte, m = bit(int(j))
+                    acc[byte] |= m
+                behind_values[id(mem)] = acc
             row |= acc
     return reach
 

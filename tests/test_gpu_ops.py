@@ -387,3 +387,101 @@ def test_argmax_rows(cuda, dtype, rows, cols):
     wide = torch.zeros(rows, cols + 16, device=cuda, dtype=dtype)
     wide[:, :cols] = x
     assert torch.equal(mc.argmax(wide[:, :cols]), want)
+
+
+def _chain(M, widths, residual_every=2):
+    """Streaming linears one behind the other (direct operands: every hop by value), some with a residual from two hops before."""
+    g = mc.Graph()
+    x, t = g.input("x", (M, widths[0])), {"x": rnd((M, widths[0]), 1.0, 1)}
+    hs = [x]
+    for i, n in enumerate(widths[1:]):
+        w = g.param(f"w{i}", (n, widths[i]))
+        t[f"w{i}"] = rnd((n, widths[i]), widths[i] ** -0.5, 10 + i)
+        res = hs[-2] if i % residual_every == 1 and hs[-2].shape == (M, n) else None
+        hs.append(g.linear(hs[-1], w, residual=res))
+    g.output(hs[-1])
+    return g, t, hs
+
+
+@pytest.mark.parametrize("M,widths", [(1, [256, 2048, 256, 2048, 256]), (2, [512, 2064, 512, 2064, 512, 16]), (8, [1040, 1024, 1040, 1024, 1040]),
+                                      (5, [2048, 2048, 2048, 2048, 48, 2048]), (1, [8208, 48, 8208, 48])])
+def test_values_instead_of_counters(cuda, M, widths):
+    """Rows of one to many vectors per thread, K that is no multiple of 2048, fewer outputs than SMs, residuals by value; launch after launch
+    with another input each, so that both copies of the buffers are used and filled again."""
+    g, t, hs = _chain(M, widths)
+    prog = mc.compile(g)
+    assert len(prog.direct) == len(widths) - 2 and len(prog.sched.wait_cnt) == 0
+    dev = {k: v.to(cuda) for k, v in t.items()}
+    for step in range(5):
+        dev["x"].copy_(rnd((M, widths[0]), 1.0, 50 + step))
+        out = prog(**dev).float()
+        ref, _ = evaluate(g, dev, cuda)
+        prog.check()
+        assert rel_l2(out, ref[0]) < TOL, step
+        # the buffers hold this launch's values
+        last = next(b for b in prog.g.buffers if b.id in prog.direct and b.name == hs[-2].buf.name)
+        assert not bool((prog.buffer(last).view(torch.int32) == -1).any())
+
+
+def test_values_that_are_nan_end_the_wait(cuda):
+    """NaN inputs, the one with all bits set among them, reach the output as NaN; the rows beside them and the launches after are right."""
+    g, t, _ = _chain(2, [512, 2048, 512, 2048, 512])
+    prog = mc.compile(g)
+    dev = {k: v.to(cuda) for k, v in t.items()}
+    clean = prog(**dev).clone()
+    x = dev["x"].clone()
+    dev["x"].view(torch.int16)[1, 100:104] = -1                      # bf16 0xffff
+    out = prog(**dev)
+    prog.check()
+    assert torch.equal(out[0], clean[0]) and bool(out[1].isnan().all())
+    dev["x"].copy_(x)
+    for _ in range(2):
+        assert torch.equal(prog(**dev), clean)
+
+
+def test_values_that_never_come_end_the_launch(cuda):
+    """A launch whose first op cannot start (a wait that cannot end) ends for the ops behind it too, which wait for values; the program gives
+    the same result after a reset."""
+    from megacute_b200 import _lib
+    g = mc.Graph()
+    x = g.input("x", (2, 512))
+    t = {"x": rnd((2, 512), 1.0, 1)}
+    h = g.unary(x, "silu")
+    for i in range(4):
+        t[f"w{i}"] = rnd((512, 512), 0.05, 2 + i)
+        h = g.linear(h, g.param(f"w{i}", (512, 512)))
+    g.output(h)
+    prog = mc.compile(g)
+    assert len(prog.direct) == 3 and len(prog.sched.wait_cnt) > 0
+    dev = {k: v.to(cuda) for k, v in t.items()}
+    want = prog(**dev).clone()
+    prog.check()
+    s = prog.sched
+    prog.set_timeout(0.02)
+    _lib.check(_lib.load().mk_program_poke_wait(prog._handle, 0, int(s.wait_cnt[0]), 1000))
+    prog(**dev)
+    with pytest.raises(_lib.MegakernelTimeout):
+        prog.check()
+    _lib.check(_lib.load().mk_program_poke_wait(prog._handle, 0, int(s.wait_cnt[0]), int(s.wait_tgt[0])))
+    prog.reset()
+    for _ in range(3):
+        assert torch.equal(prog(**dev), want)
+    prog.check()
+
+
+def test_direct_operands_are_checked_at_bind_time(cuda):
+    """A direct operand without memory for it, or of another type, is refused as the descriptors are bound."""
+    import ctypes
+    from megacute_b200 import _lib
+    g = mc.Graph()
+    g.output(g.linear(g.input("x", (1, 256)), g.param("w", (256, 256))))
+    t = {"x": rnd((1, 256), 1.0, 1).to(cuda), "w": rnd((256, 256), 0.05, 2).to(cuda)}
+    prog = mc.compile(g)
+    want = prog(**t).clone()
+    lib = _lib.load()
+    for flag in (8, 16, 32):
+        prog._desc[0].flags |= flag
+        assert lib.mk_program_set_ops(prog._handle, ctypes.addressof(prog._desc), 1, None) == -2
+        assert b"direct operands" in lib.mk_last_cuda_error()
+        prog._desc[0].flags &= ~flag
+    assert torch.equal(prog(**t), want)

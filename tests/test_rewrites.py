@@ -195,3 +195,41 @@ def test_verifier_rejects_an_op_that_overwrites_its_own_operand():
     g.linear(x, g.param("w", (256, 256)), out=x)
     with pytest.raises(VerifyError, match="with nothing between them"):
         check_hazards(schedule(g, SMS), g)
+
+
+def test_direct_buffers_and_their_schedule():
+    """Which buffers need no counters, and that the tables without them still order every hazard (the values' own order counted)."""
+    from megacute_b200.builders import llama_decode, mlp_block
+    from megacute_b200.passes import direct_buffers, run_all
+    for B, ragged, per_layer in ((1, False, 5), (2, True, 5), (5, True, 2), (16, False, 0)):        # (5 rows: the down projection is a K split)
+        g = run_all(llama_decode(B, 2048, 32, 8, 8192, 2, 256, 4096, 1e-5, ragged=ragged), 148)
+        direct = direct_buffers(g)
+        assert len(direct) == 2 * per_layer
+        s, plain = schedule(g, 148, direct), schedule(g, 148)
+        check_tables(g, s)
+        assert check_hazards(s, g) == check_hazards(plain, g)
+        assert bool(s.value_deps) == bool(direct) and (len(s.wait_cnt) < len(plain.wait_cnt)) == bool(direct)
+        if direct:                                      # without the values' order the same tables are refused
+            s.value_deps = {}
+            with pytest.raises(VerifyError):
+                check_hazards(s, g)
+    assert len(direct_buffers(run_all(mlp_block(1, 2048, 5632), 148))) == 1
+    assert not direct_buffers(run_all(mlp_block(1, 512, 512), 148))                                 # (a narrow hop alone)
+    # read by an op that cannot wait for values; visible to the caller; read in 16 bits; written in part
+    for case in ("unary", "output", "rows", "part"):
+        g = mc.Graph()
+        x, w = g.input("x", (16 if case == "rows" else 1, 2048)), g.param("w", (4096, 2048))
+        v = g.param("v", (2048, 4096))
+        if case == "part":
+            h = g.temp((1, 8192))
+            g.linear(x, w, out=h.cols_slice(0, 4096))
+            g.linear(x, w, out=h.cols_slice(4096, 4096))
+            g.output(g.linear(h.cols_slice(0, 4096), v))
+        else:
+            h = g.linear(x, w)
+            g.output(g.linear(h, v))
+            if case == "unary":
+                g.output(g.unary(h, "relu"))
+            if case == "output":
+                g.output(h)
+        assert not direct_buffers(run_all(g, 148)), case
