@@ -57,6 +57,19 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
     const bool fused = op->i[6] != 0;
     const int G = H / KVH;
     const int b = a0, kvh = a1, s = a2;
+    // one thread per 8-wide chunk of q, of the new token's k (fused, last split) and of its v; direct ones are asked for first of all
+    const int chunk = t / CPR, which = chunk - G;                         // < 0: q, 0: k, 1: v
+    const int pd = dp < CPR / 2 ? dp * 8 + D / 2 : dp * 8 - D / 2;       // partner chunk of the rotation
+    const bool direct = op->flags & MK_F_DIRECT_IN;
+    const bool mine = chunk < G || (fused && s == S - 1 && chunk < G + 2), rot = fused && which != 1;       // (v is not rotated)
+    const float* direct_at = reinterpret_cast<const float*>((which < 0 ? op->ptr[0] : op->ptr[5 + (which & 1)]) + p.direct_off) +
+                             (which < 0 ? (long long)b * op->ld[0] + (kvh * G + chunk) * D : (long long)b * op->ld[5 + (which & 1)] + kvh * D);
+    float a[8], o[8];
+    uint32_t top = 0;
+    if (direct && mine) {
+        top = load8_direct(direct_at + dp * 8, a);
+        if (rot) top = max(top, load8_direct(direct_at + pd, o));
+    }
     // one position for the batch, or (i 12: stride) one per sequence; i 13: sliding window, the last `window` tokens
     // -- the new one included -- of the sequence (0: all of them)
     const int pos = reinterpret_cast<const int*>(op->ptr[3])[(long long)b * op->i[12]];
@@ -102,7 +115,6 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
     if (!fused && wait_deps(p, c, nwait, wait_off, seq)) return;
     if (ntiles > 0) issue_tile(0);
     cp_async_commit();
-    const int pd = dp < CPR / 2 ? dp * 8 + half : dp * 8 - half;         // partner chunk of the rotation
     const float sign = dp < CPR / 2 ? -1.f : 1.f;
     float cs[8], sn[8];
     if (fused) {
@@ -122,22 +134,16 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
     // One thread per 8-wide chunk; the new token's k and v take two more chunk rows. ----
     {
         const float qscale = op->f[0] * kLog2e;
-        const int chunk = t / CPR;                                        // 0..G-1 q heads, G k_new, G+1 v_new
-        if (chunk < G || (has_new && chunk < G + 2)) {
-            const int which = chunk - G;                                  // < 0: q
+        if (mine) {
             const void* src = reinterpret_cast<const void*>(which < 0 ? op->ptr[0] : op->ptr[5 + which]);
             const long long e0 = which < 0 ? (long long)b * op->ld[0] + (kvh * G + chunk) * D
                                            : (long long)b * op->ld[5 + which] + kvh * D;
-            float a[8], o[8];
-            const bool rot = fused && which != 1;                         // v is not rotated
-            if (op->flags & MK_F_DIRECT_IN) {
-                const float* at = reinterpret_cast<const float*>(reinterpret_cast<const uint8_t*>(src) + p.direct_off) + e0;
+            if (direct) {
                 DirectWait w;
-                uint32_t top;
-                do {
-                    top = load8_direct(at + dp * 8, a);
-                    if (rot) top = max(top, load8_direct(at + pd, o));
-                } while (top == kUnwritten && w.again(p, c, seq));
+                while (top == kUnwritten && w.again(p, c, seq)) {
+                    top = load8_direct(direct_at + dp * 8, a);
+                    if (rot) top = max(top, load8_direct(direct_at + pd, o));
+                }
             } else {
                 load8(src, e0 + dp * 8, qdt, a);
                 if (rot) load8(src, e0 + pd, qdt, o);
