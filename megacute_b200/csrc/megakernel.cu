@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
                     break;
                 case MK_OP_GEMM:
                     // (runs this instruction and the CTA's following ones for as long as they are the body's own: walk.cuh)
-                    run_last = is_wide_gemm(op) ? mk_run_gemm_wide(p, idx, slot) : mk_run_gemm(p, idx, slot);
+                    run_last = is_wide_gemm(op) ? mk_run_gemm_wide(p, idx, slot) : op->ptr[11] ? mk_run_gemm(p, idx, slot) : mk_run_gemm_sync(p, idx, slot);
                     break;
                 case MK_OP_ELTWISE: run_last = mk_run_eltwise(p, op, idx, slot); break;
                 case MK_OP_ATTENTION:

@@ -28,6 +28,8 @@ __device__ int mk_op_gemv_general(const Params& p, const mk_op_desc* op, int o0,
 // arrivals of each itself (begin_op says why).  Returns the index of the last instruction executed, -1 when the CTA is
 // aborting.  (The ring position is untouched: the weight tiles have slots of their own.)
 __device__ int mk_run_gemm(const Params& p, int idx, int slot);
+// (the same for ops without tensor maps: mma.sync body)
+__device__ int mk_run_gemm_sync(const Params& p, int idx, int slot);
 // (abort path: its activation tiles still in flight have landed)
 __device__ void mk_gemm_landed();
 // (the same with output tiles of 256 rows; only for ops the host library bound to the tcgen05 body)
