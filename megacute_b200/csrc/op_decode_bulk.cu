@@ -5,11 +5,11 @@
 #include "ops.cuh"
 
 namespace mk {
+// Waits for its own dependencies and publishes its own arrivals.  Returns whether the CTA is aborting.
 __device__ bool mk_op_decode_bulk(const Params& p, const mk_op_desc* op, int b, int s, int nwait, int wait_off, int seq,
                                   int narrive, int arrive_off) {
     const SmemMap m = smem_map();
-    const int G = op->i[1] / op->i[2];
-    if (G <= 4) return op_decode_bulk<4>(p, m.ctrl, op, b, s, m.ring, nwait, wait_off, seq, narrive, arrive_off);
-    return op_decode_bulk<8>(p, m.ctrl, op, b, s, m.ring, nwait, wait_off, seq, narrive, arrive_off);
+    decode_bulk_body(p, m.ctrl, op, b, s, m.ring, nwait, wait_off, seq);
+    return publish(p, m.ctrl, narrive, arrive_off);
 }
 }  // namespace mk

@@ -63,12 +63,11 @@ struct KvPos {
 
 // ---- compute warps ----
 // All compute threads call this.  Returns after the instruction's global writes (the caller publishes).
-template <int GMAX>
+// (G <= 8 query heads per kv head: heads take rows 0..7 of the A operand, their low parts rows 8..15)
 __device__ __forceinline__ void decode_bulk_body(const Params& p, Ctrl* c, const mk_op_desc* op, int b, int s, uint8_t* ring,
                                                  int nwait, int wait_off, int seq) {
     constexpr int D = 64;
     constexpr float NEG_INF = -__builtin_huge_valf();
-    static_assert(GMAX <= 8, "heads take rows 0..7 of the A operand, their low parts rows 8..15");
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const int g = lane >> 2, q4 = lane & 3;                           // MMA row / column group of this lane
     const int H = op->i[1], KVH = op->i[2], L = op->i[4], S = op->i[5], qdt = op->i[7], odt = op->i[8];
@@ -382,14 +381,6 @@ __device__ __forceinline__ void decode_bulk_body(const Params& p, Ctrl* c, const
         store8(outp, oe + 8, odt, acc + 8);
     }
     zero_inputs();
-}
-
-// Waits for its own dependencies and publishes its own arrivals.  Returns whether the CTA is aborting.
-template <int GMAX>
-static __device__ __noinline__ bool op_decode_bulk(const Params& p, Ctrl* c, const mk_op_desc* op, int b, int s, uint8_t* ring,
-                                                   int nwait, int wait_off, int seq, int narrive, int arrive_off) {
-    decode_bulk_body<GMAX>(p, c, op, b, s, ring, nwait, wait_off, seq);
-    return publish(p, c, narrive, arrive_off);
 }
 
 }  // namespace mk
