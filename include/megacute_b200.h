@@ -195,7 +195,10 @@ void mk_program_destroy(mk_program* p);
  * on entry, as for mk_launch.  The wait and arrival tables are device memory the library cannot read:
  * every counter id in them must be below n_counters (mk_program_create checks this for its host
  * tables; here it is the caller's precondition).  grid must not exceed the device's SM count.  The
- * caller's current device is unchanged on return. */
+ * caller's current device is unchanged on return.  Direct operands (mk_program_set_direct) work here too, in the
+ * one copy that the descriptors address: a small kernel before the launch marks the direct outputs that the
+ * descriptors name as unwritten, another one behind it does so again, so their values cannot be read afterwards.
+ * A program's own memory may be used, by launches that do not overlap with the program's. */
 #define MK_NOALLOC_MAX_COUNTERS 16384
 int mk_launch_noalloc(int device, const int32_t* d_insts, int n_insts, const int32_t* d_waits, int n_waits,
                       const int32_t* d_arrives, int n_arrives, const mk_op_desc* d_ops, int n_ops,

@@ -272,6 +272,28 @@ __global__ void pack_weight_tiles(const __nv_bfloat16* __restrict__ w, long long
     }
 }
 
+// mk_launch_noalloc, before and behind the launch.  Before: counters and status words zero, every direct output (mk_device.cuh) unwritten
+// in the one copy that the descriptors address, whatever a program or a call before has left there -- else a reader finds
+// the values of that call and does not wait.  Behind (n_zero 0): unwritten again, as a program whose memory it is expects the copy
+// of its next launch.  One kernel in place of the memsets of counters and status: the call enqueues as much as without direct operands.
+__global__ void noalloc_ready(int32_t* zero, int n_zero, int32_t* status, const mk_op_desc* __restrict__ ops, int n_ops) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_zero; i += gridDim.x * blockDim.x) zero[i] = 0;
+    if (status && blockIdx.x == 0 && threadIdx.x < MK_ST_WORDS) status[threadIdx.x] = 0;
+    for (int k = blockIdx.x; k < n_ops; k += gridDim.x) {
+        const mk_op_desc* d = ops + k;
+        if (!(d->flags & MK_F_DIRECT_OUT)) continue;
+        int out, cols, dtype;
+        if (d->kind == MK_OP_GEMV && (d->flags & GEMV_F_UNITS)) { out = 2; cols = d->i[1]; dtype = d->i[5]; }
+        else if (d->kind == MK_OP_DECODE_ATTN) { out = 4; cols = d->i[1] * d->i[3]; dtype = d->i[8]; }
+        else if (d->kind == MK_OP_GATHER) { out = 2; cols = d->i[1]; dtype = d->i[3]; }
+        else continue;
+        if (dtype != DT_F32) continue;
+        uint32_t* at = reinterpret_cast<uint32_t*>(d->ptr[out]);
+        for (int r = 0; r < d->i[0]; ++r, at += d->ld[out])
+            for (int e = threadIdx.x; e < cols; e += blockDim.x) at[e] = kUnwritten;
+    }
+}
+
 }  // namespace mk
 
 // =================================================================================================
@@ -955,8 +977,9 @@ extern "C" int mk_launch_noalloc(int device, const int32_t* d_insts, int n_insts
     int32_t* scratch = g_noalloc_ptr[device];
     int32_t* d_status = scratch + MK_NOALLOC_MAX_COUNTERS;
     // the array keeps the previous call's contents: counters and status must start at zero
-    if (n_counters > 0) MK_CUDA(cudaMemsetAsync(scratch, 0, (size_t)n_counters * 4, st));
-    MK_CUDA(cudaMemsetAsync(d_status, 0, MK_ST_WORDS * 4, st));
+    const int ready_blocks = n_ops < 1024 ? n_ops : 1024;
+    mk::noalloc_ready<<<ready_blocks, 256, 0, st>>>(scratch, n_counters, d_status, d_ops, n_ops);
+    MK_CUDA(cudaGetLastError());
     mk::Params prm;
     prm.insts = reinterpret_cast<const int4*>(d_insts);
     prm.n_insts = n_insts;
@@ -974,6 +997,8 @@ extern "C" int mk_launch_noalloc(int device, const int32_t* d_insts, int n_insts
     prm.direct_next = nullptr;
     prm.direct_pieces = 0;
     mk::megakernel<false><<<grid, mk::kThreads, mk::kSmemBytes, st>>>(prm);
+    MK_CUDA(cudaGetLastError());
+    mk::noalloc_ready<<<ready_blocks, 256, 0, st>>>(nullptr, 0, nullptr, d_ops, n_ops);
     MK_CUDA(cudaGetLastError());
     if (status) {
         MK_CUDA(cudaMemcpyAsync(status, d_status, MK_ST_WORDS * 4, cudaMemcpyDeviceToHost, st));

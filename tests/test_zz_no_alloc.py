@@ -70,6 +70,59 @@ def test_noalloc_launch_matches_program_launch(cuda):
         assert torch.equal(out, want)              # same kernel, same order of operations: identical bits
 
 
+@pytest.mark.parametrize("step", [False, True])
+def test_noalloc_runs_direct_operands(cuda, step):
+    """Tables with direct operands (hops by value, no counters: linears, and a decode step with its attention and gather): every call with
+    inputs of its own, in between the program's own launches, which take the same memory in turn.  Each result is that call's."""
+    from megacute_b200 import workloads as W
+    from megacute_b200.builders import llama_decode
+    if step:
+        B, E, H, KVH, F, n, L, V = 2, 256, 4, 2, 512, 2, 256, 1000
+        g = llama_decode(B, E, H, KVH, F, n, L, V, 1e-5, fused_step=True)
+        cos, sin = W.rope_tables(L, E // H)
+        st, _ = W.llama_decode_state(B, E, H, KVH, n, L, 90, V, 1, "cpu")
+        t = dict(cos=cos, sin=sin, **W.llama_weights(E, H, KVH, F, n, V, 0, "cpu"), pos=st["pos"], k_cache=st["k_cache"], v_cache=st["v_cache"],
+                 ids=torch.zeros(B, 1, dtype=torch.int32))
+    else:
+        g, t = _graph(), {k: v.cpu() for k, v in _inputs(cuda).items()}
+    prog = mc.compile(g)
+    dev = {k: t[b.name].to(cuda) for b in prog.g.inputs + prog.g.params + prog.g.states for k in [b.name]}
+    gen = torch.Generator().manual_seed(3)
+
+    def fresh():
+        """this call's inputs, on the host and in the bound tensors -> the oracle's result"""
+        if step:
+            t["ids"] = torch.randint(0, V, (B, 1), generator=gen, dtype=torch.int32)
+        else:
+            t["x"] = torch.randn(1, 512, generator=gen).to(BF)
+        for k in dev:
+            if step and k in ("pos", "ids", "k_cache", "v_cache") or k == "x":
+                dev[k].copy_(t[k])
+        return evaluate(g, {k: t[k] for k in dev})[0][0]
+
+    want = fresh()
+    out = prog(**dev)
+    prog.check()
+    assert rel_l2(out.float().cpu(), want) < TOL and prog.direct and any(d.flags & 56 for d in prog._desc)
+    insts, waits, arrives = (a.to(cuda) for a in prog._tables)
+    desc = torch.frombuffer(bytearray(bytes(prog._desc)), dtype=torch.uint8).to(cuda)
+    lib = _lib.load()
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    status = (ctypes.c_int32 * _lib.ST_WORDS)()
+    s = prog.sched
+    for at, noalloc in enumerate((True, True, False, True, False, False, True, False)):
+        want = fresh()
+        out.zero_()
+        if noalloc:
+            rc = lib.mk_launch_noalloc(cuda.index or 0, insts.data_ptr(), s.n, waits.data_ptr(), len(s.wait_cnt), arrives.data_ptr(),
+                                       len(s.arr_cnt), desc.data_ptr(), len(prog.g.ops), s.num_counters, prog.sm_count, stream, status)
+            _lib.check(rc, f"mk_launch_noalloc call {at}")
+        else:
+            prog(**dev)
+            prog.check()
+        assert rel_l2(out.float().cpu(), want) < TOL, (at, noalloc)
+
+
 def test_noalloc_rejects_oversized_graph(cuda):
     lib = _lib.load()
     dummy = torch.zeros(64, dtype=torch.int32, device=cuda)
