@@ -35,7 +35,10 @@ template <int D>
 constexpr int kDecTileKeys = D <= 64 ? 128 : 64;     // keys per tile; 16 per computing warp
 constexpr int kMaxKvSplits = 32;          // config.py MAX_KV_SPLITS
 
-template <int D, int GMAX>
+// DIRECT: q, k_new and v_new are direct operands (mk_device.cuh).  Functions of their own, so that neither form keeps the other's
+// registers or runs its code: batch 1 at context 1024 742.6 -> 739.7 us, two sequences with head_dim 128 894 -> 890, five ragged ones
+// 1110.0 -> 1107.5; 12 to 31 sequences, which never have direct operands here, the same within 0.25 %.
+template <int D, int GMAX, bool DIRECT>
 __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_op_desc* op, int a0, int a1, int a2,
                                             uint8_t* work, int nwait, int wait_off, int seq) {
     constexpr int ROWB = D * 2 + 16;                   // padded tile row: conflict-free ldmatrix
@@ -60,13 +63,13 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
     // one thread per 8-wide chunk of q, of the new token's k (fused, last split) and of its v; direct ones are asked for first of all
     const int chunk = t / CPR, which = chunk - G;                         // < 0: q, 0: k, 1: v
     const int pd = dp < CPR / 2 ? dp * 8 + D / 2 : dp * 8 - D / 2;       // partner chunk of the rotation
-    const bool direct = op->flags & MK_F_DIRECT_IN;
     const bool mine = chunk < G || (fused && s == S - 1 && chunk < G + 2), rot = fused && which != 1;       // (v is not rotated)
-    const float* direct_at = reinterpret_cast<const float*>((which < 0 ? op->ptr[0] : op->ptr[5 + (which & 1)]) + p.direct_off) +
-                             (which < 0 ? (long long)b * op->ld[0] + (kvh * G + chunk) * D : (long long)b * op->ld[5 + (which & 1)] + kvh * D);
     float a[8], o[8];
+    const float* direct_at = nullptr;
     uint32_t top = 0;
-    if (direct && mine) {
+    if (DIRECT && mine) {
+        direct_at = reinterpret_cast<const float*>((which < 0 ? op->ptr[0] : op->ptr[5 + which]) + p.direct_off) +
+                    (which < 0 ? (long long)b * op->ld[0] + (kvh * G + chunk) * D : (long long)b * op->ld[5 + which] + kvh * D);
         top = load8_direct(direct_at + dp * 8, a);
         if (rot) top = max(top, load8_direct(direct_at + pd, o));
     }
@@ -79,7 +82,6 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
     const int k_begin = min(n, first + s * per), k_end = min(n, k_begin + per);
     const int nk = k_end - k_begin;                                       // cached keys of this split
     const bool has_new = fused && s == S - 1;
-    const int half = D / 2;
 
     uint8_t* kst = work;                                                  // NST K tiles then NST V tiles
     uint8_t* vst = work + NST * TILE_BYTES;
@@ -135,16 +137,16 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
     {
         const float qscale = op->f[0] * kLog2e;
         if (mine) {
-            const void* src = reinterpret_cast<const void*>(which < 0 ? op->ptr[0] : op->ptr[5 + which]);
-            const long long e0 = which < 0 ? (long long)b * op->ld[0] + (kvh * G + chunk) * D
-                                           : (long long)b * op->ld[5 + which] + kvh * D;
-            if (direct) {
+            if (DIRECT) {
                 DirectWait w;
                 while (top == kUnwritten && w.again(p, c, seq)) {
                     top = load8_direct(direct_at + dp * 8, a);
                     if (rot) top = max(top, load8_direct(direct_at + pd, o));
                 }
             } else {
+                const void* src = reinterpret_cast<const void*>(which < 0 ? op->ptr[0] : op->ptr[5 + which]);
+                const long long e0 = which < 0 ? (long long)b * op->ld[0] + (kvh * G + chunk) * D
+                                               : (long long)b * op->ld[5 + which] + kvh * D;
                 load8(src, e0 + dp * 8, qdt, a);
                 if (rot) load8(src, e0 + pd, qdt, o);
             }
@@ -397,23 +399,23 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
 // The op waits for its own dependencies (see decode_body) and publishes its own arrivals, so the
 // arrivals leave before the function's epilogue (callee-saved register restores come out of local
 // memory, an L2 round trip here).  Returns whether the CTA is aborting.
-template <int D, int GMAX>
+template <int D, int GMAX, bool DIRECT>
 static __device__ __noinline__ bool op_decode_attn(const Params& p, Ctrl* c, const mk_op_desc* op, int a0, int a1, int a2,
                                                    uint8_t* work, int nwait, int wait_off, int seq, int narrive,
                                                    int arrive_off) {
-    decode_body<D, GMAX>(p, c, op, a0, a1, a2, work, nwait, wait_off, seq);
+    decode_body<D, GMAX, DIRECT>(p, c, op, a0, a1, a2, work, nwait, wait_off, seq);
     return publish(p, c, narrive, arrive_off);
 }
 
 // i 10 > 1 (unsplit batched decode): kv heads a1 .. a1 + i10 - 1 of the sequence, one after the other;
 // fetch, dependency wait and arrival are paid once per instruction.  A function of its own: in the
 // single-head function the loop's extra live state costs registers (spills are L2 round trips here).
-template <int D, int GMAX>
+template <int D, int GMAX, bool DIRECT>
 static __device__ __noinline__ void decode_one_head(const Params& p, Ctrl* c, const mk_op_desc* op, int a0, int a1, int a2,
                                                     uint8_t* work, int nwait, int wait_off, int seq) {
-    decode_body<D, GMAX>(p, c, op, a0, a1, a2, work, nwait, wait_off, seq);
+    decode_body<D, GMAX, DIRECT>(p, c, op, a0, a1, a2, work, nwait, wait_off, seq);
 }
-template <int D, int GMAX>
+template <int D, int GMAX, bool DIRECT>
 static __device__ __noinline__ bool op_decode_attn_heads(const Params& p, Ctrl* c, const mk_op_desc* op, int a0, int a1, int a2,
                                                          uint8_t* work, int nwait, int wait_off, int seq, int narrive,
                                                          int arrive_off) {
@@ -421,7 +423,7 @@ static __device__ __noinline__ bool op_decode_attn_heads(const Params& p, Ctrl* 
 #pragma unroll 1
     for (int j = 0; j < hp; ++j) {
         if (j) compute_sync();                                  // the previous head's merge reads the tile buffers
-        decode_one_head<D, GMAX>(p, c, op, a0, a1 + j, a2, work, j ? 0 : nwait, wait_off, seq);
+        decode_one_head<D, GMAX, DIRECT>(p, c, op, a0, a1 + j, a2, work, j ? 0 : nwait, wait_off, seq);
         if (*(volatile int*)&c->abort) break;
     }
     return publish(p, c, narrive, arrive_off);

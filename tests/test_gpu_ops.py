@@ -485,3 +485,45 @@ def test_direct_operands_are_checked_at_bind_time(cuda):
         assert b"direct operands" in lib.mk_last_cuda_error()
         prog._desc[0].flags &= ~flag
     assert torch.equal(prog(**t), want)
+
+
+def _gated_decode(B=2, H=8, KVH=2, D=64, L=128, ctx=40):
+    """pointwise op (behind counters) -> QKV -> decode attention -> O: every hop behind the first linear by value."""
+    E = 512
+    g = mc.Graph()
+    x = g.input("x", (B, E))
+    t = {"x": rnd((B, E), 1.0, 1), "wqkv": rnd(((H + 2 * KVH) * D, E), E ** -0.5, 2), "wo": rnd((512, H * D), (H * D) ** -0.5, 3),
+         "pos": torch.full((1, 1), ctx, dtype=torch.int32)}
+    t["cos"], t["sin"] = W.rope_tables(L, D)
+    for i, n in enumerate(("k_cache", "v_cache")):
+        t[n] = rnd((B * L, KVH * D), 1.0, 4 + i)
+    cos, sin, pos = g.input("cos", (L, D)), g.input("sin", (L, D)), g.state("pos", (1, 1), torch.int32)
+    kc, vc = (g.state(n, (B * L, KVH * D)) for n in ("k_cache", "v_cache"))
+    qkv = g.linear(g.unary(x, "silu"), g.param("wqkv", t["wqkv"].shape))
+    q = g.rope_append(qkv, cos, sin, pos, kc, vc, heads=H, kv_heads=KVH, head_dim=D, max_seq=L)
+    a = g.decode_attention(q, kc, vc, pos, heads=H, kv_heads=KVH, head_dim=D, max_seq=L)
+    h = g.linear(a, g.param("wo", t["wo"].shape))
+    t["w2"], t["w3"] = rnd((512, 512), 0.04, 6), rnd((512, 512), 0.04, 7)
+    g.output(g.linear(g.linear(h, g.param("w2", (512, 512))), g.param("w3", (512, 512)), residual=h))
+    return g, t
+
+
+@pytest.mark.parametrize("H,KVH,D,B,ctx", [(8, 2, 128, 2, 40), (8, 1, 128, 1, 200), (8, 1, 64, 3, 40), (4, 4, 128, 8, 0), (16, 2, 64, 1, 127)])
+def test_decode_attention_by_value(cuda, H, KVH, D, B, ctx):
+    """Direct q, k, v and output of the decode attention at both head sizes and groups of 1, 4 and 8, launch after launch with another input."""
+    L = 256
+    g, t = _gated_decode(B, H, KVH, D, L, ctx)
+    prog = mc.compile(g)
+    att = next(o for o in prog.g.ops if o.kind == "DecodeAttention")
+    assert {att.q.buf.id, att.out.buf.id} <= prog.direct and att.k_new is not None
+    dev, ref_t = {k: v.to(cuda) for k, v in t.items()}, dict(t)
+    for step in range(4):
+        ref_t["x"] = rnd((B, 512), 1.0, 30 + step)
+        dev["x"].copy_(ref_t["x"])
+        got = prog(**dev).float().cpu()
+        prog.check()
+        ref, st = evaluate(g, ref_t)
+        assert rel_l2(got, ref[0]) < TOL, step
+        for n in ("k_cache", "v_cache"):
+            ref_t[n] = st[n]
+            assert rel_l2(dev[n].cpu().float(), st[n].float()) < TOL, (step, n)
