@@ -230,6 +230,7 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
     // Abort path only: bulk copies may still be landing in shared memory, and products reading it.  The roles that requested copies
     // wait (bounded) for theirs; a pause then covers what cannot be waited for (a copy takes a few microseconds).
     if (c->abort && (threadIdx.x & 31) == 0) {
+        if (warp == 0 && c->flag < 0) report_direct(p, c, -1 - c->flag);
         if (warp == kFeederWarp) mk_feeder_landed(left);
         if (warp == kProducerWarp) {
             wait_landed(c->full + (left >> 16), (left >> 12) & 15, left);

@@ -139,7 +139,8 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
         if (mine) {
             if (DIRECT) {
                 DirectWait w;
-                while (top == kUnwritten && w.again(p, c, seq)) {
+                while (top == kUnwritten) {
+                    if (!w.again(p, c)) { c->flag = -1 - seq; break; }
                     top = load8_direct(direct_at + dp * 8, a);
                     if (rot) top = max(top, load8_direct(direct_at + pd, o));
                 }
@@ -249,6 +250,9 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
     cp_async_wait<0>();
     if (ntiles == 0) compute_sync();                                      // q and snew visible without the loop's barriers
     phase_mark(p, c, 0);
+    // q, k or v never came: all leave (the word was set before a barrier that every thread has passed), with cache, partial sums
+    // and output untouched
+    if (DIRECT && *(volatile int*)&c->flag < 0) return;
 
     // ---- the new token (fused mode, last split): its score per head from the q parts in shared
     // memory, and its k, v appended to the cache ----

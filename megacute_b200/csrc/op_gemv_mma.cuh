@@ -109,8 +109,10 @@ __device__ __forceinline__ void gemv_mma(const Params& p, Ctrl* c, uint8_t* ring
             for (int v = t; v < nv; v += kComputeThreads) {
                 float f[8], gq[8];
                 if (DIRECT) {
+                    const float* at = reinterpret_cast<const float*>(x) + m * ldx + v * 8;
                     DirectWait w;
-                    while (load8_direct(reinterpret_cast<const float*>(x) + m * ldx + v * 8, f) == kUnwritten && w.again(p, c, seq)) {}
+                    while (load8_direct(at, f) == kUnwritten)
+                        if (!w.again(p, c)) { c->flag = -1 - seq; break; }
                 } else {
                     load8(x, m * ldx + v * 8, xdt, f);
                 }
@@ -212,7 +214,9 @@ __device__ __forceinline__ void gemv_mma(const Params& p, Ctrl* c, uint8_t* ring
         // ---- hand the partial tile to the finisher.  Four slots round-robin; a slot is reused
         // four groups later, once the finisher has freed it (it almost always has). ----
         const int sl = g & 3;
+        const int lost = DIRECT ? *(volatile int*)&c->flag : 0;
         ok = wait_barrier(p, c, &c->slot_free[sl], ((pos.comb >> sl) & 1u) ^ 1u, seq, WHERE_COMBINE) && ok;
+        if (DIRECT && lost < 0) return;                                      // values of x never came (set before the barrier above): nothing is stored
         pos.comb ^= 1u << sl;
         sts_volatile4(&red[sl * (8 * 32) + warp * 32 + lane],
                       make_float4((accs[0][0] + accs[1][0]) + (accs[2][0] + accs[3][0]), (accs[0][1] + accs[1][1]) + (accs[2][1] + accs[3][1]),
@@ -278,8 +282,13 @@ __device__ __forceinline__ void gemv_finisher(const Params& p, Ctrl* c, uint8_t*
         // (a direct residual was written hops ago: not there only when a program's first ops are late)
         auto residual = [&](long long e) {
             if (!direct_res) return load1(resp, e, rdt);
-            const float v = load1_direct(reinterpret_cast<const float*>(resp) + e);
-            return __float_as_uint(v) == kUnwritten ? wait1_direct(p, c, reinterpret_cast<const float*>(resp) + e, seq) : v;
+            const float* at = reinterpret_cast<const float*>(resp) + e;
+            float v = load1_direct(at);
+            if (__float_as_uint(v) == kUnwritten) {
+                v = wait1_direct(p, c, at, seq);
+                if (__float_as_uint(v) == kUnwritten) ok = false;
+            }
+            return v;
         };
 #pragma unroll 1
         for (int g = 0; g < ngroups; ++g) {
@@ -304,7 +313,7 @@ __device__ __forceinline__ void gemv_finisher(const Params& p, Ctrl* c, uint8_t*
             fetch_operands();
             ok = wait_barrier(p, c, &c->slot_full[sl], (fullpar >> sl) & 1u, seq, WHERE_COMBINE) && ok;
             fullpar ^= 1u << sl;
-            if (!ok) return;                                                  // the launch is failing
+            if (!__all_sync(0xffffffffu, ok)) return;                         // the launch is failing (no lane stays behind, or stores the marker)
             if (g == 0) {
                 if (rms && storer) {
 #pragma unroll

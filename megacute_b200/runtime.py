@@ -249,8 +249,11 @@ class Program:
             names = {1: "dependency counter wait timed out", 2: "shared-memory barrier wait timed out",
                      3: "bad instruction", 4: "self-check: a shared-memory barrier is in a state its protocol rules out"}
             exc = _lib.MegakernelTimeout if code in (1, 2) else _lib.MegakernelError
+            detail = f"a={a}, b={b}, c={c}"
+            if code == 1 and a == -1 and 0 <= seq < self.sched.n:       # values in place of a counter
+                detail = f"values of a direct operand of op {self.sched.op_of[seq]} {self.g.ops[self.sched.op_of[seq]].kind}"
             raise exc(f"megakernel: {names.get(code, code)} (cta {cta}, warp {warp}, inst {seq}, where {where}, "
-                      f"a={a}, b={b}, c={c}); call prog.reset() before reusing the program")
+                      f"{detail}); call prog.reset() before reusing the program")
         _lib.check(rc, "mk_program_status")
 
     def reset(self):

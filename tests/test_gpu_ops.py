@@ -508,6 +508,42 @@ def _gated_decode(B=2, H=8, KVH=2, D=64, L=128, ctx=40):
     return g, t
 
 
+def test_wait_for_values_that_ends_leaves_the_callers_tensors_alone(cuda):
+    """The values an attention and the linears behind it wait for never come: the launch ends with the status of a dependency that was not
+    met, nothing made without them is written to the caller's cache and output, and the step after a reset is right."""
+    from megacute_b200 import _lib
+    g, t = _gated_decode()
+    prog = mc.compile(g)
+    assert len(prog.direct) == 4 and len(prog.sched.wait_cnt) > 0
+    dev = {k: v.to(cuda) for k, v in t.items()}
+    s, lib = prog.sched, _lib.load()
+    out = prog(**dev)
+    prog.check()
+    ref, st = evaluate(g, t)
+    for _ in range(3):
+        for k in ("k_cache", "v_cache", "pos"):
+            dev[k].copy_(t[k])
+        out.zero_()
+        prog.set_timeout(0.02)
+        _lib.check(lib.mk_program_poke_wait(prog._handle, 0, int(s.wait_cnt[0]), 1000))
+        prog(**dev)
+        with pytest.raises(_lib.MegakernelTimeout, match="dependency"):
+            prog.check()
+        # the linear that is stuck makes q of the first kv head; other heads may have appended their rows, with their values
+        for k in ("k_cache", "v_cache"):
+            got = dev[k].cpu().float()
+            assert torch.equal(got[:, :64], t[k][:, :64].float())
+            changed = got != t[k].float()
+            assert rel_l2(torch.where(changed, got, st[k].float()), st[k].float()) < TOL
+        assert not out.any()
+        _lib.check(lib.mk_program_poke_wait(prog._handle, 0, int(s.wait_cnt[0]), int(s.wait_tgt[0])))
+        prog.reset()
+        prog.set_timeout(2.0)
+        got = prog(**dev).float().cpu()
+        prog.check()
+        assert rel_l2(got, ref[0]) < TOL and rel_l2(dev["k_cache"].cpu().float(), st["k_cache"].float()) < TOL
+
+
 @pytest.mark.parametrize("H,KVH,D,B,ctx", [(8, 2, 128, 2, 40), (8, 1, 128, 1, 200), (8, 1, 64, 3, 40), (4, 4, 128, 8, 0), (16, 2, 64, 1, 127)])
 def test_decode_attention_by_value(cuda, H, KVH, D, B, ctx):
     """Direct q, k, v and output of the decode attention at both head sizes and groups of 1, 4 and 8, launch after launch with another input."""
