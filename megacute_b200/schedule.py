@@ -394,7 +394,7 @@ class Schedule:
     arr_cnt: np.ndarray
     num_counters: int
     counter_target: np.ndarray          # [num_counters] arrivals per launch
-    value_deps: dict                    # instruction -> arrays of the instructions whose results it waits for by value (direct buffers)
+    value_deps: dict                    # instruction -> [(direct buffer's id, instructions whose results there it waits for by value)]
 
     @property
     def insts(self):
@@ -451,7 +451,7 @@ def schedule(g: Graph, sm_count: int = 148, direct=frozenset()) -> Schedule:
                     else:
                         per_inst = [np.nonzero(row)[0] + node_ranges[ka][0] for row in o]
                     for i, members in enumerate(per_inst):
-                        value_deps.setdefault(node_ranges[kb][0] + i, []).append(members)
+                        value_deps.setdefault(node_ranges[kb][0] + i, []).append((acc.buf.id, members))
                 continue
             ordered: set = set()
             need = CONFLICTS[acc.kind]

@@ -17,9 +17,11 @@ them.  Both are properties of the tables, so both are decided here, on the host,
     Happens-before closure over the encoded wait / arrival tables.  Instruction j happens before i
     when the same CTA runs j earlier (CTA c runs c, c + grid, ... in order), or i waits on a counter
     that j arrives on (a wait's target is the number of arrivals on that counter, so it waits for
-    all of them), or i looks at values of a direct buffer until j has written them, transitively.  Every pair of instructions of different ops whose accesses
+    all of them), transitively.  Every pair of instructions of different ops whose accesses
     conflict (read/write, write/write, accumulate/read-or-write on intersecting rectangles of one
     buffer) must be so ordered, earlier program position first.  Exact: no sampling of executions.
+    A read of a direct buffer is ordered behind the write whose values it waits for, that pair alone: the values are
+    loaded and stored without an order for any other access.
     The instructions of one op run in no order at all: one of them may not write what another reads (ops whose
     instructions coordinate among themselves -- decode attention, argmax -- excepted).
 
@@ -33,7 +35,7 @@ import torch
 
 from . import config as C
 from .graph import Graph
-from .schedule import CONFLICTS, Schedule, _overlap, _rect_hits, ew_rows, finalize_rows, gemm_rows, is_gemv, norm_rows, tile_op
+from .schedule import CONFLICTS, READ, WRITE, Schedule, _overlap, _rect_hits, ew_rows, finalize_rows, gemm_rows, is_gemv, norm_rows, tile_op
 
 
 class VerifyError(AssertionError):
@@ -213,7 +215,6 @@ def happens_before(s: Schedule) -> np.ndarray:
     for i in range(n):
         for c in s.arr_cnt[s.arr_ptr[i]:s.arr_ptr[i + 1]]:
             members[int(c)].append(i)
-    behind_values: dict[int, np.ndarray] = {}                    # the same per array of value_deps (shared by an op's instructions)
     behind_counter: dict[int, np.ndarray] = {}                   # counter -> everything that happens before its last arrival
     for i in range(n):
         row = reach[i]
@@ -238,18 +239,9 @@ def happens_before(s: Schedule) -> np.ndarray:
                     acc[byte] |= m
                 behind_counter[c] = acc
             row |= acc
-        for mem in s.value_deps.get(i, ()):
+        for _, mem in s.value_deps.get(i, ()):
             if len(mem) and int(mem[-1]) >= i:
                 raise VerifyError(f"instruction {i}: looks at values that instruction {int(mem[-1])} writes, which is not earlier in program order")
-            acc = behind_values.get(id(mem))
-            if acc is None:
-                acc = np.zeros(nb, np.uint8)
-                for j in mem:
-                    acc |= reach[int(j)]
-                    byte, m = bit(int(j))
-                    acc[byte] |= m
-                behind_values[id(mem)] = acc
-            row |= acc
     return reach
 
 
@@ -296,6 +288,11 @@ def check_hazards(s: Schedule, g: Graph) -> int:
                 gi, gj = l0 + li, e0 + ei
                 have = (reach[gi, gj >> 3] & (0x80 >> (gj & 7)).astype(np.uint8)) != 0
                 checked += len(gi)
+                if not have.all() and first.kind == WRITE and later.kind == READ:
+                    for i in np.unique(gi[~have]):               # waits for the values themselves?
+                        mem = [m for buf, m in s.value_deps.get(int(i), ()) if buf == first.buf.id]
+                        if mem:
+                            have |= (gi == i) & np.isin(gj, np.concatenate(mem))
                 if not have.all():
                     w = int(np.nonzero(~have)[0][0])
                     raise VerifyError(f"unordered hazard on buffer '{first.buf.name}': instruction {int(gj[w])} (op {lo} "

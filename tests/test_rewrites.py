@@ -233,3 +233,24 @@ def test_direct_buffers_and_their_schedule():
             if case == "output":
                 g.output(h)
         assert not direct_buffers(run_all(g, 148)), case
+
+
+def test_values_order_nothing_but_themselves():
+    """A linear that reads a pointwise op's result beside a direct operand made from it needs its counter: the values it waits for were
+    loaded and stored without an order for other accesses."""
+    from megacute_b200.passes import direct_buffers, run_all
+    g = mc.Graph()
+    u = g.unary(g.input("x", (1, 512)), "silu")
+    h = g.linear(u, g.param("w1", (4096, 512)))
+    g.output(g.linear(h, g.param("w2", (512, 4096)), residual=u))
+    g = run_all(g, SMS)
+    h = g.ops[1].out.buf.id
+    assert [o.kind for o in g.ops] == ["Unary", "Linear", "Linear"] and direct_buffers(g) == {h}
+    s = schedule(g, SMS, direct_buffers(g))
+    check_hazards(s, g)
+    b0 = s.node_ranges[2][0]
+    at = int(s.wait_ptr[b0])
+    assert at < len(s.wait_cnt) and all(buf == h for i in s.value_deps for buf, _ in s.value_deps[i])
+    s.wait_ptr[b0:], s.wait_cnt, s.wait_tgt = at, s.wait_cnt[:at], s.wait_tgt[:at]
+    with pytest.raises(VerifyError, match="unordered hazard"):
+        check_hazards(s, g)
