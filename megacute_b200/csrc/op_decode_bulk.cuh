@@ -353,14 +353,19 @@ __device__ __forceinline__ void decode_bulk_body(const Params& p, Ctrl* c, const
             float m2[2], l2[2];
             float4 v[2][4];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) {                                // (an odd last one twice, the second time with no weight)
+            for (int j = 0; j < 2; ++j) {                                // (an odd last one twice, the second time in place of nothing)
                 const float* row = base + min(k + j, S - 1) * ldp;
                 m2[j] = __ldcg(row + GD + g);
                 l2[j] = __ldcg(row + GD + G + g);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) v[j][e] = __ldcg(reinterpret_cast<const float4*>(row + g * D + q4 * 16 + 4 * e));
             }
-            if (k + 1 == S) m2[1] = NEG_INF;
+            if (k + 1 == S) {                                            // (zeros, not just no weight: its values may be infinite)
+                m2[1] = NEG_INF;
+                l2[1] = 0.f;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[1][e] = make_float4(0.f, 0.f, 0.f, 0.f);
+            }
             const float mnew = fmaxf(mx, fmaxf(m2[0], m2[1]));           // (a split without keys wrote zeros and -inf)
             const float w = mx == NEG_INF ? 0.f : ex2(mx - mnew), w0 = m2[0] == NEG_INF ? 0.f : ex2(m2[0] - mnew),
                         w1 = m2[1] == NEG_INF ? 0.f : ex2(m2[1] - mnew);

@@ -563,3 +563,25 @@ def test_decode_attention_by_value(cuda, H, KVH, D, B, ctx):
         for n in ("k_cache", "v_cache"):
             ref_t[n] = st[n]
             assert rel_l2(dev[n].cpu().float(), st[n].float()) < TOL, (step, n)
+
+
+@pytest.mark.parametrize("splits", [1, 2, 3, 5])
+def test_many_sequence_attention_with_infinite_values(cuda, monkeypatch, splits):
+    """Infinite elements of the new token's v reach the output as they are, whatever the number of splits (the last one merges them in pairs)."""
+    monkeypatch.setenv("MEGACUTE_B200_ATT_BULK", "1")
+    monkeypatch.setenv("MEGACUTE_B200_KV_SPLITS", str(splits))
+    B, H, KVH, D, L, ctx = 12, 16, 4, 64, 1024, 960                   # (whole tiles in every split)
+    g = mc.Graph()
+    x = rnd((B, (H + 2 * KVH) * D), 1.0, 1)
+    x[:, (H + KVH) * D + 5], x[:, (H + KVH) * D + 6] = float("inf"), -float("inf")
+    t = {"qkv": x, "pos": torch.full((1, 1), ctx, dtype=torch.int32), "k_cache": rnd((B * L, KVH * D), 1.0, 2), "v_cache": rnd((B * L, KVH * D), 1.0, 3)}
+    t["cos"], t["sin"] = W.rope_tables(L, D)
+    pos, kc, vc = g.state("pos", (1, 1), torch.int32), g.state("k_cache", (B * L, KVH * D)), g.state("v_cache", (B * L, KVH * D))
+    q = g.rope_append(g.input("qkv", x.shape), g.input("cos", (L, D)), g.input("sin", (L, D)), pos, kc, vc, heads=H, kv_heads=KVH, head_dim=D, max_seq=L)
+    g.output(g.decode_attention(q, kc, vc, pos, heads=H, kv_heads=KVH, head_dim=D, max_seq=L))
+    outs, ref, _, _, prog = run_both(g, t, cuda)
+    assert all(o.bulk and o.splits == splits for o in prog.g.ops if o.kind == "DecodeAttention")
+    got, ref = outs[0].view(B, H, D), ref[0].view(B, H, D)
+    assert torch.equal(got.isinf(), ref.isinf()) and torch.equal(got.sign()[got.isinf()], ref.sign()[ref.isinf()])
+    fin = ~ref.isinf()
+    assert int(ref.isinf().sum()) == 2 * B * H // KVH and rel_l2(got[fin], ref[fin]) < TOL
