@@ -585,3 +585,24 @@ def test_many_sequence_attention_with_infinite_values(cuda, monkeypatch, splits)
     assert torch.equal(got.isinf(), ref.isinf()) and torch.equal(got.sign()[got.isinf()], ref.sign()[ref.isinf()])
     fin = ~ref.isinf()
     assert int(ref.isinf().sum()) == 2 * B * H // KVH and rel_l2(got[fin], ref[fin]) < TOL
+
+
+@pytest.mark.parametrize("ctx", [0, 1, 15, 16, 37, 301])
+@pytest.mark.parametrize("form", ["per head", "many sequences"])
+def test_cache_rows_that_nothing_has_written_yet(cuda, monkeypatch, form, ctx):
+    """Rows at and behind the position hold NaN (memory that was never written): no output depends on them."""
+    monkeypatch.setenv("MEGACUTE_B200_ATT_BULK", str(int(form != "per head")))
+    monkeypatch.setenv("MEGACUTE_B200_KV_SPLITS", "2")
+    B, H, KVH, D, L = 9, 16, 4, 64, 384
+    g = mc.Graph()
+    t = {"qkv": rnd((B, (H + 2 * KVH) * D), 1.0, 1), "pos": torch.full((1, 1), ctx, dtype=torch.int32)}
+    t["cos"], t["sin"] = W.rope_tables(L, D)
+    for i, n in enumerate(("k_cache", "v_cache")):
+        t[n] = rnd((B * L, KVH * D), 1.0, 2 + i)
+        t[n].view(B, L, -1)[:, ctx:] = float("nan")
+    pos, kc, vc = g.state("pos", (1, 1), torch.int32), g.state("k_cache", (B * L, KVH * D)), g.state("v_cache", (B * L, KVH * D))
+    q = g.rope_append(g.input("qkv", t["qkv"].shape), g.input("cos", (L, D)), g.input("sin", (L, D)), pos, kc, vc, heads=H, kv_heads=KVH, head_dim=D, max_seq=L)
+    g.output(g.decode_attention(q, kc, vc, pos, heads=H, kv_heads=KVH, head_dim=D, max_seq=L))
+    outs, ref, _, _, prog = run_both(g, t, cuda)
+    assert all(bool(o.bulk) == (form != "per head") for o in prog.g.ops if o.kind == "DecodeAttention")
+    assert_close(outs, ref)
