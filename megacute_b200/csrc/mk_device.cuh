@@ -531,8 +531,9 @@ __device__ __forceinline__ void report(const Params& p, Ctrl* c, int code, int s
 enum { WHERE_RING_FULL = 1, WHERE_RING_EMPTY = 2, WHERE_DEP = 3, WHERE_DRAIN = 4, WHERE_COMBINE = 5, WHERE_CHECK_ARM = 6, WHERE_CHECK_RELEASE = 7, WHERE_STAGING = 8 };
 
 // `patience`: multiple of the time limit this wait allows.  A role that by design waits through everything the CTA does
-// before (the finisher warp, for the dependencies of a streaming linear far down the program) gives twice the limit, so
-// that when something earlier is stuck, the wait that is stuck reports first.
+// before (the finisher warp, for the dependencies of a streaming linear far down the program and for its partial tiles, which come
+// behind the wait for direct operands; the producer, for a free stage) gives twice the limit, so that when something earlier is
+// stuck, the wait that is stuck reports first.
 // The spinning part is a function of its own in the bodies of tile ops: those run cold, so what a wait costs when it does not have
 // to wait is the code that has to be fetched around it.  The streaming bodies of a decode step inline it (MK_INLINE_WAITS, set
 // by their translation units): there every wait does wait, and the call costs more than the code (batch-1 step 877 -> 912 us).

@@ -217,7 +217,7 @@ __device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint
             const uint32_t ph = mode == MODE_STAGES ? pos.phase : mode == MODE_WTILES ? wphase : mode == MODE_KVTILES ? kvphase : wwphase[k];
 #pragma unroll 1
             for (int s = 0; s < n && ok; ++s)
-                ok = wait_barrier(p, c, empty + s, (ph ^ (s < at ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY, wide ? 2 : 1) ? 1 : 0;
+                ok = wait_barrier(p, c, empty + s, (ph ^ (s < at ? 1u : 0u)) ^ 1u, rc.seq, WHERE_RING_EMPTY, 2) ? 1 : 0;
             // ... and until a run of 256-row tiles' epilogues have read their staging rows behind the slots
             if (ok && wide && next < MODE_WWIDE) ok = wait_word(p, c, &c->wide_done, wide_count, rc.seq, WHERE_STAGING) ? 1 : 0;
         }
@@ -376,7 +376,7 @@ __device__ __forceinline__ uint32_t producer_loop(const Params& p, Ctrl* c, uint
             continue;
         }
         int ok = 1;
-        if (lane == 0) ok = wait_barrier(p, c, &c->empty[pos.stage], pos.phase ^ 1u, rc.seq, WHERE_RING_EMPTY) ? 1 : 0;
+        if (lane == 0) ok = wait_barrier(p, c, &c->empty[pos.stage], pos.phase ^ 1u, rc.seq, WHERE_RING_EMPTY, 2) ? 1 : 0;
         if (!__shfl_sync(0xffffffffu, ok, 0)) goto left;
         const __nv_bfloat16* src; int bytes, off;
         rc.piece(lane, src, bytes, off);

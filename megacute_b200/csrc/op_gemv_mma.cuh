@@ -311,7 +311,7 @@ __device__ __forceinline__ void gemv_finisher(const Params& p, Ctrl* c, uint8_t*
                 }
             };
             fetch_operands();
-            ok = wait_barrier(p, c, &c->slot_full[sl], (fullpar >> sl) & 1u, seq, WHERE_COMBINE) && ok;
+            ok = wait_barrier(p, c, &c->slot_full[sl], (fullpar >> sl) & 1u, seq, WHERE_COMBINE, 2) && ok;
             fullpar ^= 1u << sl;
             if (!__all_sync(0xffffffffu, ok)) return;                         // the launch is failing (no lane stays behind, or stores the marker)
             if (g == 0) {
