@@ -219,7 +219,9 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
             pos.phase = (uint32_t)(npos >> 8);
             if (TRACE && threadIdx.x == 0 && !ran) {
                 const bool marks = op->kind == MK_OP_GEMV || op->kind == MK_OP_DECODE_ATTN || op->kind == MK_OP_GEMM || op->kind == MK_OP_ATTENTION;
-                trace_rec<TRACE>(p, 1, slot, in.seq, t0, c->t_dep, c->t_pub ? c->t_pub : (long long)globaltimer());
+                // (a streaming linear with a direct x has waited for its dependencies when x is staged)
+                const bool by_value = op->kind == MK_OP_GEMV && (op->flags & GEMV_F_DIRECT_X);
+                trace_rec<TRACE>(p, 1, slot, in.seq, t0, by_value ? c->t_phase[0] : c->t_dep, c->t_pub ? c->t_pub : (long long)globaltimer());
                 if (marks) trace_rec<TRACE>(p, 2, slot, in.seq, c->t_phase[0], c->t_phase[1], c->t_phase[2]);
             }
             if (aborting) break;

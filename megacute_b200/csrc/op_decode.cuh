@@ -129,7 +129,7 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
         return;
     }
     if (!fused) compute_sync();                                           // the zero fill of qs, before the rows below land
-    if (t == 0 && p.trace_cap > 0) c->t_dep = (long long)globaltimer();
+    if (!DIRECT && t == 0 && p.trace_cap > 0) c->t_dep = (long long)globaltimer();
 
     // ---- q (rotated when fused, pre-scaled to the log2 domain) as MMA A operand: rows = the G query
     // heads of this kv head, split into bf16 high and low parts so the scores keep ~16 mantissa bits.
@@ -171,6 +171,8 @@ __device__ __forceinline__ void decode_body(const Params& p, Ctrl* c, const mk_o
             }
         }
     }
+
+    if (DIRECT && t == 0 && p.trace_cap > 0) c->t_dep = (long long)globaltimer();       // (the wait was for the values)
 
     // ---- main loop: S = Q K^T and O += P V on tensor cores, every warp on its own 16 keys of the
     // tile with its own running max and sum (no barrier inside a tile) ----

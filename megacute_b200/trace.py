@@ -10,6 +10,8 @@ chrome_events, save_chrome).  This kernel has three record kinds per SM:
   role 2 "phases":   (seq, three op-internal marks) for the ops that wait for their own
                      dependencies: streaming linear (x staged, first stage landed, last group
                      done) and decode attention (tiles done, partial written, merged)
+With direct operands (values in place of counters) the dependencies are met when the values are there: a streaming
+linear has then staged x, decode attention q and the new token.
 Times are globaltimer nanoseconds rebased to the earliest record.
 
 The records are kept as one structured numpy table (``Timeline.table``) and every report is a

@@ -606,3 +606,21 @@ def test_cache_rows_that_nothing_has_written_yet(cuda, monkeypatch, form, ctx):
     outs, ref, _, _, prog = run_both(g, t, cuda)
     assert all(bool(o.bulk) == (form != "per head") for o in prog.g.ops if o.kind == "DecodeAttention")
     assert_close(outs, ref)
+
+
+def test_timeline_shows_waits_for_values(cuda):
+    """The wait of an instruction with a direct operand lasts until the values are there: most SMs have no part in a linear of 48 outputs and
+    wait for the next one's input for as long as it takes."""
+    g, t, _ = _chain(1, [2048, 2048, 48, 2048, 48, 2048])
+    prog = mc.compile(g, trace=True)
+    dev = {k: v.to(cuda) for k, v in t.items()}
+    for _ in range(3):
+        prog(**dev)
+    prog.check()
+    comp = prog.timeline().table
+    comp = comp[comp["role"] == 1]
+    assert bool((comp["t0"] <= comp["t1"]).all()) and bool((comp["t1"] <= comp["t2"]).all())
+    op = np.asarray(prog.sched.op_of)[comp["seq"]]
+    for k in (2, 4):
+        assert prog.g.ops[k].x.cols == 48 and prog.g.ops[k].x.buf.id in prog.direct
+        assert np.median((comp["t1"] - comp["t0"])[op == k]) > 500                   # (ns; a linear takes 1.5 us at least)
