@@ -434,30 +434,39 @@ static bool tile_gemm_on_tcgen05(const mk_op_desc& d) {
     return true;
 }
 
+// The same for the direct operands of a descriptor: every element of each inside the first copy of the program's direct memory
+// (the second is as large), fp32, where the body's 16-byte loads are aligned, and on a path that knows direct operands.
+static const char* direct_operands(const mk_program* p, const mk_op_desc& d) {
+    const int f = d.flags & (MK_F_DIRECT_IN | MK_F_DIRECT_OUT | MK_F_DIRECT_RES);
+    if (!f || (d.kind != MK_OP_GEMV && d.kind != MK_OP_DECODE_ATTN && d.kind != MK_OP_GATHER)) return nullptr;
+    // operand ptr[at]: d.i[0] rows of `cols` elements, ld[at] apart
+    auto inside = [&](int at, int dtype, long long cols, int align) {
+        const uint64_t base = (uint64_t)(uintptr_t)p->direct, at0 = d.ptr[at];
+        if (!p->direct || dtype != mk::DT_F32 || d.i[0] <= 0 || cols <= 0 || d.ld[at] < 0 || at0 < base || at0 - base >= p->direct_bytes) return false;
+        if (at0 % align || (d.i[0] > 1 && (long long)d.ld[at] * 4 % align)) return false;
+        const uint64_t bytes = ((uint64_t)(d.i[0] - 1) * (uint64_t)d.ld[at] + (uint64_t)cols) * 4;
+        return bytes <= p->direct_bytes - (at0 - base);
+    };
+    bool ok = true;
+    if (d.kind == MK_OP_GEMV) {
+        ok = (d.flags & mk::GEMV_F_UNITS) && (!(f & MK_F_DIRECT_IN) || inside(0, d.i[4], d.i[2], 16)) &&
+             (!(f & MK_F_DIRECT_OUT) || inside(2, d.i[5], d.i[1], 4)) && (!(f & MK_F_DIRECT_RES) || inside(4, d.i[6], d.i[1], 4));
+    } else if (d.kind == MK_OP_DECODE_ATTN) {
+        const long long q = (long long)d.i[1] * d.i[3], kv = (long long)d.i[2] * d.i[3];
+        ok = !d.i[11] && !d.i[9] &&
+             (!(f & MK_F_DIRECT_IN) || (d.i[6] && inside(0, d.i[7], q, 16) && inside(5, d.i[7], kv, 16) && inside(6, d.i[7], kv, 16))) &&
+             (!(f & MK_F_DIRECT_OUT) || inside(4, d.i[8], q, 4));
+    } else {
+        ok = f == MK_F_DIRECT_OUT && inside(2, d.i[3], d.i[1], 4);
+    }
+    return ok ? nullptr : "direct operands: path, type, extent or alignment";
+}
+
 // Bind-time check of the instruction table against the op descriptors: every argument an op body
 // turns into an address (tile, row-group, head, split indices; output-column ranges) must lie inside
 // the extents the descriptor states.  The kernel trusts its tables; this is where a table built for
 // another graph, or a descriptor with a shrunken extent, is caught -- as an error code here instead of
 // an out-of-bounds access on the device.  On failure the message names the instruction.
-static const char* direct_operands(const mk_program* p, const mk_op_desc& d) {
-    const int f = d.flags & (MK_F_DIRECT_IN | MK_F_DIRECT_OUT | MK_F_DIRECT_RES);
-    if (!f || (d.kind != MK_OP_GEMV && d.kind != MK_OP_DECODE_ATTN && d.kind != MK_OP_GATHER)) return nullptr;
-    auto inside = [&](int ptr, int dtype) {
-        return dtype == mk::DT_F32 && p->direct && d.ptr[ptr] >= (uint64_t)p->direct && d.ptr[ptr] < (uint64_t)p->direct + p->direct_bytes;
-    };
-    bool ok = true;
-    if (d.kind == MK_OP_GEMV) {
-        ok = (d.flags & mk::GEMV_F_UNITS) && (!(f & MK_F_DIRECT_IN) || inside(0, d.i[4])) && (!(f & MK_F_DIRECT_OUT) || inside(2, d.i[5])) &&
-             (!(f & MK_F_DIRECT_RES) || inside(4, d.i[6]));
-    } else if (d.kind == MK_OP_DECODE_ATTN) {
-        ok = !d.i[11] && !d.i[9] && (!(f & MK_F_DIRECT_IN) || (d.i[6] && inside(0, d.i[7]) && inside(5, d.i[7]) && inside(6, d.i[7]))) &&
-             (!(f & MK_F_DIRECT_OUT) || inside(4, d.i[8]));
-    } else {
-        ok = f == MK_F_DIRECT_OUT && inside(2, d.i[3]);
-    }
-    return ok ? nullptr : "direct operands: path, type or memory";
-}
-
 static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
     const int W = MK_INST_WORDS;
     auto ceil_div = [](long long a, long long b) { return (a + b - 1) / b; };

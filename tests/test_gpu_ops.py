@@ -424,7 +424,8 @@ def test_values_instead_of_counters(cuda, M, widths):
 
 
 def test_values_that_are_nan_end_the_wait(cuda):
-    """NaN inputs, the one with all bits set among them, reach the output as NaN; the rows beside them and the launches after are right."""
+    """NaN inputs reach the output as NaN through direct operands; the rows beside them and the launches after are right.  (The input has
+    all 16 bits set.  No op can produce the 32-bit marker itself: arithmetic makes 0x7fffffff, an embedding's low half is 0.)"""
     g, t, _ = _chain(2, [512, 2048, 512, 2048, 512])
     prog = mc.compile(g)
     dev = {k: v.to(cuda) for k, v in t.items()}
@@ -470,7 +471,7 @@ def test_values_that_never_come_end_the_launch(cuda):
 
 
 def test_direct_operands_are_checked_at_bind_time(cuda):
-    """A direct operand without memory for it, or of another type, is refused as the descriptors are bound."""
+    """A direct operand of a program without direct memory is refused as the descriptors are bound."""
     import ctypes
     from megacute_b200 import _lib
     g = mc.Graph()
@@ -624,3 +625,60 @@ def test_timeline_shows_waits_for_values(cuda):
     for k in (2, 4):
         assert prog.g.ops[k].x.cols == 48 and prog.g.ops[k].x.buf.id in prog.direct
         assert np.median((comp["t1"] - comp["t0"])[op == k]) > 500                   # (ns; a linear takes 1.5 us at least)
+
+
+def test_direct_operands_must_lie_in_their_memory(cuda):
+    """A program with direct memory: each thing its kernel relies on changed by itself is refused as the descriptors are bound -- type,
+    path, an operand that starts outside or runs past the end of the first copy, a misaligned one -- and the program still runs."""
+    import ctypes
+    from megacute_b200 import _lib
+    from megacute_b200 import config as C
+    g, t = _gated_decode()
+    prog = mc.compile(g)
+    dev = {k: v.to(cuda) for k, v in t.items()}
+    want = prog(**dev).clone()
+    prog.check()
+    lib, n = _lib.load(), len(prog.g.ops)
+    ops = {o.kind: k for k, o in enumerate(prog.g.ops)}
+    att = ops["DecodeAttention"]
+    lin = next(k for k, o in enumerate(prog.g.ops) if o.kind == "Linear" and prog._desc[k].flags & C.F_DIRECT_RES)
+    base, size = prog._direct_mem.data_ptr(), prog._direct_mem.shape[1] * 4
+    refused = []
+
+    def change(k, field, index, value):
+        d = prog._desc[k]
+        seq = getattr(d, field) if index is not None else None
+        old = seq[index] if index is not None else getattr(d, field)
+        new = value(old)
+        if index is not None:
+            seq[index] = new
+        else:
+            setattr(d, field, new)
+        rc = lib.mk_program_set_ops(prog._handle, ctypes.addressof(prog._desc), n, None)
+        refused.append((k, field, index))
+        assert rc == -2 and b"direct operands" in lib.mk_last_cuda_error(), refused[-1]
+        if index is not None:
+            seq[index] = old
+        else:
+            setattr(d, field, old)
+
+    for at, dt in ((0, 4), (4, 6)):                                           # a linear's x and residual
+        change(lin, "i", dt, lambda v: 0)                                     # another type
+        change(lin, "ptr", at, lambda v: base - 16)                           # before the memory
+        change(lin, "ptr", at, lambda v: base + size)                         # behind the first copy
+        change(lin, "ptr", at, lambda v: base + size - 16)                    # past its end
+        change(lin, "ld", at, lambda v: size // 4)                            # ... with its second row
+    change(lin, "ptr", 0, lambda v: v + 4)                                    # 16-byte loads
+    change(lin, "ld", 0, lambda v: v + 1)
+    change(lin, "flags", None, lambda v: v & ~4)                              # not the tensor-core path
+    for at in (0, 5, 6, 4):                                                   # the attention's q, k, v and output
+        change(att, "ptr", at, lambda v: base + size - 16)
+    change(att, "i", 7, lambda v: 0)
+    change(att, "i", 8, lambda v: 0)
+    change(att, "i", 9, lambda v: 1)                                          # inputs zeroed behind the read
+    change(att, "i", 6, lambda v: 0)                                          # not fused
+    assert lib.mk_program_set_ops(prog._handle, ctypes.addressof(prog._desc), n, None) == 0
+    for k in ("k_cache", "v_cache", "pos"):
+        dev[k].copy_(t[k])
+    assert torch.equal(prog(**dev), want)
+    prog.check()
