@@ -70,7 +70,7 @@ W_SEQ = 12                      # global instruction index
 # ---- device op kinds (include/megacute_b200.h: MK_OP_*)
 OP_GEMV, OP_GEMM, OP_FINALIZE, OP_ELTWISE, OP_NORM, OP_ATTENTION, OP_ROPE_APPEND, OP_DECODE_ATTN, OP_INCREMENT, \
     OP_GATHER, OP_ARGMAX = range(1, 12)
-DIRECT_MIN_COLS = 2048          # a program's only direct buffer is at least so wide (passes.direct_buffers)
+DIRECT_MIN_COLS = 4096          # of a program's one or two direct buffers one is at least so wide (passes.direct_buffers)
 F_DIRECT_IN, F_DIRECT_OUT, F_DIRECT_RES = 8, 16, 32       # descriptor flags: direct operands
 GATHER_ROWS = 8                 # rows per gather instruction (one per compute warp)
 ARGMAX_MAX_CHUNKS = 256         # column chunks per row of an argmax (the merging instruction takes one partial per thread)

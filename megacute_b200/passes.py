@@ -606,9 +606,12 @@ def direct_buffers(g: Graph) -> frozenset:
                 or (per_head(r) and r.k_new is not None and field in ("q", "k_new", "v_new") and r.q.buf is r.k_new.buf is r.v_new.buf))
         if ok:
             direct.add(b)
-    # (one narrow hop alone gains nothing -- two linears of 256 to 1024 take 14.7 us either way, of 2048 16.4 and 16.3, of 4096 24.9 and
-    # 23.1 -- and keeps its counters; a model of 256 columns and eight layers 225 and 210)
-    if len(direct) == 1 and all(b.cols < C.DIRECT_MIN_COLS for b in direct):
+    # (The first linear of a launch has no direct input, so a program with direct hops runs two forms of the streaming linear, and fetches the
+    # code of the second one cold, 1 us per launch.  A hop by value gains 0.3 us between narrow linears, 1.5 to 2.5 between wide ones: one or
+    # two narrow hops do not pay.  By value / through counters, us per call back to back: one hop of 256 columns 14.5 / 13.4, of 2048 15.1 / 14.6,
+    # of 4096 23.5 / 24.8, of 8192 59.3 / 61.6, an MLP block of one row with 5632 25.2 / 26.9; two of 256 17.0 / 16.7, of 2048 19.0 / 18.75, of 4096
+    # 31.5 / 33.4; four of 256 24.9 / 24.9, of 2048 28.1 / 29.0.)
+    if len(direct) <= 2 and all(b.cols < C.DIRECT_MIN_COLS for b in direct):
         return frozenset()
     return frozenset(b.id for b in direct)
 

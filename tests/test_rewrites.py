@@ -235,6 +235,25 @@ def test_direct_buffers_and_their_schedule():
         assert not direct_buffers(run_all(g, 148)), case
 
 
+def test_few_narrow_hops_keep_their_counters():
+    """One or two direct buffers pay from config.DIRECT_MIN_COLS columns on, three or more at any width."""
+    from megacute_b200 import config as C
+    from megacute_b200.passes import direct_buffers, run_all
+
+    def direct(*widths):
+        g = mc.Graph()
+        h = g.input("x", (1, widths[0]))
+        for i, n in enumerate(widths[1:]):
+            h = g.linear(h, g.param(f"w{i}", (n, h.cols)))
+        g.output(h)
+        return len(direct_buffers(run_all(g, SMS)))
+
+    wide = C.DIRECT_MIN_COLS
+    assert direct(512, wide - 16, 512) == 0 and direct(512, wide, 512) == 1
+    assert direct(512, wide - 16, wide - 16, 512) == 0 and direct(512, 64, wide, 512) == 2
+    assert direct(512, 64, 64, 64, 512) == 3
+
+
 def test_values_order_nothing_but_themselves():
     """A linear that reads a pointwise op's result beside a direct operand made from it needs its counter: the values it waits for were
     loaded and stored without an order for other accesses."""

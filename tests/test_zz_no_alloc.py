@@ -84,9 +84,15 @@ def test_noalloc_runs_direct_operands(cuda, step):
         t = dict(cos=cos, sin=sin, **W.llama_weights(E, H, KVH, F, n, V, 0, "cpu"), pos=st["pos"], k_cache=st["k_cache"], v_cache=st["v_cache"],
                  ids=torch.zeros(B, 1, dtype=torch.int32))
     else:
-        g, t = _graph(), {k: v.cpu() for k, v in _inputs(cuda).items()}
+        g, t = mc.Graph(), {"x": None}
+        h = g.input("x", (1, 512))
+        for i, n in enumerate((2048, 512, 1024, 512)):
+            t[f"w{i}"] = (torch.randn(n, h.cols, generator=torch.Generator().manual_seed(i)) * h.cols ** -0.5).to(BF)
+            h = g.linear(h, g.param(f"w{i}", t[f"w{i}"].shape))
+        g.output(h)
     prog = mc.compile(g)
-    dev = {k: t[b.name].to(cuda) for b in prog.g.inputs + prog.g.params + prog.g.states for k in [b.name]}
+    dev = {b.name: torch.zeros(b.rows, b.cols, dtype=b.dtype, device=cuda) if t[b.name] is None else t[b.name].to(cuda)
+           for b in prog.g.inputs + prog.g.params + prog.g.states}
     gen = torch.Generator().manual_seed(3)
 
     def fresh():
