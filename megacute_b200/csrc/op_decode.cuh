@@ -428,9 +428,9 @@ static __device__ __noinline__ bool op_decode_attn_heads(const Params& p, Ctrl* 
     const int hp = op->i[10];
 #pragma unroll 1
     for (int j = 0; j < hp; ++j) {
-        if (j) compute_sync();                                  // the previous head's merge reads the tile buffers
+        // the previous head's merge reads the tile buffers; one decision for all threads, which share this barrier with publish
+        if (j && compute_sync_or(*(volatile int*)&c->abort)) break;
         decode_one_head<D, GMAX, DIRECT>(p, c, op, a0, a1 + j, a2, work, j ? 0 : nwait, wait_off, seq);
-        if (*(volatile int*)&c->abort) break;
     }
     return publish(p, c, narrive, arrive_off);
 }

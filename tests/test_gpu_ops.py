@@ -682,3 +682,36 @@ def test_direct_operands_must_lie_in_their_memory(cuda):
         dev[k].copy_(t[k])
     assert torch.equal(prog(**dev), want)
     prog.check()
+
+
+def test_timeout_in_a_step_with_several_heads_per_instruction(cuda, monkeypatch):
+    """A wait that cannot end, at the first waiting instruction of every op of a batched decode step whose attention instructions run
+    several kv heads each: the launch ends, and the step is right once the wait is."""
+    from megacute_b200 import _lib
+    monkeypatch.setenv("MEGACUTE_B200_ATT_HEADS", "2")
+    monkeypatch.setenv("MEGACUTE_B200_ATT_BULK", "0")
+    g, params, st, _ = small_decode(B=16, E=256, H=4, KVH=2, F=512, n=1, max_seq=256, ctx=120, vocab=1000)
+    prog = mc.compile(g)
+    assert {o.heads_per_inst for o in prog.g.ops if o.kind == "DecodeAttention"} == {2}
+    dp, ds = ({k: v.to(cuda) for k, v in d.items()} for d in (params, st))
+    ref, _ = evaluate(g, {**params, **st})
+    prog(**dp, **ds)
+    prog.check()
+    s, lib = prog.sched, _lib.load()
+    prog.set_timeout(0.02)
+    for k, (i0, i1) in enumerate(s.node_ranges):
+        i = next((i for i in range(i0, i1) if s.wait_ptr[i + 1] > s.wait_ptr[i]), None)
+        if i is None:
+            continue
+        at = int(s.wait_ptr[i])
+        _lib.check(lib.mk_program_poke_wait(prog._handle, at, int(s.wait_cnt[at]), 1000))
+        prog(**dp, **ds)
+        with pytest.raises(_lib.MegakernelTimeout):
+            prog.check()
+        _lib.check(lib.mk_program_poke_wait(prog._handle, at, int(s.wait_cnt[at]), int(s.wait_tgt[at])))
+        prog.reset()
+        for n, v in st.items():
+            ds[n].copy_(v)
+        out = prog(**dp, **ds)
+        prog.check()
+        assert rel_l2(out.float().cpu(), ref[0]) < TOL, prog.g.ops[k].kind
