@@ -720,7 +720,7 @@ int mk_program_set_ops(mk_program* p, const mk_op_desc* ops, int n_ops, void* st
         // mixing fp16 activations with bf16 weights raised an illegal-instruction fault): only the packed
         // copy can provide them.  Without one, the op runs the mma.sync body, which converts in registers.
         if (xh && (pack_off || (d.ptr[1] & 15) || d.ld[1] % 8 != 0)) continue;
-        if (!encode_tile_map(maps, d.ptr[0], d.i[0], d.i[2], d.ld[0], d.i[11] == 256 ? 256 : d.i[0] <= 64 ? 64 : 128, false, xh)) continue;
+        if (!encode_tile_map(maps, d.ptr[0], d.i[0], d.i[2], d.ld[0], d.i[11] == 256 ? 256 : mk::tc_box_rows(d.i[0]), false, xh)) continue;
         // weights: the packed copy, made when a matrix (address, shape, pitch) is bound for the first
         // time and kept while it stays bound -- rebinding other operands (a new input tensor every
         // call) must not copy gigabytes of weights again; weights changed in place need

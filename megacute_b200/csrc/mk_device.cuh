@@ -49,6 +49,8 @@ constexpr int kTcTileBytes = 128 * 128;
 constexpr int kTcXStages = 6;                             // activation stages of 128 rows ...
 constexpr int kTcXHalfStages = 10;                        // ... or of 64 rows (ops with at most 64): the MMA still reads 128 rows from a
                                                           // stage's start, so half a tile of the work area must follow the last one
+// rows of one activation copy of a 128 x 128 tile: the rows there are, in whole 8-row groups of the swizzle
+__host__ __device__ constexpr int tc_box_rows(int m) { return m < 128 ? (m + 7) & ~7 : 128; }
 constexpr int kTcXOff = 512;                              // first 1024-aligned byte of the work area
 constexpr int kTcCols = 512;                              // tensor-memory columns held by the CTA: all of them (two 128 x 256 accumulators of
                                                           // the tile GEMM, scores and O of the prefill attention)

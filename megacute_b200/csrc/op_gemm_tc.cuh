@@ -4,7 +4,7 @@
 // Same instructions, descriptor and epilogue semantics as the mma.sync body (op_gemm.cuh); the host
 // library selects this body by putting the address of two tensor maps in ptr 11 (activations, then
 // weights 128 bytes further: {K, rows} bf16, 128-byte swizzle, zero fill; boxes of 64 columns x 128
-// rows, or x 64 rows for the activations of an op with at most 64 of them) and, when it has packed
+// rows, or x the rows there are, in whole groups of eight, for the activations of an op with fewer) and, when it has packed
 // the weights into tile images, the packed array in ptr 10.
 //
 // Operands are K-major 128-row x 64-column tiles (16 KB).  The 128 activation rows of the m tile are
@@ -14,9 +14,12 @@
 //   weights      producer warp -> eight single-tile slots in the ring's memory, across instruction
 //                boundaries: they depend on nothing in the launch, so the next instruction's first
 //                128 KB are already on their way while this one waits for its dependencies
-//   activations  one compute thread -> single-tile stages in the work area, after the instruction's
+//   activations  two lanes of a compute warp -> single-tile stages in the work area, after the instruction's
 //                dependencies are met: 6 stages of 128 rows, or 10 of 64 rows when the op has at most
-//                64 (the MMA still reads 128 rows: the upper 64 accumulator rows are never looked at)
+//                64.  The MMA still reads 128 rows: accumulator rows beyond the copied ones are never looked at
+//                (a copy whose box has 64 rows over a tensor of 9 to 31 is slow, whatever fills the rest: gate/up of a
+//                batch of 16 0.6 us per k-tile instead of 0.3; steps of 9, 16 and 31 sequences at context 1024
+//                1480 -> 1098, 1431 -> 1127 and 1588 -> 1364 us with boxes of the rows there are)
 //   MMA          one compute thread: 4 x tcgen05.mma (128 x 128 x 16) per k-tile; tcgen05.commit
 //                returns the activation stage and the ring slot when the MMAs that read them are done
 //   epilogue     all 8 compute warps: tensor memory -> shared memory (warp w reads lanes 32 (w & 3) .. +31,
@@ -263,6 +266,7 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
     uint8_t* xs = work + kTcXOff;
     // activation stages: whole 128-row tiles, or twice as many 64-row half tiles
     const int xbytes = M <= 64 ? kTcTileBytes / 2 : kTcTileBytes;
+    const uint32_t xcopied = (uint32_t)tc_box_rows(M) * 128u;
     const uint32_t xstages = M <= 64 ? kTcXHalfStages : kTcXStages;
 
     // Tensor memory is allocated by the CTA's first tile GEMM instruction and kept until the kernel
@@ -303,7 +307,7 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
         for (int kt = lane; kt < nk; kt += 2) {
             if (!wait_barrier(p, c, &c->x_empty[s], ((xpar0 >> s) & 1u) ^ round, seq, WHERE_RING_EMPTY)) break;
             if (!check_phase(p, c, &c->x_full[s], ((xpar0 >> s) & 1u) ^ round ^ 1u, seq, WHERE_CHECK_ARM)) break;
-            mbar_arrive_expect_tx(&c->x_full[s], (uint32_t)xbytes);
+            mbar_arrive_expect_tx(&c->x_full[s], xcopied);
             tma_load_2d(xs + s * xbytes, tmaps, kbeg + kt * 64, m0, &c->x_full[s], keep);
             s += 2;
             if (s >= xstages) { s -= xstages; round ^= 1u; }

@@ -60,6 +60,23 @@ def test_tile_epilogues(cuda, monkeypatch, M, N, K, plan, kw):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M", [9, 15, 16, 17, 31, 33, 56, 57, 64, 65, 120, 121, 127])
+def test_activation_copies_of_the_rows_there_are(cuda, M):
+    """128 x 128 tiles copy a ragged op's activation rows in whole groups of eight; what the rest of a stage holds -- another op's
+    rows, not numbers here -- reaches no output."""
+    g = mc.Graph()
+    y = g.linear(g.input("z", (128, 1024)), g.param("v", (20480, 1024)))         # every SM's stages filled with values that are not numbers
+    h = g.linear(g.input("x", (M, 1024)), g.param("w", (19000, 1024)), act="gelu_tanh")
+    g.output(y)
+    g.output(h)
+    t = {"z": torch.full((128, 1024), float("nan"), dtype=torch.bfloat16), "v": rnd((20480, 1024), 0.03, 3),
+         "x": rnd((M, 1024), 1.0, 1), "w": rnd((19000, 1024), 0.03, 2)}
+    outs, ref, _, _, prog = run_both(g, t, cuda)
+    assert prog.tcgen05_ops == 2 and outs[0].isnan().all()
+    assert torch.isfinite(outs[1]).all() and rel_l2(outs[1], ref[1]) < TOL
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("tcgen05", [True, False])
 @pytest.mark.parametrize("B,S,D,tile", [(1, 150, 64, (128, 128)), (3, 50, 128, (128, 128)), (2, 129, 64, (256, 256)), (1, 257, 128, (256, 128)),
                                         (1, 300, 128, (256, 256))])
