@@ -420,6 +420,11 @@ __device__ __forceinline__ uint32_t load8_direct(const float* at, float* f) {
     asm volatile("ld.relaxed.gpu.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(at + 4) : "memory");
     return max(max(max(w[0], w[1]), max(w[2], w[3])), max(max(w[4], w[5]), max(w[6], w[7])));
 }
+__device__ __forceinline__ uint2 load2_direct(const float* at) {
+    uint2 w;
+    asm volatile("ld.relaxed.gpu.global.v2.b32 {%0, %1}, [%2];" : "=r"(w.x), "=r"(w.y) : "l"(at) : "memory");
+    return w;
+}
 __device__ __forceinline__ float load1_direct(const float* at) {
     uint32_t w;
     asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(w) : "l"(at) : "memory");

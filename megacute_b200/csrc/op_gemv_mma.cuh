@@ -101,7 +101,7 @@ __device__ __forceinline__ void gemv_mma(const Params& p, Ctrl* c, uint8_t* ring
     // vectors and eight k-steps it saved and restored 43 callee-saved registers per call, 44 KB of local memory each way through a
     // path of 32 bytes a cycle: batch 1 at context 1024 852 -> 831 us, at 16384 985 -> 970, five sequences 1172 -> 1137, an MLP block of
     // one row 28.1 -> 27.0.  With two k-steps batch 1 is back at 844.)
-    {
+    if (M == 1 || xdt != DT_F32 || (K & 255) != 0) {
 #pragma unroll 1
         for (int m = 0; m < M; ++m) {
             float ss = 0.f;
@@ -133,6 +133,110 @@ __device__ __forceinline__ void gemv_mma(const Params& p, Ctrl* c, uint8_t* ring
             if (rms) {
                 ss = warp_sum(ss);
                 if (lane == 0) rowstat[warp * 8 + m] = ss;
+            }
+        }
+        compute_sync();
+    } else {
+        // Two rows and more.  One vector of a row at a time, as above, a row takes 0.65 us: a round trip to L2 and then as long a chain of
+        // conversions, word-wise stores and the sum's shuffles, with two warps per scheduler.  Here all rows are on their way at once, as
+        // copies into the place of their own fragments (8 elements take 32 bytes either way), without registers; then a lane makes the
+        // 16-byte fragments of its k-steps, 2 + 2 elements each, of two rows side by side (the last row of an odd number twice, with
+        // the same result).  Five rows of 2048 3.4 -> 2.1 us, eight 5.4 -> 2.9.  Direct operands are looked at in registers, two rows at a time.
+        if (!DIRECT) {
+#pragma unroll 1
+            for (int m = 0; m < M; ++m) {
+#pragma unroll 1
+                for (int v = t; v < nv; v += kComputeThreads) {
+                    const float* from = reinterpret_cast<const float*>(x) + m * ldx + v * 8;
+                    uint8_t* to = xf + m * xrow + v * 32;
+                    cp_async16(to, from, true);
+                    cp_async16(to + 16, from + 4, true);
+                }
+            }
+        }
+        // the k-steps of the vectors that this warp has copied: 16 of every 128
+        constexpr int kBlocks = DIRECT ? 1 : 2;
+        const int nb = K >> 4, u1 = warp * 8 * kBlocks + (lane >> 2), j = lane & 3;
+        auto gain2 = [&](int u, int h) { return gain ? __ldg(reinterpret_cast<const uint32_t*>(gain) + u * 8 + j + 4 * h) : 0x3f803f80u; };
+        uint32_t g1[kBlocks][2] = {};
+        if (!DIRECT && u1 < nb) {
+#pragma unroll
+            for (int q = 0; q < kBlocks; ++q) { g1[q][0] = gain2(u1 + 8 * q, 0); g1[q][1] = gain2(u1 + 8 * q, 1); }
+        }
+        if (!DIRECT) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+            __syncwarp();
+        }
+#pragma unroll 1
+        for (int m = 0; m < M; m += 2) {
+            const int m2 = min(m + 1, M - 1);
+            float s0 = 0.f, s1 = 0.f;
+            const uint32_t at = smem_u32(xf) + m * xrow + j * 16, next = m2 > m ? xrow : 0;
+#pragma unroll 1
+            for (int u = u1; u < nb; u += 64 * kBlocks) {
+                const uint32_t to = at + u * 64;
+                uint2 w[2][kBlocks][2];
+                uint32_t g[kBlocks][2];
+#pragma unroll
+                for (int q = 0; q < kBlocks; ++q) { g[q][0] = g1[q][0]; g[q][1] = g1[q][1]; }
+                if (DIRECT || u != u1) {
+#pragma unroll
+                    for (int q = 0; q < kBlocks; ++q) { g[q][0] = gain2(u + 8 * q, 0); g[q][1] = gain2(u + 8 * q, 1); }
+                }
+                if (DIRECT) {
+                    const float* from = reinterpret_cast<const float*>(x) + m * ldx + u * 16 + j * 2;
+#pragma unroll 1
+                    for (DirectWait dw;;) {
+                        uint32_t most = 0;
+#pragma unroll
+                        for (int r = 0; r < 2; ++r)
+#pragma unroll
+                            for (int q = 0; q < kBlocks; ++q)
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) w[r][q][h] = load2_direct(from + (r && m2 > m ? ldx : 0) + q * 128 + h * 8);
+#pragma unroll
+                        for (int r = 0; r < 2; ++r)
+#pragma unroll
+                            for (int q = 0; q < kBlocks; ++q)
+#pragma unroll
+                                for (int h = 0; h < 2; ++h) most = max(most, max(w[r][q][h].x, w[r][q][h].y));
+                        if (most != kUnwritten) break;
+                        if (!dw.again(p, c)) { c->flag = -1 - seq; break; }
+                    }
+                } else {
+#pragma unroll
+                    for (int q = 0; q < kBlocks; ++q)
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            w[0][q][h] = lds64(to - j * 8 + q * 512 + h * 32);
+                            w[1][q][h] = lds64(to - j * 8 + q * 512 + h * 32 + next);
+                        }
+                }
+                if (!DIRECT) __syncwarp();                                   // (the lanes of a k-step have read its 64 bytes)
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                    for (int q = 0; q < kBlocks; ++q) {
+                        uint32_t hi[2], lo[2];
+#pragma unroll
+                        for (int h = 0; h < 2; ++h) {
+                            const float vx = __uint_as_float(w[r][q][h].x), vy = __uint_as_float(w[r][q][h].y);
+                            const float y0 = vx * bf16_lo(g[q][h]), y1 = vy * bf16_hi(g[q][h]);
+                            if (r) s1 += vx * vx + vy * vy;
+                            else s0 += vx * vx + vy * vy;
+                            hi[h] = pack2(y0, y1);
+                            lo[h] = pack2(y0 - bf16_lo(hi[h]), y1 - bf16_hi(hi[h]));
+                        }
+                        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(to + q * 512 + r * next), "r"(hi[0]), "r"(hi[1]), "r"(lo[0]), "r"(lo[1])
+                                     : "memory");
+                    }
+            }
+            if (rms) {                                                       // both rows' sums: the lower half warp takes the first row's
+                const bool up = lane & 16;
+                float ss = (up ? s1 : s0) + __shfl_xor_sync(0xffffffffu, up ? s0 : s1, 16);
+#pragma unroll
+                for (int o = 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+                if ((lane & 15) == 0) rowstat[warp * 8 + (up ? m2 : m)] = ss;
             }
         }
         compute_sync();

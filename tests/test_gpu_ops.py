@@ -8,6 +8,7 @@ import pytest
 import torch
 
 import megacute_b200 as mc
+from megacute_b200 import config as C
 from megacute_b200 import workloads as W
 from oracle.graph_oracle import evaluate, rel_l2
 from tests.helpers import TOL, small_decode, to_cpu
@@ -421,6 +422,24 @@ def test_values_instead_of_counters(cuda, M, widths):
         # the buffers hold this launch's values
         last = next(b for b in prog.g.buffers if b.id in prog.direct and b.name == hs[-2].buf.name)
         assert not bool((prog.buffer(last).view(torch.int32) == -1).any())
+
+
+@pytest.mark.parametrize("by_value", [False, True])
+@pytest.mark.parametrize("M,K", [(2, 256), (2, 8192), (3, 768), (5, 2048), (7, 2304), (8, 2048), (4, 2064), (8, 272)])
+def test_rows_staged_side_by_side(cuda, monkeypatch, M, K, by_value):
+    """Two rows and more of a private fp32 activation, K a multiple of 256 (two rows at a time; an odd last row alone) or not, with the
+    norm's gain and sums of squares, rows of very different size.  One rounding of the result to bf16 is at most 2^-9; the
+    operands' high and low parts leave 2^-16 of them."""
+    monkeypatch.setattr(C, "DIRECT_MIN_COLS", 0 if by_value else 1 << 30)
+    g = mc.Graph()
+    h = g.linear(g.input("x", (M, 64)), g.param("v", (K, 64)))
+    g.output(g.linear(g.rms_norm(h, g.param("n", (1, K)), eps=1e-5), g.param("w", (1000, K))))
+    t = {"x": rnd((M, 64), 1.0, 1) * torch.tensor([4.0 ** (m % 5 - 2) for m in range(M)]).to(BF)[:, None], "v": rnd((K, 64), 0.1, 2),
+         "n": rnd((1, K), 0.3, 3, 1.0), "w": rnd((1000, K), K ** -0.5, 4)}
+    outs, ref, _, _, prog = run_both(g, t, cuda, steps=3)
+    assert len(prog.direct) == (1 if by_value else 0)
+    for r in range(M):
+        assert rel_l2(outs[0][r], ref[0][r]) < 1.05 * 2.0 ** -9, r
 
 
 def test_values_that_are_nan_end_the_wait(cuda):
