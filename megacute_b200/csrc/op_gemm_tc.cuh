@@ -36,13 +36,11 @@ namespace mk {
 
 // the same columns of two accumulators, `second` columns apart, added (second == 0: one accumulator)
 __device__ __forceinline__ void tc_ld16_sum(uint32_t taddr, uint32_t second, float* v) {
-    tc_ld16(taddr, v);
-    if (second) {
-        float w[16];
-        tc_ld16(taddr + second, w);
+    if (!second) { tc_ld16(taddr, v); return; }
+    float w[16];
+    tc_ld16x2(taddr, taddr + second, v, w);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] += w[j];
-    }
+    for (int j = 0; j < 16; ++j) v[j] += w[j];
 }
 
 // State the next tile GEMM instruction of this CTA starts from, written by one thread behind the barrier that
@@ -76,17 +74,17 @@ static __device__ __noinline__ void tc_write_rows(const mk_op_desc* op, const fl
     uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]);
     const uint8_t* bias = reinterpret_cast<const uint8_t*>(op->ptr[3]);
     const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]);
-    const int lpr = ncols >> 2;                                // lanes per row: 32, or 16 (swiglu: two rows per pass)
-    const int sub = lane / lpr, c4 = (lane % lpr) * 4, col = col0 + c4;
+    const int two = ncols == 64 ? 1 : 0;                       // swiglu: 16 lanes per row, two rows per pass
+    const int sub = two ? lane >> 4 : 0, c4 = (two ? lane & 15 : lane) * 4, col = col0 + c4;
     if (col >= n_out) return;
     float b4[4] = {0.f, 0.f, 0.f, 0.f};
     if (plain && bias) {
         const uint2 w = __ldg(reinterpret_cast<const uint2*>(bias + (long long)col * 2));
         b4[0] = bf16_lo(w.x); b4[1] = bf16_hi(w.x); b4[2] = bf16_lo(w.y); b4[3] = bf16_hi(w.y);
     }
-    const int step = kComputeWarps * (32 / lpr);
+    const int step = kComputeWarps << two;
 #pragma unroll 2
-    for (int row = warp * (32 / lpr) + sub; row < rows; row += step) {
+    for (int row = (warp << two) + sub; row < rows; row += step) {
         const float4 q = *reinterpret_cast<const float4*>(stage + row * kTcStagePitch + c4);
         float f[4] = {q.x, q.y, q.z, q.w};
         const long long eo = (long long)(m0 + row) * op->ld[2] + col;
@@ -119,11 +117,28 @@ static __device__ __noinline__ void tc_write_rows(const mk_op_desc* op, const fl
     }
 }
 
+// ... of an fp32 split-K partial: nothing but the reduce-adds.
+static __device__ __noinline__ void tc_reduce_rows(const mk_op_desc* op, const float* stage, int m0, int rows, int n0, int N) {
+    const int warp = threadIdx.x >> 5, c4 = (threadIdx.x & 31) * 4;
+    if (n0 + c4 >= N) return;
+    const long long step = (long long)kComputeWarps * op->ld[2];
+    float* O = reinterpret_cast<float*>(op->ptr[2]) + (long long)(m0 + warp) * op->ld[2] + n0 + c4;
+    const float* from = stage + warp * kTcStagePitch + c4;
+#pragma unroll 2
+    for (int row = warp; row < rows; row += kComputeWarps) {
+        const float4 q = *reinterpret_cast<const float4*>(from);
+        red_add_f32x4(O, q.x, q.y, q.z, q.w);
+        O += step;
+        from += kComputeWarps * kTcStagePitch;
+    }
+}
+
 // Epilogue, second half, plain tiles (not a split-K partial, not swiglu): out = act(acc + bias) + residual, 128 columns.
 // Specialised at compile time on output type, residual kind and whether there is an activation: with those as
 // run-time switches inside the row loop the writer was instruction-bound (4.2 us per 128 x 128 tile against 1.3 us
-// for the same stores from a specialised loop, measured stand-alone).  All residual rows of a warp (16) are
-// requested before the first is used: two loads in flight per warp made a residual tile take 8.7 us, sixteen 2.3 us.
+// for the same stores from a specialised loop, measured stand-alone).  A loop over groups of rows whose residual is requested a group
+// ahead: all sixteen rows of a warp requested at once are straight-line code that is fetched cold once per op, 6.0 us for a tile
+// with a residual inside a prompt of 333 tokens; now 3.7.
 template <int ODT, int RKIND, bool ACT>              // RKIND 0: no residual, 1: 16-bit (bf16 / fp16 by rdt), 2: fp32
 static __device__ __noinline__ void tc_store_rows_t(const mk_op_desc* op, const float* stage, int m0, int rows, int col0, int n_out) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -135,92 +150,118 @@ static __device__ __noinline__ void tc_store_rows_t(const mk_op_desc* op, const 
         const uint2 w = __ldg(reinterpret_cast<const uint2*>(bias + (long long)col * 2));
         b4[0] = bf16_lo(w.x); b4[1] = bf16_hi(w.x); b4[2] = bf16_lo(w.y); b4[3] = bf16_hi(w.y);
     }
-    constexpr int kRows = 128 / kComputeWarps;          // rows of the tile per warp
+    constexpr int kGroup = RKIND ? 4 : 2;
     const long long ldo = op->ld[2], ldr = op->ld[4];
     uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + ((long long)m0 * ldo + col) * (ODT == DT_F32 ? 4 : 2);
     const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]) + ((long long)m0 * ldr + col) * (RKIND == 2 ? 4 : 2);
-    uint2 r16[RKIND == 1 ? kRows : 1];
-    float4 r32[RKIND == 2 ? kRows : 1];
-    if (RKIND == 1) {
+    uint2 n16[kGroup];
+    float4 n32[kGroup];
+    auto request = [&](int row) {
 #pragma unroll
-        for (int j = 0; j < kRows; ++j) {
-            const int row = warp + j * kComputeWarps;
-            r16[j] = row < rows ? __ldcg(reinterpret_cast<const uint2*>(R + row * ldr * 2)) : make_uint2(0u, 0u);
+        for (int j = 0; j < kGroup; ++j) {
+            if (RKIND == 0 || row + j * kComputeWarps >= rows) break;
+            if (RKIND == 1) n16[j] = __ldcg(reinterpret_cast<const uint2*>(R + (row + j * kComputeWarps) * ldr * 2));
+            if (RKIND == 2) n32[j] = __ldcg(reinterpret_cast<const float4*>(R + (row + j * kComputeWarps) * ldr * 4));
         }
-    }
-    if (RKIND == 2) {
+    };
+    request(warp);
+#pragma unroll 1
+    for (int row0 = warp; row0 < rows; row0 += kGroup * kComputeWarps) {
+        uint2 r16[kGroup];
+        float4 r32[kGroup];
 #pragma unroll
-        for (int j = 0; j < kRows; ++j) {
-            const int row = warp + j * kComputeWarps;
-            r32[j] = row < rows ? __ldcg(reinterpret_cast<const float4*>(R + row * ldr * 4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < kGroup; ++j) {
+            if (RKIND == 1) r16[j] = n16[j];
+            if (RKIND == 2) r32[j] = n32[j];
         }
-    }
+        request(row0 + kGroup * kComputeWarps);
 #pragma unroll
-    for (int j = 0; j < kRows; ++j) {
-        const int row = warp + j * kComputeWarps;
-        if (row >= rows) break;
-        const float4 q = *reinterpret_cast<const float4*>(stage + row * kTcStagePitch + c4);
-        float f[4] = {q.x + b4[0], q.y + b4[1], q.z + b4[2], q.w + b4[3]};
-        if (ACT) {
+        for (int j = 0; j < kGroup; ++j) {
+            const int row = row0 + j * kComputeWarps;
+            if (row >= rows) break;
+            const float4 q = *reinterpret_cast<const float4*>(stage + row * kTcStagePitch + c4);
+            float f[4] = {q.x + b4[0], q.y + b4[1], q.z + b4[2], q.w + b4[3]};
+            if (ACT) {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) f[e] = apply_act(act, f[e]);
-        }
-        if (RKIND == 1) {
-            if (rdt == DT_F16) {
-                const float2 lo = unpack2h(r16[j].x), hi = unpack2h(r16[j].y);
-                f[0] += lo.x; f[1] += lo.y; f[2] += hi.x; f[3] += hi.y;
-            } else {
-                f[0] += bf16_lo(r16[j].x); f[1] += bf16_hi(r16[j].x); f[2] += bf16_lo(r16[j].y); f[3] += bf16_hi(r16[j].y);
+                for (int e = 0; e < 4; ++e) f[e] = apply_act(act, f[e]);
             }
+            if (RKIND == 1) {
+                if (rdt == DT_F16) {
+                    const float2 lo = unpack2h(r16[j].x), hi = unpack2h(r16[j].y);
+                    f[0] += lo.x; f[1] += lo.y; f[2] += hi.x; f[3] += hi.y;
+                } else {
+                    f[0] += bf16_lo(r16[j].x); f[1] += bf16_hi(r16[j].x); f[2] += bf16_lo(r16[j].y); f[3] += bf16_hi(r16[j].y);
+                }
+            }
+            if (RKIND == 2) { f[0] += r32[j].x; f[1] += r32[j].y; f[2] += r32[j].z; f[3] += r32[j].w; }
+            if (ODT == DT_F32) *reinterpret_cast<float4*>(O + row * ldo * 4) = make_float4(f[0], f[1], f[2], f[3]);
+            else if (ODT == DT_F16) *reinterpret_cast<uint2*>(O + row * ldo * 2) = make_uint2(pack2h(f[0], f[1]), pack2h(f[2], f[3]));
+            else *reinterpret_cast<uint2*>(O + row * ldo * 2) = make_uint2(pack2(f[0], f[1]), pack2(f[2], f[3]));
         }
-        if (RKIND == 2) { f[0] += r32[j].x; f[1] += r32[j].y; f[2] += r32[j].z; f[3] += r32[j].w; }
-        if (ODT == DT_F32) *reinterpret_cast<float4*>(O + row * ldo * 4) = make_float4(f[0], f[1], f[2], f[3]);
-        else if (ODT == DT_F16) *reinterpret_cast<uint2*>(O + row * ldo * 2) = make_uint2(pack2h(f[0], f[1]), pack2h(f[2], f[3]));
-        else *reinterpret_cast<uint2*>(O + row * ldo * 2) = make_uint2(pack2(f[0], f[1]), pack2(f[2], f[3]));
     }
 }
-// Rotated heads (descriptor: op_gemm.cuh): the other half of a head is in the staging rows too.  All table rows of a warp are
-// requested before the first is used.
+// Epilogue straight from tensor memory to 16-bit outputs, a row per thread and 32 bytes at a time, for tiles that read another operand
+// beside the accumulator: what the first columns need is requested before the accumulator is complete.
+//   rotated heads (descriptor: op_gemm.cuh): 16 columns of both halves of a head at a time, with the row's piece of the tables
+// Through the staging rows a tile's second half took 6.6 us, as straight-line code for 16 rows per warp that is fetched cold once per op;
+// as a loop over four rows at a time 5.3, a round trip to L2 for each turn's table rows.  This form takes 3.9 from the complete accumulator,
+// first half included (7.8): a prompt of 333 tokens 1789 -> 1752 us.
 template <int ODT>
-static __device__ __noinline__ void tc_store_rows_rope(const mk_op_desc* op, const float* stage, int m0, int rows, int col0, int n_out) {
-    constexpr int kRows = 128 / kComputeWarps;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int c4 = lane * 4, col = col0 + c4;
-    if (col >= n_out) return;
-    const int D = op->i[15], half = D >> 1, seq = op->i[16], d = c4 & (D - 1);
-    const bool rot = col < op->i[14], low = d < half, t16 = op->i[17] == DT_F16;
-    const int other = low ? c4 + half : c4 - half;
-    const long long ldo = op->ld[2];
-    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + ((long long)m0 * ldo + col) * 2;
-    uint2 cs[kRows], sn[kRows];
-    if (rot) {
-        int tok = (m0 + warp) % seq;
-#pragma unroll
-        for (int j = 0; j < kRows; ++j) {
-            if (warp + j * kComputeWarps < rows) {
-                cs[j] = __ldcg(reinterpret_cast<const uint2*>(op->ptr[6] + ((long long)tok * op->ld[6] + d) * 2));
-                sn[j] = __ldcg(reinterpret_cast<const uint2*>(op->ptr[7] + ((long long)tok * op->ld[7] + d) * 2));
-            }
-            tok += kComputeWarps;
-            while (tok >= seq) tok -= seq;
-        }
-    }
-    auto get = [&](uint32_t w) { return t16 ? unpack2h(w) : make_float2(bf16_lo(w), bf16_hi(w)); };
-    const float sign = low ? -1.f : 1.f;
-#pragma unroll
-    for (int j = 0; j < kRows; ++j) {
-        const int row = warp + j * kComputeWarps;
-        if (row >= rows) break;
-        float4 f = *reinterpret_cast<const float4*>(stage + row * kTcStagePitch + c4);
+static __device__ __noinline__ bool tc_rope_direct(const Params& p, Ctrl* c, const mk_op_desc* op, uint32_t two, uint32_t apar, int m0, int n0,
+                                                   int seq) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, qd = warp & 3, h = warp >> 2;
+    const int D = op->i[15], half = D >> 1, M = op->i[0];
+    const int row = m0 + qd * 32 + lane, safe = min(row, M - 1), tok = safe % op->i[16];
+    const bool t16 = op->i[17] == DT_F16;
+    // D = 64: the warp's 64 columns are a head; D = 128: its share of the tile's one head is 32 columns of either half
+    const int col0 = D == 64 ? 64 * h : 32 * h, d0 = D == 64 ? 0 : 32 * h;
+    const bool rot = n0 + col0 < op->i[14];
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + ((long long)safe * op->ld[2] + n0 + col0) * 2;
+    const uint8_t* C = reinterpret_cast<const uint8_t*>(op->ptr[6]) + ((long long)tok * op->ld[6] + d0) * 2;
+    const uint8_t* S = reinterpret_cast<const uint8_t*>(op->ptr[7]) + ((long long)tok * op->ld[7] + d0) * 2;
+    const bool whole = ((op->ptr[2] | (uint64_t)op->ld[2] * 2) & 31) == 0;
+    uint4 q[8];                                              // cos of both halves, sin of both halves
+    auto request = [&](int d) {
         if (rot) {
-            const float4 g = *reinterpret_cast<const float4*>(stage + row * kTcStagePitch + other);
-            const float2 c01 = get(cs[j].x), c23 = get(cs[j].y), s01 = get(sn[j].x), s23 = get(sn[j].y);
-            f = make_float4(f.x * c01.x + g.x * (sign * s01.x), f.y * c01.y + g.y * (sign * s01.y), f.z * c23.x + g.z * (sign * s23.x),
-                            f.w * c23.y + g.w * (sign * s23.y));
+#pragma unroll
+            for (int k = 0; k < 8; ++k) q[k] = __ldcg(reinterpret_cast<const uint4*>((k < 4 ? C : S) + (d + (k & 2 ? half : 0)) * 2 + (k & 1) * 16));
         }
-        *reinterpret_cast<uint2*>(O + row * ldo * 2) =
-            ODT == DT_F16 ? make_uint2(pack2h(f.x, f.y), pack2h(f.z, f.w)) : make_uint2(pack2(f.x, f.y), pack2(f.z, f.w));
+    };
+    request(0);
+    int ok = 1;
+    if (lane == 0) ok = wait_barrier(p, c, &c->acc_full, apar, seq, WHERE_COMBINE) ? 1 : 0;
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    tc_fence_after();
+    phase_mark(p, c, 2);
+    __syncwarp();
+    if (!ok || m0 + qd * 32 >= M || n0 + col0 >= op->i[1]) return ok != 0;
+    const uint32_t tl = *(volatile uint32_t*)&c->tmem_base + ((uint32_t)(qd * 32) << 16) + col0;
+    auto get = [&](uint32_t w) { return t16 ? unpack2h(w) : make_float2(bf16_lo(w), bf16_hi(w)); };
+#pragma unroll 1
+    for (int d = 0; d < 32; d += 16) {
+        float x1[16], x2[16];
+        tc_ld16_sum(tl + d, two, x1);
+        tc_ld16_sum(tl + half + d, two, x2);
+        if (rot) {
+#pragma unroll
+            for (int e = 0; e < 16; e += 2) {
+                const uint32_t* t = reinterpret_cast<const uint32_t*>(q);
+                const float2 c1 = get(t[e / 2]), c2 = get(t[8 + e / 2]), s1 = get(t[16 + e / 2]), s2 = get(t[24 + e / 2]);
+                const float u0 = x1[e], v0 = x2[e], u1 = x1[e + 1], v1 = x2[e + 1];
+                x1[e] = u0 * c1.x - v0 * s1.x;
+                x2[e] = v0 * c2.x + u0 * s2.x;
+                x1[e + 1] = u1 * c1.y - v1 * s1.y;
+                x2[e + 1] = v1 * c2.y + u1 * s2.y;
+            }
+        }
+        if (d == 0) request(16);
+        if (row < M) {
+            put16<ODT>(O + d * 2, x1, whole);
+            put16<ODT>(O + (half + d) * 2, x2, whole);
+        }
+        __syncwarp();
     }
+    return true;
 }
 template <int ODT>
 __device__ __forceinline__ void tc_store_rows_o(const mk_op_desc* op, const float* stage, int m0, int rows, int col0, int n_out) {
@@ -358,64 +399,67 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
     __syncwarp();
 
     // ---- epilogue: warp w owns lanes 32 (w & 3) .. +31 (activation rows) and column half w >> 2 ----
-    int ok = 1;
-    if (lane == 0) ok = wait_barrier(p, c, &c->acc_full, apar, seq, WHERE_COMBINE) ? 1 : 0;
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    tc_fence_after();
-    phase_mark(p, c, 2);                                                    // accumulator complete
-    __syncwarp();                                                           // (the tensor-memory loads below are .sync.aligned: whole warp, converged)
-    // first half: tensor memory -> shared memory, 16 columns at a time (32 at a time needed so many registers that each call saved 320 bytes
-    // per thread instead of 204, with almost no L1 to take them: 64 sequences at context 1024 1544 -> 1526 us, prompt of 333 tokens
-    // 1865 -> 1845, MLP block of 256 rows 57.9 -> 56.6).  Warp w reads lanes 32 (w & 3) .. +31 (activation
-    // rows) and column half w >> 2; the activation stages are free now (every MMA has completed).
-    const int qd = warp & 3, h = warp >> 2;
-    float* stage = reinterpret_cast<float*>(work + kTcXOff);
-    const int rows = min(128, M - m0);
     const uint32_t two = nk > 1 ? 128u : 0u;                               // columns to the second issuing thread's accumulator, if it has a part
-    if (ok && qd * 32 < rows) {
-        const uint32_t tl = tmem + ((uint32_t)(qd * 32) << 16);
-        float* srow = stage + (qd * 32 + lane) * kTcStagePitch;
-        float v[16];
-        if (swi) {
-            // gate columns 32 h .. +31 and the up columns 64 further of the same outputs
+    int ok = 1;
+    if (op->ptr[6] && !op->i[6] && !swi) {
+        ok = op->i[5] == DT_F16 ? tc_rope_direct<DT_F16>(p, c, op, two, apar, m0, n0, seq) : tc_rope_direct<DT_BF16>(p, c, op, two, apar, m0, n0, seq);
+    } else {
+        if (lane == 0) ok = wait_barrier(p, c, &c->acc_full, apar, seq, WHERE_COMBINE) ? 1 : 0;
+        ok = __shfl_sync(0xffffffffu, ok, 0);
+        tc_fence_after();
+        phase_mark(p, c, 2);                                                    // accumulator complete
+        __syncwarp();                                                           // (the tensor-memory loads below are .sync.aligned: whole warp, converged)
+        // first half: tensor memory -> shared memory, 16 columns at a time (32 at a time needed so many registers that each call saved 320 bytes
+        // per thread instead of 204, with almost no L1 to take them: 64 sequences at context 1024 1544 -> 1526 us, prompt of 333 tokens
+        // 1865 -> 1845, MLP block of 256 rows 57.9 -> 56.6).  Warp w reads lanes 32 (w & 3) .. +31 (activation
+        // rows) and column half w >> 2; the activation stages are free now (every MMA has completed).
+        const int qd = warp & 3, h = warp >> 2;
+        float* stage = reinterpret_cast<float*>(work + kTcXOff);
+        const int rows = min(128, M - m0);
+        if (ok && qd * 32 < rows) {
+            const uint32_t tl = tmem + ((uint32_t)(qd * 32) << 16);
+            float* srow = stage + (qd * 32 + lane) * kTcStagePitch;
+            float v[16];
+            if (swi) {
+                // gate columns 32 h .. +31 and the up columns 64 further of the same outputs
 #pragma unroll 1
-            for (int ch = 0; ch < 2; ++ch) {
-                const int tcol = h * 32 + ch * 16;
-                float u[16];
-                tc_ld16_sum(tl + tcol, two, v);
-                tc_ld16_sum(tl + 64 + tcol, two, u);
+                for (int ch = 0; ch < 2; ++ch) {
+                    const int tcol = h * 32 + ch * 16;
+                    float u[16];
+                    tc_ld16_sum(tl + tcol, two, v);
+                    tc_ld16_sum(tl + 64 + tcol, two, u);
 #pragma unroll
-                for (int j = 0; j < 16; j += 4)
-                    *reinterpret_cast<float4*>(srow + tcol + j) =
-                        make_float4(v[j] * sigmoidf_(v[j]) * u[j], v[j + 1] * sigmoidf_(v[j + 1]) * u[j + 1],
-                                    v[j + 2] * sigmoidf_(v[j + 2]) * u[j + 2], v[j + 3] * sigmoidf_(v[j + 3]) * u[j + 3]);
-            }
-        } else {
+                    for (int j = 0; j < 16; j += 4)
+                        *reinterpret_cast<float4*>(srow + tcol + j) =
+                            make_float4(v[j] * sigmoidf_(v[j]) * u[j], v[j + 1] * sigmoidf_(v[j + 1]) * u[j + 1],
+                                        v[j + 2] * sigmoidf_(v[j + 2]) * u[j + 2], v[j + 3] * sigmoidf_(v[j + 3]) * u[j + 3]);
+                }
+            } else {
 #pragma unroll 1
-            for (int ch = 0; ch < 4; ++ch) {
-                const int tcol = h * 64 + ch * 16;
-                if (n0 + tcol >= N) break;
-                tc_ld16_sum(tl + tcol, two, v);
+                for (int ch = 0; ch < 4; ++ch) {
+                    const int tcol = h * 64 + ch * 16;
+                    if (n0 + tcol >= N) break;
+                    tc_ld16_sum(tl + tcol, two, v);
 #pragma unroll
-                for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(srow + tcol + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    for (int j = 0; j < 16; j += 4) *reinterpret_cast<float4*>(srow + tcol + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                }
             }
+        }
+        tc_fence_before();
+        compute_sync();
+        if (ok) {
+            if (swi) tc_write_rows(op, stage, m0, rows, 64, a1 * 64, N / 2);
+            else if (op->i[6]) {                                                            // split-K partial: reduce-add
+                if (op->i[5] == DT_F32) tc_reduce_rows(op, stage, m0, rows, n0, N);
+                else tc_write_rows(op, stage, m0, rows, 128, n0, N);
+            }
+            else tc_store_rows(op, stage, m0, rows, n0, N);
         }
     }
     tc_fence_before();
-    compute_sync();
-    if (ok) {
-        if (swi) tc_write_rows(op, stage, m0, rows, 64, a1 * 64, N / 2);
-        else if (op->i[6]) tc_write_rows(op, stage, m0, rows, 128, n0, N);              // split-K partial: reduce-add
-        else if (op->ptr[6]) {
-            if (op->i[5] == DT_F16) tc_store_rows_rope<DT_F16>(op, stage, m0, rows, n0, N);
-            else tc_store_rows_rope<DT_BF16>(op, stage, m0, rows, n0, N);
-        }
-        else tc_store_rows(op, stage, m0, rows, n0, N);
-    }
-    tc_fence_before();
-    const bool aborting = compute_sync_or(!ok || *(volatile int*)&c->abort);
-    if (aborting) return -1;                                            // (x_par and x_left stay: wait_x_landed)
-    if (t == 0) tc_finish_state(c, uses, xpar0, ws0, wph0, nk, xstages);
+    // (no barrier: the one that publishes the instruction tells every thread of a wait that gave up, Ctrl::abort.  Thread 0 has seen the
+    // accumulator complete, so every tile has landed; else x_par and x_left stay as they are, for wait_x_landed)
+    if (t == 0 && ok) tc_finish_state(c, uses, xpar0, ws0, wph0, nk, xstages);
     return 0;
 }
 

@@ -247,40 +247,6 @@ __device__ __forceinline__ void act_all(int act, float* v) {
     }
 }
 
-// A thread writes (and, with a residual, reads) whole 32-byte pieces of its own row: whole sectors, as good as 128 bytes of four
-// rows at a time, without the detour through shared memory that the operands of the next tile are streaming through (64
-// bytes a cycle in, 96 out to the tensor core).  DiT, 32 images: 8.95 -> 8.82 ms together with the prefetch of the residual; what is
-// left (4.6 us for 256 x 256 16-bit outputs, 11 with a residual) is the memory system taking the bursts of all SMs at once.
-// `whole`: the rows start on 32-byte boundaries; else two 16-byte accesses.
-__device__ __forceinline__ void st32B(uint8_t* at, const uint32_t* w, bool whole) {
-    if (whole)
-        asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(at), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
-                     "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7])
-                     : "memory");
-    else {
-        reinterpret_cast<uint4*>(at)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        reinterpret_cast<uint4*>(at)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-    }
-}
-__device__ __forceinline__ void ld32B(const uint8_t* at, uint32_t* w, bool whole) {
-    if (whole)
-        asm volatile("ld.global.cg.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
-                     : "l"(at)
-                     : "memory");
-    else {
-        const uint4 a = __ldcg(reinterpret_cast<const uint4*>(at)), b = __ldcg(reinterpret_cast<const uint4*>(at) + 1);
-        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
-    }
-}
-// 16 columns of a row as 16-bit, 32 columns of a row
-template <int DT>
-__device__ __forceinline__ void put16(uint8_t* at, const float* v, bool whole) {
-    uint32_t w[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) w[e] = DT == DT_F16 ? pack2h(v[2 * e], v[2 * e + 1]) : pack2(v[2 * e], v[2 * e + 1]);
-    st32B(at, w, whole);
-}
 template <int DT>
 __device__ __forceinline__ void put32(uint8_t* at, const float* v, bool whole) {
     if (DT == DT_F32) {
@@ -415,19 +381,6 @@ __device__ __forceinline__ void wide_store_res(const Params& p, Ctrl* c, const m
     }
 }
 
-// 16 columns of this thread's lane, twice
-__device__ __forceinline__ void tc_ld16x2(uint32_t ta, uint32_t tb, float* a, float* b) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n\t"
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=f"(a[0]), "=f"(a[1]), "=f"(a[2]), "=f"(a[3]), "=f"(a[4]), "=f"(a[5]), "=f"(a[6]), "=f"(a[7]), "=f"(a[8]), "=f"(a[9]),
-          "=f"(a[10]), "=f"(a[11]), "=f"(a[12]), "=f"(a[13]), "=f"(a[14]), "=f"(a[15]), "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(b[3]),
-          "=f"(b[4]), "=f"(b[5]), "=f"(b[6]), "=f"(b[7]), "=f"(b[8]), "=f"(b[9]), "=f"(b[10]), "=f"(b[11]), "=f"(b[12]), "=f"(b[13]),
-          "=f"(b[14]), "=f"(b[15])
-        : "r"(ta), "r"(tb)
-        : "memory");
-}
 // 16-bit outputs whose first i 14 columns are heads (i 15 = 64 or 128 columns each) to be rotated: row r by row r mod i 16 of the 16-bit
 // cos and sin tables (ptr 6, 7).  16 columns of both halves of a head at a time, for all heads of the tile, so that a thread
 // reads its table row once per tile (64 KB beside 128 KB of output; once per head it would be 256).  The first such piece of

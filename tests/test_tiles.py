@@ -77,6 +77,37 @@ def test_activation_copies_of_the_rows_there_are(cuda, M):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K", [(9, 128, 64), (32, 136, 64), (33, 128, 128), (63, 264, 192), (97, 128, 64), (128, 8, 128)])
+@pytest.mark.parametrize("res,act", [(BF, None), (F32, None), (BF, "silu"), (None, "gelu_tanh"), (None, None)])
+def test_row_groups_of_an_epilogue(cuda, M, N, K, res, act):
+    """Rows that end anywhere in a warp's groups of four, one accumulator (one k-tile) or two, columns that end inside a tile."""
+    g = mc.Graph()
+    t = {"x": rnd((M, K), 1.0, 1), "w": rnd((N, K), K ** -0.5, 2), "b": rnd((1, N), 0.5, 3), "r": rnd((M, N), 1.0, 4).to(res or BF)}
+    y = g.linear(g.input("x", (M, K)), g.param("w", (N, K)), bias=g.param("b", (1, N)), act=act, residual=g.input("r", (M, N), res) if res else None)
+    g.output(y)
+    outs, ref, _, _, prog = run_both(g, t if res else {k: v for k, v in t.items() if k != "r"}, cuda)
+    assert prog.tcgen05_ops == 1 and rel_l2(outs[0], ref[0]) < ONE_ROUNDING
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("B,S,H,KVH,D,K", [(1, 130, 1, 1, 64, 64), (5, 30, 3, 1, 64, 128), (3, 3, 2, 2, 64, 64), (1, 128, 1, 1, 128, 64), (2, 65, 4, 2, 128, 192)])
+def test_rotated_heads_at_tile_edges(cuda, B, S, H, KVH, D, K):
+    """128 x 128 tiles whose last one is half empty or holds rotated and other heads, sequences that wrap inside a warp's rows."""
+    g = mc.Graph()
+    x, w = g.input("x", (B * S, K)), g.param("w", ((H + 2 * KVH) * D, K))
+    cos, sin = g.input("cos", (S, D)), g.input("sin", (S, D))
+    qkv = g.linear(x, w)
+    q = g.rope(qkv.cols_slice(0, H * D), cos, sin, heads=H, head_dim=D, seq=S)
+    k = g.rope(qkv.cols_slice(H * D, KVH * D), cos, sin, heads=KVH, head_dim=D, seq=S)
+    g.output(g.attention(q, k, qkv.cols_slice((H + KVH) * D, KVH * D), batch=B, heads=H, kv_heads=KVH, head_dim=D, causal=True))
+    cs, sn = W.rope_tables(S, D)
+    t = {"x": rnd((B * S, K), 1.0, 1), "w": rnd(((H + 2 * KVH) * D, K), 0.1, 2), "cos": cs, "sin": sn}
+    outs, ref, _, _, prog = run_both(g, t, cuda)
+    assert not any(o.kind == "Rope" for o in prog.g.ops) and prog.tcgen05_ops == 1
+    assert rel_l2(outs[0], ref[0]) < TOL
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("tcgen05", [True, False])
 @pytest.mark.parametrize("B,S,D,tile", [(1, 150, 64, (128, 128)), (3, 50, 128, (128, 128)), (2, 129, 64, (256, 256)), (1, 257, 128, (256, 128)),
                                         (1, 300, 128, (256, 256))])
