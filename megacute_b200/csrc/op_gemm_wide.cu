@@ -20,6 +20,22 @@ static __device__ __noinline__ int wide_run(const Params& p, int idx, int slot) 
         [&] { if (threadIdx.x == 0) m.ctrl->wide_uses += 1; });
 }
 
+// Behind the last instruction of a variant's run: is the CTA's next one of another variant?  (Out of line: so that the registers it needs
+// are not saved around the whole run: 88 -> 48 bytes.)
+static __device__ __noinline__ bool wide_goes_on(const Params& p, int last, int slot) {
+    Ctrl* c = smem_map().ctrl;
+    if (next_is(p, c, last, slot, [](const mk_op_desc* op) { return is_wide_gemm(op); })) {
+        stage_following(p, c, last + (int)gridDim.x, slot + 1);
+        return true;
+    }
+    // (behind the last instruction's barrier: nobody reads the staging rows any more)
+    if (threadIdx.x == 0) {
+        __threadfence_block();
+        *(volatile uint32_t*)&c->wide_done = c->wide_uses;
+    }
+    return false;
+}
+
 __device__ int mk_run_gemm_wide(const Params& p, int idx, int slot) {
     const SmemMap m = smem_map();
     const Meta* mt = &m.ctrl->meta;
@@ -40,17 +56,9 @@ __device__ int mk_run_gemm_wide(const Params& p, int idx, int slot) {
         }
         if (last < 0) return -1;
         slot += (last - idx) / (int)gridDim.x;                  // (the last instruction's; not Ctrl::run_slot: thread 0 may be in the next run already)
-        if (!next_is(p, m.ctrl, last, slot, [](const mk_op_desc* op) { return is_wide_gemm(op); })) {
-            // (behind the last instruction's barrier: nobody reads the staging rows any more)
-            if (threadIdx.x == 0) {
-                __threadfence_block();
-                *(volatile uint32_t*)&m.ctrl->wide_done = m.ctrl->wide_uses;
-            }
-            return last;
-        }
+        if (!wide_goes_on(p, last, slot)) return last;
         idx = last + (int)gridDim.x;
         ++slot;
-        stage_following(p, m.ctrl, idx, slot);
     }
 }
 

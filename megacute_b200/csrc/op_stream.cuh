@@ -313,121 +313,127 @@ __device__ __forceinline__ void op_eltwise(const mk_op_desc* op, int a0, int a1)
 
 // ---- norms ---------------------------------------------------------------------------------------------------------------------
 // MK_OP_NORM with i 3 >= 8 rows per instruction (descriptor: op_pointwise.cuh): rows r0 + warp, + 8, ..., a row per warp.  Bound by
-// memory latency: an SM gets what it has requested per round trip (2 us with all SMs streaming), so each warp keeps 12 KB of
-// rows on their way through the work area (DEEP; 64 rows of 2048 fp16: 26.8 -> 14.4 us).  A lane reads back what it
-// copied itself.  With one or two rows per warp there is nothing to run ahead of: the next row in registers (8 rows 5.1 us, 6.0
-// through the work area).  Gain, and scale and shift of the current
-// group of rows, stay in registers.  NPER: 8-element vectors of a row per lane.  HW: gain.  MOD: scale and shift.
-constexpr int kNormAhead = 12288;                          // bytes of rows a warp has requested
-template <int NPER, int XDT, int ODT, bool HW, bool MOD, bool DEEP>
+// memory latency: an SM gets what it has requested per round trip (2 us with all SMs streaming), so each warp keeps 10 to 12 KB of
+// rows on their way through the work area (64 rows of 2048 fp16 one row ahead: 26.8 us, so 14.4).  A lane reads back what it copied
+// itself, twice: for the sums and for the result.
+// The body runs once per op on an SM, between bodies with other registers, so what it keeps in registers is saved and restored around it
+// and what it unrolls is fetched cold: with a row, the gain and the group's scale and shift in registers it saved 296 to 464 bytes per
+// thread and took 7 us to its first row (64 rows of 1024, DiT).  So the gain, or scale and shift of the rows' group, are in shared memory
+// too: 8 bytes saved, the op 20 -> 15 us (with what lies between it and the linear in front of it), DiT of 32 images 8409 -> 8164, of 4 images
+// 3453 -> 3158, MLP block of 3001 rows 197.5 -> 193.5 us.
+// NPER: 8-element vectors of a row per lane.  HW: gain.  MOD: scale and shift.
+template <int NPER, int XDT, int ODT, bool HW, bool MOD>
 __device__ __forceinline__ void norm_stream(const mk_op_desc* op, int r0, int rows) {
-    constexpr bool kAhead = !DEEP && (XDT != DT_F32 || NPER <= 4);    // (two fp32 rows of 2048 do not fit)
-    constexpr int kPlanes = XDT == DT_F32 ? 2 : 1, kRow = NPER * kPlanes * 512, kDepth = kNormAhead / kRow;     // 16 bytes of a vector per plane
-    static_assert(kDepth >= 1 && kTcXOff + kComputeWarps * kNormAhead <= kWorkBytes, "norm rows exceed the work area");
-    const int Cc = op->i[1], rms = op->i[2], group = max(1, op->i[6]);
+    constexpr int kShared = MOD ? NPER * 2048 : HW ? NPER * 512 : 0;         // bytes of gain, or of scale and shift as fp32
+    constexpr int kAhead = (kWorkBytes - kTcXOff - kShared) / kComputeWarps;  // ... of rows a warp has requested
+    constexpr int kPlanes = XDT == DT_F32 ? 2 : 1, kRow = NPER * kPlanes * 512, kDepth = kAhead / kRow;      // 16 bytes of a vector per plane
+    constexpr int kSharedOff = kTcXOff + kComputeWarps * kDepth * kRow;
+    static_assert(kDepth >= 1 && kSharedOff + kShared <= kWorkBytes, "norm rows exceed the work area");
+    const int Cc = op->i[1], rms = op->i[2], group = MOD ? max(1, op->i[6]) : op->i[0];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = Cc >> 3;
-    const void* X = reinterpret_cast<const void*>(op->ptr[0]);
-    void* O = reinterpret_cast<void*>(op->ptr[1]);
     const float inv = 1.0f / (float)Cc, eps = op->f[0];
     const long long ldx = op->ld[0], ldo = op->ld[1];
-    Vec8<DT_BF16> gw[HW ? NPER : 1];
-    float sc[MOD ? NPER * 8 : 1], sh[MOD ? NPER * 8 : 1];
     // (columns beyond the row are clamped to its last vector and left out of the sums and stores)
-    auto column = [&](int u) { return (long long)min(lane + u * 32, nvec - 1) * 8; };
-    uint8_t* buf = smem_map().work + kTcXOff + warp * kNormAhead + lane * 16;
-    Vec8<XDT> x[NPER], nx[kAhead ? NPER : 1];
-    auto fetch = [&](int rr, Vec8<XDT>* x) {
-#pragma unroll
-        for (int u = 0; u < NPER; ++u) x[u].load(X, (r0 + rr) * ldx + column(u));
-    };
+    auto column = [&](int u) { return min(lane + u * 32, nvec - 1) * 8; };
+    uint8_t* work = smem_map().work;
+    uint8_t* buf = work + kTcXOff + warp * (kDepth * kRow) + lane * 16;
+    uint8_t* shared = work + kSharedOff;                      // (lane's vectors as in the rows; scale and shift: four planes of 16 bytes per vector)
     auto request = [&](int rr, int slot) {
         if (rr < rows) {
+            const uint8_t* from = reinterpret_cast<const uint8_t*>(op->ptr[0]) + (r0 + rr) * ldx * (kPlanes * 2);
 #pragma unroll
             for (int u = 0; u < NPER; ++u)
 #pragma unroll
-                for (int k = 0; k < kPlanes; ++k)
-                    cp_async16(buf + slot * kRow + (u * kPlanes + k) * 512,
-                               reinterpret_cast<const uint8_t*>(X) + ((r0 + rr) * ldx + column(u)) * (kPlanes * 2) + k * 16, true);
+                for (int k = 0; k < kPlanes; ++k) cp_async16(buf + slot * kRow + (u * kPlanes + k) * 512, from + column(u) * (kPlanes * 2) + k * 16, true);
         }
         cp_async_commit();
     };
-    auto modulation = [&](long long g) {
-#pragma unroll
-        for (int u = 0; u < NPER; ++u) {
-            load8(reinterpret_cast<const void*>(op->ptr[4]), g * op->ld[4] + column(u), op->i[7], sc + (MOD ? u * 8 : 0));
-            load8(reinterpret_cast<const void*>(op->ptr[5]), g * op->ld[5] + column(u), op->i[8], sh + (MOD ? u * 8 : 0));
-        }
-    };
-    if (warp >= rows) return;
-    if (DEEP) {
-#pragma unroll
-        for (int d = 0; d < kDepth; ++d) request(warp + d * kComputeWarps, d);
-    } else if (kAhead) {
-        fetch(warp, nx);
-    }
-    int grp = (r0 + warp) / group;
-    if (HW) {
-#pragma unroll
-        for (int u = 0; u < NPER; ++u) gw[HW ? u : 0].load(reinterpret_cast<const void*>(op->ptr[2]), column(u));
-    }
-    if (MOD) modulation(grp);
-    int slot = 0;
+    int next = warp, slot = 0, rr = warp;
+    // (the gain travels with the first rows, and is waited for between a warp's first sums and its first result)
+    bool gain_there = !HW;
+    if (HW)
+        for (int v = threadIdx.x; v < NPER * 32; v += kComputeThreads)
+            cp_async16(shared + v * 16, reinterpret_cast<const uint8_t*>(op->ptr[2]) + min(v, nvec - 1) * 16, true);
 #pragma unroll 1
-    for (int rr = warp; rr < rows; rr += kComputeWarps) {
-        if (DEEP) {
+    for (int d = 0; d < kDepth; ++d, next += kComputeWarps) request(next, d);
+#pragma unroll 1
+    for (int grp = r0 / group;; ++grp) {
+        const int end = MOD ? min(rows, (grp + 1) * group - r0) : rows;          // the instruction's rows of this group (most have one group)
+        if (MOD) {
+            if (grp > r0 / group) compute_sync();                                // (the group before has been read)
+            for (int v = threadIdx.x; v < 2 * NPER * 32; v += kComputeThreads) {
+                const int which = v >= NPER * 32, u = v - which * NPER * 32;
+                float f[8];
+                load8(reinterpret_cast<const void*>(op->ptr[4 + which]), (long long)grp * op->ld[4 + which] + min(u, nvec - 1) * 8, op->i[7 + which], f);
+                float4* to = reinterpret_cast<float4*>(shared) + which * NPER * 64 + u;
+                to[0] = make_float4(f[0], f[1], f[2], f[3]);
+                to[NPER * 32] = make_float4(f[4], f[5], f[6], f[7]);
+            }
+            compute_sync();
+        }
+#pragma unroll 1
+        for (; rr < end; rr += kComputeWarps, next += kComputeWarps) {
             cp_async_wait<kDepth - 1>();
-#pragma unroll
+            const uint8_t* at = buf + slot * kRow;
+            auto row = [&](int u, float* f) {
+                Vec8<XDT> x;
+                x.raw(*reinterpret_cast<const uint4*>(at + u * kPlanes * 512), *reinterpret_cast<const uint4*>(at + u * kPlanes * 512 + (kPlanes - 1) * 512));
+                x.get(f);
+            };
+            float s = 0.f, ss = 0.f;
+#pragma unroll 4
             for (int u = 0; u < NPER; ++u) {
-                const uint4* at = reinterpret_cast<const uint4*>(buf + slot * kRow + u * kPlanes * 512);
-                x[u].raw(at[0], at[kPlanes == 2 ? 32 : 0]);
+                float f[8];
+                row(u, f);
+                float a = 0.f, q = 0.f;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) { a += f[e]; q = fmaf(f[e], f[e], q); }
+                const bool in = lane + u * 32 < nvec;
+                s += in ? a : 0.f;
+                ss += in ? q : 0.f;
             }
-            request(rr + kDepth * kComputeWarps, slot);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                s += __shfl_xor_sync(0xffffffffu, s, o);
+                ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            }
+            const float mean = rms ? 0.f : s * inv;
+            const float rstd = rsqrt_approx(ss * inv - mean * mean + eps);
+            const long long out = (r0 + rr) * ldo;
+            if (!gain_there) {
+                compute_sync();
+                gain_there = true;
+            }
+#pragma unroll 2
+            for (int u = 0; u < NPER; ++u) {
+                float f[8], g[8], h[8];
+                row(u, f);
+                if (HW) unpack8(reinterpret_cast<const uint4*>(shared)[u * 32 + lane], g);
+                if (MOD) {
+                    const float4* from = reinterpret_cast<const float4*>(shared) + u * 32 + lane;
+#pragma unroll
+                    for (int k = 0; k < 2; ++k) {
+                        const float4 q = from[k * NPER * 32], r = from[(2 + k) * NPER * 32];
+                        g[4 * k] = q.x; g[4 * k + 1] = q.y; g[4 * k + 2] = q.z; g[4 * k + 3] = q.w;
+                        h[4 * k] = r.x; h[4 * k + 1] = r.y; h[4 * k + 2] = r.z; h[4 * k + 3] = r.w;
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    f[e] = (f[e] - mean) * rstd;
+                    if (HW) f[e] *= g[e];
+                    if (MOD) f[e] = fmaf(f[e], 1.0f + g[e], h[e]);
+                }
+                if (lane + u * 32 < nvec) put8<ODT>(reinterpret_cast<void*>(op->ptr[1]), out + (lane + u * 32) * 8, f);
+            }
+            request(next, slot);
             if (++slot == kDepth) slot = 0;
-        } else if (kAhead) {
-#pragma unroll
-            for (int u = 0; u < NPER; ++u) x[u] = nx[kAhead ? u : 0];
-            fetch(min(rr + kComputeWarps, rows - 1), nx);
-        } else {
-            fetch(rr, x);
         }
-        if (MOD && (r0 + rr) / group != grp) { grp = (r0 + rr) / group; modulation(grp); }
-        float s = 0.f, ss = 0.f;
-#pragma unroll
-        for (int u = 0; u < NPER; ++u) {
-            float f[8];
-            x[u].get(f);
-            float a = 0.f, q = 0.f;
-#pragma unroll
-            for (int e = 0; e < 8; ++e) { a += f[e]; q = fmaf(f[e], f[e], q); }
-            const bool in = lane + u * 32 < nvec;
-            s += in ? a : 0.f;
-            ss += in ? q : 0.f;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            s += __shfl_xor_sync(0xffffffffu, s, o);
-            ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        }
-        const float mean = rms ? 0.f : s * inv;
-        const float rstd = rsqrt_approx(ss * inv - mean * mean + eps);
-#pragma unroll
-        for (int u = 0; u < NPER; ++u) {
-            float f[8];
-            x[u].get(f);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = (f[e] - mean) * rstd;
-            if (HW) {
-                float g[8];
-                gw[HW ? u : 0].get(g);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] *= g[e];
-            }
-            if (MOD) {
-#pragma unroll
-                for (int e = 0; e < 8; ++e) f[e] = fmaf(f[e], 1.0f + sc[MOD ? u * 8 + e : 0], sh[MOD ? u * 8 + e : 0]);
-            }
-            if (lane + u * 32 < nvec) put8<ODT>(O, (r0 + rr) * ldo + (lane + u * 32) * 8, f);
-        }
+        if (end >= rows) break;
+    }
+    if (!gain_there) {                                                           // (a warp without a row)
+        cp_async_wait<0>();
+        compute_sync();
     }
 }
 
@@ -486,20 +492,19 @@ __device__ __forceinline__ void norm_two_pass(const mk_op_desc* op, int r0, int 
     }
 }
 
-// Variant of a norm: x dtype (bits 0-1), fp16 output (bit 2), vectors per lane (bit 3: 8, else 4), gain (bit 4), modulation (bit 5),
-// three or more rows per warp (bit 6)
-constexpr int NORM_DEEP = 64, NORM_ANY = 128;
+// Variant of a norm: x dtype (bits 0-1), fp16 output (bit 2), vectors per lane (bit 3: 8, else 4), gain (bit 4), modulation (bit 5)
+constexpr int NORM_ANY = 128;
 __device__ __forceinline__ int norm_variant(const mk_op_desc* op) {
     const int nper = ((op->i[1] >> 3) + 31) / 32;
     const bool w = op->ptr[2] != 0, mod = op->ptr[4] != 0;
     if (op->ptr[3] || (w && mod) || op->i[5] == DT_F32 || nper > (mod ? 4 : 8)) return NORM_ANY;
-    return (op->i[3] > 2 * kComputeWarps ? NORM_DEEP : 0) | op->i[4] | (op->i[5] == DT_F16 ? 4 : 0) | (nper > 4 ? 8 : 0) | (w ? 16 : 0) | (mod ? 32 : 0);
+    return op->i[4] | (op->i[5] == DT_F16 ? 4 : 0) | (nper > 4 ? 8 : 0) | (w ? 16 : 0) | (mod ? 32 : 0);
 }
 template <int V>
 __device__ __forceinline__ void op_norm_rows(const mk_op_desc* op, int a0) {
     const int r0 = a0 * op->i[3], rows = min(op->i[3], op->i[0] - r0);
     if constexpr (V == NORM_ANY) norm_two_pass(op, r0, rows);
-    else norm_stream<(V & 8) ? 8 : 4, V & 3, (V & 4) ? DT_F16 : DT_BF16, (V & 16) != 0, (V & 32) != 0, (V & NORM_DEEP) != 0>(op, r0, rows);
+    else norm_stream<(V & 8) ? 8 : 4, V & 3, (V & 4) ? DT_F16 : DT_BF16, (V & 16) != 0, (V & 32) != 0>(op, r0, rows);
 }
 
 }  // namespace mk

@@ -261,6 +261,27 @@ def test_norm_many_rows(cuda, rows, cols, dtype, rms, group):
     assert rel_l2(outs[0], ref[0]) < ONE_ROUNDING
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,cols,dtype,group,mod", [
+    (300, 72, F32, 3, F32), (1200, 1000, BF, 8, BF), (1208, 1024, F32, 604, F32), (2400, 264, BF, 1, BF), (261, 2048, F32, 0, BF), (2403, 1032, BF, 0, BF),
+    (9602, 520, F32, 0, BF),
+])
+def test_norm_shares_gain_and_modulation(cuda, rows, cols, dtype, group, mod):
+    """Gain and modulation in shared memory: several groups per instruction, a group per row, both types, warps without a row."""
+    g = mc.Graph()
+    x = g.input("x", (rows, cols), dtype)
+    t = {"x": rnd((rows, cols), 2.0, 1, 0.3).to(dtype)}
+    if group:
+        n = rows // group
+        y = g.modulate(g.layer_norm(x), g.input("sc", (n, cols), mod), g.input("sh", (n, cols), mod), group=group)
+        t["sc"], t["sh"] = rnd((n, cols), 0.3, 3).to(mod), rnd((n, cols), 0.3, 4).to(mod)
+    else:
+        y, t["w"] = g.rms_norm(x, g.param("w", (1, cols))), rnd((1, cols), 0.1, 2, 1.0)
+    g.output(y)
+    outs, ref, *_ = run_both(g, t, cuda)
+    assert rel_l2(outs[0], ref[0]) < ONE_ROUNDING
+
+
 def test_hoisted_linears_keep_their_order():
     """A linear moves behind the op it depends on and in front of unrelated ones only; what reads or overwrites its operands stays put."""
     g = mc.Graph()
