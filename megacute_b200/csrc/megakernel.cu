@@ -430,7 +430,7 @@ static bool tile_gemm_on_tcgen05(const mk_op_desc& d) {
     if (d.ptr[3] && (d.ptr[3] & 15)) return false;
     if (d.ptr[4] && !vec_ok(d.ptr[4], d.ld[4], rdt)) return false;
     if (d.ptr[6] && (odt == 1 || d.i[17] == 1 || !vec_ok(d.ptr[6], d.ld[6], d.i[17]) || !vec_ok(d.ptr[7], d.ld[7], d.i[17]))) return false;
-    if (d.ptr[5] && (!vec_ok(d.ptr[5], d.ld[5], d.i[13]) || d.i[11] != 256 || d.i[12] <= 0)) return false;
+    if (d.ptr[5] && (!d.ptr[4] || !vec_ok(d.ptr[5], d.ld[5], d.i[13]) || (d.i[11] != 256 && d.i[13] == 1) || d.i[12] <= 0)) return false;
     return true;
 }
 

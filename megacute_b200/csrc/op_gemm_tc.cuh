@@ -69,51 +69,21 @@ static_assert(kTcXOff + 128 * kTcStagePitch * 4 <= kWorkBytes, "epilogue staging
 static __device__ __noinline__ void tc_write_rows(const mk_op_desc* op, const float* stage, int m0, int rows, int ncols, int col0,
                                               int n_out) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int act = op->i[3], odt = op->i[5], accum = op->i[6], rdt = op->i[7];
-    const bool plain = !accum && !op->i[8];
+    const int odt = op->i[5], accum = op->i[6];
     uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]);
-    const uint8_t* bias = reinterpret_cast<const uint8_t*>(op->ptr[3]);
-    const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]);
     const int two = ncols == 64 ? 1 : 0;                       // swiglu: 16 lanes per row, two rows per pass
     const int sub = two ? lane >> 4 : 0, c4 = (two ? lane & 15 : lane) * 4, col = col0 + c4;
     if (col >= n_out) return;
-    float b4[4] = {0.f, 0.f, 0.f, 0.f};
-    if (plain && bias) {
-        const uint2 w = __ldg(reinterpret_cast<const uint2*>(bias + (long long)col * 2));
-        b4[0] = bf16_lo(w.x); b4[1] = bf16_hi(w.x); b4[2] = bf16_lo(w.y); b4[3] = bf16_hi(w.y);
-    }
     const int step = kComputeWarps << two;
 #pragma unroll 2
     for (int row = (warp << two) + sub; row < rows; row += step) {
         const float4 q = *reinterpret_cast<const float4*>(stage + row * kTcStagePitch + c4);
-        float f[4] = {q.x, q.y, q.z, q.w};
         const long long eo = (long long)(m0 + row) * op->ld[2] + col;
         if (accum) {
-            if (odt == 1) red_add_f32x4(reinterpret_cast<float*>(O) + eo, f[0], f[1], f[2], f[3]);
-            else red_add_bf16x4(O + eo * 2, f);
-            continue;
-        }
-        if (plain) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) f[j] = apply_act(act, f[j] + b4[j]);
-            if (R) {
-                const long long er = (long long)(m0 + row) * op->ld[4] + col;
-                if (rdt == DT_F32) {
-                    const float4 x = __ldcg(reinterpret_cast<const float4*>(R + er * 4));
-                    f[0] += x.x; f[1] += x.y; f[2] += x.z; f[3] += x.w;
-                } else {
-                    const uint2 w = __ldcg(reinterpret_cast<const uint2*>(R + er * 2));
-                    if (rdt == DT_F16) {
-                        const float2 lo = unpack2h(w.x), hi = unpack2h(w.y);
-                        f[0] += lo.x; f[1] += lo.y; f[2] += hi.x; f[3] += hi.y;
-                    } else {
-                        f[0] += bf16_lo(w.x); f[1] += bf16_hi(w.x); f[2] += bf16_lo(w.y); f[3] += bf16_hi(w.y);
-                    }
-                }
-            }
-        }
-        if (odt == DT_F32) *reinterpret_cast<float4*>(O + eo * 4) = make_float4(f[0], f[1], f[2], f[3]);
-        else *reinterpret_cast<uint2*>(O + eo * 2) = make_uint2(pack2t(odt, f[0], f[1]), pack2t(odt, f[2], f[3]));
+            const float f[4] = {q.x, q.y, q.z, q.w};
+            red_add_bf16x4(O + eo * 2, f);
+        } else if (odt == DT_F32) *reinterpret_cast<float4*>(O + eo * 4) = q;
+        else *reinterpret_cast<uint2*>(O + eo * 2) = make_uint2(pack2t(odt, q.x, q.y), pack2t(odt, q.z, q.w));
     }
 }
 
@@ -133,16 +103,12 @@ static __device__ __noinline__ void tc_reduce_rows(const mk_op_desc* op, const f
     }
 }
 
-// Epilogue, second half, plain tiles (not a split-K partial, not swiglu): out = act(acc + bias) + residual, 128 columns.
-// Specialised at compile time on output type, residual kind and whether there is an activation: with those as
-// run-time switches inside the row loop the writer was instruction-bound (4.2 us per 128 x 128 tile against 1.3 us
-// for the same stores from a specialised loop, measured stand-alone).  A loop over groups of rows whose residual is requested a group
-// ahead: all sixteen rows of a warp requested at once are straight-line code that is fetched cold once per op, 6.0 us for a tile
-// with a residual inside a prompt of 333 tokens; now 3.7.
-template <int ODT, int RKIND, bool ACT>              // RKIND 0: no residual, 1: 16-bit (bf16 / fp16 by rdt), 2: fp32
-static __device__ __noinline__ void tc_store_rows_t(const mk_op_desc* op, const float* stage, int m0, int rows, int col0, int n_out) {
+// Epilogue, second half, plain tiles (not a split-K partial, not swiglu, nothing behind the bias): out = acc + bias, 128 columns.
+// Specialised at compile time on the output type: with type, residual and activation as run-time switches inside the row loop the
+// writer was instruction-bound (4.2 us per 128 x 128 tile against 1.3 us for the same stores, measured stand-alone).
+template <int ODT>
+static __device__ __noinline__ void tc_store_rows(const mk_op_desc* op, const float* stage, int m0, int rows, int col0, int n_out) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int act = op->i[3], rdt = op->i[7];
     const int c4 = lane * 4, col = col0 + c4;
     if (col >= n_out) return;
     float b4[4] = {0.f, 0.f, 0.f, 0.f};
@@ -150,62 +116,135 @@ static __device__ __noinline__ void tc_store_rows_t(const mk_op_desc* op, const 
         const uint2 w = __ldg(reinterpret_cast<const uint2*>(bias + (long long)col * 2));
         b4[0] = bf16_lo(w.x); b4[1] = bf16_hi(w.x); b4[2] = bf16_lo(w.y); b4[3] = bf16_hi(w.y);
     }
-    constexpr int kGroup = RKIND ? 4 : 2;
-    const long long ldo = op->ld[2], ldr = op->ld[4];
+    const long long ldo = op->ld[2];
     uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + ((long long)m0 * ldo + col) * (ODT == DT_F32 ? 4 : 2);
-    const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]) + ((long long)m0 * ldr + col) * (RKIND == 2 ? 4 : 2);
-    uint2 n16[kGroup];
-    float4 n32[kGroup];
-    auto request = [&](int row) {
-#pragma unroll
-        for (int j = 0; j < kGroup; ++j) {
-            if (RKIND == 0 || row + j * kComputeWarps >= rows) break;
-            if (RKIND == 1) n16[j] = __ldcg(reinterpret_cast<const uint2*>(R + (row + j * kComputeWarps) * ldr * 2));
-            if (RKIND == 2) n32[j] = __ldcg(reinterpret_cast<const float4*>(R + (row + j * kComputeWarps) * ldr * 4));
-        }
-    };
-    request(warp);
-#pragma unroll 1
-    for (int row0 = warp; row0 < rows; row0 += kGroup * kComputeWarps) {
-        uint2 r16[kGroup];
-        float4 r32[kGroup];
-#pragma unroll
-        for (int j = 0; j < kGroup; ++j) {
-            if (RKIND == 1) r16[j] = n16[j];
-            if (RKIND == 2) r32[j] = n32[j];
-        }
-        request(row0 + kGroup * kComputeWarps);
-#pragma unroll
-        for (int j = 0; j < kGroup; ++j) {
-            const int row = row0 + j * kComputeWarps;
-            if (row >= rows) break;
-            const float4 q = *reinterpret_cast<const float4*>(stage + row * kTcStagePitch + c4);
-            float f[4] = {q.x + b4[0], q.y + b4[1], q.z + b4[2], q.w + b4[3]};
-            if (ACT) {
-#pragma unroll
-                for (int e = 0; e < 4; ++e) f[e] = apply_act(act, f[e]);
-            }
-            if (RKIND == 1) {
-                if (rdt == DT_F16) {
-                    const float2 lo = unpack2h(r16[j].x), hi = unpack2h(r16[j].y);
-                    f[0] += lo.x; f[1] += lo.y; f[2] += hi.x; f[3] += hi.y;
-                } else {
-                    f[0] += bf16_lo(r16[j].x); f[1] += bf16_hi(r16[j].x); f[2] += bf16_lo(r16[j].y); f[3] += bf16_hi(r16[j].y);
-                }
-            }
-            if (RKIND == 2) { f[0] += r32[j].x; f[1] += r32[j].y; f[2] += r32[j].z; f[3] += r32[j].w; }
-            if (ODT == DT_F32) *reinterpret_cast<float4*>(O + row * ldo * 4) = make_float4(f[0], f[1], f[2], f[3]);
-            else if (ODT == DT_F16) *reinterpret_cast<uint2*>(O + row * ldo * 2) = make_uint2(pack2h(f[0], f[1]), pack2h(f[2], f[3]));
-            else *reinterpret_cast<uint2*>(O + row * ldo * 2) = make_uint2(pack2(f[0], f[1]), pack2(f[2], f[3]));
-        }
+#pragma unroll 2
+    for (int row = warp; row < rows; row += kComputeWarps) {
+        const float4 q = *reinterpret_cast<const float4*>(stage + row * kTcStagePitch + c4);
+        const float f[4] = {q.x + b4[0], q.y + b4[1], q.z + b4[2], q.w + b4[3]};
+        if (ODT == DT_F32) *reinterpret_cast<float4*>(O + row * ldo * 4) = make_float4(f[0], f[1], f[2], f[3]);
+        else if (ODT == DT_F16) *reinterpret_cast<uint2*>(O + row * ldo * 2) = make_uint2(pack2h(f[0], f[1]), pack2h(f[2], f[3]));
+        else *reinterpret_cast<uint2*>(O + row * ldo * 2) = make_uint2(pack2(f[0], f[1]), pack2(f[2], f[3]));
     }
 }
-// Epilogue straight from tensor memory to 16-bit outputs, a row per thread and 32 bytes at a time, for tiles that read another operand
-// beside the accumulator: what the first columns need is requested before the accumulator is complete.
+// Epilogues straight from tensor memory, a row per thread and 16 columns at a time, for tiles that read another operand beside the
+// accumulator or compute something from it: what the first columns need is requested before the accumulator is complete, what
+// the next ones need while these are at work.  (A loop over few instructions: sixteen rows of a warp side by side, through the
+// staging rows, are straight-line code that is fetched cold once per op.  Time from the complete accumulator, inside a prompt of 333 tokens:
+// rotated heads 7.8 us, as a loop over groups of four rows 6.4, this 3.9.)
+__device__ __forceinline__ bool tc_direct_wait(const Params& p, Ctrl* c, uint32_t apar, int seq) {
+    int ok = 1;
+    if ((threadIdx.x & 31) == 0) ok = wait_barrier(p, c, &c->acc_full, apar, seq, WHERE_COMBINE) ? 1 : 0;
+    ok = __shfl_sync(0xffffffffu, ok, 0);
+    tc_fence_after();
+    phase_mark(p, c, 2);                                     // accumulator complete
+    __syncwarp();                                            // (the tensor-memory loads are .sync.aligned: whole warp, converged)
+    return ok != 0;
+}
+// an activation chosen at run time on 16 values, four at a time (rotated: register indices stay constant)
+__device__ __forceinline__ void act16(int act, float* v) {
+#pragma unroll 1
+    for (int j = 0; j < 16; j += 4) {
+        float t[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) t[e] = apply_act(act, v[e]);
+#pragma unroll
+        for (int e = 0; e < 12; ++e) v[e] = v[e + 4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) v[12 + e] = t[e];
+    }
+}
+// 64 elements of a row, as many eights of them as there are, taken 16 at a time from the front
+template <int DT> struct Row64 {
+    static constexpr int kPer8 = DT == DT_F32 ? 2 : 1;
+    uint4 w[8 * kPer8];
+    __device__ __forceinline__ void load(const uint8_t* at, int cols, bool whole) {
+#pragma unroll
+        for (int k = 0; k < 8 * kPer8; k += 2) {
+            if (kPer8 == 1 && k * 8 + 8 >= cols) {
+                if (k * 8 < cols) w[k] = __ldcg(reinterpret_cast<const uint4*>(at) + k);
+            } else if (k / kPer8 * 8 < cols) {
+                ld32B(at + k * 16, reinterpret_cast<uint32_t*>(w + k), whole);
+            }
+        }
+    }
+    // element e of the front 16 (DT_BF16: either 16-bit type, by `f16`)
+    __device__ __forceinline__ float get(int e, bool f16) const {
+        const uint32_t* q = reinterpret_cast<const uint32_t*>(w);
+        if (DT == DT_F32) return __uint_as_float(q[e]);
+        const uint32_t x = q[e >> 1];
+        if (f16) { const float2 h = unpack2h(x); return e & 1 ? h.y : h.x; }
+        return e & 1 ? bf16_hi(x) : bf16_lo(x);
+    }
+    __device__ __forceinline__ void next() {
+#pragma unroll
+        for (int k = 0; k < 6 * kPer8; ++k) w[k] = w[k + 2 * kPer8];
+    }
+};
+// out = act(acc + bias) [* gate row of i 12 rows] [+ residual].  RKIND 0: no residual, 1: 16-bit, 2: fp32.  ACT 0: none, 1: gelu, 2: any.
+// GATE: with ACT 2 decided at run time.
+template <int ODT, int RKIND, int ACT, bool GATE>
+static __device__ __noinline__ bool tc_cols_direct(const Params& p, Ctrl* c, const mk_op_desc* op, uint32_t two, uint32_t apar, int m0, int n0, int seq) {
+    constexpr int osz = ODT == DT_F32 ? 4 : 2, rsz = RKIND == 2 ? 4 : 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, qd = warp & 3, col0 = n0 + 64 * (warp >> 2);
+    const int M = op->i[0], cols = min(64, op->i[1] - col0);                     // this warp's columns
+    const int row = m0 + qd * 32 + lane, safe = min(row, M - 1);
+    const bool gated = GATE && op->ptr[5] != 0, r16 = op->i[7] == DT_F16, g16 = op->i[13] == DT_F16;
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]) + ((long long)safe * op->ld[2] + col0) * osz;
+    const uint8_t* R = RKIND ? reinterpret_cast<const uint8_t*>(op->ptr[4]) + ((long long)safe * op->ld[4] + col0) * rsz : nullptr;
+    const uint8_t* G = gated ? reinterpret_cast<const uint8_t*>(op->ptr[5]) + ((long long)(safe / op->i[12]) * op->ld[5] + col0) * 2 : nullptr;
+    const uint8_t* B = reinterpret_cast<const uint8_t*>(op->ptr[3]);
+    const bool whole = ((op->ptr[2] | (uint64_t)op->ld[2] * osz) & 31) == 0;
+    // (all of the row's piece: a step ahead, each step waits for a round trip to L2 -- 8.6 us for a tile with a residual)
+    Row64<RKIND == 2 ? DT_F32 : DT_BF16> r;
+    Row64<DT_BF16> g;
+    if (RKIND) r.load(R, cols, ((op->ptr[4] | (uint64_t)op->ld[4] * rsz) & 31) == 0);
+    if (gated) g.load(G, cols, ((op->ptr[5] | (uint64_t)op->ld[5] * 2) & 31) == 0);
+    const bool ok = tc_direct_wait(p, c, apar, seq);
+    if (!ok || m0 + qd * 32 >= M) return ok;
+    const uint32_t tl = *(volatile uint32_t*)&c->tmem_base + ((uint32_t)(qd * 32) << 16) + 64 * (warp >> 2);
+#pragma unroll 1
+    for (int k = 0; k < cols; k += 16) {
+        const bool more = k + 8 < cols;
+        float v[16];
+        tc_ld16_sum(tl + k, two, v);
+        if (B) {                                             // (the same 16 for all lanes: one line per tile and warp)
+            const uint4* at = reinterpret_cast<const uint4*>(B + (col0 + k) * 2);
+            const uint4 b[2] = {__ldg(at), more ? __ldg(at + 1) : make_uint4(0u, 0u, 0u, 0u)};
+            const uint32_t* q = reinterpret_cast<const uint32_t*>(b);
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v[e] += e & 1 ? bf16_hi(q[e >> 1]) : bf16_lo(q[e >> 1]);
+        }
+        if (ACT == 1) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v[e] = apply_act(ACT_GELU, v[e]);
+        }
+        if (ACT == 2) act16(op->i[3], v);
+        if (gated) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v[e] = fmaf(v[e], g.get(e, g16), RKIND ? r.get(e, r16) : 0.f);
+        } else if (RKIND) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v[e] += r.get(e, r16);
+        }
+        if (row < M) {
+            uint8_t* at = O + k * osz;
+            if (ODT == DT_F32) {
+                st32B(at, reinterpret_cast<const uint32_t*>(v), whole);
+                if (more) st32B(at + 32, reinterpret_cast<const uint32_t*>(v) + 8, whole);
+            } else if (more) {
+                put16<ODT>(at, v, whole);
+            } else {
+                *reinterpret_cast<uint4*>(at) = make_uint4(pack2t(ODT, v[0], v[1]), pack2t(ODT, v[2], v[3]), pack2t(ODT, v[4], v[5]), pack2t(ODT, v[6], v[7]));
+            }
+        }
+        if (RKIND) r.next();
+        if (GATE) g.next();
+        __syncwarp();
+    }
+    return true;
+}
 //   rotated heads (descriptor: op_gemm.cuh): 16 columns of both halves of a head at a time, with the row's piece of the tables
-// Through the staging rows a tile's second half took 6.6 us, as straight-line code for 16 rows per warp that is fetched cold once per op;
-// as a loop over four rows at a time 5.3, a round trip to L2 for each turn's table rows.  This form takes 3.9 from the complete accumulator,
-// first half included (7.8): a prompt of 333 tokens 1789 -> 1752 us.
 template <int ODT>
 static __device__ __noinline__ bool tc_rope_direct(const Params& p, Ctrl* c, const mk_op_desc* op, uint32_t two, uint32_t apar, int m0, int n0,
                                                    int seq) {
@@ -228,13 +267,8 @@ static __device__ __noinline__ bool tc_rope_direct(const Params& p, Ctrl* c, con
         }
     };
     request(0);
-    int ok = 1;
-    if (lane == 0) ok = wait_barrier(p, c, &c->acc_full, apar, seq, WHERE_COMBINE) ? 1 : 0;
-    ok = __shfl_sync(0xffffffffu, ok, 0);
-    tc_fence_after();
-    phase_mark(p, c, 2);
-    __syncwarp();
-    if (!ok || m0 + qd * 32 >= M || n0 + col0 >= op->i[1]) return ok != 0;
+    const bool ok = tc_direct_wait(p, c, apar, seq);
+    if (!ok || m0 + qd * 32 >= M || n0 + col0 >= op->i[1]) return ok;
     const uint32_t tl = *(volatile uint32_t*)&c->tmem_base + ((uint32_t)(qd * 32) << 16) + col0;
     auto get = [&](uint32_t w) { return t16 ? unpack2h(w) : make_float2(bf16_lo(w), bf16_hi(w)); };
 #pragma unroll 1
@@ -263,22 +297,24 @@ static __device__ __noinline__ bool tc_rope_direct(const Params& p, Ctrl* c, con
     }
     return true;
 }
+// the direct epilogue of a tile with a residual, an activation or rotated heads
 template <int ODT>
-__device__ __forceinline__ void tc_store_rows_o(const mk_op_desc* op, const float* stage, int m0, int rows, int col0, int n_out) {
-    const int rk = !op->ptr[4] ? 0 : op->i[7] == DT_F32 ? 2 : 1;
-    if (op->i[3] != ACT_NONE) {                       // activations are rare in front of a residual: one instance takes every residual kind
-        if (rk == 0) tc_store_rows_t<ODT, 0, true>(op, stage, m0, rows, col0, n_out);
-        else if (rk == 1) tc_store_rows_t<ODT, 1, true>(op, stage, m0, rows, col0, n_out);
-        else tc_store_rows_t<ODT, 2, true>(op, stage, m0, rows, col0, n_out);
-    } else if (rk == 0) tc_store_rows_t<ODT, 0, false>(op, stage, m0, rows, col0, n_out);
-    else if (rk == 1) tc_store_rows_t<ODT, 1, false>(op, stage, m0, rows, col0, n_out);
-    else tc_store_rows_t<ODT, 2, false>(op, stage, m0, rows, col0, n_out);
+__device__ __forceinline__ bool tc_direct_o(const Params& p, Ctrl* c, const mk_op_desc* op, uint32_t two, uint32_t apar, int m0, int n0, int seq) {
+    if (ODT != DT_F32 && op->ptr[6]) return tc_rope_direct<ODT>(p, c, op, two, apar, m0, n0, seq);
+    const int act = op->i[3];
+    if (!op->ptr[4]) return act == ACT_GELU ? tc_cols_direct<ODT, 0, 1, false>(p, c, op, two, apar, m0, n0, seq) : tc_cols_direct<ODT, 0, 2, false>(p, c, op, two, apar, m0, n0, seq);
+    if (op->i[7] == DT_F32) {
+        if (act != ACT_NONE) return tc_cols_direct<ODT, 2, 2, true>(p, c, op, two, apar, m0, n0, seq);
+        return op->ptr[5] ? tc_cols_direct<ODT, 2, 0, true>(p, c, op, two, apar, m0, n0, seq) : tc_cols_direct<ODT, 2, 0, false>(p, c, op, two, apar, m0, n0, seq);
+    }
+    if (act != ACT_NONE) return tc_cols_direct<ODT, 1, 2, true>(p, c, op, two, apar, m0, n0, seq);
+    return op->ptr[5] ? tc_cols_direct<ODT, 1, 0, true>(p, c, op, two, apar, m0, n0, seq) : tc_cols_direct<ODT, 1, 0, false>(p, c, op, two, apar, m0, n0, seq);
 }
-__device__ __forceinline__ void tc_store_rows(const mk_op_desc* op, const float* stage, int m0, int rows, int col0, int n_out) {
+static __device__ __noinline__ bool tc_direct(const Params& p, Ctrl* c, const mk_op_desc* op, uint32_t two, uint32_t apar, int m0, int n0, int seq) {
     const int odt = op->i[5];
-    if (odt == DT_F32) tc_store_rows_o<DT_F32>(op, stage, m0, rows, col0, n_out);
-    else if (odt == DT_F16) tc_store_rows_o<DT_F16>(op, stage, m0, rows, col0, n_out);
-    else tc_store_rows_o<DT_BF16>(op, stage, m0, rows, col0, n_out);
+    if (odt == DT_F32) return tc_direct_o<DT_F32>(p, c, op, two, apar, m0, n0, seq);
+    if (odt == DT_F16) return tc_direct_o<DT_F16>(p, c, op, two, apar, m0, n0, seq);
+    return tc_direct_o<DT_BF16>(p, c, op, two, apar, m0, n0, seq);
 }
 
 // Abort path: the activation tiles of an instruction that did not end have landed.  Stage s of lane s mod 2 was armed in this round if it
@@ -401,8 +437,8 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
     // ---- epilogue: warp w owns lanes 32 (w & 3) .. +31 (activation rows) and column half w >> 2 ----
     const uint32_t two = nk > 1 ? 128u : 0u;                               // columns to the second issuing thread's accumulator, if it has a part
     int ok = 1;
-    if (op->ptr[6] && !op->i[6] && !swi) {
-        ok = op->i[5] == DT_F16 ? tc_rope_direct<DT_F16>(p, c, op, two, apar, m0, n0, seq) : tc_rope_direct<DT_BF16>(p, c, op, two, apar, m0, n0, seq);
+    if (!op->i[6] && !swi && (op->ptr[6] || op->ptr[4] || op->i[3] != ACT_NONE)) {
+        ok = tc_direct(p, c, op, two, apar, m0, n0, seq);
     } else {
         if (lane == 0) ok = wait_barrier(p, c, &c->acc_full, apar, seq, WHERE_COMBINE) ? 1 : 0;
         ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -453,7 +489,9 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
                 if (op->i[5] == DT_F32) tc_reduce_rows(op, stage, m0, rows, n0, N);
                 else tc_write_rows(op, stage, m0, rows, 128, n0, N);
             }
-            else tc_store_rows(op, stage, m0, rows, n0, N);
+            else if (op->i[5] == DT_F32) tc_store_rows<DT_F32>(op, stage, m0, rows, n0, N);
+            else if (op->i[5] == DT_F16) tc_store_rows<DT_F16>(op, stage, m0, rows, n0, N);
+            else tc_store_rows<DT_BF16>(op, stage, m0, rows, n0, N);
         }
     }
     tc_fence_before();

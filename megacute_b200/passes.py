@@ -309,7 +309,7 @@ def _accepts(op: Op, field: str, dtype) -> bool:
         streaming = gemv_eligible(op.x.rows, op.x.cols)
         if field == "x":                                # the tensor core takes 16-bit operands; the streaming linear converts
             return streaming or not f32
-        return field in ("out", "residual", "gate")
+        return field in ("out", "residual") or (field == "gate" and (op.bm == C.GEMM_BM_WIDE or not f32))
     if k == "LinearSplit":
         return (field == "ws" and f32) or (field == "x" and not f32)
     if k == "SplitFinalize":
@@ -500,9 +500,9 @@ def fuse_pointwise(g: Graph) -> Graph:
 
 
 def fuse_gated_linear(g: Graph) -> Graph:
-    """A tile linear with 256-row tiles followed by a gated residual (``x + y * gate[g]``, made by fuse_pointwise) does the
-    gating in its epilogue: a pass over three activation-sized tensors and a dependency hop less, and the product is not
-    rounded in between.  (Few-row linears keep the op: their epilogues have no room for a third operand's latency.)
+    """A tile linear followed by a gated residual (``x + y * gate[g]``, made by fuse_pointwise) does the gating in its epilogue: a
+    pass over three activation-sized tensors and a dependency hop less (7 us per hop in a DiT block of 1024 rows), and the
+    product is not rounded in between.  (128-row tiles take a 16-bit gate only; streaming linears keep the op.)
     MEGACUTE_B200_NO_POINTWISE_FUSION=1 keeps the ops apart."""
     if os.environ.get("MEGACUTE_B200_NO_POINTWISE_FUSION") == "1":
         return g
@@ -511,7 +511,8 @@ def fuse_gated_linear(g: Graph) -> Graph:
     for i, op in enumerate(g.ops):
         prev = ops[-1] if ops else None
         if (op.kind == "Binary" and op.gate is not None and op.fn == "add" and prev is not None and prev.kind == "Linear"
-                and prev.bm == C.GEMM_BM_WIDE and prev.act != "swiglu" and prev.residual is None and prev.gate is None
+                and (prev.bm == C.GEMM_BM_WIDE or (not gemv_eligible(prev.x.rows, prev.x.cols) and op.gate.buf.dtype != torch.float32))
+                and prev.act != "swiglu" and prev.residual is None and prev.gate is None
                 and op.b.same(prev.out) and prev.out.buf.kind == "temp" and not _reads_buffer(g.ops[i + 1:], prev.out.buf, g.outputs)
                 # (the product is not stored any more: neither the residual nor the gate may be it)
                 and op.a.buf is not prev.out.buf and op.gate.buf is not prev.out.buf

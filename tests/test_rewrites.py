@@ -46,6 +46,27 @@ def test_gated_residual_of_the_product_itself(monkeypatch, form):
     assert check_rewritten(g, t) == ["Linear", "Binary"]
 
 
+@pytest.mark.parametrize("M,N", [(8, 64), (9, 64), (64, 136), (128, 64), (129, 256), (384, 128)])
+@pytest.mark.parametrize("group", [1, 3, 32])
+@pytest.mark.parametrize("gate_dtype", [BF, torch.float32, torch.float16])
+@pytest.mark.parametrize("act", [None, "gelu_tanh", "swiglu"])
+def test_gated_residual_in_the_linear(monkeypatch, M, N, group, gate_dtype, act):
+    """Which linears take a gated residual: tile linears (more than eight rows), 128-row tiles with a 16-bit gate, no swiglu."""
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 128) if a[1] % 128 == 0 else (1, 128, 128))
+    monkeypatch.setattr(passes, "choose_k_splits", lambda *a: 1)
+    M = -(-M // group) * group
+    g = mc.Graph()
+    n = N // 2 if act == "swiglu" else N
+    t = {"x": rnd((M, 64)), "w": rnd((N, 64), 0.1, 1), "r": rnd((M, n), 1.0, 2), "gate": rnd((M // group, n), 1.0, 3).to(gate_dtype)}
+    if act == "swiglu" and N % 128:
+        return
+    y = g.linear(g.input("x", (M, 64)), g.param("w", (N, 64)), act=act)
+    g.output(g.add(g.input("r", (M, n)), g.binary(y, g.input("gate", (M // group, n), gate_dtype), "mul", b_group=group)))
+    wide = M > 128 and N % 128 == 0
+    fused = act != "swiglu" and M > 8 and (wide or gate_dtype != torch.float32)
+    assert check_rewritten(g, t) == (["Linear"] if fused else ["Linear", "Binary"])
+
+
 def rotated(g, S, H=2, KVH=1, D=64, tables=lambda c, s: (c, s), qkv_dtype=None):
     """x -> q, k, v of one prompt -> rotated q and k -> attention.  `tables`: ops between the linear and the rotation."""
     x, w = g.input("x", (S, 64)), g.param("w", ((H + 2 * KVH) * D, 64))

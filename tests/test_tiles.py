@@ -28,6 +28,10 @@ ONE_ROUNDING = 1.05 * 2.0 ** -9
     (513, 256, 64, (1, 256, 256), {"res": BF, "act": "silu"}),                  # (activation in front of a residual)
     (320, 512, 256, (1, 256, 256), {"gate": 64}),                               # gated residual, 64 rows per gate row
     (320, 128, 256, (1, 256, 128), {"gate": 40}),                               # (a warp's rows span two gate rows)
+    (320, 256, 256, (1, 128, 128), {"gate": 64}),                               # ... in 128-row tiles
+    (192, 136, 192, (1, 128, 128), {"gate": 3, "bias": True}),                  # (a gate row per three rows, a last step of eight columns)
+    (400, 264, 64, (1, 128, 128), {"gate": 40, "gres": F32}),
+    (96, 1000, 128, (1, 128, 128), {"gate": 32, "act": "silu"}),
     (600, 256, 320, (3, 256, 128), {"bias": True}),                             # 5 k-tiles in 3 splits
     (200, 256, 448, (4, 128, 128), {"act": "relu"}),                            # 7 in 4, 128 x 128 tiles
     (135, 264, 448, (3, 128, 128), {"bias": True, "res": F32}),                 # (ragged in both directions, finished with a residual)
@@ -46,8 +50,8 @@ def test_tile_epilogues(cuda, monkeypatch, M, N, K, plan, kw):
         res, t["r"] = g.input("r", (M, n_out), kw["res"]), rnd((M, n_out), 1.0, 4).to(kw["res"])
     y = g.linear(x, w, bias=bias, act=kw.get("act"), residual=res)
     if kw.get("gate"):
-        r, gate = g.input("r", (M, N)), g.input("gate", (M // kw["gate"], N))
-        t["r"], t["gate"] = rnd((M, N), 1.0, 4), rnd((M // kw["gate"], N), 1.0, 5)
+        r, gate = g.input("r", (M, N), kw.get("gres", BF)), g.input("gate", (M // kw["gate"], N))
+        t["r"], t["gate"] = rnd((M, N), 1.0, 4).to(kw.get("gres", BF)), rnd((M // kw["gate"], N), 1.0, 5)
         y = g.add(r, g.binary(y, gate, "mul", b_group=kw["gate"]))
     g.output(y)
     outs, ref, _, _, prog = run_both(g, t, cuda, steps=2)                       # twice: split-K workspaces are zeroed again
