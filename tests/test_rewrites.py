@@ -47,8 +47,8 @@ def test_gated_residual_of_the_product_itself(monkeypatch, form):
 
 
 @pytest.mark.parametrize("M,N", [(8, 64), (9, 64), (64, 136), (128, 64), (129, 256), (384, 128)])
-@pytest.mark.parametrize("group", [1, 3, 32])
-@pytest.mark.parametrize("gate_dtype", [BF, torch.float32, torch.float16])
+@pytest.mark.parametrize("group", [2, 3, 32])
+@pytest.mark.parametrize("gate_dtype", [BF, torch.float32])
 @pytest.mark.parametrize("act", [None, "gelu_tanh", "swiglu"])
 def test_gated_residual_in_the_linear(monkeypatch, M, N, group, gate_dtype, act):
     """Which linears take a gated residual: tile linears (more than eight rows), 128-row tiles with a 16-bit gate, no swiglu."""
