@@ -26,7 +26,7 @@ extern "C" {
 enum {
     MK_OP_GEMV = 1,        /* linear with <= 8 activation rows: weight rows streamed through smem */
     MK_OP_GEMM = 2,        /* tiled linear, optional split-K partial (reduce-add)                   */
-    MK_OP_FINALIZE = 3,    /* out = act(ws + bias) + residual; ws = 0                               */
+    MK_OP_FINALIZE = 3,    /* out = act(ws + bias) [* gate[r / group]] + residual; ws = 0           */
     MK_OP_ELTWISE = 4,     /* unary / binary / swiglu / modulate / rope tiles                       */
     MK_OP_NORM = 5,        /* RMSNorm / LayerNorm rows                                              */
     MK_OP_ATTENTION = 6,   /* prefill flash attention tile                                          */

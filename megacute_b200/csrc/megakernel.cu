@@ -502,6 +502,7 @@ static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
                     break;
                 case MK_OP_FINALIZE:
                     if (d.i[5] <= 0 || a0 < 0 || a0 >= ceil_div(d.i[0], d.i[5]) || a1 < 0 || a1 * 512 >= d.i[1]) why = "finalize: tile outside the output";
+                    else if (d.ptr[4] && (d.i[6] <= 0 || !is_float(d.i[7]))) why = "finalize: rows per gate row or gate dtype";
                     break;
                 case MK_OP_ELTWISE:
                     if (d.i[10] <= 0 || a0 < 0 || a0 * d.i[10] >= d.i[0] || a1 < 0 || a1 * 512 >= d.i[1]) why = "pointwise: tile outside the output";

@@ -123,8 +123,9 @@ def fill(d, op: Op, addr, sm_count: int, direct=frozenset()) -> None:
         ints += gemm_k_split(op.x.cols, op.splits if split else 1)[:2]
     elif k == "SplitFinalize":
         d.kind = C.OP_FINALIZE
-        ptrs = [op.ws, op.out, op.bias, op.residual]
-        ints = [op.out.rows, op.out.cols, C.ACT_CODE[op.act], dt(op.out), dt(op.residual), finalize_rows(op.out.rows, op.out.cols)]
+        ptrs = [op.ws, op.out, op.bias, op.residual, op.gate]
+        ints = [op.out.rows, op.out.cols, C.ACT_CODE[op.act], dt(op.out), dt(op.residual), finalize_rows(op.out.rows, op.out.cols),
+                int(op.gate_group) if op.gate is not None else 1, dt(op.gate)]
     elif k in ("Unary", "Binary", "SwiGLU", "Modulate", "Rope"):
         d.kind = C.OP_ELTWISE
         R, Cc = op.out.shape

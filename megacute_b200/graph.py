@@ -111,7 +111,7 @@ OP_TABLE = {
     "Linear":          (("x", "w", "bias", "residual", "norm_w", "gate", "cos", "sin"), ("out",),
                         ("act", "rms_eps", "bm", "bn", "gate_group", "rope_cols", "head_dim", "seq")),
     "LinearSplit":     (("x", "w", "norm_w"), ("ws",), ("splits", "rms_eps", "bm", "bn")),
-    "SplitFinalize":   (("ws", "bias", "residual"), ("out", "ws"), ("act",)),
+    "SplitFinalize":   (("ws", "bias", "residual", "gate"), ("out", "ws"), ("act", "gate_group")),
     "Unary":           (("x",), ("out",), ("fn",)),
     "Binary":          (("a", "b", "gate"), ("out",), ("fn", "b_group", "gate_group")),
     "SwiGLU":          (("gate", "up"), ("out",), ("act",)),
@@ -222,6 +222,8 @@ def _chk_finalize(o):
         assert o.bias.shape == (1, o.out.cols)
     if o.residual is not None:
         assert o.residual.shape == o.out.shape
+    if o.gate is not None:          # set by passes.fuse_gated_linear only: out = residual + act(.) * gate[r // gate_group]
+        assert o.residual is not None and o.gate.shape == (-(-o.out.rows // o.gate_group), o.out.cols)
 
 
 def _chk_unary(o):

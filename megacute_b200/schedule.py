@@ -181,6 +181,9 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
         t = lambda v, kind=READ: _acc(v, kind, r0, r1, c0, c1, n=n)
         if k == "SplitFinalize":
             acc = [t(op.ws), _acc(op.bias, READ, 0, 1, c0, c1, n=n), t(op.residual), t(op.out, WRITE), t(op.ws, WRITE)]
+            if op.gate is not None:
+                gg = op.gate_group
+                acc.append(_acc(op.gate, READ, r0 // gg, -(-np.minimum(r1, R) // gg), c0, c1, n=n, covers=False))
         elif k == "Unary":
             acc = [t(op.x), t(op.out, WRITE)]
         elif k == "Binary":

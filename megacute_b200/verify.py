@@ -70,7 +70,10 @@ def operand_windows(op) -> dict:
         return win
     if k == "SplitFinalize":
         R, Cc = op.out.shape
-        return {"ws": (R, Cc), "out": (R, Cc), "bias": (1, Cc), "residual": (R, Cc)}
+        win = {"ws": (R, Cc), "out": (R, Cc), "bias": (1, Cc), "residual": (R, Cc)}
+        if op.gate is not None:
+            win["gate"] = (_ceil(R, op.gate_group), Cc)
+        return win
     if k == "Unary":
         return {"x": op.out.shape, "out": op.out.shape}
     if k == "Binary":

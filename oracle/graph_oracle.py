@@ -179,6 +179,8 @@ class Evaluator:
         if o.bias is not None:
             y = y + self.rd(o.bias)
         y = act_fn(o.act, y)
+        if getattr(o, "gate", None) is not None:        # (this repository's fused form: a gated residual)
+            y = y * self.rd(o.gate).repeat_interleave(o.gate_group, 0)
         if o.residual is not None:
             y = y + self.rd(o.residual)
         self.wr(o.out, y)

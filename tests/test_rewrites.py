@@ -50,10 +50,12 @@ def test_gated_residual_of_the_product_itself(monkeypatch, form):
 @pytest.mark.parametrize("group", [2, 3, 32])
 @pytest.mark.parametrize("gate_dtype", [BF, torch.float32])
 @pytest.mark.parametrize("act", [None, "gelu_tanh", "swiglu"])
-def test_gated_residual_in_the_linear(monkeypatch, M, N, group, gate_dtype, act):
-    """Which linears take a gated residual: tile linears (more than eight rows), 128-row tiles with a 16-bit gate, no swiglu."""
-    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 128) if a[1] % 128 == 0 else (1, 128, 128))
-    monkeypatch.setattr(passes, "choose_k_splits", lambda *a: 1)
+@pytest.mark.parametrize("splits", [1, 2])
+def test_gated_residual_in_the_linear(monkeypatch, M, N, group, gate_dtype, act, splits):
+    """Which linears take a gated residual: tile linears (more than eight rows), 128-row tiles with a 16-bit gate, no swiglu; and the
+    SplitFinalize behind K splits, with any gate."""
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (min(splits, a[4]), 256, 128) if a[1] % 128 == 0 else (min(splits, a[4]), 128, 128))
+    monkeypatch.setattr(passes, "choose_k_splits", lambda *a: splits)
     M = -(-M // group) * group
     g = mc.Graph()
     n = N // 2 if act == "swiglu" else N
@@ -64,7 +66,10 @@ def test_gated_residual_in_the_linear(monkeypatch, M, N, group, gate_dtype, act)
     g.output(g.add(g.input("r", (M, n)), g.binary(y, g.input("gate", (M // group, n), gate_dtype), "mul", b_group=group)))
     wide = M > 128 and N % 128 == 0
     fused = act != "swiglu" and M > 8 and (wide or gate_dtype != torch.float32)
-    assert check_rewritten(g, t) == (["Linear"] if fused else ["Linear", "Binary"])
+    if splits == 2 and act != "swiglu" and M > 8:
+        assert check_rewritten(g, t) == ["LinearSplit", "SplitFinalize"]
+    else:
+        assert check_rewritten(g, t) == (["Linear"] if fused else ["Linear", "Binary"])
 
 
 def rotated(g, S, H=2, KVH=1, D=64, tables=lambda c, s: (c, s), qkv_dtype=None):

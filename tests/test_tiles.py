@@ -34,6 +34,9 @@ ONE_ROUNDING = 1.05 * 2.0 ** -9
     (96, 1000, 128, (1, 128, 128), {"gate": 32, "act": "silu"}),
     (600, 256, 320, (3, 256, 128), {"bias": True}),                             # 5 k-tiles in 3 splits
     (200, 256, 448, (4, 128, 128), {"act": "relu"}),                            # 7 in 4, 128 x 128 tiles
+    (320, 1000, 448, (4, 128, 128), {"gate": 64}),                              # ... finished with a gated residual
+    (300, 136, 448, (3, 128, 128), {"gate": 3, "bias": True, "act": "silu", "gres": F32, "gdt": F32}),
+    (200, 520, 448, (2, 128, 128), {"bias": True, "act": "gelu_tanh", "res": BF}),
     (135, 264, 448, (3, 128, 128), {"bias": True, "res": F32}),                 # (ragged in both directions, finished with a residual)
     (150, 136, 96, (1, 128, 128), {}),                                          # K of whole 32s: the mma.sync body
 ])
@@ -50,13 +53,15 @@ def test_tile_epilogues(cuda, monkeypatch, M, N, K, plan, kw):
         res, t["r"] = g.input("r", (M, n_out), kw["res"]), rnd((M, n_out), 1.0, 4).to(kw["res"])
     y = g.linear(x, w, bias=bias, act=kw.get("act"), residual=res)
     if kw.get("gate"):
-        r, gate = g.input("r", (M, N), kw.get("gres", BF)), g.input("gate", (M // kw["gate"], N))
-        t["r"], t["gate"] = rnd((M, N), 1.0, 4).to(kw.get("gres", BF)), rnd((M // kw["gate"], N), 1.0, 5)
+        r, gate = g.input("r", (M, N), kw.get("gres", BF)), g.input("gate", (M // kw["gate"], N), kw.get("gdt", BF))
+        t["r"], t["gate"] = rnd((M, N), 1.0, 4).to(kw.get("gres", BF)), rnd((M // kw["gate"], N), 1.0, 5).to(kw.get("gdt", BF))
         y = g.add(r, g.binary(y, gate, "mul", b_group=kw["gate"]))
     g.output(y)
     outs, ref, _, _, prog = run_both(g, t, cuda, steps=2)                       # twice: split-K workspaces are zeroed again
     for a, b in zip(outs, ref):
         assert rel_l2(a, b) < ONE_ROUNDING
+    if kw.get("gate"):
+        assert not any(o.kind == "Binary" for o in prog.g.ops)
     if plan[0] == 1:
         lin = [o for o in prog.g.ops if o.kind == "Linear"][0]
         assert (lin.bm or 128, lin.bn or 128) == plan[1:] and prog.tcgen05_ops == (1 if K % 64 == 0 else 0)
