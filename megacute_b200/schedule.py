@@ -305,11 +305,13 @@ def finalize_rows(rows: int, cols: int) -> int:
 
 
 def norm_rows(rows: int, modulated: bool, sm_count: int) -> int:
-    """Rows per norm instruction: a single row spread over the whole CTA when the op has few rows (decode),
+    """Rows per norm instruction: a single row spread over the whole CTA when every row has an SM (decode; 64 rows 3 us, as eight
+    instructions 4, but 256 rows in two rounds 7.5) and is not modulated (that body needs three round trips more: DiT of 1 x 64 tokens
+    1956 us, with eight rows per instruction 1911; of 1 x 256 2420 -> 2136),
     else a multiple of the compute warps that gives each SM about one instruction.  Modulated rows (a DiT block's): 16, 32 or 64, so
     that an instruction waits for one 256-row tile of the linear before it and its rows share a scale and shift row
     (56 -> 64 rows at 32 images, 24 -> 32 at 12: 0.4 and 1.6 % of the step)."""
-    if rows <= C.WIDE_NORM_ROWS:
+    if rows <= sm_count and not modulated:
         return 1
     per = max(1, min(C.NORM_MAX_ROWS // C.NORM_ROWS, _ceil(_ceil(rows, C.NORM_ROWS), sm_count)))
     if modulated and per > 2:
