@@ -284,14 +284,30 @@ __device__ __forceinline__ void wide_store16(const Params& p, Ctrl* c, const mk_
             if (g == groups - 1) wide_release(p, c, a);
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = v[j] * sigmoidf_(v[j]) * u[j];
+        } else if (ACT == 1) {                               // (16 columns at a time: 32 gelus side by side are code that is fetched cold)
+#pragma unroll 1
+            for (int k = 0; k < 32; k += 16) {
+                tc_ld16(a.tacc + g * 32 + k, v);
+                if (g == groups - 1 && k) wide_release(p, c, a);
+                if (a.bias) {
+#pragma unroll
+                    for (int j = 0; j < 16; j += 8) {
+                        float b[8];
+                        unpack8(*reinterpret_cast<const uint4*>(a.bias + (g * 32 + k + j) * 2), b);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) v[j + e] += b[e];
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = apply_act(ACT_GELU, v[j]);
+                if (live) put16<F16 ? DT_F16 : DT_BF16>(O + g * 64 + k * 2, v, whole);
+                __syncwarp();
+            }
+            continue;
         } else {
             tc_ld32(a.tacc + g * 32, v);
             if (g == groups - 1) wide_release(p, c, a);
             if (a.bias) wide_bias(a.bias, g * 32, v);
-            if (ACT == 1) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) v[j] = apply_act(ACT_GELU, v[j]);
-            }
             if (ACT == 2) act_all(act, v);
         }
         if (live) put32<F16 ? DT_F16 : DT_BF16>(O + g * 64, v, whole);
