@@ -99,6 +99,8 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         c->flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // (mk_launch: what is in front of the launch in its stream has ended, and its writes are visible)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     __syncthreads();
 
     uint32_t left = 0;               // producer and feeder: copies in flight when they left their loop
@@ -829,8 +831,26 @@ int mk_launch(mk_program* p, void* stream) {
     prm.direct_off = p->direct_turn ? (long long)p->direct_bytes : 0;
     prm.direct_next = reinterpret_cast<uint4*>(p->direct + (p->direct_turn ? 0 : p->direct_bytes));
     prm.direct_pieces = (int)(p->direct_bytes / 16);
-    if (p->trace_cap > 0) mk::megakernel<true><<<p->grid, mk::kThreads, mk::kSmemBytes, st>>>(prm);
-    else mk::megakernel<false><<<p->grid, mk::kThreads, mk::kSmemBytes, st>>>(prm);
+    // Programmatic serialization behind the kernel in front in the stream: the launch is prepared while that one's last blocks run, and its
+    // blocks start when those have ended -- every SM is free then, as before -- instead of when their memory has been flushed as well; the
+    // kernel waits for that itself (griddepcontrol.wait) before it reads anything.  A launch behind another 2.3 to 3.5 us earlier: MLP
+    // block of one row 27.1 -> 23.4 us, of 64 35.9 -> 33.4, of 256 54.0 -> 51.2.  A captured launch has ordinary edges.
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) {
+        (void)cudaGetLastError();
+        capturing = cudaStreamCaptureStatusActive;
+    }
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)p->grid);
+    cfg.blockDim = dim3(mk::kThreads);
+    cfg.dynamicSmemBytes = mk::kSmemBytes;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = capturing == cudaStreamCaptureStatusNone ? 1 : 0;
+    (void)cudaLaunchKernelEx(&cfg, p->trace_cap > 0 ? mk::megakernel<true> : mk::megakernel<false>, prm);
     MK_CUDA(cudaGetLastError());
     p->direct_turn ^= 1;
     return MK_OK;

@@ -442,6 +442,63 @@ def test_rows_staged_side_by_side(cuda, monkeypatch, M, K, by_value):
         assert rel_l2(outs[0][r], ref[0][r]) < 1.05 * 2.0 ** -9, r
 
 
+@pytest.mark.parametrize("M", [1, 64])
+@pytest.mark.parametrize("where", ["default stream", "side stream", "captured"])
+def test_launches_behind_kernels_that_write_their_inputs(cuda, M, where):
+    """A launch is prepared while the kernel in front of it runs: it must still see all of that one's writes -- input, weights, the output
+    of the launch before -- and the kernel behind it all of its own."""
+    K, N = 512, 512
+    g = mc.Graph()
+    g.output(g.linear(g.rms_norm(g.input("x", (M, K)), g.param("n", (1, K)), eps=1e-5), g.param("w", (N, K))))
+    prog = mc.compile(g)
+    xs = [rnd((M, K), 1.0, i).to(cuda) for i in range(8)]
+    n, w = rnd((1, K), 0.1, 20, 1.0).to(cuda), rnd((N, K), K ** -0.5, 21).to(cuda)
+    x, out, big = torch.zeros_like(xs[0]), torch.zeros((8, M, N), dtype=BF, device=cuda), torch.zeros(1 << 24, device=cuda)
+
+    def steps():
+        for i in range(8):
+            big.add_(1.0)                        # (a kernel of all SMs whose last blocks end just before the next one)
+            x.copy_(xs[i])
+            y = prog(x=x, n=n, w=w)
+            out[i].copy_(y)
+            x.copy_(y)                           # the next launch's input is this one's output, overwritten
+            y = prog(x=x, n=n, w=w)
+            out[i].add_(y)
+
+    want = []
+    for i in range(8):
+        y0 = prog(x=xs[i], n=n, w=w).clone()
+        torch.cuda.synchronize()
+        y1 = prog(x=y0, n=n, w=w).clone()
+        torch.cuda.synchronize()
+        want.append(y0 + y1)
+    if where == "default stream":
+        for _ in range(20):
+            steps()
+    else:
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            steps()
+        side.synchronize()
+        out.zero_()
+        if where == "side stream":
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                for _ in range(20):
+                    steps()
+            side.synchronize()
+        else:
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=side):
+                steps()
+            graph.replay()
+    torch.cuda.synchronize()
+    prog.check()
+    for i in range(8):
+        assert torch.equal(out[i], want[i]), i
+
+
 def test_values_that_are_nan_end_the_wait(cuda):
     """NaN inputs reach the output as NaN through direct operands; the rows beside them and the launches after are right.  (The input has
     all 16 bits set.  No op can produce the 32-bit marker itself: arithmetic makes 0x7fffffff, an embedding's low half is 0.)"""
