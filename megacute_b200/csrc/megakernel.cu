@@ -833,8 +833,8 @@ int mk_launch(mk_program* p, void* stream) {
     prm.direct_pieces = (int)(p->direct_bytes / 16);
     // Programmatic serialization behind the kernel in front in the stream: the launch is prepared while that one's last blocks run, and its
     // blocks start when those have ended -- every SM is free then, as before -- instead of when their memory has been flushed as well; the
-    // kernel waits for that itself (griddepcontrol.wait) before it reads anything.  A launch behind another 2.3 to 3.5 us earlier: MLP
-    // block of one row 27.1 -> 23.4 us, of 64 35.9 -> 33.4, of 256 54.0 -> 51.2.  A captured launch has ordinary edges.
+    // kernel waits for that itself (griddepcontrol.wait) before it reads anything.  A launch behind another 2 us earlier: MLP
+    // block of one row 25.4 -> 23.5 us, of 64 35.6 -> 33.5, of 256 52.7 -> 50.6.  A captured launch has ordinary edges.
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) {
         (void)cudaGetLastError();
