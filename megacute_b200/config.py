@@ -28,6 +28,7 @@ INST_US, SM_GBPS = 2.0, 40.0    # split-K cost model: fixed us per instruction, 
 # cap a k-tile takes 0.26 - 0.30, 0.50 - 0.56 and 0.76 - 0.84: the same ratios)
 GEMM_BM_WIDE, GEMM_BN_WIDE, WIDE_MIN_ROWS = 256, 256, 128
 GEMM_COST_US = {(128, 128): (6.0, 0.28, 0.0), (256, 128): (2.5, 0.45, 4.0), (256, 256): (2.0, 0.70, 4.0)}
+HALVE_MIN_COLS = 4096           # a linear's last row blocks in half tiles: only with longer products (passes.halve_last_tiles)
 REDUCE_GBPS, FINALIZE_US = 2000.0, 8.0       # a K-split op: bytes of its fp32 reduce-adds; the SplitFinalize hop behind it
 
 # ---- pointwise / norm / attention tiling

@@ -18,6 +18,7 @@ runtime's kernel:
   fuse_gated_linear, fuse_rope_linear   gated residuals and the rotation of q and k into the epilogue of the
                        tile linear before them.
   hoist_linears        linears whose operands are ready long before their place move up.
+  halve_last_tiles     the last rows of a long linear of few 256 x 256 tiles in tiles half as wide.
 """
 
 from __future__ import annotations
@@ -443,6 +444,35 @@ def wide_tiles(g: Graph, sm_count: int) -> Graph:
     return out
 
 
+def halve_last_tiles(g: Graph, sm_count: int) -> Graph:
+    """A linear of 256 x 256 tiles that occupies at most three quarters of the SMs with one tile each: its last row blocks become a linear
+    of their own with 256 x 128 tiles, as many blocks as the free SMs hold.  The first row blocks' operands are there before the op in front
+    has ended, so the SMs that are free by then take a whole tile and the others, which come later, half of one (two thirds of its time).
+    3001 rows, N = 2048, K = 5632: all 96 tiles end after 68 us on 96 SMs, the 32 that start last 25 us behind the rest; now 54 us on 144.
+    MLP block of 2400 / 2700 / 3001 rows 164 -> 158, 184 -> 173, 188 -> 181 us, 4 layers of 2900 tokens (K = 8192) 1923 -> 1883.
+    With more tiles (128: MLP of 4096 rows 230 both ways) too few SMs are free.  Half tiles move a third more operand bytes per flop, so
+    that short products lose where the op behind fills the gap anyway: K = 4096 (DiT of 24 images) 6443 -> 6472, any K 6438 -> 6517."""
+    out = g.derive()
+    ops = []
+    for op in g.ops:
+        r = 0
+        if op.kind == "Linear" and (op.bm, op.bn) == (C.GEMM_BM_WIDE, C.GEMM_BN_WIDE) and op.cos is None and op.x.cols > C.HALVE_MIN_COLS:
+            M, group = op.x.rows, 1 if op.gate is None else op.gate_group
+            mt, nt = -(-M // op.bm), op.w.rows // op.bn
+            r = min(mt - 1, (sm_count - mt * nt) // nt) if 4 * mt * nt <= 3 * sm_count else 0
+            m0 = (mt - r) * op.bm
+        if r <= 0 or m0 % group or M - m0 <= C.WIDE_MIN_ROWS or os.environ.get("MEGACUTE_B200_WIDE_TILES"):
+            ops.append(op)
+            continue
+        for a, rows, bn in ((0, m0, op.bn), (m0, M - m0, C.GEMM_BN)):
+            cut = {f: getattr(op, f).rows_slice(a, rows) for f in ("x", "out", "residual") if getattr(op, f) is not None}
+            if op.gate is not None:
+                cut["gate"] = op.gate.rows_slice(a // group, rows // group)
+            ops.append(op.clone(bn=bn, **cut))
+    out.ops = ops
+    return out
+
+
 def split_argmax(g: Graph, sm_count: int) -> Graph:
     """An argmax over few long rows is cut into column chunks, about two instructions per SM in all;
     every chunk leaves its best (value, index) in a workspace and the last chunk of a row to arrive
@@ -647,6 +677,7 @@ def hoist_linears(g: Graph) -> Graph:
 
 def run_all(g: Graph, sm_count: int) -> Graph:
     """The pass pipeline of ``compile`` (reference order: runtime.py:235, plus wide_tiles, split_argmax,
-    fuse_pointwise, fuse_gated_linear, fuse_rope_linear, promote_temps, fuse_finalize_attention and hoist_linears)."""
+    fuse_pointwise, fuse_gated_linear, fuse_rope_linear, promote_temps, fuse_finalize_attention, hoist_linears and halve_last_tiles)."""
     g = split_argmax(split_kv(fuse_rope_attention(wide_tiles(split_k(fold_norms(g), sm_count), sm_count)), sm_count), sm_count)
-    return hoist_linears(fuse_finalize_attention(promote_temps(fuse_rope_linear(fuse_gated_linear(fuse_pointwise(g))))))
+    g = hoist_linears(fuse_finalize_attention(promote_temps(fuse_rope_linear(fuse_gated_linear(fuse_pointwise(g))))))
+    return halve_last_tiles(g, sm_count)

@@ -234,6 +234,65 @@ def test_tile_kinds_follow_one_another_on_a_cta(cuda, monkeypatch):
     assert prog.tcgen05_ops == len(order)
 
 
+HALVED = [  # rows, columns, K, residual type, gate group -> row blocks of the two linears (three quarters of 148 SMs: 111 tiles)
+    (2500, 2048, 4160, F32, 0, (2, 8)), (2700, 2560, 4160, BF, 0, (8, 3)), (920, 7168, 4160, None, 0, None), (700, 9216, 4160, None, 0, (2, 1)),
+    (640, 9216, 4160, None, 0, None), (2560, 2048, 4160, BF, 64, (2, 8)), (2600, 2048, 4160, F32, 40, None), (2500, 2048, 4096, F32, 0, None),
+    (3600, 2048, 4160, F32, 0, None),
+]
+
+
+def halved_graph(M, N, K, rdt, group):
+    g, t = mc.Graph(), {"x": rnd((M, K), 1.0, 1), "w": rnd((N, K), K ** -0.5, 2)}
+    y = g.linear(g.input("x", (M, K)), g.param("w", (N, K)))
+    if rdt:
+        t["r"] = rnd((M, N), 1.0, 3).to(rdt)
+        if group:
+            t["gate"] = rnd((M // group, N), 1.0, 4)
+            y = g.binary(y, g.input("gate", (M // group, N)), "mul", b_group=group)
+        y = g.add(g.input("r", (M, N), rdt), y)
+    g.output(y)
+    return g, t
+
+
+@pytest.mark.parametrize("M,N,K,rdt,group,blocks", HALVED)
+def test_which_linears_end_in_half_tiles(monkeypatch, M, N, K, rdt, group, blocks):
+    """The two linears cover the rows once, with the operands' rows beside them."""
+    monkeypatch.delenv("MEGACUTE_B200_WIDE_TILES", raising=False)
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 256))
+    ops = [o for o in passes.run_all(halved_graph(M, N, K, rdt, group)[0], 148).ops if o.kind == "Linear"]
+    if blocks is None:
+        assert len(ops) == 1 and ops[0].bn == 256
+        return
+    a, b = ops
+    assert (a.bn, b.bn, -(-a.x.rows // 256), -(-b.x.rows // 256)) == (256, 128, *blocks) and a.x.rows + b.x.rows == M
+    assert a.x.rows == 256 * blocks[0] and a.w.same(b.w)
+    for f in ("x", "out", "residual"):
+        u, v = getattr(a, f), getattr(b, f)
+        assert (u is None) == (v is None) and (u is None or (u.row0, v.row0, u.rows, v.rows) == (0, a.x.rows, a.x.rows, b.x.rows))
+    if group:
+        assert (a.gate.rows, b.gate.row0, b.gate.rows) == (a.x.rows // group, a.x.rows // group, b.x.rows // group)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,rdt,group,blocks", [c for c in HALVED if c[-1]])
+def test_half_tiles_of_the_last_rows(cuda, monkeypatch, M, N, K, rdt, group, blocks):
+    """The same bits as whole tiles give (every output is summed over K in the same order), and the oracle's values."""
+    monkeypatch.delenv("MEGACUTE_B200_WIDE_TILES", raising=False)
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 256))
+    g, t = halved_graph(M, N, K, rdt, group)
+    dev = {n: u.to(cuda) for n, u in t.items()}
+    prog = mc.compile(g)
+    assert [o.bn for o in prog.g.ops if o.kind == "Linear"] == [256, 128]
+    got = prog(**dev).clone()
+    prog.check()
+    monkeypatch.setattr(passes, "halve_last_tiles", lambda g, sm_count: g)
+    whole = mc.compile(g)
+    assert [o.bn for o in whole.g.ops if o.kind == "Linear"] == [256]
+    assert torch.equal(got, whole(**dev))
+    ref, _ = evaluate(g, dev, cuda)
+    assert rel_l2(got, ref[0]) < TOL
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("scale", [-0.3, 0.0])
 @pytest.mark.parametrize("D", [64, 128])
