@@ -22,8 +22,9 @@
 //                1480 -> 1098, 1431 -> 1127 and 1588 -> 1364 us with boxes of the rows there are)
 //   MMA          one compute thread: 4 x tcgen05.mma (128 x 128 x 16) per k-tile; tcgen05.commit
 //                returns the activation stage and the ring slot when the MMAs that read them are done
-//   epilogue     all 8 compute warps: tensor memory -> shared memory (warp w reads lanes 32 (w & 3) .. +31,
-//                column half w >> 2), then row-contiguous global stores / reductions from there
+//   epilogue     all 8 compute warps; warp w reads lanes 32 (w & 3) .. +31, column half w >> 2.  Split-K partials, swiglu, accumulating
+//                and plain tiles: tensor memory -> shared memory, then row-contiguous global stores / reductions from there.
+//                Tiles with a residual, an activation or rotated heads: straight from tensor memory, a row per thread
 // Every wait is bounded (wait_barrier); tensor memory is allocated by the first such instruction of a
 // CTA and freed by the kernel before it exits, on every path.
 #pragma once
@@ -128,8 +129,8 @@ static __device__ __noinline__ void tc_store_rows(const mk_op_desc* op, const fl
     }
 }
 // Epilogues straight from tensor memory, a row per thread and 16 columns at a time, for tiles that read another operand beside the
-// accumulator or compute something from it: what the first columns need is requested before the accumulator is complete, what
-// the next ones need while these are at work.  (A loop over few instructions: sixteen rows of a warp side by side, through the
+// accumulator or compute something from it: the row's whole piece of a residual and gate (rotated heads: the tables of the first 16
+// columns) is requested before the accumulator is complete.  (A loop over few instructions: sixteen rows of a warp side by side, through the
 // staging rows, are straight-line code that is fetched cold once per op.  Time from the complete accumulator, inside a prompt of 333 tokens:
 // rotated heads 7.8 us, as a loop over groups of four rows 6.4, this 3.9.)
 __device__ __forceinline__ bool tc_direct_wait(const Params& p, Ctrl* c, uint32_t apar, int seq) {
@@ -297,7 +298,7 @@ static __device__ __noinline__ bool tc_rope_direct(const Params& p, Ctrl* c, con
     }
     return true;
 }
-// the direct epilogue of a tile with a residual, an activation or rotated heads
+// the instance of the direct epilogue for an op
 template <int ODT>
 __device__ __forceinline__ bool tc_direct_o(const Params& p, Ctrl* c, const mk_op_desc* op, uint32_t two, uint32_t apar, int m0, int n0, int seq) {
     if (ODT != DT_F32 && op->ptr[6]) return tc_rope_direct<ODT>(p, c, op, two, apar, m0, n0, seq);
