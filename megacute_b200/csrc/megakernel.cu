@@ -523,7 +523,10 @@ static int verify_tables(const mk_program* p, const mk_op_desc* ops) {
                     break;
                 case MK_OP_DECODE_ATTN: {
                     const int hp = d.i[10] > 0 ? d.i[10] : 1;
-                    if (a0 < 0 || a0 >= d.i[0] || a1 < 0 || a1 + hp > d.i[2] || a2 < 0 || a2 >= (d.i[5] > 0 ? d.i[5] : 1))
+                    const bool own = d.i[11] && a1 != 0;                     // (many-sequence form: a range of keys of its own)
+                    const int splits = own ? a1 >> 22 : d.i[5];
+                    if (a0 < 0 || a0 >= d.i[0] || a1 < 0 || (!own && a1 + hp > d.i[2]) || a2 < 0 || a2 >= (splits > 0 ? splits : 1) ||
+                        (own && (d.i[4] >= mk::kKvShareMax || splits < 1 || splits > d.i[5] || (a1 & 2047) >= ((a1 >> 11) & 2047) || ((a1 >> 11) & 2047) > 1024)))
                         why = "decode attention: (sequence, kv head, split)";
                     break;
                 }

@@ -75,6 +75,17 @@ __host__ __device__ inline void kv_split_range(int n, int S, int s, int& k_begin
     k_begin = s * per < n ? s * per : n;
     k_end = k_begin + per < n ? k_begin + per : n;
 }
+// ... or, with a range of its own (instruction argument 1: begin | end << 11 | splits of the sequence << 22, the first two in 1024ths
+// of the keys): what it attends, and how many splits the sequence has
+constexpr int kKvShareMax = 1 << 22;
+__host__ __device__ inline int kv_share_at(int n, int u) {
+    const int at = (int)((((unsigned)n * (unsigned)u >> 10) + kKvTileRows - 1) / kKvTileRows * kKvTileRows);      // (n <= kKvShareMax)
+    return at < n ? at : n;
+}
+__host__ __device__ inline void kv_share_range(int n, int range, int& k_begin, int& k_end) {
+    k_begin = kv_share_at(n, range & 2047);
+    k_end = kv_share_at(n, (range >> 11) & 2047);
+}
 constexpr int kTcWSlots = 8;
 // tiles of 256 rows (op_gemm_tc_wide.cuh), of two kinds: 256 columns (kind 0) with three stages of 32 KB of weights and 32 KB of
 // activations, 128 columns (kind 1) with four stages of 16 KB and 32 KB.  Weight slots are in the ring's memory, three

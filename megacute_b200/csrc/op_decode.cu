@@ -27,7 +27,9 @@ static __device__ __forceinline__ bool decode_attn(const Params& p, const SmemMa
 __device__ bool mk_op_decode_attn(const Params& p, const mk_op_desc* op, int a0, int a1, int a2, int nwait, int wait_off,
                                   int seq, int narrive, int arrive_off) {
     const SmemMap m = smem_map();
-    if (op->i[11]) return mk_op_decode_bulk(p, op, a0, a2, nwait, wait_off, seq, narrive, arrive_off);
+    if (op->i[11])
+        return a1 ? mk_op_decode_bulk_own(p, op, a0, a1, a2, nwait, wait_off, seq, narrive, arrive_off)
+                  : mk_op_decode_bulk(p, op, a0, a2, nwait, wait_off, seq, narrive, arrive_off);
     if (op->flags & MK_F_DIRECT_IN) return decode_attn<true>(p, m, op, a0, a1, a2, nwait, wait_off, seq, narrive, arrive_off);
     return decode_attn<false>(p, m, op, a0, a1, a2, nwait, wait_off, seq, narrive, arrive_off);
 }

@@ -9,7 +9,13 @@ namespace mk {
 __device__ bool mk_op_decode_bulk(const Params& p, const mk_op_desc* op, int b, int s, int nwait, int wait_off, int seq,
                                   int narrive, int arrive_off) {
     const SmemMap m = smem_map();
-    decode_bulk_body(p, m.ctrl, op, b, s, m.ring, nwait, wait_off, seq);
+    decode_bulk_body<false>(p, m.ctrl, op, b, 0, s, m.ring, nwait, wait_off, seq);
+    return publish(p, m.ctrl, narrive, arrive_off);
+}
+__device__ bool mk_op_decode_bulk_own(const Params& p, const mk_op_desc* op, int b, int range, int s, int nwait, int wait_off, int seq,
+                                      int narrive, int arrive_off) {
+    const SmemMap m = smem_map();
+    decode_bulk_body<true>(p, m.ctrl, op, b, range, s, m.ring, nwait, wait_off, seq);
     return publish(p, m.ctrl, narrive, arrive_off);
 }
 }  // namespace mk

@@ -19,6 +19,9 @@
 // Bytes in flight are what sets the rate: with five slots (80 KB, ~3 in flight) the stream ran at
 // ~29 GB/s per SM, no faster than the cp.async form.
 //
+// An instruction may have a range of keys of its own (argument 1; passes.bulk_kv_shares), so that all SMs stream the same amount whatever the number
+// of sequences: 64 sequences of 4096 keys on 148 SMs instead of 128, step 2505 -> 2427 us.
+//
 // Shared-memory reads without bank conflicts.  Rows of a tile are 128 x KVH bytes apart, a multiple
 // of 128: the same 16-byte slot of every row falls into the same banks, and an MMA fragment needs
 // eight different keys at one offset.  Three freedoms of the contraction are used instead of padding:
@@ -67,7 +70,10 @@ struct KvPos {
 // ---- compute warps ----
 // All compute threads call this.  Returns after the instruction's global writes (the caller publishes).
 // (G <= 8 query heads per kv head: heads take rows 0..7 of the A operand, their low parts rows 8..15)
-__device__ __forceinline__ void decode_bulk_body(const Params& p, Ctrl* c, const mk_op_desc* op, int b, int s, uint8_t* ring,
+// OWN: the instruction has a range of keys of its own.  Two functions: with both in one, what is alive across the loop for the other form costs
+// programs of equal splits 0.5 % (16 sequences of 10000 keys 1807 -> 1816 us).
+template <bool OWN>
+__device__ __forceinline__ void decode_bulk_body(const Params& p, Ctrl* c, const mk_op_desc* op, int b, int range, int s, uint8_t* ring,
                                                  int nwait, int wait_off, int seq) {
     constexpr int D = 64;
     constexpr float NEG_INF = -__builtin_huge_valf();
@@ -81,9 +87,11 @@ __device__ __forceinline__ void decode_bulk_body(const Params& p, Ctrl* c, const
     const bool hrow = head && g < G;                                  // this lane's MMA row is a query head
     const int pos = reinterpret_cast<const int*>(op->ptr[3])[(long long)b * op->i[12]];      // (i 12: 0, or the stride of per-sequence positions)
     int k_begin, k_end;
-    kv_split_range(fused ? pos : pos + 1, S, s, k_begin, k_end);
+    if (OWN) kv_share_range(fused ? pos : pos + 1, range, k_begin, k_end);
+    else kv_split_range(fused ? pos : pos + 1, S, s, k_begin, k_end);
+    const int splits = OWN ? range >> 22 : S;                        // (S: the rows of partials per sequence)
     const int nk = k_end - k_begin;
-    const bool has_new = fused && s == S - 1;
+    const bool has_new = fused && s == splits - 1;
     KvPos kp;
     kp.slot = (int)(c->kv_cons & 0xffu);
     kp.phase = (c->kv_cons >> 8) & 1u;
@@ -325,7 +333,7 @@ __device__ __forceinline__ void decode_bulk_body(const Params& p, Ctrl* c, const
     };
     void* outp = reinterpret_cast<void*>(op->ptr[4]);
     const long long oe = (long long)b * op->ld[4] + (warp * G + g) * D + q4 * 16;
-    if (S == 1) {
+    if (splits == 1) {
         if (hrow) {
             const float inv = lrow == 0.f ? 0.f : rcp(lrow);
 #pragma unroll
@@ -350,8 +358,8 @@ __device__ __forceinline__ void decode_bulk_body(const Params& p, Ctrl* c, const
     int* count = reinterpret_cast<int*>(op->ptr[10]) + (long long)(b * KVH) * op->ld[10];
     if (t == 0) {
         const int old = arrive_acq_rel(count);
-        c->flag = (old == S - 1);
-        if (old == S - 1) *count = 0;          // back to zero for the next launch
+        c->flag = (old == splits - 1);
+        if (old == splits - 1) *count = 0;          // back to zero for the next launch
     }
     compute_sync();
     phase_mark(p, c, 2);
@@ -365,18 +373,18 @@ __device__ __forceinline__ void decode_bulk_body(const Params& p, Ctrl* c, const
 #pragma unroll
         for (int e = 0; e < 16; ++e) acc[e] = 0.f;
 #pragma unroll 1
-        for (int k = 0; k < S; k += 2) {
+        for (int k = 0; k < splits; k += 2) {
             float m2[2], l2[2];
             float4 v[2][4];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {                                // (an odd last one twice, the second time in place of nothing)
-                const float* row = base + min(k + j, S - 1) * ldp;
+                const float* row = base + min(k + j, splits - 1) * ldp;
                 m2[j] = __ldcg(row + GD + g);
                 l2[j] = __ldcg(row + GD + G + g);
 #pragma unroll
                 for (int e = 0; e < 4; ++e) v[j][e] = __ldcg(reinterpret_cast<const float4*>(row + g * D + q4 * 16 + 4 * e));
             }
-            if (k + 1 == S) {                                            // (zeros, not just no weight: its values may be infinite)
+            if (k + 1 == splits) {                                            // (zeros, not just no weight: its values may be infinite)
                 m2[1] = NEG_INF;
                 l2[1] = 0.f;
 #pragma unroll

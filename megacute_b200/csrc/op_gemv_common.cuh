@@ -96,7 +96,8 @@ struct StageCursor {
                 // pos is rewritten only by the launch's last instruction, behind every reader's arrival
                 const int posv = reinterpret_cast<const volatile int*>(op->ptr[3])[(long long)in.a0 * op->i[12]];
                 int k_begin, k_end;
-                kv_split_range(fused ? posv : posv + 1, S, in.a2, k_begin, k_end);
+                if (in.a1) kv_share_range(fused ? posv : posv + 1, in.a1, k_begin, k_end);
+                else kv_split_range(fused ? posv : posv + 1, S, in.a2, k_begin, k_end);
                 gemm = false; kv = true; attn = false; seq = in.seq;
                 kv_t = 0; kv_nt = (k_end - k_begin + kKvTileRows - 1) / kKvTileRows; kv_which = 0;
                 kv_rb = KVH * 64 * 2;

@@ -51,6 +51,8 @@ __device__ bool mk_op_decode_attn(const Params& p, const mk_op_desc* op, int a0,
 // (many-sequence form: all kv heads of a sequence per instruction, whole cache rows through bulk copies)
 __device__ bool mk_op_decode_bulk(const Params& p, const mk_op_desc* op, int b, int s, int nwait, int wait_off, int seq,
                                   int narrive, int arrive_off);
+__device__ bool mk_op_decode_bulk_own(const Params& p, const mk_op_desc* op, int b, int range, int s, int nwait, int wait_off, int seq,
+                                      int narrive, int arrive_off);
 // pointwise tiles and norms with several rows per instruction (op_stream.cuh): like mk_run_gemm, for runs of their own kind
 __device__ int mk_run_eltwise(const Params& p, const mk_op_desc* op, int idx, int slot);
 __device__ int mk_run_norm(const Params& p, const mk_op_desc* op, int idx, int slot);

@@ -125,7 +125,7 @@ OP_TABLE = {
     "DecodeAttention": (("q", "k_cache", "v_cache", "pos", "k_new", "v_new", "cos", "sin", "part", "count"),
                         ("out", "part", "count"),
                         ("batch", "heads", "kv_heads", "head_dim", "max_seq", "scale", "splits", "zero_inputs", "heads_per_inst",
-                         "bulk", "window")),
+                         "bulk", "window", "shares")),
     "Increment":       ((), ("pos",), ()),
     # the two ends of a decode step, inside the launch (no counterpart among the reference's ops: its
     # step does them in torch around the launch, examples/llama/llama1b.py:103-105)

@@ -23,6 +23,7 @@ runtime's kernel:
 
 from __future__ import annotations
 
+import functools
 import os
 
 import torch
@@ -160,15 +161,73 @@ def bulk_kv_splits(batch: int, kv_heads: int, max_seq: int, sm_count: int) -> in
     cap = max(1, min(max_seq // C.MIN_SPLIT_KEYS, C.MAX_KV_SPLITS))
     if os.environ.get("MEGACUTE_B200_KV_SPLITS"):
         return max(1, min(cap, int(os.environ["MEGACUTE_B200_KV_SPLITS"])))
+    cost = lambda s: bulk_split_cost(batch, kv_heads, max_seq, sm_count, s)
+    return min(range(1, cap + 1), key=lambda s: (round(cost(s), 9), s))
+
+
+def bulk_split_cost(batch: int, kv_heads: int, max_seq: int, sm_count: int, s: int) -> float:
+    """Modelled time (us) of the many-sequence form with s equal splits per sequence."""
     tile_us = C.BULK_TILE_US_PER_KB * kv_heads * 128 / 1024
-    best, best_cost = 1, float("inf")
-    for s in range(1, cap + 1):
-        waves = -(-(batch * s) // sm_count)
-        tiles = -(-(-(-max_seq // s)) // C.BULK_TILE_ROWS)
-        cost = waves * (max(C.BULK_FIXED_US, C.BULK_US_PER_SPLIT * s - 3.0) + tiles * tile_us)
-        if cost < best_cost - 1e-9:
-            best, best_cost = s, cost
-    return best
+    tiles = -(-(-(-max_seq // s)) // C.BULK_TILE_ROWS)
+    return -(-(batch * s) // sm_count) * (max(C.BULK_FIXED_US, C.BULK_US_PER_SPLIT * s - 3.0) + tiles * tile_us)
+
+
+@functools.lru_cache(maxsize=256)
+def bulk_kv_shares(batch: int, kv_heads: int, max_seq: int, sm_count: int) -> tuple:
+    """(modelled time, instructions) of the many-sequence form with the same amount of work on every SM: the sequences' keys, one behind
+    the other, are dealt out to the SMs, so that an SM may end one sequence and begin another, with an instruction for each.  Instructions
+    are (sequence, split, begin and end in 1024ths of its keys, splits of the sequence), in rounds: an SM's first, its second.
+
+    What bounds the form is the keys an SM can have in flight, so every SM without a split is lost: 2 splits of 64 sequences run on 128 of 148,
+    5 of 50 in rounds of 148 and 102.  Steps of 64 / 60 / 50 / 40 sequences at context 4096 / 4000 / 2000 / 4000: 2505 -> 2427, 2654 -> 2317, 1838 -> 1639,
+    2068 -> 1883 us.  A second instruction on an SM costs more than a first (BULK_SHARE_US 3 / 5 / 7 / 8: 50 sequences at 2000 -- / 1709 / 1677 / 1639),
+    so SMs with two get fewer keys.  Taken when the model puts it at most 3 us behind equal splits (-BULK_SHARE_GAIN_US): 55 x 1500, 1.2 us behind,
+    1686 -> 1534, 64 x 2000, 2.4 behind, 1819 -> 1804; 32 x 4000, 3.8 behind, 1748 -> 1780, 64 x 1024, 5 behind, 1490 -> 1499."""
+    whole = -(-max_seq // C.BULK_TILE_ROWS) * C.BULK_TILE_US_PER_KB * kv_heads * 128 / 1024       # us of a sequence
+    least = 32                                                                                   # 1024ths
+    best = (float("inf"), ())
+    low, high = 0.0, 2 * (batch * (whole + C.BULK_SHARE_US) / sm_count + C.BULK_SHARE_US)
+    for _ in range(30):                                      # the smallest load of an SM with which they are enough
+        budget = (low + high) / 2
+        sms, room, load = [[]], budget, [0.0]
+        for b in range(batch):
+            at = 0
+            while at < 1024:
+                take = int((room - C.BULK_SHARE_US) / whole * 1024)
+                if take < least and sms[-1]:
+                    sms.append([])
+                    load.append(0.0)
+                    room = budget
+                    continue
+                take = min(max(take, least), 1024 - at)
+                if 1024 - at - take < least:
+                    take = 1024 - at
+                sms[-1].append((b, at, at + take))
+                load[-1] += C.BULK_SHARE_US + take / 1024 * whole
+                room = budget - load[-1]
+                at += take
+        if len(sms) <= sm_count:
+            high = budget
+            if max(load) < best[0]:
+                best = (max(load), sms)
+        else:
+            low = budget
+    cost, sms = best
+    while 0 < len(sms) < sm_count:                           # (an SM without an instruction would shift the second round)
+        at = max(range(len(sms)), key=lambda i: max(u1 - u0 for _, u0, u1 in sms[i]))
+        k = max(range(len(sms[at])), key=lambda i: sms[at][i][2] - sms[at][i][1])
+        b, u0, u1 = sms[at][k]
+        if u1 - u0 < 2 * least:
+            return float("inf"), ()
+        sms[at][k] = (b, u0, (u0 + u1) // 2)
+        sms.append([(b, (u0 + u1) // 2, u1)])
+    pieces = sorted(x for sm in sms for x in sm)
+    first = {b: k for k, (b, _, _) in reversed(list(enumerate(pieces)))}
+    count = {b: sum(x[0] == b for x in pieces) for b in first}
+    number = {x: k - first[x[0]] for k, x in enumerate(pieces)}
+    sms = sorted(([(x[0], number[x], x[1], x[2], count[x[0]]) for x in sm] for sm in sms), key=len, reverse=True)
+    cost += max(0.0, C.BULK_US_PER_SPLIT * max(count.values()) - 3.0 - C.BULK_FIXED_US)
+    return cost, tuple(sm[k] for k in range(len(sms[0])) for sm in sms if k < len(sm))
 
 
 def split_kv(g: Graph, sm_count: int) -> Graph:
@@ -178,6 +237,10 @@ def split_kv(g: Graph, sm_count: int) -> Graph:
         if op.kind == "DecodeAttention" and op.splits == 1 and bulk_eligible(op):
             s = bulk_kv_splits(op.batch, op.kv_heads, op.max_seq, sm_count)
             op = op.clone(heads_per_inst=op.kv_heads, bulk=True)
+            cost, shares = bulk_kv_shares(op.batch, op.kv_heads, op.max_seq, sm_count)
+            if shares and not os.environ.get("MEGACUTE_B200_KV_SPLITS") and op.max_seq < C.BULK_SHARE_MAX_SEQ and max(x[4] for x in shares) <= C.MAX_KV_SPLITS and \
+                    cost < bulk_split_cost(op.batch, op.kv_heads, op.max_seq, sm_count, s) - C.BULK_SHARE_GAIN_US:
+                op, s = op.clone(shares=shares), max(x[4] for x in shares)
             if s > 1:
                 G, D = op.heads // op.kv_heads, op.head_dim
                 cols = -(-(G * D + 2 * G) // 4) * 4          # per (kv head, split): O (G x D), running max (G), sum (G)

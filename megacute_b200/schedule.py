@@ -246,6 +246,10 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
         hp = op.heads_per_inst or 1          # kv heads h .. h + hp - 1 per instruction (unsplit batched decode)
         b, h, s = (a.ravel() for a in np.meshgrid(np.arange(op.batch), np.arange(0, op.kv_heads, hp), np.arange(S),
                                                   indexing="ij"))
+        rng = h
+        if op.shares:
+            b, s, u0, u1, ns = np.array(op.shares, np.int64).T
+            h, rng = np.zeros_like(b), u0 | u1 << 11 | ns << 22
         n = len(b)
         cache = lambda v, kind: _acc(v, kind, b * L, (b + 1) * L, h * D, (h + hp) * D, n=n, covers=False)
         qcols = (h * G * D, (h + hp) * G * D)
@@ -265,7 +269,7 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
             r = b * op.kv_heads + h
             acc += [_acc(op.part, WRITE, r * S, (r + hp) * S, n=n, covers=False),
                     _acc(op.count, WRITE, r, r + hp, n=n, covers=False)]
-        return Tiled(_args(n, b, h, s), acc)
+        return Tiled(_args(n, b, rng, s), acc)
     if k == "Increment":
         return Tiled(_args(1), [_acc(op.pos, WRITE, n=1)])
     if k == "Gather":

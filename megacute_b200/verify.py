@@ -160,6 +160,21 @@ def op_grid(op, sm_count: int):
     raise NotImplementedError(k)
 
 
+def check_shares(kk: int, op, args) -> None:
+    """Instructions with a range of keys of their own: every sequence's keys are covered once, its splits counted from 0."""
+    b, s, u0, u1, n = args[:, 0], args[:, 2], args[:, 1] & 2047, (args[:, 1] >> 11) & 2047, args[:, 1] >> 22
+    order = np.lexsort((u0, b))
+    b, s, u0, u1, n = (v[order] for v in (b, s, u0, u1, n))
+    first = np.r_[True, b[1:] != b[:-1]]
+    last = np.r_[first[1:], True]
+    runs = np.diff(np.r_[np.nonzero(first)[0], len(b)])
+    ok = (b[first] == np.arange(op.batch)).all() and len(runs) == op.batch and (u0 < u1).all() and (u0[first] == 0).all() and (u1[last] == 1024).all()
+    ok = ok and (u0[1:][~first[1:]] == u1[:-1][~first[1:]]).all() and (n == np.repeat(runs, runs)).all() and runs.max() <= op.splits
+    ok = ok and (s == np.concatenate([np.arange(r) for r in runs])).all() and (args[:, 3:] == 0).all()
+    if not ok:
+        raise VerifyError(f"op {kk} {op.kind}: the shares do not partition the keys")
+
+
 def check_tables(g: Graph, sched: Schedule, tensors: dict | None = None) -> None:
     """Operand windows inside their views, views inside their buffers (and, with ``tensors`` -- buffer id
     -> bound tensor -- inside the bound storage), instruction arguments inside the op's tiling."""
@@ -187,6 +202,9 @@ def check_tables(g: Graph, sched: Schedule, tensors: dict | None = None) -> None
                                       f"is not the buffer ({b.rows} x {b.cols}, row-major)")
         a0, a1 = sched.node_ranges[kk]
         args = sched.args[a0:a1].astype(np.int64)
+        if op.kind == "DecodeAttention" and op.shares:
+            check_shares(kk, op, args)
+            continue
         lim = op_grid(op, sched.sm_count)
         if lim and lim[0] == "range":
             ok = (0 <= args[:, 0]).all() and (args[:, 0] < args[:, 1]).all() and (args[:, 1] <= lim[1]).all()

@@ -187,6 +187,19 @@ def test_decode_attention_many_sequences(cuda, monkeypatch, B, H, KVH, max_seq, 
     assert att and all(o.bulk and o.heads_per_inst == KVH and o.splits == min(splits, max_seq // 64) for o in att)
 
 
+@pytest.mark.parametrize("B,H,KVH,max_seq,ctx", [(40, 16, 8, 512, 300), (33, 8, 2, 256, 37), (64, 32, 8, 128, 0), (61, 32, 8, 384, 257), (150, 8, 8, 256, 129),
+                                                 (16, 32, 8, 1024, 960)])
+@pytest.mark.parametrize("fused", [False, True])
+def test_decode_attention_equal_shares(cuda, monkeypatch, B, H, KVH, max_seq, ctx, fused):
+    """The many-sequence form with ranges of keys of unequal length, one or two instructions per SM: contexts that leave many of them empty, that
+    end inside a tile, splits of one sequence on several SMs and of several on one."""
+    monkeypatch.setenv("MEGACUTE_B200_ATT_BULK", "1")
+    monkeypatch.setattr(C, "BULK_SHARE_GAIN_US", -1e9)
+    prog = _decode_attention_case(cuda, B, H, KVH, 64, max_seq, ctx, fused)
+    att = [o for o in prog.g.ops if o.kind == "DecodeAttention"]
+    assert att and all(o.shares and o.splits == max(x[4] for x in o.shares) for o in att)
+
+
 def _decode_attention_case(cuda, B, H, KVH, D, max_seq, ctx, fused):
     g = mc.Graph()
     qkv = g.input("qkv", (B, (H + 2 * KVH) * D))

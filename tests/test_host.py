@@ -420,3 +420,26 @@ def test_rows_per_streaming_instruction_follow_the_sm_count(sms):
         d = _lib.OpDesc()
         encode.fill(d, op, lambda v: 0, sms)
         assert sms // 2 < b - a <= sms and -(-2048 // d.i[field]) == b - a
+
+
+@pytest.mark.parametrize("batch,max_seq", [(32, 4224), (33, 128), (40, 4224), (50, 2048), (60, 8192), (64, 4224), (96, 1152), (147, 512), (200, 4224)])
+def test_equal_shares_of_many_sequences(batch, max_seq):
+    """Every key of every sequence in one instruction, as many instructions in the first round as there are SMs, later rounds on the SMs of
+    the first ones of it; and the ranges the device makes of them, at any context."""
+    from megacute_b200.passes import bulk_kv_shares
+    from megacute_b200.verify import check_shares
+    cost, shares = bulk_kv_shares(batch, 8, max_seq, 148)
+    assert shares and cost < float("inf")
+    b, s, u0, u1, n = np.array(shares).T
+    op = type("Op", (), dict(kind="DecodeAttention", batch=batch, splits=int(n.max())))()
+    args = np.zeros((len(b), 7), np.int64)
+    args[:, 0], args[:, 1], args[:, 2] = b, u0 | u1 << 11 | n << 22, s
+    check_shares(0, op, args)
+    rounds = [shares[i:i + 148] for i in range(0, len(shares), 148)]
+    assert len(rounds[0]) == 148 and (args[:, 1] < 2 ** 31).all()
+    at = lambda keys, u: min(keys, ((keys * u >> 10) + 15) // 16 * 16)             # (kv_share_at, csrc/mk_device.cuh)
+    for keys in (0, 1, 15, 16, 17, 300, max_seq - 1, max_seq):
+        got = sorted((int(x), at(keys, int(v)), at(keys, int(w))) for x, v, w in zip(b, u0, u1))
+        for q in range(batch):
+            mine = [g[1:] for g in got if g[0] == q]
+            assert mine[0][0] == 0 and mine[-1][1] == keys and all(x[1] == y[0] and x[0] <= x[1] for x, y in zip(mine, mine[1:] + [(keys, keys)]))
