@@ -139,17 +139,23 @@ def kv_heads_per_instruction(pairs: int, kv_heads: int, max_seq: int, sm_count: 
     return best
 
 
-def bulk_eligible(op: Op) -> bool:
+def bulk_eligible(op: Op, sm_count: int) -> bool:
     """Can this decode attention run in the many-sequence form (csrc/op_decode_bulk.cuh)?  One warp per
     kv head, head_dim 64, and cache views that are whole rows of their buffers, 128 bytes per kv head,
-    so that consecutive rows are one contiguous run of memory."""
+    so that consecutive rows are one contiguous run of memory.  And should it?  The per-head form has an instruction per (sequence, kv head):
+    more of them than SMs go one behind the other (8 kv heads, 20 sequences at 500 / 24 at 2000 / 24 at 4000 / 31 at 1000: 1166 -> 1103,
+    1627 -> 1295, 1981 -> 1520, 1319 -> 1241 us a step; 28 at 300 1139 -> 1134).  Fewer: where the cache is long enough for the higher rate of
+    whole rows (10 x 3000 1355 -> 1217, 16 x 4000 1464 -> 1363, 8 x 4000 1284 -> 1234, 14 x 2000 1208 -> 1178; but 16 x 1500 1152 -> 1182, 9 x 2000
+    1123 -> 1159, 16 x 1000 1081 -> 1144; the line is at 28 K rows)."""
     if os.environ.get("MEGACUTE_B200_ATT_BULK") == "0" or getattr(op, "window", 0):      # (no sliding window in that form)
         return False
     whole = all(v.col0 == 0 and v.cols == v.buf.cols for v in (op.k_cache, op.v_cache))
     ok = op.head_dim == 64 and op.kv_heads <= C.COMPUTE_WARPS and whole and op.k_cache.cols == op.kv_heads * 64
     if os.environ.get("MEGACUTE_B200_ATT_BULK") == "1":
         return ok
-    return ok and (op.batch >= C.BULK_MIN_BATCH or (op.batch >= C.BULK_MIN_BATCH_LONG and op.max_seq >= C.BULK_LONG_SEQ))
+    if op.batch >= C.BULK_MIN_BATCH or op.batch * op.kv_heads > sm_count:
+        return ok
+    return ok and op.batch >= C.BULK_MIN_BATCH_LONG and (op.max_seq >= C.BULK_LONG_SEQ or op.batch * op.max_seq * op.kv_heads >= C.BULK_MIN_PIECES)
 
 
 def bulk_kv_splits(batch: int, kv_heads: int, max_seq: int, sm_count: int) -> int:
@@ -234,7 +240,7 @@ def split_kv(g: Graph, sm_count: int) -> Graph:
     out = g.derive()
     ops = []
     for op in g.ops:
-        if op.kind == "DecodeAttention" and op.splits == 1 and bulk_eligible(op):
+        if op.kind == "DecodeAttention" and op.splits == 1 and bulk_eligible(op, sm_count):
             s = bulk_kv_splits(op.batch, op.kv_heads, op.max_seq, sm_count)
             op = op.clone(heads_per_inst=op.kv_heads, bulk=True)
             cost, shares = bulk_kv_shares(op.batch, op.kv_heads, op.max_seq, sm_count)

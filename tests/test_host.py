@@ -422,6 +422,15 @@ def test_rows_per_streaming_instruction_follow_the_sm_count(sms):
         assert sms // 2 < b - a <= sms and -(-2048 // d.i[field]) == b - a
 
 
+@pytest.mark.parametrize("B,KVH,L,want", [(18, 8, 1152, False), (19, 8, 128, True), (20, 8, 512, True), (31, 4, 512, False), (31, 4, 2048, True), (14, 8, 2048, True),
+                                          (13, 8, 2048, False), (8, 8, 3584, True), (7, 8, 8192, False), (28, 8, 256, True)])
+def test_which_decode_attention_takes_whole_rows(monkeypatch, B, KVH, L, want):
+    for k in ("MEGACUTE_B200_ATT_BULK", "MEGACUTE_B200_KV_SPLITS"):
+        monkeypatch.delenv(k, raising=False)
+    g, *_ = small_decode(B=B, n=1, E=512, H=8, KVH=KVH, F=512, vocab=512, max_seq=L, ctx=10)
+    assert [bool(o.bulk) for o in run_all(g, 148).ops if o.kind == "DecodeAttention"] == [want]
+
+
 @pytest.mark.parametrize("batch,max_seq", [(32, 4224), (33, 128), (40, 4224), (50, 2048), (60, 8192), (64, 4224), (96, 1152), (147, 512), (200, 4224)])
 def test_equal_shares_of_many_sequences(batch, max_seq):
     """Every key of every sequence in one instruction, as many instructions in the first round as there are SMs, later rounds on the SMs of
