@@ -146,7 +146,9 @@ def bulk_eligible(op: Op, sm_count: int) -> bool:
     more of them than SMs go one behind the other (8 kv heads, 20 sequences at 500 / 24 at 2000 / 24 at 4000 / 31 at 1000: 1166 -> 1103,
     1627 -> 1295, 1981 -> 1520, 1319 -> 1241 us a step; 28 at 300 1139 -> 1134).  Fewer: where the cache is long enough for the higher rate of
     whole rows (10 x 3000 1355 -> 1217, 16 x 4000 1464 -> 1363, 8 x 4000 1284 -> 1234, 14 x 2000 1208 -> 1178; but 16 x 1500 1152 -> 1182, 9 x 2000
-    1123 -> 1159, 16 x 1000 1081 -> 1144; the line is at 28 K rows)."""
+    1123 -> 1159, 16 x 1000 1081 -> 1144; the line is at 28 K rows).  Five to seven sequences hand their values on directly in the per-head form
+    and need 55 K rows (5 x 12000 1502 -> 1404, 6 x 10000 1380 -> 1355, 7 x 8000 1430 -> 1335; but 5 x 6000 1225 -> 1263, 6 x 5000 1210 -> 1234); four stay
+    (4 x 16000 1481 -> 1443, but of different lengths at 15000 1356 -> 1414, 4 x 8000 1212 -> 1271)."""
     if os.environ.get("MEGACUTE_B200_ATT_BULK") == "0" or getattr(op, "window", 0):      # (no sliding window in that form)
         return False
     whole = all(v.col0 == 0 and v.cols == v.buf.cols for v in (op.k_cache, op.v_cache))
@@ -155,7 +157,10 @@ def bulk_eligible(op: Op, sm_count: int) -> bool:
         return ok
     if op.batch >= C.BULK_MIN_BATCH or op.batch * op.kv_heads > sm_count:
         return ok
-    return ok and op.batch >= C.BULK_MIN_BATCH_LONG and (op.max_seq >= C.BULK_LONG_SEQ or op.batch * op.max_seq * op.kv_heads >= C.BULK_MIN_PIECES)
+    pieces = op.batch * op.max_seq * op.kv_heads
+    if op.batch >= C.BULK_MIN_BATCH_LONG:
+        return ok and (op.max_seq >= C.BULK_LONG_SEQ or pieces >= C.BULK_MIN_PIECES)
+    return ok and op.batch >= C.BULK_MIN_BATCH_FEW and pieces >= C.BULK_MIN_PIECES_FEW
 
 
 def bulk_kv_splits(batch: int, kv_heads: int, max_seq: int, sm_count: int) -> int:

@@ -423,7 +423,8 @@ def test_rows_per_streaming_instruction_follow_the_sm_count(sms):
 
 
 @pytest.mark.parametrize("B,KVH,L,want", [(18, 8, 1152, False), (19, 8, 128, True), (20, 8, 512, True), (31, 4, 512, False), (31, 4, 2048, True), (14, 8, 2048, True),
-                                          (13, 8, 2048, False), (8, 8, 3584, True), (7, 8, 8192, False), (28, 8, 256, True)])
+                                          (13, 8, 2048, False), (8, 8, 3584, True), (7, 8, 7936, False), (7, 8, 8064, True),
+                                          (5, 8, 11264, True), (4, 8, 14080, False), (28, 8, 256, True)])
 def test_which_decode_attention_takes_whole_rows(monkeypatch, B, KVH, L, want):
     for k in ("MEGACUTE_B200_ATT_BULK", "MEGACUTE_B200_KV_SPLITS"):
         monkeypatch.delenv(k, raising=False)
