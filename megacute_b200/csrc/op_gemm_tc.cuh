@@ -182,6 +182,13 @@ template <int DT> struct Row64 {
         for (int k = 0; k < 6 * kPer8; ++k) w[k] = w[k + 2 * kPer8];
     }
 };
+// 16 columns of a row as 16-bit, or the first eight of them where the row has `cols` left (whole eights; none: nothing)
+template <int ODT>
+__device__ __forceinline__ void put_upto16(uint8_t* at, const float* v, int cols, bool whole) {
+    if (cols >= 16) put16<ODT>(at, v, whole);
+    else if (cols > 0)
+        *reinterpret_cast<uint4*>(at) = make_uint4(pack2t(ODT, v[0], v[1]), pack2t(ODT, v[2], v[3]), pack2t(ODT, v[4], v[5]), pack2t(ODT, v[6], v[7]));
+}
 // out = act(acc + bias) [* gate row of i 12 rows] [+ residual].  RKIND 0: no residual, 1: 16-bit, 2: fp32.  ACT 0: none, 1: gelu, 2: any.
 // GATE: with ACT 2 decided at run time.
 template <int ODT, int RKIND, int ACT, bool GATE>
@@ -233,10 +240,8 @@ static __device__ __noinline__ bool tc_cols_direct(const Params& p, Ctrl* c, con
             if (ODT == DT_F32) {
                 st32B(at, reinterpret_cast<const uint32_t*>(v), whole);
                 if (more) st32B(at + 32, reinterpret_cast<const uint32_t*>(v) + 8, whole);
-            } else if (more) {
-                put16<ODT>(at, v, whole);
             } else {
-                *reinterpret_cast<uint4*>(at) = make_uint4(pack2t(ODT, v[0], v[1]), pack2t(ODT, v[2], v[3]), pack2t(ODT, v[4], v[5]), pack2t(ODT, v[6], v[7]));
+                put_upto16<ODT>(at, v, cols - k, whole);
             }
         }
         if (RKIND) r.next();
@@ -245,7 +250,8 @@ static __device__ __noinline__ bool tc_cols_direct(const Params& p, Ctrl* c, con
     }
     return true;
 }
-//   rotated heads (descriptor: op_gemm.cuh): 16 columns of both halves of a head at a time, with the row's piece of the tables
+//   rotated heads (descriptor: op_gemm.cuh): 16 columns of both halves of a head at a time, with the row's piece of the tables.  Columns behind
+//   the heads (N is whole eights, not whole heads: a gate or a router packed behind v) end anywhere in a piece: it is stored as far as N goes.
 template <int ODT>
 static __device__ __noinline__ bool tc_rope_direct(const Params& p, Ctrl* c, const mk_op_desc* op, uint32_t two, uint32_t apar, int m0, int n0,
                                                    int seq) {
@@ -269,7 +275,8 @@ static __device__ __noinline__ bool tc_rope_direct(const Params& p, Ctrl* c, con
     };
     request(0);
     const bool ok = tc_direct_wait(p, c, apar, seq);
-    if (!ok || m0 + qd * 32 >= M || n0 + col0 >= op->i[1]) return ok;
+    const int room = op->i[1] - n0 - col0;                    // columns from this warp's first to the row's end
+    if (!ok || m0 + qd * 32 >= M || room <= 0) return ok;
     const uint32_t tl = *(volatile uint32_t*)&c->tmem_base + ((uint32_t)(qd * 32) << 16) + col0;
     auto get = [&](uint32_t w) { return t16 ? unpack2h(w) : make_float2(bf16_lo(w), bf16_hi(w)); };
 #pragma unroll 1
@@ -291,8 +298,8 @@ static __device__ __noinline__ bool tc_rope_direct(const Params& p, Ctrl* c, con
         }
         if (d == 0) request(16);
         if (row < M) {
-            put16<ODT>(O + d * 2, x1, whole);
-            put16<ODT>(O + (half + d) * 2, x2, whole);
+            put_upto16<ODT>(O + d * 2, x1, room - d, whole);
+            put_upto16<ODT>(O + (half + d) * 2, x2, room - half - d, whole);
         }
         __syncwarp();
     }

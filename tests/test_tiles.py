@@ -117,6 +117,38 @@ def test_rotated_heads_at_tile_edges(cuda, B, S, H, KVH, D, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("extra", [8, 40, 72])
+@pytest.mark.parametrize("B,S,H,KVH,D,K", [(1, 100, 2, 1, 64, 64), (3, 50, 1, 1, 64, 128), (1, 100, 2, 1, 128, 64), (2, 129, 1, 1, 128, 192), (1, 9, 3, 1, 64, 64)])
+def test_columns_behind_rotated_heads(cuda, B, S, H, KVH, D, K, extra):
+    """A projection with more behind v than whole heads: rows end inside a warp's piece of columns.  Nothing reaches the next row's first
+    head or, behind the last row, the memory after the buffer."""
+    n, heads = (H + 2 * KVH) * D, H + KVH
+    g = mc.Graph()
+    x, w = g.input("x", (B * S, K)), g.param("w", (n + extra, K))
+    cos, sin = g.input("cos", (S, D)), g.input("sin", (S, D))
+    y = g.linear(x, w)
+    q = g.rope(y.cols_slice(0, H * D), cos, sin, heads=H, head_dim=D, seq=S)
+    k = g.rope(y.cols_slice(H * D, KVH * D), cos, sin, heads=KVH, head_dim=D, seq=S)
+    g.output(g.attention(q, k, y.cols_slice(heads * D, KVH * D), batch=B, heads=H, kv_heads=KVH, head_dim=D, causal=True))
+    g.output(g.unary(y.cols_slice(n, extra), "silu"))
+    cs, sn = W.rope_tables(S, D)
+    t = {"x": rnd((B * S, K), 1.0, 1), "w": rnd((n + extra, K), 0.1, 2), "cos": cs, "sin": sn}
+    prog = mc.compile(g)
+    lin = [o for o in prog.g.ops if o.kind == "Linear"][0]
+    assert lin.cos is not None and not any(o.kind == "Rope" for o in prog.g.ops)
+    buf = lin.out.buf
+    guarded = torch.full((buf.rows * buf.cols + 1024,), 7.0, dtype=buf.dtype, device=cuda)
+    prog._bufs[buf.id] = guarded[:buf.rows * buf.cols].view(buf.rows, buf.cols)
+    ref, _ = evaluate(g, t)
+    for _ in range(3):
+        outs = prog(**{name: v.to(cuda) for name, v in t.items()})
+        prog.check()
+        assert prog.tcgen05_ops == 1 and (guarded[buf.rows * buf.cols:] == 7.0).all()
+        for o, r in zip(outs, ref):
+            assert rel_l2(o, r.to(cuda)) < TOL
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("tcgen05", [True, False])
 @pytest.mark.parametrize("B,S,D,tile", [(1, 150, 64, (128, 128)), (3, 50, 128, (128, 128)), (2, 129, 64, (256, 256)), (1, 257, 128, (256, 128)),
                                         (1, 300, 128, (256, 256))])
