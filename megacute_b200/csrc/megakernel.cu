@@ -53,12 +53,11 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
             mbar_init(&c->x_full[s], 1);
             mbar_init(&c->x_empty[s], 1);
         }
-        c->x_par = 0;
         for (int s = 0; s < kTcWSlots; ++s) {
             mbar_init(&c->w_full[s], 1);
             mbar_init(&c->w_empty[s], 1);
         }
-        c->w_slot = c->w_phase = 0;
+        c->tile_state = 0;
         for (int s = 0; s < 2 * kWideStages; ++s) {
             mbar_init(&c->ww_full[0][0] + s, 2);
             mbar_init(&c->ww_empty[0][0] + s, 1);
@@ -91,7 +90,6 @@ __global__ void __launch_bounds__(kThreads, 1) megakernel(const __grid_constant_
         }
         mbar_init(&c->kv_go, 1);
         c->kv_cons = 0;
-        c->acc_uses = 0;
         c->tmem_base = kTcNoTmem;
         c->tmem_ready = 0;
         c->abort = 0;

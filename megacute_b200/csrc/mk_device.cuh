@@ -209,15 +209,16 @@ struct Ctrl {                     // lives in the last kCtrlBytes of shared memo
     unsigned long long ring_granted, ring_returned;      // ... head_dim 128: the run may use the ring's memory / is done with it
     uint32_t at_blocks[2][2];                // ... blocks of each Q tile so far, written for the next instruction during this one
     uint32_t tmem_base;               // ... tensor-memory address of the accumulator (written by tcgen05.alloc)
-    uint16_t x_par;                       // ... bit s: parity of the next completion of x_full[s] and of x_empty[s] (between
-                                          //     instructions both have completed equally often); set at an instruction's end
+    uint16_t tile_state;                  // ... what the next 128 x 128 tile instruction starts from; changes behind the barrier that ends one.  Bits 0 .. 9:
+                                          //     parity of the next completion of x_full[s] and of x_empty[s] (between instructions both have
+                                          //     completed equally often), 10: parity of acc_full, 11 .. 14: position in the weight slots and
+                                          //     its phase (weight k-tiles so far mod 16)
+    uint16_t tile_next;                   // ... the same behind the current instruction, parked by thread 0 during it
     uint8_t x_left[2];                    // ... during one, by the lane that arms every other stage, once it has: next stage | round << 4 |
                                           //     ten stages << 5; read on the abort path only.  0xff between instructions
-    uint8_t w_slot, w_phase;              // ... the MMA thread's position in the weight slots
     uint8_t at_turn;                      // tcgen05 prefill attention: which at_blocks is current (bit 0)
     uint8_t tmem_ready;               // 1 once tensor memory is allocated; written behind the barrier that follows the allocation, so
                                       //     all threads of an instruction read the same value (tmem_base changes while they arrive)
-    uint32_t acc_uses;                // ... instructions that have used acc_full (its parity)
     int abort;                    // set once a wait of this CTA gave up or saw the global abort
     int flag;                     // scratch broadcast word (split-KV last arriver; < 0: direct operands that never came)
     long long t_dep;              // tracing: when the dependencies of the current instruction were met

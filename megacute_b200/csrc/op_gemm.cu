@@ -14,7 +14,7 @@ __device__ int mk_run_gemm(const Params& p, int idx, int slot) {
         // (the weight tiles have slots and barriers of their own: the ring position is untouched)
         // (tiles of 256 rows have a translation unit of their own, op_gemm_wide.cu: the kernel calls it directly)
         [&](const mk_op_desc* op, int a0, int a1, int a2, int seq) -> int { return op_gemm_tc(p, m.ctrl, m.ring, m.work, op, a0, a1, a2, seq); },
-        [] {});
+        [&] { tc_next_state(m.ctrl); });
 }
 // ... and the mma.sync body: a walk of its own, so that its loop over tiles is no part of the other one's registers (frame 204 -> 188 bytes: prompt of
 // 333 tokens 1849 -> 1836 us, 64 sequences at context 1024 1528 -> 1526)

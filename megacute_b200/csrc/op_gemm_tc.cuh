@@ -44,19 +44,19 @@ __device__ __forceinline__ void tc_ld16_sum(uint32_t taddr, uint32_t second, flo
     for (int j = 0; j < 16; ++j) v[j] += w[j];
 }
 
-// State the next tile GEMM instruction of this CTA starts from, written by one thread behind the barrier that
-// ends the epilogue: the accumulator barrier's use count, the parities of the activation stages (stage s was
-// used once more per full round through the stages, and once more if s < nk mod stages) and the position in
-// the weight slots.
-__device__ __forceinline__ void tc_finish_state(Ctrl* c, uint32_t uses, uint32_t xpar0, uint32_t ws0, uint32_t wph0, int nk,
-                                                uint32_t xstages) {
-    c->acc_uses = uses + 1;
+// Ctrl::tile_state behind an instruction of nk k-tiles: the accumulator barrier was used once more, activation stage s once more per full round
+// through the stages and once more if s < nk mod stages, a weight slot per k-tile.  Thread 0 parks it during the instruction, and it becomes
+// the current one behind the barrier that ends it: warps that have no part in the products may read the current one as late as that.
+static_assert(kTcXHalfStages <= 10 && kTcWSlots == 8, "bits of tile_state");
+__device__ __forceinline__ void tc_park_state(Ctrl* c, uint32_t state, int nk, uint32_t xstages) {
     const uint32_t full = (uint32_t)nk / xstages, rem = (uint32_t)nk - full * xstages;
-    c->x_par = (uint16_t)(xpar0 ^ ((full & 1u) ? (1u << xstages) - 1u : 0u) ^ ((1u << rem) - 1u));
+    const uint32_t x = (full & 1u ? (1u << xstages) - 1u : 0u) ^ ((1u << rem) - 1u);
+    c->tile_next = (uint16_t)(((state ^ x ^ 1u << 10) & 0x7ffu) | ((state >> 11) + (uint32_t)nk & 15u) << 11);
+}
+__device__ __forceinline__ void tc_next_state(Ctrl* c) {
+    if (threadIdx.x) return;
+    c->tile_state = c->tile_next;
     c->x_left[0] = c->x_left[1] = 0xff;
-    const uint32_t pos = ws0 + (uint32_t)nk;               // one weight slot per k-tile
-    c->w_slot = (uint8_t)(pos % kTcWSlots);
-    c->w_phase = (uint8_t)((wph0 ^ (pos / kTcWSlots)) & 1u);
 }
 
 // Epilogue, second half.  The accumulator tile has been copied to shared memory (fp32, row pitch
@@ -332,7 +332,7 @@ static __device__ __noinline__ void wait_x_landed(Ctrl* c) {
         const int left = c->x_left[lane], next = left & 15, stages = left & 32 ? kTcXHalfStages : kTcXStages;
         if (left == 0xff) continue;
         for (int s = lane; s < stages; s += 2)
-            wait_landed(&c->x_full[s], 1, (((uint32_t)c->x_par >> s) ^ ((uint32_t)left >> 4) ^ (s < next ? 1u : 0u)) & 1u);
+            wait_landed(&c->x_full[s], 1, (((uint32_t)c->tile_state >> s) ^ ((uint32_t)left >> 4) ^ (s < next ? 1u : 0u)) & 1u);
     }
 }
 
@@ -358,7 +358,8 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
     // ends (the kernel frees it on every path); the permit to allocate is never relinquished.
     // (the test is on a word that only changes behind a barrier, so every thread takes the same branch -- not on the
     // address itself, which the allocation writes while the other warps are still arriving at the test)
-    const uint32_t uses = *(volatile uint32_t*)&c->acc_uses;
+    const uint32_t state = *(volatile uint16_t*)&c->tile_state;
+    if (t == 0) tc_park_state(c, state, nk, xstages);
     if (*(volatile uint8_t*)&c->tmem_ready == 0) {            // (the attention op may have allocated it already)
         if (warp == 0) {
             __syncwarp();          // (.sync.aligned: the whole warp, converged)
@@ -371,11 +372,10 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
         if (t == 0) c->tmem_ready = 1;                          // (read again only behind the barrier that ends this instruction)
     }
     const uint32_t tmem = *(volatile uint32_t*)&c->tmem_base;
-    const uint32_t apar = uses & 1u;
+    const uint32_t apar = state >> 10 & 1u;
 
     phase_mark(p, c, 0);
-    const uint32_t xpar0 = c->x_par;            // parities at the instruction's start (written behind the previous one's last barrier)
-    const uint32_t ws0 = c->w_slot, wph0 = c->w_phase;
+    const uint32_t xpar0 = state & 0x3ffu, ws0 = state >> 11 & 7u, wph0 = state >> 14;
     if (warp == 2 && lane < 2) {
         // ---- activation tiles: {64 K-elements, 128 rows} at (kbeg + 64 kt, m0) ----
         // earlier instructions wrote the work area through the generic proxy (all of that is behind
@@ -503,9 +503,8 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
         }
     }
     tc_fence_before();
-    // (no barrier: the one that publishes the instruction tells every thread of a wait that gave up, Ctrl::abort.  Thread 0 has seen the
-    // accumulator complete, so every tile has landed; else x_par and x_left stay as they are, for wait_x_landed)
-    if (t == 0 && ok) tc_finish_state(c, uses, xpar0, ws0, wph0, nk, xstages);
+    // (no barrier: the one that publishes the instruction tells every thread of a wait that gave up, Ctrl::abort; the state and x_left then
+    // stay as they are, for wait_x_landed)
     return 0;
 }
 

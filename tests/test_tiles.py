@@ -117,6 +117,29 @@ def test_rotated_heads_at_tile_edges(cuda, B, S, H, KVH, D, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,kw", [(1024, 4096, 64, {"res": F32}), (1024, 4160, 64, {"act": "gelu_tanh"}), (2000, 3080, 128, {"res": BF, "act": "silu"}),
+                                      (64, 40960, 64, {"res": BF})])
+def test_direct_epilogues_one_behind_the_other(cuda, monkeypatch, M, N, K, kw):
+    """Several 128 x 128 tiles per CTA whose epilogues have no barrier of their own, of one and two k-tiles: the state of the next one changes
+    while warps without a part in the products may still be at this one's start.  Many launches, the same bits."""
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 128, 128))
+    g = mc.Graph()
+    t = {"x": rnd((M, K), 1.0, 1), "w": rnd((N, K), K ** -0.5, 2)}
+    if kw.get("res"):
+        t["r"] = rnd((M, N), 1.0, 3).to(kw["res"])
+    g.output(g.linear(g.input("x", (M, K)), g.param("w", (N, K)), act=kw.get("act"), residual=g.input("r", (M, N), kw["res"]) if kw.get("res") else None))
+    dev = {n: u.to(cuda) for n, u in t.items()}
+    prog = mc.compile(g)
+    assert -(-M // 128) * -(-N // 128) > 148 and [o.kind for o in prog.g.ops] == ["Linear"]
+    got = prog(**dev).clone()
+    assert prog.tcgen05_ops == 1 and rel_l2(got, evaluate(g, dev, cuda)[0][0]) < ONE_ROUNDING
+    for _ in range(200):
+        y = prog(**dev)
+    assert torch.equal(y, got)
+    prog.check()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("extra", [8, 40, 72])
 @pytest.mark.parametrize("B,S,H,KVH,D,K", [(1, 100, 2, 1, 64, 64), (3, 50, 1, 1, 64, 128), (1, 100, 2, 1, 128, 64), (2, 129, 1, 1, 128, 192), (1, 9, 3, 1, 64, 64)])
 def test_columns_behind_rotated_heads(cuda, B, S, H, KVH, D, K, extra):
