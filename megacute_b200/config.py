@@ -38,6 +38,7 @@ FINALIZE_MIN_ROWS, FINALIZE_MIN_INSTS = 4, 96     # SplitFinalize: shorter tiles
 # Both kinds of streaming op aim at one instruction per SM: what an instruction costs whatever its size
 # (dependency wait, arrival, first L2 round trip, ~3 us) is as long as streaming 100 KB
 NORM_ROWS, NORM_MAX_ROWS = COMPUTE_WARPS, 64
+FEW_NORM_ROWS = 256
 EW_MIN_ROWS, EW_MAX_ROWS = 4, 128
 ROPE_APPEND_ROWS = COMPUTE_WARPS
 ATTN_BQ, ATTN_BK = 256, 64          # queries per prefill attention instruction (two tiles of 128), keys per tile of the mma.sync body

@@ -145,7 +145,7 @@ def fill(d, op: Op, addr, sm_count: int, direct=frozenset()) -> None:
     elif k == "Norm":
         d.kind = C.OP_NORM
         ptrs = [op.x, op.out, op.weight, op.bias, op.scale, op.shift]
-        ints = [op.x.rows, op.x.cols, int(bool(op.rms)), norm_rows(op.x.rows, op.scale is not None, sm_count), dt(op.x), dt(op.out),
+        ints = [op.x.rows, op.x.cols, int(bool(op.rms)), norm_rows(op, sm_count), dt(op.x), dt(op.out),
                 int(op.group or 1), dt(op.scale), dt(op.shift)]
         d.f[0] = float(op.eps)
     elif k == "Attention":

@@ -204,7 +204,7 @@ def tile_op(op: Op, sm_count: int) -> Tiled:
         return Tiled(_args(n, rt, ct), [a for a in acc if a is not None])
     if k == "Norm":
         R = op.x.rows
-        rows = norm_rows(R, op.scale is not None, sm_count)
+        rows = norm_rows(op, sm_count)
         rt = np.arange(_ceil(R, rows))
         n = len(rt)
         acc = [_acc(op.x, READ, rt * rows, (rt + 1) * rows, n=n), _acc(op.weight, READ, n=n), _acc(op.bias, READ, n=n),
@@ -308,14 +308,36 @@ def finalize_rows(rows: int, cols: int) -> int:
     return tr
 
 
-def norm_rows(rows: int, modulated: bool, sm_count: int) -> int:
-    """Rows per norm instruction: a single row spread over the whole CTA when every row has an SM (decode; 64 rows 3 us, as eight
-    instructions 4, but 256 rows in two rounds 7.5) and is not modulated (that body needs three round trips more: DiT of 1 x 64 tokens
-    1956 us, with eight rows per instruction 1911; of 1 x 256 2420 -> 2136),
-    else a multiple of the compute warps that gives each SM about one instruction.  Modulated rows (a DiT block's): 16, 32 or 64, so
-    that an instruction waits for one 256-row tile of the linear before it and its rows share a scale and shift row
-    (56 -> 64 rows at 32 images, 24 -> 32 at 12: 0.4 and 1.6 % of the step)."""
-    if rows <= sm_count and not modulated:
+def norm_streams(op: Op) -> bool:
+    """Has the body for several rows per norm instruction a variant of its own for this op (csrc/op_stream.cuh norm_variant)?  Else it goes over
+    each row twice with one warp."""
+    vectors = _ceil(_ceil(op.x.cols, 8), 32)                 # 8-element vectors of a row per lane
+    modulated = op.scale is not None
+    return (op.bias is None and not (op.weight is not None and modulated) and op.out.buf.dtype != torch.float32
+            and vectors <= (4 if modulated else 8))
+
+
+def norm_rows(op: Op, sm_count: int) -> int:
+    """Rows per norm instruction: a single row spread over the whole CTA, or a multiple of the compute warps, a row per warp, that gives each SM
+    about one instruction.  us per norm in a chain of them, one row / eight rows per instruction:
+
+    * plain rows of up to 2048 columns: one while every row has an SM (64 rows 3 / 4), eight beyond that (200 rows of 1024 4.2 / 3.3, of 2048
+      4.5 / 4.1; an MLP block of 150, 200, 256 rows of 2048 51.3 / 50.0, 50.6 / 49.5, 51.9 / 50.3);
+    * modulated rows of up to 1024 columns: eight, that body needs three round trips less (64 rows of 1024 4.8 / 3.8, 256 rows 8.2 / 3.8; DiT, 12
+      blocks of width 1024: 16 tokens 776 / 739, 64 816 / 797, 256 1038 / 918), unless an instruction's rows have several scale and shift
+      rows, read one after the other (150 rows, 2 per group, 5.3 / 6.7);
+    * what eight rows per instruction have no variant for (norm_streams): one up to FEW_NORM_ROWS rows.  Modulated 1152 columns: 64 rows 4.9 / 8.3, DiT of
+      64 such tokens 847 / 924; 200 rows of 4096 6.0 / 16.0, an MLP block of that width 75.1 / 81.9; 200 rows of 2048 with a bias 4.6 / 9.6,
+      into fp32 4.8 / 8.0.
+
+    Many modulated rows (a DiT block's): 8, 16, 32 or 64, so that an instruction waits for one 256-row tile of the linear before it and its rows
+    share a scale and shift row (56 -> 64 rows at 32 images, 24 -> 32 at 12: 0.4 and 1.6 % of the step)."""
+    rows, modulated = op.x.rows, op.scale is not None
+    if not norm_streams(op) or (modulated and op.group < min(rows, C.NORM_ROWS)):
+        one = rows <= C.FEW_NORM_ROWS
+    else:
+        one = rows <= sm_count and not modulated
+    if one:
         return 1
     per = max(1, min(C.NORM_MAX_ROWS // C.NORM_ROWS, _ceil(_ceil(rows, C.NORM_ROWS), sm_count)))
     if modulated and per > 2:

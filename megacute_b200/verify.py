@@ -144,7 +144,7 @@ def op_grid(op, sm_count: int):
     if k in ("Unary", "Binary", "SwiGLU", "Modulate", "Rope"):
         return (_ceil(op.out.rows, ew_rows(*op.out.shape, sm_count)), _ceil(op.out.cols, C.EW_COLS))
     if k == "Norm":
-        return (_ceil(op.x.rows, norm_rows(op.x.rows, op.scale is not None, sm_count)),)
+        return (_ceil(op.x.rows, norm_rows(op, sm_count)),)
     if k == "Attention":
         return (op.batch, op.heads, _ceil(op.seq_q, C.ATTN_BQ))
     if k == "RopeAppend":

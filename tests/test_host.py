@@ -422,6 +422,32 @@ def test_rows_per_streaming_instruction_follow_the_sm_count(sms):
         assert sms // 2 < b - a <= sms and -(-2048 // d.i[field]) == b - a
 
 
+NORMS = [  # rows, columns, kind, rows per modulation group, output type -> one row per instruction?
+    (148, 2048, "rms", 0, None, True), (149, 2048, "rms", 0, None, False), (256, 2048, "rms", 0, None, False), (256, 2056, "rms", 0, None, True),
+    (200, 4096, "rms", 0, None, True), (257, 4096, "rms", 0, None, False), (200, 1024, "bias", 0, None, True), (200, 1024, "rms", 0, torch.float32, True),
+    (1, 1024, "mod", 1, None, False), (64, 1024, "mod", 64, None, False), (256, 1024, "mod", 256, None, False), (64, 1032, "mod", 64, None, True),
+    (256, 1152, "mod", 256, None, True), (512, 1152, "mod", 256, None, False), (150, 1024, "mod", 2, None, True), (12, 264, "mod", 3, None, True),
+    (64, 512, "mod", 8, None, False), (64, 512, "mod", 64, torch.float32, True),
+]
+
+
+@pytest.mark.parametrize("rows,cols,kind,group,dtype,one", NORMS)
+def test_which_norms_take_one_row_per_instruction(rows, cols, kind, group, dtype, one):
+    """Up to 256 rows: eight per instruction only where its body has a variant for the op (the width, a bias, the output's type, one scale and
+    shift row), and, without a modulation, where not every row has an SM."""
+    from megacute_b200.schedule import norm_rows
+    g = mc.Graph()
+    x, out = g.input("x", (rows, cols)), g.temp((rows, cols), dtype=dtype) if dtype else None
+    if kind == "mod":
+        g.output(g.modulate(g.layer_norm(x), g.input("sc", (rows // group, cols)), g.input("sh", (rows // group, cols)), group=group, out=out))
+    elif kind == "bias":
+        g.output(g.layer_norm(x, g.param("w", (1, cols)), g.param("b", (1, cols)), out=out))
+    else:
+        g.output(g.rms_norm(x, g.param("w", (1, cols)), out=out))
+    op, = run_all(g, 148).ops
+    assert op.kind == "Norm" and (norm_rows(op, 148) == 1) is one
+
+
 @pytest.mark.parametrize("B,KVH,L,want", [(18, 8, 1152, False), (19, 8, 128, True), (20, 8, 512, True), (31, 4, 512, False), (31, 4, 2048, True), (14, 8, 2048, True),
                                           (13, 8, 2048, False), (8, 8, 3584, True), (7, 8, 7936, False), (7, 8, 8064, True),
                                           (5, 8, 11264, True), (4, 8, 14080, False), (28, 8, 256, True)])
