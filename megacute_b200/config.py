@@ -52,11 +52,11 @@ DEC_FIXED_US, DEC_MERGE_US, DEC_MERGE_US_PER_SPLIT, DEC_TILE_US = 4.0, 1.0, 0.05
 DEC_SHARED_US = 2.5
 # many-sequence form (one instruction = a sequence's KV split over all kv heads, whole rows through bulk copies),
 # constants measured on B200 at batch 64 (contexts 256 .. 32K, 1 .. 30 splits): used from BULK_MIN_BATCH sequences
-# on and with more (sequence, kv head) pairs than SMs, or from BULK_MIN_BATCH_LONG when the cache is at least BULK_LONG_SEQ rows long or
-# holds BULK_MIN_PIECES rows of a kv head, or from BULK_MIN_BATCH_FEW with BULK_MIN_PIECES_FEW (passes.bulk_eligible);
+# on, from BULK_MIN_BATCH_LONG when the cache is at least BULK_LONG_SEQ rows long, or from BULK_MIN_BATCH_FEW and BULK_MIN_SEQ on when the
+# per-head form has more instructions than SMs (passes.bulk_eligible);
 # us per 16-row tile per KB of cache row (all SMs streaming: the HBM rate); us per instruction = max(fixed, per split x S - 3)
-BULK_MIN_BATCH, BULK_MIN_BATCH_LONG, BULK_LONG_SEQ, BULK_MIN_PIECES = 32, 8, 8192, 28 * 1024 * 8
-BULK_MIN_BATCH_FEW, BULK_MIN_PIECES_FEW = 5, 55 * 1024 * 8
+BULK_MIN_BATCH, BULK_MIN_BATCH_LONG, BULK_LONG_SEQ = 32, 8, 8192
+BULK_MIN_BATCH_FEW, BULK_MIN_SEQ = 5, 2048
 BULK_TILE_US_PER_KB, BULK_FIXED_US, BULK_US_PER_SPLIT = 0.745, 3.0, 0.8
 BULK_TILE_ROWS = 16
 # ... with the same work on every SM (passes.bulk_kv_shares): us per instruction beside its tiles, what the plan has to gain over equal splits,

@@ -142,25 +142,24 @@ def kv_heads_per_instruction(pairs: int, kv_heads: int, max_seq: int, sm_count: 
 def bulk_eligible(op: Op, sm_count: int) -> bool:
     """Can this decode attention run in the many-sequence form (csrc/op_decode_bulk.cuh)?  One warp per
     kv head, head_dim 64, and cache views that are whole rows of their buffers, 128 bytes per kv head,
-    so that consecutive rows are one contiguous run of memory.  And should it?  The per-head form has an instruction per (sequence, kv head):
-    more of them than SMs go one behind the other (8 kv heads, 20 sequences at 500 / 24 at 2000 / 24 at 4000 / 31 at 1000: 1166 -> 1103,
-    1627 -> 1295, 1981 -> 1520, 1319 -> 1241 us a step; 28 at 300 1139 -> 1134).  Fewer: where the cache is long enough for the higher rate of
-    whole rows (10 x 3000 1355 -> 1217, 16 x 4000 1464 -> 1363, 8 x 4000 1284 -> 1234, 14 x 2000 1208 -> 1178; but 16 x 1500 1152 -> 1182, 9 x 2000
-    1123 -> 1159, 16 x 1000 1081 -> 1144; the line is at 28 K rows).  Five to seven sequences hand their values on directly in the per-head form
-    and need 55 K rows (5 x 12000 1502 -> 1404, 6 x 10000 1380 -> 1355, 7 x 8000 1430 -> 1335; but 5 x 6000 1225 -> 1263, 6 x 5000 1210 -> 1234); four stay
-    (4 x 16000 1481 -> 1443, but of different lengths at 15000 1356 -> 1414, 4 x 8000 1212 -> 1271)."""
+    so that consecutive rows are one contiguous run of memory.  And should it?  From 32 sequences on, or 8 with long caches; and where the
+    per-head form has more instructions (sequence, kv head, split) than SMs, so that they run one behind the other: their fixed cost is there at any
+    context, also while the caches are mostly empty.  us a step with full caches and with an eighth of them, per head / whole rows, 8 kv heads: 24
+    sequences x 4096 1971 / 1526 and 1326 / 1099, 24 x 2048 1614 / 1283 and 1282 / 1081, 19 x 2048 1534 / 1245 and 1210 / 1073, 13 x 6144 1793 / 1424 and 1310 /
+    1095, 10 x 3072 1338 / 1211 and 1130 / 1087, 7 x 8064 1578 / 1362 and 1165 / 1162, unsplit 30 x 4096 2009 / 1747 and 1172 / 1154, 31 x 2048 1544 / 1402 and
+    1109 / 1113; 4 kv heads: 20 x 4096 1453 / 1419 and 1170 / 1088.  Unsplit over shorter caches the gain is gone by then (20 x 512 1139 / 1111 and
+    1024 / 1058).  A form that fills the SMs once loses by whole rows as soon as caches are not full: 16 x 4096 1451 / 1378, but at a quarter
+    1071 / 1149, 8 x 4096 1274 / 1232 and 1049 / 1128, 5 x 12032 1496 / 1389 and 1067 / 1164; 4 kv heads, 31 x 2048 full 1221 / 1372."""
     if os.environ.get("MEGACUTE_B200_ATT_BULK") == "0" or getattr(op, "window", 0):      # (no sliding window in that form)
         return False
     whole = all(v.col0 == 0 and v.cols == v.buf.cols for v in (op.k_cache, op.v_cache))
     ok = op.head_dim == 64 and op.kv_heads <= C.COMPUTE_WARPS and whole and op.k_cache.cols == op.kv_heads * 64
     if os.environ.get("MEGACUTE_B200_ATT_BULK") == "1":
         return ok
-    if op.batch >= C.BULK_MIN_BATCH or op.batch * op.kv_heads > sm_count:
+    if op.batch >= C.BULK_MIN_BATCH or (op.batch >= C.BULK_MIN_BATCH_LONG and op.max_seq >= C.BULK_LONG_SEQ):
         return ok
-    pieces = op.batch * op.max_seq * op.kv_heads
-    if op.batch >= C.BULK_MIN_BATCH_LONG:
-        return ok and (op.max_seq >= C.BULK_LONG_SEQ or pieces >= C.BULK_MIN_PIECES)
-    return ok and op.batch >= C.BULK_MIN_BATCH_FEW and pieces >= C.BULK_MIN_PIECES_FEW
+    pairs = op.batch * op.kv_heads
+    return ok and op.batch >= C.BULK_MIN_BATCH_FEW and op.max_seq >= C.BULK_MIN_SEQ and pairs * kv_splits(pairs, op.max_seq, sm_count) > sm_count
 
 
 def bulk_kv_splits(batch: int, kv_heads: int, max_seq: int, sm_count: int) -> int:

@@ -448,9 +448,12 @@ def test_which_norms_take_one_row_per_instruction(rows, cols, kind, group, dtype
     assert op.kind == "Norm" and (norm_rows(op, 148) == 1) is one
 
 
-@pytest.mark.parametrize("B,KVH,L,want", [(18, 8, 1152, False), (19, 8, 128, True), (20, 8, 512, True), (31, 4, 512, False), (31, 4, 2048, True), (14, 8, 2048, True),
-                                          (13, 8, 2048, False), (8, 8, 3584, True), (7, 8, 7936, False), (7, 8, 8064, True),
-                                          (5, 8, 11264, True), (4, 8, 14080, False), (28, 8, 256, True)])
+# (the per-head form's plan: one round of the SMs, several, several unsplit over short and long caches, eight sequences with long ones, 32)
+@pytest.mark.parametrize("B,KVH,L,want", [(18, 8, 1152, False), (16, 8, 4096, False), (8, 8, 4096, False), (14, 8, 2048, False), (5, 8, 11264, False),
+                                          (6, 8, 16000, False), (9, 8, 8064, False), (31, 4, 2048, False), (4, 8, 14080, False),
+                                          (7, 8, 8064, True), (10, 8, 3072, True), (12, 8, 6144, True), (13, 8, 6144, True), (19, 8, 2048, True), (24, 4, 3072, True),
+                                          (19, 8, 128, False), (20, 8, 512, False), (31, 8, 1920, False), (28, 8, 2048, True), (31, 8, 4096, True),
+                                          (8, 8, 8192, True), (16, 8, 8192, True), (7, 8, 5632, False), (7, 8, 5760, True), (32, 8, 128, True), (32, 1, 256, True)])
 def test_which_decode_attention_takes_whole_rows(monkeypatch, B, KVH, L, want):
     for k in ("MEGACUTE_B200_ATT_BULK", "MEGACUTE_B200_KV_SPLITS"):
         monkeypatch.delenv(k, raising=False)
