@@ -59,9 +59,9 @@ BULK_MIN_BATCH, BULK_MIN_BATCH_LONG, BULK_LONG_SEQ = 32, 8, 8192
 BULK_MIN_BATCH_FEW, BULK_MIN_SEQ = 5, 2048
 BULK_TILE_US_PER_KB, BULK_FIXED_US, BULK_US_PER_SPLIT = 0.745, 3.0, 0.8
 BULK_TILE_ROWS = 16
-# ... with the same work on every SM (passes.bulk_kv_shares): us per instruction beside its tiles, what the plan has to gain over equal splits,
-# and the cache rows per sequence above which it is not used (32-bit products on the device, mk_device.cuh kKvShareMax)
-BULK_SHARE_US, BULK_SHARE_GAIN_US, BULK_SHARE_MAX_SEQ = 8.0, -3.0, 1 << 22
+# ... with the same work on every SM (passes.bulk_kv_shares): us per instruction beside its tiles, and the cache rows per sequence above which
+# it is not used (32-bit products on the device, mk_device.cuh kKvShareMax)
+BULK_SHARE_US, BULK_SHARE_MAX_SEQ = 8.0, 1 << 22
 
 # ---- instruction word layout (16 x int32)
 IW = 16

@@ -182,17 +182,26 @@ def bulk_split_cost(batch: int, kv_heads: int, max_seq: int, sm_count: int, s: i
     return -(-(batch * s) // sm_count) * (max(C.BULK_FIXED_US, C.BULK_US_PER_SPLIT * s - 3.0) + tiles * tile_us)
 
 
+def shares_pay(batch: int, splits: int, sm_count: int) -> bool:
+    """Instead of `splits` equal splits of each sequence, the same amount of keys on every SM (bulk_kv_shares)?  Where equal splits run in
+    several rounds of the SMs: then two instructions per SM cost no more than they did, at any context.  us a step, equal splits / the same
+    amount, full caches and an eighth of them: 60 sequences x 4096 rows (7 splits) 2664 / 2315 and 1620 / 1358, 50 x 2048 (5) 1807 / 1624 and 1335 / 1282, 40 x
+    4096 (7) 2072 / 1872 and 1377 / 1312, 42 x 2048 (7) 1665 / 1511 and 1335 / 1256, 58 x 2048 (5) 1830 / 1711 and 1353 / 1300, 96 x 4096 (3) 3186 / 3122 and 1558 / 1492, 200 x
+    1024 (2) 2862 / 2662 and 2011 / 1878; 4 kv heads: 60 x 4096 (7) 2528 / 2219 and 1597 / 1327.  In one round the second instruction of some SMs is a fixed
+    cost that only full caches pay for: 64 x 4224 (2) 2534 / 2462 full, 1831 / 1839 at a half, 1473 / 1532 at a quarter, 1300 / 1389 at an eighth; 44 x 4096 (3)
+    2010 / 1959, but 1211 / 1295; 32 x 8192 of 4 heads 2325 / 2303, but 1230 / 1283.  Unsplit sequences in several rounds gain nothing: 296 x 512 2619 / 2614,
+    300 x 256 2483 / 2402, at an eighth 2141 / 2165."""
+    return splits > 1 and batch * splits > sm_count
+
+
 @functools.lru_cache(maxsize=256)
 def bulk_kv_shares(batch: int, kv_heads: int, max_seq: int, sm_count: int) -> tuple:
     """(modelled time, instructions) of the many-sequence form with the same amount of work on every SM: the sequences' keys, one behind
     the other, are dealt out to the SMs, so that an SM may end one sequence and begin another, with an instruction for each.  Instructions
     are (sequence, split, begin and end in 1024ths of its keys, splits of the sequence), in rounds: an SM's first, its second.
 
-    What bounds the form is the keys an SM can have in flight, so every SM without a split is lost: 2 splits of 64 sequences run on 128 of 148,
-    5 of 50 in rounds of 148 and 102.  Steps of 64 / 60 / 50 / 40 sequences at context 4096 / 4000 / 2000 / 4000: 2505 -> 2427, 2654 -> 2317, 1838 -> 1639,
-    2068 -> 1883 us.  A second instruction on an SM costs more than a first (BULK_SHARE_US 3 / 5 / 7 / 8: 50 sequences at 2000 -- / 1709 / 1677 / 1639),
-    so SMs with two get fewer keys.  Taken when the model puts it at most 3 us behind equal splits (-BULK_SHARE_GAIN_US): 55 x 1500, 1.2 us behind,
-    1686 -> 1534, 64 x 2000, 2.4 behind, 1819 -> 1804; 32 x 4000, 3.8 behind, 1748 -> 1780, 64 x 1024, 5 behind, 1490 -> 1499."""
+    A second instruction on an SM costs more than a first (BULK_SHARE_US 3 / 5 / 7 / 8: 50 sequences at 2000 -- / 1709 / 1677 / 1639 us a step), so SMs
+    with two get fewer keys.  (When: shares_pay.)"""
     whole = -(-max_seq // C.BULK_TILE_ROWS) * C.BULK_TILE_US_PER_KB * kv_heads * 128 / 1024       # us of a sequence
     least = 32                                                                                   # 1024ths
     best = (float("inf"), ())
@@ -247,10 +256,10 @@ def split_kv(g: Graph, sm_count: int) -> Graph:
         if op.kind == "DecodeAttention" and op.splits == 1 and bulk_eligible(op, sm_count):
             s = bulk_kv_splits(op.batch, op.kv_heads, op.max_seq, sm_count)
             op = op.clone(heads_per_inst=op.kv_heads, bulk=True)
-            cost, shares = bulk_kv_shares(op.batch, op.kv_heads, op.max_seq, sm_count)
-            if shares and not os.environ.get("MEGACUTE_B200_KV_SPLITS") and op.max_seq < C.BULK_SHARE_MAX_SEQ and max(x[4] for x in shares) <= C.MAX_KV_SPLITS and \
-                    cost < bulk_split_cost(op.batch, op.kv_heads, op.max_seq, sm_count, s) - C.BULK_SHARE_GAIN_US:
-                op, s = op.clone(shares=shares), max(x[4] for x in shares)
+            if shares_pay(op.batch, s, sm_count) and not os.environ.get("MEGACUTE_B200_KV_SPLITS") and op.max_seq < C.BULK_SHARE_MAX_SEQ:
+                shares = bulk_kv_shares(op.batch, op.kv_heads, op.max_seq, sm_count)[1]
+                if shares and max(x[4] for x in shares) <= C.MAX_KV_SPLITS:
+                    op, s = op.clone(shares=shares), max(x[4] for x in shares)
             if s > 1:
                 G, D = op.heads // op.kv_heads, op.head_dim
                 cols = -(-(G * D + 2 * G) // 4) * 4          # per (kv head, split): O (G x D), running max (G), sum (G)

@@ -8,7 +8,7 @@ import pytest
 import torch
 
 import megacute_b200 as mc
-from megacute_b200 import config as C
+from megacute_b200 import config as C, passes
 from megacute_b200 import workloads as W
 from oracle.graph_oracle import evaluate, rel_l2
 from tests.helpers import TOL, small_decode, to_cpu
@@ -194,7 +194,7 @@ def test_decode_attention_equal_shares(cuda, monkeypatch, B, H, KVH, max_seq, ct
     """The many-sequence form with ranges of keys of unequal length, one or two instructions per SM: contexts that leave many of them empty, that
     end inside a tile, splits of one sequence on several SMs and of several on one."""
     monkeypatch.setenv("MEGACUTE_B200_ATT_BULK", "1")
-    monkeypatch.setattr(C, "BULK_SHARE_GAIN_US", -1e9)
+    monkeypatch.setattr(passes, "shares_pay", lambda *a: True)
     prog = _decode_attention_case(cuda, B, H, KVH, 64, max_seq, ctx, fused)
     att = [o for o in prog.g.ops if o.kind == "DecodeAttention"]
     assert att and all(o.shares and o.splits == max(x[4] for x in o.shares) for o in att)

@@ -482,3 +482,14 @@ def test_equal_shares_of_many_sequences(batch, max_seq):
         for q in range(batch):
             mine = [g[1:] for g in got if g[0] == q]
             assert mine[0][0] == 0 and mine[-1][1] == keys and all(x[1] == y[0] and x[0] <= x[1] for x, y in zip(mine, mine[1:] + [(keys, keys)]))
+
+
+@pytest.mark.parametrize("B,KVH,L,shares", [(64, 8, 4224, False), (44, 8, 4096, False), (26, 8, 4096, False), (32, 4, 8192, False), (128, 8, 2048, False), (296, 8, 512, False),
+                                            (60, 8, 4096, True), (50, 8, 2048, True), (40, 8, 4096, True), (42, 8, 2048, True), (200, 8, 1024, True), (60, 4, 4096, True)])
+def test_which_whole_row_attention_deals_out_its_keys(monkeypatch, B, KVH, L, shares):
+    """Where equal splits need one round of the SMs they stay: a second instruction on some SMs is a cost at every context."""
+    for k in ("MEGACUTE_B200_ATT_BULK", "MEGACUTE_B200_KV_SPLITS"):
+        monkeypatch.delenv(k, raising=False)
+    g, *_ = small_decode(B=B, n=1, E=512, H=8, KVH=KVH, F=512, vocab=512, max_seq=L, ctx=10)
+    op, = [o for o in run_all(g, 148).ops if o.kind == "DecodeAttention"]
+    assert op.bulk and bool(op.shares) == shares and (shares or B * op.splits <= 148 or op.splits == 1)
