@@ -833,9 +833,12 @@ int mk_launch(mk_program* p, void* stream) {
     prm.direct_next = reinterpret_cast<uint4*>(p->direct + (p->direct_turn ? 0 : p->direct_bytes));
     prm.direct_pieces = (int)(p->direct_bytes / 16);
     // Programmatic serialization behind the kernel in front in the stream: the launch is prepared while that one's last blocks run, and its
-    // blocks start when those have ended -- every SM is free then, as before -- instead of when their memory has been flushed as well; the
-    // kernel waits for that itself (griddepcontrol.wait) before it reads anything.  A launch behind another 2 us earlier: MLP
-    // block of one row 25.4 -> 23.5 us, of 64 35.6 -> 33.5, of 256 52.7 -> 50.6.  A captured launch has ordinary edges.
+    // blocks start when those have ended instead of when their memory has been flushed as well.  griddepcontrol.wait alone, in front of
+    // everything the kernel reads, carries the order: it returns when that kernel has ended and its writes are visible.  (A kernel in
+    // front that allows its dependents early, griddepcontrol.launch_dependents, has them resident beside it: this launch's blocks then hold their
+    // SMs' shared memory while they wait, and those without an SM come when it ends.  All are resident together then, as the schedule needs.)
+    // A launch behind another 2 us earlier: MLP block of one row 25.4 -> 23.5 us, of 64 35.6 -> 33.5, of 256 52.7 -> 50.6.  A captured
+    // launch has ordinary edges.
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) {
         (void)cudaGetLastError();

@@ -11,7 +11,7 @@
 // by streaming the weights), 64 rows per tile (warp tile 32 x 32): no MMAs on padding rows and more
 // weight bytes in flight.
 //
-// ptr 0 x, 1 w, 2 out (or ws), 3 bias, 4 residual, 5 gate (out = residual + act(.) * gate[r / i12], 256-row tiles only; or null)
+// ptr 0 x, 1 w, 2 out (or ws), 3 bias, 4 residual, 5 gate (out = residual + act(.) * gate[r / i12]; or null)
 // i 0 M, 1 N (weight rows), 2 K, 3 act, 4 K splits, 5 out dtype, 6 accumulate, 7 residual dtype,
 //   8 swiglu (weight tile = 64 gate rows then 64 up rows; the tile writes 64 output columns),
 //   9 x dtype (DT_BF16 or DT_F16), 10 weight rows per output tile (128, or 256: the n tile argument then

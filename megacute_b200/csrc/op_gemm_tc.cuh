@@ -10,7 +10,7 @@
 // Operands are K-major 128-row x 64-column tiles (16 KB).  The 128 activation rows of the m tile are
 // the MMA's M side, so an accumulator row (a tensor-memory lane) is an activation row and a thread of
 // the epilogue holds whole output rows: swiglu (gate columns 0..63, up columns 64..127 of the weight
-// tile) pairs values of one thread.  Rows beyond M are zero-filled by the copy and never stored.
+// tile) pairs values of one thread.  Rows beyond M are zeros or, behind the copy's box, whatever the stage held, and never stored.
 //   weights      producer warp -> eight single-tile slots in the ring's memory, across instruction
 //                boundaries: they depend on nothing in the launch, so the next instruction's first
 //                128 KB are already on their way while this one waits for its dependencies
