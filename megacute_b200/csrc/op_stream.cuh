@@ -437,6 +437,84 @@ __device__ __forceinline__ void norm_stream(const mk_op_desc* op, int r0, int ro
     }
 }
 
+// Modulated rows whose scale and shift rows change with every row or every two or three (up to 1024 columns): each warp requests its row's own in front
+// of the sums, into registers.  In shared memory, as above, they change up to eight times in eight rows, with two barriers and a round
+// trip to L2 each.  us per norm, above / here: 9600 rows of 1024 with a scale row each 101 / 26, of 512 89 / 24, 1200 rows of 1024 14 / 6, 300 rows
+// 4.1 / 3.4.  (With four rows per scale row the form above is faster up to 600 rows, 300 of 1024 3.2 / 3.4, and 256 bytes per thread are saved
+// around this one.)
+template <int XDT, int ODT>
+__device__ __forceinline__ void norm_own(const mk_op_desc* op, int r0, int rows) {
+    constexpr int NPER = 4, kPlanes = XDT == DT_F32 ? 2 : 1, kRow = NPER * kPlanes * 512, kDepth = (kWorkBytes - kTcXOff) / kComputeWarps / kRow;
+    const int Cc = op->i[1], rms = op->i[2], group = max(1, op->i[6]);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = Cc >> 3;
+    const float inv = 1.0f / (float)Cc, eps = op->f[0];
+    const long long ldx = op->ld[0], ldo = op->ld[1];
+    auto column = [&](int u) { return min(lane + u * 32, nvec - 1) * 8; };
+    uint8_t* buf = smem_map().work + kTcXOff + warp * (kDepth * kRow) + lane * 16;
+    auto request = [&](int rr, int slot) {
+        if (rr < rows) {
+            const uint8_t* from = reinterpret_cast<const uint8_t*>(op->ptr[0]) + (r0 + rr) * ldx * (kPlanes * 2);
+#pragma unroll
+            for (int u = 0; u < NPER; ++u)
+#pragma unroll
+                for (int k = 0; k < kPlanes; ++k) cp_async16(buf + slot * kRow + (u * kPlanes + k) * 512, from + column(u) * (kPlanes * 2) + k * 16, true);
+        }
+        cp_async_commit();
+    };
+    int next = warp, slot = 0;
+#pragma unroll 1
+    for (int d = 0; d < kDepth; ++d, next += kComputeWarps) request(next, d);
+#pragma unroll 1
+    for (int rr = warp; rr < rows; rr += kComputeWarps, next += kComputeWarps) {
+        const long long grp = (r0 + rr) / group;
+        Raw8 sc[NPER], sh[NPER];
+#pragma unroll
+        for (int u = 0; u < NPER; ++u) {
+            sc[u] = load8_raw(reinterpret_cast<const void*>(op->ptr[4]), grp * op->ld[4] + column(u), op->i[7]);
+            sh[u] = load8_raw(reinterpret_cast<const void*>(op->ptr[5]), grp * op->ld[5] + column(u), op->i[8]);
+        }
+        cp_async_wait<kDepth - 1>();
+        const uint8_t* at = buf + slot * kRow;
+        auto row = [&](int u, float* f) {
+            Vec8<XDT> x;
+            x.raw(*reinterpret_cast<const uint4*>(at + u * kPlanes * 512), *reinterpret_cast<const uint4*>(at + u * kPlanes * 512 + (kPlanes - 1) * 512));
+            x.get(f);
+        };
+        float s = 0.f, ss = 0.f;
+#pragma unroll
+        for (int u = 0; u < NPER; ++u) {
+            float f[8];
+            row(u, f);
+            float a = 0.f, q = 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) { a += f[e]; q = fmaf(f[e], f[e], q); }
+            const bool in = lane + u * 32 < nvec;
+            s += in ? a : 0.f;
+            ss += in ? q : 0.f;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        }
+        const float mean = rms ? 0.f : s * inv;
+        const float rstd = rsqrt_approx(ss * inv - mean * mean + eps);
+        const long long out = (r0 + rr) * ldo;
+#pragma unroll
+        for (int u = 0; u < NPER; ++u) {
+            float f[8], g[8], h[8];
+            row(u, f);
+            unpack8_raw(sc[u], op->i[7], g);
+            unpack8_raw(sh[u], op->i[8], h);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) f[e] = fmaf((f[e] - mean) * rstd, 1.0f + g[e], h[e]);
+            if (lane + u * 32 < nvec) put8<ODT>(reinterpret_cast<void*>(op->ptr[1]), out + (lane + u * 32) * 8, f);
+        }
+        request(next, slot);
+        if (++slot == kDepth) slot = 0;
+    }
+}
+
 // Any other row (longer than 2048 elements, with a bias, gain and modulation at once, fp32 modulation): two passes over global
 // memory, two vectors requested at a time.
 __device__ __forceinline__ void norm_two_pass(const mk_op_desc* op, int r0, int rows) {
@@ -492,18 +570,20 @@ __device__ __forceinline__ void norm_two_pass(const mk_op_desc* op, int r0, int 
     }
 }
 
-// Variant of a norm: x dtype (bits 0-1), fp16 output (bit 2), vectors per lane (bit 3: 8, else 4), gain (bit 4), modulation (bit 5)
-constexpr int NORM_ANY = 128;
+// Variant of a norm: x dtype (bits 0-1), fp16 output (bit 2), vectors per lane (bit 3: 8, else 4), gain (bit 4), modulation (bit 5), fewer than
+// four rows per scale and shift row (bit 6)
+constexpr int NORM_OWN = 64, NORM_ANY = 128;
 __device__ __forceinline__ int norm_variant(const mk_op_desc* op) {
     const int nper = ((op->i[1] >> 3) + 31) / 32;
     const bool w = op->ptr[2] != 0, mod = op->ptr[4] != 0;
     if (op->ptr[3] || (w && mod) || op->i[5] == DT_F32 || nper > (mod ? 4 : 8)) return NORM_ANY;
-    return op->i[4] | (op->i[5] == DT_F16 ? 4 : 0) | (nper > 4 ? 8 : 0) | (w ? 16 : 0) | (mod ? 32 : 0);
+    return op->i[4] | (op->i[5] == DT_F16 ? 4 : 0) | (nper > 4 ? 8 : 0) | (w ? 16 : 0) | (mod ? 32 : 0) | (mod && op->i[6] < 4 ? NORM_OWN : 0);
 }
 template <int V>
 __device__ __forceinline__ void op_norm_rows(const mk_op_desc* op, int a0) {
     const int r0 = a0 * op->i[3], rows = min(op->i[3], op->i[0] - r0);
     if constexpr (V == NORM_ANY) norm_two_pass(op, r0, rows);
+    else if constexpr ((V & NORM_OWN) != 0) norm_own<V & 3, (V & 4) ? DT_F16 : DT_BF16>(op, r0, rows);
     else norm_stream<(V & 8) ? 8 : 4, V & 3, (V & 4) ? DT_F16 : DT_BF16, (V & 16) != 0, (V & 32) != 0>(op, r0, rows);
 }
 

@@ -388,6 +388,7 @@ def test_norm_many_rows(cuda, rows, cols, dtype, rms, group):
 @pytest.mark.parametrize("rows,cols,dtype,group,mod", [
     (300, 72, F32, 3, F32), (1200, 1000, BF, 8, BF), (1208, 1024, F32, 604, F32), (2400, 264, BF, 1, BF), (261, 2048, F32, 0, BF), (2403, 1032, BF, 0, BF),
     (9602, 520, F32, 0, BF), (149, 2048, F32, 0, BF), (150, 1000, BF, 0, BF), (64, 1024, F32, 32, BF), (12, 264, BF, 3, BF), (3, 1024, BF, 1, F32),
+    (1500, 1024, F32, 3, F32), (9602, 520, BF, 2, BF), (2403, 1024, BF, 1, F32), (301, 8, F32, 1, BF), (1200, 72, BF, 4, BF),
     (64, 1152, F32, 64, BF), (150, 1032, BF, 2, F32), (256, 1024, F32, 256, BF), (200, 4096, BF, 0, BF), (256, 2056, F32, 0, BF),
 ])
 def test_norm_shares_gain_and_modulation(cuda, rows, cols, dtype, group, mod):
