@@ -48,6 +48,7 @@ __device__ int mk_run_norm(const Params& p, const mk_op_desc* op, int idx, int s
 #define MK_N(V) case (V): return norm_run<(V)>(p, idx, slot)
 #define MK_NT(V) MK_N((V) | DT_BF16); MK_N((V) | DT_F16); MK_N((V) | DT_F32); MK_N((V) | 4 | DT_BF16); MK_N((V) | 4 | DT_F16); MK_N((V) | 4 | DT_F32)
         MK_NT(0); MK_NT(16); MK_NT(32); MK_NT(32 | NORM_OWN); MK_NT(8); MK_NT(8 | 16);
+        MK_NT(NORM_KEEP); MK_NT(NORM_KEEP | 16); MK_NT(NORM_KEEP | 8); MK_NT(NORM_KEEP | 8 | 16);
 #undef MK_NT
 #undef MK_N
         default: return norm_run<NORM_ANY>(p, idx, slot);

@@ -437,6 +437,90 @@ __device__ __forceinline__ void norm_stream(const mk_op_desc* op, int r0, int ro
     }
 }
 
+// Plain rows, several per warp (with a gain more than four, without more than one): the row stays in registers, so that it is read from shared memory
+// once and its place is requested again before the sums; 200 bytes per thread saved around it are little beside as many rows.  us per norm in a chain
+// of them, norm_stream / here: 16384 rows of 2048 with a gain 28.0 / 23.7, of 1024 16.3 / 14.6, 9600 of 1152 16.5 / 14.7; without one 16384 of 2048
+// 23.8 / 20.8, of 1024 14.7 / 12.5, 1200 of 1024 3.8 / 3.7.  Prompts and MLP blocks the same (4 x 4096 tokens 9209 and 9246 us, runs differ by 1 %).  With a
+// gain and up to four rows per warp norm_stream is ahead where other ops lie between (MLP block of 2400 rows 161, 165 in this form).
+template <int NPER, int XDT, int ODT, bool HW>
+__device__ __forceinline__ void norm_kept_rows(const mk_op_desc* op, int r0, int rows) {
+    constexpr int kGain = HW ? NPER * 512 : 0, kPlanes = XDT == DT_F32 ? 2 : 1, kRow = NPER * kPlanes * 512;
+    constexpr int kDepth = (kWorkBytes - kTcXOff - kGain) / kComputeWarps / kRow, kGainOff = kTcXOff + kComputeWarps * kDepth * kRow;
+    static_assert(kDepth >= 1 && kGainOff + kGain <= kWorkBytes, "norm rows exceed the work area");
+    const int Cc = op->i[1], rms = op->i[2];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = Cc >> 3;
+    const float inv = 1.0f / (float)Cc, eps = op->f[0];
+    const long long ldx = op->ld[0], ldo = op->ld[1];
+    const uint8_t* X = reinterpret_cast<const uint8_t*>(op->ptr[0]) + r0 * ldx * (kPlanes * 2);
+    uint16_t* O = reinterpret_cast<uint16_t*>(op->ptr[1]) + r0 * ldo;
+    auto column = [&](int u) { return min(lane + u * 32, nvec - 1) * 8; };
+    uint8_t* buf = smem_map().work + kTcXOff + warp * (kDepth * kRow) + lane * 16;
+    auto request = [&](int rr, int slot) {
+        if (rr < rows) {
+#pragma unroll
+            for (int u = 0; u < NPER; ++u)
+#pragma unroll
+                for (int k = 0; k < kPlanes; ++k)
+                    cp_async16(buf + slot * kRow + (u * kPlanes + k) * 512, X + (rr * ldx + column(u)) * (kPlanes * 2) + k * 16, true);
+        }
+        cp_async_commit();
+    };
+    uint8_t* gain = smem_map().work + kGainOff;
+    if (HW)
+        for (int v = threadIdx.x; v < NPER * 32; v += kComputeThreads)
+            cp_async16(gain + v * 16, reinterpret_cast<const uint8_t*>(op->ptr[2]) + min(v, nvec - 1) * 16, true);
+#pragma unroll
+    for (int d = 0; d < kDepth; ++d) request(warp + d * kComputeWarps, d);
+    if (HW) {
+        cp_async_wait<kDepth - 1>();
+        compute_sync();
+    }
+    int slot = 0;
+#pragma unroll 1
+    for (int rr = warp; rr < rows; rr += kComputeWarps) {
+        cp_async_wait<kDepth - 1>();
+        Vec8<XDT> x[NPER];
+#pragma unroll
+        for (int u = 0; u < NPER; ++u) {
+            const uint4* at = reinterpret_cast<const uint4*>(buf + slot * kRow + u * kPlanes * 512);
+            x[u].raw(at[0], at[kPlanes == 2 ? 32 : 0]);
+        }
+        request(rr + kDepth * kComputeWarps, slot);
+        if (++slot == kDepth) slot = 0;
+        float s = 0.f, ss = 0.f;
+#pragma unroll
+        for (int u = 0; u < NPER; ++u) {
+            float f[8];
+            x[u].get(f);
+            float a = 0.f, q = 0.f;
+#pragma unroll
+            for (int e = 0; e < 8; ++e) { a += f[e]; q = fmaf(f[e], f[e], q); }
+            const bool in = lane + u * 32 < nvec;
+            s += in ? a : 0.f;
+            ss += in ? q : 0.f;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            s += __shfl_xor_sync(0xffffffffu, s, o);
+            ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        }
+        const float mean = rms ? 0.f : s * inv;
+        const float rstd = rsqrt_approx(ss * inv - mean * mean + eps);
+#pragma unroll
+        for (int u = 0; u < NPER; ++u) {
+            float f[8], g[8];
+            x[u].get(f);
+            if (HW) unpack8(reinterpret_cast<const uint4*>(gain)[u * 32 + lane], g);
+#pragma unroll
+            for (int e = 0; e < 8; ++e) {
+                f[e] = (f[e] - mean) * rstd;
+                if (HW) f[e] *= g[e];
+            }
+            if (lane + u * 32 < nvec) put8<ODT>(O, rr * ldo + (lane + u * 32) * 8, f);
+        }
+    }
+}
+
 // Modulated rows whose scale and shift rows change with every row or every two or three (up to 1024 columns): each warp requests its row's own in front
 // of the sums, into registers.  In shared memory, as above, they change up to eight times in eight rows, with two barriers and a round
 // trip to L2 each.  us per norm, above / here: 9600 rows of 1024 with a scale row each 101 / 26, of 512 89 / 24, 1200 rows of 1024 14 / 6, 300 rows
@@ -571,18 +655,19 @@ __device__ __forceinline__ void norm_two_pass(const mk_op_desc* op, int r0, int 
 }
 
 // Variant of a norm: x dtype (bits 0-1), fp16 output (bit 2), vectors per lane (bit 3: 8, else 4), gain (bit 4), modulation (bit 5), fewer than
-// four rows per scale and shift row (bit 6)
-constexpr int NORM_OWN = 64, NORM_ANY = 128;
+// four rows per scale and shift row (bit 6), rows kept in registers (bit 8)
+constexpr int NORM_OWN = 64, NORM_KEEP = 256, NORM_ANY = 128;
 __device__ __forceinline__ int norm_variant(const mk_op_desc* op) {
     const int nper = ((op->i[1] >> 3) + 31) / 32;
     const bool w = op->ptr[2] != 0, mod = op->ptr[4] != 0;
     if (op->ptr[3] || (w && mod) || op->i[5] == DT_F32 || nper > (mod ? 4 : 8)) return NORM_ANY;
-    return op->i[4] | (op->i[5] == DT_F16 ? 4 : 0) | (nper > 4 ? 8 : 0) | (w ? 16 : 0) | (mod ? 32 : 0) | (mod && op->i[6] < 4 ? NORM_OWN : 0);
+    return op->i[4] | (op->i[5] == DT_F16 ? 4 : 0) | (nper > 4 ? 8 : 0) | (w ? 16 : 0) | (mod ? 32 : 0) | (mod ? (op->i[6] < 4 ? NORM_OWN : 0) : op->i[3] > (w ? 4 : 1) * kComputeWarps ? NORM_KEEP : 0);
 }
 template <int V>
 __device__ __forceinline__ void op_norm_rows(const mk_op_desc* op, int a0) {
     const int r0 = a0 * op->i[3], rows = min(op->i[3], op->i[0] - r0);
     if constexpr (V == NORM_ANY) norm_two_pass(op, r0, rows);
+    else if constexpr ((V & NORM_KEEP) != 0) norm_kept_rows<(V & 8) ? 8 : 4, V & 3, (V & 4) ? DT_F16 : DT_BF16, (V & 16) != 0>(op, r0, rows);
     else if constexpr ((V & NORM_OWN) != 0) norm_own<V & 3, (V & 4) ? DT_F16 : DT_BF16>(op, r0, rows);
     else norm_stream<(V & 8) ? 8 : 4, V & 3, (V & 4) ? DT_F16 : DT_BF16, (V & 16) != 0, (V & 32) != 0>(op, r0, rows);
 }

@@ -365,7 +365,7 @@ def test_prefill_attention_scale_not_positive(cuda, D, scale):
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows,cols,dtype,rms,group", [
     (257, 2048, BF, True, 0), (1190, 1024, BF, True, 0), (2390, 1000, BF, False, 0), (3001, 2048, F32, True, 0), (2400, 1024, BF, False, 40),
-    (9600, 256, BF, True, 0), (2500, 8, F32, True, 0),
+    (9600, 256, BF, True, 0), (2500, 8, F32, True, 0), (1201, 2040, BF, False, 0), (1999, 1500, F32, False, 0),
 ])
 def test_norm_many_rows(cuda, rows, cols, dtype, rms, group):
     """8, 16, 24 and 64 rows per instruction, a last instruction with fewer, modulation rows that change inside one."""
@@ -388,7 +388,7 @@ def test_norm_many_rows(cuda, rows, cols, dtype, rms, group):
 @pytest.mark.parametrize("rows,cols,dtype,group,mod", [
     (300, 72, F32, 3, F32), (1200, 1000, BF, 8, BF), (1208, 1024, F32, 604, F32), (2400, 264, BF, 1, BF), (261, 2048, F32, 0, BF), (2403, 1032, BF, 0, BF),
     (9602, 520, F32, 0, BF), (149, 2048, F32, 0, BF), (150, 1000, BF, 0, BF), (64, 1024, F32, 32, BF), (12, 264, BF, 3, BF), (3, 1024, BF, 1, F32),
-    (1500, 1024, F32, 3, F32), (9602, 520, BF, 2, BF), (2403, 1024, BF, 1, F32), (301, 8, F32, 1, BF), (1200, 72, BF, 4, BF),
+    (5001, 2048, BF, 0, BF), (5500, 1032, F32, 0, BF), (1500, 1024, F32, 3, F32), (9602, 520, BF, 2, BF), (2403, 1024, BF, 1, F32), (301, 8, F32, 1, BF), (1200, 72, BF, 4, BF),
     (64, 1152, F32, 64, BF), (150, 1032, BF, 2, F32), (256, 1024, F32, 256, BF), (200, 4096, BF, 0, BF), (256, 2056, F32, 0, BF),
 ])
 def test_norm_shares_gain_and_modulation(cuda, rows, cols, dtype, group, mod):
