@@ -87,7 +87,8 @@ def test_activation_copies_of_the_rows_there_are(cuda, M):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K", [(9, 128, 64), (32, 136, 64), (33, 128, 128), (63, 264, 192), (97, 128, 64), (128, 8, 128)])
-@pytest.mark.parametrize("res,act", [(BF, None), (F32, None), (BF, "silu"), (None, "gelu_tanh"), (None, None)])
+@pytest.mark.parametrize("res,act", [(BF, None), (F32, None), (BF, "silu"), (None, "gelu_tanh"), (None, None), (F32, "gelu_tanh"), (F32, "silu"), (None, "silu"),
+                                     (BF, "relu"), (None, "relu")])
 def test_row_groups_of_an_epilogue(cuda, M, N, K, res, act):
     """Rows that end anywhere in a warp's groups of four, one accumulator (one k-tile) or two, columns that end inside a tile."""
     g = mc.Graph()
@@ -96,6 +97,20 @@ def test_row_groups_of_an_epilogue(cuda, M, N, K, res, act):
     g.output(y)
     outs, ref, _, _, prog = run_both(g, t if res else {k: v for k, v in t.items() if k != "r"}, cuda)
     assert prog.tcgen05_ops == 1 and rel_l2(outs[0], ref[0]) < ONE_ROUNDING
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("M", [9, 31, 32, 33, 100])
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh", "relu"])
+def test_activation_and_a_private_residual(cuda, M, act):
+    """An activation in front of a 16-bit private residual, on both sides of the number of rows that go through shared memory."""
+    g = mc.Graph()
+    y = g.linear(g.input("x", (M, 128)), g.param("v", (192, 128)))
+    y = g.linear(y, g.param("w", (192, 192)), act=act, residual=y) if M == 100 else g.linear(y, g.param("w", (192, 192)), act=act, residual=y, bias=g.param("b", (1, 192)))
+    g.output(g.linear(y, g.param("u", (64, 192))))
+    t = {"x": rnd((M, 128), 1.0, 1), "v": rnd((192, 128), 0.1, 2), "w": rnd((192, 192), 0.1, 3), "u": rnd((64, 192), 0.1, 4), "b": rnd((1, 192), 0.5, 5)}
+    outs, ref, *_ = run_both(g, t if M != 100 else {k: v for k, v in t.items() if k != "b"}, cuda)
+    assert rel_l2(outs[0], ref[0]) < 1.6 * 2.0 ** -9          # (rounding of the output to bf16 2^-9, of two activations to fp16 2^-12 each, tanh.approx 2^-11)
 
 
 @pytest.mark.gpu
@@ -365,7 +380,7 @@ def test_prefill_attention_scale_not_positive(cuda, D, scale):
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows,cols,dtype,rms,group", [
     (257, 2048, BF, True, 0), (1190, 1024, BF, True, 0), (2390, 1000, BF, False, 0), (3001, 2048, F32, True, 0), (2400, 1024, BF, False, 40),
-    (9600, 256, BF, True, 0), (2500, 8, F32, True, 0), (1201, 2040, BF, False, 0), (1999, 1500, F32, False, 0),
+    (9600, 256, BF, True, 0), (2500, 8, F32, True, 0), (1201, 2040, BF, False, 0), (1999, 1504, F32, False, 0),
 ])
 def test_norm_many_rows(cuda, rows, cols, dtype, rms, group):
     """8, 16, 24 and 64 rows per instruction, a last instruction with fewer, modulation rows that change inside one."""
