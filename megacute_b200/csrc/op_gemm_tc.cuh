@@ -24,7 +24,8 @@
 //                returns the activation stage and the ring slot when the MMAs that read them are done
 //   epilogue     all 8 compute warps; warp w reads lanes 32 (w & 3) .. +31, column half w >> 2.  Split-K partials, swiglu, accumulating
 //                and plain tiles: tensor memory -> shared memory, then row-contiguous global stores / reductions from there.
-//                Tiles with a residual, an activation or rotated heads: straight from tensor memory, a row per thread
+//                Tiles with a residual, an activation (silu and few rows: as before) or rotated heads: straight from tensor
+//                memory, a row per thread
 // Every wait is bounded (wait_barrier); tensor memory is allocated by the first such instruction of a
 // CTA and freed by the kernel before it exits, on every path.
 #pragma once
@@ -128,6 +129,36 @@ static __device__ __noinline__ void tc_store_rows(const mk_op_desc* op, const fl
         else *reinterpret_cast<uint2*>(O + row * ldo * 2) = make_uint2(pack2(f[0], f[1]), pack2(f[2], f[3]));
     }
 }
+// ... of up to 32 rows with an activation from the special function units, types and activation at run time.  Straight from tensor memory two of the
+// eight warps would have all of it.  9 rows of 256 columns, us per linear, from there / here: silu 7.6 / 6.9, with a residual 8.4 / 7.1, gelu
+// with a residual 8.0 / 7.2 (gelu alone 6.6 from there, relu 6.6).
+static __device__ __noinline__ void tc_write_few(const mk_op_desc* op, const float* stage, int rows, int col0, int n_out) {
+    const int warp = threadIdx.x >> 5, c4 = (threadIdx.x & 31) * 4, col = col0 + c4, act = op->i[3], odt = op->i[5], rdt = op->i[7];
+    if (col >= n_out) return;
+    uint8_t* O = reinterpret_cast<uint8_t*>(op->ptr[2]);
+    const uint8_t* R = reinterpret_cast<const uint8_t*>(op->ptr[4]);
+    float4 r[4];                                             // (all of the warp's rows of the residual: one round trip to L2)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int row = warp + j * kComputeWarps;
+        r[j] = R && row < rows ? load4_any(R, (long long)row * op->ld[4] + col, rdt) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    const float4 b = op->ptr[3] ? load4_any(reinterpret_cast<const uint8_t*>(op->ptr[3]), col, DT_BF16) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const int row = warp + j * kComputeWarps;
+        if (row >= rows) break;
+        const float4 q = *reinterpret_cast<const float4*>(stage + row * kTcStagePitch + c4);
+        float f[4] = {q.x + b.x, q.y + b.y, q.z + b.z, q.w + b.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) f[e] = apply_act(act, f[e]);
+        f[0] += r[j].x; f[1] += r[j].y; f[2] += r[j].z; f[3] += r[j].w;
+        const long long eo = (long long)row * op->ld[2] + col;
+        if (odt == DT_F32) *reinterpret_cast<float4*>(O + eo * 4) = make_float4(f[0], f[1], f[2], f[3]);
+        else *reinterpret_cast<uint2*>(O + eo * 2) = make_uint2(pack2t(odt, f[0], f[1]), pack2t(odt, f[2], f[3]));
+    }
+}
+
 // Epilogues straight from tensor memory, a row per thread and 16 columns at a time, for tiles that read another operand beside the
 // accumulator or compute something from it: the row's whole piece of a residual and gate (rotated heads: the tables of the first 16
 // columns) is requested before the accumulator is complete.  (A loop over few instructions: sixteen rows of a warp side by side, through the
@@ -142,8 +173,26 @@ __device__ __forceinline__ bool tc_direct_wait(const Params& p, Ctrl* c, uint32_
     __syncwarp();                                            // (the tensor-memory loads are .sync.aligned: whole warp, converged)
     return ok != 0;
 }
-// an activation chosen at run time on 16 values, four at a time (rotated: register indices stay constant)
+// an activation chosen at run time on 16 values.  The common ones side by side, the others four at a time (rotated: register indices stay constant).
+// 64 rows of 256 columns, us per linear, the writer through shared memory that had this before / this: silu 10.5 / 7.8, gelu 10.6 / 7.2, silu and
+// a residual 11.4 / 9.1; all of them rotated, silu took 0.6 more than side by side.
 __device__ __forceinline__ void act16(int act, float* v) {
+    if (act == ACT_SILU) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = apply_act(ACT_SILU, v[e]);
+        return;
+    }
+    if (act == ACT_GELU) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = apply_act(ACT_GELU, v[e]);
+        return;
+    }
+    if (act == ACT_RELU) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) v[e] = apply_act(ACT_RELU, v[e]);
+        return;
+    }
+    if (act == ACT_NONE) return;
 #pragma unroll 1
     for (int j = 0; j < 16; j += 4) {
         float t[4];
@@ -445,7 +494,8 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
     // ---- epilogue: warp w owns lanes 32 (w & 3) .. +31 (activation rows) and column half w >> 2 ----
     const uint32_t two = nk > 1 ? 128u : 0u;                               // columns to the second issuing thread's accumulator, if it has a part
     int ok = 1;
-    if (!op->i[6] && !swi && (op->ptr[6] || op->ptr[4] || op->i[3] != ACT_NONE)) {
+    const bool few = M <= 32 && !op->i[6] && !swi && !op->ptr[5] && (op->i[3] == ACT_SILU || (op->i[3] == ACT_GELU && op->ptr[4]));      // tc_write_few
+    if (!op->i[6] && !swi && !few && (op->ptr[6] || op->ptr[4] || op->i[3] != ACT_NONE)) {
         ok = tc_direct(p, c, op, two, apar, m0, n0, seq);
     } else {
         if (lane == 0) ok = wait_barrier(p, c, &c->acc_full, apar, seq, WHERE_COMBINE) ? 1 : 0;
@@ -497,6 +547,7 @@ __device__ __forceinline__ int op_gemm_tc(const Params& p, Ctrl* c, uint8_t* rin
                 if (op->i[5] == DT_F32) tc_reduce_rows(op, stage, m0, rows, n0, N);
                 else tc_write_rows(op, stage, m0, rows, 128, n0, N);
             }
+            else if (few) tc_write_few(op, stage, rows, n0, N);
             else if (op->i[5] == DT_F32) tc_store_rows<DT_F32>(op, stage, m0, rows, n0, N);
             else if (op->i[5] == DT_F16) tc_store_rows<DT_F16>(op, stage, m0, rows, n0, N);
             else tc_store_rows<DT_BF16>(op, stage, m0, rows, n0, N);

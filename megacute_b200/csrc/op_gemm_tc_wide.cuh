@@ -321,15 +321,6 @@ __device__ __forceinline__ void put4(uint8_t* at, const float4& o) {
     else if (DT == DT_F16) *reinterpret_cast<uint2*>(at) = make_uint2(pack2h(o.x, o.y), pack2h(o.z, o.w));
     else *reinterpret_cast<uint2*>(at) = make_uint2(pack2(o.x, o.y), pack2(o.z, o.w));
 }
-__device__ __forceinline__ float4 load4_any(const uint8_t* base, long long elem, int dtype) {
-    if (dtype == DT_F32) return __ldcg(reinterpret_cast<const float4*>(base + elem * 4));
-    const uint2 v = __ldcg(reinterpret_cast<const uint2*>(base + elem * 2));
-    if (dtype == DT_F16) {
-        const float2 lo = unpack2h(v.x), hi = unpack2h(v.y);
-        return make_float4(lo.x, lo.y, hi.x, hi.y);
-    }
-    return make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
-}
 
 // With a residual (out = acc + bias [times a gate row per i 12 rows: an adaLN-Zero block's gated residual] + residual): kDepth steps of 32
 // columns of the residual are requested ahead, the first while the main loop still runs (an L2 round trip beside the operand

@@ -79,6 +79,15 @@ __device__ __forceinline__ void tc_ld32(uint32_t taddr, float* v) {
 }
 
 
+__device__ __forceinline__ float4 load4_any(const uint8_t* base, long long elem, int dtype) {
+    if (dtype == DT_F32) return __ldcg(reinterpret_cast<const float4*>(base + elem * 4));
+    const uint2 v = __ldcg(reinterpret_cast<const uint2*>(base + elem * 2));
+    if (dtype == DT_F16) {
+        const float2 lo = unpack2h(v.x), hi = unpack2h(v.y);
+        return make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+    return make_float4(bf16_lo(v.x), bf16_hi(v.x), bf16_lo(v.y), bf16_hi(v.y));
+}
 // A thread writes (and, with a residual, reads) whole 32-byte pieces of its own row: whole sectors, as good as 128 bytes of four
 // rows at a time, without the detour through shared memory that the operands of the next tile are streaming through (64
 // bytes a cycle in, 96 out to the tensor core).  DiT, 32 images: 8.95 -> 8.82 ms together with the prefetch of the residual; what is
@@ -105,7 +114,7 @@ __device__ __forceinline__ void ld32B(const uint8_t* at, uint32_t* w, bool whole
         w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w; w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
     }
 }
-// 16 columns of a row as 16-bit, 32 columns of a row
+// 16 columns of a row as 16-bit
 template <int DT>
 __device__ __forceinline__ void put16(uint8_t* at, const float* v, bool whole) {
     uint32_t w[8];
