@@ -532,6 +532,8 @@ def halve_last_tiles(g: Graph, sm_count: int) -> Graph:
     has ended, so the SMs that are free by then take a whole tile and the others, which come later, half of one (two thirds of its time).
     3001 rows, N = 2048, K = 5632: all 96 tiles end after 68 us on 96 SMs, the 32 that start last 25 us behind the rest; now 54 us on 144.
     MLP block of 2400 / 2700 / 3001 rows 164 -> 158, 184 -> 173, 188 -> 181 us, 4 layers of 2900 tokens (K = 8192) 1923 -> 1883.
+    That needs a linear of at least as many products in front: with x from outside the launch all tiles start together (alone, 2500 rows, K = 8192 97.1 ->
+    99.8), and behind a short one nearly so (K = 512 in front, 3000 rows, K = 5632 107.6 -> 109.3).
     With more tiles (128: MLP of 4096 rows 230 both ways) too few SMs are free.  Half tiles move a third more operand bytes per flop, so
     that short products lose where the op behind fills the gap anyway: K = 4096 (DiT of 24 images) 6443 -> 6472, any K 6438 -> 6517."""
     out = g.derive()
@@ -541,7 +543,9 @@ def halve_last_tiles(g: Graph, sm_count: int) -> Graph:
         if op.kind == "Linear" and (op.bm, op.bn) == (C.GEMM_BM_WIDE, C.GEMM_BN_WIDE) and op.cos is None and op.x.cols > C.HALVE_MIN_COLS:
             M, group = op.x.rows, 1 if op.gate is None else op.gate_group
             mt, nt = -(-M // op.bm), op.w.rows // op.bn
-            r = min(mt - 1, (sm_count - mt * nt) // nt) if 4 * mt * nt <= 3 * sm_count else 0
+            front = next((o for o in reversed(ops) if any(v.buf is op.x.buf for v in o.writes)), None)
+            behind = front is not None and front.kind == "Linear" and front.w.rows * front.w.cols >= op.w.rows * op.w.cols
+            r = min(mt - 1, (sm_count - mt * nt) // nt) if behind and 4 * mt * nt <= 3 * sm_count else 0
             m0 = (mt - r) * op.bm
         if r <= 0 or m0 % group or M - m0 <= C.WIDE_MIN_ROWS or os.environ.get("MEGACUTE_B200_WIDE_TILES"):
             ops.append(op)

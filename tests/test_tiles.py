@@ -311,9 +311,11 @@ HALVED = [  # rows, columns, K, residual type, gate group -> row blocks of the t
 ]
 
 
-def halved_graph(M, N, K, rdt, group):
-    g, t = mc.Graph(), {"x": rnd((M, K), 1.0, 1), "w": rnd((N, K), K ** -0.5, 2)}
-    y = g.linear(g.input("x", (M, K)), g.param("w", (N, K)))
+def halved_graph(M, N, K, rdt, group, front=None):
+    """The linear behind another one of K outputs and `front` (as many as it has itself) columns."""
+    front = front or N
+    g, t = mc.Graph(), {"x": rnd((M, front), 1.0, 1), "v": rnd((K, front), front ** -0.5, 5), "w": rnd((N, K), K ** -0.5, 2)}
+    y = g.linear(g.linear(g.input("x", (M, front)), g.param("v", (K, front))), g.param("w", (N, K)))
     if rdt:
         t["r"] = rnd((M, N), 1.0, 3).to(rdt)
         if group:
@@ -328,8 +330,10 @@ def halved_graph(M, N, K, rdt, group):
 def test_which_linears_end_in_half_tiles(monkeypatch, M, N, K, rdt, group, blocks):
     """The two linears cover the rows once, with the operands' rows beside them."""
     monkeypatch.delenv("MEGACUTE_B200_WIDE_TILES", raising=False)
-    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 256))
-    ops = [o for o in passes.run_all(halved_graph(M, N, K, rdt, group)[0], 148).ops if o.kind == "Linear"]
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 256) if a[1] == N else (1, 128, 128))
+    halves = lambda **kw: [o for o in passes.run_all(halved_graph(M, N, K, rdt, group, **kw)[0], 148).ops if o.kind == "Linear" and o.w.buf.name == "w"]
+    assert len(halves(front=N - 8)) == 1                       # (not behind a shorter one; alone: below)
+    ops = halves()
     if blocks is None:
         assert len(ops) == 1 and ops[0].bn == 256
         return
@@ -343,21 +347,28 @@ def test_which_linears_end_in_half_tiles(monkeypatch, M, N, K, rdt, group, block
         assert (a.gate.rows, b.gate.row0, b.gate.rows) == (a.x.rows // group, a.x.rows // group, b.x.rows // group)
 
 
+def test_a_linear_of_the_launchs_inputs_keeps_whole_tiles(monkeypatch):
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 256))
+    g = mc.Graph()
+    g.output(g.linear(g.input("x", (2500, 4160)), g.param("w", (2048, 4160))))
+    assert [o.bn for o in passes.run_all(g, 148).ops] == [256]
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K,rdt,group,blocks", [c for c in HALVED if c[-1]])
 def test_half_tiles_of_the_last_rows(cuda, monkeypatch, M, N, K, rdt, group, blocks):
     """The same bits as whole tiles give (every output is summed over K in the same order), and the oracle's values."""
     monkeypatch.delenv("MEGACUTE_B200_WIDE_TILES", raising=False)
-    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 256))
+    monkeypatch.setattr(passes, "plan_tiles", lambda *a: (1, 256, 256) if a[1] == N else (1, 128, 128))
     g, t = halved_graph(M, N, K, rdt, group)
     dev = {n: u.to(cuda) for n, u in t.items()}
     prog = mc.compile(g)
-    assert [o.bn for o in prog.g.ops if o.kind == "Linear"] == [256, 128]
+    assert [o.bn for o in prog.g.ops if o.kind == "Linear" and o.w.buf.name == "w"] == [256, 128]
     got = prog(**dev).clone()
     prog.check()
     monkeypatch.setattr(passes, "halve_last_tiles", lambda g, sm_count: g)
     whole = mc.compile(g)
-    assert [o.bn for o in whole.g.ops if o.kind == "Linear"] == [256]
+    assert [o.bn for o in whole.g.ops if o.kind == "Linear" and o.w.buf.name == "w"] == [256]
     assert torch.equal(got, whole(**dev))
     ref, _ = evaluate(g, dev, cuda)
     assert rel_l2(got, ref[0]) < TOL
