@@ -439,8 +439,8 @@ __device__ __forceinline__ void norm_stream(const mk_op_desc* op, int r0, int ro
 
 // Plain rows, several per warp (with a gain more than four, without more than one): the row stays in registers, so that it is read from shared memory
 // once and its place is requested again before the sums; 200 bytes per thread saved around it are little beside as many rows.  us per norm in a chain
-// of them, norm_stream / here: 16384 rows of 2048 with a gain 28.0 / 23.7, of 1024 16.3 / 14.6, 9600 of 1152 16.5 / 14.7; without one 16384 of 2048
-// 23.8 / 20.8, of 1024 14.7 / 12.5, 1200 of 1024 3.8 / 3.7.  Prompts and MLP blocks the same (4 x 4096 tokens 9209 and 9246 us, runs differ by 1 %).  With a
+// of them, norm_stream / here: 9600 rows of 2048 with a gain 16.9 / 14.0, of 1024 10.4 / 9.1, of 1152 16.5 / 15.0; without one 9600 of 2048
+// 14.3 / 12.1, of 1152 14.0 / 13.1, 1200 of 1024 3.8 / 3.6.  (Addresses in 64 bits from the start: in 32 the unmodulated rows of 2048 took 13.1.)  Prompts and MLP blocks the same (4 x 4096 tokens 9209 and 9246 us, runs differ by 1 %).  With a
 // gain and up to four rows per warp norm_stream is ahead where other ops lie between (MLP block of 2400 rows 161, 165 in this form).
 template <int NPER, int XDT, int ODT, bool HW>
 __device__ __forceinline__ void norm_kept_rows(const mk_op_desc* op, int r0, int rows) {
@@ -451,9 +451,9 @@ __device__ __forceinline__ void norm_kept_rows(const mk_op_desc* op, int r0, int
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nvec = Cc >> 3;
     const float inv = 1.0f / (float)Cc, eps = op->f[0];
     const long long ldx = op->ld[0], ldo = op->ld[1];
-    const uint8_t* X = reinterpret_cast<const uint8_t*>(op->ptr[0]) + r0 * ldx * (kPlanes * 2);
-    uint16_t* O = reinterpret_cast<uint16_t*>(op->ptr[1]) + r0 * ldo;
-    auto column = [&](int u) { return min(lane + u * 32, nvec - 1) * 8; };
+    const uint8_t* X = reinterpret_cast<const uint8_t*>(op->ptr[0]);
+    void* O = reinterpret_cast<void*>(op->ptr[1]);
+    auto column = [&](int u) { return (long long)min(lane + u * 32, nvec - 1) * 8; };
     uint8_t* buf = smem_map().work + kTcXOff + warp * (kDepth * kRow) + lane * 16;
     auto request = [&](int rr, int slot) {
         if (rr < rows) {
@@ -461,7 +461,7 @@ __device__ __forceinline__ void norm_kept_rows(const mk_op_desc* op, int r0, int
             for (int u = 0; u < NPER; ++u)
 #pragma unroll
                 for (int k = 0; k < kPlanes; ++k)
-                    cp_async16(buf + slot * kRow + (u * kPlanes + k) * 512, X + (rr * ldx + column(u)) * (kPlanes * 2) + k * 16, true);
+                    cp_async16(buf + slot * kRow + (u * kPlanes + k) * 512, X + ((r0 + rr) * ldx + column(u)) * (kPlanes * 2) + k * 16, true);
         }
         cp_async_commit();
     };
@@ -508,15 +508,17 @@ __device__ __forceinline__ void norm_kept_rows(const mk_op_desc* op, int r0, int
         const float rstd = rsqrt_approx(ss * inv - mean * mean + eps);
 #pragma unroll
         for (int u = 0; u < NPER; ++u) {
-            float f[8], g[8];
+            float f[8];
             x[u].get(f);
-            if (HW) unpack8(reinterpret_cast<const uint4*>(gain)[u * 32 + lane], g);
 #pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                f[e] = (f[e] - mean) * rstd;
-                if (HW) f[e] *= g[e];
+            for (int e = 0; e < 8; ++e) f[e] = (f[e] - mean) * rstd;
+            if (HW) {
+                float g[8];
+                unpack8(reinterpret_cast<const uint4*>(gain)[u * 32 + lane], g);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[e] *= g[e];
             }
-            if (lane + u * 32 < nvec) put8<ODT>(O, rr * ldo + (lane + u * 32) * 8, f);
+            if (lane + u * 32 < nvec) put8<ODT>(O, (r0 + rr) * ldo + (lane + u * 32) * 8, f);
         }
     }
 }
