@@ -384,10 +384,11 @@ struct DeviceGuard {
 
 // Tensor map over a row-major bf16 matrix {cols, rows} with row pitch `ld` elements: boxes of 64
 // columns x `box_rows` rows, stored with the 128-byte swizzle (the operand tile layout of the tcgen05 tile
-// GEMM), rows outside the matrix read as zero.  The driver entry point is looked up once; false
+// GEMM), rows outside the matrix read as zero.  `batch` > 0: that many such matrices, one behind the other, in a third dimension, so that
+// a box that goes past the end of one reads zeros and not the next.  The driver entry point is looked up once; false
 // when it is missing or refuses the arguments (the kernel then runs its mma.sync body).
 static bool encode_tile_map(void* out, uint64_t base, long long rows, long long cols, long long ld, int box_rows, bool streamed,
-                            bool fp16 = false) {
+                            bool fp16 = false, long long batch = 0) {
     typedef CUresult (*encode_fn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -403,12 +404,12 @@ static bool encode_tile_map(void* out, uint64_t base, long long rows, long long 
         (void)cudaGetLastError();
     }
     if (!fn || (base & 15) || (ld % 8) || rows <= 0 || cols < 64 || ld < cols) return false;
-    const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
+    const cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
+    const cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)rows * (cuuint64_t)ld * 2};
+    const cuuint32_t box[3] = {64, (cuuint32_t)box_rows, 1};
+    const cuuint32_t estr[3] = {1, 1, 1};
     alignas(64) CUtensorMap m;
-    if (fn(&m, fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, reinterpret_cast<void*>(base), dims, strides, box, estr,
+    if (fn(&m, fp16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, batch > 0 ? 3 : 2, reinterpret_cast<void*>(base), dims, strides, box, estr,
            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
            streamed ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -704,9 +705,9 @@ int mk_program_set_ops(mk_program* p, const mk_op_desc* ops, int n_ops, void* st
             // (that body takes a row's maximum before it scales, and counts masked scores as -inf: the scale has to be positive)
             if (!(d.f[0] > 0.f)) continue;
             const bool h16 = d.i[8] == mk::DT_F16;
-            if (encode_tile_map(maps, d.ptr[0], B * Sq, H * D, d.ld[0], 128, false, h16) &&
-                encode_tile_map(maps + 128, d.ptr[1], B * Sk, KVH * D, d.ld[1], 128, false, h16) &&
-                encode_tile_map(maps + 256, d.ptr[2], B * Sk, KVH * D, d.ld[2], 128, false, h16)) {
+            if (encode_tile_map(maps, d.ptr[0], Sq, H * D, d.ld[0], 128, false, h16, B) &&
+                encode_tile_map(maps + 128, d.ptr[1], Sk, KVH * D, d.ld[1], 128, false, h16, B) &&
+                encode_tile_map(maps + 256, d.ptr[2], Sk, KVH * D, d.ld[2], 128, false, h16, B)) {
                 d.ptr[11] = reinterpret_cast<uint64_t>(p->d_tmaps + (size_t)k * kMapBytes);
                 any_map = true;
                 ++n_attn;

@@ -59,11 +59,13 @@ __device__ __forceinline__ int at_blocks(const mk_op_desc* op, int qi, int t) { 
     return (kend + 127) / 128;
 }
 
-// 2-D tiled bulk tensor copy global -> shared without a cache hint
-__device__ __forceinline__ void tma_load_2d_plain(void* dst, const void* tmap, int x, int y, unsigned long long* bar) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+// 3-D tiled bulk tensor copy global -> shared without a cache hint: columns, rows of a sequence, sequence.  Rows behind a sequence's last one are zeros
+// and not the next sequence's: masked keys have no weight, but what they are multiplied with must be a number (nor need the next
+// sequence's rows have been written yet).
+__device__ __forceinline__ void tma_load_3d_plain(void* dst, const void* tmap, int x, int y, int z, unsigned long long* bar) {
+    asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
                      smem_u32(dst)),
-                 "l"(tmap), "r"(x), "r"(y), "r"(smem_u32(bar))
+                 "l"(tmap), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
                  : "memory");
 }
 // 32 consecutive fp32 columns of this thread's lane, tensor memory <- registers
@@ -151,7 +153,7 @@ __device__ __forceinline__ bool at_feed(const Params& p, Ctrl* c, uint8_t* ring,
                                         uint32_t told) {
     using M = AtMap<D>;
     const int lane = threadIdx.x & 31;
-    const int Sq = op->i[1], Sk = op->i[2], hk = in.a1 / (op->i[3] / op->i[4]);
+    const int Sq = op->i[1], hk = in.a1 / (op->i[3] / op->i[4]);
     const int nb0 = at_blocks(op, in.a2, 0), nb1 = at_blocks(op, in.a2, 1), nb = max(nb0, nb1);
     const uint8_t* tmaps = reinterpret_cast<const uint8_t*>(op->ptr[11]);
     AttnBars* a = &c->attn;
@@ -177,16 +179,15 @@ __device__ __forceinline__ bool at_feed(const Params& p, Ctrl* c, uint8_t* ring,
         ok = wait_barrier(p, c, &a->q_free, (f.insts & 1u) ^ 1u, in.seq, WHERE_RING_EMPTY, 2) &&
              check_phase(p, c, &a->q_full, f.insts & 1u, in.seq, WHERE_CHECK_ARM);
         if (ok) {
-            const int qtiles = in.a2 * 256 + 128 < Sq ? 2 : 1, qrow = in.a0 * Sq + in.a2 * 256;
+            const int qtiles = in.a2 * 256 + 128 < Sq ? 2 : 1;
             mbar_arrive_expect_tx(&a->q_full, (uint32_t)(qtiles * M::kTile));
             ++f.q;
             for (int t = 0; t < qtiles; ++t)
                 for (int s = 0; s < D / 64; ++s)
-                    tma_load_2d_plain(ring + M::kQ + t * M::kTile + s * kTcTileBytes, tmaps, in.a1 * D + s * 64, qrow + t * 128, &a->q_full);
+                    tma_load_3d_plain(ring + M::kQ + t * M::kTile + s * kTcTileBytes, tmaps, in.a1 * D + s * 64, in.a2 * 256 + t * 128, in.a0, &a->q_full);
             c->wide_info[told & 3u] = make_int4(-(nb0 | nb1 << 15), D, op->i[8] == DT_F16 ? 1 : 0, in.seq);
             mbar_arrive(&c->wide_told[told & 3u]);
         }
-        const int krow = in.a0 * Sk;
         for (int j = 0; j < nb && ok; ++j) {
             const uint32_t n = f.tiles + (uint32_t)j, u = n & 1u, ph = (n >> 1) & 1u;
             ok = wait_barrier(p, c, &a->k_empty[u], ph ^ 1u, in.seq, WHERE_RING_EMPTY, 2) && check_phase(p, c, &a->k_full[u], ph, in.seq, WHERE_CHECK_ARM);
@@ -194,13 +195,13 @@ __device__ __forceinline__ bool at_feed(const Params& p, Ctrl* c, uint8_t* ring,
             mbar_arrive_expect_tx(&a->k_full[u], (uint32_t)M::kTile);
             ++f.k;
             for (int s = 0; s < D / 64; ++s)
-                tma_load_2d_plain(ring + M::kK + u * M::kTile + s * kTcTileBytes, tmaps + 128, hk * D + s * 64, krow + j * 128, &a->k_full[u]);
+                tma_load_3d_plain(ring + M::kK + u * M::kTile + s * kTcTileBytes, tmaps + 128, hk * D + s * 64, j * 128, in.a0, &a->k_full[u]);
             ok = wait_barrier(p, c, &a->v_empty[u], ph ^ 1u, in.seq, WHERE_RING_EMPTY, 2) && check_phase(p, c, &a->v_full[u], ph, in.seq, WHERE_CHECK_ARM);
             if (!ok) break;
             mbar_arrive_expect_tx(&a->v_full[u], (uint32_t)M::kTile);
             ++f.v;
             for (int s = 0; s < D / 64; ++s)
-                tma_load_2d_plain(ring + M::kV + u * M::kTile + s * kTcTileBytes, tmaps + 256, hk * D + s * 64, krow + j * 128, &a->v_full[u]);
+                tma_load_3d_plain(ring + M::kV + u * M::kTile + s * kTcTileBytes, tmaps + 256, hk * D + s * 64, j * 128, in.a0, &a->v_full[u]);
         }
     }
     ++f.insts;

@@ -375,6 +375,29 @@ def test_half_tiles_of_the_last_rows(cuda, monkeypatch, M, N, K, rdt, group, blo
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("tcgen05", [True, False])
+@pytest.mark.parametrize("S,D,causal", [(64, 64, False), (64, 128, True), (100, 64, True), (129, 64, False), (200, 128, False), (300, 64, True), (257, 128, True), (7, 64, True)])
+def test_attention_of_sequences_beside_one_that_is_not_numbers(cuda, monkeypatch, S, D, causal, tcgen05):
+    """Keys and values behind a sequence's last one are the next sequence's (or not written yet): they have no weight, whatever they are."""
+    if not tcgen05:
+        monkeypatch.setenv("MEGACUTE_B200_ATTN_TCGEN05", "0")
+    B, H, KVH = 4, 4, 2
+    g = mc.Graph()
+    q, k, v = g.input("q", (B * S, H * D)), g.input("k", (B * S, KVH * D)), g.input("v", (B * S, KVH * D))
+    g.output(g.attention(q, k, v, batch=B, heads=H, kv_heads=KVH, head_dim=D, causal=causal))
+    t = {"q": rnd((B * S, H * D), 1.0, 1), "k": rnd((B * S, KVH * D), 1.0, 2), "v": rnd((B * S, KVH * D), 1.0, 3)}
+    ref, _ = evaluate(g, t)
+    t["k"][S:2 * S], t["v"][S:2 * S], t["v"][3 * S:] = float("nan"), float("nan"), float("inf")
+    prog = mc.compile(g)
+    out = prog(**{n: u.to(cuda) for n, u in t.items()}).float().cpu()
+    prog.check()
+    assert prog.tcgen05_attention_ops == (1 if tcgen05 else 0)
+    for b in (0, 2):
+        assert rel_l2(out[b * S:(b + 1) * S], ref[0][b * S:(b + 1) * S]) < TOL
+    assert not torch.isfinite(out[S:2 * S]).any() and not torch.isfinite(out[3 * S:]).any()
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("scale", [-0.3, 0.0])
 @pytest.mark.parametrize("D", [64, 128])
 def test_prefill_attention_scale_not_positive(cuda, D, scale):
