@@ -174,8 +174,8 @@ __device__ __forceinline__ bool tc_direct_wait(const Params& p, Ctrl* c, uint32_
     return ok != 0;
 }
 // an activation chosen at run time on 16 values.  The common ones side by side, the others four at a time (rotated: register indices stay constant).
-// 64 rows of 256 columns, us per linear, the writer through shared memory that had this before / this: silu 10.5 / 7.8, gelu 10.6 / 7.2, silu and
-// a residual 11.4 / 9.1; all of them rotated, silu took 0.6 more than side by side.
+// us per linear of 256 columns, the writer through shared memory that had this before / all of them rotated / this: 64 rows, silu 10.6 / 13.0 / 8.1, relu
+// 10.3 / 11.5 / 7.3, gelu and a residual 11.4 / 14.9 / 9.2; 200 rows, silu 14.9 / 13.1 / 8.1.
 __device__ __forceinline__ void act16(int act, float* v) {
     if (act == ACT_SILU) {
 #pragma unroll

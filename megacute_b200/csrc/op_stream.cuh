@@ -525,9 +525,9 @@ __device__ __forceinline__ void norm_kept_rows(const mk_op_desc* op, int r0, int
 
 // Modulated rows whose scale and shift rows change with every row or every two or three (up to 1024 columns): each warp requests its row's own in front
 // of the sums, into registers.  In shared memory, as above, they change up to eight times in eight rows, with two barriers and a round
-// trip to L2 each.  us per norm, above / here: 9600 rows of 1024 with a scale row each 101 / 26, of 512 89 / 24, 1200 rows of 1024 14 / 6, 300 rows
-// 4.1 / 3.4.  (With four rows per scale row the form above is faster up to 600 rows, 300 of 1024 3.2 / 3.4, and 256 bytes per thread are saved
-// around this one.)
+// trip to L2 each.  us per norm, above / here: 9600 rows of 1024 with a scale row each 102 / 23, of 512 80 / 20, 1200 rows of 1024 20 / 5.9, 300 rows
+// 7.2 / 6.9; two rows per scale row 49 / 21, 42 / 20, 11 / 5.9, 6.9 / 6.9.  (256 bytes per thread are saved around this body; four rows per scale row take
+// 7.1 above for 1200 rows of 1024, less than the 7.4 they took with everything in registers.)
 template <int XDT, int ODT>
 __device__ __forceinline__ void norm_own(const mk_op_desc* op, int r0, int rows) {
     constexpr int NPER = 4, kPlanes = XDT == DT_F32 ? 2 : 1, kRow = NPER * kPlanes * 512, kDepth = (kWorkBytes - kTcXOff) / kComputeWarps / kRow;
