@@ -132,9 +132,9 @@ int mk_program_set_direct(mk_program* p, void* memory, size_t bytes, void* strea
 /* One launch of the persistent kernel on `stream` (asynchronous).  Replaces
  * self._compiled(views, insts, waits, arrives, counters, trace, epoch) (runtime.py:383-384);
  * the launch epoch is kept inside the program and the counters are cleared only before it would
- * overflow (runtime.py:377-380).  The epoch is an argument of the launch: one captured into a CUDA graph
- * is for a single replay, in the order of the captures.  A further replay finds the counters of the one
- * before and orders nothing (mk_launch_noalloc clears its counters itself and may be replayed). */
+ * overflow (runtime.py:377-380).  A launch may be captured into a CUDA graph and replayed, by itself or between
+ * other launches of the program, one at a time: from the first captured one on each launch clears the
+ * counters first.  Operands are those bound when the graph runs; bind them before the capture. */
 int mk_launch(mk_program* p, void* stream);
 
 /* Longest time any device-side wait may spin before the launch gives up with MK_DEV_TIMEOUT_*. */

@@ -342,6 +342,7 @@ struct mk_program {
     uint8_t* direct = nullptr;       // direct operands (mk_program_set_direct): two copies of direct_bytes
     size_t direct_bytes = 0;
     int direct_turn = 0;             // ... the copy that the next launch uses
+    bool captured = false;           // a launch has been captured: all from then on clear what they count and wait for (mk_launch)
 };
 
 static const size_t kMapBytes = 512;       // tensor-map space per op
@@ -810,11 +811,21 @@ int mk_launch(mk_program* p, void* stream) {
     if (!p) return MK_E_ARG;
     MK_ON_DEVICE(p->device);
     cudaStream_t st = (cudaStream_t)stream;
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) {
+        (void)cudaGetLastError();
+        capturing = cudaStreamCaptureStatusInvalidated;
+    }
+    // The epoch and the copy of the direct operands are arguments of the launch, so a captured one has them for good.  From the first captured
+    // launch on, each clears the counters, marks its copy of the direct operands and is the first of its epoch, captured or not: a
+    // replay waits for its own values, whatever ran in between.  (A memset or two per launch, 2 us each, that other programs do without.)
+    if (capturing == cudaStreamCaptureStatusActive) p->captured = true;
     const int max_epoch = 0x7fffffff / (p->max_target > 0 ? p->max_target : 1) - 1;
-    if (p->epoch >= max_epoch) {
+    if (p->captured || p->epoch >= max_epoch) {
         MK_CUDA(cudaMemsetAsync(p->d_counters, 0, (size_t)p->n_counters * 4, st));
         p->epoch = 0;
     }
+    if (p->captured && p->direct) MK_CUDA(cudaMemsetAsync(p->direct + (p->direct_turn ? p->direct_bytes : 0), 0xff, p->direct_bytes, st));
     p->epoch += 1;
     p->last_stream = st;
     mk::Params prm;
@@ -840,11 +851,6 @@ int mk_launch(mk_program* p, void* stream) {
     // SMs' shared memory while they wait, and those without an SM come when it ends.  All are resident together then, as the schedule needs.)
     // A launch behind another 2 us earlier: MLP block of one row 25.4 -> 23.5 us, of 64 35.6 -> 33.5, of 256 52.7 -> 50.6.  A captured
     // launch has ordinary edges.
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &capturing) != cudaSuccess) {
-        (void)cudaGetLastError();
-        capturing = cudaStreamCaptureStatusActive;
-    }
     cudaLaunchAttribute attr;
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;

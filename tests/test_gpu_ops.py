@@ -512,6 +512,44 @@ def test_launches_behind_kernels_that_write_their_inputs(cuda, M, where):
         assert torch.equal(out[i], want[i]), i
 
 
+@pytest.mark.parametrize("M", [1, 4, 64])
+def test_replays_of_a_captured_launch(cuda, M):
+    """A graph of one launch, replayed: each replay waits for its own values, in private buffers that hold no numbers and behind replays and
+    launches with other inputs."""
+    K = 4096 if M == 1 else 512                  # (one row: direct operands)
+    g = mc.Graph()
+    y = g.input("x", (M, K))
+    for i in range(4):
+        y = g.linear(g.rms_norm(y, g.param("n", (1, K)), eps=1e-5), g.param(f"w{i}", (K, K)), act="gelu_tanh")
+    g.output(y)
+    prog = mc.compile(g)
+    t = {"n": rnd((1, K), 0.1, 20, 1.0).to(cuda), **{f"w{i}": rnd((K, K), 2 * K ** -0.5, 21 + i).to(cuda) for i in range(4)}}
+    xs = [rnd((M, K), 1.0, i).to(cuda) for i in range(5)]
+    x = torch.zeros_like(xs[0])
+    want = [prog(x=v, **t).clone() for v in xs]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        prog(x=x, **t)
+    side.synchronize()
+    assert len(prog.direct) == (3 if M == 1 else len(prog.direct))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        out = prog(x=x, **t)
+    private = [prog._bufs[b.id] for b in prog.g.buffers if b.kind == "temp" and b.id not in prog.direct]
+    for k in (0, 1, 2, 3, 4, 1, 0):
+        for b in private:
+            b.fill_(float("nan"))
+        x.copy_(xs[k])
+        graph.replay()
+        torch.cuda.synchronize()
+        assert rel_l2(out.float().cpu(), want[k].float().cpu()) < TOL, k
+        if k in (2, 4):                          # a launch of its own between replays
+            x.copy_(xs[3])
+            assert rel_l2(prog(x=x, **t).float().cpu(), want[3].float().cpu()) < TOL
+    prog.check()
+
+
 def test_values_that_are_nan_end_the_wait(cuda):
     """NaN inputs reach the output as NaN through direct operands; the rows beside them and the launches after are right.  (The input has
     all 16 bits set.  No op can produce the 32-bit marker itself: arithmetic makes 0x7fffffff, an embedding's low half is 0.)"""
